@@ -27,6 +27,9 @@ enum FlagWord : int {
     FLAG_DIV_ZERO   = 0, // a divisor was 0 (reference: "Division by zero")
     FLAG_LOG_DOMAIN = 1, // an input of log was <= 0
     FLAG_TIMEOUT    = 2, // a bounded in-kernel wait ran out (value = 1 + the block that gave up)
+    FLAG_WIDE       = 4, // an operand of the product being prepared does not fit float16 pairs (half_split.cuh);
+                         // cleared by the product's own kernel
+    FLAG_WIDE_READERS = 5, // CTAs of that kernel that have read it
     FLAG_COUNT      = 8
 };
 
@@ -120,20 +123,36 @@ __device__ __forceinline__ void griddep_launch_dependents() {
 }
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_dependent(
-    void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args &&...args) {
+inline cudaError_t launch_dependent_cluster(
+    void (*kernel)(KArgs...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args &&...args) {
     static const bool enabled = getenv("CAMEL_TENSOR_NO_PDL") == nullptr;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim          = grid;
     cfg.blockDim         = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream           = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
     cfg.attrs    = attr;
-    cfg.numAttrs = enabled && !profiling_enabled() ? 1 : 0;
+    cfg.numAttrs = 0;
+    if (cluster > 1) {
+        attr[cfg.numAttrs].id               = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = (unsigned)cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
+    }
+    if (enabled && !profiling_enabled()) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+        ++cfg.numAttrs;
+    }
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_dependent(
+    void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args &&...args) {
+    return launch_dependent_cluster(kernel, 1, grid, block, smem, s, std::forward<Args>(args)...);
 }
 #endif
 
@@ -156,7 +175,8 @@ inline bool valid_dtype(int dt) { return dt == CT_F32 || dt == CT_I64 || dt == C
 
 // Entry points of the other translation units used across files.
 // The B operand of a float32 GEMM already in the layout the tensor-core kernel reads: transposed
-// [n][kp] hi/lo planes (3xTF32) or one bf16 plane, built once from a [k][n] weight matrix.
+// [n][kp] hi/lo planes (tf32, and scaled float16 pairs where the matrix fits them) or one bf16 plane, built
+// once from a [k][n] weight matrix.
 struct PackedWeights {
     uint32_t magic;
     int mode;
@@ -165,12 +185,55 @@ struct PackedWeights {
     const float *src; // the matrix the planes were built from
     void *base;       // one device allocation holding the planes
     void *hi, *lo;
+    void *hi16, *lo16; // float16 planes and inverse column scales; null: the matrix needs tf32
+    float *scale;
 };
 constexpr uint32_t kPackedMagic = 0x43545057u; // "CTPW"
 
 ct_status gemm_f32_tc(
     DeviceState *st, const float *a, const float *b, const float *bias, int64_t m, int64_t k,
     int64_t n, int act, float *out, const PackedWeights *packed = nullptr, bool a_is_km = false);
+// One operand of gemm_half (gemm_half.cu): K-major planes [rows][kp] of float16 pairs with an inverse scale
+// per row, and of tf32 terms, which are read instead where *wide is non-zero (or the caller forces it).
+struct HalfOperand {
+    const void *hi16, *lo16;
+    const float *scale;
+    const void *hi32, *lo32;
+    const uint32_t *wide;
+    int64_t rows;
+};
+// Row bands of one launch, see ct_matmul_packed_bands.
+struct HalfBands {
+    int bands = 0;
+    int first[9];
+    int64_t out_off[8];
+    uint32_t *done = nullptr;
+};
+// out[z][m][n] = act(A . B[z]^T + bias) over prepared planes, B holding `batch` operands of b.rows / batch rows.  own_flag: the operands' word is FLAG_WIDE of the
+// device state, which the launch clears for the next product.
+ct_status gemm_half(
+    DeviceState *st, const HalfOperand &a, const HalfOperand &b, int64_t kp, const float *bias, int act, float *out,
+    bool force_wide, bool own_flag, bool allow_splitk, const HalfBands *bands, int batch = 1, bool bias_per_row = false);
+int half_tile_columns(const DeviceState *st, int64_t m, int64_t n, int64_t batch = 1);
+// Pre-passes: rows of a row-major matrix, columns of one (transposed planes); both raise *wide.  `zero`
+// words are cleared on the way (col_max of a following half_split_cols, which needs them at zero).
+// both_forms: the tf32 planes are written as well (no half_wide_planes needed).
+ct_status half_split_rows(
+    DeviceState *st, const float *in, int64_t k, int64_t kp, const HalfOperand &o, bool both_forms, uint32_t *zero,
+    int64_t zero_count);
+bool half_cols_is_short(int64_t kp); // one pass, which needs no col_max and can write both forms
+ct_status half_split_cols(
+    DeviceState *st, const float *in, int64_t k, int64_t kp, const HalfOperand &o, bool both_forms, uint32_t *col_max);
+ct_status half_split_both(
+    DeviceState *st, const float *a, const HalfOperand &oa, const float *b, const HalfOperand &ob, int64_t k, int64_t kp,
+    bool both_forms, bool *done);
+// tf32 planes of both operands where *wide is set (n == 0 / m == 0: that operand has them already).
+ct_status half_wide_planes(
+    DeviceState *st, const uint32_t *wide, const float *a, int64_t m, bool a_is_km, void *a_hi, void *a_lo, const float *b,
+    int64_t n, void *b_hi, void *b_lo, int64_t k, int64_t kp);
+ct_status half_widen_rows(
+    DeviceState *st, const uint32_t *wide, const void *hi16, const void *lo16, const float *scale, int64_t rows, int64_t kp,
+    void *hi32, void *lo32);
 // Geometry of a stride-1 convolution run as an implicit GEMM over NHWC input planes.
 struct ConvGeom {
     int c_pad;  // channels rounded up to the k-block

@@ -111,13 +111,7 @@ struct GemmParams {
 
 // The band plan of the product being enqueued (set under the entry point's lock by
 // ct_matmul_packed_bands, read by launch_gemm); bands == 0: none.
-struct BandPlan {
-    int bands = 0;
-    int first[9];
-    int64_t out_off[8];
-    uint32_t *done = nullptr;
-};
-BandPlan g_band_plan;
+HalfBands g_band_plan;
 
 // ---- operand pre-pass ---------------------------------------------------------------------
 
@@ -1299,8 +1293,8 @@ ct_status encode_fn(EncodeTiledFn *out) {
 
 } // namespace
 
-ct_status encode_tiled_map_f32(
-    CUtensorMap *map, const void *base, int rank, const uint64_t *dims, const uint64_t *strides, const uint32_t *box,
+static ct_status encode_tiled_map(
+    CUtensorMapDataType type, CUtensorMap *map, const void *base, int rank, const uint64_t *dims, const uint64_t *strides, const uint32_t *box,
     int swizzle_bytes) {
     EncodeTiledFn fn;
     CT_TRY(encode_fn(&fn));
@@ -1314,7 +1308,7 @@ ct_status encode_tiled_map_f32(
             s[i] = strides[i];
     }
     CUresult r = fn(
-        map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (cuuint32_t)rank, const_cast<void *>(base), d, s, b, e,
+        map, type, (cuuint32_t)rank, const_cast<void *>(base), d, s, b, e,
         CU_TENSOR_MAP_INTERLEAVE_NONE,
         swizzle_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
                              : (swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE),
@@ -1322,6 +1316,18 @@ ct_status encode_tiled_map_f32(
     if (r != CUDA_SUCCESS)
         return fail(CT_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
     return CT_OK;
+}
+
+ct_status encode_tiled_map_f32(
+    CUtensorMap *map, const void *base, int rank, const uint64_t *dims, const uint64_t *strides, const uint32_t *box,
+    int swizzle_bytes) {
+    return encode_tiled_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, map, base, rank, dims, strides, box, swizzle_bytes);
+}
+
+ct_status encode_tiled_map_f16(
+    CUtensorMap *map, const void *base, int rank, const uint64_t *dims, const uint64_t *strides, const uint32_t *box,
+    int swizzle_bytes) {
+    return encode_tiled_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, map, base, rank, dims, strides, box, swizzle_bytes);
 }
 
 namespace {
@@ -1672,6 +1678,63 @@ ct_status split_rows_planes(
 // Largest k for which the kernel's int32 TMA coordinates and k-block counter are safe.
 constexpr int64_t kMaxDim = 1ll << 30;
 
+// The float32 product in split float16 (gemm_half.cu).  Workspace: inverse scales and column maxima, then
+// the operand planes - float16 pairs, or, where the pre-pass finds a row too wide for them, the tf32 planes
+// in the same place (the product reads one or the other), so no more than tf32 planes alone would take.
+// Operands whose tf32 planes are at most kBothFormsBytes get them at once, next to the float16 ones: at
+// 512^3 those 4 MB stay in L2 and cost less than the conditional launch (about 2 us).
+constexpr int64_t kBothFormsBytes = 4 << 20;
+
+static ct_status gemm_f32_split(
+    DeviceState *st, const float *a, const float *b, const float *bias, int64_t m, int64_t k, int64_t n, int64_t kp,
+    int act, float *out, const PackedWeights *packed, bool a_is_km) {
+    auto align_up         = [](size_t v) { return (v + 1023) & ~(size_t)1023; };
+    const size_t a32      = align_up((size_t)m * kp * 4), b32 = packed ? 0 : align_up((size_t)n * kp * 4);
+    const size_t a16      = align_up((size_t)m * kp * 2), b16 = packed ? 0 : align_up((size_t)n * kp * 2);
+    const size_t a_words  = align_up((size_t)m * 4), b_words = align_up((size_t)n * 4);
+    const bool both_forms = half_cols_is_short(kp) && 8 * (m + (packed ? 0 : n)) * kp <= kBothFormsBytes;
+    const size_t wide_at  = both_forms ? 2 * (a16 + b16) : 0; // where the tf32 planes start
+    CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, 2 * a_words + 2 * b_words + wide_at + 2 * (a32 + b32)));
+    uint8_t *ws     = static_cast<uint8_t *>(st->gemm_ws);
+    float *a_scale  = reinterpret_cast<float *>(ws), *b_scale = reinterpret_cast<float *>(ws + 2 * a_words);
+    uint32_t *a_max = reinterpret_cast<uint32_t *>(ws + a_words);
+    uint32_t *b_max = reinterpret_cast<uint32_t *>(ws + 2 * a_words + b_words);
+    uint8_t *p16 = ws + 2 * a_words + 2 * b_words, *p32 = p16 + wide_at;
+    uint32_t *wide = st->flags_dev + FLAG_WIDE;
+    HalfOperand oa{p16, p16 + a16, a_scale, p32, p32 + a32, wide, m};
+    HalfOperand ob{p16 + 2 * a16, p16 + 2 * a16 + b16, b_scale, p32 + 2 * a32, p32 + 2 * a32 + b32, wide, n};
+    const bool force_wide = packed && !packed->hi16;
+    if (packed) {
+        ob.hi32 = packed->hi, ob.lo32 = packed->lo, ob.scale = packed->scale;
+        ob.hi16 = force_wide ? packed->hi : packed->hi16, ob.lo16 = force_wide ? packed->lo : packed->lo16;
+    }
+    {
+        ProfScope prof("gemm_prepass");
+        const bool two_pass = !half_cols_is_short(kp); // columns longer than a block's shared memory
+        bool both           = false;                   // one launch for both operands
+        if (force_wide)
+            CT_TRY(split_rows_planes(st, MODE_3X, a, m, k, kp, const_cast<void *>(oa.hi32), const_cast<void *>(oa.lo32)));
+        else if (!packed && !a_is_km)
+            CT_TRY(half_split_both(st, a, oa, b, ob, k, kp, both_forms, &both));
+        if (!force_wide && !both) {
+            if (a_is_km && two_pass)
+                CT_CUDA(cudaMemsetAsync(a_max, 0, a_words, stream()));
+            if (a_is_km && !packed && two_pass)
+                CT_CUDA(cudaMemsetAsync(b_max, 0, b_words, stream()));
+            if (a_is_km)
+                CT_TRY(half_split_cols(st, a, k, kp, oa, both_forms, a_max));
+            else
+                CT_TRY(half_split_rows(st, a, k, kp, oa, both_forms, b_max, !packed && two_pass ? n : 0));
+            if (!packed)
+                CT_TRY(half_split_cols(st, b, k, kp, ob, both_forms, b_max));
+        }
+        if (!force_wide && !both_forms)
+            CT_TRY(half_wide_planes(st, wide, a, m, a_is_km, const_cast<void *>(oa.hi32), const_cast<void *>(oa.lo32), b,
+                                    packed ? 0 : n, const_cast<void *>(ob.hi32), const_cast<void *>(ob.lo32), k, kp));
+    }
+    return gemm_half(st, oa, ob, kp, bias, act, out, force_wide, !force_wide, true, nullptr);
+}
+
 ct_status gemm_f32_tc(
     DeviceState *st, const float *a, const float *b, const float *bias, int64_t m, int64_t k,
     int64_t n, int act, float *out, const PackedWeights *packed, bool a_is_km) {
@@ -1697,6 +1760,8 @@ ct_status gemm_f32_tc(
                 CT_ERR_INVALID,
                 "dense: the packed weights were built from another matrix, shape, precision or device");
     }
+    if (mode == MODE_3X)
+        return gemm_f32_split(st, a, b, bias, m, k, n, kp, act, out, packed, a_is_km);
     size_t a_plane      = align_up((size_t)m * kp * elem);
     size_t b_plane      = packed ? 0 : align_up((size_t)n * kp * elem);
     size_t total        = planes * (a_plane + b_plane);
@@ -1716,10 +1781,7 @@ ct_status gemm_f32_tc(
         dim3 grid((unsigned)((m + 31) / 32), (unsigned)(kp / 32));
         if (grid.y > 65535)
             return fail(CT_ERR_TOO_LARGE, "gemm: k too large for the operand pre-pass");
-        if (mode == MODE_3X)
-            split_transpose_kernel<MODE_3X><<<grid, 256, 0, stream()>>>(a, k, m, kp, a_hi, a_lo);
-        else
-            split_transpose_kernel<MODE_BF><<<grid, 256, 0, stream()>>>(a, k, m, kp, a_hi, a_lo);
+        split_transpose_kernel<MODE_BF><<<grid, 256, 0, stream()>>>(a, k, m, kp, a_hi, a_lo);
         CT_LAUNCH_CHECK("split_transpose");
     } else {
         ProfScope prof("gemm_prepass");
@@ -1730,10 +1792,7 @@ ct_status gemm_f32_tc(
         dim3 grid((unsigned)((n + 31) / 32), (unsigned)(kp / 32));
         if (grid.y > 65535)
             return fail(CT_ERR_TOO_LARGE, "gemm: k too large for the operand pre-pass");
-        if (mode == MODE_3X)
-            split_transpose_kernel<MODE_3X><<<grid, 256, 0, stream()>>>(b, k, n, kp, b_hi, b_lo);
-        else
-            split_transpose_kernel<MODE_BF><<<grid, 256, 0, stream()>>>(b, k, n, kp, b_hi, b_lo);
+        split_transpose_kernel<MODE_BF><<<grid, 256, 0, stream()>>>(b, k, n, kp, b_hi, b_lo);
         CT_LAUNCH_CHECK("split_transpose");
     }
 
@@ -1766,9 +1825,31 @@ extern "C" ct_status ct_weights_pack(const float *w, int64_t k, int64_t n, void 
     dim3 grid((unsigned)((n + 31) / 32), (unsigned)(kp / 32));
     if (grid.y > 65535)
         return fail(CT_ERR_TOO_LARGE, "ct_weights_pack: k too large for the operand pre-pass");
+    // 3xTF32: the float16 pairs that products normally read, and the tf32 planes for a left operand (or
+    // these weights) too wide for them; [hi][lo][hi16][lo16][scale][col max][word]
+    const size_t plane16 = mode == MODE_3X ? ((size_t)n * kp * 2 + 1023) & ~(size_t)1023 : 0;
+    const size_t words   = mode == MODE_3X ? ((size_t)n * 4 + 1023) & ~(size_t)1023 : 0;
     void *base = nullptr;
-    CT_TRY(ct_alloc(&base, plane * planes));
+    CT_TRY(ct_alloc(&base, plane * planes + 2 * plane16 + 2 * words + (mode == MODE_3X ? 4 : 0)));
     void *hi = base, *lo = static_cast<uint8_t *>(base) + plane;
+    uint8_t *half_base = static_cast<uint8_t *>(base) + plane * planes;
+    void *hi16 = nullptr, *lo16 = nullptr;
+    float *scale   = nullptr;
+    uint32_t *wide = nullptr;
+    if (mode == MODE_3X) {
+        hi16 = half_base, lo16 = half_base + plane16;
+        scale = reinterpret_cast<float *>(half_base + 2 * plane16);
+        wide  = reinterpret_cast<uint32_t *>(half_base + 2 * plane16 + 2 * words);
+        ProfScope prof("weights_pack");
+        uint32_t *col_max = reinterpret_cast<uint32_t *>(half_base + 2 * plane16 + words);
+        cudaError_t e     = cudaMemsetAsync(col_max, 0, words + 4, stream());
+        ct_status s       = e != cudaSuccess ? cuda_fail(e, "weights_pack")
+                                             : half_split_cols(st, w, k, kp, HalfOperand{hi16, lo16, scale, nullptr, nullptr, wide, n}, false, col_max);
+        if (s != CT_OK) {
+            ct_free(base);
+            return s;
+        }
+    }
     {
         ProfScope prof("weights_pack");
         if (mode == MODE_3X)
@@ -1783,14 +1864,19 @@ extern "C" ct_status ct_weights_pack(const float *w, int64_t k, int64_t n, void 
         count_launch(1);
     }
     // the handle may be used from any stream afterwards: finish the one-time pass here
-    cudaError_t se = cudaStreamSynchronize(stream());
+    uint32_t is_wide = 0;
+    cudaError_t se   = wide ? cudaMemcpyAsync(&is_wide, wide, sizeof(is_wide), cudaMemcpyDeviceToHost, stream()) : cudaSuccess;
+    if (se == cudaSuccess)
+        se = cudaStreamSynchronize(stream());
     if (se != cudaSuccess) {
         ct_free(base);
         return cuda_fail(se, "weights_pack");
     }
+    if (is_wide)
+        hi16 = lo16 = nullptr;
     int dev = -1;
     CT_CUDA(cudaGetDevice(&dev));
-    PackedWeights *pw = new PackedWeights{kPackedMagic, mode, dev, k, n, kp, w, base, hi, lo};
+    PackedWeights *pw = new PackedWeights{kPackedMagic, mode, dev, k, n, kp, w, base, hi, lo, hi16, lo16, scale};
     *packed_out       = pw;
     return CT_OK;
 }
@@ -1824,6 +1910,11 @@ struct PackedRows {
     void *base;
     uint8_t *hi, *lo;
     size_t row_bytes; // bytes of one row of a plane
+    // 3xTF32: float16 pairs, inverse row scales and the word that says that the rows need the tf32 planes
+    // (hi, lo), which are written only then
+    uint8_t *hi16, *lo16;
+    float *scale;
+    uint32_t *wide;
 };
 constexpr uint32_t kPackedRowsMagic = 0x43545052u; // "CTPR"
 
@@ -1848,15 +1939,23 @@ extern "C" ct_status ct_rows_pack(const float *a, int64_t m, int64_t k, void **p
     if (pr && (pr->magic != kPackedRowsMagic || pr->mode != mode || pr->m != m || pr->k != k || pr->device != dev))
         return fail(CT_ERR_INVALID, "ct_rows_pack: the handle belongs to another shape, precision or device");
     if (!pr) {
-        const size_t plane = ((size_t)m * kp * elem + 1023) & ~(size_t)1023;
-        void *base         = nullptr;
-        CT_TRY(ct_alloc(&base, plane * planes));
-        uint8_t *hi = static_cast<uint8_t *>(base);
-        pr          = new PackedRows{kPackedRowsMagic, mode, dev, m, k, kp, base, hi, hi + plane, (size_t)kp * elem};
+        const size_t plane   = ((size_t)m * kp * elem + 1023) & ~(size_t)1023;
+        const size_t plane16 = mode == MODE_3X ? ((size_t)m * kp * 2 + 1023) & ~(size_t)1023 : 0;
+        const size_t words   = mode == MODE_3X ? ((size_t)m * 4 + 1023) & ~(size_t)1023 : 0;
+        void *base           = nullptr;
+        CT_TRY(ct_alloc(&base, plane * planes + 2 * plane16 + words + (mode == MODE_3X ? 4 : 0)));
+        uint8_t *hi = static_cast<uint8_t *>(base), *hi16 = hi + plane * planes;
+        pr          = new PackedRows{kPackedRowsMagic, mode, dev, m, k, kp, base, hi, hi + plane, (size_t)kp * elem, hi16,
+                                     hi16 + plane16, reinterpret_cast<float *>(hi16 + 2 * plane16),
+                                     reinterpret_cast<uint32_t *>(hi16 + 2 * plane16 + words)};
         *packed_inout = pr;
     }
     ProfScope prof("gemm_prepass");
-    return split_rows_planes(st, mode, a, m, k, kp, pr->hi, pr->lo);
+    if (mode != MODE_3X)
+        return split_rows_planes(st, mode, a, m, k, kp, pr->hi, pr->lo);
+    CT_CUDA(cudaMemsetAsync(pr->wide, 0, sizeof(uint32_t), stream()));
+    CT_TRY(half_split_rows(st, a, k, kp, HalfOperand{pr->hi16, pr->lo16, pr->scale, nullptr, nullptr, pr->wide, m}, false, nullptr, 0));
+    return half_wide_planes(st, pr->wide, a, m, false, pr->hi, pr->lo, nullptr, 0, nullptr, nullptr, k, kp);
 }
 
 extern "C" ct_status ct_rows_free(void *packed) {
@@ -1869,6 +1968,23 @@ extern "C" ct_status ct_rows_free(void *packed) {
     ct_status st = ct_free(pr->base);
     delete pr;
     return st;
+}
+
+// Rows [row0, row0 + rows) of a packed left operand times packed weights, split float16 or tf32.
+static ct_status gemm_packed_rows(
+    DeviceState *st, const PackedRows *pr, int64_t row0, int64_t rows, const PackedWeights *pw, float *out,
+    const HalfBands *bands) {
+    const size_t at = (size_t)row0 * pr->kp;
+    HalfOperand oa{pr->hi16 + at * 2, pr->lo16 + at * 2, pr->scale + row0, pr->hi + at * 4, pr->lo + at * 4, pr->wide, rows};
+    HalfOperand ob{pw->hi16, pw->lo16, pw->scale, pw->hi, pw->lo, pr->wide, pw->n};
+    const bool force_wide = pw->hi16 == nullptr;
+    if (force_wide) {
+        // each call widens the rows it reads: calls on several streams share no state
+        ob.hi16 = pw->hi, ob.lo16 = pw->lo;
+        CT_TRY(half_widen_rows(st, pr->wide, oa.hi16, oa.lo16, oa.scale, rows, pr->kp, const_cast<void *>(oa.hi32),
+                               const_cast<void *>(oa.lo32)));
+    }
+    return gemm_half(st, oa, ob, pr->kp, nullptr, CT_ACT_NONE, out, force_wide, false, false, bands);
 }
 
 extern "C" ct_status ct_matmul_packed_rows(
@@ -1890,6 +2006,8 @@ extern "C" ct_status ct_matmul_packed_rows(
         return CT_OK;
     if (!out)
         return fail(CT_ERR_INVALID, "ct_matmul_packed_rows: null pointer");
+    if (pr->mode == MODE_3X)
+        return gemm_packed_rows(st, pr, row0, rows, pw, out, nullptr);
     g_no_splitk   = true; // the split-K partial sums live in a shared workspace
     ct_status res = gemm_planes(
         st, pr->mode, pr->hi + (size_t)row0 * pr->row_bytes, pr->lo + (size_t)row0 * pr->row_bytes, pw->hi, pw->lo,
@@ -1920,7 +2038,7 @@ extern "C" ct_status ct_matmul_packed_bands(
         return fail(CT_ERR_INVALID, "ct_matmul_packed_bands: operands of different inner size, precision or device");
     if (nbands < 1 || nbands > 8 || !band_rows_host || !band_out_host || !band_done_dev)
         return fail(CT_ERR_INVALID, "ct_matmul_packed_bands: 1 to 8 bands, with rows, outputs and counters");
-    BandPlan plan;
+    HalfBands plan;
     plan.bands   = nbands;
     plan.done    = band_done_dev;
     int64_t row  = 0;
@@ -1945,6 +2063,8 @@ extern "C" ct_status ct_matmul_packed_bands(
     for (int b = 0; b < nbands; ++b)
         if (band_tiles_host)
             band_tiles_host[b] = (uint32_t)((plan.first[b + 1] - plan.first[b]) * tiles_n);
+    if (pr->mode == MODE_3X)
+        return gemm_packed_rows(st, pr, 0, pr->m, pw, band_out_host[0], &plan);
     g_no_splitk   = true; // the split-K partial sums live in a shared workspace
     g_band_plan   = plan;
     ct_status res = gemm_planes(st, pr->mode, pr->hi, pr->lo, pw->hi, pw->lo, pr->m, pw->n, pr->kp, nullptr, CT_ACT_NONE,

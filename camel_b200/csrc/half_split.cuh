@@ -1,0 +1,54 @@
+// Splitting float32 matrices into scaled float16 pairs for the tensor-core contractions.
+//
+// A float32 value is carried as two 11-bit significands, as in the 3xTF32 split (split.cuh), but in
+// float16, whose MMAs take 16 values of k in the time a tf32 MMA takes 8 and whose planes are half as
+// large.  float16's five exponent bits are made up for by an exact power of two per row of the left
+// operand and per column of the right one (the row's largest magnitude is moved to [2^14, 2^15)) and by
+// storing the low term 2^11 times larger:
+//     v * 2^(14-e) = hi + lo * 2^-11,   hi = half(v * 2^(14-e)),   lo = half((v * 2^(14-e) - hi) * 2^11)
+// For |v| >= 2^-28 of its row's largest value that is v to 22 bits, exactly the 3xTF32 representation
+// (both terms convert to tf32 without rounding).  Below, hi becomes subnormal and the error stays at
+// 2^-36 of the scaled value: still 2^-17 relative at 2^-33 of the largest.  A matrix with a smaller
+// non-zero value than that, or a row whose exponent is beyond +-60, raises a device word, and the
+// product is then computed from tf32 planes instead (same launch sequence, no host involvement).
+#pragma once
+
+#include <cuda_fp16.h>
+
+#include <cstdint>
+
+namespace ct {
+
+constexpr float kHalfLoScale    = 2048.0f;              // 2^11
+constexpr float kHalfLoInv      = 1.0f / 2048.0f;
+constexpr float kHalfSmallest   = 1.0f / (1u << 19);    // scaled magnitudes below this lose more than 2^-17
+constexpr int kHalfMaxExponent  = 60;
+
+// magnitude bits of a finite value, 0 for infinities and NaN (they are carried by hi alone)
+__device__ __forceinline__ uint32_t finite_magnitude(float v) {
+    const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
+    return u < 0x7f800000u ? u : 0u;
+}
+
+__device__ __forceinline__ float exact_pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
+
+// From the largest magnitude of a row: the factor that brings it to [2^14, 2^15) and its inverse.
+// False when the exponent is beyond what the float16 form takes.
+__device__ __forceinline__ bool half_scale(uint32_t max_bits, float &scale, float &inverse) {
+    int e = max_bits == 0 ? 14 : (int)(max_bits >> 23) - 127;
+    const bool ok = e >= -kHalfMaxExponent && e <= kHalfMaxExponent;
+    e       = e < -kHalfMaxExponent ? -kHalfMaxExponent : (e > kHalfMaxExponent ? kHalfMaxExponent : e);
+    scale   = exact_pow2(14 - e);
+    inverse = exact_pow2(e - 14);
+    return ok;
+}
+
+// v is already scaled.  Returns true when v is too small beside its row's largest value.
+__device__ __forceinline__ bool split_half(float v, __half &hi, __half &lo) {
+    hi = __float2half_rn(v);
+    const float d = (v - __half2float(hi)) * kHalfLoScale; // exact for finite v
+    lo = isfinite(v) ? __float2half_rn(d) : __half(0.0f);
+    return v != 0.0f && fabsf(v) < kHalfSmallest;
+}
+
+} // namespace ct

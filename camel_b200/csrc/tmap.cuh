@@ -14,6 +14,10 @@ namespace ct {
 ct_status encode_tiled_map_f32(
     CUtensorMap *map, const void *base, int rank, const uint64_t *dims, const uint64_t *strides, const uint32_t *box,
     int swizzle_bytes);
+// The same for float16 elements.
+ct_status encode_tiled_map_f16(
+    CUtensorMap *map, const void *base, int rank, const uint64_t *dims, const uint64_t *strides, const uint32_t *box,
+    int swizzle_bytes);
 
 // conv2d with the filters in tensor memory (conv_tmem.cu).
 bool conv_tmem_applicable(int64_t c, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw, int64_t stride,

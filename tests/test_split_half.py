@@ -1,0 +1,108 @@
+"""GPU: the contractions in split float16 (gemm_half.cu, conv_halo.cu, the strided convolution's patches)
+at the sizes where their tiling changes, and on operands that float16 pairs cannot hold, which have to
+take the tf32 planes instead; the few-column products at the edges of their row and k tiles.
+
+Bounds.  A value is carried to 2^-22 of itself (2^-17 for the few below 2^-28 of their row's largest), the
+product of two so carried to 2^-21, and the tensor core truncates once per addition into an accumulator
+that takes at most 96 of them (tf32) or 64 (float16) before it is drained: 2^-24 each relative to the sum of
+magnitudes so far.  96 * 2^-24 + 2^-21 < 6.3e-6 of sum |a||b|.  Float64 sums are rounded once: 2^-24.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+BOUND = 6.3e-6
+
+
+@pytest.fixture(scope="module")
+def T():
+    from camel_b200 import tensor
+
+    return tensor
+
+
+def _product(T, a, b):
+    out = T.matmul(T.from_numpy(a), T.from_numpy(b)).numpy()
+    T.check_async()
+    return out
+
+
+def _check(got, a, b):
+    a64, b64 = a.astype(np.float64), b.astype(np.float64)
+    err = np.abs(got - a64 @ b64)
+    assert np.all(err <= BOUND * (np.abs(a64) @ np.abs(b64)) + 1e-300)
+
+
+# one tile and its edges; slices in a cluster with an empty last one (k = 320: five groups of 64 over four);
+# the drain after 1024 values of k; pairs of CTAs with a ragged last tile; long columns (two passes over B);
+# few rows and a long k (slices through the workspace)
+SHAPES = [(64, 64, 64), (128, 32, 128), (129, 33, 257), (128, 320, 128), (65, 1025, 130), (300, 2080, 260),
+          (4100, 96, 1030), (2304, 1056, 2306), (130, 4128, 131), (40, 9000, 70), (33, 4096, 36)]
+
+
+@pytest.mark.parametrize("m,k,n", SHAPES)
+def test_product_narrow_scaled_and_wide_operands(T, m, k, n):
+    rng = np.random.default_rng(m + 7 * k + n)
+    a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    b = rng.uniform(-1, 1, (k, n)).astype(np.float32)
+    plain = _product(T, a, b)
+    _check(plain, a, b)
+    # rows and columns of very different sizes, each narrow in itself
+    ra = np.exp2(rng.integers(-50, 50, (m, 1))).astype(np.float32)
+    cb = np.exp2(rng.integers(-50, 50, (1, n))).astype(np.float32)
+    _check(_product(T, a * ra, b * cb), a * ra, b * cb)
+    # rows that span ninety powers of two: no float16 scale fits them
+    wide_a = a * np.exp2(rng.integers(-45, 45, (m, k))).astype(np.float32)
+    wide_b = b * np.exp2(rng.integers(-45, 45, (k, n))).astype(np.float32)
+    _check(_product(T, wide_a, b), wide_a, b)
+    _check(_product(T, a, wide_b), a, wide_b)
+    # one huge value that meets a zero must not cost the others their digits
+    spike, gate = a.copy(), b.copy()
+    spike[:, 3], gate[3, :] = 1e20, 0.0
+    _check(_product(T, spike, gate), spike, gate)
+    assert _product(T, a, b).tobytes() == plain.tobytes()  # nothing is left of the wide calls
+
+
+def test_infinities_and_nan_stay_in_their_rows(T):
+    rng = np.random.default_rng(5)
+    a = rng.uniform(0.5, 1, (200, 96)).astype(np.float32)
+    b = rng.uniform(0.5, 1, (96, 140)).astype(np.float32)
+    clean = _product(T, a, b)
+    a[7, 11], a[9, 3] = np.inf, np.nan
+    got = _product(T, a, b)
+    assert not np.isfinite(got[[7, 9]]).any()
+    rest = np.setdiff1d(np.arange(200), [7, 9])
+    assert got[rest].tobytes() == clean[rest].tobytes()
+
+
+@pytest.mark.parametrize("wide", ["left", "weights", "both"])
+def test_packed_weights_and_row_panels_agree_on_wide_operands(T, wide):
+    import ctypes as C
+
+    from camel_b200._lib import check, lib
+
+    rng = np.random.default_rng(11)
+    m, k, n = 384, 200, 300
+    a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    w = rng.uniform(-1, 1, (k, n)).astype(np.float32)
+    if wide in ("left", "both"):
+        a *= np.exp2(rng.integers(-45, 45, a.shape)).astype(np.float32)
+    if wide in ("weights", "both"):
+        w *= np.exp2(rng.integers(-45, 45, w.shape)).astype(np.float32)
+    ta, tw, out = T.from_numpy(a), T.from_numpy(w), T.zeros((m, n))
+    ap, wp = C.c_void_p(), C.c_void_p()
+    check(lib.ct_rows_pack(ta.ptr, m, k, C.byref(ap)))
+    check(lib.ct_weights_pack(tw.ptr, k, n, C.byref(wp)))
+    try:
+        check(lib.ct_dense_packed(ta.ptr, tw.ptr, wp, None, m, k, n, 0, out.ptr, None))
+        T.check_async()
+        whole = out.numpy()
+        _check(whole, a, w)
+        for row0, rows in ((0, 128), (128, 256)):
+            check(lib.ct_matmul_packed_rows(ap, row0, rows, wp, out.ptr + row0 * n * 4))
+        T.check_async()
+        _check(out.numpy(), a, w)
+    finally:
+        check(lib.ct_rows_free(ap))
+        check(lib.ct_weights_free(wp))
