@@ -389,19 +389,55 @@ __global__ void __launch_bounds__(kHThreads, 1)
             const float rs = (!wide && row0 + lane < p.m) ? p.row_scale[row0 + lane] : 1.0f;
 
             float acc[C::kCols];
-#pragma unroll
-            for (int j = 0; j < C::kCols; ++j)
-                acc[j] = 0.0f;
             const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(set * 2 * BN + half * C::kCols);
             bool ok                  = true;
-            auto drain = [&](int which, float weight) {
+            auto await = [&](int which) {
                 const int a    = set * 2 + which;
                 const bool got = mbar_wait(smem_u32(&bar_acc_full[a]), (full_phase >> a) & 1u, abort_flag);
                 full_phase ^= 1u << a;
                 ok = __all_sync(0xffffffffu, got);
-                if (!ok)
-                    return;
                 tc_fence_after_sync();
+                return ok;
+            };
+            auto hand_back = [&](int which) {
+                const uint32_t bar = smem_u32(&bar_acc_empty[set * 2 + which]);
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) {
+                    if (CG == 2)
+                        mbar_arrive_cluster(leader_addr(bar));
+                    else
+                        mbar_arrive(bar);
+                }
+            };
+            // 3 x f16: leading accumulator of every chunk but the last, then the cross products (the next tile
+            // starts with those: hand that accumulator back first), then the last chunk.  The first of them is read
+            // straight into the sums, with one wait for all its columns.
+            const int events = wide || nkb == 0 ? num_chunks : num_chunks + 1;
+            auto which_of    = [&](int c) { return wide ? (c & 1) : (c == num_chunks - 1 ? 1 : 0); };
+            if (events > 0 && await(which_of(0))) {
+                const int which    = which_of(0);
+                const float weight = !wide && which ? kHalfLoInv : 1.0f;
+                uint32_t r[C::kCols / 32][32];
+#pragma unroll
+                for (int g = 0; g < C::kCols / 32; ++g)
+                    tmem_ld_32x32(lane_base + (uint32_t)(which * BN + g * 32), r[g]);
+                tmem_ld_wait();
+                hand_back(which);
+#pragma unroll
+                for (int j = 0; j < C::kCols; ++j)
+                    acc[j] = __fmul_rn(__uint_as_float(r[j / 32][j % 32]), weight);
+            } else {
+#pragma unroll
+                for (int j = 0; j < C::kCols; ++j)
+                    acc[j] = 0.0f;
+            }
+#pragma unroll 1
+            for (int c = 1; c < events && ok; ++c) {
+                const int which    = which_of(c);
+                const float weight = !wide && which ? kHalfLoInv : 1.0f;
+                if (!await(which))
+                    break;
 #pragma unroll
                 for (int g = 0; g < C::kCols / 16; ++g) {
                     uint32_t r[16];
@@ -411,22 +447,7 @@ __global__ void __launch_bounds__(kHThreads, 1)
                     for (int j = 0; j < 16; ++j)
                         acc[g * 16 + j] = __fadd_rn(acc[g * 16 + j], __fmul_rn(__uint_as_float(r[j]), weight));
                 }
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) {
-                    if (CG == 2)
-                        mbar_arrive_cluster(leader_addr(smem_u32(&bar_acc_empty[a])));
-                    else
-                        mbar_arrive(smem_u32(&bar_acc_empty[a]));
-                }
-            };
-            // 3 x f16: leading accumulator of every chunk but the last, then the cross products (the next tile
-            // starts with those: hand that accumulator back first), then the last chunk
-            const int events = wide || nkb == 0 ? num_chunks : num_chunks + 1;
-#pragma unroll 1
-            for (int c = 0; c < events && ok; ++c) {
-                const int which = wide ? (c & 1) : (c == num_chunks - 1 ? 1 : 0);
-                drain(which, !wide && which ? kHalfLoInv : 1.0f);
+                hand_back(which);
             }
             if (!ok)
                 break;
@@ -618,8 +639,8 @@ HalfPlanes planes_of(const HalfOperand &o, bool both_forms) {
 }
 
 // in [rows][k] -> float16 planes [rows][kp], inverse row scales.  TPR threads per row keep the row in
-// registers (V float4 each) between finding its largest magnitude and splitting it; longer rows are read
-// twice (the second time from L2).  Bound by memory: 4 bytes read and 4 written per value.
+// registers (V float4 each, rows of up to 16384) between finding its largest magnitude and splitting it;
+// longer rows are read twice (the second time from L2).  Bound by memory: 4 bytes read and 4 written per value.
 template <int TPR, int V>
 __device__ __forceinline__ void half_rows(
     int64_t block, const float *__restrict__ in, int64_t rows, int64_t k, int64_t kp, const HalfPlanes &p, int vec_ok) {
@@ -988,8 +1009,10 @@ ct_status half_split_rows(
         CT_ROWS(32, 8, (rows + 7) / 8);
     else if (kp <= 4096)
         CT_ROWS(256, 4, rows);
-    else
+    else if (kp <= 8192)
         CT_ROWS(256, 8, rows);
+    else
+        CT_ROWS(256, 16, rows);
 #undef CT_ROWS
     CT_LAUNCH_CHECK("half_rows");
     return CT_OK;
