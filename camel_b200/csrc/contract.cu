@@ -3,6 +3,7 @@
 #include "common.cuh"
 #include "tmap.cuh"
 #include "split.cuh"
+#include "half_split.cuh"
 
 #include <cuda_bf16.h>
 
@@ -27,7 +28,9 @@ template <int MODE>
 __global__ void __launch_bounds__(256) im2col_planes_kernel(
     const float *__restrict__ x, int64_t c, int64_t h, int64_t w, int64_t kh, int64_t kw,
     int64_t stride, int64_t pad, int64_t ho, int64_t wo, int64_t kdim, int64_t kp, int64_t total,
-    void *__restrict__ p_hi, void *__restrict__ p_lo) {
+    void *__restrict__ p_hi, void *__restrict__ p_lo, const uint32_t *__restrict__ only_if) {
+    if (only_if && *reinterpret_cast<const volatile uint32_t *>(only_if) == 0)
+        return; // the float16 planes of im2col_half_kernel hold the patches
     int64_t step = (int64_t)gridDim.x * 256;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += step) {
         int64_t kk  = i % kp;
@@ -50,6 +53,77 @@ __global__ void __launch_bounds__(256) im2col_planes_kernel(
             static_cast<__nv_bfloat16 *>(p_hi)[i] = __float2bfloat16_rn(v);
         }
     }
+}
+
+// The same as scaled float16 pairs (half_split.cuh), a warp per patch: the patch stays in registers between
+// its largest magnitude and the split.  Where in the image patch element kk lies - (offset, r, s) - comes from
+// a table in shared memory that a block builds once; with an element per thread and 64-bit divisions for each
+// of them the pass took 218 us for 64 x 48 x 57 x 57 at stride 2, seven times what its stores cost.
+constexpr int kPatchRegs = 16; // pairs of values per lane: patches of up to 1024 values
+template <int V>
+__global__ void __launch_bounds__(256) im2col_half_kernel(
+    const float *__restrict__ x, int c, int h, int w, int kh, int kw, int stride, int pad, int ho, int wo, int kdim, int kp,
+    int64_t rows, __half *__restrict__ p_hi, __half *__restrict__ p_lo, float *__restrict__ scale_out,
+    uint32_t *__restrict__ wide) {
+    extern __shared__ int2 where[]; // element kk: offset from the patch's origin in its image, r << 16 | s
+    griddep_launch_dependents();
+    for (int kk = threadIdx.x; kk < kp; kk += 256) {
+        const int s = kk % kw, r = (kk / kw) % kh, ic = kk / (kw * kh);
+        where[kk] = kk < kdim ? make_int2((ic * h + r) * w + s, (r << 16) | s) : make_int2(0, 0x7fff7fff);
+    }
+    __syncthreads();
+    griddep_wait();
+    const int lane = threadIdx.x & 31, pix = ho * wo;
+    bool bad       = false;
+    for (int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (int64_t)gridDim.x * 8) {
+        const int img = (int)(row / pix), p = (int)(row - (int64_t)img * pix);
+        const int oy = p / wo, y0 = oy * stride - pad, x0 = (p - oy * wo) * stride - pad;
+        const float *src = x + (int64_t)img * c * h * w + (int64_t)y0 * w + x0;
+        auto load        = [&](int kk) {
+            const int2 at = where[kk];
+            const int iy = y0 + (at.y >> 16), ix = x0 + (at.y & 0xffff);
+            return (iy >= 0 && iy < h && ix >= 0 && ix < w) ? __ldg(src + at.x) : 0.0f; // padding elements lie far outside
+        };
+        float2 v[V];
+        uint32_t mx = 0;
+        const bool fits = kp <= 64 * V;
+        if (fits) {
+#pragma unroll
+            for (int j = 0; j < V; ++j) {
+                const int kk = 64 * j + 2 * lane;
+                v[j]         = kk < kp ? make_float2(load(kk), load(kk + 1)) : make_float2(0.0f, 0.0f);
+            }
+#pragma unroll
+            for (int j = 0; j < V; ++j)
+                mx = max(mx, max(finite_magnitude(v[j].x), finite_magnitude(v[j].y)));
+        } else {
+            for (int kk = lane; kk < kdim; kk += 32)
+                mx = max(mx, finite_magnitude(load(kk)));
+        }
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        float scale, inverse;
+        bad |= !half_scale(mx, scale, inverse);
+        if (lane == 0)
+            scale_out[row] = inverse;
+        auto put = [&](int kk, float a, float b) {
+            __half hi[2], lo[2];
+            bad |= split_half(a * scale, hi[0], lo[0]);
+            bad |= split_half(b * scale, hi[1], lo[1]);
+            *reinterpret_cast<__half2 *>(p_hi + row * kp + kk) = *reinterpret_cast<__half2 *>(hi);
+            *reinterpret_cast<__half2 *>(p_lo + row * kp + kk) = *reinterpret_cast<__half2 *>(lo);
+        };
+        if (fits) {
+#pragma unroll
+            for (int j = 0; j < V; ++j)
+                if (64 * j + 2 * lane < kp)
+                    put(64 * j + 2 * lane, v[j].x, v[j].y);
+        } else {
+            for (int kk = 2 * lane; kk < kp; kk += 64)
+                put(kk, load(kk), load(kk + 1));
+        }
+    }
+    if (bad)
+        *wide = 1u;
 }
 
 // Weights [ko][c][kh][kw] -> A-operand planes [ko][taps * c_pad] with k = (r*kw + s) * c_pad + ic:
@@ -654,6 +728,43 @@ static ct_status conv2d_run(
     int64_t kp       = (kdim + kblock - 1) / kblock * kblock;
     size_t w_plane   = align_up((size_t)ko * kp * elem);
     size_t p_plane   = align_up((size_t)n * pix * kp * elem);
+    // 32-bit indices inside an image and over the patches, coordinates that leave room for the mark of a padding
+    // element, a table of the patch in shared memory
+    if (mode == 0 && c * h * wd <= 0x3fffffff && pix <= 0x3fffffff && n * pix <= 0x3fffffff && h < 0x3fff && wd < 0x3fff &&
+        pad < 0x3fff && kh < 0x3fff && kw < 0x3fff && kp <= 4096) {
+        // split float16: [w scale][patch scale][w hi16][w lo16][w hi][w lo][patches], the patches as float16
+        // pairs or, where the word says so, as tf32 planes in the same place
+        const size_t w16 = align_up((size_t)ko * kp * 2), p16 = align_up((size_t)n * pix * kp * 2);
+        const size_t w_words = align_up((size_t)ko * 4), p_words = align_up((size_t)n * pix * 4);
+        CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, w_words + p_words + 2 * w16 + 2 * w_plane + 2 * p_plane));
+        uint8_t *ws     = static_cast<uint8_t *>(st->gemm_ws);
+        uint8_t *planes = ws + w_words + p_words, *w32 = planes + 2 * w16, *patches = w32 + 2 * w_plane;
+        uint32_t *wide  = st->flags_dev + FLAG_WIDE;
+        HalfOperand oa{planes, planes + w16, reinterpret_cast<float *>(ws), w32, w32 + w_plane, wide, ko};
+        HalfOperand ob{patches, patches + p16, reinterpret_cast<float *>(ws + w_words), patches, patches + p_plane, wide, n * pix};
+        {
+            ProfScope prof("im2col");
+            CT_TRY(half_split_rows(st, w, kdim, kp, oa, true, nullptr, 0));
+            const unsigned blocks = capped_blocks(st, n * pix * 32, 8);
+#define CT_PATCHES(V)                                                                                                   \
+    CT_CUDA(launch_dependent(im2col_half_kernel<V>, dim3(blocks), dim3(256), (size_t)kp * sizeof(int2), stream(), x, (int)c, \
+                             (int)h, (int)wd, (int)kh, (int)kw, (int)stride, (int)pad, (int)ho, (int)wo, (int)kdim, (int)kp,  \
+                             n * pix, reinterpret_cast<__half *>(patches), reinterpret_cast<__half *>(patches + p16),       \
+                             const_cast<float *>(ob.scale), wide))
+            if (kp <= 256)
+                CT_PATCHES(4);
+            else if (kp <= 512)
+                CT_PATCHES(8);
+            else
+                CT_PATCHES(kPatchRegs);
+#undef CT_PATCHES
+            CT_LAUNCH_CHECK("im2col_half");
+            im2col_planes_kernel<0><<<capped_blocks(st, n * pix * kp, 4), 256, 0, stream()>>>(
+                x, c, h, wd, kh, kw, stride, pad, ho, wo, kdim, kp, n * pix * kp, patches, patches + p_plane, wide);
+            CT_LAUNCH_CHECK("im2col_planes");
+        }
+        return gemm_half(st, oa, ob, kp, bias, act, out, false, true, false, nullptr, (int)n, true);
+    }
     CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, planes * (w_plane + p_plane)));
     uint8_t *ws = static_cast<uint8_t *>(st->gemm_ws);
     void *w_hi = ws, *w_lo = ws + w_plane;
@@ -664,10 +775,10 @@ static ct_status conv2d_run(
         ProfScope prof("im2col");
         if (mode == 0)
         im2col_planes_kernel<0><<<capped_blocks(st, total, 32), 256, 0, stream()>>>(
-            x, c, h, wd, kh, kw, stride, pad, ho, wo, kdim, kp, total, p_hi, p_lo);
+            x, c, h, wd, kh, kw, stride, pad, ho, wo, kdim, kp, total, p_hi, p_lo, nullptr);
     else
         im2col_planes_kernel<1><<<capped_blocks(st, total, 32), 256, 0, stream()>>>(
-            x, c, h, wd, kh, kw, stride, pad, ho, wo, kdim, kp, total, p_hi, p_lo);
+            x, c, h, wd, kh, kw, stride, pad, ho, wo, kdim, kp, total, p_hi, p_lo, nullptr);
     }
     CT_LAUNCH_CHECK("im2col_planes");
     return gemm_planes(

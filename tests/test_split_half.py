@@ -106,3 +106,34 @@ def test_packed_weights_and_row_panels_agree_on_wide_operands(T, wide):
     finally:
         check(lib.ct_rows_free(ap))
         check(lib.ct_weights_free(wp))
+
+
+def _conv64(x, w, stride, pad):
+    n, c, h, wd = x.shape
+    ko, _, kh, kw = w.shape
+    xp = np.pad(x.astype(np.float64), ((0, 0), (0, 0), (pad, pad), (pad, pad)))
+    win = np.lib.stride_tricks.sliding_window_view(xp, (kh, kw), (2, 3))[:, :, ::stride, ::stride]
+    return np.einsum("nchwrs,kcrs->nkhw", win, w.astype(np.float64), optimize=True)
+
+
+# (n, c, h, w, ko, kernel, stride, pad): patches in registers and read twice (k = 1200), odd sizes; halos with a
+# partial last tile, channels that do not fill a block, more than 128 filters, 1 x 1 and 5 x 5 taps
+CONVS = [(3, 48, 21, 23, 70, 3, 2, 1), (2, 8, 33, 21, 20, 3, 2, 0), (2, 48, 15, 16, 40, 5, 3, 2), (2, 12, 24, 24, 65, 5, 1, 2)]
+
+
+@pytest.mark.parametrize("shape", CONVS)
+@pytest.mark.parametrize("kind", ["plain", "wide input", "wide filters"])
+def test_convolution_narrow_and_wide(T, shape, kind):
+    n, c, h, wd, ko, kern, stride, pad = shape
+    rng = np.random.default_rng(sum(shape))
+    x = rng.standard_normal((n, c, h, wd)).astype(np.float32)
+    w = rng.standard_normal((ko, c, kern, kern)).astype(np.float32)
+    if kind == "wide input":
+        x *= np.exp2(rng.integers(-45, 45, x.shape)).astype(np.float32)
+    if kind == "wide filters":
+        w *= np.exp2(rng.integers(-45, 45, w.shape)).astype(np.float32)
+    got = T.conv2d(T.from_numpy(x), T.from_numpy(w), None, stride, pad).numpy()
+    T.check_async()
+    # a halo layer's k (at most 1024) is one accumulation: up to 384 tf32 additions instead of 96
+    bound = 384 * 2.0**-24 + 2.0**-21
+    assert np.all(np.abs(got - _conv64(x, w, stride, pad)) <= bound * _conv64(np.abs(x), np.abs(w), stride, pad) + 1e-300)
