@@ -692,6 +692,9 @@ static ct_status conv2d_run(
     }
     if (th > 0) {
         int64_t c_pad  = (c + kblock - 1) / kblock * kblock;
+        if (mode == 0 && pool == 0 && conv_halo_applicable(c_pad, h, wd, ko, kh, kw, stride, pad))
+            // many filters: one input halo per tile and channel block serves every tap (conv_halo.cu)
+            return conv_halo(st, x, w, n, c, c_pad, h, wd, ko, kh, kw, pad, bias, act, out);
         int64_t taps   = kh * kw;
         int64_t kp_i   = taps * c_pad;
         size_t w_plane = align_up((size_t)ko * kp_i * elem);
@@ -712,9 +715,6 @@ static ct_status conv2d_run(
             CT_LAUNCH_CHECK("conv_weight_planes");
             CT_TRY(nhwc_planes(st, mode, x, n, c, h * wd, c_pad, x_hi, x_lo));
         }
-        if (mode == 0 && pool == 0 && conv_halo_applicable(c_pad, h, wd, ko, kh, kw, stride, pad))
-            // many filters: one input halo per tile and channel block serves every tap (conv_halo.cu)
-            return conv_halo_stream(st, w_hi, w_lo, x_hi, x_lo, n, c_pad, h, wd, ko, kh, kw, pad, bias, act, out);
         ConvGeom g;
         g.c_pad = (int)c_pad;
         g.h = (int)h, g.w = (int)wd, g.ho = (int)ho, g.wo = (int)wo;

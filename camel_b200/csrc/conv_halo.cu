@@ -12,11 +12,21 @@
 // moved by r * PW + s rows of 64 bytes (a position's row in the box is y * PW + x).  Pixel planes
 // enter shared memory once per nine taps; per k-block 19 KB in instead of 44.
 //
-// Structure as the streaming kernel: one CTA per SM walks the tiles, two TMEM accumulators, the
-// epilogue of tile i (drain, bias, relu, store) runs under the MMAs of tile i + 1.  Two rings of
-// stages: filter k-blocks (one per tap and channel block) and halos (one per channel block).
-// Rows = 128 output channels, columns = positions.  Every wait is bounded.
+// Arithmetic: split float16 (half_split.cuh), scaled per filter and per image - a scale has to be constant
+// along k, and an output's patch crosses the whole halo - with the cross products in an accumulator of their
+// own, as in gemm_half.cu.  A 64-byte row then holds 32 channels, so the layer takes half the MMAs, half the
+// filter stages and half the plane traffic of the tf32 form.  Where an image or a filter spans too many powers
+// of two, the pre-pass raises a device word, wide_nhwc_kernel writes tf32 planes and this kernel runs the same
+// loop over those (16 channels per row).
+//
+// One CTA per SM walks the tiles.  Both accumulators (512 columns) belong to one tile; the epilogue reads the
+// cross products first, which the next tile starts with, so the tensor pipe waits for about the drain of
+// the leading accumulator (a few hundred of ~14,000 clocks per tile of 64 channels) and the store runs under
+// the next tile's MMAs.  Two rings of stages: filter k-blocks (one per tap and channel block) and halos (one
+// per channel block).  Rows = 128 output channels, columns = positions.  Every wait is bounded.
 #include "common.cuh"
+#include "half_split.cuh"
+#include "split.cuh"
 #include "tc_ptx.cuh"
 #include "tmap.cuh"
 
@@ -47,8 +57,7 @@ namespace {
 
 using namespace ptx;
 
-constexpr int kH_RowB       = 64;                     // bytes of k per operand row and k-block: 16 float32
-constexpr int kH_BlockK     = 16;
+constexpr int kH_RowB       = 64;                     // bytes of k per operand row and k-block: 32 float16 / 16 tf32
 constexpr int kH_AStages    = 4;
 constexpr int kH_HaloStages = 2;
 constexpr int kH_ABytes     = 128 * kH_RowB;          // one filter plane of a k-block
@@ -68,7 +77,9 @@ struct ConvHaloParams {
     int kh, kw, pad;
     int ho, wo, pw;   // pw = w + 2 pad
     int th, tiles_y;
-    int cblocks;      // channel blocks of 16
+    const uint32_t *wide;      // non-zero: the planes are tf32
+    const float *filter_scale; // [ko] inverse scales
+    const float *image_scale;  // [batch]
     int c_pad;        // channels of the planes (k offset of a tap in the filter planes: tap * c_pad)
     int n_mma;        // th * pw rounded up to 16
     int box_bytes;    // one plane's halo box
@@ -76,14 +87,17 @@ struct ConvHaloParams {
     int act;
 };
 
+struct ConvHaloMaps {
+    CUtensorMap w16_hi, w16_lo, x16_hi, x16_lo;
+    CUtensorMap w32_hi, w32_lo, x32_hi, x32_lo;
+};
+
 __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
-    const __grid_constant__ CUtensorMap map_w_hi, const __grid_constant__ CUtensorMap map_w_lo,
-    const __grid_constant__ CUtensorMap map_x_hi, const __grid_constant__ CUtensorMap map_x_lo,
-    const ConvHaloParams p, const int total_tiles) {
+    const __grid_constant__ ConvHaloMaps maps, const __grid_constant__ ConvHaloParams p, const int total_tiles) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t bar_a_full[kH_AStages], bar_a_empty[kH_AStages];
     __shared__ uint64_t bar_h_full[kH_HaloStages], bar_h_empty[kH_HaloStages];
-    __shared__ uint64_t bar_tmem_full[2], bar_tmem_empty[2];
+    __shared__ uint64_t bar_tmem_full[2], bar_tmem_empty[2]; // 0: leading accumulator, 1: cross products
     __shared__ uint64_t bar_done;
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag_s;
@@ -122,10 +136,10 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
         }
         mbar_init(smem_u32(&bar_done), 1);
         mbar_fence_init();
-        prefetch_tensormap(&map_w_hi);
-        prefetch_tensormap(&map_w_lo);
-        prefetch_tensormap(&map_x_hi);
-        prefetch_tensormap(&map_x_lo);
+        prefetch_tensormap(&maps.w16_hi);
+        prefetch_tensormap(&maps.w16_lo);
+        prefetch_tensormap(&maps.x16_hi);
+        prefetch_tensormap(&maps.x16_lo);
     }
     if (warp == 1) {
         tmem_alloc(smem_u32(&tmem_base_slot), 512);
@@ -136,6 +150,9 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
     const int taps           = p.kh * p.kw;
+    const bool wide          = *reinterpret_cast<const volatile uint32_t *>(p.wide) != 0;
+    const int block_k        = wide ? 16 : 32; // channels per k-block
+    const int cblocks        = p.c_pad / block_k;
 
     // tile -> (row tile of output channels, tile row, image): neighbouring CTAs take the row tiles
     // of one pixel tile, so they read the same halo out of L2
@@ -149,12 +166,14 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
     if (warp == 0) {
         // ===== TMA producer =====
         if (lane == 0) {
+            const CUtensorMap *mw_hi = wide ? &maps.w32_hi : &maps.w16_hi, *mw_lo = wide ? &maps.w32_lo : &maps.w16_lo;
+            const CUtensorMap *mx_hi = wide ? &maps.x32_hi : &maps.x16_hi, *mx_lo = wide ? &maps.x32_lo : &maps.x16_lo;
             int ka = 0, kh2 = 0; // filter k-blocks and halos issued so far
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
                 int tm, ty, img;
                 coords(tile, tm, ty, img);
-                for (int cb = 0; cb < p.cblocks && ok; ++cb, ++kh2) {
+                for (int cb = 0; cb < cblocks && ok; ++cb, ++kh2) {
                     const int hs = kh2 % kH_HaloStages;
                     if (!mbar_wait(smem_u32(&bar_h_empty[hs]), ((uint32_t)(kh2 / kH_HaloStages) & 1u) ^ 1u, abort_flag)) {
                         ok = false;
@@ -163,8 +182,8 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                     const uint32_t hfull = smem_u32(&bar_h_full[hs]);
                     const uint32_t hdst  = halo_base + (uint32_t)hs * halo_stage;
                     mbar_expect_tx(hfull, 2u * (uint32_t)p.box_bytes);
-                    tma_load_4d(hdst, &map_x_hi, hfull, cb * kH_BlockK, -p.pad, ty * p.th - p.pad, img);
-                    tma_load_4d(hdst + (uint32_t)p.halo_plane_bytes, &map_x_lo, hfull, cb * kH_BlockK, -p.pad,
+                    tma_load_4d(hdst, mx_hi, hfull, cb * block_k, -p.pad, ty * p.th - p.pad, img);
+                    tma_load_4d(hdst + (uint32_t)p.halo_plane_bytes, mx_lo, hfull, cb * block_k, -p.pad,
                                 ty * p.th - p.pad, img);
                     for (int tap = 0; tap < taps; ++tap, ++ka) {
                         const int s = ka % kH_AStages;
@@ -175,9 +194,9 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                         const uint32_t full = smem_u32(&bar_a_full[s]);
                         const uint32_t dst  = smem_base + (uint32_t)s * kH_AStageBytes;
                         mbar_expect_tx(full, (uint32_t)kH_AStageBytes);
-                        const int32_t kc = tap * p.c_pad + cb * kH_BlockK;
-                        tma_load_2d(dst, &map_w_hi, full, kc, tm * 128);
-                        tma_load_2d(dst + kH_ABytes, &map_w_lo, full, kc, tm * 128);
+                        const int32_t kc = tap * p.c_pad + cb * block_k;
+                        tma_load_2d(dst, mw_hi, full, kc, tm * 128);
+                        tma_load_2d(dst + kH_ABytes, mw_lo, full, kc, tm * 128);
                     }
                 }
             }
@@ -198,24 +217,22 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
             }
         }
     } else if (warp == 1) {
-        // ===== MMA issuer: accumulator buffer i & 1 for the CTA's i-th tile =====
+        // ===== MMA issuer =====
         if (lane == 0) {
-            const uint32_t idesc = make_idesc(2u, 128, (uint32_t)p.n_mma);
+            const uint32_t idesc = make_idesc(wide ? 2u : 0u, 128, (uint32_t)p.n_mma);
             int ka = 0, kh2 = 0, i = 0;
             bool ok = true;
             const long long t_start = CH_CLOCK();
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++i) {
-                const int buf = i & 1;
-                const long long t0 = CH_CLOCK();
-                if (!mbar_wait(smem_u32(&bar_tmem_empty[buf]), (((uint32_t)i >> 1) & 1u) ^ 1u, abort_flag)) {
-                    ok = false;
-                    break;
-                }
-                CH_ACCUM(0, CH_CLOCK() - t0); // waiting for an accumulator
-                tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + (uint32_t)buf * 256u;
+                // the accumulators of the previous tile have been read
+                auto wait_empty = [&](int acc) {
+                    const bool got = mbar_wait(smem_u32(&bar_tmem_empty[acc]), ((uint32_t)i & 1u) ^ 1u, abort_flag);
+                    tc_fence_after_sync();
+                    return got;
+                };
+                const uint32_t d_main = tmem_base, d_cross = tmem_base + 256u;
                 bool first = true;
-                for (int cb = 0; cb < p.cblocks && ok; ++cb, ++kh2) {
+                for (int cb = 0; cb < cblocks && ok; ++cb, ++kh2) {
                     const int hs = kh2 % kH_HaloStages;
                     const long long t1 = CH_CLOCK();
                     if (!mbar_wait(smem_u32(&bar_h_full[hs]), (uint32_t)(kh2 / kH_HaloStages) & 1u, abort_flag)) {
@@ -241,22 +258,45 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                             const uint32_t shift = (uint32_t)(r * p.pw + sx) * (uint32_t)kH_RowB;
                             const uint64_t da_hi = smem_desc_k<kH_RowB>(a_hi), da_lo = smem_desc_k<kH_RowB>(a_lo);
                             const uint64_t db_hi = smem_desc_k<kH_RowB>(x_hi + shift), db_lo = smem_desc_k<kH_RowB>(x_lo + shift);
+                            if (!wide) {
+                                if (first && !wait_empty(1)) {
+                                    ok = false;
+                                    break;
+                                }
+                                mma_f16(d_cross, da_lo, db_hi, idesc, first ? 0u : 1u);
+                                mma_f16(d_cross, da_hi, db_lo, idesc, 1u);
+                                mma_f16(d_cross, da_lo + 2, db_hi + 2, idesc, 1u);
+                                mma_f16(d_cross, da_hi + 2, db_lo + 2, idesc, 1u);
+                                if (first && !wait_empty(0)) {
+                                    ok = false;
+                                    break;
+                                }
+                                mma_f16(d_main, da_hi, db_hi, idesc, first ? 0u : 1u);
+                                mma_f16(d_main, da_hi + 2, db_hi + 2, idesc, 1u);
+                            } else {
+                                if (first && !wait_empty(0)) {
+                                    ok = false;
+                                    break;
+                                }
 #pragma unroll
-                            for (int kk = 0; kk < kH_RowB / 32; ++kk) {
-                                const uint64_t adv = (uint64_t)(kk * 32 >> 4);
-                                mma_tf32(d_tmem, da_lo + adv, db_hi + adv, idesc, first ? 0u : 1u);
-                                mma_tf32(d_tmem, da_hi + adv, db_lo + adv, idesc, 1u);
-                                mma_tf32(d_tmem, da_hi + adv, db_hi + adv, idesc, 1u);
-                                first = false;
+                                for (int kk = 0; kk < kH_RowB / 32; ++kk) {
+                                    mma_tf32(d_main, da_lo + 2 * kk, db_hi + 2 * kk, idesc, first && kk == 0 ? 0u : 1u);
+                                    mma_tf32(d_main, da_hi + 2 * kk, db_lo + 2 * kk, idesc, 1u);
+                                    mma_tf32(d_main, da_hi + 2 * kk, db_hi + 2 * kk, idesc, 1u);
+                                }
                             }
+                            first = false;
                             tc_commit(smem_u32(&bar_a_empty[s]));
                         }
                     }
                     if (ok)
                         tc_commit(smem_u32(&bar_h_empty[hs])); // the halo is free once its taps' MMAs have retired
                 }
-                if (ok)
-                    tc_commit(smem_u32(&bar_tmem_full[buf]));
+                if (ok) {
+                    if (!wide)
+                        tc_commit(smem_u32(&bar_tmem_full[1]));
+                    tc_commit(smem_u32(&bar_tmem_full[0]));
+                }
             }
             CH_ACCUM(3, CH_CLOCK() - t_start); // the MMA thread's whole loop
             CH_ACCUM(4, i);
@@ -291,30 +331,55 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
             int tm, ty, img;
             coords(tile, tm, ty, img);
-            const int buf = i & 1;
+            const int row0     = tm * 128 + quarter * 32; // first output channel of this warp's block
+            const float rs     = (!wide && row0 + lane < p.ko) ? p.filter_scale[row0 + lane] : 1.0f;
+            const float is     = wide ? 1.0f : p.image_scale[img];
             const long long e0 = CH_CLOCK();
-            bool got = mbar_wait(smem_u32(&bar_tmem_full[buf]), ((uint32_t)i >> 1) & 1u, abort_flag);
-            if (!__all_sync(0xffffffffu, got))
-                break;
-            const long long e1 = CH_CLOCK();
-            tc_fence_after_sync();
             float acc[128];
-            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256 + half * 128);
+            const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 128);
+            auto await = [&](int which) {
+                const bool got = mbar_wait(smem_u32(&bar_tmem_full[which]), (uint32_t)i & 1u, abort_flag);
+                tc_fence_after_sync();
+                return __all_sync(0xffffffffu, got) != 0;
+            };
+            auto hand_back = [&](int which) {
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive(smem_u32(&bar_tmem_empty[which]));
+            };
+            // the cross products (tf32: the one accumulator) straight into the sums, with one wait for all columns
+            const int first_acc = wide ? 0 : 1;
+            if (!await(first_acc))
+                break;
+            {
+                uint32_t r[4][32];
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                uint32_t r[32];
-                tmem_ld_32x32(taddr + g * 32, r);
+                for (int g = 0; g < 4; ++g)
+                    tmem_ld_32x32(lane_base + (uint32_t)(first_acc * 256 + g * 32), r[g]);
                 tmem_ld_wait();
+                hand_back(first_acc);
+                const float weight = wide ? 1.0f : kHalfLoInv;
 #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    acc[g * 32 + j] = __uint_as_float(r[j]);
+                for (int j = 0; j < 128; ++j)
+                    acc[j] = __fmul_rn(__uint_as_float(r[j / 32][j % 32]), weight);
             }
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0)
-                mbar_arrive(smem_u32(&bar_tmem_empty[buf]));
+            if (!wide) {
+                if (!await(0))
+                    break;
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                    uint32_t r[16];
+                    tmem_ld_32x16(lane_base + g * 16, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        acc[g * 16 + j] = __fadd_rn(acc[g * 16 + j], __uint_as_float(r[j]));
+                }
+                hand_back(0);
+            }
+            const long long e1 = CH_CLOCK();
 
-            const int row0 = tm * 128 + quarter * 32; // first output channel of this warp's block
             const int y0   = ty * p.th;
             // positions of rows past the image's last row (a partial last tile) are dropped:
             // position col lies in row col / pw, so the valid ones are col < rows_left * pw
@@ -327,8 +392,8 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                 float4 *mine = reinterpret_cast<float4 *>(stg + lane * kH_EpiRowBytes);
 #pragma unroll
                 for (int j = 0; j < 16; ++j)
-                    mine[j] = make_float4(acc[h2 * 64 + 4 * j], acc[h2 * 64 + 4 * j + 1], acc[h2 * 64 + 4 * j + 2],
-                                          acc[h2 * 64 + 4 * j + 3]);
+                    mine[j] = make_float4(__fmul_rn(acc[h2 * 64 + 4 * j], rs), __fmul_rn(acc[h2 * 64 + 4 * j + 1], rs),
+                                          __fmul_rn(acc[h2 * 64 + 4 * j + 2], rs), __fmul_rn(acc[h2 * 64 + 4 * j + 3], rs));
                 __syncwarp();
 #pragma unroll 4
                 for (int it = 0; it < 16; ++it) {
@@ -342,7 +407,7 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             if (off[h2][q] >= 0 && col_base + h2 * 64 + q < col_limit) {
-                                float x = v[q];
+                                float x = __fmul_rn(v[q], is);
                                 if (p.bias)
                                     x = __fadd_rn(x, b);
                                 if (p.act == CT_ACT_RELU)
@@ -368,8 +433,146 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 512);
     }
-    if (threadIdx.x == 0 && *abort_flag)
-        atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
+    if (threadIdx.x == 0) {
+        if (*abort_flag)
+            atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
+        // the last CTA clears the pre-pass's word for the next product
+        if (atomicAdd(p.flags + FLAG_WIDE_READERS, 1u) + 1u == gridDim.x) {
+            p.flags[FLAG_WIDE_READERS] = 0u;
+            p.flags[FLAG_WIDE]         = 0u;
+        }
+    }
+}
+
+// ---- pre-pass -----------------------------------------------------------------------------
+
+// Largest magnitude of each image ([batch][count] floats), as bits, by atomic maximum into img_max (zeroed).  An
+// infinity or NaN counts as what it is: half_scale refuses it and the layer takes the tf32 planes.
+__global__ void __launch_bounds__(256) image_max_kernel(
+    const float *__restrict__ x, int64_t count, int slices, int vec_ok, uint32_t *__restrict__ img_max) {
+    const int64_t img = blockIdx.x / slices;
+    const int slice   = blockIdx.x - (int)img * slices;
+    const float *src  = x + img * count;
+    uint32_t mx       = 0;
+    if (vec_ok) {
+        const float4 *s4 = reinterpret_cast<const float4 *>(src);
+#pragma unroll 8
+        for (int64_t i = (int64_t)slice * 256 + threadIdx.x; i < count / 4; i += (int64_t)slices * 256) {
+            const float4 q = s4[i];
+            mx = max(max(mx, max(__float_as_uint(q.x) & 0x7fffffffu, __float_as_uint(q.y) & 0x7fffffffu)),
+                     max(__float_as_uint(q.z) & 0x7fffffffu, __float_as_uint(q.w) & 0x7fffffffu));
+        }
+    } else {
+#pragma unroll 8
+        for (int64_t i = (int64_t)slice * 256 + threadIdx.x; i < count; i += (int64_t)slices * 256)
+            mx = max(mx, __float_as_uint(src[i]) & 0x7fffffffu);
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if ((threadIdx.x & 31) == 0 && mx)
+        atomicMax(img_max + img, mx);
+}
+
+// x [batch][c][hw] -> NHWC float16 planes [batch][hw][c_pad] under the image's scale.  A block takes 64
+// channels by 64 positions through shared memory: reads of 256 contiguous bytes, writes of 128.  The images are
+// taken last to first: the end of the tensor is what image_max_kernel has just left in L2.
+__global__ void __launch_bounds__(256) nhwc_half_kernel(
+    const float *__restrict__ x, int c, int64_t hw, int c_pad, const uint32_t *__restrict__ img_max, __half *__restrict__ p_hi,
+    __half *__restrict__ p_lo, float *__restrict__ image_scale, uint32_t *__restrict__ wide) {
+    __shared__ float tile[64][65];
+    const int64_t img = gridDim.z - 1 - blockIdx.z;
+    const int64_t q0  = (int64_t)blockIdx.x * 64;
+    const int c0      = (int)blockIdx.y * 64;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float *src = x + (img * c + c0) * hw + q0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const int ch = warp + 8 * j, q = lane + 32 * t;
+            tile[ch][q]  = (c0 + ch < c && q0 + q < hw) ? __ldcs(src + ch * hw + q) : 0.0f;
+        }
+    float scale, inverse;
+    bool bad = !half_scale(img_max[img], scale, inverse);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+        image_scale[img] = inverse;
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const int chunk = threadIdx.x & 7, q = (threadIdx.x >> 3) + 32 * t;
+        if (q0 + q < hw && c0 + chunk * 8 < c_pad) {
+            __half hi[8], lo[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                bad |= split_half(tile[chunk * 8 + j][q] * scale, hi[j], lo[j]);
+            const int64_t at = (img * hw + q0 + q) * c_pad + c0 + chunk * 8;
+            *reinterpret_cast<uint4 *>(p_hi + at) = *reinterpret_cast<uint4 *>(hi);
+            *reinterpret_cast<uint4 *>(p_lo + at) = *reinterpret_cast<uint4 *>(lo);
+        }
+    }
+    if (bad)
+        *wide = 1u;
+}
+
+// Filters [ko][c][taps] -> planes [ko][taps * c_pad], tap-major k, both forms; a block per filter.
+__global__ void __launch_bounds__(256) filter_planes_kernel(
+    const float *__restrict__ w, int c, int taps, int c_pad, __half *__restrict__ hi16, __half *__restrict__ lo16,
+    float *__restrict__ hi32, float *__restrict__ lo32, float *__restrict__ filter_scale, uint32_t *__restrict__ wide) {
+    __shared__ uint32_t max_s[8];
+    const int64_t o  = blockIdx.x;
+    const float *src = w + o * c * taps;
+    uint32_t mx      = 0;
+    for (int i = threadIdx.x; i < c * taps; i += 256)
+        mx = max(mx, finite_magnitude(src[i]));
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if ((threadIdx.x & 31) == 0)
+        max_s[threadIdx.x >> 5] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        mx = max(mx, max_s[j]);
+    float scale, inverse;
+    bool bad = !half_scale(mx, scale, inverse);
+    if (threadIdx.x == 0)
+        filter_scale[o] = inverse;
+    for (int i = threadIdx.x; i < taps * c_pad; i += 256) {
+        const int tap = i / c_pad, ic = i - tap * c_pad;
+        const float v    = ic < c ? src[ic * taps + tap] : 0.0f;
+        const int64_t at = o * taps * c_pad + i;
+        bad |= split_half(v * scale, hi16[at], lo16[at]);
+        split_tf32(v, hi32[at], lo32[at]);
+    }
+    if (bad)
+        *wide = 1u;
+}
+
+// The tf32 NHWC planes, where the word says that they are needed; returns at once otherwise.
+__global__ void __launch_bounds__(256) wide_nhwc_kernel(
+    const uint32_t *__restrict__ wide, const float *__restrict__ x, int64_t batch, int c, int64_t hw, int c_pad,
+    float *__restrict__ hi, float *__restrict__ lo) {
+    __shared__ float tile[32][33];
+    if (*reinterpret_cast<const volatile uint32_t *>(wide) == 0)
+        return;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int64_t tiles_q = (hw + 31) / 32, tiles_c = c_pad / 32;
+    for (int64_t t = blockIdx.x; t < batch * tiles_q * tiles_c; t += gridDim.x) {
+        const int64_t img = t / (tiles_q * tiles_c), rest = t - img * tiles_q * tiles_c;
+        const int64_t q0 = rest / tiles_c * 32, c0 = rest % tiles_c * 32;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int64_t ch = c0 + ty + 8 * j, q = q0 + tx;
+            tile[ty + 8 * j][tx] = (ch < c && q < hw) ? x[(img * c + ch) * hw + q] : 0.0f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int64_t q = q0 + ty + 8 * j;
+            if (q < hw) {
+                const int64_t at = (img * hw + q) * c_pad + c0 + tx;
+                split_tf32(tile[tx][ty + 8 * j], hi[at], lo[at]);
+            }
+        }
+        __syncthreads();
+    }
 }
 
 struct HaloGeom {
@@ -400,34 +603,83 @@ bool halo_geometry(int64_t h, int64_t w, int64_t kh, int64_t kw, int64_t pad, Ha
 
 } // namespace
 
-// Whether the halo kernel takes this layer (3xTF32 only): stride 1, more than 64 filters (fewer go
+// NHWC float16 planes of x [batch][c][hw] under a scale per image; image_max: batch words of scratch.
+ct_status nhwc_half_planes(
+    DeviceState *st, const float *x, int64_t batch, int64_t c, int64_t hw, int64_t c_pad, void *hi, void *lo, uint32_t *image_max,
+    float *image_scale, uint32_t *wide) {
+    (void)st;
+    CT_CUDA(cudaMemsetAsync(image_max, 0, (size_t)batch * 4, stream()));
+    const int64_t count = c * hw;
+    const int slices    = (int)(count / 16384 < 1 ? 1 : (count / 16384 > 64 ? 64 : count / 16384));
+    const int vec       = (count & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    image_max_kernel<<<(unsigned)(batch * slices), 256, 0, stream()>>>(x, count, slices, vec, image_max);
+    CT_LAUNCH_CHECK("image_max");
+    const dim3 grid((unsigned)((hw + 63) / 64), (unsigned)((c_pad + 63) / 64), (unsigned)batch);
+    nhwc_half_kernel<<<grid, 256, 0, stream()>>>(x, (int)c, hw, (int)c_pad, image_max, static_cast<__half *>(hi),
+                                                 static_cast<__half *>(lo), image_scale, wide);
+    CT_LAUNCH_CHECK("nhwc_half");
+    return CT_OK;
+}
+
+// The tf32 planes instead, where *wide says so.
+ct_status nhwc_wide_planes(
+    DeviceState *st, const uint32_t *wide, const float *x, int64_t batch, int64_t c, int64_t hw, int64_t c_pad, void *hi, void *lo) {
+    wide_nhwc_kernel<<<(unsigned)st->sm_count * 2, 256, 0, stream()>>>(wide, x, batch, (int)c, hw, (int)c_pad,
+                                                                       static_cast<float *>(hi), static_cast<float *>(lo));
+    CT_LAUNCH_CHECK("wide_nhwc");
+    return CT_OK;
+}
+
+// Whether the halo kernel takes this layer (float32 mode only): stride 1, more than 64 filters (fewer go
 // to the kernels that put pixels on the rows or filters in tensor memory), a k range short enough
 // for one accumulation, and a tile that is reasonably full.
 bool conv_halo_applicable(int64_t c_pad, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw, int64_t stride,
                           int64_t pad) {
     HaloGeom g;
-    if (stride != 1 || ko <= 64 || kh * kw * c_pad > 1024 || (c_pad % kH_BlockK) != 0)
+    if (stride != 1 || ko <= 64 || kh * kw * c_pad > 1024 || (c_pad % 32) != 0)
         return false;
     if (!halo_geometry(h, w, kh, kw, pad, &g))
         return false;
     return (int64_t)g.th * g.wo * 10 >= (int64_t)g.n_mma * 7; // at least 70 % of the columns carry an output
 }
 
-// w_hi / w_lo: filter planes [ko][taps * c_pad] (tap-major k); x_hi / x_lo: NHWC planes [batch][h][w][c_pad].
-ct_status conv_halo_stream(
-    DeviceState *st, const void *w_hi, const void *w_lo, const void *x_hi, const void *x_lo, int64_t batch,
-    int64_t c_pad, int64_t h, int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t pad, const float *bias, int act,
-    float *out) {
+// Workspace: [filter scale][image scale][image max][w hi16][w lo16][w hi][w lo][x planes]; the x planes are
+// float16 pairs or, where they do not fit those, tf32 in the same place: no more than tf32 planes alone take.
+ct_status conv_halo(
+    DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t c_pad, int64_t h, int64_t wd, int64_t ko,
+    int64_t kh, int64_t kw, int64_t pad, const float *bias, int act, float *out) {
     HaloGeom g;
     if (!halo_geometry(h, wd, kh, kw, pad, &g))
         return fail(CT_ERR_INVALID, "conv2d: internal tile shape not usable");
+    auto align_up          = [](size_t v) { return (v + 1023) & ~(size_t)1023; };
+    const int64_t taps     = kh * kw, hw = h * wd;
+    const size_t w16       = align_up((size_t)ko * taps * c_pad * 2), w32 = align_up((size_t)ko * taps * c_pad * 4);
+    const size_t x16       = align_up((size_t)batch * hw * c_pad * 2), x32 = align_up((size_t)batch * hw * c_pad * 4);
+    const size_t w_words   = align_up((size_t)ko * 4), x_words = align_up((size_t)batch * 4);
+    if (batch > 65535 || c_pad / 32 > 65535)
+        return fail(CT_ERR_TOO_LARGE, "conv2d: batch or channel count too large for the layout pre-pass");
+    CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, w_words + 2 * x_words + 2 * w16 + 2 * w32 + 2 * x32));
+    uint8_t *ws            = static_cast<uint8_t *>(st->gemm_ws);
+    float *filter_scale    = reinterpret_cast<float *>(ws), *image_scale = reinterpret_cast<float *>(ws + w_words);
+    uint32_t *image_max    = reinterpret_cast<uint32_t *>(ws + w_words + x_words);
+    uint8_t *w16_hi        = ws + w_words + 2 * x_words, *w32_hi = w16_hi + 2 * w16, *xp = w32_hi + 2 * w32;
+    uint32_t *wide         = st->flags_dev + FLAG_WIDE;
+    {
+        ProfScope prof("conv_prepass");
+        filter_planes_kernel<<<(unsigned)ko, 256, 0, stream()>>>(
+            w, (int)c, (int)taps, (int)c_pad, reinterpret_cast<__half *>(w16_hi), reinterpret_cast<__half *>(w16_hi + w16),
+            reinterpret_cast<float *>(w32_hi), reinterpret_cast<float *>(w32_hi + w32), filter_scale, wide);
+        CT_LAUNCH_CHECK("filter_planes");
+        CT_TRY(nhwc_half_planes(st, x, batch, c, hw, c_pad, xp, xp + x16, image_max, image_scale, wide));
+        CT_TRY(nhwc_wide_planes(st, wide, x, batch, c, hw, c_pad, xp, xp + x32));
+    }
     ConvHaloParams p;
+    p.wide = wide, p.filter_scale = filter_scale, p.image_scale = image_scale;
     p.bias = bias, p.out = out, p.flags = st->flags_dev;
     p.ko = (int)ko, p.tiles_m = (int)((ko + 127) / 128);
     p.kh = (int)kh, p.kw = (int)kw, p.pad = (int)pad;
     p.ho = g.ho, p.wo = g.wo, p.pw = g.pw, p.th = g.th;
     p.tiles_y = (g.ho + g.th - 1) / g.th;
-    p.cblocks = (int)(c_pad / kH_BlockK);
     p.c_pad   = (int)c_pad;
     p.n_mma   = g.n_mma;
     p.box_bytes        = g.box_rows * g.pw * kH_RowB;
@@ -436,18 +688,22 @@ ct_status conv_halo_stream(
     const int64_t tiles = (int64_t)p.tiles_m * p.tiles_y * batch;
     if (tiles > 0x7fffffffll)
         return fail(CT_ERR_TOO_LARGE, "conv2d: too many tiles");
-    CUtensorMap mw_hi, mw_lo, mx_hi, mx_lo;
-    const uint64_t kp = (uint64_t)(kh * kw * c_pad);
-    const uint64_t wdims[2] = {kp, (uint64_t)ko}, wstr[1] = {kp * 4};
-    const uint32_t wbox[2]  = {kH_BlockK, 128};
-    CT_TRY(encode_tiled_map_f32(&mw_hi, w_hi, 2, wdims, wstr, wbox, kH_RowB));
-    CT_TRY(encode_tiled_map_f32(&mw_lo, w_lo, 2, wdims, wstr, wbox, kH_RowB));
-    const uint64_t row = (uint64_t)c_pad * 4;
-    const uint64_t xdims[4] = {(uint64_t)c_pad, (uint64_t)wd, (uint64_t)h, (uint64_t)batch};
-    const uint64_t xstr[3]  = {row, row * (uint64_t)wd, row * (uint64_t)wd * (uint64_t)h};
-    const uint32_t xbox[4]  = {kH_BlockK, (uint32_t)g.pw, (uint32_t)g.box_rows, 1};
-    CT_TRY(encode_tiled_map_f32(&mx_hi, x_hi, 4, xdims, xstr, xbox, kH_RowB));
-    CT_TRY(encode_tiled_map_f32(&mx_lo, x_lo, 4, xdims, xstr, xbox, kH_RowB));
+    ConvHaloMaps maps;
+    auto encode = [&](CUtensorMap *mw, const uint8_t *wp, CUtensorMap *mx, const uint8_t *xpl, int elem) {
+        const uint64_t kp = (uint64_t)(taps * c_pad), row = (uint64_t)(c_pad * elem);
+        const uint64_t wdims[2] = {kp, (uint64_t)ko}, wstr[1] = {kp * (uint64_t)elem};
+        const uint32_t wbox[2]  = {(uint32_t)(kH_RowB / elem), 128};
+        const uint64_t xdims[4] = {(uint64_t)c_pad, (uint64_t)wd, (uint64_t)h, (uint64_t)batch};
+        const uint64_t xstr[3]  = {row, row * (uint64_t)wd, row * (uint64_t)wd * (uint64_t)h};
+        const uint32_t xbox[4]  = {(uint32_t)(kH_RowB / elem), (uint32_t)g.pw, (uint32_t)g.box_rows, 1};
+        auto fn = elem == 4 ? encode_tiled_map_f32 : encode_tiled_map_f16;
+        CT_TRY(fn(mw, wp, 2, wdims, wstr, wbox, kH_RowB));
+        return fn(mx, xpl, 4, xdims, xstr, xbox, kH_RowB);
+    };
+    CT_TRY(encode(&maps.w16_hi, w16_hi, &maps.x16_hi, xp, 2));
+    CT_TRY(encode(&maps.w16_lo, w16_hi + w16, &maps.x16_lo, xp + x16, 2));
+    CT_TRY(encode(&maps.w32_hi, w32_hi, &maps.x32_hi, xp, 4));
+    CT_TRY(encode(&maps.w32_lo, w32_hi + w32, &maps.x32_lo, xp + x32, 4));
     // the kernel also has a little static shared memory (barriers, the bias): ask for exactly what
     // this geometry needs, remembering the largest request per device
     static size_t attr_bytes_dev[16] = {};
@@ -458,7 +714,7 @@ ct_status conv_halo_stream(
     }
     const unsigned grid = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
     ProfScope prof("gemm_tc");
-    conv_halo_stream_kernel<<<grid, kH_Threads, g.smem, stream()>>>(mw_hi, mw_lo, mx_hi, mx_lo, p, (int)tiles);
+    conv_halo_stream_kernel<<<grid, kH_Threads, g.smem, stream()>>>(maps, p, (int)tiles);
     CT_LAUNCH_CHECK("conv_halo_stream");
     return CT_OK;
 }

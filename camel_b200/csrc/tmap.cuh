@@ -31,9 +31,14 @@ ct_status conv_tmem_filters(
 // conv2d with one input halo per tile and channel block serving every tap (conv_halo.cu).
 bool conv_halo_applicable(int64_t c_pad, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw, int64_t stride,
                           int64_t pad);
-ct_status conv_halo_stream(
-    DeviceState *st, const void *w_hi, const void *w_lo, const void *x_hi, const void *x_lo, int64_t batch,
-    int64_t c_pad, int64_t h, int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t pad, const float *bias, int act,
-    float *out);
+ct_status nhwc_half_planes(
+    DeviceState *st, const float *x, int64_t batch, int64_t c, int64_t hw, int64_t c_pad, void *hi, void *lo, uint32_t *image_max,
+    float *image_scale, uint32_t *wide);
+ct_status nhwc_wide_planes(
+    DeviceState *st, const uint32_t *wide, const float *x, int64_t batch, int64_t c, int64_t hw, int64_t c_pad, void *hi, void *lo);
+// x NCHW and w OIHW float32; c_pad: channels rounded up to 32.
+ct_status conv_halo(
+    DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t c_pad, int64_t h, int64_t wd, int64_t ko,
+    int64_t kh, int64_t kw, int64_t pad, const float *bias, int act, float *out);
 
 } // namespace ct

@@ -118,7 +118,8 @@ def _conv64(x, w, stride, pad):
 
 # (n, c, h, w, ko, kernel, stride, pad): patches in registers and read twice (k = 1200), odd sizes; halos with a
 # partial last tile, channels that do not fill a block, more than 128 filters, 1 x 1 and 5 x 5 taps
-CONVS = [(3, 48, 21, 23, 70, 3, 2, 1), (2, 8, 33, 21, 20, 3, 2, 0), (2, 48, 15, 16, 40, 5, 3, 2), (2, 12, 24, 24, 65, 5, 1, 2)]
+CONVS = [(3, 48, 21, 23, 70, 3, 2, 1), (2, 8, 33, 21, 20, 3, 2, 0), (2, 48, 15, 16, 40, 5, 3, 2), (2, 12, 24, 24, 65, 5, 1, 2),
+         (2, 64, 30, 28, 128, 3, 1, 1), (3, 40, 14, 14, 136, 3, 1, 0), (2, 100, 17, 19, 72, 1, 1, 0), (2, 20, 57, 56, 72, 5, 1, 2)]
 
 
 @pytest.mark.parametrize("shape", CONVS)
