@@ -34,6 +34,7 @@
 // kernel, not per value.  One CTA per SM walks the tiles.  Every wait is bounded.
 #include "common.cuh"
 #include "tc_ptx.cuh"
+#include "half_split.cuh"
 #include "split.cuh"
 #include "tmap.cuh"
 
@@ -90,6 +91,7 @@ struct ConvTmemParams {
     int plane_bytes;  // shared-memory bytes reserved per plane (box plus the rows shifted reads run into)
     int stages;
     int act, pool;
+    const uint32_t *only_if; // non-null: the launch does nothing unless this word is set
     // raw mode (the input is read as it is, NCHW float32, and split into planes inside the kernel)
     int box_w;        // floats per row of the raw box (a multiple of four)
     int off_x;        // the tile's first position (x = -pad) sits this many floats into a raw row
@@ -142,17 +144,19 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
     __shared__ uint64_t bar_done;
     __shared__ uint64_t bar_epi; // the four epilogue warps meet here (bounded, unlike bar.sync)
     __shared__ uint32_t tmem_base_slot;
-    __shared__ int abort_flag_s;
+    __shared__ int abort_flag_s, idle_s;
     volatile int *abort_flag = &abort_flag_s;
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0) {
         abort_flag_s = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
+        idle_s       = *reinterpret_cast<const volatile uint32_t *>(p.only_if) == 0 ? 1 : 0;
+    }
     __syncthreads();
-    if (abort_flag_s)
-        return;
+    if (abort_flag_s || idle_s)
+        return; // nothing raised the word: conv_tmem_half_kernel has computed the layer
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t stage_bytes = 2u * (uint32_t)p.plane_bytes;
@@ -563,6 +567,485 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 512);
     }
+    if (threadIdx.x == 0) {
+        if (*abort_flag)
+            atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
+        // the last CTA clears the word for the next product
+        if (atomicAdd(p.flags + FLAG_WIDE_READERS, 1u) + 1u == gridDim.x) {
+            p.flags[FLAG_WIDE_READERS] = 0u;
+            p.flags[FLAG_WIDE]         = 0u;
+        }
+    }
+}
+
+// ---- the same in split float16 ------------------------------------------------------------
+//
+// Two 11-bit terms in float16 instead of tf32 (half_split.cuh): 16 channels per MMA instead of 8, so half the
+// MMAs, half the filter columns in tensor memory and half the plane bytes.  The filters are scaled per
+// filter, the pixels per tile (the converting warps see the whole box before they split it) or, from planes,
+// per image.  The low terms are stored 2^11 times larger, so hi and lo products have accumulators of their own:
+//     D1 = [W_hi; W_lo] x X_hi,  D2 = [W_hi; W_lo] x X_lo   (128 x 128 each, next to at most 192 filter columns)
+// and a thread that drains row m forms D1 + 2^-11 D2 before anything is parked, which leaves the rest of the
+// epilogue as it is above (hi row + lo row).  Eight warps convert (four needed 4250 clocks per tile where the
+// MMAs now take 2628) and what sets the pace is the epilogue.  A value, tile or filter that float16 pairs
+// cannot hold raises FLAG_WIDE; conv_tmem_filters_kernel, launched behind this one, then computes the layer again.
+constexpr int kTH_CvtWarps = 8;
+constexpr int kTH_Threads  = 64 + 32 * kTH_CvtWarps + 32 * kTA_EpiWarps;
+constexpr int kTH_D1 = 192, kTH_D2 = 320; // accumulator columns behind 24 k-steps of 8 filter columns
+constexpr int kTH_RowB = 64;              // a position's 32 channels
+
+__device__ __forceinline__ void mma_f16_a_tmem(
+    uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "}\n"
+        :
+        : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+template <bool RAW>
+__global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
+    const __grid_constant__ CUtensorMap map_x_hi, const __grid_constant__ CUtensorMap map_x_lo,
+    const __grid_constant__ ConvTmemParams p, const float *__restrict__ image_scale, const int total_tiles) {
+    constexpr int kMaxStages = 4;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t bar_full[kMaxStages], bar_empty[kMaxStages];
+    __shared__ uint64_t bar_raw_full[kTA_RawStages], bar_raw_empty[kTA_RawStages];
+    __shared__ uint64_t bar_scale_empty[kMaxStages]; // the tile's scale has been read by the epilogue
+    __shared__ uint64_t bar_tmem_full, bar_tmem_empty, bar_done, bar_epi, bar_cvt;
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int abort_flag_s;
+    __shared__ uint32_t cvt_max[2][kTH_CvtWarps];
+    __shared__ float tile_scale[kMaxStages]; // inverse scale of the tile in each plane stage
+    __shared__ float filter_inv[64];
+    __shared__ uint32_t filter_max[64];
+    volatile int *abort_flag = &abort_flag_s;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0)
+        abort_flag_s = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
+    __syncthreads();
+    if (abort_flag_s)
+        return;
+
+    const uint32_t smem_base   = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t stage_bytes = 2u * (uint32_t)p.plane_bytes;
+    const uint32_t raw_base    = smem_base + (uint32_t)p.stages * stage_bytes;
+    const uint32_t raw_all     = RAW ? (uint32_t)kTA_RawStages * (uint32_t)p.raw_stride : 0u;
+    float *staging = reinterpret_cast<float *>(smem_raw + (raw_base - smem_u32(smem_raw)) + raw_all);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < p.stages; ++s) {
+            mbar_init(smem_u32(&bar_full[s]), RAW ? kTH_CvtWarps : 1);
+            mbar_init(smem_u32(&bar_empty[s]), 1);
+            mbar_init(smem_u32(&bar_scale_empty[s]), kTA_EpiWarps);
+        }
+        for (int s = 0; s < kTA_RawStages; ++s) {
+            mbar_init(smem_u32(&bar_raw_full[s]), 1);
+            mbar_init(smem_u32(&bar_raw_empty[s]), kTH_CvtWarps);
+        }
+        mbar_init(smem_u32(&bar_tmem_full), 1);
+        mbar_init(smem_u32(&bar_tmem_empty), kTA_EpiWarps);
+        mbar_init(smem_u32(&bar_done), 1);
+        mbar_init(smem_u32(&bar_epi), kTA_EpiWarps);
+        mbar_init(smem_u32(&bar_cvt), kTH_CvtWarps);
+        mbar_fence_init();
+        prefetch_tensormap(&map_x_hi);
+        prefetch_tensormap(&map_x_lo);
+    }
+    for (int f = warp; f < 64; f += kTH_Threads / 32) { // largest magnitude of each filter, a warp per filter
+        uint32_t mx = 0;
+        if (f < p.ko)
+#pragma unroll 4
+            for (int e = lane; e < p.c * p.kh * p.kw; e += 32)
+                mx = max(mx, __float_as_uint(p.w[(int64_t)f * p.c * p.kh * p.kw + e]) & 0x7fffffffu);
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        if (lane == 0)
+            filter_max[f] = mx;
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(&tmem_base_slot), 512);
+        tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = tmem_base_slot;
+    bool bad = false; // something float16 pairs cannot hold
+
+    // ---- the filters go to tensor memory, once: warps 2..5 own the four lane quarters ----------
+    if (warp >= 2 && warp < 6) {
+        const int quarter = warp & 3;
+        const int m = quarter * 32 + lane, ch = m & 63; // TMEM lane = row of the A operand; filter
+        const bool lo_row = m >= 64;
+        const int taps    = p.kh * p.kw;
+        const float *src  = p.w + (int64_t)ch * p.c * taps;
+        const uint32_t mx = filter_max[ch];
+        float scale = 1.0f, inverse = 1.0f;
+        bad = mx >= 0x7f800000u || !half_scale(mx, scale, inverse);
+        if (!lo_row)
+            filter_inv[ch] = inverse;
+#pragma unroll 2
+        for (int ks = 0; ks < 2 * taps; ++ks) {
+            const int tap = ks >> 1, c0 = (ks & 1) * 16;
+            uint32_t v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                __half part[2];
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    const int ic  = c0 + 2 * j + t;
+                    const float x = (ch < p.ko && ic < p.c) ? src[ic * taps + tap] : 0.0f;
+                    __half hi, lo;
+                    bad |= split_half(x * scale, hi, lo);
+                    part[t] = lo_row ? lo : hi;
+                }
+                v[j] = *reinterpret_cast<uint32_t *>(part);
+            }
+            tmem_st_32x32_x8(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ks * 8), v);
+        }
+        tmem_st_wait();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+
+    if (warp == 0) {
+        // ===== TMA producer: one halo box per plane and tile (raw mode: one box of the input) =====
+        if (lane == 0) {
+            int i = 0;
+            const int nstages = RAW ? kTA_RawStages : p.stages;
+            for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
+                const int img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
+                const int s       = i % nstages;
+                const uint32_t ph = (uint32_t)(i / nstages) & 1u;
+                if (!mbar_wait_patient(smem_u32(RAW ? &bar_raw_empty[s] : &bar_empty[s]), ph ^ 1u, abort_flag))
+                    break;
+                const int32_t h0 = ty * p.th - p.pad;
+                if (RAW) {
+                    const uint32_t full = smem_u32(&bar_raw_full[s]);
+                    mbar_expect_tx(full, (uint32_t)p.raw_bytes);
+                    // the box starts off_x floats left of x = -pad so that its first byte is 16-byte aligned
+                    tma_load_4d(raw_base + (uint32_t)s * (uint32_t)p.raw_stride, &map_x_hi, full, -p.pad - p.off_x, h0, 0, img);
+                } else {
+                    const uint32_t full = smem_u32(&bar_full[s]), dst = smem_base + (uint32_t)s * stage_bytes;
+                    mbar_expect_tx(full, 2u * (uint32_t)p.box_bytes);
+                    tma_load_4d(dst, &map_x_hi, full, 0, -p.pad, h0, img);
+                    tma_load_4d(dst + (uint32_t)p.plane_bytes, &map_x_lo, full, 0, -p.pad, h0, img);
+                }
+            }
+            if (*abort_flag) {
+                // unwind: let the copies still in flight land before the CTA goes away
+                for (int k2 = i - nstages < 0 ? 0 : i - nstages; k2 < i; ++k2) {
+                    const uint32_t bar = smem_u32(RAW ? &bar_raw_full[k2 % nstages] : &bar_full[k2 % nstages]);
+                    const uint64_t t0  = globaltimer_ns();
+                    while (!mbar_try_wait(bar, (uint32_t)(k2 / nstages) & 1u) && globaltimer_ns() - t0 < kWaitBudgetNs) {
+                    }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ===== MMA issuer =====
+        if (lane == 0) {
+            const uint32_t idesc = make_idesc(0u, 128, (uint32_t)kTA_N);
+            const uint32_t d1 = tmem_base + (uint32_t)kTH_D1, d2 = tmem_base + (uint32_t)kTH_D2;
+            int i   = 0;
+            bool ok = true;
+            for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
+                const int s = i % p.stages;
+                // the accumulators of the previous tile have been read, the planes are complete
+                ok = mbar_wait(smem_u32(&bar_tmem_empty), ((uint32_t)i & 1u) ^ 1u, abort_flag) &&
+                     mbar_wait(smem_u32(&bar_full[s]), (uint32_t)(i / p.stages) & 1u, abort_flag);
+                if (!ok)
+                    break;
+                tc_fence_after_sync();
+                const uint32_t x_hi = smem_base + (uint32_t)s * stage_bytes, x_lo = x_hi + (uint32_t)p.plane_bytes;
+                int ks = 0;
+                for (int r = 0; r < p.kh; ++r) {
+                    for (int sx = 0; sx < p.kw; ++sx) {
+                        // the tap's pixels: the same box, (r * pw + sx) rows further on
+                        const uint32_t shift = (uint32_t)(r * p.pw + sx) * (uint32_t)kTH_RowB;
+                        const uint64_t db_hi = smem_desc_k<kTH_RowB>(x_hi + shift), db_lo = smem_desc_k<kTH_RowB>(x_lo + shift);
+#pragma unroll
+                        for (int kk = 0; kk < 2; ++kk, ++ks) {
+                            const uint32_t a_tmem = tmem_base + (uint32_t)(ks * 8);
+                            mma_f16_a_tmem(d1, a_tmem, db_hi + 2 * kk, idesc, ks == 0 ? 0u : 1u);
+                            mma_f16_a_tmem(d2, a_tmem, db_lo + 2 * kk, idesc, ks == 0 ? 0u : 1u);
+                        }
+                    }
+                }
+                tc_commit(smem_u32(&bar_empty[s]));  // the stage is free once these MMAs have retired
+                tc_commit(smem_u32(&bar_tmem_full)); // and the accumulators are complete
+            }
+            if (!ok || *abort_flag) {
+                tc_commit(smem_u32(&bar_done));
+                const uint64_t t0 = globaltimer_ns();
+                while (!mbar_try_wait(smem_u32(&bar_done), 0) && globaltimer_ns() - t0 < kWaitBudgetNs) {
+                }
+            }
+        }
+    } else if (warp < 2 + kTH_CvtWarps) {
+        // ===== raw mode: float32 box -> float16 planes (warps before the epilogue's: see above) =====
+        if (RAW) {
+            const int ct      = threadIdx.x - 64;
+            const int npos    = p.box_rows * p.pw;
+            const int cstride = p.box_rows * p.box_w; // floats between two channels of one position
+            int i = 0;
+            for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
+                const int rs = i % kTA_RawStages, s = i % p.stages;
+                bool got = mbar_wait_patient(smem_u32(&bar_raw_full[rs]), (uint32_t)(i / kTA_RawStages) & 1u, abort_flag);
+                if (!__all_sync(0xffffffffu, got))
+                    break;
+                const float *raw = reinterpret_cast<const float *>(smem_raw + (raw_base - smem_u32(smem_raw)) + (uint32_t)rs * (uint32_t)p.raw_stride);
+                // the tile's largest magnitude (the whole box, alignment columns included: they are pixels or zero)
+                uint32_t mx       = 0;
+                const float4 *r4  = reinterpret_cast<const float4 *>(raw);
+#pragma unroll 4
+                for (int e = ct; e < p.raw_bytes / 16; e += 32 * kTH_CvtWarps) {
+                    const float4 q = r4[e];
+                    mx = max(max(max(mx, __float_as_uint(q.x) & 0x7fffffffu), __float_as_uint(q.y) & 0x7fffffffu),
+                             max(__float_as_uint(q.z) & 0x7fffffffu, __float_as_uint(q.w) & 0x7fffffffu));
+                }
+                mx = __reduce_max_sync(0xffffffffu, mx);
+                if (lane == 0) {
+                    cvt_max[i & 1][warp - 2] = mx;
+                    mbar_arrive(smem_u32(&bar_cvt));
+                }
+                got = mbar_wait(smem_u32(&bar_cvt), (uint32_t)i & 1u, abort_flag) && // all eight maxima
+                      mbar_wait_patient(smem_u32(&bar_empty[s]), ((uint32_t)(i / p.stages) & 1u) ^ 1u, abort_flag) &&
+                      mbar_wait_patient(smem_u32(&bar_scale_empty[s]), ((uint32_t)(i / p.stages) & 1u) ^ 1u, abort_flag);
+                if (!__all_sync(0xffffffffu, got))
+                    break;
+#pragma unroll
+                for (int u = 0; u < kTH_CvtWarps; ++u)
+                    mx = max(mx, cvt_max[i & 1][u]);
+                float scale, inverse;
+                bad |= mx >= 0x7f800000u || !half_scale(mx, scale, inverse);
+                if (ct == 0)
+                    tile_scale[s] = inverse;
+                uint8_t *x_hi = smem_raw + (smem_base - smem_u32(smem_raw)) + (uint32_t)s * stage_bytes;
+                uint8_t *x_lo = x_hi + p.plane_bytes;
+                // a thread takes a position: 32 channels become the 64-byte row y * pw + x of both planes, 16-byte
+                // chunk j at j ^ ((row >> 1) & 3), the 64-byte swizzle
+                for (int pos = ct; pos < npos; pos += 32 * kTH_CvtWarps) {
+                    const int y = pos / p.pw, x = pos - y * p.pw;
+                    const float *src = raw + y * p.box_w + x + p.off_x;
+                    const uint32_t row_off = (uint32_t)pos * (uint32_t)kTH_RowB, sw = ((uint32_t)pos >> 1) & 3u;
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        float v[16];
+#pragma unroll
+                        for (int t = 0; t < 16; ++t)
+                            v[t] = src[(16 * half + t) * cstride];
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+                            __half2 hi[4], lo[4];
+#pragma unroll
+                            for (int t = 0; t < 4; ++t) {
+                                const float a = __fmul_rn(v[8 * j + 2 * t], scale), b = __fmul_rn(v[8 * j + 2 * t + 1], scale);
+                                hi[t] = __floats2half2_rn(a, b);
+                                lo[t] = __floats2half2_rn(__fmul_rn(__fsub_rn(a, __low2float(hi[t])), kHalfLoScale),
+                                                          __fmul_rn(__fsub_rn(b, __high2float(hi[t])), kHalfLoScale));
+                                bad |= (a != 0.0f && fabsf(a) < kHalfSmallest) || (b != 0.0f && fabsf(b) < kHalfSmallest);
+                            }
+                            const uint32_t at = row_off + (((uint32_t)(2 * half + j) ^ sw) << 4);
+                            *reinterpret_cast<uint4 *>(x_hi + at) = *reinterpret_cast<uint4 *>(hi);
+                            *reinterpret_cast<uint4 *>(x_lo + at) = *reinterpret_cast<uint4 *>(lo);
+                        }
+                    }
+                }
+                // written through the generic proxy, read by the tensor core's asynchronous proxy
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(smem_u32(&bar_full[s]));
+                    mbar_arrive(smem_u32(&bar_raw_empty[rs]));
+                }
+            }
+        }
+    } else {
+        // ===== epilogue =====
+        const int quarter = warp & 3;                // TMEM lanes this warp may read
+        const int ew      = warp - 2 - kTH_CvtWarps; // 0..7: which channels this warp writes out
+        const int half    = ew >> 2;                 // which 64 columns of the accumulators it drains
+        uint32_t epi_phase = 0;
+        auto epi_sync = [&]() -> bool {
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(smem_u32(&bar_epi));
+            bool ok = mbar_wait_patient(smem_u32(&bar_epi), epi_phase, abort_flag);
+            epi_phase ^= 1u;
+            return __all_sync(0xffffffffu, ok);
+        };
+        // where this lane's positions land, once for the whole kernel (see conv_tmem_filters_kernel)
+        int off[4], yy[4];
+        const int npos = p.th * p.pw;
+        const int pw2 = p.wo >> 1, ph2 = p.ho >> 1;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const int pos = lane + 32 * g;
+            off[g] = -1, yy[g] = 0;
+            if (p.pool == 0) {
+                const int y = pos / p.pw, x = pos - y * p.pw;
+                if (pos < npos && x < p.wo)
+                    off[g] = y * p.wo + x, yy[g] = y;
+            } else {
+                const int py = pos / pw2, px = pos - py * pw2;
+                if (py < (p.th >> 1))
+                    off[g] = (2 * py) * p.pw + 2 * px, yy[g] = py; // here: the window's first position
+            }
+        }
+        float bias_r[64 / kTA_EpiWarps];
+#pragma unroll
+        for (int j = 0; j < 64 / kTA_EpiWarps; ++j) {
+            const int ch = ew + kTA_EpiWarps * j;
+            bias_r[j]    = (p.bias && ch < p.ko) ? p.bias[ch] : 0.0f;
+        }
+        const int m       = quarter * 32 + lane;
+        const float row_f = m < 64 ? filter_inv[m] : filter_inv[m - 64] * kHalfLoInv;
+        int i = 0;
+        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
+            const int img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
+            bool got = mbar_wait_patient(smem_u32(&bar_tmem_full), (uint32_t)i & 1u, abort_flag);
+            if (!__all_sync(0xffffffffu, got))
+                break;
+            const float is = RAW ? *const_cast<volatile float *>(&tile_scale[i % p.stages]) : image_scale[img];
+            const int y0   = ty * p.th;
+            tc_fence_after_sync();
+            float4 *mine         = reinterpret_cast<float4 *>(staging + m * kTA_StageRowF + half * 64);
+            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 64);
+            // D1 + 2^-11 D2, sixteen columns of each at a time; the accumulators are handed back before anything
+            // is parked
+            float t[64];
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                uint32_t a[16], b[16];
+                tmem_ld_32x16(taddr + kTH_D1 + 16 * g, a);
+                tmem_ld_32x16(taddr + kTH_D2 + 16 * g, b);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    t[16 * g + j] = __fadd_rn(__uint_as_float(a[j]), __fmul_rn(__uint_as_float(b[j]), kHalfLoInv));
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(smem_u32(&bar_tmem_empty)); // the next tile's MMAs may start
+                mbar_arrive(smem_u32(&bar_scale_empty[i % p.stages]));
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                mine[j] = make_float4(__fmul_rn(t[4 * j], row_f), __fmul_rn(t[4 * j + 1], row_f),
+                                      __fmul_rn(t[4 * j + 2], row_f), __fmul_rn(t[4 * j + 3], row_f));
+            if (!epi_sync())
+                break;
+            unsigned okmask = 0;
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+                if (off[g] >= 0 && (p.pool ? (y0 >> 1) + yy[g] < ph2 : y0 + yy[g] < p.ho))
+                    okmask |= 1u << g;
+            // two channels at a time, every load of the pair before the first dependent instruction, masked stores
+            if (p.pool == 0) {
+#pragma unroll
+                for (int jj = 0; jj < 64 / kTA_EpiWarps; jj += 2) {
+                    float h[2][4], l[2][4];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const float *hi = staging + (ew + kTA_EpiWarps * (jj + u)) * kTA_StageRowF + lane, *lo = hi + 64 * kTA_StageRowF;
+#pragma unroll
+                        for (int g = 0; g < 4; ++g)
+                            h[u][g] = hi[32 * g], l[u][g] = lo[32 * g];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const int ch = ew + kTA_EpiWarps * (jj + u);
+                        float *plane = p.out + (((int64_t)img * p.ko + ch) * p.ho + y0) * p.wo;
+                        const unsigned mask = ch < p.ko ? okmask : 0u;
+#pragma unroll
+                        for (int g = 0; g < 4; ++g) {
+                            float v = __fmul_rn(__fadd_rn(h[u][g], l[u][g]), is);
+                            if (p.bias)
+                                v = __fadd_rn(v, bias_r[jj + u]);
+                            if (p.act == CT_ACT_RELU)
+                                v = __fmul_rn(v, v > 0.0f ? 1.0f : 0.0f);
+                            if (mask & (1u << g))
+                                plane[off[g]] = v;
+                        }
+                    }
+                }
+            } else {
+                // 2x2 max-pool of the activated values; window order and strict '>' as in maxpool2d.  Four channels
+                // at a time with all their loads first, a window row as one 8-byte read where rows are even: with
+                // scalar reads for two channels this phase took 3500 clocks per tile, the longest of all.
+                const int groups = ((p.th >> 1) * pw2 + 31) >> 5;
+                const bool even  = (p.pw & 1) == 0;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    if (g >= groups)
+                        break;
+                    const bool live = (okmask >> g) & 1u;
+                    const int pos   = live ? off[g] : 0;
+#pragma unroll
+                    for (int jj = 0; jj < 64 / kTA_EpiWarps; jj += 4) {
+                        float2 h[4][2], l[4][2];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const float *hi = staging + (ew + kTA_EpiWarps * (jj + u)) * kTA_StageRowF + pos, *lo = hi + 64 * kTA_StageRowF;
+                            if (even) {
+                                h[u][0] = *reinterpret_cast<const float2 *>(hi), h[u][1] = *reinterpret_cast<const float2 *>(hi + p.pw);
+                                l[u][0] = *reinterpret_cast<const float2 *>(lo), l[u][1] = *reinterpret_cast<const float2 *>(lo + p.pw);
+                            } else {
+                                h[u][0] = make_float2(hi[0], hi[1]), h[u][1] = make_float2(hi[p.pw], hi[p.pw + 1]);
+                                l[u][0] = make_float2(lo[0], lo[1]), l[u][1] = make_float2(lo[p.pw], lo[p.pw + 1]);
+                            }
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int ch = ew + kTA_EpiWarps * (jj + u);
+                            const float hv[4] = {h[u][0].x, h[u][0].y, h[u][1].x, h[u][1].y};
+                            const float lv[4] = {l[u][0].x, l[u][0].y, l[u][1].x, l[u][1].y};
+                            float v[4];
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                v[q] = __fmul_rn(__fadd_rn(hv[q], lv[q]), is);
+                                if (p.bias)
+                                    v[q] = __fadd_rn(v[q], bias_r[jj + u]);
+                                if (p.act == CT_ACT_RELU)
+                                    v[q] = __fmul_rn(v[q], v[q] > 0.0f ? 1.0f : 0.0f);
+                            }
+                            float best = v[0];
+                            if (v[1] > best)
+                                best = v[1];
+                            if (v[2] > best)
+                                best = v[2];
+                            if (v[3] > best)
+                                best = v[3];
+                            if (live && ch < p.ko) {
+                                float *plane = p.out + (((int64_t)img * p.ko + ch) * ph2 + (y0 >> 1)) * pw2;
+                                plane[lane + 32 * g] = best; // pooled pixels of a tile are consecutive
+                            }
+                        }
+                    }
+                }
+            }
+            if (!epi_sync()) // the staging block is rewritten by the next tile
+                break;
+        }
+    }
+
+    if (bad)
+        p.flags[FLAG_WIDE] = 1u;
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after_sync();
+        tmem_dealloc(tmem_base, 512);
+    }
     if (threadIdx.x == 0 && *abort_flag)
         atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
 }
@@ -595,7 +1078,8 @@ bool conv_tmem_applicable(int64_t c, int64_t h, int64_t w, int64_t ko, int64_t k
 }
 
 // Shared-memory plan of a launch: tile rows, bytes per plane and per raw box, pipeline stages.
-static bool conv_tmem_plan(ConvTmemParams &p, int64_t h, int64_t wd, int64_t kh, int64_t kw, int64_t pad, int pool, bool raw) {
+static bool conv_tmem_plan(
+    ConvTmemParams &p, int64_t h, int64_t wd, int64_t kh, int64_t kw, int64_t pad, int pool, bool raw, int row_bytes = 128) {
     p.pad = (int)pad, p.kh = (int)kh, p.kw = (int)kw;
     p.pw  = (int)(wd + 2 * pad);
     p.wo  = p.pw - (int)kw + 1;
@@ -608,12 +1092,12 @@ static bool conv_tmem_plan(ConvTmemParams &p, int64_t h, int64_t wd, int64_t kh,
     p.tiles_y  = (p.ho + p.th - 1) / p.th;
     p.ksteps   = (int)(kh * kw * 4);
     p.box_rows = p.th + (int)kh - 1;
-    p.box_bytes = p.box_rows * p.pw * 128;
+    p.box_bytes = p.box_rows * p.pw * row_bytes;
     // a tap's shifted window of kTA_N rows may run past the box: reserve those rows too
     int rows_needed = ((int)kh - 1) * p.pw + ((int)kw - 1) + kTA_N;
     if (rows_needed < p.box_rows * p.pw)
         rows_needed = p.box_rows * p.pw;
-    p.plane_bytes = (rows_needed * 128 + 1023) & ~1023;
+    p.plane_bytes = (rows_needed * row_bytes + 1023) & ~1023;
     // raw mode: the box starts at the 16-byte boundary at or left of x = -pad and is a whole number
     // of 16-byte units wide
     const int pad_up = ((int)pad + 3) & ~3;
@@ -633,64 +1117,96 @@ static bool conv_tmem_plan(ConvTmemParams &p, int64_t h, int64_t wd, int64_t kh,
 // Whether the kernel can read this input as it is (NCHW float32) instead of pre-split NHWC planes:
 // the tensor map over it needs row strides of whole 16-byte units and an aligned base, and the raw
 // boxes have to fit into shared memory beside two stages of planes.
-bool conv_tmem_reads_input_directly(const float *x, int64_t h, int64_t w, int64_t kh, int64_t kw, int64_t pad, int pool) {
+static bool conv_tmem_reads_input_directly(const float *x, int64_t h, int64_t w, int64_t kh, int64_t kw, int64_t pad, int pool) {
     if ((w & 3) != 0 || (reinterpret_cast<uintptr_t>(x) & 15u) != 0)
         return false;
     ConvTmemParams p;
     return conv_tmem_plan(p, h, w, kh, kw, pad, pool, true);
 }
 
-// x_raw != nullptr: the input itself, [batch][c][h][w] float32 (see conv_tmem_reads_input_directly);
-// else x_hi / x_lo: NHWC planes [batch][h][w][32] of the input (float32 hi / lo parts).
+// x NCHW float32.  The layer in split float16, and behind it the tf32 form, which does nothing unless the first
+// (or its pre-pass) has raised FLAG_WIDE.  Where the rows allow a tensor map over it the input is read as it is;
+// else from NHWC planes in the workspace: [image scale][image max][planes], float16 first, tf32 in the same place.
 ct_status conv_tmem_filters(
-    DeviceState *st, const float *x_raw, const void *x_hi, const void *x_lo, const float *w, const float *bias,
-    int64_t batch, int64_t c, int64_t h, int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t pad, int act, int pool,
-    float *out) {
-    const bool raw = x_raw != nullptr;
-    ConvTmemParams p;
-    p.w = w, p.bias = bias, p.out = out, p.flags = st->flags_dev;
-    p.ko = (int)ko, p.c = (int)c;
-    p.act = act, p.pool = pool;
-    if (!conv_tmem_plan(p, h, wd, kh, kw, pad, pool, raw))
-        return fail(CT_ERR_INVALID, "conv2d: internal tile shape %d x %d not usable", p.th, p.pw);
-    const int box_rows = p.box_rows;
-    const int64_t tiles = (int64_t)p.tiles_y * batch;
+    DeviceState *st, const float *x, const float *w, const float *bias, int64_t batch, int64_t c, int64_t h, int64_t wd,
+    int64_t ko, int64_t kh, int64_t kw, int64_t pad, int act, int pool, float *out) {
+    const bool raw = conv_tmem_reads_input_directly(x, h, wd, kh, kw, pad, pool);
+    ConvTmemParams p[2]; // float16, tf32
+    for (int f = 0; f < 2; ++f) {
+        p[f].w = w, p[f].bias = bias, p[f].out = out, p[f].flags = st->flags_dev;
+        p[f].ko = (int)ko, p[f].c = (int)c;
+        p[f].act = act, p[f].pool = pool;
+        p[f].only_if = st->flags_dev + FLAG_WIDE;
+        if (!conv_tmem_plan(p[f], h, wd, kh, kw, pad, pool, raw, f == 0 ? kTH_RowB : 128))
+            return fail(CT_ERR_INVALID, "conv2d: internal tile shape %d x %d not usable", p[f].th, p[f].pw);
+    }
+    const int64_t tiles = (int64_t)p[0].tiles_y * batch;
     if (tiles > 0x7fffffffll)
         return fail(CT_ERR_TOO_LARGE, "conv2d: too many tiles");
-    CUtensorMap mx_hi, mx_lo;
+    static bool attr_set_dev[16] = {}; // the attribute belongs to a device's context
+    if (!attr_set_dev[st->device & 15]) {
+        CT_CUDA(cudaFuncSetAttribute(conv_tmem_filters_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        CT_CUDA(cudaFuncSetAttribute(conv_tmem_filters_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        CT_CUDA(cudaFuncSetAttribute(conv_tmem_half_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        CT_CUDA(cudaFuncSetAttribute(conv_tmem_half_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        attr_set_dev[st->device & 15] = true;
+    }
+    auto smem_of = [&](const ConvTmemParams &q) {
+        return (size_t)q.stages * 2 * q.plane_bytes + (raw ? (size_t)kTA_RawStages * q.raw_stride : 0) + kTA_StagingBytes + 1024;
+    };
+    const unsigned grid = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
     if (raw) {
         // the input [batch][c][h][w]; box = box_w floats x box_rows rows x 32 channels of one image, not
         // swizzled; outside the image and past the last channel it reads as zero: padding for free
+        CUtensorMap map;
         const uint64_t dims[4]    = {(uint64_t)wd, (uint64_t)h, (uint64_t)c, (uint64_t)batch};
         const uint64_t strides[3] = {4ull * (uint64_t)wd, 4ull * (uint64_t)wd * (uint64_t)h,
                                      4ull * (uint64_t)wd * (uint64_t)h * (uint64_t)c};
-        const uint32_t box[4]     = {(uint32_t)p.box_w, (uint32_t)box_rows, 32, 1};
-        CT_TRY(encode_tiled_map_f32(&mx_hi, x_raw, 4, dims, strides, box, /*swizzle_bytes=*/0));
-        mx_lo = mx_hi;
-    } else {
-        // planes [batch][h][w][32 channels]; box = 32 channels x pw positions x (th + kh - 1) rows of one
-        // image, 128-byte swizzle; positions outside the image read as zero: the padding
-        const uint64_t dims[4]    = {32, (uint64_t)wd, (uint64_t)h, (uint64_t)batch};
-        const uint64_t strides[3] = {128, 128ull * (uint64_t)wd, 128ull * (uint64_t)wd * (uint64_t)h};
-        const uint32_t box[4]     = {32, (uint32_t)p.pw, (uint32_t)box_rows, 1};
-        CT_TRY(encode_tiled_map_f32(&mx_hi, x_hi, 4, dims, strides, box, /*swizzle_bytes=*/128));
-        CT_TRY(encode_tiled_map_f32(&mx_lo, x_lo, 4, dims, strides, box, 128));
+        const uint32_t box[4]     = {(uint32_t)p[0].box_w, (uint32_t)p[0].box_rows, 32, 1};
+        CT_TRY(encode_tiled_map_f32(&map, x, 4, dims, strides, box, /*swizzle_bytes=*/0));
+        ProfScope prof("gemm_tc");
+        conv_tmem_half_kernel<true><<<grid, kTH_Threads, smem_of(p[0]), stream()>>>(map, map, p[0], nullptr, (int)tiles);
+        CT_LAUNCH_CHECK("conv_tmem_half");
+        conv_tmem_filters_kernel<true><<<grid, kTA_ThreadsRaw, smem_of(p[1]), stream()>>>(map, map, p[1], (int)tiles);
+        CT_LAUNCH_CHECK("conv_tmem_filters");
+        return CT_OK;
     }
-    const size_t smem = (size_t)p.stages * 2 * p.plane_bytes + (raw ? (size_t)kTA_RawStages * p.raw_stride : 0) +
-                        kTA_StagingBytes + 1024;
-    static bool attr_set_dev[16] = {}; // the attribute belongs to a device's context
-    bool &attr_set = attr_set_dev[st->device & 15];
-    if (!attr_set) {
-        CT_CUDA(cudaFuncSetAttribute(conv_tmem_filters_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        CT_CUDA(cudaFuncSetAttribute(conv_tmem_filters_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        attr_set = true;
+    auto align_up        = [](size_t v) { return (v + 1023) & ~(size_t)1023; };
+    const size_t words   = align_up((size_t)batch * 4);
+    const size_t plane32 = align_up((size_t)batch * h * wd * 32 * 4), plane16 = align_up((size_t)batch * h * wd * 32 * 2);
+    if (batch > 65535)
+        return fail(CT_ERR_TOO_LARGE, "conv2d: batch or channel count too large for the layout pre-pass");
+    CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, 2 * words + 2 * plane32));
+    uint8_t *ws = static_cast<uint8_t *>(st->gemm_ws), *planes = ws + 2 * words;
+    float *image_scale = reinterpret_cast<float *>(ws);
+    {
+        ProfScope prof("conv_prepass");
+        CT_TRY(nhwc_half_planes(st, x, batch, c, h * wd, 32, planes, planes + plane16, reinterpret_cast<uint32_t *>(ws + words),
+                                image_scale, st->flags_dev + FLAG_WIDE));
     }
-    const unsigned grid = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
+    // planes [batch][h][w][32 channels]; box = 32 channels x pw positions x (th + kh - 1) rows of one image,
+    // swizzled over a row; positions outside the image read as zero: the padding
+    auto encode = [&](CUtensorMap *map, const void *base, int elem) {
+        const uint64_t row = 32ull * (uint64_t)elem;
+        const uint64_t dims[4] = {32, (uint64_t)wd, (uint64_t)h, (uint64_t)batch};
+        const uint64_t strides[3] = {row, row * (uint64_t)wd, row * (uint64_t)wd * (uint64_t)h};
+        const uint32_t box[4] = {32, (uint32_t)p[0].pw, (uint32_t)p[0].box_rows, 1};
+        return elem == 4 ? encode_tiled_map_f32(map, base, 4, dims, strides, box, 128)
+                         : encode_tiled_map_f16(map, base, 4, dims, strides, box, kTH_RowB);
+    };
+    CUtensorMap m16_hi, m16_lo, m32_hi, m32_lo;
+    CT_TRY(encode(&m16_hi, planes, 2));
+    CT_TRY(encode(&m16_lo, planes + plane16, 2));
+    CT_TRY(encode(&m32_hi, planes, 4));
+    CT_TRY(encode(&m32_lo, planes + plane32, 4));
+    {
+        ProfScope prof("gemm_tc");
+        conv_tmem_half_kernel<false><<<grid, kTH_Threads, smem_of(p[0]), stream()>>>(m16_hi, m16_lo, p[0], image_scale, (int)tiles);
+        CT_LAUNCH_CHECK("conv_tmem_half");
+    }
+    CT_TRY(nhwc_wide_planes(st, st->flags_dev + FLAG_WIDE, x, batch, c, h * wd, 32, planes, planes + plane32));
     ProfScope prof("gemm_tc");
-    if (raw)
-        conv_tmem_filters_kernel<true><<<grid, kTA_ThreadsRaw, smem, stream()>>>(mx_hi, mx_lo, p, (int)tiles);
-    else
-        conv_tmem_filters_kernel<false><<<grid, kTA_Threads, smem, stream()>>>(mx_hi, mx_lo, p, (int)tiles);
+    conv_tmem_filters_kernel<false><<<grid, kTA_Threads, smem_of(p[1]), stream()>>>(m32_hi, m32_lo, p[1], (int)tiles);
     CT_LAUNCH_CHECK("conv_tmem_filters");
     return CT_OK;
 }

@@ -22,11 +22,9 @@ ct_status encode_tiled_map_f16(
 // conv2d with the filters in tensor memory (conv_tmem.cu).
 bool conv_tmem_applicable(int64_t c, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw, int64_t stride,
                           int64_t pad, bool *pool_ok = nullptr);
-bool conv_tmem_reads_input_directly(const float *x, int64_t h, int64_t w, int64_t kh, int64_t kw, int64_t pad, int pool);
 ct_status conv_tmem_filters(
-    DeviceState *st, const float *x_raw, const void *x_hi, const void *x_lo, const float *w, const float *bias,
-    int64_t batch, int64_t c, int64_t h, int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t pad, int act, int pool,
-    float *out);
+    DeviceState *st, const float *x, const float *w, const float *bias, int64_t batch, int64_t c, int64_t h, int64_t wd,
+    int64_t ko, int64_t kh, int64_t kw, int64_t pad, int act, int pool, float *out);
 
 // conv2d with one input halo per tile and channel block serving every tap (conv_halo.cu).
 bool conv_halo_applicable(int64_t c_pad, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw, int64_t stride,
