@@ -8,6 +8,7 @@
 #include "common.cuh"
 #include "fastmath.cuh"
 
+#include <algorithm>
 #include <cmath>
 
 namespace ct {
@@ -167,38 +168,6 @@ __device__ __forceinline__ void skinny_finish_logit(
         argmax[row] = best_idx;
 }
 
-// The same for two rows at once, one per half-warp: `sub` is the lane within its half.
-__device__ __forceinline__ void skinny_finish_logit_half(
-    float logit, int64_t row, bool row_valid, int n, int act, int sub, float *__restrict__ out,
-    int64_t *__restrict__ argmax) {
-    bool live = sub < n && row_valid;
-    if (act == CT_ACT_RELU)
-        logit = __fmul_rn(logit, logit > 0.0f ? 1.0f : 0.0f);
-    if (act != CT_ACT_SOFTMAX) {
-        if (live)
-            out[row * n + sub] = logit;
-        return;
-    }
-    float best   = __shfl_sync(0xffffffffu, logit, 0, 16);
-    int best_idx = 0;
-    for (int j = 1; j < n; ++j) {
-        float v = __shfl_sync(0xffffffffu, logit, j, 16);
-        if (v > best) {
-            best     = v;
-            best_idx = j;
-        }
-    }
-    float e  = sub < n ? exp_f32(__fsub_rn(logit, best)) : 0.0f;
-    double s = 0.0;
-    for (int j = 0; j < n; ++j)
-        s += (double)__shfl_sync(0xffffffffu, e, j, 16);
-    float d = (float)s;
-    if (live)
-        out[row * n + sub] = __fdiv_rn(e, d);
-    if (argmax && sub == 0 && row_valid)
-        argmax[row] = best_idx;
-}
-
 // Finishes one output row held as per-lane partial sums: butterfly reduction, then bias,
 // activation, and (for softmax) the row softmax / argmax across the first n lanes.
 template <int N_MAX>
@@ -323,226 +292,307 @@ ct_status launch_skinny_smem(
     return CT_OK;
 }
 
-__device__ __forceinline__ void cp_async_16(void *smem_dst, const void *gmem_src) {
-    uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(gmem_src) : "memory");
+// Few output columns (n <= 16), many rows: the classifier layer and its forward pass in training.  Lanes own
+// values of k, registers own rows: a warp walks k in steps of 32 with R rows at a time, so the activations
+// are read from global memory as they lie (128 contiguous bytes per row and step, any alignment, no staging),
+// and a lane's weights - n doubles, read from shared memory where the whole matrix sits widened for the life
+// of the block - feed R float64 FMAs each.  What bounds it: per step a warp takes 2 n shared-memory cycles and
+// n R / 2 cycles of the SM's float64 pipe, so R = 8 leaves the pipe (and the read of x) as the bound; with rows
+// on lanes and a broadcast weight per FMA, as before, shared memory took four times what the pipe did.
+// 60000 x 785 x 10: 139 -> 80 us (the pipe alone 26, the read of x 29); the rest is issue, two other instructions
+// per FMA, of them the conversions to float64 at 16 per clock and SM.
+//
+// The float64 sums of the lanes are added by exchanging rows first (each step halves the rows a lane keeps),
+// then across what is left; every lane of a group of 32 / R then holds its row's n sums, adds the bias, rounds
+// once and does the activation; softmax and argmax scan the columns in order like the reference.
+constexpr int kFewWarps = 8;
+constexpr int kFewRing  = 64; // activations in a lane's ring: 8 warps x 64 x 128 B = 64 KB an SM, 1 - R / 64 of it in flight
+
+// Asynchronous 4-byte copies into a ring that only the copying lane reads: the depth of the prefetch is then in
+// shared memory and in the hardware's group count, not in registers and their scoreboards - with register
+// prefetch these kernels ran at one memory latency per step whatever its depth.  Zero where !ok.
+__device__ __forceinline__ void copy_async_4(uint32_t dst, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_4(uint32_t dst, const float *src, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING> __device__ __forceinline__ void copy_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
 }
 
-__device__ __forceinline__ void cp_async_4(void *smem_dst, const void *gmem_src) {
-    unsigned dst = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(gmem_src) : "memory");
+// Doubles between two k in shared memory: n rounded up to even, and an odd number of 16-byte units so that the
+// 128-bit reads of consecutive lanes fall into distinct banks.
+template <int NE> struct FewStride { static constexpr int value = (NE / 2) % 2 == 1 ? NE : NE + 2; };
+
+template <int NE, int GROUP>
+__device__ __forceinline__ void few_finish(
+    const double (&sum)[NE], const float *__restrict__ bias, int64_t row, bool row_ok, int n, int act, int sub, float *__restrict__ out, int64_t *__restrict__ argmax) {
+    float logit[NE];
+#pragma unroll
+    for (int j = 0; j < NE; ++j) {
+        double v = sum[j];
+        if (bias && j < n)
+            v += (double)__ldg(bias + j); // the bias is the last term of the float64 sum
+        logit[j] = (float)v;
+        if (act == CT_ACT_RELU)
+            logit[j] = __fmul_rn(logit[j], logit[j] > 0.0f ? 1.0f : 0.0f);
+    }
+    if (act == CT_ACT_SOFTMAX) {
+        float best   = logit[0];
+        int best_idx = 0;
+#pragma unroll
+        for (int j = 1; j < NE; ++j)
+            if (j < n && logit[j] > best)
+                best = logit[j], best_idx = j;
+        if (argmax && sub == 0 && row_ok)
+            argmax[row] = best_idx;
+        // lane `sub` of the group has columns sub, sub + GROUP, ...: its exponentials, then everybody's in column order
+        constexpr int OWN = (NE + GROUP - 1) / GROUP;
+        float own[OWN];
+#pragma unroll
+        for (int u = 0; u < OWN; ++u) {
+            float v = 0.0f;
+#pragma unroll
+            for (int q = 0; q < GROUP; ++q)
+                if (u * GROUP + q < NE && q == sub)
+                    v = logit[u * GROUP + q];
+            own[u] = u * GROUP + sub < n ? exp_f32(__fsub_rn(v, best)) : 0.0f;
+        }
+        double s = 0.0;
+#pragma unroll
+        for (int j = 0; j < NE; ++j) {
+            const float e = __shfl_sync(0xffffffffu, own[j / GROUP], j % GROUP, GROUP);
+            if (j < n)
+                s += (double)e;
+        }
+        const float d = (float)s;
+#pragma unroll
+        for (int u = 0; u < OWN; ++u)
+            if (u * GROUP + sub < n && row_ok)
+                out[row * n + u * GROUP + sub] = __fdiv_rn(own[u], d);
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < NE; ++j)
+        if (j < n && j % GROUP == sub && row_ok)
+            out[row * n + j] = logit[j];
 }
 
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-
-// Waits until at most `pending` of this thread's committed copy groups are still in flight.
-__device__ __forceinline__ void cp_async_wait_pending(int pending) {
-    switch (pending) {
-    case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
-    case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
-    case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
-    case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
-    case 4: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
-    case 5: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
-    case 6: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
-    default: asm volatile("cp.async.wait_group 7;" ::: "memory"); break;
+// acc[r][j] of all lanes -> sum[j] of row `lane / (32 / R)` in every lane.
+template <int R, int NE>
+__device__ __forceinline__ void few_reduce(double (&acc)[R][NE], int lane, double (&sum)[NE]) {
+#pragma unroll
+    for (int half = R / 2, o = 16; half >= 1; half /= 2, o /= 2) {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int r = 0; r < half; ++r)
+#pragma unroll
+            for (int j = 0; j < NE; ++j) {
+                const double give = upper ? acc[r][j] : acc[r + half][j];
+                const double keep = upper ? acc[r + half][j] : acc[r][j];
+                acc[r][j]         = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+    }
+#pragma unroll
+    for (int j = 0; j < NE; ++j) {
+#pragma unroll
+        for (int o = 16 / R; o >= 1; o /= 2)
+            acc[0][j] += __shfl_xor_sync(0xffffffffu, acc[0][j], o);
+        sum[j] = acc[0][j];
     }
 }
 
-// Row-tiled variant for the classifier layer of a large batch.  A block owns 32 rows; warp s owns
-// the k-slice [s*ks, (s+1)*ks) and lane r owns row r, so every weight read is one broadcast
-// shared-memory wavefront for 32 rows (the warp-per-row kernel above re-reads the whole weight
-// matrix from shared memory for every row, which bounds it).  The activations of a slice arrive
-// by 16-byte asynchronous copies in 32-wide k chunks, each its own commit group, so arithmetic on
-// chunk c overlaps the arrival of the later chunks; the weights of the slice are widened to
-// float64 once per block.  NP = ceil(n/2) column pairs; the float64 partial sums of the sixteen
-// slices are added in slice order, then bias, activation and softmax / argmax as above.
-constexpr int kSkinnyWarps = 16; // k-slices per block
-
-#ifdef CT_GEMM_TRACE
-__device__ unsigned long long g_skinny_trace[1024 * 8];
-#define SK_STAMP(slot)                                                                     \
-    do {                                                                                   \
-        if (threadIdx.x == 0 && blockIdx.x < 1024)                                         \
-            g_skinny_trace[blockIdx.x * 8 + (slot)] = (unsigned long long)clock64();       \
-    } while (0)
-#else
-#define SK_STAMP(slot) do { } while (0)
-#endif
-
-template <int NP>
-__global__ void __launch_bounds__(32 * kSkinnyWarps, 1) gemm_skinny_tile_kernel(
-    const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ bias,
-    int64_t m, int k, int n, int ks, int x_aligned, int act, float *__restrict__ out,
-    int64_t *__restrict__ argmax) {
-    constexpr int NE = 2 * NP;
-    extern __shared__ __align__(16) unsigned char skinny_smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int xs_stride = ks + 4; // floats; (ks + 4) / 4 is odd, so 128-bit row reads spread over the banks
-    float *xs           = reinterpret_cast<float *>(skinny_smem) + (size_t)warp * 32 * xs_stride;
-    double *ws = reinterpret_cast<double *>(skinny_smem + (size_t)kSkinnyWarps * 32 * xs_stride * sizeof(float)) +
-                 (size_t)warp * ks * NE;
-    const int64_t row0 = (int64_t)blockIdx.x * 32;
-    const int k0       = warp * ks;
-    int klen           = k - k0;
-    klen               = klen < 0 ? 0 : (klen > ks ? ks : klen);
-    const int nchunks  = (klen + 31) >> 5;
+template <int NE, int R>
+__global__ void __launch_bounds__(32 * kFewWarps, 1) gemm_few_columns_kernel(
+    const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ bias, int64_t m, int k, int n,
+    int act, float *__restrict__ out, int64_t *__restrict__ argmax) {
+    constexpr int S = FewStride<NE>::value, D = kFewRing / R; // steps in the ring
+    extern __shared__ __align__(16) double w_few[]; // [k rounded up to 32][S], then the warps' rings [D][R][32] floats
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int steps = (k + 31) >> 5;
     griddep_launch_dependents();
     griddep_wait(); // activations (and possibly weights) come from the previous kernel
-    SK_STAMP(0);
-    // weights of the slice, w[(k0 + kk) * n + j] -> ws[kk * NE + j], widened once.  The first round of
-    // loads is issued before the activation copies so that its latency passes while those are issued.
-    const float *wsrc    = w + (int64_t)k0 * n;
-    const int total      = klen * n;
-    constexpr int kLoads = 20; // independent loads in flight per lane: one round for 64 x 10 weights
-    float tmp[kLoads];
-    auto load_round = [&](int base) {
+    // the walk of a warp: tiles of R rows, 32 values of k a step; the fetch runs D - 1 steps ahead of it, across tiles
+    const int64_t tiles = (m + R - 1) / R, first = (int64_t)blockIdx.x + (int64_t)warp * gridDim.x;
+    const int64_t stride = (int64_t)gridDim.x * kFewWarps;
+    float *ring = reinterpret_cast<float *>(w_few + (size_t)steps * 32 * S) + warp * kFewRing * 32 + lane;
+    const uint32_t ring_a = (uint32_t)__cvta_generic_to_shared(ring);
+    int64_t f_tile = first;
+    int f_step = 0, f_slot = 0;
+    const float *f_src = x + first * R * k + lane; // this lane's element of the first row
+    auto fetch = [&]() {
+        if (f_tile < tiles) {
+            const uint32_t dst = ring_a + (uint32_t)(f_slot * R) * 128u;
+            const int kk       = f_step * 32 + lane;
+            if (f_tile * R + R <= m && f_step * 32 + 32 <= k) {
 #pragma unroll
-        for (int u = 0; u < kLoads; ++u) {
-            int i  = base + u * 32;
-            tmp[u] = i < total ? __ldg(wsrc + i) : 0.0f;
-        }
-    };
-    auto store_round = [&](int base) {
+                for (int r = 0; r < R; ++r)
+                    copy_async_4(dst + (uint32_t)r * 128u, f_src + (int64_t)r * k);
+            } else {
 #pragma unroll
-        for (int u = 0; u < kLoads; ++u) {
-            int i = base + u * 32;
-            if (i < total) {
-                // n is NE or NE - 1: divisions by constants instead of one by a run-time value
-                int kk = n == NE ? i / NE : i / (NE > 1 ? NE - 1 : 1);
-                int j  = i - kk * n;
-                ws[kk * NE + j] = (double)tmp[u];
-            }
-        }
-    };
-    load_round(lane);
-    // activations: chunk c covers k0 + [32c, 32c+32) of the block's 32 rows; eight lanes copy one row's 128 bytes
-    for (int c = 0; c < nchunks; ++c) {
-        if (x_aligned) {
-            for (int idx = lane; idx < 256; idx += 32) {
-                int r = idx >> 3, kk = c * 32 + (idx & 7) * 4;
-                if (kk < klen && row0 + r < m)
-                    cp_async_16(xs + r * xs_stride + kk, x + (row0 + r) * k + k0 + kk);
-            }
-        } else {
-            // k is not a multiple of four (784 features and a bias column): rows start at any
-            // 4-byte address, so a warp copies the 32 floats of a row's chunk one per lane
-            const int kk = c * 32 + lane;
-            if (kk < klen) {
-                const float *src = x + row0 * k + k0 + kk;
-                float *dst       = xs + kk;
-                const int rows   = m - row0 < 32 ? (int)(m - row0) : 32;
-#pragma unroll 4
-                for (int r = 0; r < rows; ++r, src += k, dst += xs_stride)
-                    cp_async_4(dst, src);
-            }
-        }
-        cp_async_commit();
-    }
-    // the arithmetic walks k in fours: zero what lies between the end of the slice and the next four
-    const int kpad = (klen + 3) & ~3;
-    if (kpad > klen) {
-        const int extra = kpad - klen;
-        for (int idx = lane; idx < 32 * extra; idx += 32)
-            xs[(idx / extra) * xs_stride + klen + idx % extra] = 0.0f;
-        for (int idx = lane; idx < extra * NE; idx += 32)
-            ws[klen * NE + idx] = 0.0;
-    }
-    SK_STAMP(1);
-    store_round(lane);
-    for (int base = lane + 32 * kLoads; base < total; base += 32 * kLoads) {
-        load_round(base);
-        store_round(base);
-    }
-    if (n < NE)
-        for (int kk = lane; kk < klen; kk += 32)
-            ws[kk * NE + n] = 0.0;
-    __syncwarp();
-    SK_STAMP(2);
-    double acc[NE];
-#pragma unroll
-    for (int j = 0; j < NE; ++j)
-        acc[j] = 0.0;
-    const float *xrow = xs + lane * xs_stride;
-    for (int c = 0; c < nchunks; ++c) {
-        cp_async_wait_pending(nchunks - 1 - c);
-        __syncwarp();
-        if (c == 0)
-            SK_STAMP(3);
-        int kend = (c + 1) * 32 < klen ? (c + 1) * 32 : klen;
-#pragma unroll 4
-        for (int kk = c * 32; kk < kend; kk += 4) {
-            float4 q     = *reinterpret_cast<const float4 *>(xrow + kk);
-            double xd[4] = {(double)q.x, (double)q.y, (double)q.z, (double)q.w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const double2 *wp = reinterpret_cast<const double2 *>(ws + (kk + u) * NE);
-#pragma unroll
-                for (int j = 0; j < NP; ++j) {
-                    double2 wv = wp[j];
-                    // float32 x float32 is exact in float64, so the fused form rounds like mul, add
-                    acc[2 * j]     = __fma_rn(xd[u], wv.x, acc[2 * j]);
-                    acc[2 * j + 1] = __fma_rn(xd[u], wv.y, acc[2 * j + 1]);
+                for (int r = 0; r < R; ++r) {
+                    const bool ok = kk < k && f_tile * R + r < m;
+                    copy_async_4(dst + (uint32_t)r * 128u, ok ? f_src + (int64_t)r * k : x, ok);
                 }
             }
+            f_src += 32;
+            if (++f_step == steps) {
+                f_step = 0, f_tile += stride;
+                f_src = x + f_tile * R * k + lane;
+            }
         }
-    }
-    SK_STAMP(4);
-    __syncthreads(); // every warp is done with its activations: the region becomes the partial sums
-    double *red = reinterpret_cast<double *>(skinny_smem);
+        copy_async_commit();
+        f_slot = f_slot + 1 == D ? 0 : f_slot + 1;
+    };
+#pragma unroll 1
+    for (int d = 0; d < D - 1; ++d)
+        fetch();
+    // the weights, widened once per block: a thread takes rows of w
+#pragma unroll 4
+    for (int kk = threadIdx.x; kk < steps * 32; kk += 32 * kFewWarps) {
+        float v[NE];
 #pragma unroll
-    for (int j = 0; j < NE; ++j)
-        red[((size_t)warp * 32 + lane) * NE + j] = acc[j];
+        for (int j = 0; j < NE; ++j)
+            v[j] = (kk < k && j < n) ? __ldg(w + (int64_t)kk * n + j) : 0.0f;
+#pragma unroll
+        for (int j = 0; j < NE; j += 2)
+            *reinterpret_cast<double2 *>(w_few + kk * S + j) = make_double2((double)v[j], (double)v[j + 1]);
+    }
     __syncthreads();
-    SK_STAMP(5);
-    // two rows per warp, one per half-warp; lane (sub) j < n of a half finishes column j
-    static_assert(kSkinnyWarps == 16, "the finish phase maps one row to each half-warp");
-    {
-        const int sub = lane & 15;
-        const int r   = warp * 2 + (lane >> 4);
-        float logit   = 0.0f;
-        if (sub < n) {
-            double part[kSkinnyWarps];
+    int slot = 0;
+    for (int64_t t = first; t < tiles; t += stride) {
+        const int64_t row0 = t * R;
+        double acc[R][NE];
 #pragma unroll
-            for (int s = 0; s < kSkinnyWarps; ++s)
-                part[s] = red[((size_t)s * 32 + r) * NE + sub];
-            double v = 0.0;
+        for (int r = 0; r < R; ++r)
 #pragma unroll
-            for (int s = 0; s < kSkinnyWarps; ++s)
-                v += part[s];
-            if (bias)
-                v += (double)bias[sub];
-            logit = (float)v;
+            for (int j = 0; j < NE; ++j)
+                acc[r][j] = 0.0;
+#pragma unroll 1
+        for (int step = 0; step < steps; ++step) {
+            copy_async_wait<D - 2>();
+            double xv[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                xv[r] = (double)ring[(slot * R + r) * 32];
+            slot = slot + 1 == D ? 0 : slot + 1;
+            const double2 *wp = reinterpret_cast<const double2 *>(w_few + (step * 32 + lane) * S);
+#pragma unroll
+            for (int j = 0; j < NE / 2; ++j) {
+                const double2 wv = wp[j];
+                // float32 x float32 is exact in float64, so the fused form rounds like mul, add
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    acc[r][2 * j]     = __fma_rn(xv[r], wv.x, acc[r][2 * j]);
+                    acc[r][2 * j + 1] = __fma_rn(xv[r], wv.y, acc[r][2 * j + 1]);
+                }
+            }
+            fetch(); // into the slot before this one, whose values have been used
         }
-        skinny_finish_logit_half(logit, row0 + r, row0 + r < m, n, act, sub, out, argmax);
+        double sum[NE];
+        few_reduce<R, NE>(acc, lane, sum);
+        constexpr int group = 32 / R;
+        const int64_t row   = row0 + lane / group;
+        few_finish<NE, group>(sum, bias, row, row < m, n, act, lane % group, out, argmax);
     }
-    SK_STAMP(6);
 }
 
-// Slice length of the tiled kernel: a multiple of 8 so that (ks + 4) / 4 is odd.
-inline int skinny_tile_slice(int64_t k) { return (int)((((k + kSkinnyWarps - 1) / kSkinnyWarps) + 7) / 8 * 8); }
-
-inline size_t skinny_tile_smem(int64_t k, int np) {
-    int ks    = skinny_tile_slice(k);
-    size_t xs = (size_t)kSkinnyWarps * 32 * (ks + 4) * sizeof(float);
-    size_t ws = (size_t)kSkinnyWarps * ks * 2 * np * sizeof(double);
-    size_t rd = (size_t)kSkinnyWarps * 32 * 2 * np * sizeof(double);
-    return (xs > rd ? xs : rd) + ws;
+// Few rows (a small request), or a weight matrix too long for shared memory: a block takes R rows, its eight
+// warps an eighth of k each, weights straight from L2; the warps' sums meet in shared memory in warp order.
+template <int NE, int R>
+__global__ void __launch_bounds__(32 * kFewWarps) gemm_few_rows_kernel(
+    const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ bias, int64_t m, int64_t k, int n,
+    int act, float *__restrict__ out, int64_t *__restrict__ argmax) {
+    __shared__ double part[kFewWarps][R][NE];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    griddep_launch_dependents();
+    griddep_wait();
+    const int64_t row0 = (int64_t)blockIdx.x * R;
+    const int rows     = m - row0 < R ? (int)(m - row0) : R;
+    double acc[R][NE];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < NE; ++j)
+            acc[r][j] = 0.0;
+#pragma unroll 4
+    for (int64_t kk = warp * 32 + lane; kk < k; kk += 32 * kFewWarps) {
+        float q[R], wv[NE];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            q[r] = r < rows ? x[(row0 + r) * k + kk] : 0.0f;
+#pragma unroll
+        for (int j = 0; j < NE; ++j)
+            wv[j] = j < n ? __ldg(w + kk * n + j) : 0.0f;
+#pragma unroll
+        for (int j = 0; j < NE; ++j) {
+            const double wd = (double)wv[j];
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                acc[r][j] = __fma_rn((double)q[r], wd, acc[r][j]);
+        }
+    }
+    double sum[NE];
+    few_reduce<R, NE>(acc, lane, sum);
+    constexpr int group = 32 / R;
+    if (lane % group == 0)
+#pragma unroll
+        for (int j = 0; j < NE; ++j)
+            part[warp][lane / group][j] = sum[j];
+    __syncthreads();
+    if (warp == 0) {
+        const int r = lane / group;
+#pragma unroll
+        for (int j = 0; j < NE; ++j) {
+            double v = part[0][r][j];
+#pragma unroll
+            for (int u = 1; u < kFewWarps; ++u)
+                v += part[u][r][j];
+            sum[j] = v;
+        }
+        few_finish<NE, group>(sum, bias, row0 + r, row0 + r < m, n, act, lane % group, out, argmax);
+    }
 }
 
-template <int NP>
-ct_status launch_skinny_tile(
-    const float *a, const float *b, const float *bias, int64_t m, int64_t k, int n, int act, float *out,
+template <int NE>
+ct_status launch_few(
+    DeviceState *st, const float *a, const float *b, const float *bias, int64_t m, int64_t k, int n, int act, float *out,
     int64_t *argmax) {
-    size_t smem = skinny_tile_smem(k, NP);
-    if (smem > 48 * 1024)
-        CT_CUDA(cudaFuncSetAttribute(
-            gemm_skinny_tile_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CT_CUDA(launch_dependent(
-        gemm_skinny_tile_kernel<NP>, dim3((unsigned)((m + 31) / 32)), dim3(32 * kSkinnyWarps), smem, stream(), a, b, bias,
-        m, (int)k, n, skinny_tile_slice(k), (int)((k & 3) == 0 && (reinterpret_cast<uintptr_t>(a) & 15u) == 0), act, out,
-        argmax));
-    CT_LAUNCH_CHECK("gemm_skinny_tile");
+    const size_t smem = (size_t)((k + 31) / 32 * 32) * FewStride<NE>::value * sizeof(double) + kFewWarps * kFewRing * 128;
+    // Resident weights pay from where a block's warps get a few tiles each (k = 785, n = 10: 9.7 against 21.8 us at
+    // 2048 rows, 12.5 us both ways at 1024); below, and for weights beyond shared memory, blocks of four (two) rows
+    // read them from L2.
+    if (smem <= 220 * 1024 && m >= 2048) {
+        // eight rows per warp where there are rows enough for two such tiles each and the sums stay in registers
+        const bool deep = NE <= 12 && m >= (int64_t)st->sm_count * kFewWarps * 8 * 2;
+        static bool attr_set_dev[16] = {};
+        if (!attr_set_dev[st->device & 15]) {
+            CT_CUDA(cudaFuncSetAttribute(gemm_few_columns_kernel<NE, (NE <= 12 ? 8 : 4)>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+            CT_CUDA(cudaFuncSetAttribute(gemm_few_columns_kernel<NE, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+            attr_set_dev[st->device & 15] = true;
+        }
+        constexpr int kDeep  = NE <= 12 ? 8 : 4;
+        const int rows       = deep ? kDeep : 4;
+        const int64_t tiles  = (m + rows - 1) / rows;
+        const unsigned grid  = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
+        if (deep)
+            CT_CUDA(launch_dependent(gemm_few_columns_kernel<NE, kDeep>, dim3(grid), dim3(32 * kFewWarps), smem, stream(), a, b, bias, m,
+                                     (int)k, n, act, out, argmax));
+        else
+            CT_CUDA(launch_dependent(gemm_few_columns_kernel<NE, 4>, dim3(grid), dim3(32 * kFewWarps), smem, stream(), a, b, bias, m,
+                                     (int)k, n, act, out, argmax));
+        CT_LAUNCH_CHECK("gemm_few_columns");
+        return CT_OK;
+    }
+    if (m <= 2 * st->sm_count)
+        CT_CUDA(launch_dependent(gemm_few_rows_kernel<NE, 2>, dim3((unsigned)((m + 1) / 2)), dim3(32 * kFewWarps), 0, stream(), a, b,
+                                 bias, m, k, n, act, out, argmax));
+    else
+        CT_CUDA(launch_dependent(gemm_few_rows_kernel<NE, 4>, dim3((unsigned)((m + 3) / 4)), dim3(32 * kFewWarps), 0, stream(), a, b,
+                                 bias, m, k, n, act, out, argmax));
+    CT_LAUNCH_CHECK("gemm_few_rows");
     return CT_OK;
 }
 
@@ -572,44 +622,32 @@ ct_status matmul_generic(
 // the slices' float64 sums are added in slice order by gemm_tn_skinny_finish_kernel, so the result
 // does not depend on scheduling.  Bound by the float64 pipe and the read of X, which are about
 // equal at n = 10.
-constexpr int kTnThreads = 128;
+//
+// R and the warps of a block are chosen so that the block's warps cover the output rows evenly: with blocks of
+// 4 x 128 rows, 785 features made every other block a quarter full.  785 x 60000 x 10: 94 -> 90 us, 785 x 256 x 10:
+// 18 us.
+constexpr int kTnMinThreads = 64, kTnMaxThreads = 160; // two blocks to an SM at 200 registers
 constexpr int kTnChunk   = 32; // rows of b staged per step
-constexpr int kTnGroup   = 4;  // k steps whose operands are fetched together, one group ahead
-
-template <int V> struct TnCount {
-    static constexpr int value = V;
-};
-
-// A read-only load that stays where it is written: the compiler may otherwise move a plain load
-// down to its first use, which undoes fetching the operands a group ahead.  0 where !ok.
-__device__ __forceinline__ float tn_load_early(const float *p, bool ok) {
-    float v;
-    asm volatile(
-        "{ .reg .pred q; setp.ne.u32 q, %2, 0; mov.f32 %0, 0f00000000; @q ld.global.nc.f32 %0, [%1]; }"
-        : "=f"(v)
-        : "l"(p), "r"((unsigned)ok));
-    return v;
-}
+constexpr int kTnGroup   = 2;  // k steps fetched together
+constexpr int kTnGroups  = 6;  // groups in a warp's ring, all but one in flight
 
 __device__ __forceinline__ void tn_block_barrier() {
     // a named barrier counts arriving threads, wherever in the code they arrive from: the warps of a
     // block run differently specialised copies of the loop below
-    asm volatile("bar.sync 1, %0;" ::"n"(kTnThreads) : "memory");
+    asm volatile("bar.sync 1, %0;" ::"r"(blockDim.x) : "memory");
 }
 
 template <int NMAX, int R>
-__global__ void __launch_bounds__(kTnThreads, 2) gemm_tn_skinny_kernel(
+__global__ void __launch_bounds__(kTnMaxThreads, 2) gemm_tn_skinny_kernel(
     const float *__restrict__ a_km, const float *__restrict__ b, int64_t m, int64_t k, int n, int64_t k_per_slice,
     double *__restrict__ partial) {
     constexpr int G  = kTnGroup;
-    constexpr int BL = (kTnChunk * NMAX + kTnThreads - 1) / kTnThreads; // staged b values per thread
-    __shared__ double bs[2][kTnChunk][NMAX];
+    constexpr int BL = (kTnChunk * NMAX + kTnMinThreads - 1) / kTnMinThreads; // staged b values per thread
+    __shared__ __align__(16) double bs[2][kTnChunk][NMAX];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t warp_row = ((int64_t)blockIdx.x * (kTnThreads / 32) + warp) * (32 * R);
+    const int threads      = (int)blockDim.x;
+    const int64_t warp_row = ((int64_t)blockIdx.x * (threads / 32) + warp) * (32 * R);
     const int64_t row0     = warp_row + lane;
-    // 32-row groups of this warp that hold rows at all: the others cost no loads and no arithmetic
-    const int64_t left = m - warp_row;
-    const int ractive  = left <= 0 ? 0 : (left >= 32 * R ? R : (int)((left + 31) / 32));
     const int64_t k0   = (int64_t)blockIdx.y * k_per_slice;
     const int64_t k1   = k0 + k_per_slice < k ? k0 + k_per_slice : k;
 
@@ -617,110 +655,112 @@ __global__ void __launch_bounds__(kTnThreads, 2) gemm_tn_skinny_kernel(
     auto fetch_b = [&](int64_t kc) {
 #pragma unroll
         for (int u = 0; u < BL; ++u) {
-            int idx = threadIdx.x + u * kTnThreads;
-            int kk = idx / NMAX, j = idx - kk * NMAX;
+            const int idx = threadIdx.x + u * threads;
+            if (u * threads >= kTnChunk * NMAX)
+                break;
+            const int kk = idx / NMAX, j = idx - kk * NMAX;
             bnext[u] = (idx < kTnChunk * NMAX && kc + kk < k1 && j < n) ? __ldg(b + (kc + kk) * n + j) : 0.0f;
         }
     };
     auto store_b = [&](int buf) {
 #pragma unroll
         for (int u = 0; u < BL; ++u) {
-            int idx = threadIdx.x + u * kTnThreads;
+            const int idx = threadIdx.x + u * threads;
+            if (u * threads >= kTnChunk * NMAX)
+                break;
             if (idx < kTnChunk * NMAX)
                 (&bs[buf][0][0])[idx] = (double)bnext[u];
         }
     };
 
-    auto run = [&](auto count) {
-        constexpr int RA = decltype(count)::value; // 32-row groups this warp computes
-        constexpr int RN = RA > 0 ? RA : 1;
-        double acc[RN][NMAX];
+    double acc[R][NMAX];
 #pragma unroll
-        for (int r = 0; r < RN; ++r)
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < NMAX; ++j)
+            acc[r][j] = 0.0;
+    // the operand arrives G k steps at a time in a ring of its own for each lane
+    __shared__ float ring_s[kTnMaxThreads / 32][kTnGroups][G][R][32];
+    float(*ring)[G][R][32] = ring_s[warp];
+    const float *pa        = a_km + k0 * m + row0; // row `next` of the operand, this lane's first column
+    int64_t next           = k0;
+    int put = 0, get = 0;
+    const uint32_t ring_a = (uint32_t)__cvta_generic_to_shared(&ring[0][0][0][lane]);
+    const bool full       = warp_row + 32 * R <= m;
+    auto fetch_a = [&]() {
+        const uint32_t dst = ring_a + (uint32_t)put * (G * R * 128u);
+        if (full && next + G <= k1) {
+#pragma unroll
+            for (int u = 0; u < G; ++u) {
+                const float *src = pa + u * m;
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    copy_async_4(dst + (uint32_t)(u * R + r) * 128u, src + 32 * r);
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const bool ok = next + u < k1 && row0 + 32 * r < m;
+                    copy_async_4(dst + (uint32_t)(u * R + r) * 128u, ok ? pa + u * m + 32 * r : a_km, ok);
+                }
+        }
+        copy_async_commit();
+        pa += G * m;
+        next += G;
+        put = put + 1 == kTnGroups ? 0 : put + 1;
+    };
+    auto compute = [&](int buf, int g) {
+        copy_async_wait<kTnGroups - 2>();
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+            double av[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                av[r] = (double)ring[get][u][r][lane];
+#pragma unroll
+            for (int j = 0; j < NMAX; j += 2) {
+                const double2 bj = *reinterpret_cast<const double2 *>(&bs[buf][g + u][j]);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    acc[r][j]     = fma(av[r], bj.x, acc[r][j]);
+                    acc[r][j + 1] = fma(av[r], bj.y, acc[r][j + 1]);
+                }
+            }
+        }
+        get = get + 1 == kTnGroups ? 0 : get + 1;
+    };
+    fetch_b(k0);
+#pragma unroll 1
+    for (int d = 0; d < kTnGroups - 1; ++d)
+        fetch_a();
+    store_b(0);
+    tn_block_barrier();
+    int buf = 0;
+    for (int64_t kc = k0; kc < k1; kc += kTnChunk, buf ^= 1) {
+        const bool more = kc + kTnChunk < k1;
+        if (more)
+            fetch_b(kc + kTnChunk);
+#pragma unroll 1
+        for (int g = 0; g < kTnChunk; g += G) {
+            compute(buf, g);
+            fetch_a(); // may already belong to the next chunk; zeros past the slice
+        }
+        if (more)
+            store_b(buf ^ 1); // nobody reads that buffer any more: all warps passed the last barrier
+        tn_block_barrier();
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (row0 + 32 * r < m) {
+            double *dst = partial + ((int64_t)blockIdx.y * m + row0 + 32 * r) * n;
 #pragma unroll
             for (int j = 0; j < NMAX; ++j)
-                acc[r][j] = 0.0;
-        bool rowok[RN];
-#pragma unroll
-        for (int r = 0; r < RN; ++r)
-            rowok[r] = row0 + 32 * r < m;
-        // operands of G k steps are fetched one group ahead of their use, into two register sets
-        float abuf[2][G][RN];
-        const float *pa = a_km + k0 * m + row0; // row `next` of the operand, this lane's first column
-        int64_t next    = k0;
-        auto fetch_a    = [&](float(&dst)[G][RN]) {
-            if (RA > 0) {
-#pragma unroll
-                for (int u = 0; u < G; ++u)
-#pragma unroll
-                    for (int r = 0; r < RN; ++r)
-                        dst[u][r] = tn_load_early(pa + u * m + 32 * r, next + u < k1 && rowok[r]);
-                pa += G * m;
-                next += G;
-            }
-        };
-        auto compute = [&](const float(&src)[G][RN], int buf, int g) {
-            if (RA > 0) {
-#pragma unroll
-                for (int u = 0; u < G; ++u) {
-                    double av[RN];
-#pragma unroll
-                    for (int r = 0; r < RN; ++r)
-                        av[r] = (double)src[u][r];
-#pragma unroll
-                    for (int j = 0; j < NMAX; ++j) {
-                        double bj = bs[buf][g + u][j];
-#pragma unroll
-                        for (int r = 0; r < RN; ++r)
-                            acc[r][j] = fma(av[r], bj, acc[r][j]);
-                    }
-                }
-            }
-        };
-        fetch_b(k0);
-        fetch_a(abuf[0]);
-        store_b(0);
-        tn_block_barrier();
-        int buf = 0;
-        for (int64_t kc = k0; kc < k1; kc += kTnChunk, buf ^= 1) {
-            const bool more = kc + kTnChunk < k1;
-            if (more)
-                fetch_b(kc + kTnChunk);
-#pragma unroll 1
-            for (int g = 0; g < kTnChunk; g += 2 * G) {
-                fetch_a(abuf[1]);
-                compute(abuf[0], buf, g);
-                fetch_a(abuf[0]); // may already belong to the next chunk; zeros past the slice
-                compute(abuf[1], buf, g + G);
-            }
-            if (more)
-                store_b(buf ^ 1); // nobody reads that buffer any more: all warps passed the last barrier
-            tn_block_barrier();
+                if (j < n)
+                    dst[j] = acc[r][j];
         }
-        if (RA > 0) {
-#pragma unroll
-            for (int r = 0; r < RN; ++r) {
-                if (rowok[r]) {
-                    double *dst = partial + ((int64_t)blockIdx.y * m + row0 + 32 * r) * n;
-#pragma unroll
-                    for (int j = 0; j < NMAX; ++j)
-                        if (j < n)
-                            dst[j] = acc[r][j];
-                }
-            }
-        }
-    };
-    static_assert(R == 1 || R == 2 || R == 4, "row groups per warp");
-    if (ractive == R)
-        run(TnCount<R>{});
-    else if (ractive == 0)
-        run(TnCount<0>{});
-    else if (R == 4 && ractive == 3)
-        run(TnCount<(R == 4 ? 3 : 1)>{});
-    else if (R == 4 && ractive == 2)
-        run(TnCount<(R == 4 ? 2 : 1)>{});
-    else
-        run(TnCount<1>{});
+    }
 }
 
 // One warp per output element: lane l adds the slices l, l + 32, ... in that order, then the lanes'
@@ -744,11 +784,20 @@ __global__ void __launch_bounds__(256) gemm_tn_skinny_finish_kernel(
 template <int NMAX, int R>
 static ct_status launch_tn_skinny(
     DeviceState *st, const float *a_km, const float *b, int64_t m, int64_t k, int n, float *out) {
-    const int64_t rows_per_block = (int64_t)(kTnThreads / 32) * 32 * R;
-    const int64_t mblocks        = (m + rows_per_block - 1) / rows_per_block;
-    // one wave: two blocks fit an SM, and rounding the slice length up only takes blocks away
-    int64_t slices = 2 * (int64_t)st->sm_count / mblocks;
-    const int64_t most           = (k + 4 * kTnChunk - 1) / (4 * kTnChunk); // at least four chunks per slice
+    const int64_t warps   = (m + 32 * R - 1) / (32 * R);
+    const int64_t mblocks = (warps + kTnMaxThreads / 32 - 1) / (kTnMaxThreads / 32);
+    const int threads     = (int)std::max<int64_t>(kTnMinThreads, (warps + mblocks - 1) / mblocks * 32);
+    // one wave of blocks; rounding the slice length up only takes blocks away
+    static std::atomic<int> per_sm[kTnMaxThreads / 32 + 1];
+    int fit = per_sm[threads / 32].load(std::memory_order_relaxed);
+    if (fit == 0) {
+        CT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, gemm_tn_skinny_kernel<NMAX, R>, threads, 0));
+        fit = fit < 1 ? 1 : fit;
+        per_sm[threads / 32].store(fit, std::memory_order_relaxed);
+    }
+    int64_t slices     = fit * (int64_t)st->sm_count / mblocks;
+    // a warp takes about a fifth of a microsecond per k whatever the size, so a short k is cut down to single chunks
+    const int64_t most = (k + kTnChunk - 1) / kTnChunk;
     if (slices > most)
         slices = most;
     if (slices < 1)
@@ -763,7 +812,7 @@ static ct_status launch_tn_skinny(
     CT_TRY(ensure_ws(&st->splitk_ws, &st->splitk_ws_bytes, (size_t)slices * m * n * sizeof(double)));
     auto *partial = static_cast<double *>(st->splitk_ws);
     dim3 grid((unsigned)mblocks, (unsigned)slices);
-    gemm_tn_skinny_kernel<NMAX, R><<<grid, kTnThreads, 0, stream()>>>(a_km, b, m, k, n, k_per_slice, partial);
+    gemm_tn_skinny_kernel<NMAX, R><<<grid, threads, 0, stream()>>>(a_km, b, m, k, n, k_per_slice, partial);
     CT_LAUNCH_CHECK("gemm_tn_skinny");
     const int64_t mn = m * n;
     gemm_tn_skinny_finish_kernel<<<(unsigned)((mn * 32 + 255) / 256), 256, 0, stream()>>>(partial, mn, (int)slices, out);
@@ -778,17 +827,26 @@ ct_status gemm_f32_tn_skinny(
     if (n > 32 || m > 0x7fffffffll * 64)
         return fail(CT_ERR_INVALID, "transposed skinny GEMM takes at most 32 output columns");
     ProfScope prof("gemm_skinny");
+    // Rows per lane: up to four cost the reads of b in shared memory (2 n cycles per warp and k), more cost
+    // float64 FMAs (R n / 2); take what covers the m / 32 row groups with the least of it.
+    const int64_t groups = (m + 31) / 32;
+    auto cost            = [&](int64_t r) { return (groups + r - 1) / r * (r > 4 ? r : 4); };
+    const bool five      = cost(5) < cost(4);
+#define CT_TN(NMAX)                                                                 \
+    return five ? launch_tn_skinny<NMAX, 5>(st, a_km, b, m, k, (int)n, out) \
+                : launch_tn_skinny<NMAX, 4>(st, a_km, b, m, k, (int)n, out)
     switch ((n + 1) / 2) {
-    case 1: return launch_tn_skinny<2, 4>(st, a_km, b, m, k, (int)n, out);
-    case 2: return launch_tn_skinny<4, 4>(st, a_km, b, m, k, (int)n, out);
-    case 3: return launch_tn_skinny<6, 4>(st, a_km, b, m, k, (int)n, out);
-    case 4: return launch_tn_skinny<8, 4>(st, a_km, b, m, k, (int)n, out);
-    case 5: return launch_tn_skinny<10, 4>(st, a_km, b, m, k, (int)n, out);
-    case 6: return launch_tn_skinny<12, 2>(st, a_km, b, m, k, (int)n, out);
-    case 7: return launch_tn_skinny<14, 2>(st, a_km, b, m, k, (int)n, out);
-    case 8: return launch_tn_skinny<16, 2>(st, a_km, b, m, k, (int)n, out);
+    case 1: CT_TN(2);
+    case 2: CT_TN(4);
+    case 3: CT_TN(6);
+    case 4: CT_TN(8);
+    case 5: CT_TN(10);
+    case 6: return launch_tn_skinny<12, 3>(st, a_km, b, m, k, (int)n, out);
+    case 7: return launch_tn_skinny<14, 3>(st, a_km, b, m, k, (int)n, out);
+    case 8: return launch_tn_skinny<16, 3>(st, a_km, b, m, k, (int)n, out);
     default: break;
     }
+#undef CT_TN
     if (n <= 24)
         return launch_tn_skinny<24, 1>(st, a_km, b, m, k, (int)n, out);
     return launch_tn_skinny<32, 1>(st, a_km, b, m, k, (int)n, out);
@@ -803,24 +861,19 @@ ct_status gemm_f32_skinny(
         return fail(CT_ERR_INVALID, "skinny GEMM takes at most 32 output columns");
     unsigned blocks = (unsigned)((m + 7) / 8);
     ProfScope prof("gemm_skinny");
-    const int np = (int)((n + 1) / 2);
-    if (m >= 256 && n <= 16 && k >= 32 && k <= (1 << 20) && skinny_tile_smem(k, np) <= 220 * 1024) {
-        switch (np) {
-        case 1: return launch_skinny_tile<1>(a, b, bias, m, k, (int)n, act, out, argmax);
-        case 2: return launch_skinny_tile<2>(a, b, bias, m, k, (int)n, act, out, argmax);
-        case 3: return launch_skinny_tile<3>(a, b, bias, m, k, (int)n, act, out, argmax);
-        case 4: return launch_skinny_tile<4>(a, b, bias, m, k, (int)n, act, out, argmax);
-        case 5: return launch_skinny_tile<5>(a, b, bias, m, k, (int)n, act, out, argmax);
-        case 6: return launch_skinny_tile<6>(a, b, bias, m, k, (int)n, act, out, argmax);
-        case 7: return launch_skinny_tile<7>(a, b, bias, m, k, (int)n, act, out, argmax);
-        default: return launch_skinny_tile<8>(a, b, bias, m, k, (int)n, act, out, argmax);
+    if (n <= 16 && m <= 0x7fffffffll && k <= 0x7fffffffll) {
+        switch ((n + 1) / 2) {
+        case 1: return launch_few<2>(st, a, b, bias, m, k, (int)n, act, out, argmax);
+        case 2: return launch_few<4>(st, a, b, bias, m, k, (int)n, act, out, argmax);
+        case 3: return launch_few<6>(st, a, b, bias, m, k, (int)n, act, out, argmax);
+        case 4: return launch_few<8>(st, a, b, bias, m, k, (int)n, act, out, argmax);
+        case 5: return launch_few<10>(st, a, b, bias, m, k, (int)n, act, out, argmax);
+        case 6: return launch_few<12>(st, a, b, bias, m, k, (int)n, act, out, argmax);
+        case 7: return launch_few<14>(st, a, b, bias, m, k, (int)n, act, out, argmax);
+        default: return launch_few<16>(st, a, b, bias, m, k, (int)n, act, out, argmax);
         }
     }
     if ((size_t)k * n * sizeof(double) <= 200 * 1024 && k > 0) {
-        if (n <= 8)
-            return launch_skinny_smem<8>(st, a, b, bias, m, k, (int)n, act, out, argmax);
-        if (n <= 16)
-            return launch_skinny_smem<16>(st, a, b, bias, m, k, (int)n, act, out, argmax);
         return launch_skinny_smem<32>(st, a, b, bias, m, k, (int)n, act, out, argmax);
     }
     if (n <= 8)
@@ -834,9 +887,3 @@ ct_status gemm_f32_skinny(
 }
 
 } // namespace ct
-
-#ifdef CT_GEMM_TRACE
-extern "C" int ct_debug_skinny_trace(unsigned long long *host, int count) {
-    return (int)cudaMemcpyFromSymbol(host, ct::g_skinny_trace, sizeof(unsigned long long) * (size_t)count);
-}
-#endif

@@ -38,7 +38,7 @@ def _check(got, a, b):
 # the drain after 1024 values of k; pairs of CTAs with a ragged last tile; long columns (two passes over B);
 # few rows and a long k (slices through the workspace)
 SHAPES = [(64, 64, 64), (128, 32, 128), (129, 33, 257), (128, 320, 128), (65, 1025, 130), (300, 2080, 260),
-          (4100, 96, 1030), (2304, 1056, 2306), (130, 4128, 131), (40, 9000, 70), (33, 4096, 36)]
+          (4100, 96, 1030), (2304, 1056, 2306), (130, 4128, 131), (40, 9000, 70), (33, 4096, 36), (70, 1500, 66)]
 
 
 @pytest.mark.parametrize("m,k,n", SHAPES)
@@ -138,3 +138,24 @@ def test_convolution_narrow_and_wide(T, shape, kind):
     # a halo layer's k (at most 1024) is one accumulation: up to 384 tf32 additions instead of 96
     bound = 384 * 2.0**-24 + 2.0**-21
     assert np.all(np.abs(got - _conv64(x, w, stride, pad)) <= bound * _conv64(np.abs(x), np.abs(w), stride, pad) + 1e-300)
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 297, 2048, 2051, 19001])
+@pytest.mark.parametrize("k,n", [(1, 3), (31, 1), (33, 16), (785, 10), (96, 13)])
+def test_few_columns(T, m, k, n):
+    rng = np.random.default_rng(m + k + n)
+    x = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    w = rng.uniform(-1, 1, (k, n)).astype(np.float32)
+    b = rng.uniform(-1, 1, n).astype(np.float32)
+    tx, tw, tb = T.from_numpy(x), T.from_numpy(w), T.from_numpy(b)
+    z = x.astype(np.float64) @ w.astype(np.float64) + b
+    # float64 sums in another order, rounded once
+    g = rng.uniform(-1, 1, (m, n)).astype(np.float32)
+    zt = x.astype(np.float64).T @ g.astype(np.float64)
+    assert np.all(np.abs(T.matmul_tn(tx, T.from_numpy(g)).numpy() - zt) <= 2.0**-24 * np.abs(zt) + 1e-12)
+    assert np.all(np.abs(T.dense(tx, tw, tb).numpy() - z) <= 2.0**-24 * np.abs(z) + 1e-13)
+    logits = T.dense(tx, tw, tb).numpy()
+    probs, arg = T.dense(tx, tw, tb, "softmax", with_argmax=True)
+    assert np.array_equal(arg.numpy(), logits.argmax(1))  # first maximum wins in both
+    e = np.exp(logits.astype(np.float64) - logits.max(1, keepdims=True))
+    assert np.all(np.abs(probs.numpy() - e / e.sum(1, keepdims=True)) <= 4 * 2.0**-24)
