@@ -221,7 +221,7 @@ int half_tile_columns(const DeviceState *st, int64_t m, int64_t n, int64_t batch
 ct_status half_split_rows(
     DeviceState *st, const float *in, int64_t k, int64_t kp, const HalfOperand &o, bool both_forms, uint32_t *zero,
     int64_t zero_count);
-bool half_cols_is_short(int64_t kp); // one pass, which needs no col_max and can write both forms
+bool half_cols_is_short(int64_t kp); // one pass, which needs no col_max
 ct_status half_split_cols(
     DeviceState *st, const float *in, int64_t k, int64_t kp, const HalfOperand &o, bool both_forms, uint32_t *col_max);
 ct_status half_split_both(

@@ -2,9 +2,9 @@
 //
 // Each operand value is two 11-bit significands (half_split.cuh); three MMAs of kind::f16 per 16
 // values of k - lo.hi, hi.lo and hi.hi - give the 3xTF32 product at twice its rate, from planes of
-// half the size.  What bounds it: the tensor pipe (three MMAs per product: a third of the f16 rate).
-// 4096 x 1024 x 1024 (one wave of 128 x 256 tiles) and 16384^3, per product: see the table in the
-// launch code below.
+// half the size.  What bounds it: the tensor pipe (three MMAs per product: a third of the f16 rate) for large
+// products - 16384^3: 35.5 -> 21.7 ms, 405 TFLOP/s under the power cap - and for one wave of tiles the set-up,
+// first operands and final store around 14 us of MMAs - 4096 x 1024 x 1024: 36 -> 27 us.
 //
 // Accumulation.  The low terms are stored 2^11 times larger, so the two cross products have an
 // accumulator of their own (joined with weight 2^-11 at the end); the leading accumulator then sees one
@@ -764,9 +764,7 @@ __global__ void __launch_bounds__(256) half_col_max_kernel(
 
 // in [k][n] -> transposed float16 planes [n][kp], inverse column scales.  Blocks of 64 k x 32 columns.
 __global__ void __launch_bounds__(256) half_cols_kernel(
-    const float *__restrict__ in, int64_t k, int64_t n, int64_t kp, __half *__restrict__ p_hi,
-    __half *__restrict__ p_lo, const uint32_t *__restrict__ col_max, float *__restrict__ col_scale,
-    uint32_t *__restrict__ wide) {
+    const float *__restrict__ in, int64_t k, int64_t n, int64_t kp, const HalfPlanes p, const uint32_t *__restrict__ col_max) {
     __shared__ float tile[64][33];
     griddep_launch_dependents();
     griddep_wait();
@@ -786,22 +784,31 @@ __global__ void __launch_bounds__(256) half_cols_kernel(
             float scale, inverse;
             bad |= !half_scale(col_max[nn], scale, inverse);
             if (blockIdx.y == 0 && tx == 0)
-                col_scale[nn] = inverse;
+                p.scale[nn] = inverse;
+            const float v0 = tile[tx * 2][ty + j * 8], v1 = tile[tx * 2 + 1][ty + j * 8];
             __half hi[2], lo[2];
-            bad |= split_half(tile[tx * 2][ty + j * 8] * scale, hi[0], lo[0]);
-            bad |= split_half(tile[tx * 2 + 1][ty + j * 8] * scale, hi[1], lo[1]);
-            *reinterpret_cast<__half2 *>(p_hi + nn * kp + kk) = *reinterpret_cast<__half2 *>(hi);
-            *reinterpret_cast<__half2 *>(p_lo + nn * kp + kk) = *reinterpret_cast<__half2 *>(lo);
+            bad |= split_half(v0 * scale, hi[0], lo[0]);
+            bad |= split_half(v1 * scale, hi[1], lo[1]);
+            *reinterpret_cast<__half2 *>(p.hi16 + nn * kp + kk) = *reinterpret_cast<__half2 *>(hi);
+            *reinterpret_cast<__half2 *>(p.lo16 + nn * kp + kk) = *reinterpret_cast<__half2 *>(lo);
+            if (p.hi32) {
+                float2 h, l;
+                split_tf32_flat(v0, h.x, l.x);
+                split_tf32_flat(v1, h.y, l.y);
+                *reinterpret_cast<float2 *>(p.hi32 + nn * kp + kk) = h;
+                *reinterpret_cast<float2 *>(p.lo32 + nn * kp + kk) = l;
+            }
         }
     }
     if (bad)
-        *wide = 1u;
+        *p.wide = 1u;
 }
 
 // The same for k <= kShortK in one pass: a block keeps the whole length of 8 columns (32 bytes of each row, a
-// sector) in shared memory between the maximum and the split, a warp per column.
+// sector) in shared memory between the maximum and the split, a warp per column.  Up to 1024, where six such blocks
+// share an SM: at 4096 there was one, with too few loads in flight (two passes over the columns are faster).
 constexpr int kShortCols = 8;
-constexpr int kShortK    = 4096;
+constexpr int kShortK    = 1024;
 constexpr int kShortPad  = kShortCols + 1;
 
 __device__ __forceinline__ void half_cols_short(
@@ -1027,12 +1034,6 @@ ct_status half_split_cols(
     const HalfPlanes p = planes_of(o, both_forms);
     const unsigned strips = (unsigned)((n + 31) / 32);
     if (half_cols_is_short(kp)) {
-        static bool attr_set_dev[16] = {};
-        if (!attr_set_dev[st->device & 15]) {
-            CT_CUDA(cudaFuncSetAttribute(half_cols_short_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kShortK * kShortPad * 4));
-            attr_set_dev[st->device & 15] = true;
-        }
         CT_CUDA(launch_dependent(half_cols_short_kernel, dim3((unsigned)((n + kShortCols - 1) / kShortCols)), dim3(256),
                                  (size_t)kp * kShortPad * 4, stream(), in, k, n, kp, p));
         CT_LAUNCH_CHECK("half_cols_short");
@@ -1046,8 +1047,8 @@ ct_status half_split_cols(
         return fail(CT_ERR_TOO_LARGE, "gemm: k too large for the operand pre-pass");
     CT_CUDA(launch_dependent(half_col_max_kernel, dim3(strips, (unsigned)slices), dim3(256), 0, stream(), in, k, n, rows, col_max));
     CT_LAUNCH_CHECK("half_col_max");
-    CT_CUDA(launch_dependent(half_cols_kernel, dim3(strips, (unsigned)slabs), dim3(256), 0, stream(), in, k, n, kp, p.hi16, p.lo16,
-                             static_cast<const uint32_t *>(col_max), p.scale, p.wide));
+    CT_CUDA(launch_dependent(half_cols_kernel, dim3(strips, (unsigned)slabs), dim3(256), 0, stream(), in, k, n, kp, p,
+                             static_cast<const uint32_t *>(col_max)));
     CT_LAUNCH_CHECK("half_cols");
     return CT_OK;
 }

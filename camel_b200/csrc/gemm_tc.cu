@@ -1692,7 +1692,7 @@ static ct_status gemm_f32_split(
     const size_t a32      = align_up((size_t)m * kp * 4), b32 = packed ? 0 : align_up((size_t)n * kp * 4);
     const size_t a16      = align_up((size_t)m * kp * 2), b16 = packed ? 0 : align_up((size_t)n * kp * 2);
     const size_t a_words  = align_up((size_t)m * 4), b_words = align_up((size_t)n * 4);
-    const bool both_forms = half_cols_is_short(kp) && 8 * (m + (packed ? 0 : n)) * kp <= kBothFormsBytes;
+    const bool both_forms = 8 * (m + (packed ? 0 : n)) * kp <= kBothFormsBytes;
     const size_t wide_at  = both_forms ? 2 * (a16 + b16) : 0; // where the tf32 planes start
     CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, 2 * a_words + 2 * b_words + wide_at + 2 * (a32 + b32)));
     uint8_t *ws     = static_cast<uint8_t *>(st->gemm_ws);
