@@ -375,12 +375,6 @@ class MlpWorkload(Workload):
     def algorithmic_per_step(self):
         return 2.0 * self.batch * (784 * 1024 + 1024 * 1024)  # the two tensor-core layers
 
-    def ncu_traffic(self):
-        if self.batch != 4096:
-            return None, "captured at batch 4096 only"
-        return 38.1e6, ("ncu capture of this workload: 43.4 MB (k=1024) and 32.9 MB (k=784) per launch = the "
-                        "operand planes read once; the result stays in L2")
-
     def resident_bytes(self):
         return self.x.nbytes + sum(t.nbytes for t in self.w) + 2 * self.batch * 1024 * 4
 
@@ -435,12 +429,6 @@ class GemmWorkload(Workload):
 
     def algorithmic_per_step(self):
         return 2.0 * self.n ** 3
-
-    def ncu_traffic(self):
-        if self.n == 4096:
-            return 690.7e6, "ncu capture at 4096^3 (335 MB algorithmic: operand tiles re-read 2.1x)"
-        return None, ("captured at 4096^3 only: the re-read factor depends on how the raster groups fit in L2 "
-                      "and does not scale with the flops")
 
     def resident_bytes(self):
         return 3 * self.n * self.n * 4
@@ -574,14 +562,6 @@ class ConvWorkload(Workload):
 
     def algorithmic_per_step(self):
         return self.flops
-
-    def ncu_traffic(self):
-        # batch-32 capture: 52.1 MB read = the NHWC and weight planes once; reads scale with the batch,
-        # and at full size the whole result goes to DRAM (at batch 32 most of it was still in L2)
-        reads = 52.1e6 * self.batch / 32.0
-        writes = self.batch * 128 * 56 * 56 * 4.0
-        return reads + writes, ("ncu capture at batch 32: reads scaled by the batch (planes are read once), "
-                                "writes = the size of the result")
 
     def resident_bytes(self):
         return self.h2d + self.d2h
@@ -1081,7 +1061,8 @@ def measured_mma_peaks(lib, check, sampler):
 
 def roofline_of(wl, m, pk, mma, precision):
     """roofline object of one measured workload.  Tensor-bound kernels are held against the measured
-    MMA rate of this run (tf32 / 3 for the 3xTF32 scheme): the burst figure for launches shorter
+    MMA rate of this run (kind::f16; a third of it for float32 operands, which are split into two
+    float16 terms and take three MMAs per product): the burst figure for launches shorter
     than 5 ms, the sustained one for longer launches; the figure derived from the driver-written
     bf16 GEMM peak is kept beside it.  `frac_at_clock` holds the kernel against the pipe's rate per SM cycle
     (cycle stamps inside the measuring kernel) times the median SM clock sampled during this workload."""
@@ -1091,24 +1072,18 @@ def roofline_of(wl, m, pk, mma, precision):
            "avg_launch_ms": dom_ms}
     if wl.bound == "tensor":
         achieved = alg / (dom_ms / 1e3) / 1e12 if dom_ms > 0 else 0.0
-        kind = "bf16" if precision == "bf16" else "tf32"
+        kind = "bf16"  # kind::f16 with bf16 operands: the rate float16 operands have too
         div = 1.0 if precision == "bf16" else 3.0
-        derived = pk["bf16_tflops"] / (1.0 if precision == "bf16" else 6.0)
+        derived = pk["bf16_tflops"] / div
         if mma is not None:
             which = "burst" if dom_ms < 5.0 else "sustained"
 
             def pipe(w):
-                # a tf32 MMA moves the bytes of a bf16 MMA with half the k: the pipe gives tf32 half the
-                # bf16 rate.  On some GPUs of the pool the tf32 measuring loop itself reads a quarter
-                # lower than that (while the GEMM kernels run as fast as elsewhere), so the ceiling is
-                # the larger of the two readings: never flatter the kernel with a slow measurement.
-                if kind == "bf16":
-                    return mma["bf16"][f"{w}_tflops"]
-                return max(mma["tf32"][f"{w}_tflops"], mma["bf16"][f"{w}_tflops"] / 2.0)
+                return mma["bf16"][f"{w}_tflops"]
 
             peak = pipe(which) / div
             note = (f"measured in this run: tcgen05.mma back to back on resident operands, {which} figure"
-                    + ("" if precision == "bf16" else ", the larger of kind::tf32 and kind::f16 / 2, / 3 (three MMAs per product)"))
+                    + ("" if precision == "bf16" else ", / 3 (three MMAs per product)"))
             out["peak_burst"] = pipe("burst") / div
             out["peak_sustained"] = pipe("sustained") / div
         else:
@@ -1120,8 +1095,6 @@ def roofline_of(wl, m, pk, mma, precision):
         fpc = None
         if mma is not None and mma[kind].get("flop_per_clk_per_sm"):
             fpc = mma[kind]["flop_per_clk_per_sm"]
-            if kind == "tf32" and mma["bf16"].get("flop_per_clk_per_sm"):
-                fpc = max(fpc, mma["bf16"]["flop_per_clk_per_sm"] / 2.0)
         if fpc and c.get("sm_mhz"):
             # the pipe's rate per SM clock (cycle stamps inside the measuring kernel) x SMs x the clock
             # sampled during this workload: what the MMAs alone would reach at the clock the power
@@ -1433,7 +1406,7 @@ def run_gpu(args, rank, world):
         cpu = cpu_baseline(args) if world == 1 and not args.no_cpu_baseline else None
         line = {"metric": wl.metric, "value": value, "unit": wl.unit, "n_gpus": world, "steps": args.steps,
                 "warmup": max(args.warmup, 3), "ms_per_step": ms_per_step, "higher_is_better": True,
-                "scaling": wl.scaling, "vs_baseline": None, "dtype": "f32 (3xTF32 tensor-core products, f32 accumulate)"
+                "scaling": wl.scaling, "vs_baseline": None, "dtype": "f32 (operands split into two 11-bit terms, three tensor-core MMAs per product, f32 accumulate)"
                 if args.precision != "bf16" else "bf16 in / f32 accumulate", "data": "synthetic",
                 "config": {"parallelism": f"{world} ranks, independent shards, no data-path collective",
                            **wl.config(), "l2": "flushed between steps" if m["flush"] else "inputs larger than L2"},

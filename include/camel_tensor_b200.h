@@ -67,7 +67,10 @@ typedef enum ct_activation {
 
 /* Arithmetic of the tensor-core contractions. */
 typedef enum ct_precision {
-    CT_PREC_3XTF32 = 0, /* fp32 in, split into two TF32 terms, three MMAs, fp32 accumulate */
+    CT_PREC_3XTF32 = 0, /* fp32 in, split into two terms of TF32's 11 significant bits, three MMAs, fp32
+                         * accumulate.  The terms are float16 pairs under an exact power-of-two scale per
+                         * row and column; operands whose rows span more than 33 powers of two (or whose
+                         * exponent is beyond +-60) are computed from tf32 terms, decided on the device. */
     CT_PREC_BF16   = 1  /* inputs rounded to bf16 once, fp32 accumulate (reported separately) */
 } ct_precision;
 
@@ -106,8 +109,8 @@ ct_status ct_profile_read(const char *kernel, double *total_ms_host, uint64_t *l
  * 128 x 256 x (32 bytes of k) back to back on operands already in shared memory (kind::tf32 for
  * CT_PREC_3XTF32, kind::f16 on bf16 for CT_PREC_BF16), `launches` launches in a row, timed with
  * CUDA events.  A short burst (one launch of ~50 us) and a seconds-long run give the two figures
- * a roofline needs: the 3xTF32 contractions spend three such MMAs per product, so their ceiling
- * is the tf32 figure / 3.  No reference counterpart (a measurement, not an operator). */
+ * a roofline needs: the float32 contractions spend three MMAs per product, so their ceiling is
+ * a third of the kind::f16 figure (of the tf32 figure for operands that need tf32 terms).  No reference counterpart (a measurement, not an operator). */
 ct_status ct_measure_mma_peak(
     ct_precision kind, int mma_groups, int launches, double *tflops_host, double *ms_host);
 /* The same measurement for another MMA shape: mma_m = 64 or 128 rows, mma_n = 16..256 columns (a
