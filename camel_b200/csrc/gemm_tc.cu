@@ -1760,7 +1760,14 @@ ct_status gemm_f32_tc(
                 CT_ERR_INVALID,
                 "dense: the packed weights were built from another matrix, shape, precision or device");
     }
-    if (mode == MODE_3X)
+    // One tile of rows, or at most nine tiles, and a long k: the product is a fraction of the operands' pre-pass, and what
+    // the tf32 planes need - one pass over B and two launches less - outweighs it (70 x 4000 x 70 22.6 against 26.8 us,
+    // 128 x 8000 x 128 26.5 against 32.6, 129 x 8000 x 129 30.8 against 35.7, 100 x 16000 x 9000 579 against 603; but
+    // 64 x 1500 x 64 22.5 against 17.6).  Only products whose k is sliced over CTAs: the others keep the bytes of
+    // ct_matmul_packed_rows.
+    const int64_t tiles  = ((m + BM - 1) / BM) * ((n + 127) / 128);
+    const bool tf32_form = kp > 2048 && (m <= BM || tiles <= 9) && tiles * 2 <= st->sm_count;
+    if (mode == MODE_3X && !tf32_form)
         return gemm_f32_split(st, a, b, bias, m, k, n, kp, act, out, packed, a_is_km);
     size_t a_plane      = align_up((size_t)m * kp * elem);
     size_t b_plane      = packed ? 0 : align_up((size_t)n * kp * elem);
@@ -1781,7 +1788,10 @@ ct_status gemm_f32_tc(
         dim3 grid((unsigned)((m + 31) / 32), (unsigned)(kp / 32));
         if (grid.y > 65535)
             return fail(CT_ERR_TOO_LARGE, "gemm: k too large for the operand pre-pass");
-        split_transpose_kernel<MODE_BF><<<grid, 256, 0, stream()>>>(a, k, m, kp, a_hi, a_lo);
+        if (mode == MODE_3X)
+            split_transpose_kernel<MODE_3X><<<grid, 256, 0, stream()>>>(a, k, m, kp, a_hi, a_lo);
+        else
+            split_transpose_kernel<MODE_BF><<<grid, 256, 0, stream()>>>(a, k, m, kp, a_hi, a_lo);
         CT_LAUNCH_CHECK("split_transpose");
     } else {
         ProfScope prof("gemm_prepass");
@@ -1792,7 +1802,10 @@ ct_status gemm_f32_tc(
         dim3 grid((unsigned)((n + 31) / 32), (unsigned)(kp / 32));
         if (grid.y > 65535)
             return fail(CT_ERR_TOO_LARGE, "gemm: k too large for the operand pre-pass");
-        split_transpose_kernel<MODE_BF><<<grid, 256, 0, stream()>>>(b, k, n, kp, b_hi, b_lo);
+        if (mode == MODE_3X)
+            split_transpose_kernel<MODE_3X><<<grid, 256, 0, stream()>>>(b, k, n, kp, b_hi, b_lo);
+        else
+            split_transpose_kernel<MODE_BF><<<grid, 256, 0, stream()>>>(b, k, n, kp, b_hi, b_lo);
         CT_LAUNCH_CHECK("split_transpose");
     }
 
