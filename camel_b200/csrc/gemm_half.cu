@@ -1137,8 +1137,10 @@ ct_status gemm_half(
         splits = (int)std::min<int64_t>(std::min<int64_t>(st->sm_count / tiles, p.k_groups / 8), 32);
         if (splits <= 8) {
             splits = 1;
-            while (splits < 8 && tiles * splits * 2 <= st->sm_count && p.k_groups >= splits * 4)
-                splits *= 2; // at least 128 values of k each
+            // at least 128 values of k each; eight slices only up to half of the machine - whole clusters of eight
+            // do not fit every SM, and 16 of them (2000 x 1024 x 100) ran in two waves
+            while (splits < 8 && tiles * splits * 2 <= (splits == 4 ? st->sm_count / 2 : st->sm_count) && p.k_groups >= splits * 4)
+                splits *= 2;
             p.cluster_split = splits;
         }
         p.groups_per_split = splits > 1 ? (p.k_groups + splits - 1) / splits : 0;
