@@ -138,7 +138,11 @@ __global__ void __launch_bounds__(kHThreads, 1)
     __shared__ uint64_t bar_done;
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag_s;
-    __shared__ int tile_stores[2]; // epilogue warps that have stored the tile (bands only)
+    // epilogue warps that have stored a tile (bands only), a counter per tile that may be under way: accumulators
+    // are handed back before the store, so a warp can be kSets tiles ahead of another (one that has no columns to
+    // store always is)
+    static_assert(C::kSets < 4, "tile_stores");
+    __shared__ int tile_stores[4];
     volatile int *abort_flag = &abort_flag_s;
 
     const int warp = threadIdx.x >> 5;
@@ -161,7 +165,7 @@ __global__ void __launch_bounds__(kHThreads, 1)
         }
         mbar_init(smem_u32(&bar_done), 1);
         mbar_fence_init();
-        tile_stores[0] = tile_stores[1] = 0;
+        tile_stores[0] = tile_stores[1] = tile_stores[2] = tile_stores[3] = 0;
         prefetch_tensormap(&maps.a16_hi);
         prefetch_tensormap(&maps.a16_lo);
         prefetch_tensormap(&maps.b16_hi);
@@ -528,12 +532,12 @@ __global__ void __launch_bounds__(kHThreads, 1)
                 __syncwarp(); // the block is rewritten by the next 32 columns
             }
             if (p.bands > 0) {
-                // the last warp to have stored the tile counts it (a warp is at most one tile ahead of another,
-                // so two counters taken in turn are enough)
+                // the last warp to have stored the tile counts it; tile i + 4 comes to the same counter only after
+                // every warp is past tile i
                 __threadfence();
                 __syncwarp();
-                if (lane == 0 && atomicAdd(&tile_stores[i & 1], 1) == kHEpiWarps - 1) {
-                    tile_stores[i & 1] = 0;
+                if (lane == 0 && atomicAdd(&tile_stores[i & 3], 1) == kHEpiWarps - 1) {
+                    tile_stores[i & 3] = 0;
                     __threadfence();
                     atomicAdd(p.band_done + band, 1u);
                 }

@@ -108,6 +108,39 @@ def test_packed_weights_and_row_panels_agree_on_wide_operands(T, wide):
         check(lib.ct_weights_free(wp))
 
 
+def test_band_counts_where_every_block_walks_several_tiles_of_both_accumulator_sets(T):
+    """n <= 64: half of the storing warps have nothing to store and run ahead of the others, over four tiles a block."""
+    import ctypes as C
+
+    import torch
+
+    from camel_b200._lib import check, lib
+
+    rng = np.random.default_rng(12)
+    m, k, n = 4 * 148 * 128 - 60, 40, 64
+    a, w = T.from_numpy(rng.uniform(-1, 1, (m, k)).astype(np.float32)), T.from_numpy(rng.uniform(-1, 1, (k, n)).astype(np.float32))
+    want, got = T.zeros((m, n)), T.zeros((m, n))
+    ap, wp = C.c_void_p(), C.c_void_p()
+    check(lib.ct_rows_pack(a.ptr, m, k, C.byref(ap)))
+    check(lib.ct_weights_pack(w.ptr, k, n, C.byref(wp)))
+    try:
+        check(lib.ct_matmul_packed_rows(ap, 0, m, wp, want.ptr))
+        bands = [148 * 128, 2 * 148 * 128, m - 3 * 148 * 128]
+        first = [0, bands[0], bands[0] + bands[1]]
+        done, tiles = torch.zeros(3, dtype=torch.int32, device="cuda"), (C.c_uint32 * 3)()
+        torch.cuda.synchronize()
+        check(lib.ct_matmul_packed_bands(ap, wp, 3, (C.c_int64 * 3)(*bands),
+                                         (C.c_void_p * 3)(*[got.ptr + f * n * 4 for f in first]), done.data_ptr(), tiles))
+        T.check_async()
+        assert list(tiles) == [148, 296, 148]
+        assert done.cpu().tolist() == list(tiles)
+        assert got.numpy().tobytes() == want.numpy().tobytes()
+        _check(want.numpy(), a.numpy(), w.numpy())
+    finally:
+        check(lib.ct_rows_free(ap))
+        check(lib.ct_weights_free(wp))
+
+
 def _conv64(x, w, stride, pad):
     n, c, h, wd = x.shape
     ko, _, kh, kw = w.shape
