@@ -105,11 +105,10 @@ __global__ void __launch_bounds__(256) im2col_half_kernel(
         bad |= !half_scale(mx, scale, inverse);
         if (lane == 0)
             scale_out[row] = inverse;
-        int small = 0; // values too small beside the patch's largest: one in 256 is let pass
         auto put = [&](int kk, float a, float b) {
             __half hi[2], lo[2];
-            small += split_half(a * scale, hi[0], lo[0]) ? 1 : 0;
-            small += split_half(b * scale, hi[1], lo[1]) ? 1 : 0;
+            bad |= split_half(a * scale, hi[0], lo[0]);
+            bad |= split_half(b * scale, hi[1], lo[1]);
             *reinterpret_cast<__half2 *>(p_hi + row * kp + kk) = *reinterpret_cast<__half2 *>(hi);
             *reinterpret_cast<__half2 *>(p_lo + row * kp + kk) = *reinterpret_cast<__half2 *>(lo);
         };
@@ -122,7 +121,6 @@ __global__ void __launch_bounds__(256) im2col_half_kernel(
             for (int kk = 2 * lane; kk < kp; kk += 64)
                 put(kk, load(kk), load(kk + 1));
         }
-        bad |= __reduce_add_sync(0xffffffffu, small) > kdim / 256;
     }
     if (bad)
         *wide = 1u;

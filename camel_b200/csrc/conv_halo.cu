@@ -479,8 +479,7 @@ __global__ void __launch_bounds__(256) nhwc_half_kernel(
     const float *__restrict__ x, int c, int64_t hw, int c_pad, const uint32_t *img_max, __half *__restrict__ p_hi,
     __half *__restrict__ p_lo, float *__restrict__ image_scale, uint32_t *__restrict__ wide) {
     __shared__ float tile[64][65];
-    uint32_t *img_small = const_cast<uint32_t *>(img_max) + gridDim.z; // values so far that are too small beside their image's largest
-    const int64_t img   = gridDim.z - 1 - blockIdx.z;
+    const int64_t img = gridDim.z - 1 - blockIdx.z;
     const int64_t q0  = (int64_t)blockIdx.x * 64;
     const int c0      = (int)blockIdx.y * 64;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -493,8 +492,7 @@ __global__ void __launch_bounds__(256) nhwc_half_kernel(
             tile[ch][q]  = (c0 + ch < c && q0 + q < hw) ? __ldcs(src + ch * hw + q) : 0.0f;
         }
     float scale, inverse;
-    const bool bad = !half_scale(img_max[img], scale, inverse);
-    int small      = 0;
+    bool bad = !half_scale(img_max[img], scale, inverse);
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
         image_scale[img] = inverse;
     __syncthreads();
@@ -505,17 +503,12 @@ __global__ void __launch_bounds__(256) nhwc_half_kernel(
             __half hi[8], lo[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-                small += split_half(tile[chunk * 8 + j][q] * scale, hi[j], lo[j]) ? 1 : 0;
+                bad |= split_half(tile[chunk * 8 + j][q] * scale, hi[j], lo[j]);
             const int64_t at = (img * hw + q0 + q) * c_pad + c0 + chunk * 8;
             *reinterpret_cast<uint4 *>(p_hi + at) = *reinterpret_cast<uint4 *>(hi);
             *reinterpret_cast<uint4 *>(p_lo + at) = *reinterpret_cast<uint4 *>(lo);
         }
     }
-    // A large image of ordinary (normal) values has one that small now and then; only more than one, and more than
-    // one in 65536, send the layer to the tf32 planes.
-    small = __reduce_add_sync(0xffffffffu, small);
-    if (small && lane == 0 && (int64_t)atomicAdd(img_small + img, (uint32_t)small) + small > 1 + (int64_t)c * hw / 65536)
-        *wide = 1u;
     if (bad)
         *wide = 1u;
 }
@@ -610,12 +603,12 @@ bool halo_geometry(int64_t h, int64_t w, int64_t kh, int64_t kw, int64_t pad, Ha
 
 } // namespace
 
-// NHWC float16 planes of x [batch][c][hw] under a scale per image; image_max: 2 * batch words of scratch.
+// NHWC float16 planes of x [batch][c][hw] under a scale per image; image_max: batch words of scratch.
 ct_status nhwc_half_planes(
     DeviceState *st, const float *x, int64_t batch, int64_t c, int64_t hw, int64_t c_pad, void *hi, void *lo, uint32_t *image_max,
     float *image_scale, uint32_t *wide) {
     (void)st;
-    CT_CUDA(cudaMemsetAsync(image_max, 0, (size_t)batch * 8, stream()));
+    CT_CUDA(cudaMemsetAsync(image_max, 0, (size_t)batch * 4, stream()));
     const int64_t count = c * hw;
     const int slices    = (int)(count / 16384 < 1 ? 1 : (count / 16384 > 64 ? 64 : count / 16384));
     const int vec       = (count & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
@@ -662,7 +655,7 @@ ct_status conv_halo(
     const int64_t taps     = kh * kw, hw = h * wd;
     const size_t w16       = align_up((size_t)ko * taps * c_pad * 2), w32 = align_up((size_t)ko * taps * c_pad * 4);
     const size_t x16       = align_up((size_t)batch * hw * c_pad * 2), x32 = align_up((size_t)batch * hw * c_pad * 4);
-    const size_t w_words   = align_up((size_t)ko * 4), x_words = align_up((size_t)batch * 8);
+    const size_t w_words   = align_up((size_t)ko * 4), x_words = align_up((size_t)batch * 4);
     if (batch > 65535 || c_pad / 32 > 65535)
         return fail(CT_ERR_TOO_LARGE, "conv2d: batch or channel count too large for the layout pre-pass");
     CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, w_words + 2 * x_words + 2 * w16 + 2 * w32 + 2 * x32));

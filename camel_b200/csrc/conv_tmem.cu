@@ -831,7 +831,6 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                 uint8_t *x_lo = x_hi + p.plane_bytes;
                 // a thread takes a position: 32 channels become the 64-byte row y * pw + x of both planes, 16-byte
                 // chunk j at j ^ ((row >> 1) & 3), the 64-byte swizzle
-                int small = 0; // values too small beside the tile's largest: one to a warp's share is let pass
                 for (int pos = ct; pos < npos; pos += 32 * kTH_CvtWarps) {
                     const int y = pos / p.pw, x = pos - y * p.pw;
                     const float *src = raw + y * p.box_w + x + p.off_x;
@@ -851,7 +850,7 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                                 hi[t] = __floats2half2_rn(a, b);
                                 lo[t] = __floats2half2_rn(__fmul_rn(__fsub_rn(a, __low2float(hi[t])), kHalfLoScale),
                                                           __fmul_rn(__fsub_rn(b, __high2float(hi[t])), kHalfLoScale));
-                                small += (a != 0.0f && fabsf(a) < kHalfSmallest) + (b != 0.0f && fabsf(b) < kHalfSmallest);
+                                bad |= (a != 0.0f && fabsf(a) < kHalfSmallest) || (b != 0.0f && fabsf(b) < kHalfSmallest);
                             }
                             const uint32_t at = row_off + (((uint32_t)(2 * half + j) ^ sw) << 4);
                             *reinterpret_cast<uint4 *>(x_hi + at) = *reinterpret_cast<uint4 *>(hi);
@@ -859,7 +858,6 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                         }
                     }
                 }
-                bad |= __reduce_add_sync(0xffffffffu, small) > 1;
                 // written through the generic proxy, read by the tensor core's asynchronous proxy
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
@@ -1174,7 +1172,7 @@ ct_status conv_tmem_filters(
         return CT_OK;
     }
     auto align_up        = [](size_t v) { return (v + 1023) & ~(size_t)1023; };
-    const size_t words   = align_up((size_t)batch * 8);
+    const size_t words   = align_up((size_t)batch * 4);
     const size_t plane32 = align_up((size_t)batch * h * wd * 32 * 4), plane16 = align_up((size_t)batch * h * wd * 32 * 2);
     if (batch > 65535)
         return fail(CT_ERR_TOO_LARGE, "conv2d: batch or channel count too large for the layout pre-pass");

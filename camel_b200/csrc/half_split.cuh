@@ -6,14 +6,11 @@
 // operand and per column of the right one (the row's largest magnitude is moved to [2^14, 2^15)) and by
 // storing the low term 2^11 times larger:
 //     v * 2^(14-e) = hi + lo * 2^-11,   hi = half(v * 2^(14-e)),   lo = half((v * 2^(14-e) - hi) * 2^11)
-// For |v| >= 2^-28 of its row's largest value that is v to 22 bits, exactly the 3xTF32 representation
-// (both terms convert to tf32 without rounding).  Below, hi becomes subnormal and the error stays at
-// 2^-36 of the scaled value: still 2^-17 relative at 2^-33 of the largest.  A matrix with a smaller
-// non-zero value than that, or a row whose exponent is beyond +-60, raises a device word, and the
-// product is then computed from tf32 planes instead (same launch sequence, no host involvement).
-// Convolution inputs, where hundreds of millions of ordinary values share few scales, let isolated ones
-// pass (one in 65536 of an image, one of a warp's share of a tile, one in 256 of a patch); their error is
-// 2^-51 of the largest value.
+// The pair holds a scaled value to an absolute error of 2^-36 at worst (lo's quantum is then 2^-24) and to 2^-23
+// of itself from 2^-13 up, which is what a pair of tf32 terms holds of any value; from 2^-12 up the two terms are the
+// same two 11-bit numbers whatever the scale (every bit of lo lies above float16's smallest).  A matrix with a
+// smaller non-zero value - 2^-27 of its row's largest or less - or a row whose exponent is beyond +-60 raises a
+// device word, and the product is then computed from tf32 planes instead (same launch sequence, no host involvement).
 #pragma once
 
 #include <cuda_fp16.h>
@@ -24,7 +21,7 @@ namespace ct {
 
 constexpr float kHalfLoScale    = 2048.0f;              // 2^11
 constexpr float kHalfLoInv      = 1.0f / 2048.0f;
-constexpr float kHalfSmallest   = 1.0f / (1u << 19);    // scaled magnitudes below this lose more than 2^-17
+constexpr float kHalfSmallest   = 1.0f / (1u << 13);    // scaled magnitudes below this may lose more than 2^-23
 constexpr int kHalfMaxExponent  = 60;
 
 // magnitude bits of a finite value, 0 for infinities and NaN (they are carried by hi alone)

@@ -69,7 +69,7 @@ typedef enum ct_activation {
 typedef enum ct_precision {
     CT_PREC_3XTF32 = 0, /* fp32 in, split into two terms of TF32's 11 significant bits, three MMAs, fp32
                          * accumulate.  The terms are float16 pairs under an exact power-of-two scale per
-                         * row and column; operands whose rows span more than 33 powers of two (or whose
+                         * row and column; operands whose rows span more than 26 powers of two (or whose
                          * exponent is beyond +-60) are computed from tf32 terms, decided on the device. */
     CT_PREC_BF16   = 1  /* inputs rounded to bf16 once, fp32 accumulate (reported separately) */
 } ct_precision;

@@ -2,8 +2,7 @@
 at the sizes where their tiling changes, and on operands that float16 pairs cannot hold, which have to
 take the tf32 planes instead; the few-column products at the edges of their row and k tiles.
 
-Bounds.  A value is carried to 2^-22 of itself (2^-17 for the few below 2^-28 of their row's largest), the
-product of two so carried to 2^-21, and the tensor core truncates once per addition into an accumulator
+Bounds.  A value is carried to 2^-23 of itself, the product of two so carried to 2^-21, and the tensor core truncates once per addition into an accumulator
 that takes at most 96 of them (tf32) or 64 (float16) before it is drained: 2^-24 each relative to the sum of
 magnitudes so far.  96 * 2^-24 + 2^-21 < 6.3e-6 of sum |a||b|.  Float64 sums are rounded once: 2^-24.
 """
@@ -147,6 +146,53 @@ def _conv64(x, w, stride, pad):
     xp = np.pad(x.astype(np.float64), ((0, 0), (0, 0), (pad, pad), (pad, pad)))
     win = np.lib.stride_tricks.sliding_window_view(xp, (kh, kw), (2, 3))[:, :, ::stride, ::stride]
     return np.einsum("nchwrs,kcrs->nkhw", win, w.astype(np.float64), optimize=True)
+
+
+# an output that depends on one product: both values to 2^-23, 2^-22 for the product of their low terms, which is left
+# out, three additions cut off at 2^-23 each, two roundings of the sums and scales
+SINGLE = 8 * 2.0**-23
+
+
+def _beside_large(rng, shape):
+    """Values from 2^-20 to 2^-60 of a largest one that is 2^16."""
+    return (rng.uniform(1, 2, shape) * np.exp2(rng.integers(-44, -4, shape)) * rng.choice([-1, 1], shape)).astype(np.float32)
+
+
+@pytest.mark.parametrize("size", [96, 288, 1100, 2300])
+@pytest.mark.parametrize("side", ["left", "right"])
+def test_small_values_keep_their_digits_beside_large_ones(T, size, side):
+    rng = np.random.default_rng(size)
+    a = _beside_large(rng, (size, size))
+    a[:, 0] = 2.0**16
+    b = np.diag(rng.uniform(1, 2, size)).astype(np.float32)
+    b[0, 0] = 0.0
+    got = _product(T, a, b) if side == "left" else _product(T, b, a.T.copy()).T
+    want = a.astype(np.float64) * np.diag(b).astype(np.float64)
+    assert np.all(np.abs(got - want) <= SINGLE * np.abs(want))
+
+
+# strided; halo; filters in tensor memory from the input itself, from planes, and with a tile of odd rows
+@pytest.mark.parametrize("shape", [(2, 48, 21, 23, 70, 3, 2, 1), (2, 64, 30, 28, 128, 3, 1, 1), (2, 32, 28, 28, 64, 3, 1, 1),
+                                   (2, 20, 26, 27, 40, 3, 1, 1), (2, 20, 16, 18, 40, 3, 1, 0)])
+@pytest.mark.parametrize("kind", ["input", "isolated", "filters"])
+def test_convolution_keeps_small_values_beside_large_ones(T, shape, kind):
+    n, c, h, wd, ko, kern, stride, pad = shape
+    rng = np.random.default_rng(sum(shape))
+    x, w = np.zeros((n, c, h, wd), np.float32), np.zeros((ko, c, kern, kern), np.float32)
+    x[:, 1, 1::5, 2::5] = rng.uniform(1, 2, x[:, 1, 1::5, 2::5].shape)
+    w[:, 1] = rng.uniform(1, 2, (ko, kern, kern))
+    if kind == "input":  # a channel of large values that meets zero weights
+        x[:, 1, 1::5, 2::5] = _beside_large(rng, x[:, 1, 1::5, 2::5].shape)
+        x[:, 0] = 2.0**16
+    elif kind == "isolated":  # one huge pixel beside one ordinary one
+        x[:] = 0
+        x[0, 0, 0, 0], x[0, 1, h - 2, wd - 2] = 1e16, 1.5
+    else:  # a large weight that meets a channel of zeros
+        w[:, 1], w[:, 0, 0, 0] = _beside_large(rng, (ko, kern, kern)), 2.0**16
+    want = _conv64(x, w, stride, pad)
+    got = T.conv2d(T.from_numpy(x), T.from_numpy(w), None, stride, pad).numpy()
+    T.check_async()
+    assert np.all(np.abs(got - want) <= SINGLE * np.abs(want))
 
 
 # (n, c, h, w, ko, kernel, stride, pad): patches in registers and read twice (k = 1200), odd sizes; halos with a
