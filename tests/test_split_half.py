@@ -153,16 +153,17 @@ def _conv64(x, w, stride, pad):
 SINGLE = 8 * 2.0**-23
 
 
-def _beside_large(rng, shape):
-    """Values from 2^-20 to 2^-60 of a largest one that is 2^16."""
-    return (rng.uniform(1, 2, shape) * np.exp2(rng.integers(-44, -4, shape)) * rng.choice([-1, 1], shape)).astype(np.float32)
+def _beside_large(rng, shape, lowest):
+    """Values from 2^(lowest - 16) to 2^-20 of a largest one that is 2^16."""
+    return (rng.uniform(1, 2, shape) * np.exp2(rng.integers(lowest, -4, shape)) * rng.choice([-1, 1], shape)).astype(np.float32)
 
 
 @pytest.mark.parametrize("size", [96, 288, 1100, 2300])
 @pytest.mark.parametrize("side", ["left", "right"])
-def test_small_values_keep_their_digits_beside_large_ones(T, size, side):
+@pytest.mark.parametrize("lowest", [-9, -16, -44])
+def test_small_values_keep_their_digits_beside_large_ones(T, size, side, lowest):
     rng = np.random.default_rng(size)
-    a = _beside_large(rng, (size, size))
+    a = _beside_large(rng, (size, size), lowest)
     a[:, 0] = 2.0**16
     b = np.diag(rng.uniform(1, 2, size)).astype(np.float32)
     b[0, 0] = 0.0
@@ -175,20 +176,21 @@ def test_small_values_keep_their_digits_beside_large_ones(T, size, side):
 @pytest.mark.parametrize("shape", [(2, 48, 21, 23, 70, 3, 2, 1), (2, 64, 30, 28, 128, 3, 1, 1), (2, 32, 28, 28, 64, 3, 1, 1),
                                    (2, 20, 26, 27, 40, 3, 1, 1), (2, 20, 16, 18, 40, 3, 1, 0)])
 @pytest.mark.parametrize("kind", ["input", "isolated", "filters"])
-def test_convolution_keeps_small_values_beside_large_ones(T, shape, kind):
+@pytest.mark.parametrize("lowest", [-9, -16, -44])
+def test_convolution_keeps_small_values_beside_large_ones(T, shape, kind, lowest):
     n, c, h, wd, ko, kern, stride, pad = shape
     rng = np.random.default_rng(sum(shape))
     x, w = np.zeros((n, c, h, wd), np.float32), np.zeros((ko, c, kern, kern), np.float32)
     x[:, 1, 1::5, 2::5] = rng.uniform(1, 2, x[:, 1, 1::5, 2::5].shape)
     w[:, 1] = rng.uniform(1, 2, (ko, kern, kern))
     if kind == "input":  # a channel of large values that meets zero weights
-        x[:, 1, 1::5, 2::5] = _beside_large(rng, x[:, 1, 1::5, 2::5].shape)
+        x[:, 1, 1::5, 2::5] = _beside_large(rng, x[:, 1, 1::5, 2::5].shape, lowest)
         x[:, 0] = 2.0**16
     elif kind == "isolated":  # one huge pixel beside one ordinary one
         x[:] = 0
         x[0, 0, 0, 0], x[0, 1, h - 2, wd - 2] = 1e16, 1.5
     else:  # a large weight that meets a channel of zeros
-        w[:, 1], w[:, 0, 0, 0] = _beside_large(rng, (ko, kern, kern)), 2.0**16
+        w[:, 1], w[:, 0, 0, 0] = _beside_large(rng, (ko, kern, kern), lowest), 2.0**16
     want = _conv64(x, w, stride, pad)
     got = T.conv2d(T.from_numpy(x), T.from_numpy(w), None, stride, pad).numpy()
     T.check_async()
