@@ -15,9 +15,9 @@
 // Arithmetic: split float16 (half_split.cuh), scaled per filter and per image - a scale has to be constant
 // along k, and an output's patch crosses the whole halo - with the cross products in an accumulator of their
 // own, as in gemm_half.cu.  A 64-byte row then holds 32 channels, so the layer takes half the MMAs, half the
-// filter stages and half the plane traffic of the tf32 form.  Where an image or a filter spans too many powers
-// of two, the pre-pass raises a device word, wide_nhwc_kernel writes tf32 planes and this kernel runs the same
-// loop over those (16 channels per row).
+// filter stages and half the plane traffic of the tf32 form.  An image that spans too many powers of two - or
+// every image, where a filter does - has tf32 planes in the same place, and this kernel runs the same loop over
+// those for its tiles (16 channels per row); the other images of the batch are not touched by it.
 //
 // One CTA per SM walks the tiles.  Both accumulators (512 columns) belong to one tile; the epilogue reads the
 // cross products first, which the next tile starts with, so the tensor pipe waits for about the drain of
@@ -77,9 +77,8 @@ struct ConvHaloParams {
     int kh, kw, pad;
     int ho, wo, pw;   // pw = w + 2 pad
     int th, tiles_y;
-    const uint32_t *wide;      // non-zero: the planes are tf32
     const float *filter_scale; // [ko] inverse scales
-    const float *image_scale;  // [batch]
+    const float *image_scale;  // [batch]; 0: this image's planes are tf32
     int c_pad;        // channels of the planes (k offset of a tap in the filter planes: tap * c_pad)
     int n_mma;        // th * pw rounded up to 16
     int box_bytes;    // one plane's halo box
@@ -150,9 +149,6 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
     const int taps           = p.kh * p.kw;
-    const bool wide          = *reinterpret_cast<const volatile uint32_t *>(p.wide) != 0;
-    const int block_k        = wide ? 16 : 32; // channels per k-block
-    const int cblocks        = p.c_pad / block_k;
 
     // tile -> (row tile of output channels, tile row, image): neighbouring CTAs take the row tiles
     // of one pixel tile, so they read the same halo out of L2
@@ -166,13 +162,15 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
     if (warp == 0) {
         // ===== TMA producer =====
         if (lane == 0) {
-            const CUtensorMap *mw_hi = wide ? &maps.w32_hi : &maps.w16_hi, *mw_lo = wide ? &maps.w32_lo : &maps.w16_lo;
-            const CUtensorMap *mx_hi = wide ? &maps.x32_hi : &maps.x16_hi, *mx_lo = wide ? &maps.x32_lo : &maps.x16_lo;
             int ka = 0, kh2 = 0; // filter k-blocks and halos issued so far
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
                 int tm, ty, img;
                 coords(tile, tm, ty, img);
+                const bool wide          = __ldg(p.image_scale + img) == 0.0f;
+                const CUtensorMap *mw_hi = wide ? &maps.w32_hi : &maps.w16_hi, *mw_lo = wide ? &maps.w32_lo : &maps.w16_lo;
+                const CUtensorMap *mx_hi = wide ? &maps.x32_hi : &maps.x16_hi, *mx_lo = wide ? &maps.x32_lo : &maps.x16_lo;
+                const int block_k = wide ? 16 : 32, cblocks = p.c_pad / block_k; // channels per k-block
                 for (int cb = 0; cb < cblocks && ok; ++cb, ++kh2) {
                     const int hs = kh2 % kH_HaloStages;
                     if (!mbar_wait(smem_u32(&bar_h_empty[hs]), ((uint32_t)(kh2 / kH_HaloStages) & 1u) ^ 1u, abort_flag)) {
@@ -219,14 +217,18 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
     } else if (warp == 1) {
         // ===== MMA issuer =====
         if (lane == 0) {
-            const uint32_t idesc = make_idesc(wide ? 2u : 0u, 128, (uint32_t)p.n_mma);
-            int ka = 0, kh2 = 0, i = 0;
+            int ka = 0, kh2 = 0, i = 0, crosses = 0; // tiles so far, and those of them with cross products
             bool ok = true;
             const long long t_start = CH_CLOCK();
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++i) {
+                int tm, ty, img;
+                coords(tile, tm, ty, img);
+                const bool wide      = __ldg(p.image_scale + img) == 0.0f; // looked up while the MMAs of the last tile run
+                const uint32_t idesc = make_idesc(wide ? 2u : 0u, 128, (uint32_t)p.n_mma);
+                const int cblocks    = p.c_pad / (wide ? 16 : 32);
                 // the accumulators of the previous tile have been read
                 auto wait_empty = [&](int acc) {
-                    const bool got = mbar_wait(smem_u32(&bar_tmem_empty[acc]), ((uint32_t)i & 1u) ^ 1u, abort_flag);
+                    const bool got = mbar_wait(smem_u32(&bar_tmem_empty[acc]), ((uint32_t)(acc ? crosses : i) & 1u) ^ 1u, abort_flag);
                     tc_fence_after_sync();
                     return got;
                 };
@@ -293,8 +295,10 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                         tc_commit(smem_u32(&bar_h_empty[hs])); // the halo is free once its taps' MMAs have retired
                 }
                 if (ok) {
-                    if (!wide)
+                    if (!wide) {
                         tc_commit(smem_u32(&bar_tmem_full[1]));
+                        ++crosses;
+                    }
                     tc_commit(smem_u32(&bar_tmem_full[0]));
                 }
             }
@@ -327,18 +331,20 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                 off[h2][q] = (col < npos && x < p.wo) ? y * p.wo + x : -1;
             }
         const int col_base = half * 128 + sub * 4;
-        int i = 0;
+        int i = 0, crosses = 0;
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
             int tm, ty, img;
             coords(tile, tm, ty, img);
             const int row0     = tm * 128 + quarter * 32; // first output channel of this warp's block
+            const float inv    = p.image_scale[img];
+            const bool wide    = inv == 0.0f;
             const float rs     = (!wide && row0 + lane < p.ko) ? p.filter_scale[row0 + lane] : 1.0f;
-            const float is     = wide ? 1.0f : p.image_scale[img];
+            const float is     = wide ? 1.0f : inv;
             const long long e0 = CH_CLOCK();
             float acc[128];
             const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 128);
             auto await = [&](int which) {
-                const bool got = mbar_wait(smem_u32(&bar_tmem_full[which]), (uint32_t)i & 1u, abort_flag);
+                const bool got = mbar_wait(smem_u32(&bar_tmem_full[which]), (uint32_t)(which ? crosses++ : i) & 1u, abort_flag);
                 tc_fence_after_sync();
                 return __all_sync(0xffffffffu, got) != 0;
             };
@@ -433,51 +439,80 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 512);
     }
-    if (threadIdx.x == 0) {
-        if (*abort_flag)
-            atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
-        // the last CTA clears the pre-pass's word for the next product
-        if (atomicAdd(p.flags + FLAG_WIDE_READERS, 1u) + 1u == gridDim.x) {
-            p.flags[FLAG_WIDE_READERS] = 0u;
-            p.flags[FLAG_WIDE]         = 0u;
-        }
-    }
+    if (threadIdx.x == 0 && *abort_flag)
+        atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
 }
 
 // ---- pre-pass -----------------------------------------------------------------------------
+//
+// Two launches: the range of every image, in slices, next to the filters (both forms of their planes, a block per
+// filter); then the input as NHWC planes, in the form that the image's range allows.
 
-// Largest magnitude of each image ([batch][count] floats), as bits, by atomic maximum into img_max (zeroed).  An
-// infinity or NaN counts as what it is: half_scale refuses it and the layer takes the tf32 planes.
-__global__ void __launch_bounds__(256) image_max_kernel(
-    const float *__restrict__ x, int64_t count, int slices, int vec_ok, uint32_t *__restrict__ img_max) {
-    const int64_t img = blockIdx.x / slices;
-    const int slice   = blockIdx.x - (int)img * slices;
-    const float *src  = x + img * count;
-    uint32_t mx       = 0;
-    if (vec_ok) {
+// Blocks 0 .. ko - 1: filter [c][taps] -> planes [taps * c_pad], tap-major k (none if hi16 is null), and its inverse
+// scale, 0 where the range of the filter does not fit float16 pairs.  The others: slice (blockIdx.x - ko) of the images
+// ([batch][count] floats, `slices` to an image).
+struct FilterPlanes {
+    __half *hi16, *lo16;
+    float *hi32, *lo32;
+    float *scale;
+};
+__global__ void __launch_bounds__(256) conv_range_kernel(
+    const float *__restrict__ w, int c, int taps, int c_pad, int ko, const FilterPlanes f, const float *__restrict__ x,
+    int64_t count, int slices, int vec_ok, uint2 *__restrict__ ranges) {
+    __shared__ uint2 part[8];
+    const bool filter = (int64_t)blockIdx.x < ko;
+    const int64_t o   = filter ? blockIdx.x : (blockIdx.x - ko) / slices;
+    const int slice   = filter ? 0 : (int)(blockIdx.x - ko - o * slices);
+    const float *src  = filter ? w + o * c * taps : x + o * count;
+    const int64_t n   = filter ? (int64_t)c * taps : count;
+    const int64_t step = filter ? 256 : (int64_t)slices * 256;
+    uint2 r            = make_uint2(0u, kNoneSmallest);
+    if (!filter && vec_ok) {
         const float4 *s4 = reinterpret_cast<const float4 *>(src);
 #pragma unroll 8
-        for (int64_t i = (int64_t)slice * 256 + threadIdx.x; i < count / 4; i += (int64_t)slices * 256) {
+        for (int64_t i = (int64_t)slice * 256 + threadIdx.x; i < n / 4; i += step) {
             const float4 q = s4[i];
-            mx = max(max(mx, max(__float_as_uint(q.x) & 0x7fffffffu, __float_as_uint(q.y) & 0x7fffffffu)),
-                     max(__float_as_uint(q.z) & 0x7fffffffu, __float_as_uint(q.w) & 0x7fffffffu));
+            range_take(r, q.x), range_take(r, q.y), range_take(r, q.z), range_take(r, q.w);
         }
     } else {
 #pragma unroll 8
-        for (int64_t i = (int64_t)slice * 256 + threadIdx.x; i < count; i += (int64_t)slices * 256)
-            mx = max(mx, __float_as_uint(src[i]) & 0x7fffffffu);
+        for (int64_t i = (int64_t)slice * 256 + threadIdx.x; i < n; i += step)
+            range_take(r, src[i]);
     }
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if ((threadIdx.x & 31) == 0 && mx)
-        atomicMax(img_max + img, mx);
+    r = range_warp(r);
+    if ((threadIdx.x & 31) == 0)
+        part[threadIdx.x >> 5] = r;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        r = range_join(r, part[j]);
+    if (!filter) {
+        if (threadIdx.x == 0)
+            ranges[o * slices + slice] = r;
+        return;
+    }
+    float scale, inverse;
+    const bool fits = half_range_fits(r, scale, inverse);
+    if (threadIdx.x == 0)
+        f.scale[o] = fits ? inverse : 0.0f;
+    if (f.hi16 == nullptr)
+        return;
+    for (int i = threadIdx.x; i < taps * c_pad; i += 256) {
+        const int tap = i / c_pad, ic = i - tap * c_pad;
+        const float v    = ic < c ? src[ic * taps + tap] : 0.0f;
+        const int64_t at = o * taps * c_pad + i;
+        split_half(v * scale, f.hi16[at], f.lo16[at]);
+        split_tf32(v, f.hi32[at], f.lo32[at]);
+    }
 }
 
-// x [batch][c][hw] -> NHWC float16 planes [batch][hw][c_pad] under the image's scale.  A block takes 64
-// channels by 64 positions through shared memory: reads of 256 contiguous bytes, writes of 128.  The images are
-// taken last to first: the end of the tensor is what image_max_kernel has just left in L2.
-__global__ void __launch_bounds__(256) nhwc_half_kernel(
-    const float *__restrict__ x, int c, int64_t hw, int c_pad, const uint32_t *img_max, __half *__restrict__ p_hi,
-    __half *__restrict__ p_lo, float *__restrict__ image_scale, uint32_t *__restrict__ wide) {
+// x [batch][c][hw] -> NHWC planes [hw][c_pad], hi then lo, in the image's slot of 8 bytes per value: float16 pairs
+// under the image's scale, or tf32 terms (image_scale 0) where the image or any filter does not fit those.  A
+// block takes 64 channels by 64 positions through shared memory: reads of 256 contiguous bytes, writes of 128.  The
+// images are taken last to first: the end of the tensor is what conv_range_kernel has just left in L2.
+__global__ void __launch_bounds__(256) conv_planes_kernel(
+    const float *__restrict__ x, int c, int64_t hw, int c_pad, const uint2 *__restrict__ ranges, int slices,
+    const float *__restrict__ filter_scale, int ko, uint8_t *__restrict__ slots, float *__restrict__ image_scale) {
     __shared__ float tile[64][65];
     const int64_t img = gridDim.z - 1 - blockIdx.z;
     const int64_t q0  = (int64_t)blockIdx.x * 64;
@@ -491,87 +526,44 @@ __global__ void __launch_bounds__(256) nhwc_half_kernel(
             const int ch = warp + 8 * j, q = lane + 32 * t;
             tile[ch][q]  = (c0 + ch < c && q0 + q < hw) ? __ldcs(src + ch * hw + q) : 0.0f;
         }
+    uint2 r = make_uint2(0u, kNoneSmallest);
+    for (int s = lane; s < slices; s += 32)
+        r = range_join(r, ranges[img * slices + s]);
+    int bad_filter = 0;
+    for (int o = threadIdx.x; o < ko; o += 256)
+        bad_filter |= filter_scale[o] == 0.0f ? 1 : 0;
     float scale, inverse;
-    bool bad = !half_scale(img_max[img], scale, inverse);
+    const bool fits = half_range_fits(range_warp(r), scale, inverse) & !__syncthreads_or(bad_filter);
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
-        image_scale[img] = inverse;
-    __syncthreads();
+        image_scale[img] = fits ? inverse : 0.0f;
+    const int64_t plane = hw * c_pad;
+    uint8_t *slot       = slots + img * plane * 8;
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
         const int chunk = threadIdx.x & 7, q = (threadIdx.x >> 3) + 32 * t;
-        if (q0 + q < hw && c0 + chunk * 8 < c_pad) {
+        if (q0 + q >= hw || c0 + chunk * 8 >= c_pad)
+            continue;
+        const int64_t at = (q0 + q) * c_pad + c0 + chunk * 8;
+        if (fits) {
             __half hi[8], lo[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-                bad |= split_half(tile[chunk * 8 + j][q] * scale, hi[j], lo[j]);
-            const int64_t at = (img * hw + q0 + q) * c_pad + c0 + chunk * 8;
-            *reinterpret_cast<uint4 *>(p_hi + at) = *reinterpret_cast<uint4 *>(hi);
-            *reinterpret_cast<uint4 *>(p_lo + at) = *reinterpret_cast<uint4 *>(lo);
-        }
-    }
-    if (bad)
-        *wide = 1u;
-}
-
-// Filters [ko][c][taps] -> planes [ko][taps * c_pad], tap-major k, both forms; a block per filter.
-__global__ void __launch_bounds__(256) filter_planes_kernel(
-    const float *__restrict__ w, int c, int taps, int c_pad, __half *__restrict__ hi16, __half *__restrict__ lo16,
-    float *__restrict__ hi32, float *__restrict__ lo32, float *__restrict__ filter_scale, uint32_t *__restrict__ wide) {
-    __shared__ uint32_t max_s[8];
-    const int64_t o  = blockIdx.x;
-    const float *src = w + o * c * taps;
-    uint32_t mx      = 0;
-    for (int i = threadIdx.x; i < c * taps; i += 256)
-        mx = max(mx, finite_magnitude(src[i]));
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if ((threadIdx.x & 31) == 0)
-        max_s[threadIdx.x >> 5] = mx;
-    __syncthreads();
+                split_half(tile[chunk * 8 + j][q] * scale, hi[j], lo[j]);
+            __half *p_hi = reinterpret_cast<__half *>(slot) + at;
+            *reinterpret_cast<uint4 *>(p_hi)         = *reinterpret_cast<uint4 *>(hi);
+            *reinterpret_cast<uint4 *>(p_hi + plane) = *reinterpret_cast<uint4 *>(lo);
+        } else {
+            float *p_hi = reinterpret_cast<float *>(slot) + at;
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-        mx = max(mx, max_s[j]);
-    float scale, inverse;
-    bool bad = !half_scale(mx, scale, inverse);
-    if (threadIdx.x == 0)
-        filter_scale[o] = inverse;
-    for (int i = threadIdx.x; i < taps * c_pad; i += 256) {
-        const int tap = i / c_pad, ic = i - tap * c_pad;
-        const float v    = ic < c ? src[ic * taps + tap] : 0.0f;
-        const int64_t at = o * taps * c_pad + i;
-        bad |= split_half(v * scale, hi16[at], lo16[at]);
-        split_tf32(v, hi32[at], lo32[at]);
-    }
-    if (bad)
-        *wide = 1u;
-}
-
-// The tf32 NHWC planes, where the word says that they are needed; returns at once otherwise.
-__global__ void __launch_bounds__(256) wide_nhwc_kernel(
-    const uint32_t *__restrict__ wide, const float *__restrict__ x, int64_t batch, int c, int64_t hw, int c_pad,
-    float *__restrict__ hi, float *__restrict__ lo) {
-    __shared__ float tile[32][33];
-    if (*reinterpret_cast<const volatile uint32_t *>(wide) == 0)
-        return;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t tiles_q = (hw + 31) / 32, tiles_c = c_pad / 32;
-    for (int64_t t = blockIdx.x; t < batch * tiles_q * tiles_c; t += gridDim.x) {
-        const int64_t img = t / (tiles_q * tiles_c), rest = t - img * tiles_q * tiles_c;
-        const int64_t q0 = rest / tiles_c * 32, c0 = rest % tiles_c * 32;
+            for (int j = 0; j < 8; j += 4) {
+                float hi[4], lo[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int64_t ch = c0 + ty + 8 * j, q = q0 + tx;
-            tile[ty + 8 * j][tx] = (ch < c && q < hw) ? x[(img * c + ch) * hw + q] : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int64_t q = q0 + ty + 8 * j;
-            if (q < hw) {
-                const int64_t at = (img * hw + q) * c_pad + c0 + tx;
-                split_tf32(tile[tx][ty + 8 * j], hi[at], lo[at]);
+                for (int u = 0; u < 4; ++u)
+                    split_tf32_flat(tile[chunk * 8 + j + u][q], hi[u], lo[u]);
+                *reinterpret_cast<float4 *>(p_hi + j)         = make_float4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<float4 *>(p_hi + plane + j) = make_float4(lo[0], lo[1], lo[2], lo[3]);
             }
         }
-        __syncthreads();
     }
 }
 
@@ -603,30 +595,34 @@ bool halo_geometry(int64_t h, int64_t w, int64_t kh, int64_t kw, int64_t pad, Ha
 
 } // namespace
 
-// NHWC float16 planes of x [batch][c][hw] under a scale per image; image_max: batch words of scratch.
-ct_status nhwc_half_planes(
-    DeviceState *st, const float *x, int64_t batch, int64_t c, int64_t hw, int64_t c_pad, void *hi, void *lo, uint32_t *image_max,
-    float *image_scale, uint32_t *wide) {
-    (void)st;
-    CT_CUDA(cudaMemsetAsync(image_max, 0, (size_t)batch * 4, stream()));
-    const int64_t count = c * hw;
-    const int slices    = (int)(count / 16384 < 1 ? 1 : (count / 16384 > 64 ? 64 : count / 16384));
-    const int vec       = (count & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-    image_max_kernel<<<(unsigned)(batch * slices), 256, 0, stream()>>>(x, count, slices, vec, image_max);
-    CT_LAUNCH_CHECK("image_max");
-    const dim3 grid((unsigned)((hw + 63) / 64), (unsigned)((c_pad + 63) / 64), (unsigned)batch);
-    nhwc_half_kernel<<<grid, 256, 0, stream()>>>(x, (int)c, hw, (int)c_pad, image_max, static_cast<__half *>(hi),
-                                                 static_cast<__half *>(lo), image_scale, wide);
-    CT_LAUNCH_CHECK("nhwc_half");
-    return CT_OK;
+// Slices of an image in conv_range_kernel.
+int conv_range_slices(int64_t count) {
+    return (int)(count / 4096 < 1 ? 1 : (count / 4096 > 64 ? 64 : count / 4096));
 }
 
-// The tf32 planes instead, where *wide says so.
-ct_status nhwc_wide_planes(
-    DeviceState *st, const uint32_t *wide, const float *x, int64_t batch, int64_t c, int64_t hw, int64_t c_pad, void *hi, void *lo) {
-    wide_nhwc_kernel<<<(unsigned)st->sm_count * 2, 256, 0, stream()>>>(wide, x, batch, (int)c, hw, (int)c_pad,
-                                                                       static_cast<float *>(hi), static_cast<float *>(lo));
-    CT_LAUNCH_CHECK("wide_nhwc");
+// The pre-pass of a layer: the filters' scales and (filters16 non-null) planes, the images' planes and scales.
+// ranges: batch * conv_range_slices(c * hw) pairs of words.
+ct_status conv_prepass(
+    DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t hw, int64_t c_pad, int64_t ko, int64_t taps,
+    void *filters16, void *filters32, size_t plane16, size_t plane32, float *filter_scale, void *ranges, float *image_scale,
+    void *slots) {
+    (void)st;
+    if (batch > 65535 || c_pad / 32 > 65535)
+        return fail(CT_ERR_TOO_LARGE, "conv2d: batch or channel count too large for the layout pre-pass");
+    const int64_t count = c * hw;
+    const int slices    = conv_range_slices(count);
+    const int vec       = (count & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    uint8_t *f16 = static_cast<uint8_t *>(filters16), *f32 = static_cast<uint8_t *>(filters32);
+    const FilterPlanes f{reinterpret_cast<__half *>(f16), reinterpret_cast<__half *>(f16 + plane16), reinterpret_cast<float *>(f32),
+                         reinterpret_cast<float *>(f32 + plane32), filter_scale};
+    ProfScope prof("conv_prepass");
+    conv_range_kernel<<<(unsigned)(ko + batch * slices), 256, 0, stream()>>>(
+        w, (int)c, (int)taps, (int)c_pad, (int)ko, f, x, count, slices, vec, static_cast<uint2 *>(ranges));
+    CT_LAUNCH_CHECK("conv_range");
+    const dim3 grid((unsigned)((hw + 63) / 64), (unsigned)((c_pad + 63) / 64), (unsigned)batch);
+    conv_planes_kernel<<<grid, 256, 0, stream()>>>(x, (int)c, hw, (int)c_pad, static_cast<uint2 *>(ranges), slices, filter_scale, (int)ko,
+                                                   static_cast<uint8_t *>(slots), image_scale);
+    CT_LAUNCH_CHECK("conv_planes");
     return CT_OK;
 }
 
@@ -643,8 +639,8 @@ bool conv_halo_applicable(int64_t c_pad, int64_t h, int64_t w, int64_t ko, int64
     return (int64_t)g.th * g.wo * 10 >= (int64_t)g.n_mma * 7; // at least 70 % of the columns carry an output
 }
 
-// Workspace: [filter scale][image scale][image max][w hi16][w lo16][w hi][w lo][x planes]; the x planes are
-// float16 pairs or, where they do not fit those, tf32 in the same place: no more than tf32 planes alone take.
+// Workspace: [filter scale][image scale][image ranges][w hi16][w lo16][w hi][w lo][image slots]; a slot holds an
+// image's planes, float16 pairs or, where it does not fit those, tf32: no more than tf32 planes alone take.
 ct_status conv_halo(
     DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t c_pad, int64_t h, int64_t wd, int64_t ko,
     int64_t kh, int64_t kw, int64_t pad, const float *bias, int act, float *out) {
@@ -654,27 +650,17 @@ ct_status conv_halo(
     auto align_up          = [](size_t v) { return (v + 1023) & ~(size_t)1023; };
     const int64_t taps     = kh * kw, hw = h * wd;
     const size_t w16       = align_up((size_t)ko * taps * c_pad * 2), w32 = align_up((size_t)ko * taps * c_pad * 4);
-    const size_t x16       = align_up((size_t)batch * hw * c_pad * 2), x32 = align_up((size_t)batch * hw * c_pad * 4);
+    const size_t slot      = (size_t)hw * c_pad * 8;
     const size_t w_words   = align_up((size_t)ko * 4), x_words = align_up((size_t)batch * 4);
-    if (batch > 65535 || c_pad / 32 > 65535)
-        return fail(CT_ERR_TOO_LARGE, "conv2d: batch or channel count too large for the layout pre-pass");
-    CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, w_words + 2 * x_words + 2 * w16 + 2 * w32 + 2 * x32));
+    const size_t ranges    = align_up((size_t)batch * conv_range_slices(c * hw) * 8);
+    CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, w_words + x_words + ranges + 2 * w16 + 2 * w32 + (size_t)batch * slot));
     uint8_t *ws            = static_cast<uint8_t *>(st->gemm_ws);
     float *filter_scale    = reinterpret_cast<float *>(ws), *image_scale = reinterpret_cast<float *>(ws + w_words);
-    uint32_t *image_max    = reinterpret_cast<uint32_t *>(ws + w_words + x_words);
-    uint8_t *w16_hi        = ws + w_words + 2 * x_words, *w32_hi = w16_hi + 2 * w16, *xp = w32_hi + 2 * w32;
-    uint32_t *wide         = st->flags_dev + FLAG_WIDE;
-    {
-        ProfScope prof("conv_prepass");
-        filter_planes_kernel<<<(unsigned)ko, 256, 0, stream()>>>(
-            w, (int)c, (int)taps, (int)c_pad, reinterpret_cast<__half *>(w16_hi), reinterpret_cast<__half *>(w16_hi + w16),
-            reinterpret_cast<float *>(w32_hi), reinterpret_cast<float *>(w32_hi + w32), filter_scale, wide);
-        CT_LAUNCH_CHECK("filter_planes");
-        CT_TRY(nhwc_half_planes(st, x, batch, c, hw, c_pad, xp, xp + x16, image_max, image_scale, wide));
-        CT_TRY(nhwc_wide_planes(st, wide, x, batch, c, hw, c_pad, xp, xp + x32));
-    }
+    uint8_t *w16_hi        = ws + w_words + x_words + ranges, *w32_hi = w16_hi + 2 * w16, *xp = w32_hi + 2 * w32;
+    CT_TRY(conv_prepass(st, x, w, batch, c, hw, c_pad, ko, taps, w16_hi, w32_hi, w16, w32, filter_scale, ws + w_words + x_words,
+                        image_scale, xp));
     ConvHaloParams p;
-    p.wide = wide, p.filter_scale = filter_scale, p.image_scale = image_scale;
+    p.filter_scale = filter_scale, p.image_scale = image_scale;
     p.bias = bias, p.out = out, p.flags = st->flags_dev;
     p.ko = (int)ko, p.tiles_m = (int)((ko + 127) / 128);
     p.kh = (int)kh, p.kw = (int)kw, p.pad = (int)pad;
@@ -694,16 +680,16 @@ ct_status conv_halo(
         const uint64_t wdims[2] = {kp, (uint64_t)ko}, wstr[1] = {kp * (uint64_t)elem};
         const uint32_t wbox[2]  = {(uint32_t)(kH_RowB / elem), 128};
         const uint64_t xdims[4] = {(uint64_t)c_pad, (uint64_t)wd, (uint64_t)h, (uint64_t)batch};
-        const uint64_t xstr[3]  = {row, row * (uint64_t)wd, row * (uint64_t)wd * (uint64_t)h};
+        const uint64_t xstr[3]  = {row, row * (uint64_t)wd, slot};
         const uint32_t xbox[4]  = {(uint32_t)(kH_RowB / elem), (uint32_t)g.pw, (uint32_t)g.box_rows, 1};
         auto fn = elem == 4 ? encode_tiled_map_f32 : encode_tiled_map_f16;
         CT_TRY(fn(mw, wp, 2, wdims, wstr, wbox, kH_RowB));
         return fn(mx, xpl, 4, xdims, xstr, xbox, kH_RowB);
     };
     CT_TRY(encode(&maps.w16_hi, w16_hi, &maps.x16_hi, xp, 2));
-    CT_TRY(encode(&maps.w16_lo, w16_hi + w16, &maps.x16_lo, xp + x16, 2));
+    CT_TRY(encode(&maps.w16_lo, w16_hi + w16, &maps.x16_lo, xp + slot / 4, 2));
     CT_TRY(encode(&maps.w32_hi, w32_hi, &maps.x32_hi, xp, 4));
-    CT_TRY(encode(&maps.w32_lo, w32_hi + w32, &maps.x32_lo, xp + x32, 4));
+    CT_TRY(encode(&maps.w32_lo, w32_hi + w32, &maps.x32_lo, xp + slot / 2, 4));
     // the kernel also has a little static shared memory (barriers, the bias): ask for exactly what
     // this geometry needs, remembering the largest request per device
     static size_t attr_bytes_dev[16] = {};

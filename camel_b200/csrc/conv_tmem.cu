@@ -38,6 +38,8 @@
 #include "split.cuh"
 #include "tmap.cuh"
 
+#include <algorithm>
+
 // Optional per-CTA clock accounting for tuning; compiled in only with -DCT_CONV_TRACE.
 #ifdef CT_CONV_TRACE
 __device__ unsigned long long g_conv_trace[256 * 16];
@@ -91,7 +93,9 @@ struct ConvTmemParams {
     int plane_bytes;  // shared-memory bytes reserved per plane (box plus the rows shifted reads run into)
     int stages;
     int act, pool;
-    const uint32_t *only_if; // non-null: the launch does nothing unless this word is set
+    const float *image_scale; // planes: [batch] inverse scales, 0 for an image that needs tf32 terms
+    uint2 *tile_range;        // raw: [total tiles] range of the values of each tile, and one entry whose .x says that
+                              // the filters need tf32 terms
     // raw mode (the input is read as it is, NCHW float32, and split into planes inside the kernel)
     int box_w;        // floats per row of the raw box (a multiple of four)
     int off_x;        // the tile's first position (x = -pad) sits this many floats into a raw row
@@ -99,6 +103,40 @@ struct ConvTmemParams {
     int raw_bytes;    // bytes of one raw box: 32 channels x box_rows x box_w floats
     int raw_stride;   // shared-memory bytes reserved per raw stage
 };
+
+// Whether image `img` is left to the tf32 form: its values, over all its tiles (every pixel is in one of them), or the
+// filters do not fit float16 pairs.  A property of the image alone, so that its bits do not depend on how the launch
+// was cut into tiles (the fused pool takes rows by twos), on what else is in the batch, or on how it was read.
+template <bool RAW> __device__ __forceinline__ bool image_needs_tf32(const ConvTmemParams &p, int img, int total_tiles) {
+    if (!RAW)
+        return __ldg(p.image_scale + img) == 0.0f;
+    const uint32_t filters = p.tile_range[total_tiles].x;
+    const uint2 *src       = p.tile_range + (int64_t)img * p.tiles_y;
+    uint2 range            = make_uint2(0u, kNoneSmallest);
+    for (int t = 0; t < p.tiles_y; t += 8) {
+        uint2 r[8]; // eight loads in flight: one after the other they cost an idle launch 4 us
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            r[j] = src[min(t + j, p.tiles_y - 1)];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            range = range_join(range, r[j]);
+    }
+    float scale, inverse;
+    return filters != 0u || !half_range_fits(range, scale, inverse);
+}
+
+// Tiles of a block of the tf32 form, a bit each: at most kTA_MaxOwn to a block (the grid grows beyond that).
+constexpr int kTA_MaxOwn = 4096;
+__device__ __forceinline__ int next_own(const uint32_t *mask, int q, int own) {
+    while (q < own) {
+        const uint32_t bits = mask[q >> 5] >> (q & 31);
+        if (bits)
+            return q + __ffs(bits) - 1;
+        q = (q | 31) + 1;
+    }
+    return own;
+}
 
 __device__ __forceinline__ void tmem_st_32x32_x8(uint32_t taddr, const uint32_t (&r)[8]) {
     asm volatile(
@@ -144,19 +182,28 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
     __shared__ uint64_t bar_done;
     __shared__ uint64_t bar_epi; // the four epilogue warps meet here (bounded, unlike bar.sync)
     __shared__ uint32_t tmem_base_slot;
-    __shared__ int abort_flag_s, idle_s;
+    __shared__ int abort_flag_s;
+    __shared__ uint32_t own_mask[kTA_MaxOwn / 32];
     volatile int *abort_flag = &abort_flag_s;
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    if (threadIdx.x == 0) {
-        abort_flag_s = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
-        idle_s       = *reinterpret_cast<const volatile uint32_t *>(p.only_if) == 0 ? 1 : 0;
+    // this block's tiles, blockIdx.x + q gridDim.x, whose images the float16 form leaves to this one
+    const int own = (total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
+    int any       = 0;
+    for (int q0 = warp * 32; q0 < own; q0 += (int)blockDim.x) {
+        const int q         = q0 + lane;
+        const bool mine     = q < own && image_needs_tf32<RAW>(p, ((int)blockIdx.x + q * (int)gridDim.x) / p.tiles_y, total_tiles);
+        const uint32_t bits = __ballot_sync(0xffffffffu, mine);
+        any |= bits != 0u;
+        if (lane == 0)
+            own_mask[q0 >> 5] = bits;
     }
-    __syncthreads();
-    if (abort_flag_s || idle_s)
-        return; // nothing raised the word: conv_tmem_half_kernel has computed the layer
+    if (threadIdx.x == 0)
+        abort_flag_s = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
+    if (!__syncthreads_or(any) || abort_flag_s)
+        return; // conv_tmem_half_kernel has computed them all
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t stage_bytes = 2u * (uint32_t)p.plane_bytes;
@@ -224,7 +271,8 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
             int i = 0;
             bool ok = true;
             const int nstages = RAW ? kTA_RawStages : p.stages;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++i) {
+            for (int q = next_own(own_mask, 0, own); q < own && ok; q = next_own(own_mask, q + 1, own), ++i) {
+                const int tile = (int)blockIdx.x + q * (int)gridDim.x;
                 const int img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
                 const int s       = i % nstages;
                 const uint32_t ph = (uint32_t)(i / nstages) & 1u;
@@ -267,7 +315,7 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
             int i = 0;
             bool ok = true;
             const long long t_start = CV_CLOCK();
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++i) {
+            for (int q = next_own(own_mask, 0, own); q < own && ok; q = next_own(own_mask, q + 1, own), ++i) {
                 const int s       = i % p.stages;
                 const uint32_t ph = (uint32_t)(i / p.stages) & 1u;
                 // the accumulator of the previous tile has been drained
@@ -326,7 +374,7 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
         const int npos = p.box_rows * p.pw;
         const int cstride = p.box_rows * p.box_w; // floats between two channels of one position
         int i = 0;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
+        for (int q = next_own(own_mask, 0, own); q < own; q = next_own(own_mask, q + 1, own), ++i) {
             const int rs       = i % kTA_RawStages;
             const uint32_t rph = (uint32_t)(i / kTA_RawStages) & 1u;
             const int s        = i % p.stages;
@@ -423,7 +471,8 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
             bias_r[j]    = (p.bias && ch < p.ko) ? p.bias[ch] : 0.0f;
         }
         int i = 0;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
+        for (int q = next_own(own_mask, 0, own); q < own; q = next_own(own_mask, q + 1, own), ++i) {
+            const int tile = (int)blockIdx.x + q * (int)gridDim.x;
             const int img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
             const long long e0 = CV_CLOCK();
             bool got = mbar_wait_patient(smem_u32(&bar_tmem_full), (uint32_t)i & 1u, abort_flag);
@@ -567,15 +616,8 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 512);
     }
-    if (threadIdx.x == 0) {
-        if (*abort_flag)
-            atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
-        // the last CTA clears the word for the next product
-        if (atomicAdd(p.flags + FLAG_WIDE_READERS, 1u) + 1u == gridDim.x) {
-            p.flags[FLAG_WIDE_READERS] = 0u;
-            p.flags[FLAG_WIDE]         = 0u;
-        }
-    }
+    if (threadIdx.x == 0 && *abort_flag)
+        atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
 }
 
 // ---- the same in split float16 ------------------------------------------------------------
@@ -587,8 +629,9 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
 //     D1 = [W_hi; W_lo] x X_hi,  D2 = [W_hi; W_lo] x X_lo   (128 x 128 each, next to at most 192 filter columns)
 // and a thread that drains row m forms D1 + 2^-11 D2 before anything is parked, which leaves the rest of the
 // epilogue as it is above (hi row + lo row).  Eight warps convert (four needed 4250 clocks per tile where the
-// MMAs now take 2628) and what sets the pace is the epilogue.  A value, tile or filter that float16 pairs
-// cannot hold raises FLAG_WIDE; conv_tmem_filters_kernel, launched behind this one, then computes the layer again.
+// MMAs now take 2628) and what sets the pace is the epilogue.  The converting warps also leave the range of every
+// tile in the call's own scratch; conv_tmem_filters_kernel, launched behind this one, computes the images that
+// float16 pairs cannot hold.  A tile that shows that by itself is not converted, multiplied or stored here.
 constexpr int kTH_CvtWarps = 8;
 constexpr int kTH_Threads  = 64 + 32 * kTH_CvtWarps + 32 * kTA_EpiWarps;
 constexpr int kTH_D1 = 192, kTH_D2 = 320; // accumulator columns behind 24 k-steps of 8 filter columns
@@ -610,7 +653,7 @@ __device__ __forceinline__ void mma_f16_a_tmem(
 template <bool RAW>
 __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
     const __grid_constant__ CUtensorMap map_x_hi, const __grid_constant__ CUtensorMap map_x_lo,
-    const __grid_constant__ ConvTmemParams p, const float *__restrict__ image_scale, const int total_tiles) {
+    const __grid_constant__ ConvTmemParams p, const int total_tiles) {
     constexpr int kMaxStages = 4;
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t bar_full[kMaxStages], bar_empty[kMaxStages];
@@ -618,16 +661,17 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
     __shared__ uint64_t bar_scale_empty[kMaxStages]; // the tile's scale has been read by the epilogue
     __shared__ uint64_t bar_tmem_full, bar_tmem_empty, bar_done, bar_epi, bar_cvt;
     __shared__ uint32_t tmem_base_slot;
-    __shared__ int abort_flag_s;
-    __shared__ uint32_t cvt_max[2][kTH_CvtWarps];
-    __shared__ float tile_scale[kMaxStages]; // inverse scale of the tile in each plane stage
+    __shared__ int abort_flag_s, filters_wide_s;
+    __shared__ uint2 cvt_range[2][kTH_CvtWarps];
+    __shared__ float tile_scale[kMaxStages]; // inverse scale of the tile in each plane stage; 0: left to the tf32 form
     __shared__ float filter_inv[64];
-    __shared__ uint32_t filter_max[64];
     volatile int *abort_flag = &abort_flag_s;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x == 0)
-        abort_flag_s = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
+    if (threadIdx.x == 0) {
+        abort_flag_s   = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
+        filters_wide_s = 0;
+    }
     __syncthreads();
     if (abort_flag_s)
         return;
@@ -657,15 +701,20 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
         prefetch_tensormap(&map_x_hi);
         prefetch_tensormap(&map_x_lo);
     }
-    for (int f = warp; f < 64; f += kTH_Threads / 32) { // largest magnitude of each filter, a warp per filter
-        uint32_t mx = 0;
+    for (int f = warp; f < 64; f += kTH_Threads / 32) { // range of each filter, a warp per filter
+        uint2 range = make_uint2(0u, kNoneSmallest);
         if (f < p.ko)
 #pragma unroll 4
             for (int e = lane; e < p.c * p.kh * p.kw; e += 32)
-                mx = max(mx, __float_as_uint(p.w[(int64_t)f * p.c * p.kh * p.kw + e]) & 0x7fffffffu);
-        mx = __reduce_max_sync(0xffffffffu, mx);
-        if (lane == 0)
-            filter_max[f] = mx;
+                range_take(range, p.w[(int64_t)f * p.c * p.kh * p.kw + e]);
+        range = range_warp(range);
+        float scale, inverse;
+        const bool fits = half_range_fits(range, scale, inverse);
+        if (lane == 0) {
+            filter_inv[f] = inverse;
+            if (!fits)
+                filters_wide_s = 1;
+        }
     }
     if (warp == 1) {
         tmem_alloc(smem_u32(&tmem_base_slot), 512);
@@ -675,20 +724,18 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
-    bool bad = false; // something float16 pairs cannot hold
+    const bool filters_wide  = filters_wide_s != 0; // every tile is left to the tf32 form
+    if (RAW && blockIdx.x == 0 && threadIdx.x == 0)
+        p.tile_range[total_tiles] = make_uint2(filters_wide ? 1u : 0u, 0u);
 
     // ---- the filters go to tensor memory, once: warps 2..5 own the four lane quarters ----------
-    if (warp >= 2 && warp < 6) {
+    if (warp >= 2 && warp < 6 && !filters_wide) {
         const int quarter = warp & 3;
         const int m = quarter * 32 + lane, ch = m & 63; // TMEM lane = row of the A operand; filter
         const bool lo_row = m >= 64;
         const int taps    = p.kh * p.kw;
         const float *src  = p.w + (int64_t)ch * p.c * taps;
-        const uint32_t mx = filter_max[ch];
-        float scale = 1.0f, inverse = 1.0f;
-        bad = mx >= 0x7f800000u || !half_scale(mx, scale, inverse);
-        if (!lo_row)
-            filter_inv[ch] = inverse;
+        const float scale = 1.0f / filter_inv[ch]; // both are powers of two
 #pragma unroll 2
         for (int ks = 0; ks < 2 * taps; ++ks) {
             const int tap = ks >> 1, c0 = (ks & 1) * 16;
@@ -701,7 +748,7 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                     const int ic  = c0 + 2 * j + t;
                     const float x = (ch < p.ko && ic < p.c) ? src[ic * taps + tap] : 0.0f;
                     __half hi, lo;
-                    bad |= split_half(x * scale, hi, lo);
+                    split_half(x * scale, hi, lo);
                     part[t] = lo_row ? lo : hi;
                 }
                 v[j] = *reinterpret_cast<uint32_t *>(part);
@@ -714,13 +761,16 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
     __syncthreads();
     tc_fence_after_sync();
 
-    if (warp == 0) {
+    if (filters_wide) {
+    } else if (warp == 0) {
         // ===== TMA producer: one halo box per plane and tile (raw mode: one box of the input) =====
         if (lane == 0) {
             int i = 0;
             const int nstages = RAW ? kTA_RawStages : p.stages;
-            for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
+            for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
                 const int img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
+                if (!RAW && image_needs_tf32<RAW>(p, img, total_tiles))
+                    continue;
                 const int s       = i % nstages;
                 const uint32_t ph = (uint32_t)(i / nstages) & 1u;
                 if (!mbar_wait_patient(smem_u32(RAW ? &bar_raw_empty[s] : &bar_empty[s]), ph ^ 1u, abort_flag))
@@ -737,6 +787,7 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                     tma_load_4d(dst, &map_x_hi, full, 0, -p.pad, h0, img);
                     tma_load_4d(dst + (uint32_t)p.plane_bytes, &map_x_lo, full, 0, -p.pad, h0, img);
                 }
+                ++i;
             }
             if (*abort_flag) {
                 // unwind: let the copies still in flight land before the CTA goes away
@@ -755,7 +806,9 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
             const uint32_t d1 = tmem_base + (uint32_t)kTH_D1, d2 = tmem_base + (uint32_t)kTH_D2;
             int i   = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
+            for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
+                if (!RAW && image_needs_tf32<RAW>(p, tile / p.tiles_y, total_tiles))
+                    continue;
                 const int s = i % p.stages;
                 // the accumulators of the previous tile have been read, the planes are complete
                 ok = mbar_wait(smem_u32(&bar_tmem_empty), ((uint32_t)i & 1u) ^ 1u, abort_flag) &&
@@ -765,7 +818,8 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                 tc_fence_after_sync();
                 const uint32_t x_hi = smem_base + (uint32_t)s * stage_bytes, x_lo = x_hi + (uint32_t)p.plane_bytes;
                 int ks = 0;
-                for (int r = 0; r < p.kh; ++r) {
+                const int rows = RAW && *const_cast<volatile float *>(&tile_scale[s]) == 0.0f ? 0 : p.kh;
+                for (int r = 0; r < rows; ++r) {
                     for (int sx = 0; sx < p.kw; ++sx) {
                         // the tap's pixels: the same box, (r * pw + sx) rows further on
                         const uint32_t shift = (uint32_t)(r * p.pw + sx) * (uint32_t)kTH_RowB;
@@ -780,6 +834,7 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                 }
                 tc_commit(smem_u32(&bar_empty[s]));  // the stage is free once these MMAs have retired
                 tc_commit(smem_u32(&bar_tmem_full)); // and the accumulators are complete
+                ++i;
             }
             if (!ok || *abort_flag) {
                 tc_commit(smem_u32(&bar_done));
@@ -801,37 +856,38 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                 if (!__all_sync(0xffffffffu, got))
                     break;
                 const float *raw = reinterpret_cast<const float *>(smem_raw + (raw_base - smem_u32(smem_raw)) + (uint32_t)rs * (uint32_t)p.raw_stride);
-                // the tile's largest magnitude (the whole box, alignment columns included: they are pixels or zero)
-                uint32_t mx       = 0;
+                // the tile's range (the whole box, alignment columns included: they are pixels or zero)
+                uint2 range       = make_uint2(0u, kNoneSmallest);
                 const float4 *r4  = reinterpret_cast<const float4 *>(raw);
 #pragma unroll 4
                 for (int e = ct; e < p.raw_bytes / 16; e += 32 * kTH_CvtWarps) {
                     const float4 q = r4[e];
-                    mx = max(max(max(mx, __float_as_uint(q.x) & 0x7fffffffu), __float_as_uint(q.y) & 0x7fffffffu),
-                             max(__float_as_uint(q.z) & 0x7fffffffu, __float_as_uint(q.w) & 0x7fffffffu));
+                    range_take(range, q.x), range_take(range, q.y), range_take(range, q.z), range_take(range, q.w);
                 }
-                mx = __reduce_max_sync(0xffffffffu, mx);
+                range = range_warp(range);
                 if (lane == 0) {
-                    cvt_max[i & 1][warp - 2] = mx;
+                    cvt_range[i & 1][warp - 2] = range;
                     mbar_arrive(smem_u32(&bar_cvt));
                 }
-                got = mbar_wait(smem_u32(&bar_cvt), (uint32_t)i & 1u, abort_flag) && // all eight maxima
+                got = mbar_wait(smem_u32(&bar_cvt), (uint32_t)i & 1u, abort_flag) && // all eight ranges
                       mbar_wait_patient(smem_u32(&bar_empty[s]), ((uint32_t)(i / p.stages) & 1u) ^ 1u, abort_flag) &&
                       mbar_wait_patient(smem_u32(&bar_scale_empty[s]), ((uint32_t)(i / p.stages) & 1u) ^ 1u, abort_flag);
                 if (!__all_sync(0xffffffffu, got))
                     break;
 #pragma unroll
                 for (int u = 0; u < kTH_CvtWarps; ++u)
-                    mx = max(mx, cvt_max[i & 1][u]);
+                    range = range_join(range, cvt_range[i & 1][u]);
                 float scale, inverse;
-                bad |= mx >= 0x7f800000u || !half_scale(mx, scale, inverse);
-                if (ct == 0)
-                    tile_scale[s] = inverse;
+                const bool fits = half_range_fits(range, scale, inverse);
+                if (ct == 0) {
+                    tile_scale[s]      = fits ? inverse : 0.0f;
+                    p.tile_range[tile] = range;
+                }
                 uint8_t *x_hi = smem_raw + (smem_base - smem_u32(smem_raw)) + (uint32_t)s * stage_bytes;
                 uint8_t *x_lo = x_hi + p.plane_bytes;
                 // a thread takes a position: 32 channels become the 64-byte row y * pw + x of both planes, 16-byte
                 // chunk j at j ^ ((row >> 1) & 3), the 64-byte swizzle
-                for (int pos = ct; pos < npos; pos += 32 * kTH_CvtWarps) {
+                for (int pos = fits ? ct : npos; pos < npos; pos += 32 * kTH_CvtWarps) {
                     const int y = pos / p.pw, x = pos - y * p.pw;
                     const float *src = raw + y * p.box_w + x + p.off_x;
                     const uint32_t row_off = (uint32_t)pos * (uint32_t)kTH_RowB, sw = ((uint32_t)pos >> 1) & 3u;
@@ -850,7 +906,6 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                                 hi[t] = __floats2half2_rn(a, b);
                                 lo[t] = __floats2half2_rn(__fmul_rn(__fsub_rn(a, __low2float(hi[t])), kHalfLoScale),
                                                           __fmul_rn(__fsub_rn(b, __high2float(hi[t])), kHalfLoScale));
-                                bad |= (a != 0.0f && fabsf(a) < kHalfSmallest) || (b != 0.0f && fabsf(b) < kHalfSmallest);
                             }
                             const uint32_t at = row_off + (((uint32_t)(2 * half + j) ^ sw) << 4);
                             *reinterpret_cast<uint4 *>(x_hi + at) = *reinterpret_cast<uint4 *>(hi);
@@ -910,12 +965,24 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
         int i = 0;
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
             const int img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
+            if (!RAW && image_needs_tf32<RAW>(p, img, total_tiles)) {
+                --i;
+                continue;
+            }
             bool got = mbar_wait_patient(smem_u32(&bar_tmem_full), (uint32_t)i & 1u, abort_flag);
             if (!__all_sync(0xffffffffu, got))
                 break;
-            const float is = RAW ? *const_cast<volatile float *>(&tile_scale[i % p.stages]) : image_scale[img];
+            const float is = RAW ? *const_cast<volatile float *>(&tile_scale[i % p.stages]) : p.image_scale[img];
             const int y0   = ty * p.th;
             tc_fence_after_sync();
+            if (RAW && is == 0.0f) {
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(smem_u32(&bar_tmem_empty));
+                    mbar_arrive(smem_u32(&bar_scale_empty[i % p.stages]));
+                }
+                continue;
+            }
             float4 *mine         = reinterpret_cast<float4 *>(staging + m * kTA_StageRowF + half * 64);
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 64);
             // D1 + 2^-11 D2, sixteen columns of each at a time; the accumulators are handed back before anything
@@ -1037,8 +1104,6 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
         }
     }
 
-    if (bad)
-        p.flags[FLAG_WIDE] = 1u;
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 1) {
@@ -1124,9 +1189,10 @@ static bool conv_tmem_reads_input_directly(const float *x, int64_t h, int64_t w,
     return conv_tmem_plan(p, h, w, kh, kw, pad, pool, true);
 }
 
-// x NCHW float32.  The layer in split float16, and behind it the tf32 form, which does nothing unless the first
-// (or its pre-pass) has raised FLAG_WIDE.  Where the rows allow a tensor map over it the input is read as it is;
-// else from NHWC planes in the workspace: [image scale][image max][planes], float16 first, tf32 in the same place.
+// x NCHW float32.  The layer in split float16, and behind it the tf32 form for the images that need it.  Where the
+// rows allow a tensor map over it the input is read as it is, with the tiles' ranges in scratch of this call's own (such
+// a layer shares no memory with calls on other streams); else from planes in the workspace:
+// [filter scale][image scale][image ranges][image slots].
 ct_status conv_tmem_filters(
     DeviceState *st, const float *x, const float *w, const float *bias, int64_t batch, int64_t c, int64_t h, int64_t wd,
     int64_t ko, int64_t kh, int64_t kw, int64_t pad, int act, int pool, float *out) {
@@ -1136,7 +1202,7 @@ ct_status conv_tmem_filters(
         p[f].w = w, p[f].bias = bias, p[f].out = out, p[f].flags = st->flags_dev;
         p[f].ko = (int)ko, p[f].c = (int)c;
         p[f].act = act, p[f].pool = pool;
-        p[f].only_if = st->flags_dev + FLAG_WIDE;
+        p[f].image_scale = nullptr, p[f].tile_range = nullptr;
         if (!conv_tmem_plan(p[f], h, wd, kh, kw, pad, pool, raw, f == 0 ? kTH_RowB : 128))
             return fail(CT_ERR_INVALID, "conv2d: internal tile shape %d x %d not usable", p[f].th, p[f].pw);
     }
@@ -1154,7 +1220,8 @@ ct_status conv_tmem_filters(
     auto smem_of = [&](const ConvTmemParams &q) {
         return (size_t)q.stages * 2 * q.plane_bytes + (raw ? (size_t)kTA_RawStages * q.raw_stride : 0) + kTA_StagingBytes + 1024;
     };
-    const unsigned grid = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
+    const unsigned grid   = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
+    const unsigned grid32 = (unsigned)std::max<int64_t>(grid, (tiles + kTA_MaxOwn - 1) / kTA_MaxOwn);
     if (raw) {
         // the input [batch][c][h][w]; box = box_w floats x box_rows rows x 32 channels of one image, not
         // swizzled; outside the image and past the last channel it reads as zero: padding for free
@@ -1164,49 +1231,50 @@ ct_status conv_tmem_filters(
                                      4ull * (uint64_t)wd * (uint64_t)h * (uint64_t)c};
         const uint32_t box[4]     = {(uint32_t)p[0].box_w, (uint32_t)p[0].box_rows, 32, 1};
         CT_TRY(encode_tiled_map_f32(&map, x, 4, dims, strides, box, /*swizzle_bytes=*/0));
-        ProfScope prof("gemm_tc");
-        conv_tmem_half_kernel<true><<<grid, kTH_Threads, smem_of(p[0]), stream()>>>(map, map, p[0], nullptr, (int)tiles);
-        CT_LAUNCH_CHECK("conv_tmem_half");
-        conv_tmem_filters_kernel<true><<<grid, kTA_ThreadsRaw, smem_of(p[1]), stream()>>>(map, map, p[1], (int)tiles);
-        CT_LAUNCH_CHECK("conv_tmem_filters");
+        void *ranges = nullptr;
+        CT_TRY(ct_alloc(&ranges, (size_t)(tiles + 1) * sizeof(uint2)));
+        p[0].tile_range = p[1].tile_range = static_cast<uint2 *>(ranges);
+        cudaError_t launched;
+        {
+            ProfScope prof("gemm_tc");
+            conv_tmem_half_kernel<true><<<grid, kTH_Threads, smem_of(p[0]), stream()>>>(map, map, p[0], (int)tiles);
+            conv_tmem_filters_kernel<true><<<grid32, kTA_ThreadsRaw, smem_of(p[1]), stream()>>>(map, map, p[1], (int)tiles);
+            launched = cudaGetLastError();
+        }
+        CT_TRY(ct_free(ranges)); // in stream order, behind both
+        if (launched != cudaSuccess)
+            return cuda_fail(launched, "conv_tmem");
+        count_launch(2);
         return CT_OK;
     }
-    auto align_up        = [](size_t v) { return (v + 1023) & ~(size_t)1023; };
-    const size_t words   = align_up((size_t)batch * 4);
-    const size_t plane32 = align_up((size_t)batch * h * wd * 32 * 4), plane16 = align_up((size_t)batch * h * wd * 32 * 2);
-    if (batch > 65535)
-        return fail(CT_ERR_TOO_LARGE, "conv2d: batch or channel count too large for the layout pre-pass");
-    CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, 2 * words + 2 * plane32));
-    uint8_t *ws = static_cast<uint8_t *>(st->gemm_ws), *planes = ws + 2 * words;
-    float *image_scale = reinterpret_cast<float *>(ws);
-    {
-        ProfScope prof("conv_prepass");
-        CT_TRY(nhwc_half_planes(st, x, batch, c, h * wd, 32, planes, planes + plane16, reinterpret_cast<uint32_t *>(ws + words),
-                                image_scale, st->flags_dev + FLAG_WIDE));
-    }
+    auto align_up       = [](size_t v) { return (v + 1023) & ~(size_t)1023; };
+    const size_t f_words = align_up((size_t)ko * 4), words = align_up((size_t)batch * 4), slot = (size_t)h * wd * 32 * 8;
+    const size_t ranges  = align_up((size_t)batch * conv_range_slices(c * h * wd) * 8);
+    CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, f_words + words + ranges + (size_t)batch * slot));
+    uint8_t *ws = static_cast<uint8_t *>(st->gemm_ws), *planes = ws + f_words + words + ranges;
+    float *image_scale = reinterpret_cast<float *>(ws + f_words);
+    CT_TRY(conv_prepass(st, x, w, batch, c, h * wd, 32, ko, kh * kw, nullptr, nullptr, 0, 0, reinterpret_cast<float *>(ws),
+                        ws + f_words + words, image_scale, planes));
+    p[0].image_scale = p[1].image_scale = image_scale;
     // planes [batch][h][w][32 channels]; box = 32 channels x pw positions x (th + kh - 1) rows of one image,
     // swizzled over a row; positions outside the image read as zero: the padding
     auto encode = [&](CUtensorMap *map, const void *base, int elem) {
         const uint64_t row = 32ull * (uint64_t)elem;
         const uint64_t dims[4] = {32, (uint64_t)wd, (uint64_t)h, (uint64_t)batch};
-        const uint64_t strides[3] = {row, row * (uint64_t)wd, row * (uint64_t)wd * (uint64_t)h};
+        const uint64_t strides[3] = {row, row * (uint64_t)wd, slot};
         const uint32_t box[4] = {32, (uint32_t)p[0].pw, (uint32_t)p[0].box_rows, 1};
         return elem == 4 ? encode_tiled_map_f32(map, base, 4, dims, strides, box, 128)
                          : encode_tiled_map_f16(map, base, 4, dims, strides, box, kTH_RowB);
     };
     CUtensorMap m16_hi, m16_lo, m32_hi, m32_lo;
     CT_TRY(encode(&m16_hi, planes, 2));
-    CT_TRY(encode(&m16_lo, planes + plane16, 2));
+    CT_TRY(encode(&m16_lo, planes + slot / 4, 2));
     CT_TRY(encode(&m32_hi, planes, 4));
-    CT_TRY(encode(&m32_lo, planes + plane32, 4));
-    {
-        ProfScope prof("gemm_tc");
-        conv_tmem_half_kernel<false><<<grid, kTH_Threads, smem_of(p[0]), stream()>>>(m16_hi, m16_lo, p[0], image_scale, (int)tiles);
-        CT_LAUNCH_CHECK("conv_tmem_half");
-    }
-    CT_TRY(nhwc_wide_planes(st, st->flags_dev + FLAG_WIDE, x, batch, c, h * wd, 32, planes, planes + plane32));
+    CT_TRY(encode(&m32_lo, planes + slot / 2, 4));
     ProfScope prof("gemm_tc");
-    conv_tmem_filters_kernel<false><<<grid, kTA_Threads, smem_of(p[1]), stream()>>>(m32_hi, m32_lo, p[1], (int)tiles);
+    conv_tmem_half_kernel<false><<<grid, kTH_Threads, smem_of(p[0]), stream()>>>(m16_hi, m16_lo, p[0], (int)tiles);
+    CT_LAUNCH_CHECK("conv_tmem_half");
+    conv_tmem_filters_kernel<false><<<grid32, kTA_Threads, smem_of(p[1]), stream()>>>(m32_hi, m32_lo, p[1], (int)tiles);
     CT_LAUNCH_CHECK("conv_tmem_filters");
     return CT_OK;
 }

@@ -11,6 +11,7 @@
 // same two 11-bit numbers whatever the scale (every bit of lo lies above float16's smallest).  A matrix with a
 // smaller non-zero value - 2^-27 of its row's largest or less - or a row whose exponent is beyond +-60 raises a
 // device word, and the product is then computed from tf32 planes instead (same launch sequence, no host involvement).
+// Convolutions decide it per image (and per layer for its filters), see half_range_fits.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -41,6 +42,28 @@ __device__ __forceinline__ bool half_scale(uint32_t max_bits, float &scale, floa
     scale   = exact_pow2(14 - e);
     inverse = exact_pow2(e - 14);
     return ok;
+}
+
+// The range of the values that share a scale, gathered with two instructions a value: .x the largest magnitude (an
+// infinity or NaN as what it is), .y the smallest non-zero one less 1 (all ones: there is none).
+constexpr uint32_t kNoneSmallest = 0xffffffffu;
+__device__ __forceinline__ void range_take(uint2 &r, float v) {
+    const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
+    r.x = max(r.x, u);
+    r.y = min(r.y, u - 1u);
+}
+__device__ __forceinline__ uint2 range_join(uint2 a, uint2 b) { return make_uint2(max(a.x, b.x), min(a.y, b.y)); }
+__device__ __forceinline__ uint2 range_warp(uint2 r) {
+    return make_uint2(__reduce_max_sync(0xffffffffu, r.x), __reduce_min_sync(0xffffffffu, r.y));
+}
+
+// Whether float16 pairs under one scale hold every value of the range as the two 11-bit terms that any other
+// scale would give: the rule of the convolutions, whose scales belong to an image or to a tile of it.  An image for
+// which this is true has the same bits in its outputs whatever part of it a scale was taken over.
+constexpr float kHalfExact = 1.0f / (1u << 12);
+__device__ __forceinline__ bool half_range_fits(uint2 r, float &scale, float &inverse) {
+    const bool ok = half_scale(r.x, scale, inverse);
+    return ok && (r.y == kNoneSmallest || __uint_as_float(r.y + 1u) * scale >= kHalfExact);
 }
 
 // v is already scaled.  Returns true when v is too small beside its row's largest value.

@@ -197,6 +197,76 @@ def test_convolution_keeps_small_values_beside_large_ones(T, shape, kind, lowest
     assert np.all(np.abs(got - want) <= SINGLE * np.abs(want))
 
 
+def _conv_at(T, x, w, stride, pad, off=0):
+    """The layer on an input that starts `off` floats into its buffer."""
+    from camel_b200._lib import check, lib
+
+    n, c, h, wd = x.shape
+    ko, _, kh, kw = w.shape
+    tx = T.from_numpy(np.concatenate([np.zeros(off, np.float32), x.ravel()]))
+    tw, out = T.from_numpy(w), T.zeros((n, ko, (h + 2 * pad - kh) // stride + 1, (wd + 2 * pad - kw) // stride + 1))
+    check(lib.ct_conv2d(tx.ptr + 4 * off, tw.ptr, None, n, c, h, wd, ko, kh, kw, stride, pad, 0, out.ptr))
+    T.check_async()
+    return out.numpy()
+
+
+# filters in tensor memory (tiles of seven rows, of six with the pool; of four), halos
+@pytest.mark.parametrize("shape", [(5, 32, 16, 16, 64, 3), (4, 30, 28, 28, 60, 3), (3, 64, 30, 28, 128, 3)])
+def test_bits_of_an_image_depend_on_that_image_alone(T, shape):
+    """Not on the other images of the batch, on the fused pool, or on whether the input is read as it is or from planes."""
+    n, c, h, wd, ko, kern = shape
+    rng = np.random.default_rng(sum(shape))
+    x = rng.standard_normal((n, c, h, wd)).astype(np.float32)
+    w = rng.standard_normal((ko, c, kern, kern)).astype(np.float32)
+    clean = _conv_at(T, x, w, 1, 1)
+    wide = x.copy()
+    wide[1, 3, h - 1, 2], wide[1, 2, 0, 0] = 2.0**-30, 2.0**3  # image 1 spans too much, its tiles do not
+    wide[2, 0, h // 2] *= 2.0**-28                             # image 2 does inside a tile as well
+    got = _conv_at(T, wide, w, 1, 1)
+    others = [i for i in range(n) if i not in (1, 2)]
+    assert got[others].tobytes() == clean[others].tobytes()
+    for i in (1, 2):
+        assert _conv_at(T, np.stack([wide[i]] * n), w, 1, 1)[0].tobytes() == got[i].tobytes()
+    assert _conv_at(T, wide, w, 1, 1, off=1).tobytes() == got.tobytes()
+    pooled = T.conv2d(T.from_numpy(wide), T.from_numpy(w), None, 1, 1, pool=2).numpy()
+    assert pooled.tobytes() == T.maxpool2d(T.from_numpy(got), 2).numpy().tobytes()
+    assert np.all(np.abs(got - _conv64(wide, w, 1, 1)) <= (384 * 2.0**-24 + 2.0**-21) * _conv64(np.abs(wide), np.abs(w), 1, 1))
+
+
+def test_few_channel_layers_on_two_streams_share_no_state(T):
+    """Wide and ordinary inputs side by side; neither layer uses the library's workspaces."""
+    import ctypes as C
+
+    from camel_b200._lib import check, lib
+
+    rng = np.random.default_rng(21)
+    x = [rng.standard_normal((40, 32, 28, 28)).astype(np.float32) for _ in range(2)]
+    x[1] *= np.exp2(rng.integers(-45, 45, x[1].shape)).astype(np.float32)
+    w = rng.standard_normal((64, 32, 3, 3)).astype(np.float32)
+    want = [_conv_at(T, v, w, 1, 1).tobytes() for v in x]
+    tx, tw = [T.from_numpy(v) for v in x], T.from_numpy(w)
+    outs = [[T.zeros((40, 64, 28, 28)) for _ in range(6)] for _ in range(2)]
+    streams = [C.c_void_p(), C.c_void_p()]
+    T.sync()
+    for s in streams:
+        check(lib.ct_stream_create(C.byref(s)))
+    try:
+        for i in range(6):
+            for j, s in enumerate(streams):
+                check(lib.ct_set_stream(s))
+                check(lib.ct_conv2d(tx[j].ptr, tw.ptr, None, 40, 32, 28, 28, 64, 3, 3, 1, 1, 0, outs[j][i].ptr))
+        for s in streams:
+            check(lib.ct_set_stream(s))
+            check(lib.ct_sync())
+    finally:
+        check(lib.ct_set_stream(None))
+        for s in streams:
+            check(lib.ct_stream_destroy(s))
+    T.check_async()
+    for j in range(2):
+        assert all(o.numpy().tobytes() == want[j] for o in outs[j])
+
+
 # (n, c, h, w, ko, kernel, stride, pad): patches in registers and read twice (k = 1200), odd sizes; halos with a
 # partial last tile, channels that do not fill a block, more than 128 filters, 1 x 1 and 5 x 5 taps
 CONVS = [(3, 48, 21, 23, 70, 3, 2, 1), (2, 8, 33, 21, 20, 3, 2, 0), (2, 48, 15, 16, 40, 5, 3, 2), (2, 12, 24, 24, 65, 5, 1, 2),
