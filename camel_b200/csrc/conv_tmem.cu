@@ -138,6 +138,28 @@ __device__ __forceinline__ int next_own(const uint32_t *mask, int q, int own) {
     return own;
 }
 
+// The filters [ko][row] in shared memory, rows an odd number of floats apart so that lanes that own filters read distinct
+// banks; a warp per filter, which it hands to `seen` as it goes (every lane has its share).  Read from global
+// memory by the lanes that write them to tensor memory - 128 threads, a sector for every value - the set-up took
+// 35 of the 41 us of a layer on four images.
+__device__ __forceinline__ int filter_stride(const ConvTmemParams &p) { return (p.c * p.kh * p.kw) | 1; }
+template <typename Seen>
+__device__ __forceinline__ void stage_filters(const ConvTmemParams &p, float *rows, int warp, int warps, int lane, Seen seen) {
+    const int row = p.c * p.kh * p.kw, stride = filter_stride(p);
+    for (int f = warp; f < p.ko; f += warps) {
+        uint2 range = make_uint2(0u, kNoneSmallest);
+#pragma unroll 4
+        for (int e = lane; e < row; e += 32) {
+            const float v = p.w[(int64_t)f * row + e];
+            range_take(range, v);
+            rows[f * stride + e] = v;
+        }
+        seen(f, range);
+    }
+}
+// ... and of a region that the asynchronous proxy writes next.
+__device__ __forceinline__ void filters_taken() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 __device__ __forceinline__ void tmem_st_32x32_x8(uint32_t taddr, const uint32_t (&r)[8]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
@@ -233,6 +255,8 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
         tmem_alloc(smem_u32(&tmem_base_slot), 512);
         tmem_relinquish();
     }
+    float *filters = reinterpret_cast<float *>(smem_raw + (smem_base - smem_u32(smem_raw))); // where the stages will be
+    stage_filters(p, filters, warp, (int)blockDim.x / 32, lane, [](int, uint2) {});
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -245,21 +269,22 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
         const int ch      = m & 63;                   // filter
         const bool lo_row = m >= 64;                  // rows 64..127: the low parts
         const int taps    = p.kh * p.kw;
+        const float *src  = filters + ch * filter_stride(p);
+#pragma unroll 2
         for (int ks = 0; ks < p.ksteps; ++ks) {
             const int tap = ks >> 2, c0 = (ks & 3) * 8;
             uint32_t v[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                float x = 0.0f;
-                if (ch < p.ko && c0 + j < p.c)
-                    x = p.w[((int64_t)ch * p.c + (c0 + j)) * taps + tap];
+                const float x = (ch < p.ko && c0 + j < p.c) ? src[(c0 + j) * taps + tap] : 0.0f;
                 float hi, lo;
-                split_tf32(x, hi, lo);
+                split_tf32_flat(x, hi, lo);
                 v[j] = __float_as_uint(lo_row ? lo : hi);
             }
             tmem_st_32x32_x8(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ks * 8), v);
         }
         tmem_st_wait();
+        filters_taken();
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -672,6 +697,8 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
         abort_flag_s   = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
         filters_wide_s = 0;
     }
+    if (threadIdx.x < 64)
+        filter_inv[threadIdx.x] = 1.0f; // rows without a filter are zero
     __syncthreads();
     if (abort_flag_s)
         return;
@@ -701,21 +728,16 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
         prefetch_tensormap(&map_x_hi);
         prefetch_tensormap(&map_x_lo);
     }
-    for (int f = warp; f < 64; f += kTH_Threads / 32) { // range of each filter, a warp per filter
-        uint2 range = make_uint2(0u, kNoneSmallest);
-        if (f < p.ko)
-#pragma unroll 4
-            for (int e = lane; e < p.c * p.kh * p.kw; e += 32)
-                range_take(range, p.w[(int64_t)f * p.c * p.kh * p.kw + e]);
-        range = range_warp(range);
+    float *filters = reinterpret_cast<float *>(smem_raw + (smem_base - smem_u32(smem_raw))); // where the stages will be
+    stage_filters(p, filters, warp, kTH_Threads / 32, lane, [&](int f, uint2 range) {
         float scale, inverse;
-        const bool fits = half_range_fits(range, scale, inverse);
+        const bool fits = half_range_fits(range_warp(range), scale, inverse);
         if (lane == 0) {
             filter_inv[f] = inverse;
             if (!fits)
                 filters_wide_s = 1;
         }
-    }
+    });
     if (warp == 1) {
         tmem_alloc(smem_u32(&tmem_base_slot), 512);
         tmem_relinquish();
@@ -734,7 +756,7 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
         const int m = quarter * 32 + lane, ch = m & 63; // TMEM lane = row of the A operand; filter
         const bool lo_row = m >= 64;
         const int taps    = p.kh * p.kw;
-        const float *src  = p.w + (int64_t)ch * p.c * taps;
+        const float *src  = filters + ch * filter_stride(p);
         const float scale = 1.0f / filter_inv[ch]; // both are powers of two
 #pragma unroll 2
         for (int ks = 0; ks < 2 * taps; ++ks) {
@@ -756,6 +778,7 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
             tmem_st_32x32_x8(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ks * 8), v);
         }
         tmem_st_wait();
+        filters_taken();
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -1173,6 +1196,8 @@ static bool conv_tmem_plan(
     if (raw && (p.box_w > 256 || p.box_rows > 256))
         return false;
     const int budget = 226 * 1024 - 1024 - kTA_StagingBytes - (raw ? kTA_RawStages * p.raw_stride : 0);
+    // (stages, boxes and the staging block also hold the filters for a moment at the start: at least 42 KB to spare over all
+    // shapes that conv_tmem_applicable accepts)
     p.stages         = budget / (2 * p.plane_bytes);
     if (p.stages > 4)
         p.stages = 4;
