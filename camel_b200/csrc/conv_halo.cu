@@ -30,6 +30,8 @@
 #include "tc_ptx.cuh"
 #include "tmap.cuh"
 
+#include <algorithm>
+
 // Optional per-CTA clock accounting for tuning; compiled in only with -DCT_CONV_TRACE.
 #ifdef CT_CONV_TRACE
 __device__ unsigned long long g_halo_trace[256 * 16];
@@ -519,12 +521,13 @@ __global__ void __launch_bounds__(256) conv_planes_kernel(
     const int c0      = (int)blockIdx.y * 64;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float *src = x + (img * c + c0) * hw + q0;
+    float v[16]; // every load before the first use of any
 #pragma unroll
     for (int j = 0; j < 8; ++j)
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
             const int ch = warp + 8 * j, q = lane + 32 * t;
-            tile[ch][q]  = (c0 + ch < c && q0 + q < hw) ? __ldcs(src + ch * hw + q) : 0.0f;
+            v[2 * j + t] = (c0 + ch < c && q0 + q < hw) ? __ldcs(src + ch * hw + q) : 0.0f;
         }
     uint2 r = make_uint2(0u, kNoneSmallest);
     for (int s = lane; s < slices; s += 32)
@@ -532,6 +535,9 @@ __global__ void __launch_bounds__(256) conv_planes_kernel(
     int bad_filter = 0;
     for (int o = threadIdx.x; o < ko; o += 256)
         bad_filter |= filter_scale[o] == 0.0f ? 1 : 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        tile[warp + 8 * (j >> 1)][lane + 32 * (j & 1)] = v[j];
     float scale, inverse;
     const bool fits = half_range_fits(range_warp(r), scale, inverse) & !__syncthreads_or(bad_filter);
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
@@ -545,10 +551,10 @@ __global__ void __launch_bounds__(256) conv_planes_kernel(
             continue;
         const int64_t at = (q0 + q) * c_pad + c0 + chunk * 8;
         if (fits) {
-            __half hi[8], lo[8];
+            __half2 hi[4], lo[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                split_half(tile[chunk * 8 + j][q] * scale, hi[j], lo[j]);
+            for (int j = 0; j < 4; ++j)
+                split_half_pair(tile[chunk * 8 + 2 * j][q] * scale, tile[chunk * 8 + 2 * j + 1][q] * scale, hi[j], lo[j]);
             __half *p_hi = reinterpret_cast<__half *>(slot) + at;
             *reinterpret_cast<uint4 *>(p_hi)         = *reinterpret_cast<uint4 *>(hi);
             *reinterpret_cast<uint4 *>(p_hi + plane) = *reinterpret_cast<uint4 *>(lo);
@@ -595,13 +601,15 @@ bool halo_geometry(int64_t h, int64_t w, int64_t kh, int64_t kw, int64_t pad, Ha
 
 } // namespace
 
-// Slices of an image in conv_range_kernel.
-int conv_range_slices(int64_t count) {
-    return (int)(count / 4096 < 1 ? 1 : (count / 4096 > 64 ? 64 : count / 4096));
+// Slices of an image in conv_range_kernel: 16 float4 to a thread where there are images enough, down to four where there
+// are few.
+int conv_range_slices(int64_t batch, int64_t count) {
+    const int64_t few = std::min<int64_t>(count / 4096, 1024 / batch);
+    return (int)std::min<int64_t>(64, std::max<int64_t>(1, std::max(count / 16384, few)));
 }
 
 // The pre-pass of a layer: the filters' scales and (filters16 non-null) planes, the images' planes and scales.
-// ranges: batch * conv_range_slices(c * hw) pairs of words.
+// ranges: batch * conv_range_slices(batch, c * hw) pairs of words.
 ct_status conv_prepass(
     DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t hw, int64_t c_pad, int64_t ko, int64_t taps,
     void *filters16, void *filters32, size_t plane16, size_t plane32, float *filter_scale, void *ranges, float *image_scale,
@@ -610,7 +618,7 @@ ct_status conv_prepass(
     if (batch > 65535 || c_pad / 32 > 65535)
         return fail(CT_ERR_TOO_LARGE, "conv2d: batch or channel count too large for the layout pre-pass");
     const int64_t count = c * hw;
-    const int slices    = conv_range_slices(count);
+    const int slices    = conv_range_slices(batch, count);
     const int vec       = (count & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
     uint8_t *f16 = static_cast<uint8_t *>(filters16), *f32 = static_cast<uint8_t *>(filters32);
     const FilterPlanes f{reinterpret_cast<__half *>(f16), reinterpret_cast<__half *>(f16 + plane16), reinterpret_cast<float *>(f32),
@@ -652,7 +660,7 @@ ct_status conv_halo(
     const size_t w16       = align_up((size_t)ko * taps * c_pad * 2), w32 = align_up((size_t)ko * taps * c_pad * 4);
     const size_t slot      = (size_t)hw * c_pad * 8;
     const size_t w_words   = align_up((size_t)ko * 4), x_words = align_up((size_t)batch * 4);
-    const size_t ranges    = align_up((size_t)batch * conv_range_slices(c * hw) * 8);
+    const size_t ranges    = align_up((size_t)batch * conv_range_slices(batch, c * hw) * 8);
     CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, w_words + x_words + ranges + 2 * w16 + 2 * w32 + (size_t)batch * slot));
     uint8_t *ws            = static_cast<uint8_t *>(st->gemm_ws);
     float *filter_scale    = reinterpret_cast<float *>(ws), *image_scale = reinterpret_cast<float *>(ws + w_words);

@@ -764,16 +764,12 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
             uint32_t v[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                __half part[2];
-#pragma unroll
-                for (int t = 0; t < 2; ++t) {
-                    const int ic  = c0 + 2 * j + t;
-                    const float x = (ch < p.ko && ic < p.c) ? src[ic * taps + tap] : 0.0f;
-                    __half hi, lo;
-                    split_half(x * scale, hi, lo);
-                    part[t] = lo_row ? lo : hi;
-                }
-                v[j] = *reinterpret_cast<uint32_t *>(part);
+                const int ic  = c0 + 2 * j;
+                const float a = (ch < p.ko && ic < p.c) ? src[ic * taps + tap] : 0.0f;
+                const float b = (ch < p.ko && ic + 1 < p.c) ? src[(ic + 1) * taps + tap] : 0.0f;
+                __half2 hi, lo;
+                split_half_pair(a * scale, b * scale, hi, lo);
+                v[j] = lo_row ? *reinterpret_cast<uint32_t *>(&lo) : *reinterpret_cast<uint32_t *>(&hi);
             }
             tmem_st_32x32_x8(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ks * 8), v);
         }
@@ -925,10 +921,7 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                             __half2 hi[4], lo[4];
 #pragma unroll
                             for (int t = 0; t < 4; ++t) {
-                                const float a = __fmul_rn(v[8 * j + 2 * t], scale), b = __fmul_rn(v[8 * j + 2 * t + 1], scale);
-                                hi[t] = __floats2half2_rn(a, b);
-                                lo[t] = __floats2half2_rn(__fmul_rn(__fsub_rn(a, __low2float(hi[t])), kHalfLoScale),
-                                                          __fmul_rn(__fsub_rn(b, __high2float(hi[t])), kHalfLoScale));
+                                split_half_pair(__fmul_rn(v[8 * j + 2 * t], scale), __fmul_rn(v[8 * j + 2 * t + 1], scale), hi[t], lo[t]);
                             }
                             const uint32_t at = row_off + (((uint32_t)(2 * half + j) ^ sw) << 4);
                             *reinterpret_cast<uint4 *>(x_hi + at) = *reinterpret_cast<uint4 *>(hi);
@@ -1274,7 +1267,7 @@ ct_status conv_tmem_filters(
     }
     auto align_up       = [](size_t v) { return (v + 1023) & ~(size_t)1023; };
     const size_t f_words = align_up((size_t)ko * 4), words = align_up((size_t)batch * 4), slot = (size_t)h * wd * 32 * 8;
-    const size_t ranges  = align_up((size_t)batch * conv_range_slices(c * h * wd) * 8);
+    const size_t ranges  = align_up((size_t)batch * conv_range_slices(batch, c * h * wd) * 8);
     CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, f_words + words + ranges + (size_t)batch * slot));
     uint8_t *ws = static_cast<uint8_t *>(st->gemm_ws), *planes = ws + f_words + words + ranges;
     float *image_scale = reinterpret_cast<float *>(ws + f_words);

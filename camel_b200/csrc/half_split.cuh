@@ -74,4 +74,10 @@ __device__ __forceinline__ bool split_half(float v, __half &hi, __half &lo) {
     return v != 0.0f && fabsf(v) < kHalfSmallest;
 }
 
+// Two scaled values of a range that fits (half_range_fits): finite, no exceptions.
+__device__ __forceinline__ void split_half_pair(float a, float b, __half2 &hi, __half2 &lo) {
+    hi = __floats2half2_rn(a, b);
+    lo = __floats2half2_rn(__fmul_rn(__fsub_rn(a, __low2float(hi)), kHalfLoScale), __fmul_rn(__fsub_rn(b, __high2float(hi)), kHalfLoScale));
+}
+
 } // namespace ct

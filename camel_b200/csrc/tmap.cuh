@@ -29,7 +29,7 @@ ct_status conv_tmem_filters(
 // conv2d with one input halo per tile and channel block serving every tap (conv_halo.cu).
 bool conv_halo_applicable(int64_t c_pad, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw, int64_t stride,
                           int64_t pad);
-int conv_range_slices(int64_t count);
+int conv_range_slices(int64_t batch, int64_t count);
 ct_status conv_prepass(
     DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t hw, int64_t c_pad, int64_t ko, int64_t taps,
     void *filters16, void *filters32, size_t plane16, size_t plane32, float *filter_scale, void *ranges, float *image_scale,
