@@ -27,18 +27,18 @@ enum FlagWord : int {
     FLAG_DIV_ZERO   = 0, // a divisor was 0 (reference: "Division by zero")
     FLAG_LOG_DOMAIN = 1, // an input of log was <= 0
     FLAG_TIMEOUT    = 2, // a bounded in-kernel wait ran out (value = 1 + the block that gave up)
-    FLAG_WIDE       = 4, // an operand of the product being prepared does not fit float16 pairs (half_split.cuh);
-                         // cleared by the product's own kernel
-    FLAG_WIDE_READERS = 5, // CTAs of that kernel that have read it
+    FLAG_EXCEPTION_READERS = 4, // CTAs of a product that have read the exceptions of its operands (half_split.cuh)
     FLAG_COUNT      = 8
 };
 
+struct HalfExceptions;
 struct DeviceState {
     bool ready           = false;
     int device           = -1;
     int sm_count         = 0;
     uint32_t *flags_dev  = nullptr; // FLAG_COUNT words
     uint32_t *flags_host = nullptr; // pinned mirror
+    struct HalfExceptions *exceptions_dev = nullptr; // of the operands of the product being prepared
     void *reduce_ws      = nullptr; // partials of the two-pass reductions
     size_t reduce_ws_bytes = 0;
     void *gemm_ws        = nullptr; // split operand planes of the tensor-core GEMM
@@ -187,6 +187,7 @@ struct PackedWeights {
     void *hi, *lo;
     void *hi16, *lo16; // float16 planes and inverse column scales; null: the matrix needs tf32
     float *scale;
+    HalfExceptions *exceptions; // of the float16 planes
 };
 constexpr uint32_t kPackedMagic = 0x43545057u; // "CTPW"
 
@@ -194,13 +195,15 @@ ct_status gemm_f32_tc(
     DeviceState *st, const float *a, const float *b, const float *bias, int64_t m, int64_t k,
     int64_t n, int act, float *out, const PackedWeights *packed = nullptr, bool a_is_km = false);
 // One operand of gemm_half (gemm_half.cu): K-major planes [rows][kp] of float16 pairs with an inverse scale
-// per row, and of tf32 terms, which are read instead where *wide is non-zero (or the caller forces it).
+// per row, and of tf32 terms, which are read instead where the exceptions say so (or the caller forces it).
 struct HalfOperand {
     const void *hi16, *lo16;
     const float *scale;
     const void *hi32, *lo32;
-    const uint32_t *wide;
+    HalfExceptions *exceptions;
+    int operand; // 0 left, 1 right: whose exceptions in the list are this one's
     int64_t rows;
+    int64_t line0 = 0; // the exceptions' line of row 0 (a row range of a packed operand)
 };
 // Row bands of one launch, see ct_matmul_packed_bands.
 struct HalfBands {
@@ -209,14 +212,14 @@ struct HalfBands {
     int64_t out_off[8];
     uint32_t *done = nullptr;
 };
-// out[z][m][n] = act(A . B[z]^T + bias) over prepared planes, B holding `batch` operands of b.rows / batch rows.  own_flag: the operands' word is FLAG_WIDE of the
-// device state, which the launch clears for the next product.
+// out[z][m][n] = act(A . B[z]^T + bias) over prepared planes, B holding `batch` operands of b.rows / batch rows.
+// Exceptions that are the device state's are cleared by the launch for the next product.
 ct_status gemm_half(
     DeviceState *st, const HalfOperand &a, const HalfOperand &b, int64_t kp, const float *bias, int act, float *out,
-    bool force_wide, bool own_flag, bool allow_splitk, const HalfBands *bands, int batch = 1, bool bias_per_row = false);
+    bool force_wide, bool allow_splitk, const HalfBands *bands, int batch = 1, bool bias_per_row = false);
 int half_tile_columns(const DeviceState *st, int64_t m, int64_t n, int64_t batch = 1);
-// Pre-passes: rows of a row-major matrix, columns of one (transposed planes); both raise *wide.  `zero`
-// words are cleared on the way (col_max of a following half_split_cols, which needs them at zero).
+// Pre-passes: rows of a row-major matrix, columns of one (transposed planes); both record exceptions.  `zero`
+// words are cleared on the way (scales and col_max of a following half_split_cols, which needs them at zero).
 // both_forms: the tf32 planes are written as well (no half_wide_planes needed).
 ct_status half_split_rows(
     DeviceState *st, const float *in, int64_t k, int64_t kp, const HalfOperand &o, bool both_forms, uint32_t *zero,
@@ -227,13 +230,11 @@ ct_status half_split_cols(
 ct_status half_split_both(
     DeviceState *st, const float *a, const HalfOperand &oa, const float *b, const HalfOperand &ob, int64_t k, int64_t kp,
     bool both_forms, bool *done);
-// tf32 planes of both operands where *wide is set (n == 0 / m == 0: that operand has them already).
+// tf32 planes of both operands where either needs them (n == 0 / m == 0: that operand has them already).
 ct_status half_wide_planes(
-    DeviceState *st, const uint32_t *wide, const float *a, int64_t m, bool a_is_km, void *a_hi, void *a_lo, const float *b,
+    DeviceState *st, const HalfExceptions *ea, const HalfExceptions *eb, const float *a, int64_t m, bool a_is_km, void *a_hi, void *a_lo, const float *b,
     int64_t n, void *b_hi, void *b_lo, int64_t k, int64_t kp);
-ct_status half_widen_rows(
-    DeviceState *st, const uint32_t *wide, const void *hi16, const void *lo16, const float *scale, int64_t rows, int64_t kp,
-    void *hi32, void *lo32);
+ct_status half_widen_rows(DeviceState *st, const HalfOperand &o, int64_t kp);
 // Geometry of a stride-1 convolution run as an implicit GEMM over NHWC input planes.
 struct ConvGeom {
     int c_pad;  // channels rounded up to the k-block

@@ -28,8 +28,8 @@ template <int MODE>
 __global__ void __launch_bounds__(256) im2col_planes_kernel(
     const float *__restrict__ x, int64_t c, int64_t h, int64_t w, int64_t kh, int64_t kw,
     int64_t stride, int64_t pad, int64_t ho, int64_t wo, int64_t kdim, int64_t kp, int64_t total,
-    void *__restrict__ p_hi, void *__restrict__ p_lo, const uint32_t *__restrict__ only_if) {
-    if (only_if && *reinterpret_cast<const volatile uint32_t *>(only_if) == 0)
+    void *__restrict__ p_hi, void *__restrict__ p_lo, const HalfExceptions *__restrict__ only_if) {
+    if (only_if && !half_wide(only_if, only_if))
         return; // the float16 planes of im2col_half_kernel hold the patches
     int64_t step = (int64_t)gridDim.x * 256;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += step) {
@@ -64,7 +64,7 @@ template <int V>
 __global__ void __launch_bounds__(256) im2col_half_kernel(
     const float *__restrict__ x, int c, int h, int w, int kh, int kw, int stride, int pad, int ho, int wo, int kdim, int kp,
     int64_t rows, __half *__restrict__ p_hi, __half *__restrict__ p_lo, float *__restrict__ scale_out,
-    uint32_t *__restrict__ wide) {
+    HalfExceptions *__restrict__ exceptions) {
     extern __shared__ int2 where[]; // element kk: offset from the patch's origin in its image, r << 16 | s
     griddep_launch_dependents();
     for (int kk = threadIdx.x; kk < kp; kk += 256) {
@@ -74,7 +74,6 @@ __global__ void __launch_bounds__(256) im2col_half_kernel(
     __syncthreads();
     griddep_wait();
     const int lane = threadIdx.x & 31, pix = ho * wo;
-    bool bad       = false;
     for (int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (int64_t)gridDim.x * 8) {
         const int img = (int)(row / pix), p = (int)(row - (int64_t)img * pix);
         const int oy = p / wo, y0 = oy * stride - pad, x0 = (p - oy * wo) * stride - pad;
@@ -85,7 +84,7 @@ __global__ void __launch_bounds__(256) im2col_half_kernel(
             return (iy >= 0 && iy < h && ix >= 0 && ix < w) ? __ldg(src + at.x) : 0.0f; // padding elements lie far outside
         };
         float2 v[V];
-        uint32_t mx = 0;
+        uint2 range = make_uint2(0u, kNoneSmallest);
         const bool fits = kp <= 64 * V;
         if (fits) {
 #pragma unroll
@@ -95,22 +94,32 @@ __global__ void __launch_bounds__(256) im2col_half_kernel(
             }
 #pragma unroll
             for (int j = 0; j < V; ++j)
-                mx = max(mx, max(finite_magnitude(v[j].x), finite_magnitude(v[j].y)));
+                range_take(range, v[j].x), range_take(range, v[j].y);
         } else {
             for (int kk = lane; kk < kdim; kk += 32)
-                mx = max(mx, finite_magnitude(load(kk)));
+                range_take(range, load(kk));
         }
-        mx = __reduce_max_sync(0xffffffffu, mx);
+        range             = range_warp(range);
+        const bool finite = range.x < 0x7f800000u;
+        if (!finite) { // rare: the scale is that of the finite values
+            range = make_uint2(0u, kNoneSmallest);
+            for (int kk = lane; kk < kdim; kk += 32)
+                range_take(range, isfinite(load(kk)) ? load(kk) : 0.0f);
+            range = range_warp(range);
+        }
         float scale, inverse;
-        bad |= !half_scale(mx, scale, inverse);
-        if (lane == 0)
-            scale_out[row] = inverse;
+        const bool ok    = half_scale(range.x, scale, inverse);
+        const bool plain = finite && (range.y == kNoneSmallest || __uint_as_float(range.y + 1u) * scale >= kHalfSmallest);
+        bool bad         = false;
         auto put = [&](int kk, float a, float b) {
-            __half hi[2], lo[2];
-            bad |= split_half(a * scale, hi[0], lo[0]);
-            bad |= split_half(b * scale, hi[1], lo[1]);
-            *reinterpret_cast<__half2 *>(p_hi + row * kp + kk) = *reinterpret_cast<__half2 *>(hi);
-            *reinterpret_cast<__half2 *>(p_lo + row * kp + kk) = *reinterpret_cast<__half2 *>(lo);
+            __half2 hi, lo;
+            split_half_pair(a * scale, b * scale, hi, lo);
+            if (!plain) {
+                split_half(a, scale, hi.x, lo.x);
+                split_half(b, scale, hi.y, lo.y);
+            }
+            *reinterpret_cast<__half2 *>(p_hi + row * kp + kk) = hi;
+            *reinterpret_cast<__half2 *>(p_lo + row * kp + kk) = lo;
         };
         if (fits) {
 #pragma unroll
@@ -121,9 +130,15 @@ __global__ void __launch_bounds__(256) im2col_half_kernel(
             for (int kk = 2 * lane; kk < kp; kk += 64)
                 put(kk, load(kk), load(kk + 1));
         }
+        if (!plain) // the patch is read once more
+            for (int kk = lane; kk < kp && !__all_sync(0xffffffffu, half_overfull(exceptions)); kk += 32)
+                bad |= half_record(exceptions, load(kk), scale, 1, row, kk);
+        if (lane == 0) {
+            scale_out[row] = bad ? -inverse : inverse;
+            if (!ok)
+                exceptions->wide = 1u;
+        }
     }
-    if (bad)
-        *wide = 1u;
 }
 
 // Weights [ko][c][kh][kw] -> A-operand planes [ko][taps * c_pad] with k = (r*kw + s) * c_pad + ic:
@@ -722,15 +737,14 @@ static ct_status conv2d_run(
     if (mode == 0 && c * h * wd <= 0x3fffffff && pix <= 0x3fffffff && n * pix <= 0x3fffffff && h < 0x3fff && wd < 0x3fff &&
         pad < 0x3fff && kh < 0x3fff && kw < 0x3fff && kp <= 4096) {
         // split float16: [w scale][patch scale][w hi16][w lo16][w hi][w lo][patches], the patches as float16
-        // pairs or, where the word says so, as tf32 planes in the same place
+        // pairs or, where the exceptions say so, as tf32 planes in the same place
         const size_t w16 = align_up((size_t)ko * kp * 2), p16 = align_up((size_t)n * pix * kp * 2);
         const size_t w_words = align_up((size_t)ko * 4), p_words = align_up((size_t)n * pix * 4);
         CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, w_words + p_words + 2 * w16 + 2 * w_plane + 2 * p_plane));
         uint8_t *ws     = static_cast<uint8_t *>(st->gemm_ws);
         uint8_t *planes = ws + w_words + p_words, *w32 = planes + 2 * w16, *patches = w32 + 2 * w_plane;
-        uint32_t *wide  = st->flags_dev + FLAG_WIDE;
-        HalfOperand oa{planes, planes + w16, reinterpret_cast<float *>(ws), w32, w32 + w_plane, wide, ko};
-        HalfOperand ob{patches, patches + p16, reinterpret_cast<float *>(ws + w_words), patches, patches + p_plane, wide, n * pix};
+        HalfOperand oa{planes, planes + w16, reinterpret_cast<float *>(ws), w32, w32 + w_plane, st->exceptions_dev, 0, ko};
+        HalfOperand ob{patches, patches + p16, reinterpret_cast<float *>(ws + w_words), patches, patches + p_plane, st->exceptions_dev, 1, n * pix};
         {
             ProfScope prof("im2col");
             CT_TRY(half_split_rows(st, w, kdim, kp, oa, true, nullptr, 0));
@@ -739,7 +753,7 @@ static ct_status conv2d_run(
     CT_CUDA(launch_dependent(im2col_half_kernel<V>, dim3(blocks), dim3(256), (size_t)kp * sizeof(int2), stream(), x, (int)c, \
                              (int)h, (int)wd, (int)kh, (int)kw, (int)stride, (int)pad, (int)ho, (int)wo, (int)kdim, (int)kp,  \
                              n * pix, reinterpret_cast<__half *>(patches), reinterpret_cast<__half *>(patches + p16),       \
-                             const_cast<float *>(ob.scale), wide))
+                             const_cast<float *>(ob.scale), ob.exceptions))
             if (kp <= 256)
                 CT_PATCHES(4);
             else if (kp <= 512)
@@ -749,10 +763,10 @@ static ct_status conv2d_run(
 #undef CT_PATCHES
             CT_LAUNCH_CHECK("im2col_half");
             im2col_planes_kernel<0><<<capped_blocks(st, n * pix * kp, 4), 256, 0, stream()>>>(
-                x, c, h, wd, kh, kw, stride, pad, ho, wo, kdim, kp, n * pix * kp, patches, patches + p_plane, wide);
+                x, c, h, wd, kh, kw, stride, pad, ho, wo, kdim, kp, n * pix * kp, patches, patches + p_plane, st->exceptions_dev);
             CT_LAUNCH_CHECK("im2col_planes");
         }
-        return gemm_half(st, oa, ob, kp, bias, act, out, false, true, false, nullptr, (int)n, true);
+        return gemm_half(st, oa, ob, kp, bias, act, out, false, false, nullptr, (int)n, true);
     }
     CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, planes * (w_plane + p_plane)));
     uint8_t *ws = static_cast<uint8_t *>(st->gemm_ws);

@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(256) conv_range_kernel(
         const int tap = i / c_pad, ic = i - tap * c_pad;
         const float v    = ic < c ? src[ic * taps + tap] : 0.0f;
         const int64_t at = o * taps * c_pad + i;
-        split_half(v * scale, f.hi16[at], f.lo16[at]);
+        split_half(v, scale, f.hi16[at], f.lo16[at]);
         split_tf32(v, f.hi32[at], f.lo32[at]);
     }
 }

@@ -12,8 +12,9 @@
 // every addition - is a sixth per value of k of what the single 3xTF32 accumulator collects.  It is
 // drained into registers every 1024 values of k and summed there with round-to-nearest adds.
 //
-// Matrices whose rows span too many powers of two for float16 raise a device word in the pre-pass.  The
-// wide_planes kernel (which returns at once otherwise) then writes tf32 planes, and the GEMM kernel runs
+// Values that float16 pairs hold in fewer bits than tf32 pairs would are listed by the pre-pass, and their products
+// are added in the epilogue of the rows and columns they belong to.  Where there are too many for that, the
+// wide_planes kernel (which returns at once otherwise) writes tf32 planes, and the GEMM kernel runs
 // the same loop over those: same stage layout, same descriptors, kind::tf32, 8 values of k per MMA, all
 // three products into one accumulator drained every 256 values of k.
 //
@@ -68,17 +69,20 @@ struct HalfGemmParams {
     int group_m;            // row tiles that sweep the column tiles together
     int total_tiles;
     int batch;              // > 1: B holds that many right operands of n rows each, outputs out_batch_stride apart
-    const float *row_scale; // [m]: inverse scale of each row of A
+    const float *row_scale; // [m]: inverse scale of each row of A, negative for a row with exceptions
     const float *col_scale; // [batch][n]
+    const __half *a_hi, *a_lo, *b_hi, *b_lo; // the float16 planes and lists, for those rows
+    int kp;
+    HalfExceptions *exceptions_a, *exceptions_b;
+    int a_line0;
     const float *bias;
     int bias_per_row;       // bias indexed by output row
     int act;
     float *out;
     int64_t out_batch_stride;
     uint32_t *flags;
-    const uint32_t *wide_a, *wide_b; // device words: non-zero = the tf32 planes hold the operands
-    int force_wide;
-    int reset_flags;                 // the words are the library's own: the last CTA clears them
+    int force_wide;                         // the tf32 planes hold the operands, whatever the exceptions say
+    HalfExceptions *reset;                  // the library's own list, if one of them is that: the last CTA clears it
     // row bands, see ct_matmul_packed_bands
     int bands;
     int band_first[9];
@@ -118,6 +122,140 @@ __device__ __forceinline__ void half_tile(const HalfGemmParams &p, int tile, int
     tn                  = in_group / gm;
 }
 
+// ---- exceptions (half_split.cuh) -------------------------------------------------------------
+//
+// exception_a . b + held_a . exception_b is what the accumulators lack of an output whose row or column has
+// exceptions, the planes holding zeros in their place.  Sums run in order of k, whatever order the pre-pass found them in.
+
+__device__ __forceinline__ float half_held(const __half *hi, const __half *lo, int64_t at, float inverse) {
+    return (__half2float(hi[at]) + __half2float(lo[at]) * kHalfLoInv) * fabsf(inverse);
+}
+// Entry of a line with the smallest k above `after`, -1 if there is none.
+__device__ __forceinline__ int half_next(const HalfExceptions *x, int n, int operand, int64_t line, int after) {
+    int best = -1, best_k = 0;
+    for (int i = 0; i < n; ++i) {
+        const int l = x->e[i].line, k = x->e[i].k;
+        if (l == line * 2 + operand && k > after && (best < 0 || k < best_k))
+            best = i, best_k = k;
+    }
+    return best;
+}
+
+// What `count` outputs of row `row` lack, columns (lines of B) line + 32 g for g < count, into sum[].
+template <int G>
+__device__ __forceinline__ void half_missing(
+    const HalfGemmParams &p, int64_t row, bool a_has, int64_t line, int count, float (&sum)[G]) {
+    const HalfExceptions *xa = p.exceptions_a, *xb = p.exceptions_b;
+    const int nb = (int)xb->count;
+    float sc[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+        sum[g] = 0.0f, sc[g] = g < count ? p.col_scale[line + 32 * g] : 1.0f;
+    if (a_has) {
+        const int na = (int)xa->count;
+        for (int k = -1, i; (i = half_next(xa, na, 0, row + p.a_line0, k)) >= 0;) {
+            k             = xa->e[i].k;
+            const float a = xa->e[i].value;
+            float b[G];
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+                b[g] = g < count ? half_held(p.b_hi, p.b_lo, (line + 32 * g) * p.kp + k, sc[g]) : 0.0f;
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                if (sc[g] < 0.0f) {
+                    const int j = half_next(xb, nb, 1, line + 32 * g, k - 1);
+                    if (j >= 0 && xb->e[j].k == k)
+                        b[g] += xb->e[j].value;
+                }
+                sum[g] = __fmaf_rn(a, b[g], sum[g]);
+            }
+        }
+    }
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+        if (sc[g] < 0.0f)
+            for (int k = -1, j; (j = half_next(xb, nb, 1, line + 32 * g, k)) >= 0;) {
+                k      = xb->e[j].k;
+                sum[g] = __fmaf_rn(half_held(p.a_hi, p.a_lo, row * p.kp + k, p.row_scale[row]), xb->e[j].value, sum[g]);
+            }
+}
+
+// Finishes what a warp has stored without bias and activation because it lacks the exceptions' products: the rows and
+// columns of its 32 x (32 G) block that have exceptions.  Called when the tile's sums are out of registers: a call among the stores cost
+// every tile 300 bytes of spills.  Only these outputs are read back, a row at once: one exception in 1537 x 771 x 2050
+// costs its tile about 3 us.
+template <int G>
+__device__ __noinline__ void half_finish(
+    const HalfGemmParams &p, float *out_z, int64_t row0, int rows, int64_t col0, int64_t line0, bool add) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp(); // the stores of the other lanes
+    auto finish = [&](float x, float missing, int64_t row, int64_t col) {
+        if (add) // once, where k is sliced
+            x = __fadd_rn(x, missing);
+        if (p.bias)
+            x = __fadd_rn(x, p.bias[p.bias_per_row ? row : col]);
+        if (p.act == CT_ACT_RELU)
+            x = __fmul_rn(x, x > 0.0f ? 1.0f : 0.0f);
+        out_z[row * p.n + col] = x;
+    };
+    const bool row_has      = lane < rows && p.row_scale[row0 + lane] < 0.0f;
+    const uint32_t row_mask = __ballot_sync(0xffffffffu, row_has);
+    const int64_t col       = col0 + lane;
+    const int count         = (int)(p.n <= col ? 0 : min((int64_t)G, (p.n - col + 31) / 32));
+    for (uint32_t m = row_mask; m; m &= m - 1) {
+        const int64_t row = row0 + __ffs(m) - 1;
+        float x[G], missing[G];
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+            x[g] = g < count ? out_z[row * p.n + col + 32 * g] : 0.0f;
+        half_missing<G>(p, row, true, line0 + col, count, missing);
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+            if (g < count)
+                finish(x[g], missing[g], row, col + 32 * g);
+    }
+    for (int g = 0; g < G; ++g)
+        for (uint32_t m = __ballot_sync(0xffffffffu, g < count && p.col_scale[line0 + col + 32 * g] < 0.0f); m; m &= m - 1) { // lane = row
+            const int64_t c = col0 + 32 * g + __ffs(m) - 1;
+            if (lane < rows && !row_has) {
+                float missing[1];
+                const float x = out_z[(row0 + lane) * p.n + c];
+                half_missing<1>(p, row0 + lane, false, line0 + c, 1, missing);
+                finish(x, missing[0], row0 + lane, c);
+            }
+        }
+}
+
+// A tile added up by its cluster, where a row or column of it has exceptions: rows r0 .. of the tile at (row0, col0),
+// whose slices' sums lie at `sums` in the CTAs.
+__device__ __noinline__ void half_finish_slices(
+    const HalfGemmParams &p, uint32_t sums, int slices, int r0, int rows, int64_t row0, int64_t col0, int bn) {
+    for (int i = threadIdx.x; i < rows * bn; i += kHThreads) {
+        const int r = r0 + i / bn, c = i % bn;
+        const int64_t row = row0 + r, col = col0 + c;
+        if (row >= p.m || col >= p.n)
+            continue;
+        float x = 0.0f;
+        for (int z = 0; z < slices; ++z) {
+            const float4 q = ld_cluster_f4(sums + (uint32_t)r * (uint32_t)(bn * 4) + (uint32_t)(((c >> 2) ^ (r & 7)) << 4), (uint32_t)z);
+            const float v  = (c & 2) ? ((c & 1) ? q.w : q.z) : ((c & 1) ? q.y : q.x);
+            x              = z == 0 ? v : __fadd_rn(x, v);
+        }
+        float missing[1];
+        const float cs = p.col_scale[col], rs = p.row_scale[row];
+        x = __fmul_rn(x, fabsf(cs));
+        if (rs < 0.0f || cs < 0.0f) {
+            half_missing<1>(p, row, rs < 0.0f, col, 1, missing);
+            x = __fadd_rn(x, missing[0]);
+        }
+        if (p.bias)
+            x = __fadd_rn(x, p.bias[p.bias_per_row ? row : col]);
+        if (p.act == CT_ACT_RELU)
+            x = __fmul_rn(x, x > 0.0f ? 1.0f : 0.0f);
+        p.out[row * p.n + col] = x;
+    }
+}
+
 template <int BN, int CG>
 __global__ void __launch_bounds__(kHThreads, 1)
     gemm_half_kernel(const __grid_constant__ HalfMaps maps, const __grid_constant__ HalfGemmParams p) {
@@ -137,7 +275,7 @@ __global__ void __launch_bounds__(kHThreads, 1)
     __shared__ uint64_t bar_acc_full[2 * C::kSets], bar_acc_empty[2 * C::kSets];
     __shared__ uint64_t bar_done;
     __shared__ uint32_t tmem_base_slot;
-    __shared__ int abort_flag_s;
+    __shared__ int abort_flag_s, lacking_s;
     // epilogue warps that have stored a tile (bands only), a counter per tile that may be under way: accumulators
     // are handed back before the store, so a warp can be kSets tiles ahead of another (one that has no columns to
     // store always is)
@@ -166,6 +304,7 @@ __global__ void __launch_bounds__(kHThreads, 1)
         mbar_init(smem_u32(&bar_done), 1);
         mbar_fence_init();
         tile_stores[0] = tile_stores[1] = tile_stores[2] = tile_stores[3] = 0;
+        lacking_s = 0;
         prefetch_tensormap(&maps.a16_hi);
         prefetch_tensormap(&maps.a16_lo);
         prefetch_tensormap(&maps.b16_hi);
@@ -191,8 +330,7 @@ __global__ void __launch_bounds__(kHThreads, 1)
     // everything above is set-up that does not depend on earlier kernels; the planes, the words and the
     // output may
     griddep_wait();
-    const bool wide = p.force_wide || *reinterpret_cast<const volatile uint32_t *>(p.wide_a) != 0 ||
-                      *reinterpret_cast<const volatile uint32_t *>(p.wide_b) != 0;
+    const bool wide = p.force_wide || half_wide(p.exceptions_a, p.exceptions_b);
     const int k_step    = wide ? RB / 4 : RB / 2; // values of k per stage
     const int per_group = 64 / k_step;            // stages per 64 values of k
     const int chunk     = (wide ? kChunkWide : kChunkHalf) / k_step;
@@ -383,14 +521,19 @@ __global__ void __launch_bounds__(kHThreads, 1)
             // handed round by shuffles when the tile is stored (no barrier between the epilogue warps: after
             // a failed wait they leave one by one)
             float cs[C::kCols / 32], bb[C::kCols / 32];
+            bool lacking = false; // a row or column of this warp's has exceptions
 #pragma unroll
             for (int g = 0; g < C::kCols / 32; ++g) {
                 const int64_t col = tile_c0 + half * C::kCols + g * 32 + lane;
                 cs[g]             = (!wide && col < p.n) ? p.col_scale[(p.batch > 1 ? tz * p.n : 0) + col] : 1.0f;
+                lacking |= cs[g] < 0.0f;
+                cs[g] = fabsf(cs[g]);
                 bb[g]             = (p.bias && !p.bias_per_row && col < p.n) ? p.bias[col] : 0.0f;
             }
             const float row_bias = (p.bias_per_row && row0 + lane < p.m) ? p.bias[row0 + lane] : 0.0f;
-            const float rs = (!wide && row0 + lane < p.m) ? p.row_scale[row0 + lane] : 1.0f;
+            float rs = (!wide && row0 + lane < p.m) ? p.row_scale[row0 + lane] : 1.0f;
+            lacking  = __any_sync(0xffffffffu, lacking || rs < 0.0f);
+            rs       = fabsf(rs);
 
             float acc[C::kCols];
             const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(set * 2 * BN + half * C::kCols);
@@ -457,6 +600,8 @@ __global__ void __launch_bounds__(kHThreads, 1)
                 break;
 
             if (slices > 1) {
+                if (lacking && lane == 0)
+                    lacking_s = 1; // every slice sees the same rows and columns
                 // this slice's 128 x 128 sums go to the idle operand stages (every MMA has retired), rows of 512
                 // bytes, float4 slots XOR-swizzled; the cluster adds them up below
                 uint8_t *part = smem_raw + (smem_base - smem_u32(smem_raw)) + (uint32_t)(quarter * 32 + lane) * (BN * 4u);
@@ -529,8 +674,19 @@ __global__ void __launch_bounds__(kHThreads, 1)
                             dst[(int64_t)r * p.n] = x;
                     }
                 }
+                if (lacking) { // their outputs without bias and activation again: half_finish has the rest
+                    const bool col_has      = lane < cols_left && p.col_scale[(p.batch > 1 ? tz * p.n : 0) + tile_c0 + c0 + lane] < 0.0f;
+                    const uint32_t row_mask = __ballot_sync(0xffffffffu, lane < rows_left && p.row_scale[row0 + lane] < 0.0f);
+#pragma unroll 1
+                    for (int r = 0; r < rows_left; ++r)
+                        if (((row_mask >> r & 1u) || col_has) && lane < cols_left)
+                            out_z[(row0 + r) * p.n + tile_c0 + c0 + lane] = __fmul_rn(
+                                *reinterpret_cast<const float *>(stg + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4), cs[g]);
+                }
                 __syncwarp(); // the block is rewritten by the next 32 columns
             }
+            if (lacking)
+                half_finish<C::kCols / 32>(p, out_z, row0, rows_left, tile_c0 + half * C::kCols, p.batch > 1 ? tz * p.n : 0, first_group == 0);
             if (p.bands > 0) {
                 // the last warp to have stored the tile counts it; tile i + 4 comes to the same counter only after
                 // every warp is past tile i
@@ -554,7 +710,9 @@ __global__ void __launch_bounds__(kHThreads, 1)
         half_tile(p, first, tm, tn, tz, band);
         const int rows_each = kHM / slices;
         const bool vec      = (p.n & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
-        if (!failed && !abort_flag_s)
+        if (!failed && !abort_flag_s && lacking_s)
+            half_finish_slices(p, smem_base, slices, (int)cluster_rank() * rows_each, rows_each, (int64_t)tm * kHM, (int64_t)tn * BN, BN);
+        else if (!failed && !abort_flag_s)
             for (int i = threadIdx.x; i < rows_each * (BN / 4); i += kHThreads) {
                 const int r = (int)cluster_rank() * rows_each + i / (BN / 4), slot = i % (BN / 4);
                 const int64_t row = (int64_t)tm * kHM + r, col = (int64_t)tn * BN + slot * 4;
@@ -614,11 +772,11 @@ __global__ void __launch_bounds__(kHThreads, 1)
                 atomicAdd(p.band_done + band, 1u);
             }
         }
-        if (p.reset_flags) {
-            // the last CTA to get here clears the pre-pass's word for the next product
-            if (atomicAdd(p.flags + FLAG_WIDE_READERS, 1u) + 1u == gridDim.x) {
-                p.flags[FLAG_WIDE_READERS] = 0u;
-                p.flags[FLAG_WIDE]         = 0u;
+        if (p.reset) {
+            // the last CTA to get here clears it for the next product
+            if (atomicAdd(p.flags + FLAG_EXCEPTION_READERS, 1u) + 1u == gridDim.x) {
+                p.flags[FLAG_EXCEPTION_READERS] = 0u;
+                p.reset->wide = p.reset->count = 0u;
             }
         }
     }
@@ -626,20 +784,45 @@ __global__ void __launch_bounds__(kHThreads, 1)
 
 // ---- operand pre-pass ---------------------------------------------------------------------
 
-// What a pre-pass writes: float16 planes, inverse scales, the word for rows that do not fit them and, for
+// What a pre-pass writes: float16 planes, inverse scales (negative: a row with exceptions), the exceptions and, for
 // small operands (hi32 non-null), the tf32 planes as well, which then need no launch of their own.
 struct HalfPlanes {
     __half *hi16, *lo16;
     float *scale;
-    uint32_t *wide;
+    HalfExceptions *exceptions;
+    int operand;
     float *hi32, *lo32;
 };
 
 HalfPlanes planes_of(const HalfOperand &o, bool both_forms) {
     return HalfPlanes{static_cast<__half *>(const_cast<void *>(o.hi16)), static_cast<__half *>(const_cast<void *>(o.lo16)),
-                      const_cast<float *>(o.scale), const_cast<uint32_t *>(o.wide),
+                      const_cast<float *>(o.scale), o.exceptions, o.operand,
                       both_forms ? static_cast<float *>(const_cast<void *>(o.hi32)) : nullptr,
                       both_forms ? static_cast<float *>(const_cast<void *>(o.lo32)) : nullptr};
+}
+
+// A line whose range is not plain - it has exceptions, infinities or NaN - is split as if it had none and then put
+// right here: zeros and an entry in the list for each exception, no low term for the others.  Called by `threads`
+// threads, whole warps; true if there are exceptions.
+__device__ __noinline__ bool half_repair(
+    const float *src, int64_t stride, int64_t k, float scale, __half *hi, __half *lo, HalfExceptions *x, int operand, int64_t line, int t,
+    int threads) {
+    bool found = false;
+    for (int64_t c = t; __any_sync(0xffffffffu, c < k); c += threads) {
+        if (__all_sync(0xffffffffu, half_overfull(x)))
+            return true; // the planes will not be read
+        const float v = c < k ? src[c * stride] : 0.0f;
+        found |= half_record(x, v, scale, operand, line, c);
+        if (half_exception(v, scale))
+            hi[c] = __half(0.0f), lo[c] = __half(0.0f);
+        else if (!isfinite(v))
+            lo[c] = __half(0.0f);
+    }
+    return found;
+}
+// Whether a line with this range (half_split.cuh) and scale needs it.
+__device__ __forceinline__ bool half_not_plain(uint2 range, float scale) {
+    return range.x >= 0x7f800000u || (range.y != kNoneSmallest && __uint_as_float(range.y + 1u) * scale < kHalfSmallest);
 }
 
 // in [rows][k] -> float16 planes [rows][kp], inverse row scales.  TPR threads per row keep the row in
@@ -648,7 +831,7 @@ HalfPlanes planes_of(const HalfOperand &o, bool both_forms) {
 template <int TPR, int V>
 __device__ __forceinline__ void half_rows(
     int64_t block, const float *__restrict__ in, int64_t rows, int64_t k, int64_t kp, const HalfPlanes &p, int vec_ok) {
-    __shared__ uint32_t max_s[8];
+    __shared__ uint2 range_s[8];
     constexpr int RPB = 256 / TPR;
     const int t       = threadIdx.x % TPR;
     const int64_t row = block * RPB + threadIdx.x / TPR;
@@ -666,10 +849,20 @@ __device__ __forceinline__ void half_rows(
         return q;
     };
     float4 v[V];
-    uint32_t mx = 0;
+    uint2 range = make_uint2(0u, kNoneSmallest);
     auto take   = [&](const float4 &q) {
-        mx = max(max(mx, max(finite_magnitude(q.x), finite_magnitude(q.y))),
-                 max(finite_magnitude(q.z), finite_magnitude(q.w)));
+        range_take(range, q.x), range_take(range, q.y), range_take(range, q.z), range_take(range, q.w);
+    };
+    auto reduce = [&]() {
+        range = range_warp(range);
+        if (TPR == 256) {
+            if ((threadIdx.x & 31) == 0)
+                range_s[threadIdx.x >> 5] = range;
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < 8; ++w)
+                range = range_join(range, range_s[w]);
+        }
     };
     const bool fits = kp <= TPR * V * 4;
     if (fits) {
@@ -685,25 +878,22 @@ __device__ __forceinline__ void half_rows(
         for (int64_t c = t * 4; c < k; c += TPR * 4)
             take(load(c));
     }
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if (TPR == 256) {
-        if ((threadIdx.x & 31) == 0)
-            max_s[threadIdx.x >> 5] = mx;
-        __syncthreads();
-#pragma unroll
-        for (int w = 0; w < 8; ++w)
-            mx = max(mx, max_s[w]);
+    reduce();
+    const bool finite = range.x < 0x7f800000u;
+    if (!finite) { // rare: the scale is that of the finite values
+        if (TPR == 256)
+            __syncthreads();
+        range = make_uint2(0u, kNoneSmallest);
+        for (int64_t c = t; c < k; c += TPR)
+            range_take(range, isfinite(src[c]) ? src[c] : 0.0f);
+        reduce();
     }
     float scale, inverse;
-    bool bad = !half_scale(mx, scale, inverse);
-    if (t == 0)
-        p.scale[row] = inverse;
-    auto put = [&](int64_t c, const float4 &q) {
-        __half hi[4], lo[4];
-        bad |= split_half(q.x * scale, hi[0], lo[0]);
-        bad |= split_half(q.y * scale, hi[1], lo[1]);
-        bad |= split_half(q.z * scale, hi[2], lo[2]);
-        bad |= split_half(q.w * scale, hi[3], lo[3]);
+    const bool ok = half_scale(range.x, scale, inverse);
+    auto put      = [&](int64_t c, const float4 &q) {
+        __half2 hi[2], lo[2];
+        split_half_pair(q.x * scale, q.y * scale, hi[0], lo[0]);
+        split_half_pair(q.z * scale, q.w * scale, hi[1], lo[1]);
         *reinterpret_cast<uint2 *>(p.hi16 + row * kp + c) = *reinterpret_cast<uint2 *>(hi);
         *reinterpret_cast<uint2 *>(p.lo16 + row * kp + c) = *reinterpret_cast<uint2 *>(lo);
         if (p.hi32) {
@@ -727,8 +917,21 @@ __device__ __forceinline__ void half_rows(
         for (int64_t c = t * 4; c < kp; c += TPR * 4)
             put(c, c < k ? load(c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f));
     }
-    if (bad)
-        *p.wide = 1u;
+    bool bad = false;
+    if (!finite || half_not_plain(range, scale)) { // rare, and the same for all threads of the row
+        if (TPR == 256)
+            __syncthreads();
+        else
+            __syncwarp();
+        bad = half_repair(src, 1, k, scale, p.hi16 + row * kp, p.lo16 + row * kp, p.exceptions, p.operand, row, t, TPR);
+        if (TPR == 256)
+            bad = __syncthreads_or(bad) != 0;
+    }
+    if (t == 0) {
+        p.scale[row] = bad ? -inverse : inverse;
+        if (!ok)
+            p.exceptions->wide = 1u;
+    }
 }
 
 template <int TPR, int V>
@@ -738,7 +941,7 @@ __global__ void __launch_bounds__(256) half_rows_kernel(
     griddep_launch_dependents();
     griddep_wait();
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < zero_count; i += (int64_t)gridDim.x * 256)
-        zero[i] = 0u; // the column maxima of the right operand, accumulated by the next kernel
+        zero[i] = 0u; // scales and column maxima of the right operand, accumulated by the next kernels
     half_rows<TPR, V>((int64_t)blockIdx.x, in, rows, k, kp, p, vec_ok);
 }
 
@@ -766,7 +969,8 @@ __global__ void __launch_bounds__(256) half_col_max_kernel(
     }
 }
 
-// in [k][n] -> transposed float16 planes [n][kp], inverse column scales.  Blocks of 64 k x 32 columns.
+// in [k][n] -> transposed float16 planes [n][kp], inverse column scales.  Blocks of 64 k x 32 columns, a warp to a
+// column: the first block of a column writes its scale, any of them its sign (both by OR, the scales start at zero).
 __global__ void __launch_bounds__(256) half_cols_kernel(
     const float *__restrict__ in, int64_t k, int64_t n, int64_t kp, const HalfPlanes p, const uint32_t *__restrict__ col_max) {
     __shared__ float tile[64][33];
@@ -780,21 +984,30 @@ __global__ void __launch_bounds__(256) half_cols_kernel(
         tile[ty + j * 8][tx] = (kk < k && nn < n) ? in[kk * n + nn] : 0.0f;
     }
     __syncthreads();
-    bool bad = false;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const int64_t nn = n0 + ty + j * 8, kk = k0 + tx * 2;
-        if (nn < n && kk < kp) {
-            float scale, inverse;
-            bad |= !half_scale(col_max[nn], scale, inverse);
-            if (blockIdx.y == 0 && tx == 0)
-                p.scale[nn] = inverse;
-            const float v0 = tile[tx * 2][ty + j * 8], v1 = tile[tx * 2 + 1][ty + j * 8];
-            __half hi[2], lo[2];
-            bad |= split_half(v0 * scale, hi[0], lo[0]);
-            bad |= split_half(v1 * scale, hi[1], lo[1]);
-            *reinterpret_cast<__half2 *>(p.hi16 + nn * kp + kk) = *reinterpret_cast<__half2 *>(hi);
-            *reinterpret_cast<__half2 *>(p.lo16 + nn * kp + kk) = *reinterpret_cast<__half2 *>(lo);
+        if (nn >= n)
+            break; // the whole warp
+        float scale, inverse;
+        const bool ok  = half_scale(col_max[nn], scale, inverse);
+        const float v0 = tile[tx * 2][ty + j * 8], v1 = tile[tx * 2 + 1][ty + j * 8];
+        uint32_t *word = reinterpret_cast<uint32_t *>(p.scale + nn);
+        if (blockIdx.y == 0 && tx == 0) {
+            atomicOr(word, __float_as_uint(inverse));
+            if (!ok)
+                p.exceptions->wide = 1u;
+        }
+        const bool special = half_exception(v0, scale) || half_exception(v1, scale) || !isfinite(v0) || !isfinite(v1);
+        if (kk < kp) {
+            __half2 hi, lo;
+            split_half_pair(v0 * scale, v1 * scale, hi, lo);
+            if (special) {
+                split_half(v0, scale, hi.x, lo.x);
+                split_half(v1, scale, hi.y, lo.y);
+            }
+            *reinterpret_cast<__half2 *>(p.hi16 + nn * kp + kk) = hi;
+            *reinterpret_cast<__half2 *>(p.lo16 + nn * kp + kk) = lo;
             if (p.hi32) {
                 float2 h, l;
                 split_tf32_flat(v0, h.x, l.x);
@@ -803,9 +1016,13 @@ __global__ void __launch_bounds__(256) half_cols_kernel(
                 *reinterpret_cast<float2 *>(p.lo32 + nn * kp + kk) = l;
             }
         }
+        if (__any_sync(0xffffffffu, special)) {
+            bool found = half_record(p.exceptions, v0, scale, p.operand, nn, kk);
+            found |= half_record(p.exceptions, v1, scale, p.operand, nn, kk + 1);
+            if (found && tx == 0)
+                atomicOr(word, 0x80000000u);
+        }
     }
-    if (bad)
-        *p.wide = 1u;
 }
 
 // The same for k <= kShortK in one pass: a block keeps the whole length of 8 columns (32 bytes of each row, a
@@ -826,24 +1043,28 @@ __device__ __forceinline__ void half_cols_short(
         tile[kk * kShortPad + tx] = (col_ok && kk < k) ? src[(int64_t)kk * n] : 0.0f;
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t mx    = 0;
+    uint2 range    = make_uint2(0u, kNoneSmallest);
     for (int kk = lane; kk < (int)kp; kk += 32)
-        mx = max(mx, finite_magnitude(tile[kk * kShortPad + warp]));
-    mx = __reduce_max_sync(0xffffffffu, mx);
+        range_take(range, tile[kk * kShortPad + warp]);
+    range             = range_warp(range);
+    const bool finite = range.x < 0x7f800000u;
+    if (!finite) {
+        range = make_uint2(0u, kNoneSmallest);
+        for (int kk = lane; kk < (int)kp; kk += 32)
+            range_take(range, isfinite(tile[kk * kShortPad + warp]) ? tile[kk * kShortPad + warp] : 0.0f);
+        range = range_warp(range);
+    }
     float scale, inverse;
-    bool bad         = !half_scale(mx, scale, inverse);
+    const bool ok    = half_scale(range.x, scale, inverse);
     const int64_t nn = n0 + warp;
     if (nn >= n)
         return;
-    if (lane == 0)
-        p.scale[nn] = inverse;
     for (int kk = lane * 2; kk < (int)kp; kk += 64) {
-        __half hi[2], lo[2];
+        __half2 hi, lo;
         const float v0 = tile[kk * kShortPad + warp], v1 = tile[(kk + 1) * kShortPad + warp];
-        bad |= split_half(v0 * scale, hi[0], lo[0]);
-        bad |= split_half(v1 * scale, hi[1], lo[1]);
-        *reinterpret_cast<__half2 *>(p.hi16 + nn * kp + kk) = *reinterpret_cast<__half2 *>(hi);
-        *reinterpret_cast<__half2 *>(p.lo16 + nn * kp + kk) = *reinterpret_cast<__half2 *>(lo);
+        split_half_pair(v0 * scale, v1 * scale, hi, lo);
+        *reinterpret_cast<__half2 *>(p.hi16 + nn * kp + kk) = hi;
+        *reinterpret_cast<__half2 *>(p.lo16 + nn * kp + kk) = lo;
         if (p.hi32) {
             float2 h, l;
             split_tf32_flat(v0, h.x, l.x);
@@ -852,8 +1073,16 @@ __device__ __forceinline__ void half_cols_short(
             *reinterpret_cast<float2 *>(p.lo32 + nn * kp + kk) = l;
         }
     }
-    if (bad)
-        *p.wide = 1u;
+    bool bad = false;
+    if (!finite || half_not_plain(range, scale)) {
+        __syncwarp();
+        bad = half_repair(in + nn, n, k, scale, p.hi16 + nn * kp, p.lo16 + nn * kp, p.exceptions, p.operand, nn, lane, 32);
+    }
+    if (lane == 0) {
+        p.scale[nn] = bad ? -inverse : inverse;
+        if (!ok)
+            p.exceptions->wide = 1u;
+    }
 }
 
 __global__ void __launch_bounds__(256) half_cols_short_kernel(
@@ -879,7 +1108,9 @@ __global__ void __launch_bounds__(256) half_both_kernel(
         half_cols_short(tile_short, (int)blockIdx.x - row_blocks, b, k, n, kp, pb);
 }
 
-// The tf32 planes of operands that float16 pairs cannot hold; returns at once where *wide is 0.
+// The tf32 planes of operands that float16 pairs cannot hold; returns at once where both can be held.  Blocks of 64 k
+// x 64 rows, sixteen loads to a thread in flight, two blocks to an SM: with four loads the pass took 57 us for
+// 4096 x 1024 x 1024, and more blocks make the idle launch longer.
 struct WideOperand {
     const float *in;   // [rows][k], or [k][rows] when transposed
     int64_t rows;      // 0: nothing to do
@@ -888,53 +1119,73 @@ struct WideOperand {
 };
 
 __global__ void __launch_bounds__(256) wide_planes_kernel(
-    const uint32_t *__restrict__ wide, const WideOperand a, const WideOperand b, int64_t k, int64_t kp) {
-    __shared__ float tile[32][33];
+    const HalfExceptions *__restrict__ ea, const HalfExceptions *__restrict__ eb, const WideOperand a, const WideOperand b,
+    int64_t k, int64_t kp) {
+    __shared__ float tile[64][65];
     griddep_launch_dependents();
     griddep_wait();
-    if (*reinterpret_cast<const volatile uint32_t *>(wide) == 0)
+    if (!half_wide(ea, eb))
         return;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     for (int which = 0; which < 2; ++which) {
         const WideOperand &o  = which ? b : a;
-        const int64_t tiles_k = kp / 32, tiles = ((o.rows + 31) / 32) * tiles_k;
+        const int64_t tiles_k = (kp + 63) / 64, tiles = ((o.rows + 63) / 64) * tiles_k;
         for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-            const int64_t r0 = t / tiles_k * 32, k0 = t % tiles_k * 32;
+            const int64_t r0 = t / tiles_k * 64, k0 = t % tiles_k * 64;
+            float v[16]; // row r0 + ty + 8 (u >> 1), value k0 + tx + 32 (u & 1)
             if (o.transposed) {
+                // value k0 + ty + 8 (u >> 1) of row r0 + tx + 32 (u & 1)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int64_t kk = k0 + ty + j * 8, rr = r0 + tx;
-                    tile[tx][ty + j * 8] = (kk < k && rr < o.rows) ? o.in[kk * o.rows + rr] : 0.0f;
+                for (int u = 0; u < 16; ++u) {
+                    const int64_t kk = k0 + ty + 8 * (u >> 1), rr = r0 + tx + 32 * (u & 1);
+                    v[u]             = (kk < k && rr < o.rows) ? o.in[kk * o.rows + rr] : 0.0f;
                 }
+#pragma unroll
+                for (int u = 0; u < 16; ++u)
+                    tile[tx + 32 * (u & 1)][ty + 8 * (u >> 1)] = v[u];
                 __syncthreads();
+#pragma unroll
+                for (int u = 0; u < 16; ++u)
+                    v[u] = tile[ty + 8 * (u >> 1)][tx + 32 * (u & 1)];
+                __syncthreads();
+            } else {
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    const int64_t rr = r0 + ty + 8 * (u >> 1), kk = k0 + tx + 32 * (u & 1);
+                    v[u]             = (rr < o.rows && kk < k) ? o.in[rr * k + kk] : 0.0f;
+                }
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int64_t rr = r0 + ty + j * 8, kk = k0 + tx;
-                if (rr < o.rows) {
-                    const float v = o.transposed ? tile[ty + j * 8][tx] : (kk < k ? o.in[rr * k + kk] : 0.0f);
+            for (int u = 0; u < 16; ++u) {
+                const int64_t rr = r0 + ty + 8 * (u >> 1), kk = k0 + tx + 32 * (u & 1);
+                if (rr < o.rows && kk < kp) {
                     float hi, lo;
-                    split_tf32(v, hi, lo);
+                    split_tf32_flat(v[u], hi, lo);
                     o.hi[rr * kp + kk] = hi;
                     o.lo[rr * kp + kk] = lo;
                 }
             }
-            __syncthreads();
         }
     }
 }
 
-// tf32 planes from float16 planes (both terms convert exactly), for a row range of a packed left operand
-// whose right operand is wide; returns at once where the left operand is wide itself and has them already.
+// tf32 planes from float16 planes (both terms convert exactly) and the exceptions, for a row range of a packed left
+// operand whose right operand is wide; returns at once where the left operand is wide itself and has them already.
 __global__ void __launch_bounds__(256) widen_planes_kernel(
-    const uint32_t *__restrict__ wide, const __half *__restrict__ hi16, const __half *__restrict__ lo16,
+    const HalfExceptions *__restrict__ x, int line0, const __half *__restrict__ hi16, const __half *__restrict__ lo16,
     const float *__restrict__ row_scale, int64_t rows, int64_t kp, float *__restrict__ hi32, float *__restrict__ lo32) {
-    if (*reinterpret_cast<const volatile uint32_t *>(wide) != 0)
+    if (half_wide(x, x))
         return;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < rows * kp; i += (int64_t)gridDim.x * 256) {
-        const float s = row_scale[i / kp];
-        hi32[i]       = __half2float(hi16[i]) * s;
-        lo32[i]       = __half2float(lo16[i]) * kHalfLoInv * s;
+        const int64_t row = i / kp;
+        const float s = row_scale[row], inverse = fabsf(s);
+        float hi = __half2float(hi16[i]) * inverse, lo = __half2float(lo16[i]) * kHalfLoInv * inverse;
+        if (s < 0.0f)
+            for (int e = 0; e < (int)x->count; ++e)
+                if (x->e[e].line == (row + line0) * 2 && x->e[e].k == i - row * kp)
+                    split_tf32(x->e[e].value, hi, lo);
+        hi32[i] = hi;
+        lo32[i] = lo;
     }
 }
 
@@ -1081,21 +1332,19 @@ ct_status half_split_both(
 }
 
 ct_status half_wide_planes(
-    DeviceState *st, const uint32_t *wide, const float *a, int64_t m, bool a_is_km, void *a_hi, void *a_lo, const float *b,
+    DeviceState *st, const HalfExceptions *ea, const HalfExceptions *eb, const float *a, int64_t m, bool a_is_km, void *a_hi, void *a_lo, const float *b,
     int64_t n, void *b_hi, void *b_lo, int64_t k, int64_t kp) {
     const WideOperand oa{a, m, a_is_km ? 1 : 0, static_cast<float *>(a_hi), static_cast<float *>(a_lo)};
     const WideOperand ob{b, n, 1, static_cast<float *>(b_hi), static_cast<float *>(b_lo)};
-    CT_CUDA(launch_dependent(wide_planes_kernel, dim3((unsigned)st->sm_count * 2), dim3(256), 0, stream(), wide, oa, ob, k, kp));
+    CT_CUDA(launch_dependent(wide_planes_kernel, dim3((unsigned)st->sm_count * 2), dim3(256), 0, stream(), ea, eb, oa, ob, k, kp));
     CT_LAUNCH_CHECK("wide_planes");
     return CT_OK;
 }
 
-ct_status half_widen_rows(
-    DeviceState *st, const uint32_t *wide, const void *hi16, const void *lo16, const float *scale, int64_t rows, int64_t kp,
-    void *hi32, void *lo32) {
+ct_status half_widen_rows(DeviceState *st, const HalfOperand &o, int64_t kp) {
     widen_planes_kernel<<<(unsigned)st->sm_count * 4, 256, 0, stream()>>>(
-        wide, static_cast<const __half *>(hi16), static_cast<const __half *>(lo16), scale, rows, kp,
-        static_cast<float *>(hi32), static_cast<float *>(lo32));
+        o.exceptions, (int)o.line0, static_cast<const __half *>(o.hi16), static_cast<const __half *>(o.lo16), o.scale, o.rows, kp,
+        static_cast<float *>(const_cast<void *>(o.hi32)), static_cast<float *>(const_cast<void *>(o.lo32)));
     CT_LAUNCH_CHECK("widen_planes");
     return CT_OK;
 }
@@ -1108,7 +1357,7 @@ int half_tile_columns(const DeviceState *st, int64_t m, int64_t n, int64_t batch
 
 ct_status gemm_half(
     DeviceState *st, const HalfOperand &a, const HalfOperand &b, int64_t kp, const float *bias, int act, float *out,
-    bool force_wide, bool own_flag, bool allow_splitk, const HalfBands *bands, int batch, bool bias_per_row) {
+    bool force_wide, bool allow_splitk, const HalfBands *bands, int batch, bool bias_per_row) {
     const int64_t m = a.rows, n = b.rows / batch;
     const int bn    = half_tile_columns(st, m, n, batch);
     HalfGemmParams p{};
@@ -1120,10 +1369,13 @@ ct_status gemm_half(
     p.row_scale   = a.scale;
     p.col_scale   = b.scale;
     p.flags       = st->flags_dev;
-    p.wide_a      = a.wide;
-    p.wide_b      = b.wide;
-    p.force_wide  = force_wide ? 1 : 0;
-    p.reset_flags = own_flag ? 1 : 0;
+    p.a_hi = static_cast<const __half *>(a.hi16), p.a_lo = static_cast<const __half *>(a.lo16);
+    p.b_hi = static_cast<const __half *>(b.hi16), p.b_lo = static_cast<const __half *>(b.lo16);
+    p.kp           = (int)kp;
+    p.exceptions_a = a.exceptions, p.exceptions_b = b.exceptions;
+    p.a_line0      = (int)a.line0;
+    p.force_wide   = force_wide ? 1 : 0;
+    p.reset        = a.exceptions == st->exceptions_dev || b.exceptions == st->exceptions_dev ? st->exceptions_dev : nullptr;
     if (bands) {
         p.bands     = bands->bands;
         p.band_done = bands->done;

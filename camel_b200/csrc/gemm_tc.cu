@@ -33,6 +33,7 @@
 //   ct_matmul_f32_static    the GEMM for callers that may not allocate device memory
 #include "common.cuh"
 #include "tc_ptx.cuh"
+#include "half_split.cuh"
 #include "split.cuh"
 #include "tmap.cuh"
 
@@ -1679,7 +1680,7 @@ ct_status split_rows_planes(
 constexpr int64_t kMaxDim = 1ll << 30;
 
 // The float32 product in split float16 (gemm_half.cu).  Workspace: inverse scales and column maxima, then
-// the operand planes - float16 pairs, or, where the pre-pass finds a row too wide for them, the tf32 planes
+// the operand planes - float16 pairs, or, where the pre-pass finds too many exceptions, the tf32 planes
 // in the same place (the product reads one or the other), so no more than tf32 planes alone would take.
 // Operands whose tf32 planes are at most kBothFormsBytes get them at once, next to the float16 ones: at
 // 512^3 those 4 MB stay in L2 and cost less than the conditional launch (about 2 us).
@@ -1700,12 +1701,11 @@ static ct_status gemm_f32_split(
     uint32_t *a_max = reinterpret_cast<uint32_t *>(ws + a_words);
     uint32_t *b_max = reinterpret_cast<uint32_t *>(ws + 2 * a_words + b_words);
     uint8_t *p16 = ws + 2 * a_words + 2 * b_words, *p32 = p16 + wide_at;
-    uint32_t *wide = st->flags_dev + FLAG_WIDE;
-    HalfOperand oa{p16, p16 + a16, a_scale, p32, p32 + a32, wide, m};
-    HalfOperand ob{p16 + 2 * a16, p16 + 2 * a16 + b16, b_scale, p32 + 2 * a32, p32 + 2 * a32 + b32, wide, n};
+    HalfOperand oa{p16, p16 + a16, a_scale, p32, p32 + a32, st->exceptions_dev, 0, m};
+    HalfOperand ob{p16 + 2 * a16, p16 + 2 * a16 + b16, b_scale, p32 + 2 * a32, p32 + 2 * a32 + b32, st->exceptions_dev, 1, n};
     const bool force_wide = packed && !packed->hi16;
     if (packed) {
-        ob.hi32 = packed->hi, ob.lo32 = packed->lo, ob.scale = packed->scale;
+        ob.hi32 = packed->hi, ob.lo32 = packed->lo, ob.scale = packed->scale, ob.exceptions = packed->exceptions;
         ob.hi16 = force_wide ? packed->hi : packed->hi16, ob.lo16 = force_wide ? packed->lo : packed->lo16;
     }
     {
@@ -1718,21 +1718,22 @@ static ct_status gemm_f32_split(
             CT_TRY(half_split_both(st, a, oa, b, ob, k, kp, both_forms, &both));
         if (!force_wide && !both) {
             if (a_is_km && two_pass)
-                CT_CUDA(cudaMemsetAsync(a_max, 0, a_words, stream()));
+                CT_CUDA(cudaMemsetAsync(a_scale, 0, 2 * a_words, stream()));
             if (a_is_km && !packed && two_pass)
-                CT_CUDA(cudaMemsetAsync(b_max, 0, b_words, stream()));
+                CT_CUDA(cudaMemsetAsync(b_scale, 0, 2 * b_words, stream()));
             if (a_is_km)
                 CT_TRY(half_split_cols(st, a, k, kp, oa, both_forms, a_max));
             else
-                CT_TRY(half_split_rows(st, a, k, kp, oa, both_forms, b_max, !packed && two_pass ? n : 0));
+                CT_TRY(half_split_rows(st, a, k, kp, oa, both_forms, reinterpret_cast<uint32_t *>(b_scale),
+                                       !packed && two_pass ? (int64_t)(2 * b_words / 4) : 0));
             if (!packed)
                 CT_TRY(half_split_cols(st, b, k, kp, ob, both_forms, b_max));
         }
         if (!force_wide && !both_forms)
-            CT_TRY(half_wide_planes(st, wide, a, m, a_is_km, const_cast<void *>(oa.hi32), const_cast<void *>(oa.lo32), b,
+            CT_TRY(half_wide_planes(st, oa.exceptions, ob.exceptions, a, m, a_is_km, const_cast<void *>(oa.hi32), const_cast<void *>(oa.lo32), b,
                                     packed ? 0 : n, const_cast<void *>(ob.hi32), const_cast<void *>(ob.lo32), k, kp));
     }
-    return gemm_half(st, oa, ob, kp, bias, act, out, force_wide, !force_wide, true, nullptr);
+    return gemm_half(st, oa, ob, kp, bias, act, out, force_wide, true, nullptr);
 }
 
 ct_status gemm_f32_tc(
@@ -1839,25 +1840,25 @@ extern "C" ct_status ct_weights_pack(const float *w, int64_t k, int64_t n, void 
     if (grid.y > 65535)
         return fail(CT_ERR_TOO_LARGE, "ct_weights_pack: k too large for the operand pre-pass");
     // 3xTF32: the float16 pairs that products normally read, and the tf32 planes for a left operand (or
-    // these weights) too wide for them; [hi][lo][hi16][lo16][scale][col max][word]
+    // these weights) too wide for them; [hi][lo][hi16][lo16][scale][col max][exceptions]
     const size_t plane16 = mode == MODE_3X ? ((size_t)n * kp * 2 + 1023) & ~(size_t)1023 : 0;
     const size_t words   = mode == MODE_3X ? ((size_t)n * 4 + 1023) & ~(size_t)1023 : 0;
     void *base = nullptr;
-    CT_TRY(ct_alloc(&base, plane * planes + 2 * plane16 + 2 * words + (mode == MODE_3X ? 4 : 0)));
+    CT_TRY(ct_alloc(&base, plane * planes + 2 * plane16 + 2 * words + (mode == MODE_3X ? sizeof(HalfExceptions) : 0)));
     void *hi = base, *lo = static_cast<uint8_t *>(base) + plane;
     uint8_t *half_base = static_cast<uint8_t *>(base) + plane * planes;
     void *hi16 = nullptr, *lo16 = nullptr;
-    float *scale   = nullptr;
-    uint32_t *wide = nullptr;
+    float *scale               = nullptr;
+    HalfExceptions *exceptions = nullptr;
     if (mode == MODE_3X) {
         hi16 = half_base, lo16 = half_base + plane16;
         scale = reinterpret_cast<float *>(half_base + 2 * plane16);
-        wide  = reinterpret_cast<uint32_t *>(half_base + 2 * plane16 + 2 * words);
+        exceptions = reinterpret_cast<HalfExceptions *>(half_base + 2 * plane16 + 2 * words);
         ProfScope prof("weights_pack");
         uint32_t *col_max = reinterpret_cast<uint32_t *>(half_base + 2 * plane16 + words);
-        cudaError_t e     = cudaMemsetAsync(col_max, 0, words + 4, stream());
+        cudaError_t e     = cudaMemsetAsync(scale, 0, 2 * words + sizeof(HalfExceptions), stream());
         ct_status s       = e != cudaSuccess ? cuda_fail(e, "weights_pack")
-                                             : half_split_cols(st, w, k, kp, HalfOperand{hi16, lo16, scale, nullptr, nullptr, wide, n}, false, col_max);
+                                             : half_split_cols(st, w, k, kp, HalfOperand{hi16, lo16, scale, nullptr, nullptr, exceptions, 1, n}, false, col_max);
         if (s != CT_OK) {
             ct_free(base);
             return s;
@@ -1877,19 +1878,19 @@ extern "C" ct_status ct_weights_pack(const float *w, int64_t k, int64_t n, void 
         count_launch(1);
     }
     // the handle may be used from any stream afterwards: finish the one-time pass here
-    uint32_t is_wide = 0;
-    cudaError_t se   = wide ? cudaMemcpyAsync(&is_wide, wide, sizeof(is_wide), cudaMemcpyDeviceToHost, stream()) : cudaSuccess;
+    uint32_t found[2] = {0, 0}; // wide, count
+    cudaError_t se    = exceptions ? cudaMemcpyAsync(found, exceptions, sizeof(found), cudaMemcpyDeviceToHost, stream()) : cudaSuccess;
     if (se == cudaSuccess)
         se = cudaStreamSynchronize(stream());
     if (se != cudaSuccess) {
         ct_free(base);
         return cuda_fail(se, "weights_pack");
     }
-    if (is_wide)
+    if (found[0] != 0 || found[1] > kHalfExceptions)
         hi16 = lo16 = nullptr;
     int dev = -1;
     CT_CUDA(cudaGetDevice(&dev));
-    PackedWeights *pw = new PackedWeights{kPackedMagic, mode, dev, k, n, kp, w, base, hi, lo, hi16, lo16, scale};
+    PackedWeights *pw = new PackedWeights{kPackedMagic, mode, dev, k, n, kp, w, base, hi, lo, hi16, lo16, scale, exceptions};
     *packed_out       = pw;
     return CT_OK;
 }
@@ -1923,11 +1924,11 @@ struct PackedRows {
     void *base;
     uint8_t *hi, *lo;
     size_t row_bytes; // bytes of one row of a plane
-    // 3xTF32: float16 pairs, inverse row scales and the word that says that the rows need the tf32 planes
-    // (hi, lo), which are written only then
+    // 3xTF32: float16 pairs, inverse row scales and the exceptions, which may say that the rows need the tf32 planes
+    // (hi, lo); those are written only then
     uint8_t *hi16, *lo16;
     float *scale;
-    uint32_t *wide;
+    HalfExceptions *exceptions;
 };
 constexpr uint32_t kPackedRowsMagic = 0x43545052u; // "CTPR"
 
@@ -1956,19 +1957,19 @@ extern "C" ct_status ct_rows_pack(const float *a, int64_t m, int64_t k, void **p
         const size_t plane16 = mode == MODE_3X ? ((size_t)m * kp * 2 + 1023) & ~(size_t)1023 : 0;
         const size_t words   = mode == MODE_3X ? ((size_t)m * 4 + 1023) & ~(size_t)1023 : 0;
         void *base           = nullptr;
-        CT_TRY(ct_alloc(&base, plane * planes + 2 * plane16 + words + (mode == MODE_3X ? 4 : 0)));
+        CT_TRY(ct_alloc(&base, plane * planes + 2 * plane16 + words + (mode == MODE_3X ? sizeof(HalfExceptions) : 0)));
         uint8_t *hi = static_cast<uint8_t *>(base), *hi16 = hi + plane * planes;
         pr          = new PackedRows{kPackedRowsMagic, mode, dev, m, k, kp, base, hi, hi + plane, (size_t)kp * elem, hi16,
                                      hi16 + plane16, reinterpret_cast<float *>(hi16 + 2 * plane16),
-                                     reinterpret_cast<uint32_t *>(hi16 + 2 * plane16 + words)};
+                                     reinterpret_cast<HalfExceptions *>(hi16 + 2 * plane16 + words)};
         *packed_inout = pr;
     }
     ProfScope prof("gemm_prepass");
     if (mode != MODE_3X)
         return split_rows_planes(st, mode, a, m, k, kp, pr->hi, pr->lo);
-    CT_CUDA(cudaMemsetAsync(pr->wide, 0, sizeof(uint32_t), stream()));
-    CT_TRY(half_split_rows(st, a, k, kp, HalfOperand{pr->hi16, pr->lo16, pr->scale, nullptr, nullptr, pr->wide, m}, false, nullptr, 0));
-    return half_wide_planes(st, pr->wide, a, m, false, pr->hi, pr->lo, nullptr, 0, nullptr, nullptr, k, kp);
+    CT_CUDA(cudaMemsetAsync(pr->exceptions, 0, 2 * sizeof(uint32_t), stream()));
+    CT_TRY(half_split_rows(st, a, k, kp, HalfOperand{pr->hi16, pr->lo16, pr->scale, nullptr, nullptr, pr->exceptions, 0, m}, false, nullptr, 0));
+    return half_wide_planes(st, pr->exceptions, pr->exceptions, a, m, false, pr->hi, pr->lo, nullptr, 0, nullptr, nullptr, k, kp);
 }
 
 extern "C" ct_status ct_rows_free(void *packed) {
@@ -1988,16 +1989,15 @@ static ct_status gemm_packed_rows(
     DeviceState *st, const PackedRows *pr, int64_t row0, int64_t rows, const PackedWeights *pw, float *out,
     const HalfBands *bands) {
     const size_t at = (size_t)row0 * pr->kp;
-    HalfOperand oa{pr->hi16 + at * 2, pr->lo16 + at * 2, pr->scale + row0, pr->hi + at * 4, pr->lo + at * 4, pr->wide, rows};
-    HalfOperand ob{pw->hi16, pw->lo16, pw->scale, pw->hi, pw->lo, pr->wide, pw->n};
+    HalfOperand oa{pr->hi16 + at * 2, pr->lo16 + at * 2, pr->scale + row0, pr->hi + at * 4, pr->lo + at * 4, pr->exceptions, 0, rows, row0};
+    HalfOperand ob{pw->hi16, pw->lo16, pw->scale, pw->hi, pw->lo, pw->exceptions, 1, pw->n};
     const bool force_wide = pw->hi16 == nullptr;
     if (force_wide) {
         // each call widens the rows it reads: calls on several streams share no state
         ob.hi16 = pw->hi, ob.lo16 = pw->lo;
-        CT_TRY(half_widen_rows(st, pr->wide, oa.hi16, oa.lo16, oa.scale, rows, pr->kp, const_cast<void *>(oa.hi32),
-                               const_cast<void *>(oa.lo32)));
+        CT_TRY(half_widen_rows(st, oa, pr->kp));
     }
-    return gemm_half(st, oa, ob, pr->kp, nullptr, CT_ACT_NONE, out, force_wide, false, false, bands);
+    return gemm_half(st, oa, ob, pr->kp, nullptr, CT_ACT_NONE, out, force_wide, false, bands);
 }
 
 extern "C" ct_status ct_matmul_packed_rows(

@@ -8,10 +8,15 @@
 //     v * 2^(14-e) = hi + lo * 2^-11,   hi = half(v * 2^(14-e)),   lo = half((v * 2^(14-e) - hi) * 2^11)
 // The pair holds a scaled value to an absolute error of 2^-36 at worst (lo's quantum is then 2^-24) and to 2^-23
 // of itself from 2^-13 up, which is what a pair of tf32 terms holds of any value; from 2^-12 up the two terms are the
-// same two 11-bit numbers whatever the scale (every bit of lo lies above float16's smallest).  A matrix with a
-// smaller non-zero value - 2^-27 of its row's largest or less - or a row whose exponent is beyond +-60 raises a
-// device word, and the product is then computed from tf32 planes instead (same launch sequence, no host involvement).
-// Convolutions decide it per image (and per layer for its filters), see half_range_fits.
+// same two 11-bit numbers whatever the scale (every bit of lo lies above float16's smallest).
+//
+// Values below that are exceptions (2^-27 of their row's largest, or less): hi would be subnormal, lo more than 2^-11 of
+// it, and the product of two low terms, which no MMA computes, no longer negligible.  Matrices of ordinary values have
+// a few per hundred million, so the pre-pass stores zeros for them, lists up to kHalfExceptions of a product, marks
+// their rows by the sign of the scale, and the product's epilogue adds value . other operand to the outputs of
+// those rows and columns.  A matrix with more of them, or with a row whose exponent is beyond +-60, is computed from
+// tf32 planes instead (same launch sequence, no host involvement).  Convolutions of stride 1 decide that per image
+// (and per layer for its filters), see half_range_fits.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -22,8 +27,19 @@ namespace ct {
 
 constexpr float kHalfLoScale    = 2048.0f;              // 2^11
 constexpr float kHalfLoInv      = 1.0f / 2048.0f;
-constexpr float kHalfSmallest   = 1.0f / (1u << 13);    // scaled magnitudes below this may lose more than 2^-23
+constexpr float kHalfSmallest   = 1.0f / (1u << 13);    // scaled magnitudes below this are exceptions
 constexpr int kHalfMaxExponent  = 60;
+
+struct HalfException {
+    int line, k; // 2 * row of the planes + operand (0 left, 1 right), position in the row
+    float value; // the planes hold 0 there
+};
+constexpr int kHalfExceptions = 32;
+struct alignas(8) HalfExceptions {
+    uint32_t wide;  // a row's exponent does not fit
+    uint32_t count; // exceptions found; more than the list holds: the operands need tf32 planes
+    HalfException e[kHalfExceptions];
+};
 
 // magnitude bits of a finite value, 0 for infinities and NaN (they are carried by hi alone)
 __device__ __forceinline__ uint32_t finite_magnitude(float v) {
@@ -66,18 +82,51 @@ __device__ __forceinline__ bool half_range_fits(uint2 r, float &scale, float &in
     return ok && (r.y == kNoneSmallest || __uint_as_float(r.y + 1u) * scale >= kHalfExact);
 }
 
-// v is already scaled.  Returns true when v is too small beside its row's largest value.
-__device__ __forceinline__ bool split_half(float v, __half &hi, __half &lo) {
+__device__ __forceinline__ bool half_exception(float v, float scale) { return v != 0.0f && fabsf(v * scale) < kHalfSmallest; }
+
+// Returns true, and zeros, for an exception.
+__device__ __forceinline__ bool split_half(float v, float scale, __half &hi, __half &lo) {
+    const bool exception = half_exception(v, scale);
+    v  = exception ? 0.0f : v * scale;
     hi = __float2half_rn(v);
     const float d = (v - __half2float(hi)) * kHalfLoScale; // exact for finite v
     lo = isfinite(v) ? __float2half_rn(d) : __half(0.0f);
-    return v != 0.0f && fabsf(v) < kHalfSmallest;
+    return exception;
 }
 
 // Two scaled values of a range that fits (half_range_fits): finite, no exceptions.
 __device__ __forceinline__ void split_half_pair(float a, float b, __half2 &hi, __half2 &lo) {
     hi = __floats2half2_rn(a, b);
     lo = __floats2half2_rn(__fmul_rn(__fsub_rn(a, __low2float(hi)), kHalfLoScale), __fmul_rn(__fsub_rn(b, __high2float(hi)), kHalfLoScale));
+}
+
+// Whether either operand needs its tf32 planes: one 8-byte load for each list (operands prepared together share one), both
+// in flight - as four loads in a row they cost an idle launch 3 us.
+__device__ __forceinline__ bool half_wide(const HalfExceptions *a, const HalfExceptions *b) {
+    const uint64_t va = *reinterpret_cast<const volatile uint64_t *>(a), vb = *reinterpret_cast<const volatile uint64_t *>(b);
+    return ((uint32_t)va | (uint32_t)vb) != 0u || max((uint32_t)(va >> 32), (uint32_t)(vb >> 32)) > kHalfExceptions;
+}
+
+// More exceptions than the list holds: the rest need not be looked for.
+__device__ __forceinline__ bool half_overfull(const HalfExceptions *x) {
+    return const_cast<const volatile HalfExceptions *>(x)->count > kHalfExceptions;
+}
+
+// A whole warp records its lanes' exceptions among the values v; true if there were any.  Once the list is over-full the
+// count is left alone: a matrix of nothing else would queue up at one word.
+__device__ __forceinline__ bool half_record(HalfExceptions *x, float v, float scale, int operand, int64_t line, int64_t k) {
+    const bool mine     = half_exception(v, scale);
+    const uint32_t mask = __ballot_sync(0xffffffffu, mine);
+    if (mask == 0u)
+        return false;
+    const int lane = threadIdx.x & 31;
+    uint32_t at    = kHalfExceptions;
+    if (lane == 0 && !half_overfull(x))
+        at = atomicAdd(&x->count, (uint32_t)__popc(mask));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(mask & ((1u << lane) - 1u));
+    if (mine && at < kHalfExceptions)
+        x->e[at] = HalfException{(int)line * 2 + operand, (int)k, v};
+    return true;
 }
 
 } // namespace ct

@@ -1,5 +1,6 @@
 // Library state: error text, device/stream selection, storage entry points.
 #include "common.cuh"
+#include "half_split.cuh"
 
 #include <atomic>
 #include <cctype>
@@ -146,6 +147,8 @@ ct_status current(DeviceState **out) {
             st->sm_count = prop.multiProcessorCount;
             CT_CUDA(cudaMalloc(&st->flags_dev, FLAG_COUNT * sizeof(uint32_t)));
             CT_CUDA(cudaMemset(st->flags_dev, 0, FLAG_COUNT * sizeof(uint32_t)));
+            CT_CUDA(cudaMalloc(&st->exceptions_dev, sizeof(HalfExceptions)));
+            CT_CUDA(cudaMemset(st->exceptions_dev, 0, sizeof(HalfExceptions)));
             CT_CUDA(cudaMallocHost(&st->flags_host, FLAG_COUNT * sizeof(uint32_t)));
             memset(st->flags_host, 0, FLAG_COUNT * sizeof(uint32_t));
             // Tensor storage comes from the device's stream-ordered pool; keep freed blocks cached
@@ -186,7 +189,6 @@ ct_status ensure_ws(void **ptr, size_t *cap, size_t bytes) {
 }
 
 ct_status clear_data_flags(DeviceState *st) {
-    static_assert(FLAG_WIDE_READERS == FLAG_WIDE + 1, "cleared together by report_timeout");
     static_assert(FLAG_DIV_ZERO == 0 && FLAG_LOG_DOMAIN == 1 && FLAG_TIMEOUT == 2, "layout of the error words");
     CT_CUDA(cudaMemsetAsync(st->flags_dev, 0, 2 * sizeof(uint32_t), stream()));
     return CT_OK;
@@ -196,8 +198,9 @@ ct_status report_timeout(DeviceState *st, const char *what) {
     if (!st->flags_host[FLAG_TIMEOUT])
         return CT_OK;
     uint32_t where = st->flags_host[FLAG_TIMEOUT] - 1;
-    // the launches that gave up or never started may have left the words they would have cleared
-    CT_CUDA(cudaMemsetAsync(st->flags_dev + FLAG_WIDE, 0, 2 * sizeof(uint32_t), stream()));
+    // the launches that gave up or never started may have left what they would have cleared
+    CT_CUDA(cudaMemsetAsync(st->flags_dev + FLAG_EXCEPTION_READERS, 0, sizeof(uint32_t), stream()));
+    CT_CUDA(cudaMemsetAsync(st->exceptions_dev, 0, sizeof(HalfExceptions), stream()));
     CT_CUDA(cudaMemsetAsync(st->flags_dev + FLAG_TIMEOUT, 0, sizeof(uint32_t), stream()));
     return fail(
         CT_ERR_TIMEOUT,

@@ -69,8 +69,12 @@ typedef enum ct_activation {
 typedef enum ct_precision {
     CT_PREC_3XTF32 = 0, /* fp32 in, split into two terms of TF32's 11 significant bits, three MMAs, fp32
                          * accumulate.  The terms are float16 pairs under an exact power-of-two scale per
-                         * row and column; operands whose rows span more than 26 powers of two (or whose
-                         * exponent is beyond +-60) are computed from tf32 terms, decided on the device. */
+                         * row and column, which hold 27 powers of two as well as tf32 terms do.  Smaller
+                         * values beside a row's largest are multiplied in float32 apart, up to 32 of them
+                         * in a product's operands; with more, or a row whose largest exponent is beyond
+                         * +-60, the product is computed from tf32 terms.  Convolutions of stride 1 take
+                         * tf32 terms for the images that span more than 26 powers of two, and for all
+                         * images where a filter does.  All of it is decided on the device. */
     CT_PREC_BF16   = 1  /* inputs rounded to bf16 once, fp32 accumulate (reported separately) */
 } ct_precision;
 

@@ -1,6 +1,6 @@
 """GPU: the contractions in split float16 (gemm_half.cu, conv_halo.cu, the strided convolution's patches)
-at the sizes where their tiling changes, and on operands that float16 pairs cannot hold, which have to
-take the tf32 planes instead; the few-column products at the edges of their row and k tiles.
+at the sizes where their tiling changes, and on operands that float16 pairs cannot hold: few such values,
+which are multiplied apart, and many, which have to take the tf32 planes; the few-column products at the edges of their row and k tiles.
 
 Bounds.  A value is carried to 2^-23 of itself, the product of two so carried to 2^-21, and the tensor core truncates once per addition into an accumulator
 that takes at most 96 of them (tf32) or 64 (float16) before it is drained: 2^-24 each relative to the sum of
@@ -170,6 +170,64 @@ def test_small_values_keep_their_digits_beside_large_ones(T, size, side, lowest)
     got = _product(T, a, b) if side == "left" else _product(T, b, a.T.copy()).T
     want = a.astype(np.float64) * np.diag(b).astype(np.float64)
     assert np.all(np.abs(got - want) <= SINGLE * np.abs(want))
+
+
+def _with_exceptions(rng, m, k, n, count):
+    """Ordinary operands with `count` values in each that a float16 pair cannot hold, and the outputs that depend on
+    one of those alone (or on one of each, at the same k)."""
+    a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    b = rng.uniform(-1, 1, (k, n)).astype(np.float32)
+    rows, cols = rng.choice(m, count, replace=False), rng.choice(n, count, replace=False)
+    ks = rng.choice(np.arange(1, k), count, replace=False)
+    tiny = (rng.uniform(1, 2, (2, count)) * np.exp2(rng.integers(-50, -29, (2, count)))).astype(np.float32)
+    a[:, 0] = rng.uniform(0.5, 1, m)
+    a[rows, 0] = 0.0
+    b[:, cols] = 0.0
+    b[0, cols] = 0.75                    # keeps the column's scale; meets the zeros of a
+    for t in range(count):
+        a[rows[t], ks[t]] = tiny[0, t]
+        b[ks[t], cols[t]] = tiny[1, t] if t % 2 else 0.5
+        a[rows[t], ks[t - 1]] = a[rows[t], ks[t - 1]] or 0.25
+    return a, b, rows, cols
+
+
+# slices in a cluster; two passes over B; pairs; slices through the workspace; one wave of small tiles; more than a list holds
+@pytest.mark.parametrize("m,k,n,count", [(128, 96, 200, 5), (300, 600, 300, 9), (600, 1500, 400, 12), (2600, 1100, 1500, 30),
+                                         (1290, 4700, 128, 7), (1000, 300, 1000, 20), (700, 1200, 800, 40)])
+@pytest.mark.parametrize("form", ["plain", "transposed", "weights", "rows"])
+def test_values_that_float16_pairs_cannot_hold_are_put_right(T, m, k, n, count, form):
+    import ctypes as C
+
+    from camel_b200._lib import check, lib
+
+    rng = np.random.default_rng(m + k + n)
+    a, b, rows, cols = _with_exceptions(rng, m, k, n, count)
+    bias = rng.uniform(-1, 1, n).astype(np.float32)
+    bias[cols] = 0.0
+    ta, tb, out = T.from_numpy(a), T.from_numpy(b), T.zeros((m, n))
+    if form == "plain":
+        check(lib.ct_dense(ta.ptr, tb.ptr, T.from_numpy(bias).ptr, m, k, n, 0, out.ptr, None))
+    elif form == "transposed":
+        out, bias = T.matmul_tn(T.from_numpy(a.T.copy()), tb), 0.0 * bias
+    else:
+        ap, wp, bias = C.c_void_p(), C.c_void_p(), 0.0 * bias
+        check(lib.ct_weights_pack(tb.ptr, k, n, C.byref(wp)))
+        check(lib.ct_rows_pack(ta.ptr, m, k, C.byref(ap)))
+        if form == "weights":
+            check(lib.ct_dense_packed(ta.ptr, tb.ptr, wp, None, m, k, n, 0, out.ptr, None))
+        else:
+            for row0 in range(0, m, 128):
+                check(lib.ct_matmul_packed_rows(ap, row0, min(128, m - row0), wp, out.ptr + row0 * n * 4))
+        T.check_async()
+        check(lib.ct_rows_free(ap))
+        check(lib.ct_weights_free(wp))
+    got = out.numpy()
+    T.check_async()
+    a64, b64 = a.astype(np.float64), b.astype(np.float64)
+    want = a64 @ b64 + bias
+    assert np.all(np.abs(got - want) <= BOUND * (np.abs(a64) @ np.abs(b64) + np.abs(bias)))
+    for t in range(count):  # column t holds 0.75 at k = 0, where row t is zero, and one value that meets the row's small one
+        assert abs(got[rows[t], cols[t]] - want[rows[t], cols[t]]) <= SINGLE * abs(want[rows[t], cols[t]])
 
 
 # strided; halo; filters in tensor memory from the input itself, from planes, and with a tile of odd rows
