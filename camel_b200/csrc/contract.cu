@@ -28,9 +28,7 @@ template <int MODE>
 __global__ void __launch_bounds__(256) im2col_planes_kernel(
     const float *__restrict__ x, int64_t c, int64_t h, int64_t w, int64_t kh, int64_t kw,
     int64_t stride, int64_t pad, int64_t ho, int64_t wo, int64_t kdim, int64_t kp, int64_t total,
-    void *__restrict__ p_hi, void *__restrict__ p_lo, const HalfExceptions *__restrict__ only_if) {
-    if (only_if && !half_wide(only_if, only_if))
-        return; // the float16 planes of im2col_half_kernel hold the patches
+    void *__restrict__ p_hi, void *__restrict__ p_lo) {
     int64_t step = (int64_t)gridDim.x * 256;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += step) {
         int64_t kk  = i % kp;
@@ -59,20 +57,28 @@ __global__ void __launch_bounds__(256) im2col_planes_kernel(
 // its largest magnitude and the split.  Where in the image patch element kk lies - (offset, r, s) - comes from
 // a table in shared memory that a block builds once; with an element per thread and 64-bit divisions for each
 // of them the pass took 218 us for 64 x 48 x 57 x 57 at stride 2, seven times what its stores cost.
+// WIDE: the tf32 terms instead, in planes of floats, where the exceptions ask for them.
 constexpr int kPatchRegs = 16; // pairs of values per lane: patches of up to 1024 values
-template <int V>
+template <int V, bool WIDE>
 __global__ void __launch_bounds__(256) im2col_half_kernel(
     const float *__restrict__ x, int c, int h, int w, int kh, int kw, int stride, int pad, int ho, int wo, int kdim, int kp,
-    int64_t rows, __half *__restrict__ p_hi, __half *__restrict__ p_lo, float *__restrict__ scale_out,
+    int64_t rows, void *__restrict__ plane_hi, void *__restrict__ plane_lo, float *__restrict__ scale_out,
     HalfExceptions *__restrict__ exceptions) {
     extern __shared__ int2 where[]; // element kk: offset from the patch's origin in its image, r << 16 | s
+    __half *p_hi = static_cast<__half *>(plane_hi), *p_lo = static_cast<__half *>(plane_lo);
     griddep_launch_dependents();
+    if (WIDE) {
+        griddep_wait();
+        if (!half_wide(exceptions, exceptions))
+            return;
+    }
     for (int kk = threadIdx.x; kk < kp; kk += 256) {
         const int s = kk % kw, r = (kk / kw) % kh, ic = kk / (kw * kh);
         where[kk] = kk < kdim ? make_int2((ic * h + r) * w + s, (r << 16) | s) : make_int2(0, 0x7fff7fff);
     }
     __syncthreads();
-    griddep_wait();
+    if (!WIDE)
+        griddep_wait();
     const int lane = threadIdx.x & 31, pix = ho * wo;
     for (int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (int64_t)gridDim.x * 8) {
         const int img = (int)(row / pix), p = (int)(row - (int64_t)img * pix);
@@ -83,6 +89,18 @@ __global__ void __launch_bounds__(256) im2col_half_kernel(
             const int iy = y0 + (at.y >> 16), ix = x0 + (at.y & 0xffff);
             return (iy >= 0 && iy < h && ix >= 0 && ix < w) ? __ldg(src + at.x) : 0.0f; // padding elements lie far outside
         };
+        if (WIDE) {
+            float *hi = static_cast<float *>(plane_hi) + row * kp, *lo = static_cast<float *>(plane_lo) + row * kp;
+#pragma unroll 4
+            for (int kk = 2 * lane; kk < kp; kk += 64) {
+                float2 h, l;
+                split_tf32_flat(load(kk), h.x, l.x);
+                split_tf32_flat(load(kk + 1), h.y, l.y);
+                *reinterpret_cast<float2 *>(hi + kk) = h;
+                *reinterpret_cast<float2 *>(lo + kk) = l;
+            }
+            continue;
+        }
         float2 v[V];
         uint2 range = make_uint2(0u, kNoneSmallest);
         const bool fits = kp <= 64 * V;
@@ -749,22 +767,20 @@ static ct_status conv2d_run(
             ProfScope prof("im2col");
             CT_TRY(half_split_rows(st, w, kdim, kp, oa, true, nullptr, 0));
             const unsigned blocks = capped_blocks(st, n * pix * 32, 8);
-#define CT_PATCHES(V)                                                                                                   \
-    CT_CUDA(launch_dependent(im2col_half_kernel<V>, dim3(blocks), dim3(256), (size_t)kp * sizeof(int2), stream(), x, (int)c, \
+#define CT_PATCHES(V, WIDE, LO)                                                                                              \
+    CT_CUDA(launch_dependent(im2col_half_kernel<V, WIDE>, dim3(blocks), dim3(256), (size_t)kp * sizeof(int2), stream(), x, (int)c, \
                              (int)h, (int)wd, (int)kh, (int)kw, (int)stride, (int)pad, (int)ho, (int)wo, (int)kdim, (int)kp,  \
-                             n * pix, reinterpret_cast<__half *>(patches), reinterpret_cast<__half *>(patches + p16),       \
-                             const_cast<float *>(ob.scale), ob.exceptions))
+                             n * pix, static_cast<void *>(patches), static_cast<void *>(LO), const_cast<float *>(ob.scale), ob.exceptions))
             if (kp <= 256)
-                CT_PATCHES(4);
+                CT_PATCHES(4, false, patches + p16);
             else if (kp <= 512)
-                CT_PATCHES(8);
+                CT_PATCHES(8, false, patches + p16);
             else
-                CT_PATCHES(kPatchRegs);
-#undef CT_PATCHES
+                CT_PATCHES(kPatchRegs, false, patches + p16);
             CT_LAUNCH_CHECK("im2col_half");
-            im2col_planes_kernel<0><<<capped_blocks(st, n * pix * kp, 4), 256, 0, stream()>>>(
-                x, c, h, wd, kh, kw, stride, pad, ho, wo, kdim, kp, n * pix * kp, patches, patches + p_plane, st->exceptions_dev);
-            CT_LAUNCH_CHECK("im2col_planes");
+            CT_PATCHES(1, true, patches + p_plane);
+#undef CT_PATCHES
+            CT_LAUNCH_CHECK("im2col_wide");
         }
         return gemm_half(st, oa, ob, kp, bias, act, out, false, false, nullptr, (int)n, true);
     }
@@ -778,10 +794,10 @@ static ct_status conv2d_run(
         ProfScope prof("im2col");
         if (mode == 0)
         im2col_planes_kernel<0><<<capped_blocks(st, total, 32), 256, 0, stream()>>>(
-            x, c, h, wd, kh, kw, stride, pad, ho, wo, kdim, kp, total, p_hi, p_lo, nullptr);
+            x, c, h, wd, kh, kw, stride, pad, ho, wo, kdim, kp, total, p_hi, p_lo);
     else
         im2col_planes_kernel<1><<<capped_blocks(st, total, 32), 256, 0, stream()>>>(
-            x, c, h, wd, kh, kw, stride, pad, ho, wo, kdim, kp, total, p_hi, p_lo, nullptr);
+            x, c, h, wd, kh, kw, stride, pad, ho, wo, kdim, kp, total, p_hi, p_lo);
     }
     CT_LAUNCH_CHECK("im2col_planes");
     return gemm_planes(
