@@ -226,34 +226,56 @@ __device__ __noinline__ void half_finish(
         }
 }
 
-// A tile added up by its cluster, where a row or column of it has exceptions: rows r0 .. of the tile at (row0, col0),
-// whose slices' sums lie at `sums` in the CTAs.
+// The same for a tile added up by its cluster: the rows r0 .. of this CTA's share and the columns that have exceptions,
+// from the slices' sums at `sums` in the CTAs.  The flags of 32 rows or columns are looked at together; a warp takes
+// every tenth of those that have any.
+template <int BN>
 __device__ __noinline__ void half_finish_slices(
-    const HalfGemmParams &p, uint32_t sums, int slices, int r0, int rows, int64_t row0, int64_t col0, int bn) {
-    for (int i = threadIdx.x; i < rows * bn; i += kHThreads) {
-        const int r = r0 + i / bn, c = i % bn;
+    const HalfGemmParams &p, uint32_t sums, int slices, int r0, int rows, int64_t row0, int64_t col0) {
+    constexpr int kWarps = kHThreads / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto store = [&](int r, int c, float missing) {
         const int64_t row = row0 + r, col = col0 + c;
-        if (row >= p.m || col >= p.n)
-            continue;
         float x = 0.0f;
         for (int z = 0; z < slices; ++z) {
-            const float4 q = ld_cluster_f4(sums + (uint32_t)r * (uint32_t)(bn * 4) + (uint32_t)(((c >> 2) ^ (r & 7)) << 4), (uint32_t)z);
+            const float4 q = ld_cluster_f4(sums + (uint32_t)r * (uint32_t)(BN * 4) + (uint32_t)(((c >> 2) ^ (r & 7)) << 4), (uint32_t)z);
             const float v  = (c & 2) ? ((c & 1) ? q.w : q.z) : ((c & 1) ? q.y : q.x);
             x              = z == 0 ? v : __fadd_rn(x, v);
         }
-        float missing[1];
-        const float cs = p.col_scale[col], rs = p.row_scale[row];
-        x = __fmul_rn(x, fabsf(cs));
-        if (rs < 0.0f || cs < 0.0f) {
-            half_missing<1>(p, row, rs < 0.0f, col, 1, missing);
-            x = __fadd_rn(x, missing[0]);
-        }
+        x = __fadd_rn(__fmul_rn(x, fabsf(p.col_scale[col])), missing);
         if (p.bias)
             x = __fadd_rn(x, p.bias[p.bias_per_row ? row : col]);
         if (p.act == CT_ACT_RELU)
             x = __fmul_rn(x, x > 0.0f ? 1.0f : 0.0f);
         p.out[row * p.n + col] = x;
-    }
+    };
+    auto row_has = [&](int r) { return row0 + r < p.m && p.row_scale[row0 + r] < 0.0f; };
+    for (int b = 0; b < rows; b += 32)
+        for (uint32_t m = __ballot_sync(0xffffffffu, b + lane < rows && row_has(r0 + b + lane)); m; m &= m - 1) {
+            const int r = b + __ffs(m) - 1;
+            if (r % kWarps != warp)
+                continue;
+            const int64_t col = col0 + lane;
+            const int count   = (int)(p.n <= col ? 0 : min((int64_t)(BN / 32), (p.n - col + 31) / 32));
+            float missing[BN / 32];
+            half_missing<BN / 32>(p, row0 + r0 + r, true, col, count, missing);
+#pragma unroll
+            for (int u = 0; u < BN / 32; ++u)
+                if (u < count)
+                    store(r0 + r, lane + 32 * u, missing[u]);
+        }
+    for (int b = 0; b < BN; b += 32)
+        for (uint32_t m = __ballot_sync(0xffffffffu, col0 + b + lane < p.n && p.col_scale[col0 + b + lane] < 0.0f); m; m &= m - 1) {
+            const int c = b + __ffs(m) - 1;
+            if (c % kWarps != warp)
+                continue;
+            for (int r = r0 + lane; r < r0 + rows; r += 32)
+                if (row0 + r < p.m && !row_has(r)) {
+                    float missing[1];
+                    half_missing<1>(p, row0 + r, false, col0 + c, 1, missing);
+                    store(r, c, missing[0]);
+                }
+        }
 }
 
 template <int BN, int CG>
@@ -710,9 +732,7 @@ __global__ void __launch_bounds__(kHThreads, 1)
         half_tile(p, first, tm, tn, tz, band);
         const int rows_each = kHM / slices;
         const bool vec      = (p.n & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
-        if (!failed && !abort_flag_s && lacking_s)
-            half_finish_slices(p, smem_base, slices, (int)cluster_rank() * rows_each, rows_each, (int64_t)tm * kHM, (int64_t)tn * BN, BN);
-        else if (!failed && !abort_flag_s)
+        if (!failed && !abort_flag_s)
             for (int i = threadIdx.x; i < rows_each * (BN / 4); i += kHThreads) {
                 const int r = (int)cluster_rank() * rows_each + i / (BN / 4), slot = i % (BN / 4);
                 const int64_t row = (int64_t)tm * kHM + r, col = (int64_t)tn * BN + slot * 4;
@@ -729,7 +749,7 @@ __global__ void __launch_bounds__(kHThreads, 1)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     if (col + q < p.n) {
-                        x[q] = __fmul_rn(x[q], wide ? 1.0f : p.col_scale[col + q]);
+                        x[q] = __fmul_rn(x[q], wide ? 1.0f : fabsf(p.col_scale[col + q]));
                         if (p.bias)
                             x[q] = __fadd_rn(x[q], p.bias[p.bias_per_row ? row : col + q]);
                         if (p.act == CT_ACT_RELU)
@@ -746,6 +766,10 @@ __global__ void __launch_bounds__(kHThreads, 1)
                             dst[q] = x[q];
                 }
             }
+        if (lacking_s && !failed && !abort_flag_s) {
+            __syncthreads(); // what follows writes some of these outputs again
+            half_finish_slices<BN>(p, smem_base, slices, (int)cluster_rank() * rows_each, rows_each, (int64_t)tm * kHM, (int64_t)tn * BN);
+        }
         cluster_sync(); // a CTA's sums stay until every other CTA has read them
     }
 

@@ -100,11 +100,16 @@ __device__ __forceinline__ void split_half_pair(float a, float b, __half2 &hi, _
     lo = __floats2half2_rn(__fmul_rn(__fsub_rn(a, __low2float(hi)), kHalfLoScale), __fmul_rn(__fsub_rn(b, __high2float(hi)), kHalfLoScale));
 }
 
-// Whether either operand needs its tf32 planes: one 8-byte load for each list (operands prepared together share one), both
-// in flight - as four loads in a row they cost an idle launch 3 us.
+// Whether either operand needs its tf32 planes: one 8-byte load for each list, and one in all where they share it.  As
+// four loads in a row they cost an idle launch 3 us, and a second volatile load of the same words 0.8 us.
 __device__ __forceinline__ bool half_wide(const HalfExceptions *a, const HalfExceptions *b) {
-    const uint64_t va = *reinterpret_cast<const volatile uint64_t *>(a), vb = *reinterpret_cast<const volatile uint64_t *>(b);
-    return ((uint32_t)va | (uint32_t)vb) != 0u || max((uint32_t)(va >> 32), (uint32_t)(vb >> 32)) > kHalfExceptions;
+    const uint64_t va = *reinterpret_cast<const volatile uint64_t *>(a);
+    bool wide         = (uint32_t)va != 0u || (uint32_t)(va >> 32) > kHalfExceptions;
+    if (a != b) {
+        const uint64_t vb = *reinterpret_cast<const volatile uint64_t *>(b);
+        wide |= (uint32_t)vb != 0u || (uint32_t)(vb >> 32) > kHalfExceptions;
+    }
+    return wide;
 }
 
 // More exceptions than the list holds: the rest need not be looked for.
