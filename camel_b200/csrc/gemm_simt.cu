@@ -9,6 +9,7 @@
 #include "fastmath.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 
 namespace ct {
@@ -307,6 +308,7 @@ ct_status launch_skinny_smem(
 // once and does the activation; softmax and argmax scan the columns in order like the reference.
 constexpr int kFewWarps = 8;
 constexpr int kFewRing  = 64; // activations in a lane's ring: 8 warps x 64 x 128 B = 64 KB an SM, 1 - R / 64 of it in flight
+constexpr int kFewRingShort = 16; // where the weights leave room for no more
 
 // Asynchronous 4-byte copies into a ring that only the copying lane reads: the depth of the prefetch is then in
 // shared memory and in the hardware's group count, not in registers and their scoreboards - with register
@@ -404,11 +406,11 @@ __device__ __forceinline__ void few_reduce(double (&acc)[R][NE], int lane, doubl
     }
 }
 
-template <int NE, int R>
+template <int NE, int R, int RING>
 __global__ void __launch_bounds__(32 * kFewWarps, 1) gemm_few_columns_kernel(
     const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ bias, int64_t m, int k, int n,
     int act, float *__restrict__ out, int64_t *__restrict__ argmax) {
-    constexpr int S = FewStride<NE>::value, D = kFewRing / R; // steps in the ring
+    constexpr int S = FewStride<NE>::value, D = RING / R; // steps in the ring
     extern __shared__ __align__(16) double w_few[]; // [k rounded up to 32][S], then the warps' rings [D][R][32] floats
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int steps = (k + 31) >> 5;
@@ -417,7 +419,7 @@ __global__ void __launch_bounds__(32 * kFewWarps, 1) gemm_few_columns_kernel(
     // the walk of a warp: tiles of R rows, 32 values of k a step; the fetch runs D - 1 steps ahead of it, across tiles
     const int64_t tiles = (m + R - 1) / R, first = (int64_t)blockIdx.x + (int64_t)warp * gridDim.x;
     const int64_t stride = (int64_t)gridDim.x * kFewWarps;
-    float *ring = reinterpret_cast<float *>(w_few + (size_t)steps * 32 * S) + warp * kFewRing * 32 + lane;
+    float *ring = reinterpret_cast<float *>(w_few + (size_t)steps * 32 * S) + warp * RING * 32 + lane;
     const uint32_t ring_a = (uint32_t)__cvta_generic_to_shared(ring);
     int64_t f_tile = first;
     int f_step = 0, f_slot = 0;
@@ -556,42 +558,65 @@ __global__ void __launch_bounds__(32 * kFewWarps) gemm_few_rows_kernel(
     }
 }
 
+// Blocks of gemm_few_rows_kernel that fit the machine at once.
+template <int NE, int R> int few_rows_per_wave(const DeviceState *st) {
+    static std::atomic<int> per_sm{0};
+    int fit = per_sm.load(std::memory_order_relaxed);
+    if (fit == 0) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, gemm_few_rows_kernel<NE, R>, 32 * kFewWarps, 0) != cudaSuccess || fit < 1)
+            fit = 1;
+        per_sm.store(fit, std::memory_order_relaxed);
+    }
+    return fit * st->sm_count;
+}
+
 template <int NE>
 ct_status launch_few(
     DeviceState *st, const float *a, const float *b, const float *bias, int64_t m, int64_t k, int n, int act, float *out,
     int64_t *argmax) {
-    const size_t smem = (size_t)((k + 31) / 32 * 32) * FewStride<NE>::value * sizeof(double) + kFewWarps * kFewRing * 128;
-    // Resident weights pay from where a block's warps get a few tiles each (k = 785, n = 10: 9.7 against 21.8 us at
-    // 2048 rows, 12.5 us both ways at 1024); below, and for weights beyond shared memory, blocks of four (two) rows
-    // read them from L2.
-    if (smem <= 220 * 1024 && m >= 2048) {
+    constexpr size_t kMost = 220 * 1024;
+    const size_t weights   = (size_t)((k + 31) / 32 * 32) * FewStride<NE>::value * sizeof(double);
+    const bool longer      = weights + kFewWarps * kFewRing * 128 > kMost;
+    const size_t smem      = weights + kFewWarps * (longer ? kFewRingShort : kFewRing) * 128;
+    // What the two kernels take, in us.  Blocks of four (two) rows: a wave of them costs the same whatever k is beyond
+    // 800, and there are few to a wave (one to an SM at ten columns).  Resident weights: staging them, then a cost
+    // per activation and FMA.  Measured / by these (k x n at m): blocks 785 x 10 7.0 / 7.0 at 512 and 11.4 / 12.5 at 640,
+    // 785 x 16 9.9 / 11.0 and 17.6 / 20.6, 300 x 10 6.3 / 6.7 at 640, 785 x 5 8.9 / 8.8 at 2047; resident 785 x 10
+    // 9.3 / 9.7 at 640 and 11.2 / 13.2 at 4096, 785 x 16 13.7 / 13.2 at 640, 1500 x 10 14.6 / 15.2, 785 x 5 7.1 / 8.4 at 2047.
+    const int64_t blocks = m <= 2 * st->sm_count ? (m + 1) / 2 : (m + 3) / 4;
+    const int wave       = m <= 2 * st->sm_count ? few_rows_per_wave<NE, 2>(st) : few_rows_per_wave<NE, 4>(st);
+    const double by_rows = 1.5 + (double)((blocks + wave - 1) / wave) * ((NE > 12 ? 2.0 : 0.8) + 6e-4 * NE * (double)std::min<int64_t>(k, 800));
+    const double resident = 3.5 + 7e-4 * NE * (double)k + (double)m * (double)k * (6e-7 + 7e-8 * NE);
+    if (smem <= kMost && resident < by_rows) {
         // eight rows per warp where there are rows enough for two such tiles each and the sums stay in registers
-        const bool deep = NE <= 12 && m >= (int64_t)st->sm_count * kFewWarps * 8 * 2;
+        const bool deep = NE <= 12 && !longer && m >= (int64_t)st->sm_count * kFewWarps * 8 * 2;
+        constexpr int kDeep     = NE <= 12 ? 8 : 4;
         static bool attr_set_dev[16] = {};
         if (!attr_set_dev[st->device & 15]) {
-            CT_CUDA(cudaFuncSetAttribute(gemm_few_columns_kernel<NE, (NE <= 12 ? 8 : 4)>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-            CT_CUDA(cudaFuncSetAttribute(gemm_few_columns_kernel<NE, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+            CT_CUDA(cudaFuncSetAttribute(gemm_few_columns_kernel<NE, kDeep, kFewRing>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
+            CT_CUDA(cudaFuncSetAttribute(gemm_few_columns_kernel<NE, 4, kFewRing>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
+            CT_CUDA(cudaFuncSetAttribute(gemm_few_columns_kernel<NE, 4, kFewRingShort>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
             attr_set_dev[st->device & 15] = true;
         }
-        constexpr int kDeep  = NE <= 12 ? 8 : 4;
-        const int rows       = deep ? kDeep : 4;
-        const int64_t tiles  = (m + rows - 1) / rows;
-        const unsigned grid  = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
-        if (deep)
-            CT_CUDA(launch_dependent(gemm_few_columns_kernel<NE, kDeep>, dim3(grid), dim3(32 * kFewWarps), smem, stream(), a, b, bias, m,
-                                     (int)k, n, act, out, argmax));
-        else
-            CT_CUDA(launch_dependent(gemm_few_columns_kernel<NE, 4>, dim3(grid), dim3(32 * kFewWarps), smem, stream(), a, b, bias, m,
-                                     (int)k, n, act, out, argmax));
+        const int rows      = deep ? kDeep : 4;
+        const int64_t tiles = (m + rows - 1) / rows;
+        const unsigned grid = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
+        auto kernel         = longer ? gemm_few_columns_kernel<NE, 4, kFewRingShort>
+                                     : (deep ? gemm_few_columns_kernel<NE, kDeep, kFewRing> : gemm_few_columns_kernel<NE, 4, kFewRing>);
+        CT_CUDA(launch_dependent(kernel, dim3(grid), dim3(32 * kFewWarps), smem, stream(), a, b, bias, m, (int)k, n, act, out, argmax));
         CT_LAUNCH_CHECK("gemm_few_columns");
         return CT_OK;
     }
+    // weights that fit shared memory only without padding and ring: 1500 x 16 121 against 153 us at 8192 rows, 751 against
+    // 1255 at 60000, 76 both ways at 4096; up to eight columns the blocks of rows are faster (3000 x 8: 189 against 228)
+    if (smem > kMost && NE > 8 && m >= 4096 && (size_t)k * n * sizeof(double) <= 200 * 1024)
+        return launch_skinny_smem<16>(st, a, b, bias, m, k, n, act, out, argmax);
     if (m <= 2 * st->sm_count)
-        CT_CUDA(launch_dependent(gemm_few_rows_kernel<NE, 2>, dim3((unsigned)((m + 1) / 2)), dim3(32 * kFewWarps), 0, stream(), a, b,
-                                 bias, m, k, n, act, out, argmax));
+        CT_CUDA(launch_dependent(gemm_few_rows_kernel<NE, 2>, dim3((unsigned)blocks), dim3(32 * kFewWarps), 0, stream(), a, b, bias, m, k, n,
+                                 act, out, argmax));
     else
-        CT_CUDA(launch_dependent(gemm_few_rows_kernel<NE, 4>, dim3((unsigned)((m + 3) / 4)), dim3(32 * kFewWarps), 0, stream(), a, b,
-                                 bias, m, k, n, act, out, argmax));
+        CT_CUDA(launch_dependent(gemm_few_rows_kernel<NE, 4>, dim3((unsigned)blocks), dim3(32 * kFewWarps), 0, stream(), a, b, bias, m, k, n,
+                                 act, out, argmax));
     CT_LAUNCH_CHECK("gemm_few_rows");
     return CT_OK;
 }
@@ -876,12 +901,7 @@ ct_status gemm_f32_skinny(
     if ((size_t)k * n * sizeof(double) <= 200 * 1024 && k > 0) {
         return launch_skinny_smem<32>(st, a, b, bias, m, k, (int)n, act, out, argmax);
     }
-    if (n <= 8)
-        gemm_skinny_kernel<8><<<blocks, 256, 0, stream()>>>(a, b, bias, m, k, (int)n, act, out, argmax);
-    else if (n <= 16)
-        gemm_skinny_kernel<16><<<blocks, 256, 0, stream()>>>(a, b, bias, m, k, (int)n, act, out, argmax);
-    else
-        gemm_skinny_kernel<32><<<blocks, 256, 0, stream()>>>(a, b, bias, m, k, (int)n, act, out, argmax);
+    gemm_skinny_kernel<32><<<blocks, 256, 0, stream()>>>(a, b, bias, m, k, (int)n, act, out, argmax);
     CT_LAUNCH_CHECK("gemm_skinny");
     return CT_OK;
 }
