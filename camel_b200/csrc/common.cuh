@@ -217,7 +217,7 @@ struct HalfBands {
 ct_status gemm_half(
     DeviceState *st, const HalfOperand &a, const HalfOperand &b, int64_t kp, const float *bias, int act, float *out,
     bool force_wide, bool allow_splitk, const HalfBands *bands, int batch = 1, bool bias_per_row = false);
-int half_tile_columns(const DeviceState *st, int64_t m, int64_t n, int64_t batch = 1);
+int gemm_tile_columns(const DeviceState *st, int64_t m, int64_t n, int64_t batch = 1); // of gemm_half and gemm_planes
 // Pre-passes: rows of a row-major matrix, columns of one (transposed planes); both record exceptions.  `zero`
 // words are cleared on the way (scales and col_max of a following half_split_cols, which needs them at zero).
 // both_forms: the tf32 planes are written as well (no half_wide_planes needed).

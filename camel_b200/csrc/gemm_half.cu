@@ -1374,7 +1374,7 @@ ct_status half_widen_rows(DeviceState *st, const HalfOperand &o, int64_t kp) {
 }
 
 // Tile width: 128 x 256 where such tiles fill at least half of the machine, else 128 x 128.
-int half_tile_columns(const DeviceState *st, int64_t m, int64_t n, int64_t batch) {
+int gemm_tile_columns(const DeviceState *st, int64_t m, int64_t n, int64_t batch) {
     const int64_t tiles256 = ((m + kHM - 1) / kHM) * ((n + 255) / 256) * batch;
     return n > 128 && tiles256 >= st->sm_count / 2 ? 256 : 128;
 }
@@ -1383,7 +1383,7 @@ ct_status gemm_half(
     DeviceState *st, const HalfOperand &a, const HalfOperand &b, int64_t kp, const float *bias, int act, float *out,
     bool force_wide, bool allow_splitk, const HalfBands *bands, int batch, bool bias_per_row) {
     const int64_t m = a.rows, n = b.rows / batch;
-    const int bn    = half_tile_columns(st, m, n, batch);
+    const int bn    = gemm_tile_columns(st, m, n, batch);
     HalfGemmParams p{};
     p.m = m, p.n = n;
     p.batch            = batch;

@@ -1573,8 +1573,7 @@ ct_status gemm_planes(
     const void *b_lo, int64_t m, int64_t n, int64_t kp, const float *bias, int act, float *out,
     int batch, int64_t out_batch_stride, int bias_per_row, const ConvGeom *conv) {
     // 128 x 256 tiles when they fill the machine, 128 x 128 otherwise
-    int64_t tiles256 = ((m + BM - 1) / BM) * ((n + 255) / 256) * batch;
-    bool wide        = n > 128 && tiles256 >= st->sm_count / 2;
+    bool wide = gemm_tile_columns(st, m, n, batch) == 256;
     if (conv && m <= 64 && conv->wo <= 128 && kp <= 1024 * (mode == MODE_3X ? 1 : 2) && bias_per_row == (bias ? 1 : 0)) {
         // few output channels: pixels on the accumulator rows, channels on its columns; the whole k
         // range is one accumulation, so k stays within what keeps the error at float32 level
@@ -2056,7 +2055,6 @@ extern "C" ct_status ct_matmul_packed_bands(
     plan.done    = band_done_dev;
     int64_t row  = 0;
     plan.first[0] = 0;
-    const bool wide = pw->n > 128; // the tile width launch_gemm will pick is decided in gemm_planes; counts below use it
     for (int b = 0; b < nbands; ++b) {
         const int64_t rows = band_rows_host[b];
         if (rows <= 0 || !band_out_host[b] || (b + 1 < nbands && rows % BM != 0))
@@ -2069,10 +2067,9 @@ extern "C" ct_status ct_matmul_packed_bands(
     if (row != pr->m)
         return fail(CT_ERR_INVALID, "ct_matmul_packed_bands: the bands hold %lld rows, the packed matrix %lld",
                     (long long)row, (long long)pr->m);
-    // the tile width gemm_planes will choose (same rule)
-    const int64_t tiles256 = ((pr->m + BM - 1) / BM) * ((pw->n + 255) / 256);
-    const bool bn256       = wide && tiles256 >= st->sm_count / 2;
-    const int64_t tiles_n  = (pw->n + (bn256 ? 255 : 127)) / (bn256 ? 256 : 128);
+    // what the launch below takes: a count that it does not reach would leave the waiting stream waiting
+    const int tile        = gemm_tile_columns(st, pr->m, pw->n);
+    const int64_t tiles_n = (pw->n + tile - 1) / tile;
     for (int b = 0; b < nbands; ++b)
         if (band_tiles_host)
             band_tiles_host[b] = (uint32_t)((plan.first[b + 1] - plan.first[b]) * tiles_n);
