@@ -1409,8 +1409,9 @@ ct_status gemm_half(
             p.band_out_off[i] = bands->out_off[i];
     }
     // Few output tiles: slice k across CTAs so that more of the machine works.  Up to eight slices of a tile
-    // are a cluster that adds them up itself; only where one to nine tiles and a long k (a 12544 -> 128 layer
-    // on a small batch) leave room for more do the partial sums go through a workspace and a second launch.
+    // are a cluster that adds them up itself; only where ten to sixteen tiles and a k beyond 4500 (a 12544 -> 128 layer
+    // on 1153 to 2048 rows; fewer tiles with such a k take the tf32 planes) leave room for more do the partial sums go
+    // through a workspace and a second launch.
     const int64_t tiles = ((m + kHM - 1) / kHM) * ((n + bn - 1) / bn);
     int splits          = 1;
     if (allow_splitk && !bands && batch == 1 && bn == 128 && tiles * 2 <= st->sm_count) {

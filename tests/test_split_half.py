@@ -33,11 +33,13 @@ def _check(got, a, b):
     assert np.all(err <= BOUND * (np.abs(a64) @ np.abs(b64)) + 1e-300)
 
 
-# one tile and its edges; slices in a cluster with an empty last one (k = 320: five groups of 64 over four);
-# the drain after 1024 values of k; pairs of CTAs with a ragged last tile; long columns (two passes over B);
-# few rows and a long k (slices through the workspace)
-SHAPES = [(64, 64, 64), (128, 32, 128), (129, 33, 257), (128, 320, 128), (65, 1025, 130), (300, 2080, 260),
-          (4100, 96, 1030), (2304, 1056, 2306), (130, 4128, 131), (40, 9000, 70), (33, 4096, 36), (70, 1500, 66)]
+# one tile and its edges; slices in a cluster, the last one empty (k = 570: nine groups of 64 over four slices;
+# 1088: seventeen over eight); the drain after 1024 values of k; long columns (two passes over B); pairs of CTAs with a
+# ragged last tile, also without slices beyond 2048; ten tiles and a long k (slices through the workspace); several
+# tiles to a block over both accumulator sets; at most nine tiles or one row of them and k beyond 2048 (tf32 planes)
+SHAPES = [(64, 64, 64), (128, 32, 128), (129, 33, 257), (128, 570, 128), (100, 1088, 130), (65, 1025, 130), (70, 1500, 66),
+          (4100, 96, 1030), (2304, 1056, 2306), (1100, 2208, 2306), (1280, 5000, 128), (40000, 96, 100),
+          (300, 2080, 260), (130, 4128, 131), (40, 9000, 70)]
 
 
 @pytest.mark.parametrize("m,k,n", SHAPES)
