@@ -767,9 +767,9 @@ class KernelFamilyWorkload(Workload):
             self.rows, self.k = 16384, 8192
             self.x = wrap(rand(self.rows, self.k))
             self.packed = C.c_void_p()
-            self.bytes = 12.0 * self.rows * self.k
+            self.bytes = 8.0 * self.rows * self.k
             self.dominant = "gemm_prepass"
-            self.desc = f"operand pre-pass of the 3xTF32 GEMM over {self.rows} x {self.k} float32 (4 B read, 8 B written per element)"
+            self.desc = f"operand pre-pass of the float32 GEMM over {self.rows} x {self.k} values (4 B read, 4 B written as float16 pairs per element)"
         else:
             raise ValueError(kind)
 
