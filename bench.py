@@ -1,9 +1,9 @@
 #!/usr/bin/env python
 """Benchmark of the tensor hot path: `python bench.py --gpus N --steps K --warmup W`.
 
-With no --workload the headline is the MLP forward; the same run then
-measures, a few steps each, every other configuration and kernel family and attaches them to the
-one JSON line under "extras" (so that every quoted number has a line in a driver-run record).
+With no --workload the headline is the MLP forward; the same run then measures, a few steps each, every
+other configuration and kernel family.  Standard output is ONE JSON line, the headline's, kept short enough
+for a reader that takes the end of a log; the other measurements are JSON lines on standard error.
 
 Workloads (seeded synthetic inputs with the shapes and distributions of the reference
 configurations; no dataset is used):
@@ -226,8 +226,8 @@ def run_reference(args, rank):
     t = max(r[2] for r in results)  # the slowest shard bounds the step
     value = units * workers / t
     # the same workload description as the GPU arm prints for this --workload
-    workload = {"mlp": "mlp_forward 784-1024-1024-10 relu,relu,softmax+argmax (BASELINE configs[1])",
-                "gemm": f"gemm fp32 M=N=K={args.size} U(-1,1) (BASELINE configs[4] per-GPU problem)"}[args.workload]
+    workload = {"mlp": "mlp_forward 784-1024-1024-10 relu,relu,softmax+argmax",
+                "gemm": f"gemm fp32 M=N=K={args.size} U(-1,1)"}[args.workload]
     line = {"impl": "reference", "metric": metric, "value": value, "unit": unit, "n_gpus": args.gpus, "steps": steps,
             "warmup": warmup, "ms_per_step": t * 1e3, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f32 (float64 accumulate, the reference's arithmetic)", "data": "synthetic",
@@ -379,7 +379,7 @@ class MlpWorkload(Workload):
         return self.x.nbytes + sum(t.nbytes for t in self.w) + 2 * self.batch * 1024 * 4
 
     def config(self):
-        return {"workload": "mlp_forward 784-1024-1024-10 relu,relu,softmax+argmax (BASELINE configs[1])",
+        return {"workload": "mlp_forward 784-1024-1024-10 relu,relu,softmax+argmax",
                 "batch_per_gpu": self.batch, "precision": "3xtf32",
                 "weights": "tensor-core layout kept with each weight tensor (built at first use)"
                 if self.T._weight_cache else "transposed and split at every call"}
@@ -434,12 +434,12 @@ class GemmWorkload(Workload):
         return 3 * self.n * self.n * 4
 
     def config(self):
-        return {"workload": f"gemm fp32 M=N=K={self.n} U(-1,1) (BASELINE configs[4] per-GPU problem)",
+        return {"workload": f"gemm fp32 M=N=K={self.n} U(-1,1)",
                 "precision": self.precision}
 
 
 class ShardedGemmWorkload(Workload):
-    """BASELINE configs[4] as one job: C = A.B with M=N=K=n, A split by rows over the ranks, B
+    """One product as one job: C = A.B with M=N=K=n, A split by rows over the ranks, B
     replicated (placed once, outside the timed region), every rank ends up with all of C.  The
     only exchange is the all-gather of C row blocks (NCCL over NVLink); it is issued per row panel
     on a side stream so that panel j travels while panel j+1 is computed.  Strong scaling."""
@@ -530,7 +530,7 @@ class ShardedGemmWorkload(Workload):
     def config(self):
         return {"workload": f"gemm fp32 M=N=K={self.n}, A row-sharded over {self.world} ranks, C all-gathered "
                             f"in place in {self.panels} bands of halving size (one launch, a band travels as soon as its tiles are done), B and its tensor-core layout "
-                            f"placed once (BASELINE configs[4])",
+                            f"placed once",
                 "precision": "3xtf32", "e2e": "same as value: operands are resident by construction",
                 "parallelism": f"{self.world} ranks, rows of A and C sharded, NCCL all-gather of C on a side stream"}
 
@@ -567,7 +567,7 @@ class ConvWorkload(Workload):
         return self.h2d + self.d2h
 
     def config(self):
-        return {"workload": "conv2d 64->128 56x56 3x3 pad1 +bias +relu (BASELINE configs[2])",
+        return {"workload": "conv2d 64->128 56x56 3x3 pad1 +bias +relu",
                 "batch_per_gpu": self.batch, "precision": "3xtf32"}
 
 
@@ -755,7 +755,7 @@ class KernelFamilyWorkload(Workload):
             self.x = wrap(rand(2048, 64, 28, 28))
             self.bytes = 5.0 * self.x.numel
             self.dominant = "maxpool"
-            self.desc = "maxpool2d 2x2 of 2048 x 64 x 28 x 28 (BASELINE configs[3] layer shape, a quarter of its batch)"
+            self.desc = "maxpool2d 2x2 of 2048 x 64 x 28 x 28"
         elif kind == "fill":
             self.n = 1 << 28
             self.out = T.Tensor(0, (self.n,))
@@ -812,7 +812,7 @@ class KernelFamilyWorkload(Workload):
 
 
 class Gemm512Workload(Workload):
-    """BASELINE configs[0]: fp32 GEMM M=N=K=512, U(-1,1), seed 0, through the matmul operator.
+    """fp32 GEMM M=N=K=512, U(-1,1), seed 0, through the matmul operator.
     0.27 GFLOP: launch- and latency-bound, reported without a roofline expectation."""
 
     name, metric, unit = "gemm512", "gemm_fp32_tflops", "TFLOP/s"
@@ -837,12 +837,12 @@ class Gemm512Workload(Workload):
         return 3 * 512 * 512 * 4
 
     def config(self):
-        return {"workload": "gemm fp32 M=N=K=512 U(-1,1) seed 0 (BASELINE configs[0]): latency-bound",
+        return {"workload": "gemm fp32 M=N=K=512 U(-1,1) seed 0: latency-bound",
                 "precision": "3xtf32"}
 
 
 class CnnWorkload(Workload):
-    """conv 1->32 +relu, conv 32->64 +relu, 2x2 maxpool, flatten,
+    """A small CNN: conv 1->32 +relu, conv 32->64 +relu, 2x2 maxpool, flatten,
     dense 12544->128 +relu, dense 128->10 +softmax, on 1x28x28 Uniform(0,1) images."""
 
     name, metric, unit = "cnn", "cnn_forward_samples_per_s", "samples/s"
@@ -921,7 +921,7 @@ class CnnWorkload(Workload):
         return self.batch * 64 * 28 * 28 * 4
 
     def config(self):
-        return {"workload": "cnn_forward conv32-conv64-pool-dense128-dense10 on 1x28x28 (BASELINE configs[3])",
+        return {"workload": "cnn_forward conv32-conv64-pool-dense128-dense10 on 1x28x28",
                 "batch_per_gpu": self.batch, "precision": "3xtf32",
                 "weights": "tensor-core layout kept with each weight tensor (built at first use)"
                 if self.T._weight_cache else "transposed and split at every call"}
@@ -1412,41 +1412,42 @@ def run_gpu(args, rank, world):
                            **wl.config(), "l2": "flushed between steps" if m["flush"] else "inputs larger than L2"},
                 "timed_region": {"blocks_of_steps": m["blocks"], "gpu_s": m["gpu_s"],
                                  "rule": "blocks of exactly `steps` timed steps; ms_per_step is the median block's"},
-                "gpu_launches": m["launches"], "roofline": roofline, "clocks": m["clocks"],
-                "kernel_families_per_step": m["scopes"]}
+                "gpu_launches": m["launches"], "roofline": roofline, "clocks": m["clocks"]}
+        details = {"kernel_families_per_step": m["scopes"]}
         if plugin is not None:
             # the headline end-to-end figure: through the plugin's operator bodies, host buffers in and out
             fused = plugin["fused_operators"]
             line["e2e"] = {"value": wl.batch * world / fused["seconds_per_step"], "unit": wl.unit,
                            "h2d_bytes_per_step": wl.h2d, "d2h_bytes_per_step": wl.d2h,
                            "seconds_per_step": fused["seconds_per_step"], "launches_per_step": fused["launches_per_step"],
-                           "mode": "per step: host batch in page-locked memory -> tensor (one synchronous copy), dense_relu, "
-                                   "dense_relu, dense_softmax, argmax through operator_t, host read-back of both results; "
-                                   "wall clock in C++ around the step, median step, slowest rank"}
+                           # host batch in page-locked memory -> tensor (one synchronous copy), dense_relu, dense_relu,
+                           # dense_softmax, argmax through operator_t, host read-back of both results
+                           "mode": "plugin operators, page-locked host batch in, both results read back; wall clock, median step"}
             pageable = plugin["fused_operators_pageable"]
-            line["e2e_plugin_pageable_host"] = {
+            details["e2e_plugin_pageable_host"] = {
                 "value": wl.batch * world / pageable["seconds_per_step"], "unit": wl.unit,
                 "seconds_per_step": pageable["seconds_per_step"],
                 "mode": "the same step with the host batch in ordinary (pageable) memory, where the reference's "
                         "allocator keeps large tensors: the copy is staged by the driver"}
             small = plugin["small_operators"]
-            line["e2e_plugin_small_operators"] = {
+            details["e2e_plugin_small_operators"] = {
                 "value": wl.batch * world / small["seconds_per_step"], "unit": wl.unit,
                 "seconds_per_step": small["seconds_per_step"], "launches_per_step": small["launches_per_step"],
                 "mode": "the same step written with the module's small operators (x @ w, h * (h > 0), the softmax "
                         "function of mnist.cml:13-25): deferred expressions recognised and fused by the plugin"}
             if e2e is not None:
-                line["e2e_pipelined"] = e2e
+                details["e2e_pipelined"] = e2e
         elif e2e is not None:
             line["e2e"] = e2e
         if mma is not None:
-            line["mma_peak"] = mma
-        if extras is not None:
-            line["extras"] = extras
+            details["mma_peak"] = mma
         if training is not None:
-            line["plugin_training_step"] = training
+            details["plugin_training_step"] = training
         if cpu is not None:
             line["cpu_baseline"] = cpu
+        for extra in [{"detail": k, "of": wl.metric, "measured": v} for k, v in details.items()] + (extras or []):
+            print(json.dumps(extra), file=sys.stderr)
+        sys.stderr.flush()
         print(json.dumps(line))
     if sampler is not None:
         sampler.stop()
@@ -1489,7 +1490,7 @@ def main():
                     choices=["default", "mlp", "gemm", "gemm512", "gemm_sharded", "conv", "cnn", "add", "relu", "exp", "log",
                              "mul", "scale", "gt", "sum", "softmax", "sum_axis0", "sum_axis1", "max_axis1",
                              "argmax_axis1", "argmax_rows", "transpose", "maxpool", "fill", "split_rows", "mma_peak"],
-                    help="default: the MLP forward as the headline plus every other workload under `extras`")
+                    help="default: the MLP forward as the headline, then every other workload (on standard error)")
     ap.add_argument("--no-extras", action="store_true", help="the headline only")
     ap.add_argument("--no-peak", action="store_true",
                     help="skip the tensor-pipe measurement (thousands of launches: unwanted under a profiler); the "
