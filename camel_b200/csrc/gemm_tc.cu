@@ -1763,10 +1763,12 @@ ct_status gemm_f32_tc(
     // One tile of rows, or at most nine tiles, and a long k: the product is a fraction of the operands' pre-pass, and what
     // the tf32 planes need - one pass over B and two launches less - outweighs it (70 x 4000 x 70 22.6 against 26.8 us,
     // 128 x 8000 x 128 26.5 against 32.6, 129 x 8000 x 129 30.8 against 35.7, 100 x 16000 x 9000 579 against 603; but
-    // 64 x 1500 x 64 22.5 against 17.6).  Only products whose k is sliced over CTAs: the others keep the bytes of
-    // ct_matmul_packed_rows.
+    // 64 x 1500 x 64 22.5 against 17.6).  Up to eighteen tiles while gemm_half keeps their slices in clusters, of which
+    // four are all it takes then (500 x 3000 x 500 31 against 35; beyond k = 4608 it has more slices, and 1000 x 8000 x 200
+    // is 53 against 48, 200 x 8000 x 1000 58 against 60).  Only products whose k is sliced over CTAs: the others keep the
+    // bytes of ct_matmul_packed_rows.
     const int64_t tiles  = ((m + BM - 1) / BM) * ((n + 127) / 128);
-    const bool tf32_form = kp > 2048 && (m <= BM || tiles <= 9) && tiles * 2 <= st->sm_count;
+    const bool tf32_form = kp > 2048 && (m <= BM || tiles <= (kp <= 4608 ? 18 : 9)) && tiles * 2 <= st->sm_count;
     if (mode == MODE_3X && !tf32_form)
         return gemm_f32_split(st, a, b, bias, m, k, n, kp, act, out, packed, a_is_km);
     size_t a_plane      = align_up((size_t)m * kp * elem);
