@@ -295,7 +295,8 @@ ct_status ct_dense(
  * caller keeps w_dev unchanged and alive (shapes with n <= 32 read w_dev itself).  Tensors of the
  * reference are immutable values (every operator returns a new tensor), which is what makes
  * caching by tensor sound; the reference itself has no counterpart of these two calls.
- * ct_weights_pack cannot be recorded into a graph. */
+ * A handle holds 12 bytes of device memory per value (float16 pairs and tf32 terms; 2 under
+ * CT_PREC_BF16).  ct_weights_pack cannot be recorded into a graph. */
 ct_status ct_weights_pack(const float *w_dev, int64_t k, int64_t n, void **packed_out);
 ct_status ct_weights_free(void *packed);
 
@@ -303,7 +304,7 @@ ct_status ct_weights_free(void *packed);
  * panels of a sharded product, each sent on its way while the next is computed).  ct_rows_pack
  * splits a [m][k] float32 matrix into planes of its own on the current stream; *packed_inout is
  * NULL on the first call and the returned handle afterwards, whose buffers are then refilled (same
- * shape and precision) without allocating.  ct_matmul_packed_rows computes
+ * shape and precision) without allocating; 12 bytes per value as above.  ct_matmul_packed_rows computes
  * out[rows][n] = A[row0 .. row0+rows) . W from two packed operands; it touches none of the
  * library's cached workspaces, so calls made under different ct_set_stream streams may run at the
  * same time (the caller orders them after the ct_rows_pack with events).  Same arithmetic as
@@ -357,7 +358,8 @@ ct_status ct_maxpool2d(
     float *out_dev);
 
 /* float32 matmul for callers that must not allocate.  No counterpart in the reference: it is
- * ct_matmul (float32 x float32, 3xTF32) with the kernel's operand planes held in a fixed
+ * ct_matmul (float32 x float32) with tf32 terms for all operands (three MMAs of kind::tf32; ct_matmul itself
+ * takes float16 pairs, see ct_precision: same error bound, other bits) and the kernel's operand planes in a fixed
  * 16 MiB array inside the library instead of a workspace that grows on demand.  It is meant for
  * a host that calls into the library where device allocation is off limits - under a fixed
  * memory budget, while other threads have work in flight that a cudaMalloc would stall, or in

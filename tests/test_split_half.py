@@ -327,6 +327,50 @@ def test_few_channel_layers_on_two_streams_share_no_state(T):
         assert all(o.numpy().tobytes() == want[j] for o in outs[j])
 
 
+# filters in tensor memory, halos, patches; a product of one wave and one with a conditional launch in front
+@pytest.mark.parametrize("what", [(6, 32, 28, 28, 64, 3, 1, 1), (3, 64, 30, 28, 128, 3, 1, 1), (2, 48, 21, 23, 70, 3, 2, 1),
+                                  (256, 200, 256), (1500, 700, 900)])
+def test_recorded_calls_decide_on_every_replay(T, what):
+    """The same graph over ordinary values, one small one, and values that need tf32 terms: the bytes of eager calls."""
+    import ctypes as C
+
+    from camel_b200._lib import check, lib
+
+    rng = np.random.default_rng(sum(what))
+    conv = len(what) > 3
+    shape = what[:4] if conv else what[:2]
+    plain = rng.standard_normal(shape).astype(np.float32)
+    one, wide = plain.copy(), plain * np.exp2(rng.integers(-45, 45, shape)).astype(np.float32)
+    one.flat[one.size // 3] = 1e-12
+    w = rng.standard_normal((what[4], what[1], what[5], what[5]) if conv else what[1:]).astype(np.float32)
+    inputs, tw = [T.from_numpy(v) for v in (plain, one, wide, plain)], T.from_numpy(w)
+    if conv:
+        n, c, h, wd, ko, kern, stride, pad = what
+        out_shape = (n, ko, (h + 2 * pad - kern) // stride + 1, (wd + 2 * pad - kern) // stride + 1)
+        call = lambda x, o: check(lib.ct_conv2d(x.ptr, tw.ptr, None, n, c, h, wd, ko, kern, kern, stride, pad, 1, o.ptr))  # noqa: E731
+    else:
+        out_shape = (what[0], what[2])
+        call = lambda x, o: check(lib.ct_dense(x.ptr, tw.ptr, None, *what, 1, o.ptr, None))  # noqa: E731
+    want = []
+    for x in inputs:
+        o = T.zeros(out_shape)
+        call(x, o)
+        want.append(o.numpy().tobytes())
+    x, out, graph = T.from_numpy(plain), T.zeros(out_shape), C.c_void_p()
+    call(x, out)
+    check(lib.ct_graph_begin())
+    call(x, out)
+    check(lib.ct_graph_end(C.byref(graph)))
+    try:
+        for v, bytes_ in zip(inputs, want):
+            check(lib.ct_d2d(x.ptr, v.ptr, plain.nbytes))
+            check(lib.ct_graph_launch(graph))
+            assert out.numpy().tobytes() == bytes_
+        T.check_async()
+    finally:
+        check(lib.ct_graph_destroy(graph))
+
+
 # (n, c, h, w, ko, kernel, stride, pad): patches in registers and read twice (k = 1200), odd sizes; halos with a
 # partial last tile, channels that do not fill a block, more than 128 filters, 1 x 1 and 5 x 5 taps
 CONVS = [(3, 48, 21, 23, 70, 3, 2, 1), (2, 8, 33, 21, 20, 3, 2, 0), (2, 48, 15, 16, 40, 5, 3, 2), (2, 12, 24, 24, 65, 5, 1, 2),
