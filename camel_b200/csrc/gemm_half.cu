@@ -1375,6 +1375,28 @@ ct_status half_widen_rows(DeviceState *st, const HalfOperand &o, int64_t kp) {
     return CT_OK;
 }
 
+// How many clusters of `size` CTAs of the 128 x 128 product run at the same time.
+static int half_clusters(const DeviceState *st, int size) {
+    static int known[16][4] = {}; // per device, by log2(size); under the entry points' lock
+    int &count = known[st->device & 15][size == 8 ? 3 : size / 2];
+    if (count == 0) {
+        using C = HalfCfg<128, 1>;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)size, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)(st->sm_count / size * size)), cfg.blockDim = dim3(kHThreads);
+        cfg.dynamicSmemBytes = C::kSmemBytes;
+        cfg.attrs = attr, cfg.numAttrs = 1;
+        if (cudaFuncSetAttribute(gemm_half_kernel<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&count, gemm_half_kernel<128, 1>, &cfg) != cudaSuccess || count < 1) {
+            cudaGetLastError();
+            count = st->sm_count / size / 2 + 1; // not known: half of the machine
+        }
+    }
+    return count;
+}
+
 // Tile width: 128 x 256 where such tiles fill at least half of the machine, else 128 x 128.
 int gemm_tile_columns(const DeviceState *st, int64_t m, int64_t n, int64_t batch) {
     const int64_t tiles256 = ((m + kHM - 1) / kHM) * ((n + 255) / 256) * batch;
@@ -1420,9 +1442,10 @@ ct_status gemm_half(
         splits = (int)std::min<int64_t>(std::min<int64_t>(st->sm_count / tiles, p.k_groups / 8), 32);
         if (splits <= 8) {
             splits = 1;
-            // at least 128 values of k each; eight slices only up to half of the machine - whole clusters of eight
-            // do not fit every SM, and 16 of them (2000 x 1024 x 100) ran in two waves
-            while (splits < 8 && tiles * splits * 2 <= (splits == 4 ? st->sm_count / 2 : st->sm_count) && p.k_groups >= splits * 4)
+            // at least 128 values of k each, and as many slices as whole clusters of them fit the machine at once, which
+            // is fewer than its SMs would hold: 33 of four and 15 of eight (36 of four ran in two waves, 1498 x 2747 x 320
+            // 57 us where two slices take 49; 16 of eight, 2000 x 1024 x 100, 32 us where four take 25)
+            while (splits < 8 && tiles <= half_clusters(st, splits * 2) && p.k_groups >= splits * 4)
                 splits *= 2;
             p.cluster_split = splits;
         }
