@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256) im2col_planes_kernel(
 // WIDE: the tf32 terms instead, in planes of floats, where the exceptions ask for them.
 constexpr int kPatchRegs = 16; // pairs of values per lane: patches of up to 1024 values
 template <int V, bool WIDE>
-__global__ void __launch_bounds__(256) im2col_half_kernel(
+__global__ void __launch_bounds__(256, V == kPatchRegs ? 4 : 0) im2col_half_kernel(
     const float *__restrict__ x, int c, int h, int w, int kh, int kw, int stride, int pad, int ho, int wo, int kdim, int kp,
     int64_t rows, void *__restrict__ plane_hi, void *__restrict__ plane_lo, float *__restrict__ scale_out,
     HalfExceptions *__restrict__ exceptions) {
@@ -86,9 +86,12 @@ __global__ void __launch_bounds__(256) im2col_half_kernel(
         const float *src = x + (int64_t)img * c * h * w + (int64_t)y0 * w + x0;
         auto load        = [&](int kk) {
             const int2 at = where[kk];
-            const int iy = y0 + (at.y >> 16), ix = x0 + (at.y & 0xffff);
-            return (iy >= 0 && iy < h && ix >= 0 && ix < w) ? __ldg(src + at.x) : 0.0f; // padding elements lie far outside
+            const int iy = y0 + (at.y >> 16), ix = x0 + (at.y & 0xffff); // padding elements lie far outside
+            return ((unsigned)iy < (unsigned)h && (unsigned)ix < (unsigned)w) ? __ldg(src + at.x) : 0.0f;
         };
+        // a long patch that lies inside its image needs no coordinates: most do, and issue is what bounds its two readings
+        const bool inside = y0 >= 0 && x0 >= 0 && y0 + kh <= h && x0 + kw <= w;
+        auto load_inside  = [&](int kk) { return kk < kdim ? __ldg(src + where[kk].x) : 0.0f; };
         if (WIDE) {
             float *hi = static_cast<float *>(plane_hi) + row * kp, *lo = static_cast<float *>(plane_lo) + row * kp;
 #pragma unroll 4
@@ -113,6 +116,10 @@ __global__ void __launch_bounds__(256) im2col_half_kernel(
 #pragma unroll
             for (int j = 0; j < V; ++j)
                 range_take(range, v[j].x), range_take(range, v[j].y);
+        } else if (inside) {
+#pragma unroll 4
+            for (int kk = lane; kk < kdim; kk += 32)
+                range_take(range, load_inside(kk));
         } else {
             for (int kk = lane; kk < kdim; kk += 32)
                 range_take(range, load(kk));
@@ -144,6 +151,10 @@ __global__ void __launch_bounds__(256) im2col_half_kernel(
             for (int j = 0; j < V; ++j)
                 if (64 * j + 2 * lane < kp)
                     put(64 * j + 2 * lane, v[j].x, v[j].y);
+        } else if (inside) {
+#pragma unroll 4
+            for (int kk = 2 * lane; kk < kp; kk += 64)
+                put(kk, load_inside(kk), load_inside(kk + 1));
         } else {
             for (int kk = 2 * lane; kk < kp; kk += 64)
                 put(kk, load(kk), load(kk + 1));
