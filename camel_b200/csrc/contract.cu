@@ -609,6 +609,14 @@ static int pooled_tile_rows(int64_t ho, int64_t wo) {
     return (int)(th & ~(int64_t)1);
 }
 
+// Float32 layers that conv_halo takes: all that fit its tiles, but for those with few channels on both sides, whose filters
+// stay on chip (conv_tmem.cu), and a handful of channels, most of whose block of 32 would be padding.
+static bool conv2d_takes_halo(
+    int64_t n, int64_t c, int64_t h, int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t stride, int64_t pad) {
+    return c >= 8 && n <= 65535 && !conv_tmem_applicable(c, h, wd, ko, kh, kw, stride, pad) &&
+           conv_halo_applicable((c + 31) / 32 * 32, h, wd, ko, kh, kw, stride, pad);
+}
+
 static ct_status conv2d_run(
     const float *x, const float *w, const float *bias, int64_t n, int64_t c, int64_t h,
     int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t stride, int64_t pad,
@@ -641,7 +649,8 @@ ct_status ct_conv2d_maxpool2(
     // two-step form run the same arithmetic; the pool is fused where that kernel can do it
     bool tmem_pool         = false;
     const bool tmem_kernel = kblock == 32 && conv_tmem_applicable(c, h, wd, ko, kh, kw, stride, pad, &tmem_pool);
-    const bool fused = tensor_core && stride == 1 && c >= 16 && (wo & 1) == 0 && (ho & 1) == 0 && conv_tile_rows(ho, wo) > 0 &&
+    const bool halo_kernel = kblock == 32 && conv2d_takes_halo(n, c, h, wd, ko, kh, kw, stride, pad);
+    const bool fused = tensor_core && !halo_kernel && stride == 1 && c >= 16 && (wo & 1) == 0 && (ho & 1) == 0 && conv_tile_rows(ho, wo) > 0 &&
                        n > 0 && (tmem_kernel ? tmem_pool : swap_kernel);
     if (fused)
         return conv2d_run(x, w, bias, n, c, h, wd, ko, kh, kw, stride, pad, act, out, 2);
@@ -723,11 +732,11 @@ static ct_status conv2d_run(
         // few channels on both sides: the filters stay in tensor memory, a tile's input is fetched once
         return conv_tmem_filters(st, x, w, bias, n, c, h, wd, ko, kh, kw, pad, act, pool, out);
     }
+    if (mode == 0 && pool == 0 && conv2d_takes_halo(n, c, h, wd, ko, kh, kw, stride, pad))
+        // one input halo per tile and channel block serves every tap (conv_halo.cu)
+        return conv_halo(st, x, w, n, c, (c + 31) / 32 * 32, h, wd, ko, kh, kw, stride, pad, bias, act, out);
     if (th > 0) {
         int64_t c_pad  = (c + kblock - 1) / kblock * kblock;
-        if (mode == 0 && pool == 0 && conv_halo_applicable(c_pad, h, wd, ko, kh, kw, stride, pad))
-            // many filters: one input halo per tile and channel block serves every tap (conv_halo.cu)
-            return conv_halo(st, x, w, n, c, c_pad, h, wd, ko, kh, kw, pad, bias, act, out);
         int64_t taps   = kh * kw;
         int64_t kp_i   = taps * c_pad;
         size_t w_plane = align_up((size_t)ko * kp_i * elem);

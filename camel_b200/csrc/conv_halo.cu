@@ -1,5 +1,5 @@
-// Implicit-GEMM conv2d (stride 1) for layers with many output channels: the input halo of a tile is
-// fetched once per channel block and serves all filter taps.
+// Implicit-GEMM conv2d (stride 1 to 3): the input halo of a tile is fetched once per channel block and serves all
+// filter taps.
 //
 // The streaming implicit GEMM of gemm_tc.cu fetches, for every (tap, channel block), the tile's
 // pixels again - the same values shifted by the tap.  Shared memory then carries, per k-block of 16
@@ -18,6 +18,11 @@
 // filter stages and half the plane traffic of the tf32 form.  An image that spans too many powers of two - or
 // every image, where a filter does - has tf32 planes in the same place, and this kernel runs the same loop over
 // those for its tiles (16 channels per row); the other images of the batch are not touched by it.
+//
+// Strides: the rows and columns of the input that are alike modulo the stride are sub-images of the planes, and a tap is a
+// shift inside one of them, so a strided layer is the same loop with a halo per sub-image; its patches are never written
+// (64 x 48 x 57 x 57 -> 96 at stride 2: 121 us through a patch matrix, 77 so).  Longer k than 1024: the leading
+// accumulator is drained every 1024 values, as in gemm_half.cu.
 //
 // One CTA per SM walks the tiles.  Both accumulators (512 columns) belong to one tile; the epilogue reads the
 // cross products first, which the next tile starts with, so the tensor pipe waits for about the drain of
@@ -61,14 +66,19 @@ using namespace ptx;
 
 constexpr int kH_RowB       = 64;                     // bytes of k per operand row and k-block: 32 float16 / 16 tf32
 constexpr int kH_AStages    = 4;
-constexpr int kH_HaloStages = 2;
+constexpr int kH_HaloStages = 4;                      // at most; as many as shared memory holds
 constexpr int kH_ABytes     = 128 * kH_RowB;          // one filter plane of a k-block
 constexpr int kH_AStageBytes = 2 * kH_ABytes;         // hi + lo
 constexpr int kH_EpiWarps   = 8;
 constexpr int kH_Threads    = 64 + 32 * kH_EpiWarps;
-constexpr int kH_EpiRowBytes  = 64 * 4 + 16;          // 64 columns staged at a time, rows padded
+constexpr int kH_EpiRowBytes  = 32 * 4 + 16;          // 32 columns staged at a time, rows padded
 constexpr int kH_EpiWarpBytes = 32 * kH_EpiRowBytes;
 constexpr int kH_EpiBytes     = kH_EpiWarps * kH_EpiWarpBytes;
+constexpr int kH_MinFilters = 17;
+constexpr int kH_MaxTaps    = 32;
+constexpr int kH_MaxStride  = 3;
+constexpr int kH_MaxHalos   = kH_MaxStride * kH_MaxStride;
+constexpr int kH_MaxK       = 1024; // values of k per drain of the leading accumulator
 constexpr int kH_BiasSlots    = 256;                  // output channels whose bias is kept in shared memory
 
 struct ConvHaloParams {
@@ -76,15 +86,24 @@ struct ConvHaloParams {
     float *out;       // [batch][ko][ho][wo]
     uint32_t *flags;
     int ko, tiles_m;
-    int kh, kw, pad;
-    int ho, wo, pw;   // pw = w + 2 pad
+    int ho, wo, pw;   // pw: positions of a tile row
     int th, tiles_y;
+    // The filter taps in the order of the halos that they read (one halo for stride 1; the rows and columns of the input
+    // that are alike modulo the stride are a sub-image each).
+    int halos;                          // per channel block
+    uint8_t halo_image[kH_MaxHalos];    // its sub-image
+    uint8_t halo_taps[kH_MaxHalos + 1]; // its first tap in the list; the last entry is the number of taps
+    uint8_t tap[kH_MaxTaps];            // r * kw + s
+    uint16_t tap_shift[kH_MaxTaps];     // position of the tap's first pixel in the box
+    int box_x0, box_y0;                 // of tile row 0 in the sub-images
+    int chunk_blocks;                   // blocks of 32 channels per drain of the leading accumulator
+    int c;                              // channels of the layer
     const float *filter_scale; // [ko] inverse scales
     const float *image_scale;  // [batch]; 0: this image's planes are tf32
     int c_pad;        // channels of the planes (k offset of a tap in the filter planes: tap * c_pad)
     int n_mma;        // th * pw rounded up to 16
     int box_bytes;    // one plane's halo box
-    int halo_plane_bytes;
+    int halo_plane_bytes, halo_stages;
     int act;
 };
 
@@ -94,7 +113,7 @@ struct ConvHaloMaps {
 };
 
 __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
-    const __grid_constant__ ConvHaloMaps maps, const __grid_constant__ ConvHaloParams p, const int total_tiles) {
+    const __grid_constant__ ConvHaloMaps maps, const __grid_constant__ ConvHaloParams p, const int all_tiles) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t bar_a_full[kH_AStages], bar_a_empty[kH_AStages];
     __shared__ uint64_t bar_h_full[kH_HaloStages], bar_h_empty[kH_HaloStages];
@@ -109,18 +128,11 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    if (threadIdx.x == 0)
-        abort_flag_s = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
-    for (int c = threadIdx.x; c < kH_BiasSlots; c += kH_Threads)
-        bias_s[c] = (p.bias && c < p.ko) ? p.bias[c] : 0.0f;
-    __syncthreads();
-    if (abort_flag_s)
-        return;
-
+    griddep_launch_dependents();
     const uint32_t smem_base  = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t halo_base  = smem_base + kH_AStages * kH_AStageBytes;
     const uint32_t halo_stage = 2u * (uint32_t)p.halo_plane_bytes;
-    uint8_t *epi_base = smem_raw + (smem_base - smem_u32(smem_raw)) + kH_AStages * kH_AStageBytes + kH_HaloStages * halo_stage;
+    uint8_t *epi_base = smem_raw + (smem_base - smem_u32(smem_raw)) + kH_AStages * kH_AStageBytes + (uint32_t)p.halo_stages * halo_stage;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kH_AStages; ++s) {
@@ -146,11 +158,18 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
         tmem_alloc(smem_u32(&tmem_base_slot), 512);
         tmem_relinquish();
     }
+    griddep_wait(); // the planes, the scales and what the caller's earlier kernels wrote
+    if (threadIdx.x == 0)
+        abort_flag_s = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
+    for (int c = threadIdx.x; c < kH_BiasSlots; c += kH_Threads)
+        bias_s[c] = (p.bias && c < p.ko) ? p.bias[c] : 0.0f;
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
-    const int taps           = p.kh * p.kw;
+    const bool failed        = abort_flag_s != 0; // an earlier launch failed: no work
+    const int total_tiles    = failed ? 0 : all_tiles;
+    __syncthreads(); // every thread has read abort_flag_s before a role may raise it
 
     // tile -> (row tile of output channels, tile row, image): neighbouring CTAs take the row tiles
     // of one pixel tile, so they read the same halo out of L2
@@ -169,34 +188,36 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
                 int tm, ty, img;
                 coords(tile, tm, ty, img);
-                const bool wide          = __ldg(p.image_scale + img) == 0.0f;
+                const bool wide          = p.image_scale[img] == 0.0f;
                 const CUtensorMap *mw_hi = wide ? &maps.w32_hi : &maps.w16_hi, *mw_lo = wide ? &maps.w32_lo : &maps.w16_lo;
                 const CUtensorMap *mx_hi = wide ? &maps.x32_hi : &maps.x16_hi, *mx_lo = wide ? &maps.x32_lo : &maps.x16_lo;
                 const int block_k = wide ? 16 : 32, cblocks = p.c_pad / block_k; // channels per k-block
-                for (int cb = 0; cb < cblocks && ok; ++cb, ++kh2) {
-                    const int hs = kh2 % kH_HaloStages;
-                    if (!mbar_wait(smem_u32(&bar_h_empty[hs]), ((uint32_t)(kh2 / kH_HaloStages) & 1u) ^ 1u, abort_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t hfull = smem_u32(&bar_h_full[hs]);
-                    const uint32_t hdst  = halo_base + (uint32_t)hs * halo_stage;
-                    mbar_expect_tx(hfull, 2u * (uint32_t)p.box_bytes);
-                    tma_load_4d(hdst, mx_hi, hfull, cb * block_k, -p.pad, ty * p.th - p.pad, img);
-                    tma_load_4d(hdst + (uint32_t)p.halo_plane_bytes, mx_lo, hfull, cb * block_k, -p.pad,
-                                ty * p.th - p.pad, img);
-                    for (int tap = 0; tap < taps; ++tap, ++ka) {
-                        const int s = ka % kH_AStages;
-                        if (!mbar_wait(smem_u32(&bar_a_empty[s]), ((uint32_t)(ka / kH_AStages) & 1u) ^ 1u, abort_flag)) {
+                for (int cb = 0; cb < cblocks && ok; ++cb) {
+                    for (int h = 0; h < p.halos && ok; ++h, ++kh2) {
+                        const int hs = kh2 % p.halo_stages;
+                        if (!mbar_wait(smem_u32(&bar_h_empty[hs]), ((uint32_t)(kh2 / p.halo_stages) & 1u) ^ 1u, abort_flag)) {
                             ok = false;
                             break;
                         }
-                        const uint32_t full = smem_u32(&bar_a_full[s]);
-                        const uint32_t dst  = smem_base + (uint32_t)s * kH_AStageBytes;
-                        mbar_expect_tx(full, (uint32_t)kH_AStageBytes);
-                        const int32_t kc = tap * p.c_pad + cb * block_k;
-                        tma_load_2d(dst, mw_hi, full, kc, tm * 128);
-                        tma_load_2d(dst + kH_ABytes, mw_lo, full, kc, tm * 128);
+                        const uint32_t hfull = smem_u32(&bar_h_full[hs]);
+                        const uint32_t hdst  = halo_base + (uint32_t)hs * halo_stage;
+                        const int y0 = ty * p.th + p.box_y0, sub = p.halo_image[h];
+                        mbar_expect_tx(hfull, 2u * (uint32_t)p.box_bytes);
+                        tma_load_5d(hdst, mx_hi, hfull, cb * block_k, p.box_x0, y0, sub, img);
+                        tma_load_5d(hdst + (uint32_t)p.halo_plane_bytes, mx_lo, hfull, cb * block_k, p.box_x0, y0, sub, img);
+                        for (int t = p.halo_taps[h]; t < p.halo_taps[h + 1]; ++t, ++ka) {
+                            const int s = ka % kH_AStages;
+                            if (!mbar_wait(smem_u32(&bar_a_empty[s]), ((uint32_t)(ka / kH_AStages) & 1u) ^ 1u, abort_flag)) {
+                                ok = false;
+                                break;
+                            }
+                            const uint32_t full = smem_u32(&bar_a_full[s]);
+                            const uint32_t dst  = smem_base + (uint32_t)s * kH_AStageBytes;
+                            mbar_expect_tx(full, (uint32_t)kH_AStageBytes);
+                            const int32_t kc = p.tap[t] * p.c_pad + cb * block_k;
+                            tma_load_2d(dst, mw_hi, full, kc, tm * 128);
+                            tma_load_2d(dst + kH_ABytes, mw_lo, full, kc, tm * 128);
+                        }
                     }
                 }
             }
@@ -208,9 +229,9 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                            globaltimer_ns() - t0 < kWaitBudgetNs) {
                     }
                 }
-                for (int k2 = kh2 - kH_HaloStages < 0 ? 0 : kh2 - kH_HaloStages; k2 < kh2; ++k2) {
+                for (int k2 = kh2 - p.halo_stages < 0 ? 0 : kh2 - p.halo_stages; k2 < kh2; ++k2) {
                     const uint64_t t0 = globaltimer_ns();
-                    while (!mbar_try_wait(smem_u32(&bar_h_full[k2 % kH_HaloStages]), (uint32_t)(k2 / kH_HaloStages) & 1u) &&
+                    while (!mbar_try_wait(smem_u32(&bar_h_full[k2 % p.halo_stages]), (uint32_t)(k2 / p.halo_stages) & 1u) &&
                            globaltimer_ns() - t0 < kWaitBudgetNs) {
                     }
                 }
@@ -219,36 +240,36 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
     } else if (warp == 1) {
         // ===== MMA issuer =====
         if (lane == 0) {
-            int ka = 0, kh2 = 0, i = 0, crosses = 0; // tiles so far, and those of them with cross products
+            int ka = 0, kh2 = 0, i = 0, crosses = 0, mains = 0; // accumulations begun so far
             bool ok = true;
             const long long t_start = CH_CLOCK();
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++i) {
                 int tm, ty, img;
                 coords(tile, tm, ty, img);
-                const bool wide      = __ldg(p.image_scale + img) == 0.0f; // looked up while the MMAs of the last tile run
+                const bool wide      = p.image_scale[img] == 0.0f; // looked up while the MMAs of the last tile run
                 const uint32_t idesc = make_idesc(wide ? 2u : 0u, 128, (uint32_t)p.n_mma);
-                const int cblocks    = p.c_pad / (wide ? 16 : 32);
-                // the accumulators of the previous tile have been read
+                const int cblocks = p.c_pad / (wide ? 16 : 32), chunk = p.chunk_blocks * (wide ? 2 : 1);
+                // what the accumulator held before has been read
                 auto wait_empty = [&](int acc) {
-                    const bool got = mbar_wait(smem_u32(&bar_tmem_empty[acc]), ((uint32_t)(acc ? crosses : i) & 1u) ^ 1u, abort_flag);
+                    const bool got = mbar_wait(smem_u32(&bar_tmem_empty[acc]), ((uint32_t)(acc ? crosses++ : mains++) & 1u) ^ 1u, abort_flag);
                     tc_fence_after_sync();
                     return got;
                 };
                 const uint32_t d_main = tmem_base, d_cross = tmem_base + 256u;
-                bool first = true;
-                for (int cb = 0; cb < cblocks && ok; ++cb, ++kh2) {
-                    const int hs = kh2 % kH_HaloStages;
-                    const long long t1 = CH_CLOCK();
-                    if (!mbar_wait(smem_u32(&bar_h_full[hs]), (uint32_t)(kh2 / kH_HaloStages) & 1u, abort_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    CH_ACCUM(1, CH_CLOCK() - t1); // waiting for a halo
-                    const uint32_t x_hi = halo_base + (uint32_t)hs * halo_stage;
-                    const uint32_t x_lo = x_hi + (uint32_t)p.halo_plane_bytes;
-                    int tap = 0;
-                    for (int r = 0; r < p.kh && ok; ++r) {
-                        for (int sx = 0; sx < p.kw; ++sx, ++tap, ++ka) {
+                bool first_cross = true, first_main = true;
+                for (int cb = 0; cb < cblocks && ok; ++cb) {
+                    const bool two = p.c - cb * 32 > 16; // k-steps of this block that hold channels
+                    for (int h = 0; h < p.halos && ok; ++h, ++kh2) {
+                        const int hs = kh2 % p.halo_stages;
+                        const long long t1 = CH_CLOCK();
+                        if (!mbar_wait(smem_u32(&bar_h_full[hs]), (uint32_t)(kh2 / p.halo_stages) & 1u, abort_flag)) {
+                            ok = false;
+                            break;
+                        }
+                        CH_ACCUM(1, CH_CLOCK() - t1); // waiting for a halo
+                        const uint32_t x_hi = halo_base + (uint32_t)hs * halo_stage;
+                        const uint32_t x_lo = x_hi + (uint32_t)p.halo_plane_bytes;
+                        for (int t = p.halo_taps[h]; t < p.halo_taps[h + 1]; ++t, ++ka) {
                             const int s = ka % kH_AStages;
                             const long long t2 = CH_CLOCK();
                             if (!mbar_wait(smem_u32(&bar_a_full[s]), (uint32_t)(ka / kH_AStages) & 1u, abort_flag)) {
@@ -258,49 +279,55 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                             CH_ACCUM(2, CH_CLOCK() - t2); // waiting for filter planes
                             tc_fence_after_sync();
                             const uint32_t a_hi = smem_base + (uint32_t)s * kH_AStageBytes, a_lo = a_hi + kH_ABytes;
-                            // the tap's pixels: the halo, (r * pw + sx) rows of 64 bytes further on
-                            const uint32_t shift = (uint32_t)(r * p.pw + sx) * (uint32_t)kH_RowB;
+                            // the tap's pixels: the halo, so many rows of 64 bytes further on
+                            const uint32_t shift = (uint32_t)p.tap_shift[t] * (uint32_t)kH_RowB;
                             const uint64_t da_hi = smem_desc_k<kH_RowB>(a_hi), da_lo = smem_desc_k<kH_RowB>(a_lo);
                             const uint64_t db_hi = smem_desc_k<kH_RowB>(x_hi + shift), db_lo = smem_desc_k<kH_RowB>(x_lo + shift);
                             if (!wide) {
-                                if (first && !wait_empty(1)) {
+                                if (first_cross && !wait_empty(1)) {
                                     ok = false;
                                     break;
                                 }
-                                mma_f16(d_cross, da_lo, db_hi, idesc, first ? 0u : 1u);
+                                mma_f16(d_cross, da_lo, db_hi, idesc, first_cross ? 0u : 1u);
                                 mma_f16(d_cross, da_hi, db_lo, idesc, 1u);
-                                mma_f16(d_cross, da_lo + 2, db_hi + 2, idesc, 1u);
-                                mma_f16(d_cross, da_hi + 2, db_lo + 2, idesc, 1u);
-                                if (first && !wait_empty(0)) {
+                                if (two) {
+                                    mma_f16(d_cross, da_lo + 2, db_hi + 2, idesc, 1u);
+                                    mma_f16(d_cross, da_hi + 2, db_lo + 2, idesc, 1u);
+                                }
+                                if (first_main && !wait_empty(0)) {
                                     ok = false;
                                     break;
                                 }
-                                mma_f16(d_main, da_hi, db_hi, idesc, first ? 0u : 1u);
-                                mma_f16(d_main, da_hi + 2, db_hi + 2, idesc, 1u);
+                                mma_f16(d_main, da_hi, db_hi, idesc, first_main ? 0u : 1u);
+                                if (two)
+                                    mma_f16(d_main, da_hi + 2, db_hi + 2, idesc, 1u);
+                                first_cross = false;
                             } else {
-                                if (first && !wait_empty(0)) {
+                                if (first_main && !wait_empty(0)) {
                                     ok = false;
                                     break;
                                 }
 #pragma unroll
                                 for (int kk = 0; kk < kH_RowB / 32; ++kk) {
-                                    mma_tf32(d_main, da_lo + 2 * kk, db_hi + 2 * kk, idesc, first && kk == 0 ? 0u : 1u);
+                                    mma_tf32(d_main, da_lo + 2 * kk, db_hi + 2 * kk, idesc, first_main && kk == 0 ? 0u : 1u);
                                     mma_tf32(d_main, da_hi + 2 * kk, db_lo + 2 * kk, idesc, 1u);
                                     mma_tf32(d_main, da_hi + 2 * kk, db_hi + 2 * kk, idesc, 1u);
                                 }
                             }
-                            first = false;
+                            first_main = false;
                             tc_commit(smem_u32(&bar_a_empty[s]));
                         }
+                        if (ok)
+                            tc_commit(smem_u32(&bar_h_empty[hs])); // the halo is free once its taps' MMAs have retired
                     }
-                    if (ok)
-                        tc_commit(smem_u32(&bar_h_empty[hs])); // the halo is free once its taps' MMAs have retired
+                    if (ok && cb + 1 < cblocks && (cb + 1) % chunk == 0) {
+                        tc_commit(smem_u32(&bar_tmem_full[0]));
+                        first_main = true;
+                    }
                 }
                 if (ok) {
-                    if (!wide) {
+                    if (!wide)
                         tc_commit(smem_u32(&bar_tmem_full[1]));
-                        ++crosses;
-                    }
                     tc_commit(smem_u32(&bar_tmem_full[0]));
                 }
             }
@@ -319,22 +346,18 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
         const int quarter = warp & 3;
         const int half    = ew >> 2;
         uint8_t *stg      = epi_base + (uint32_t)ew * kH_EpiWarpBytes;
-        const int sub = lane & 15, rr = lane >> 4;
-        // where this lane's columns land: column col = half * 128 + h2 * 64 + sub * 4 + q is position
+        // where this lane's columns land: column col = half * 128 + 32 j + lane is position
         // (y, x) = (col / pw, col % pw); -1 for the halo columns and past the tile
-        int off[2][4];
+        int off[4];
         const int npos = p.th * p.pw;
 #pragma unroll
-        for (int h2 = 0; h2 < 2; ++h2)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int col = half * 128 + h2 * 64 + sub * 4 + q;
-                const int y = col / p.pw, x = col - y * p.pw;
-                off[h2][q] = (col < npos && x < p.wo) ? y * p.wo + x : -1;
-            }
-        const int col_base = half * 128 + sub * 4;
-        int i = 0, crosses = 0;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
+        for (int j = 0; j < 4; ++j) {
+            const int col = half * 128 + 32 * j + lane;
+            const int y = col / p.pw, x = col - y * p.pw;
+            off[j] = (col < npos && x < p.wo) ? y * p.wo + x : -1;
+        }
+        int mains = 0, crosses = 0;
+        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
             int tm, ty, img;
             coords(tile, tm, ty, img);
             const int row0     = tm * 128 + quarter * 32; // first output channel of this warp's block
@@ -346,7 +369,7 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
             float acc[128];
             const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 128);
             auto await = [&](int which) {
-                const bool got = mbar_wait(smem_u32(&bar_tmem_full[which]), (uint32_t)(which ? crosses++ : i) & 1u, abort_flag);
+                const bool got = mbar_wait(smem_u32(&bar_tmem_full[which]), (uint32_t)(which ? crosses++ : mains++) & 1u, abort_flag);
                 tc_fence_after_sync();
                 return __all_sync(0xffffffffu, got) != 0;
             };
@@ -356,8 +379,12 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                 if (lane == 0)
                     mbar_arrive(smem_u32(&bar_tmem_empty[which]));
             };
-            // the cross products (tf32: the one accumulator) straight into the sums, with one wait for all columns
-            const int first_acc = wide ? 0 : 1;
+            // The leading accumulator of every chunk but the last, the cross products, the last chunk (tf32: the chunks).
+            // The first of them straight into the sums, with one wait for all columns.
+            const int cblocks = p.c_pad / 32, chunks = (cblocks + p.chunk_blocks - 1) / p.chunk_blocks;
+            const int events  = wide ? chunks : chunks + 1;
+            auto which_of     = [&](int e) { return !wide && e == chunks - 1 ? 1 : 0; };
+            const int first_acc = which_of(0);
             if (!await(first_acc))
                 break;
             {
@@ -367,65 +394,79 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                     tmem_ld_32x32(lane_base + (uint32_t)(first_acc * 256 + g * 32), r[g]);
                 tmem_ld_wait();
                 hand_back(first_acc);
-                const float weight = wide ? 1.0f : kHalfLoInv;
+                const float weight = first_acc ? kHalfLoInv : 1.0f;
 #pragma unroll
                 for (int j = 0; j < 128; ++j)
                     acc[j] = __fmul_rn(__uint_as_float(r[j / 32][j % 32]), weight);
             }
-            if (!wide) {
-                if (!await(0))
+            bool ok = true;
+#pragma unroll 1
+            for (int e = 1; e < events; ++e) {
+                const int which    = which_of(e);
+                const float weight = which ? kHalfLoInv : 1.0f;
+                ok                 = await(which);
+                if (!ok)
                     break;
 #pragma unroll
                 for (int g = 0; g < 8; ++g) {
                     uint32_t r[16];
-                    tmem_ld_32x16(lane_base + g * 16, r);
+                    tmem_ld_32x16(lane_base + (uint32_t)(which * 256 + g * 16), r);
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        acc[g * 16 + j] = __fadd_rn(acc[g * 16 + j], __uint_as_float(r[j]));
+                        acc[g * 16 + j] = __fadd_rn(acc[g * 16 + j], __fmul_rn(__uint_as_float(r[j]), weight));
                 }
-                hand_back(0);
+                hand_back(which);
             }
+            if (!ok)
+                break;
             const long long e1 = CH_CLOCK();
 
             const int y0   = ty * p.th;
             // positions of rows past the image's last row (a partial last tile) are dropped:
             // position col lies in row col / pw, so the valid ones are col < rows_left * pw
             const int col_limit = (p.ho - y0 < p.th ? p.ho - y0 : p.th) * p.pw;
+            const int64_t plane = (int64_t)p.ho * p.wo;
             float *out_img = p.out + ((int64_t)img * p.ko) * p.ho * p.wo + (int64_t)y0 * p.wo;
 #pragma unroll
-            for (int h2 = 0; h2 < 2; ++h2) {
-                if (half * 128 + h2 * 64 >= npos)
+            for (int g = 0; g < 4; ++g) {
+                if (half * 128 + g * 32 >= npos)
                     break;
                 float4 *mine = reinterpret_cast<float4 *>(stg + lane * kH_EpiRowBytes);
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    mine[j] = make_float4(__fmul_rn(acc[h2 * 64 + 4 * j], rs), __fmul_rn(acc[h2 * 64 + 4 * j + 1], rs),
-                                          __fmul_rn(acc[h2 * 64 + 4 * j + 2], rs), __fmul_rn(acc[h2 * 64 + 4 * j + 3], rs));
+                for (int j = 0; j < 8; ++j)
+                    mine[j] = make_float4(__fmul_rn(acc[g * 32 + 4 * j], rs), __fmul_rn(acc[g * 32 + 4 * j + 1], rs),
+                                          __fmul_rn(acc[g * 32 + 4 * j + 2], rs), __fmul_rn(acc[g * 32 + 4 * j + 3], rs));
                 __syncwarp();
-#pragma unroll 4
-                for (int it = 0; it < 16; ++it) {
-                    const int r_in = it * 2 + rr; // channel within the warp's 32
-                    const int ch   = row0 + r_in;
-                    if (ch < p.ko) {
-                        const float4 q4 = *reinterpret_cast<const float4 *>(stg + r_in * kH_EpiRowBytes + sub * 16);
-                        const float v[4] = {q4.x, q4.y, q4.z, q4.w};
-                        const float b    = ch < kH_BiasSlots ? bias_s[ch] : (p.bias ? p.bias[ch] : 0.0f);
-                        float *plane     = out_img + (int64_t)ch * p.ho * p.wo;
+                // a column per lane, so that a store covers consecutive pixels of a channel (four columns per lane wrote every
+                // sector four times: 256 x 64 x 56 x 56 -> 128 530 us, 491 so); the reads of eight channels before their stores
+                const bool stored = off[g] >= 0 && half * 128 + g * 32 + lane < col_limit;
+                const float *src  = reinterpret_cast<const float *>(stg) + lane;
+                float *dst        = out_img + (int64_t)row0 * plane + (stored ? off[g] : 0);
+#pragma unroll 2
+                for (int r0 = 0; r0 < 32; r0 += 8) {
+                    if (row0 + r0 >= p.ko)
+                        break;
+                    float x[8], b[8];
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            if (off[h2][q] >= 0 && col_base + h2 * 64 + q < col_limit) {
-                                float x = __fmul_rn(v[q], is);
-                                if (p.bias)
-                                    x = __fadd_rn(x, b);
-                                if (p.act == CT_ACT_RELU)
-                                    x = __fmul_rn(x, x > 0.0f ? 1.0f : 0.0f);
-                                plane[off[h2][q]] = x;
-                            }
-                        }
+                    for (int u = 0; u < 8; ++u) {
+                        const int ch = row0 + r0 + u;
+                        x[u]         = src[(r0 + u) * (kH_EpiRowBytes / 4)];
+                        b[u]         = !p.bias || ch >= p.ko ? 0.0f : (ch < kH_BiasSlots ? bias_s[ch] : p.bias[ch]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        float y = __fmul_rn(x[u], is);
+                        if (p.bias)
+                            y = __fadd_rn(y, b[u]);
+                        if (p.act == CT_ACT_RELU)
+                            y = __fmul_rn(y, y > 0.0f ? 1.0f : 0.0f);
+                        if (stored && row0 + r0 + u < p.ko)
+                            *dst = y;
+                        dst += plane;
                     }
                 }
-                __syncwarp(); // the block is rewritten by the next half / tile
+                __syncwarp(); // the block is rewritten by the next columns
             }
             if (warp == 2 && lane == 0) {
                 CH_ACCUM(5, e1 - e0);          // epilogue: waiting for a complete accumulator
@@ -441,7 +482,7 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 512);
     }
-    if (threadIdx.x == 0 && *abort_flag)
+    if (threadIdx.x == 0 && !failed && *abort_flag)
         atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
 }
 
@@ -462,6 +503,8 @@ __global__ void __launch_bounds__(256) conv_range_kernel(
     const float *__restrict__ w, int c, int taps, int c_pad, int ko, const FilterPlanes f, const float *__restrict__ x,
     int64_t count, int slices, int vec_ok, uint2 *__restrict__ ranges) {
     __shared__ uint2 part[8];
+    griddep_launch_dependents();
+    griddep_wait();
     const bool filter = (int64_t)blockIdx.x < ko;
     const int64_t o   = filter ? blockIdx.x : (blockIdx.x - ko) / slices;
     const int slice   = filter ? 0 : (int)(blockIdx.x - ko - o * slices);
@@ -512,23 +555,44 @@ __global__ void __launch_bounds__(256) conv_range_kernel(
 // under the image's scale, or tf32 terms (image_scale 0) where the image or any filter does not fit those.  A
 // block takes 64 channels by 64 positions through shared memory: reads of 256 contiguous bytes, writes of 128.  The
 // images are taken last to first: the end of the tensor is what conv_range_kernel has just left in L2.
+// Sub-images (ConvSubImages, hs x ws each): zeros where the image has no such row or column, those that no tap reads are
+// left out.
+struct PlaneGeom {
+    int h, w, hs, ws;
+    ConvSubImages sub;
+};
 __global__ void __launch_bounds__(256) conv_planes_kernel(
-    const float *__restrict__ x, int c, int64_t hw, int c_pad, const uint2 *__restrict__ ranges, int slices,
+    const float *__restrict__ x, int c, const PlaneGeom geom, int c_pad, const uint2 *__restrict__ ranges, int slices,
     const float *__restrict__ filter_scale, int ko, uint8_t *__restrict__ slots, float *__restrict__ image_scale) {
     __shared__ float tile[64][65];
+    griddep_launch_dependents();
+    griddep_wait();
     const int64_t img = gridDim.z - 1 - blockIdx.z;
     const int64_t q0  = (int64_t)blockIdx.x * 64;
     const int c0      = (int)blockIdx.y * 64;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float *src = x + (img * c + c0) * hw + q0;
+    const int64_t in_hw = (int64_t)geom.h * geom.w;
+    const int row_mod = geom.sub.row_mod, col_mod = geom.sub.col_mod, width = geom.ws * col_mod;
+    const int64_t hw  = (int64_t)geom.hs * row_mod * width; // positions of the image grown to whole multiples
+    const bool apart  = row_mod * col_mod > 1;
+    const float *src  = x + (img * c + c0) * in_hw;
+    // position q of the grown image in the input (-1: not there)
+    auto source = [&](int64_t q) -> int64_t {
+        if (!apart)
+            return q < hw ? q : -1;
+        const int row = (int)q / width, col = (int)q - row * width;
+        return q < hw && row < geom.h && col < geom.w ? (int64_t)row * geom.w + col : -1;
+    };
     float v[16]; // every load before the first use of any
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int t = 0; t < 2; ++t) {
+        const int64_t from = source(q0 + lane + 32 * t);
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            const int ch = warp + 8 * j, q = lane + 32 * t;
-            v[2 * j + t] = (c0 + ch < c && q0 + q < hw) ? __ldcs(src + ch * hw + q) : 0.0f;
+        for (int j = 0; j < 8; ++j) {
+            const int ch = warp + 8 * j;
+            v[2 * j + t] = (c0 + ch < c && from >= 0) ? __ldcs(src + ch * in_hw + from) : 0.0f;
         }
+    }
     uint2 r = make_uint2(0u, kNoneSmallest);
     for (int s = lane; s < slices; s += 32)
         r = range_join(r, ranges[img * slices + s]);
@@ -549,7 +613,19 @@ __global__ void __launch_bounds__(256) conv_planes_kernel(
         const int chunk = threadIdx.x & 7, q = (threadIdx.x >> 3) + 32 * t;
         if (q0 + q >= hw || c0 + chunk * 8 >= c_pad)
             continue;
-        const int64_t at = (q0 + q) * c_pad + c0 + chunk * 8;
+        int64_t to = q0 + q;
+        if (apart) {
+            const int row = (int)to / width, col = (int)to - row * width, sub = row % row_mod * col_mod + col % col_mod;
+            if (!(geom.sub.used >> sub & 1u))
+                continue;
+            if (fits || !geom.sub.tf32_plain)
+                to = ((int64_t)sub * geom.hs + row / row_mod) * geom.ws + col / col_mod;
+            else if (row < geom.h && col < geom.w)
+                to = (int64_t)row * geom.w + col;
+            else
+                continue;
+        }
+        const int64_t at = to * c_pad + c0 + chunk * 8;
         if (fits) {
             __half2 hi[4], lo[4];
 #pragma unroll
@@ -574,29 +650,44 @@ __global__ void __launch_bounds__(256) conv_planes_kernel(
 }
 
 struct HaloGeom {
-    int pw, wo, ho, th, n_mma, box_rows, plane_bytes;
+    int pw, wo, ho, th, n_mma, box_rows, plane_bytes, stages;
+    int hs, ws;         // extents of a sub-image
+    int y_min, x_min;   // smallest row and column offset of a tap in its sub-image
     size_t smem;
 };
 
-bool halo_geometry(int64_t h, int64_t w, int64_t kh, int64_t kw, int64_t pad, HaloGeom *g) {
-    const int64_t pw = w + 2 * pad, wo = pw - kw + 1, ho = h + 2 * pad - kh + 1;
-    if (wo < 1 || ho < 1 || pw > 256)
+int floor_div(int64_t a, int64_t b) { return (int)(a >= 0 ? a / b : -((-a + b - 1) / b)); }
+
+// Tap (r, q) of output (oy, ox) reads input row oy * stride - pad + r = stride * (oy + a) + py: row oy + a of the
+// sub-image py, and so for columns.  A tile is th rows of pw = wo + (largest - smallest b) positions.
+bool halo_geometry(int64_t h, int64_t w, int64_t kh, int64_t kw, int64_t stride, int64_t pad, HaloGeom *g) {
+    if (w + 2 * pad < kw || h + 2 * pad < kh || pad > 256 || kh > 256 || kw > 256)
         return false;
-    int64_t th = 256 / pw;
-    if (th > ho)
-        th = ho;
-    if (th < 1 || th + kh - 1 > 256)
+    const int64_t wo = (w + 2 * pad - kw) / stride + 1, ho = (h + 2 * pad - kh) / stride + 1;
+    g->y_min = floor_div(-pad, stride), g->x_min = floor_div(-pad, stride);
+    const int64_t span_y = floor_div(kh - 1 - pad, stride) - g->y_min, span_x = floor_div(kw - 1 - pad, stride) - g->x_min;
+    const int64_t pw = wo + span_x;
+    g->hs = (int)((h + stride - 1) / stride), g->ws = (int)((w + stride - 1) / stride);
+    if (pw > 256)
         return false;
-    g->pw = (int)pw, g->wo = (int)wo, g->ho = (int)ho, g->th = (int)th;
-    g->n_mma    = (int)((th * pw + 15) / 16 * 16);
-    g->box_rows = (int)(th + kh - 1);
-    // a tap's shifted window of n_mma rows may run past the box: reserve those rows too
-    int64_t rows = (kh - 1) * pw + (kw - 1) + g->n_mma;
-    if (rows < (int64_t)g->box_rows * pw)
-        rows = (int64_t)g->box_rows * pw;
-    g->plane_bytes = (int)((rows * kH_RowB + 1023) & ~1023ll);
-    g->smem = (size_t)kH_AStages * kH_AStageBytes + (size_t)kH_HaloStages * 2 * g->plane_bytes + kH_EpiBytes + 1024;
-    return g->smem <= 225 * 1024; // 227 KB per CTA less the kernel's static shared memory
+    // as many rows as 256 columns of the accumulator and the shared memory take
+    for (int64_t th = std::min<int64_t>(256 / pw, ho); th >= 1; --th) {
+        if (th + span_y > 256)
+            continue;
+        g->pw = (int)pw, g->wo = (int)wo, g->ho = (int)ho, g->th = (int)th;
+        g->n_mma    = (int)((th * pw + 15) / 16 * 16);
+        g->box_rows = (int)(th + span_y);
+        // a tap's shifted window of n_mma rows may run past the box: reserve those rows too
+        const int64_t rows = std::max<int64_t>(span_y * pw + span_x + g->n_mma, (int64_t)g->box_rows * pw);
+        g->plane_bytes     = (int)((rows * kH_RowB + 1023) & ~1023ll);
+        // 227 KB per CTA less the kernel's static shared memory
+        const int rest = 225 * 1024 - kH_AStages * kH_AStageBytes - kH_EpiBytes - 1024;
+        g->stages      = std::min(kH_HaloStages, rest / (2 * g->plane_bytes));
+        g->smem = (size_t)kH_AStages * kH_AStageBytes + (size_t)g->stages * 2 * g->plane_bytes + kH_EpiBytes + 1024;
+        if (g->stages >= 2)
+            return true;
+    }
+    return false;
 }
 
 } // namespace
@@ -611,10 +702,11 @@ int conv_range_slices(int64_t batch, int64_t count) {
 // The pre-pass of a layer: the filters' scales and (filters16 non-null) planes, the images' planes and scales.
 // ranges: batch * conv_range_slices(batch, c * hw) pairs of words.
 ct_status conv_prepass(
-    DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t hw, int64_t c_pad, int64_t ko, int64_t taps,
-    void *filters16, void *filters32, size_t plane16, size_t plane32, float *filter_scale, void *ranges, float *image_scale,
-    void *slots) {
+    DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t h, int64_t wd, int64_t c_pad, int64_t ko,
+    int64_t taps, void *filters16, void *filters32, size_t plane16, size_t plane32, float *filter_scale, void *ranges, float *image_scale,
+    void *slots, const ConvSubImages &sub) {
     (void)st;
+    const int64_t hw = h * wd;
     if (batch > 65535 || c_pad / 32 > 65535)
         return fail(CT_ERR_TOO_LARGE, "conv2d: batch or channel count too large for the layout pre-pass");
     const int64_t count = c * hw;
@@ -624,61 +716,82 @@ ct_status conv_prepass(
     const FilterPlanes f{reinterpret_cast<__half *>(f16), reinterpret_cast<__half *>(f16 + plane16), reinterpret_cast<float *>(f32),
                          reinterpret_cast<float *>(f32 + plane32), filter_scale};
     ProfScope prof("conv_prepass");
-    conv_range_kernel<<<(unsigned)(ko + batch * slices), 256, 0, stream()>>>(
-        w, (int)c, (int)taps, (int)c_pad, (int)ko, f, x, count, slices, vec, static_cast<uint2 *>(ranges));
+    CT_CUDA(launch_dependent(conv_range_kernel, dim3((unsigned)(ko + batch * slices)), dim3(256), 0, stream(), w, (int)c, (int)taps,
+                             (int)c_pad, (int)ko, f, x, count, slices, vec, static_cast<uint2 *>(ranges)));
     CT_LAUNCH_CHECK("conv_range");
-    const dim3 grid((unsigned)((hw + 63) / 64), (unsigned)((c_pad + 63) / 64), (unsigned)batch);
-    conv_planes_kernel<<<grid, 256, 0, stream()>>>(x, (int)c, hw, (int)c_pad, static_cast<uint2 *>(ranges), slices, filter_scale, (int)ko,
-                                                   static_cast<uint8_t *>(slots), image_scale);
+    const PlaneGeom geom{(int)h, (int)wd, (int)((h + sub.row_mod - 1) / sub.row_mod), (int)((wd + sub.col_mod - 1) / sub.col_mod), sub};
+    const int64_t positions = (int64_t)geom.hs * geom.ws * sub.row_mod * sub.col_mod;
+    const dim3 grid((unsigned)((positions + 63) / 64), (unsigned)((c_pad + 63) / 64), (unsigned)batch);
+    CT_CUDA(launch_dependent(conv_planes_kernel, grid, dim3(256), 0, stream(), x, (int)c, geom, (int)c_pad, static_cast<const uint2 *>(ranges),
+                             slices, static_cast<const float *>(filter_scale), (int)ko, static_cast<uint8_t *>(slots), image_scale));
     CT_LAUNCH_CHECK("conv_planes");
     return CT_OK;
 }
 
-// Whether the halo kernel takes this layer (float32 mode only): stride 1, more than 64 filters (fewer go
-// to the kernels that put pixels on the rows or filters in tensor memory), a k range short enough
-// for one accumulation, and a tile that is reasonably full.
+// Whether the halo kernel takes this layer (float32 mode only): filters and strides within its tables, whole k-blocks
+// of a tap list within one drain, and a tile that is reasonably full.
 bool conv_halo_applicable(int64_t c_pad, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw, int64_t stride,
                           int64_t pad) {
     HaloGeom g;
-    if (stride != 1 || ko <= 64 || kh * kw * c_pad > 1024 || (c_pad % 32) != 0)
+    if (stride < 1 || stride > kH_MaxStride || ko < kH_MinFilters || kh * kw > kH_MaxTaps || (c_pad % 32) != 0 ||
+        c_pad > (1 << 20) || h > 0x3fff || w > 0x3fff)
         return false;
-    if (!halo_geometry(h, w, kh, kw, pad, &g))
+    if (!halo_geometry(h, w, kh, kw, stride, pad, &g))
         return false;
-    return (int64_t)g.th * g.wo * 10 >= (int64_t)g.n_mma * 7; // at least 70 % of the columns carry an output
+    // at least 70 % of the columns carry an output, and not a few rows only because shared memory holds no more
+    return (int64_t)g.th * g.wo * 10 >= (int64_t)g.n_mma * 7 && (g.n_mma >= 128 || g.th == g.ho);
 }
 
 // Workspace: [filter scale][image scale][image ranges][w hi16][w lo16][w hi][w lo][image slots]; a slot holds an
 // image's planes, float16 pairs or, where it does not fit those, tf32: no more than tf32 planes alone take.
 ct_status conv_halo(
     DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t c_pad, int64_t h, int64_t wd, int64_t ko,
-    int64_t kh, int64_t kw, int64_t pad, const float *bias, int act, float *out) {
+    int64_t kh, int64_t kw, int64_t stride, int64_t pad, const float *bias, int act, float *out) {
     HaloGeom g;
-    if (!halo_geometry(h, wd, kh, kw, pad, &g))
+    if (!halo_geometry(h, wd, kh, kw, stride, pad, &g))
         return fail(CT_ERR_INVALID, "conv2d: internal tile shape not usable");
     auto align_up          = [](size_t v) { return (v + 1023) & ~(size_t)1023; };
-    const int64_t taps     = kh * kw, hw = h * wd;
+    const int64_t taps     = kh * kw, subs = stride * stride, sub = (int64_t)g.hs * g.ws, hw = sub * subs;
     const size_t w16       = align_up((size_t)ko * taps * c_pad * 2), w32 = align_up((size_t)ko * taps * c_pad * 4);
     const size_t slot      = (size_t)hw * c_pad * 8;
     const size_t w_words   = align_up((size_t)ko * 4), x_words = align_up((size_t)batch * 4);
-    const size_t ranges    = align_up((size_t)batch * conv_range_slices(batch, c * hw) * 8);
+    const size_t ranges    = align_up((size_t)batch * conv_range_slices(batch, c * h * wd) * 8);
     CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, w_words + x_words + ranges + 2 * w16 + 2 * w32 + (size_t)batch * slot));
     uint8_t *ws            = static_cast<uint8_t *>(st->gemm_ws);
     float *filter_scale    = reinterpret_cast<float *>(ws), *image_scale = reinterpret_cast<float *>(ws + w_words);
     uint8_t *w16_hi        = ws + w_words + x_words + ranges, *w32_hi = w16_hi + 2 * w16, *xp = w32_hi + 2 * w32;
-    CT_TRY(conv_prepass(st, x, w, batch, c, hw, c_pad, ko, taps, w16_hi, w32_hi, w16, w32, filter_scale, ws + w_words + x_words,
-                        image_scale, xp));
     ConvHaloParams p;
     p.filter_scale = filter_scale, p.image_scale = image_scale;
     p.bias = bias, p.out = out, p.flags = st->flags_dev;
     p.ko = (int)ko, p.tiles_m = (int)((ko + 127) / 128);
-    p.kh = (int)kh, p.kw = (int)kw, p.pad = (int)pad;
     p.ho = g.ho, p.wo = g.wo, p.pw = g.pw, p.th = g.th;
     p.tiles_y = (g.ho + g.th - 1) / g.th;
+    p.box_x0 = g.x_min, p.box_y0 = g.y_min;
+    p.chunk_blocks = (int)std::max<int64_t>(1, kH_MaxK / (32 * taps));
+    p.c       = (int)c;
     p.c_pad   = (int)c_pad;
     p.n_mma   = g.n_mma;
     p.box_bytes        = g.box_rows * g.pw * kH_RowB;
-    p.halo_plane_bytes = g.plane_bytes;
+    p.halo_plane_bytes = g.plane_bytes, p.halo_stages = g.stages;
     p.act = act;
+    p.halos = 0, p.halo_taps[0] = 0;
+    uint32_t used = 0;
+    for (int image = 0, listed = 0; image < (int)subs; ++image) {
+        for (int t = 0; t < (int)taps; ++t) {
+            const int r = t / (int)kw - (int)pad, q = t % (int)kw - (int)pad, a = floor_div(r, stride), b = floor_div(q, stride);
+            if ((r - a * (int)stride) * (int)stride + (q - b * (int)stride) != image)
+                continue;
+            p.tap[listed]         = (uint8_t)t;
+            p.tap_shift[listed++] = (uint16_t)((a - g.y_min) * g.pw + (b - g.x_min));
+        }
+        if (listed > p.halo_taps[p.halos]) {
+            p.halo_image[p.halos]  = (uint8_t)image;
+            p.halo_taps[++p.halos] = (uint8_t)listed;
+            used |= 1u << image;
+        }
+    }
+    CT_TRY(conv_prepass(st, x, w, batch, c, h, wd, c_pad, ko, taps, w16_hi, w32_hi, w16, w32, filter_scale, ws + w_words + x_words,
+                        image_scale, xp, ConvSubImages{(int)stride, (int)stride, used, false}));
     const int64_t tiles = (int64_t)p.tiles_m * p.tiles_y * batch;
     if (tiles > 0x7fffffffll)
         return fail(CT_ERR_TOO_LARGE, "conv2d: too many tiles");
@@ -687,12 +800,12 @@ ct_status conv_halo(
         const uint64_t kp = (uint64_t)(taps * c_pad), row = (uint64_t)(c_pad * elem);
         const uint64_t wdims[2] = {kp, (uint64_t)ko}, wstr[1] = {kp * (uint64_t)elem};
         const uint32_t wbox[2]  = {(uint32_t)(kH_RowB / elem), 128};
-        const uint64_t xdims[4] = {(uint64_t)c_pad, (uint64_t)wd, (uint64_t)h, (uint64_t)batch};
-        const uint64_t xstr[3]  = {row, row * (uint64_t)wd, slot};
-        const uint32_t xbox[4]  = {(uint32_t)(kH_RowB / elem), (uint32_t)g.pw, (uint32_t)g.box_rows, 1};
+        const uint64_t xdims[5] = {(uint64_t)c_pad, (uint64_t)g.ws, (uint64_t)g.hs, (uint64_t)subs, (uint64_t)batch};
+        const uint64_t xstr[4]  = {row, row * (uint64_t)g.ws, row * (uint64_t)sub, slot};
+        const uint32_t xbox[5]  = {(uint32_t)(kH_RowB / elem), (uint32_t)g.pw, (uint32_t)g.box_rows, 1, 1};
         auto fn = elem == 4 ? encode_tiled_map_f32 : encode_tiled_map_f16;
         CT_TRY(fn(mw, wp, 2, wdims, wstr, wbox, kH_RowB));
-        return fn(mx, xpl, 4, xdims, xstr, xbox, kH_RowB);
+        return fn(mx, xpl, 5, xdims, xstr, xbox, kH_RowB);
     };
     CT_TRY(encode(&maps.w16_hi, w16_hi, &maps.x16_hi, xp, 2));
     CT_TRY(encode(&maps.w16_lo, w16_hi + w16, &maps.x16_lo, xp + slot / 4, 2));
@@ -708,7 +821,7 @@ ct_status conv_halo(
     }
     const unsigned grid = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
     ProfScope prof("gemm_tc");
-    conv_halo_stream_kernel<<<grid, kH_Threads, g.smem, stream()>>>(maps, p, (int)tiles);
+    CT_CUDA(launch_dependent(conv_halo_stream_kernel, dim3(grid), dim3(kH_Threads), g.smem, stream(), maps, p, (int)tiles));
     CT_LAUNCH_CHECK("conv_halo_stream");
     return CT_OK;
 }

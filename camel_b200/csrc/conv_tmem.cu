@@ -1271,8 +1271,8 @@ ct_status conv_tmem_filters(
     CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, f_words + words + ranges + (size_t)batch * slot));
     uint8_t *ws = static_cast<uint8_t *>(st->gemm_ws), *planes = ws + f_words + words + ranges;
     float *image_scale = reinterpret_cast<float *>(ws + f_words);
-    CT_TRY(conv_prepass(st, x, w, batch, c, h * wd, 32, ko, kh * kw, nullptr, nullptr, 0, 0, reinterpret_cast<float *>(ws),
-                        ws + f_words + words, image_scale, planes));
+    CT_TRY(conv_prepass(st, x, w, batch, c, h, wd, 32, ko, kh * kw, nullptr, nullptr, 0, 0, reinterpret_cast<float *>(ws),
+                        ws + f_words + words, image_scale, planes, ConvSubImages{}));
     p[0].image_scale = p[1].image_scale = image_scale;
     // planes [batch][h][w][32 channels]; box = 32 channels x pw positions x (th + kh - 1) rows of one image,
     // swizzled over a row; positions outside the image read as zero: the padding

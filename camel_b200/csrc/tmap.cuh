@@ -29,14 +29,21 @@ ct_status conv_tmem_filters(
 // conv2d with one input halo per tile and channel block serving every tap (conv_halo.cu).
 bool conv_halo_applicable(int64_t c_pad, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw, int64_t stride,
                           int64_t pad);
+// The float16 planes of an image: sub-images of the rows (columns) that are alike modulo row_mod (col_mod), a bit of `used`
+// for each that is needed.  tf32_plain: tf32 planes are not taken apart.
+struct ConvSubImages {
+    int row_mod = 1, col_mod = 1;
+    uint32_t used = 1;
+    bool tf32_plain = false;
+};
 int conv_range_slices(int64_t batch, int64_t count);
 ct_status conv_prepass(
-    DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t hw, int64_t c_pad, int64_t ko, int64_t taps,
-    void *filters16, void *filters32, size_t plane16, size_t plane32, float *filter_scale, void *ranges, float *image_scale,
-    void *slots);
+    DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t h, int64_t wd, int64_t c_pad, int64_t ko,
+    int64_t taps, void *filters16, void *filters32, size_t plane16, size_t plane32, float *filter_scale, void *ranges, float *image_scale,
+    void *slots, const ConvSubImages &sub);
 // x NCHW and w OIHW float32; c_pad: channels rounded up to 32.
 ct_status conv_halo(
     DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t c_pad, int64_t h, int64_t wd, int64_t ko,
-    int64_t kh, int64_t kw, int64_t pad, const float *bias, int act, float *out);
+    int64_t kh, int64_t kw, int64_t stride, int64_t pad, const float *bias, int act, float *out);
 
 } // namespace ct
