@@ -728,7 +728,7 @@ static ct_status conv2d_run(
     // patch matrix is never materialised - each k-block is one shifted 4-D TMA box.
     const int th = (stride == 1 && c >= 16 && wo <= 256 && wd <= 0x7fffffff && h <= 0x7fffffff)
                        ? conv_tile_rows(ho, wo) : 0;
-    if (th > 0 && mode == 0 && conv_tmem_applicable(c, h, wd, ko, kh, kw, stride, pad)) {
+    if ((th > 0 || c >= 8) && mode == 0 && conv_tmem_applicable(c, h, wd, ko, kh, kw, stride, pad)) {
         // few channels on both sides: the filters stay in tensor memory, a tile's input is fetched once
         return conv_tmem_filters(st, x, w, bias, n, c, h, wd, ko, kh, kw, pad, act, pool, out);
     }

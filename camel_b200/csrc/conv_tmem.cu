@@ -94,8 +94,9 @@ struct ConvTmemParams {
     int stages;
     int act, pool;
     const float *image_scale; // planes: [batch] inverse scales, 0 for an image that needs tf32 terms
-    uint2 *tile_range;        // raw: [total tiles] range of the values of each tile, and one entry whose .x says that
-                              // the filters need tf32 terms
+    uint2 *tile_range;        // raw: [range_tiles to an image] range of the values of each of conv_pairs_kernel's tiles, and
+                              // behind them one entry whose .x says that the filters need tf32 terms
+    int range_tiles, range_total;
     // raw mode (the input is read as it is, NCHW float32, and split into planes inside the kernel)
     int box_w;        // floats per row of the raw box (a multiple of four)
     int off_x;        // the tile's first position (x = -pad) sits this many floats into a raw row
@@ -107,17 +108,17 @@ struct ConvTmemParams {
 // Whether image `img` is left to the tf32 form: its values, over all its tiles (every pixel is in one of them), or the
 // filters do not fit float16 pairs.  A property of the image alone, so that its bits do not depend on how the launch
 // was cut into tiles (the fused pool takes rows by twos), on what else is in the batch, or on how it was read.
-template <bool RAW> __device__ __forceinline__ bool image_needs_tf32(const ConvTmemParams &p, int img, int total_tiles) {
+template <bool RAW> __device__ __forceinline__ bool image_needs_tf32(const ConvTmemParams &p, int img) {
     if (!RAW)
         return __ldg(p.image_scale + img) == 0.0f;
-    const uint32_t filters = p.tile_range[total_tiles].x;
-    const uint2 *src       = p.tile_range + (int64_t)img * p.tiles_y;
+    const uint32_t filters = p.tile_range[p.range_total].x;
+    const uint2 *src       = p.tile_range + (int64_t)img * p.range_tiles;
     uint2 range            = make_uint2(0u, kNoneSmallest);
-    for (int t = 0; t < p.tiles_y; t += 8) {
+    for (int t = 0; t < p.range_tiles; t += 8) {
         uint2 r[8]; // eight loads in flight: one after the other they cost an idle launch 4 us
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            r[j] = src[min(t + j, p.tiles_y - 1)];
+            r[j] = src[min(t + j, p.range_tiles - 1)];
 #pragma unroll
         for (int j = 0; j < 8; ++j)
             range = range_join(range, r[j]);
@@ -142,15 +143,14 @@ __device__ __forceinline__ int next_own(const uint32_t *mask, int q, int own) {
 // banks; a warp per filter, which it hands to `seen` as it goes (every lane has its share).  Read from global
 // memory by the lanes that write them to tensor memory - 128 threads, a sector for every value - the set-up took
 // 35 of the 41 us of a layer on four images.
-__device__ __forceinline__ int filter_stride(const ConvTmemParams &p) { return (p.c * p.kh * p.kw) | 1; }
 template <typename Seen>
-__device__ __forceinline__ void stage_filters(const ConvTmemParams &p, float *rows, int warp, int warps, int lane, Seen seen) {
-    const int row = p.c * p.kh * p.kw, stride = filter_stride(p);
-    for (int f = warp; f < p.ko; f += warps) {
+__device__ __forceinline__ void stage_filters(const float *w, int ko, int row, float *rows, int warp, int warps, int lane, Seen seen) {
+    const int stride = row | 1;
+    for (int f = warp; f < ko; f += warps) {
         uint2 range = make_uint2(0u, kNoneSmallest);
 #pragma unroll 4
         for (int e = lane; e < row; e += 32) {
-            const float v = p.w[(int64_t)f * row + e];
+            const float v = w[(int64_t)f * row + e];
             range_take(range, v);
             rows[f * stride + e] = v;
         }
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
     int any       = 0;
     for (int q0 = warp * 32; q0 < own; q0 += (int)blockDim.x) {
         const int q         = q0 + lane;
-        const bool mine     = q < own && image_needs_tf32<RAW>(p, ((int)blockIdx.x + q * (int)gridDim.x) / p.tiles_y, total_tiles);
+        const bool mine     = q < own && image_needs_tf32<RAW>(p, ((int)blockIdx.x + q * (int)gridDim.x) / p.tiles_y);
         const uint32_t bits = __ballot_sync(0xffffffffu, mine);
         any |= bits != 0u;
         if (lane == 0)
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
     if (threadIdx.x == 0)
         abort_flag_s = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
     if (!__syncthreads_or(any) || abort_flag_s)
-        return; // conv_tmem_half_kernel has computed them all
+        return; // conv_pairs_kernel has computed them all
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t stage_bytes = 2u * (uint32_t)p.plane_bytes;
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
         tmem_relinquish();
     }
     float *filters = reinterpret_cast<float *>(smem_raw + (smem_base - smem_u32(smem_raw))); // where the stages will be
-    stage_filters(p, filters, warp, (int)blockDim.x / 32, lane, [](int, uint2) {});
+    stage_filters(p.w, p.ko, p.c * p.kh * p.kw, filters, warp, (int)blockDim.x / 32, lane, [](int, uint2) {});
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
         const int ch      = m & 63;                   // filter
         const bool lo_row = m >= 64;                  // rows 64..127: the low parts
         const int taps    = p.kh * p.kw;
-        const float *src  = filters + ch * filter_stride(p);
+        const float *src  = filters + ch * ((p.c * taps) | 1);
 #pragma unroll 2
         for (int ks = 0; ks < p.ksteps; ++ks) {
             const int tap = ks >> 2, c0 = (ks & 3) * 8;
@@ -645,51 +645,69 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
         atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
 }
 
-// ---- the same in split float16 ------------------------------------------------------------
+// ---- split float16 --------------------------------------------------------------------------
 //
-// Two 11-bit terms in float16 instead of tf32 (half_split.cuh): 16 channels per MMA instead of 8, so half the
-// MMAs, half the filter columns in tensor memory and half the plane bytes.  The filters are scaled per
-// filter, the pixels per tile (the converting warps see the whole box before they split it) or, from planes,
-// per image.  The low terms are stored 2^11 times larger, so hi and lo products have accumulators of their own:
-//     D1 = [W_hi; W_lo] x X_hi,  D2 = [W_hi; W_lo] x X_lo   (128 x 128 each, next to at most 192 filter columns)
-// and a thread that drains row m forms D1 + 2^-11 D2 before anything is parked, which leaves the rest of the
-// epilogue as it is above (hi row + lo row).  Eight warps convert (four needed 4250 clocks per tile where the
-// MMAs now take 2628) and what sets the pace is the epilogue.  The converting warps also leave the range of every
-// tile in the call's own scratch; conv_tmem_filters_kernel, launched behind this one, computes the images that
-// float16 pairs cannot hold.  A tile that shows that by itself is not converted, multiplied or stored here.
-constexpr int kTH_CvtWarps = 8;
-constexpr int kTH_Threads  = 64 + 32 * kTH_CvtWarps + 32 * kTA_EpiWarps;
-constexpr int kTH_D1 = 192, kTH_D2 = 320; // accumulator columns behind 24 k-steps of 8 filter columns
-constexpr int kTH_RowB = 64;              // a position's 32 channels
+// Two 11-bit terms in float16 instead of tf32 (half_split.cuh), pixels on the accumulator rows.  A tile is 2 jp output
+// rows of an image: its even rows are the 128 rows of one accumulator, its odd rows those of another, positions j * pw + x
+// each.  The input rows of a tile lie in shared memory as two regions, even and odd rows of the box, so that filter tap
+// (r, s) is, for the even (odd) output rows, region r & 1 ((r + 1) & 1) through a descriptor moved by
+// (r >> 1) * pw + s (((r + 1) >> 1) * pw + s) rows.  The filters are the B operand and stay in shared memory for the
+// whole launch, hi terms before lo terms for each tap.  Per 16 channels and tap two MMAs an accumulator:
+//     [main | cross] += X_hi x [W_hi; W_lo]     N = 2 kop
+//             cross  += X_lo x W_hi             N = kop
+// with the low terms stored 2^11 times larger and the cross products in columns of their own, as in gemm_half.cu.
+//
+// Why so.  With the filters on the rows and in tensor memory (hi and lo terms on rows 0 - 63 and 64 - 127, the layout of the
+// tf32 form above) the two halves of an output met in shared memory, 128 KB a tile of 128 positions, and that epilogue
+// took 5200 clocks where the MMAs took 2628.  Here a lane holds a pixel and its registers channels: the two accumulators'
+// rows are vertical neighbours, horizontal ones are lanes, so the sum, the activation, the 2x2 maximum and the store
+// need no shared memory at all, and a store covers consecutive pixels of a channel.
+//
+// Scales: per filter, and per tile (raw: the converting warps see the whole box before they split it) or, from planes, per
+// image.  The converting warps also leave the range of every tile in the call's own scratch; conv_tmem_filters_kernel,
+// launched behind this one, computes the images that float16 pairs cannot hold.  A tile that shows that by itself is
+// not converted, multiplied or stored here.
+constexpr int kCP_CvtWarps  = 8;
+constexpr int kCP_EpiWarps  = 8;
+constexpr int kCP_Threads   = 64 + 32 * (kCP_CvtWarps + kCP_EpiWarps);
+constexpr int kCP_RowB      = 64; // a position's 32 channels
+constexpr int kCP_MaxStages = 4;
+constexpr int kCP_Smem      = 226 * 1024;
 
-__device__ __forceinline__ void mma_f16_a_tmem(
-    uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-        "}\n"
-        :
-        : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
+struct ConvPairParams {
+    const float *w;    // filters [ko][c][kh][kw], float32
+    const float *bias;
+    float *out;        // [batch][ko][ho][wo], or [batch][ko][ho/2][wo/2] with pool
+    uint32_t *flags;
+    int ko, kop, c, kh, kw, pad; // kop: ko rounded up to 16
+    int ho, wo, pw;    // pw = input width + 2 pad
+    int jp, tiles_y;   // pairs of output rows per tile, tiles per image
+    int region_rows;   // input rows of a region
+    int region_bytes;  // shared memory of a region of one plane
+    int filter_bytes;
+    int stages;
+    int act, pool;
+    const float *image_scale; // planes: [batch] inverse scales, 0 for an image that needs tf32 terms
+    uint2 *tile_range;        // as in ConvTmemParams
+    // raw mode, as in ConvTmemParams
+    int box_w, off_x, box_rows, raw_bytes, raw_stride;
+};
 
 template <bool RAW>
-__global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
+__global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
     const __grid_constant__ CUtensorMap map_x_hi, const __grid_constant__ CUtensorMap map_x_lo,
-    const __grid_constant__ ConvTmemParams p, const int total_tiles) {
-    constexpr int kMaxStages = 4;
+    const __grid_constant__ ConvPairParams p, const int total_tiles) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t bar_full[kMaxStages], bar_empty[kMaxStages];
-    __shared__ uint64_t bar_raw_full[kTA_RawStages], bar_raw_empty[kTA_RawStages];
-    __shared__ uint64_t bar_scale_empty[kMaxStages]; // the tile's scale has been read by the epilogue
-    __shared__ uint64_t bar_tmem_full, bar_tmem_empty, bar_done, bar_epi, bar_cvt;
+    __shared__ uint64_t bar_full[kCP_MaxStages], bar_empty[kCP_MaxStages];
+    __shared__ uint64_t bar_raw_full, bar_raw_empty;
+    __shared__ uint64_t bar_scale_empty[kCP_MaxStages]; // the tile's scale has been read by the epilogue
+    __shared__ uint64_t bar_acc_full[2], bar_acc_empty[2]; // tiles alternate between two sets of 256 columns
+    __shared__ uint64_t bar_done, bar_cvt;
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag_s, filters_wide_s;
-    __shared__ uint2 cvt_range[2][kTH_CvtWarps];
-    __shared__ float tile_scale[kMaxStages]; // inverse scale of the tile in each plane stage; 0: left to the tf32 form
-    __shared__ float filter_inv[64];
+    __shared__ uint2 cvt_range[2][kCP_CvtWarps];
+    __shared__ float tile_scale[kCP_MaxStages]; // inverse scale of the tile in each plane stage; 0: left to the tf32 form
+    __shared__ __align__(16) float filter_inv[64], bias_s[64];
     volatile int *abort_flag = &abort_flag_s;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -697,39 +715,42 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
         abort_flag_s   = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
         filters_wide_s = 0;
     }
-    if (threadIdx.x < 64)
-        filter_inv[threadIdx.x] = 1.0f; // rows without a filter are zero
+    if (threadIdx.x < 64) {
+        filter_inv[threadIdx.x] = 1.0f;
+        bias_s[threadIdx.x]     = p.bias && (int)threadIdx.x < p.ko ? p.bias[threadIdx.x] : 0.0f;
+    }
     __syncthreads();
     if (abort_flag_s)
         return;
 
     const uint32_t smem_base   = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t stage_bytes = 2u * (uint32_t)p.plane_bytes;
-    const uint32_t raw_base    = smem_base + (uint32_t)p.stages * stage_bytes;
-    const uint32_t raw_all     = RAW ? (uint32_t)kTA_RawStages * (uint32_t)p.raw_stride : 0u;
-    float *staging = reinterpret_cast<float *>(smem_raw + (raw_base - smem_u32(smem_raw)) + raw_all);
+    uint8_t *const smem_ptr    = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t region      = (uint32_t)p.region_bytes;
+    const uint32_t stage_bytes = 4u * region; // hi even, hi odd, lo even, lo odd
+    const uint32_t stage_base  = smem_base + (uint32_t)p.filter_bytes;
+    const uint32_t raw_base    = stage_base + (uint32_t)p.stages * stage_bytes;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
-            mbar_init(smem_u32(&bar_full[s]), RAW ? kTH_CvtWarps : 1);
+            mbar_init(smem_u32(&bar_full[s]), RAW ? kCP_CvtWarps : 1);
             mbar_init(smem_u32(&bar_empty[s]), 1);
-            mbar_init(smem_u32(&bar_scale_empty[s]), kTA_EpiWarps);
+            mbar_init(smem_u32(&bar_scale_empty[s]), kCP_EpiWarps);
         }
-        for (int s = 0; s < kTA_RawStages; ++s) {
-            mbar_init(smem_u32(&bar_raw_full[s]), 1);
-            mbar_init(smem_u32(&bar_raw_empty[s]), kTH_CvtWarps);
+        mbar_init(smem_u32(&bar_raw_full), 1);
+        mbar_init(smem_u32(&bar_raw_empty), kCP_CvtWarps);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(smem_u32(&bar_acc_full[b]), 1);
+            mbar_init(smem_u32(&bar_acc_empty[b]), kCP_EpiWarps);
         }
-        mbar_init(smem_u32(&bar_tmem_full), 1);
-        mbar_init(smem_u32(&bar_tmem_empty), kTA_EpiWarps);
         mbar_init(smem_u32(&bar_done), 1);
-        mbar_init(smem_u32(&bar_epi), kTA_EpiWarps);
-        mbar_init(smem_u32(&bar_cvt), kTH_CvtWarps);
+        mbar_init(smem_u32(&bar_cvt), kCP_CvtWarps);
         mbar_fence_init();
         prefetch_tensormap(&map_x_hi);
         prefetch_tensormap(&map_x_lo);
     }
-    float *filters = reinterpret_cast<float *>(smem_raw + (smem_base - smem_u32(smem_raw))); // where the stages will be
-    stage_filters(p, filters, warp, kTH_Threads / 32, lane, [&](int f, uint2 range) {
+    float *filters = reinterpret_cast<float *>(smem_ptr + p.filter_bytes); // where the stages will be
+    const int taps = p.kh * p.kw, filter_stride = (p.c * taps) | 1;
+    stage_filters(p.w, p.ko, p.c * taps, filters, warp, kCP_Threads / 32, lane, [&](int f, uint2 range) {
         float scale, inverse;
         const bool fits = half_range_fits(range_warp(range), scale, inverse);
         if (lane == 0) {
@@ -750,68 +771,62 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
     if (RAW && blockIdx.x == 0 && threadIdx.x == 0)
         p.tile_range[total_tiles] = make_uint2(filters_wide ? 1u : 0u, 0u);
 
-    // ---- the filters go to tensor memory, once: warps 2..5 own the four lane quarters ----------
-    if (warp >= 2 && warp < 6 && !filters_wide) {
-        const int quarter = warp & 3;
-        const int m = quarter * 32 + lane, ch = m & 63; // TMEM lane = row of the A operand; filter
-        const bool lo_row = m >= 64;
-        const int taps    = p.kh * p.kw;
-        const float *src  = filters + ch * filter_stride(p);
-        const float scale = 1.0f / filter_inv[ch]; // both are powers of two
-#pragma unroll 2
-        for (int ks = 0; ks < 2 * taps; ++ks) {
-            const int tap = ks >> 1, c0 = (ks & 1) * 16;
-            uint32_t v[8];
+    // ---- the filters' planes, once: per tap kop rows of hi terms, then kop of lo terms, 64-byte rows, swizzled ----
+    if (!filters_wide)
+        for (int i = threadIdx.x; i < taps * p.kop * 4; i += kCP_Threads) {
+            const int chunk = i & 3, f = (i >> 2) % p.kop, tap = (i >> 2) / p.kop, c0 = chunk * 8;
+            const float *src  = filters + f * filter_stride;
+            const float scale = 1.0f / filter_inv[f]; // both are powers of two
+            __half2 hi[4], lo[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < 4; ++j) {
                 const int ic  = c0 + 2 * j;
-                const float a = (ch < p.ko && ic < p.c) ? src[ic * taps + tap] : 0.0f;
-                const float b = (ch < p.ko && ic + 1 < p.c) ? src[(ic + 1) * taps + tap] : 0.0f;
-                __half2 hi, lo;
-                split_half_pair(a * scale, b * scale, hi, lo);
-                v[j] = lo_row ? *reinterpret_cast<uint32_t *>(&lo) : *reinterpret_cast<uint32_t *>(&hi);
+                const float a = (f < p.ko && ic < p.c) ? src[ic * taps + tap] : 0.0f;
+                const float b = (f < p.ko && ic + 1 < p.c) ? src[(ic + 1) * taps + tap] : 0.0f;
+                split_half_pair(a * scale, b * scale, hi[j], lo[j]);
             }
-            tmem_st_32x32_x8(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ks * 8), v);
+            auto at = [&](int row) { return smem_ptr + ((size_t)tap * 2 * p.kop + row) * kCP_RowB + ((chunk ^ ((row >> 1) & 3)) << 4); };
+            *reinterpret_cast<uint4 *>(at(f))         = *reinterpret_cast<uint4 *>(hi);
+            *reinterpret_cast<uint4 *>(at(p.kop + f)) = *reinterpret_cast<uint4 *>(lo);
         }
-        tmem_st_wait();
-        filters_taken();
-    }
-    tc_fence_before_sync();
+    filters_taken();
     __syncthreads();
-    tc_fence_after_sync();
 
     if (filters_wide) {
     } else if (warp == 0) {
-        // ===== TMA producer: one halo box per plane and tile (raw mode: one box of the input) =====
+        // ===== TMA producer: one box per plane and region (raw mode: one box of the input) =====
         if (lane == 0) {
             int i = 0;
-            const int nstages = RAW ? kTA_RawStages : p.stages;
+            const int nstages = RAW ? 1 : p.stages;
             for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
                 const int img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
-                if (!RAW && image_needs_tf32<RAW>(p, img, total_tiles))
+                if (!RAW && p.image_scale[img] == 0.0f)
                     continue;
                 const int s       = i % nstages;
                 const uint32_t ph = (uint32_t)(i / nstages) & 1u;
-                if (!mbar_wait_patient(smem_u32(RAW ? &bar_raw_empty[s] : &bar_empty[s]), ph ^ 1u, abort_flag))
+                if (!mbar_wait_patient(smem_u32(RAW ? &bar_raw_empty : &bar_empty[s]), ph ^ 1u, abort_flag))
                     break;
-                const int32_t h0 = ty * p.th - p.pad;
+                const int32_t h0 = ty * 2 * p.jp - p.pad;
                 if (RAW) {
-                    const uint32_t full = smem_u32(&bar_raw_full[s]);
+                    const uint32_t full = smem_u32(&bar_raw_full);
                     mbar_expect_tx(full, (uint32_t)p.raw_bytes);
                     // the box starts off_x floats left of x = -pad so that its first byte is 16-byte aligned
-                    tma_load_4d(raw_base + (uint32_t)s * (uint32_t)p.raw_stride, &map_x_hi, full, -p.pad - p.off_x, h0, 0, img);
+                    tma_load_4d(raw_base, &map_x_hi, full, -p.pad - p.off_x, h0, 0, img);
                 } else {
-                    const uint32_t full = smem_u32(&bar_full[s]), dst = smem_base + (uint32_t)s * stage_bytes;
-                    mbar_expect_tx(full, 2u * (uint32_t)p.box_bytes);
-                    tma_load_4d(dst, &map_x_hi, full, 0, -p.pad, h0, img);
-                    tma_load_4d(dst + (uint32_t)p.plane_bytes, &map_x_lo, full, 0, -p.pad, h0, img);
+                    const uint32_t full = smem_u32(&bar_full[s]), dst = stage_base + (uint32_t)s * stage_bytes;
+                    mbar_expect_tx(full, 4u * (uint32_t)(p.region_rows * p.pw * kCP_RowB));
+                    for (int g = 0; g < 2; ++g) { // region g: rows h0 + g + 2 i, which lie in one of the two sub-images
+                        const int32_t row = (h0 + g) >> 1, sub = (h0 + g) & 1;
+                        tma_load_5d(dst + (uint32_t)g * region, &map_x_hi, full, 0, -p.pad, row, sub, img);
+                        tma_load_5d(dst + (uint32_t)(2 + g) * region, &map_x_lo, full, 0, -p.pad, row, sub, img);
+                    }
                 }
                 ++i;
             }
             if (*abort_flag) {
                 // unwind: let the copies still in flight land before the CTA goes away
                 for (int k2 = i - nstages < 0 ? 0 : i - nstages; k2 < i; ++k2) {
-                    const uint32_t bar = smem_u32(RAW ? &bar_raw_full[k2 % nstages] : &bar_full[k2 % nstages]);
+                    const uint32_t bar = smem_u32(RAW ? &bar_raw_full : &bar_full[k2 % nstages]);
                     const uint64_t t0  = globaltimer_ns();
                     while (!mbar_try_wait(bar, (uint32_t)(k2 / nstages) & 1u) && globaltimer_ns() - t0 < kWaitBudgetNs) {
                     }
@@ -821,38 +836,49 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
     } else if (warp == 1) {
         // ===== MMA issuer =====
         if (lane == 0) {
-            const uint32_t idesc = make_idesc(0u, 128, (uint32_t)kTA_N);
-            const uint32_t d1 = tmem_base + (uint32_t)kTH_D1, d2 = tmem_base + (uint32_t)kTH_D2;
+            const uint32_t idesc2 = make_idesc(0u, 128, (uint32_t)(2 * p.kop)), idesc1 = make_idesc(0u, 128, (uint32_t)p.kop);
+            const bool two = p.c > 16; // k-steps that hold channels
+            // descriptors are moved by adding to their address field (16-byte units; shared memory is far below its range)
+            const uint64_t filter0 = smem_desc_k<kCP_RowB>(smem_base), lo_terms = (uint64_t)(2 * region >> 4);
+            const uint64_t filter_step = (uint64_t)(2 * p.kop * kCP_RowB >> 4);
+            const uint32_t kop = (uint32_t)p.kop;
             int i   = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-                if (!RAW && image_needs_tf32<RAW>(p, tile / p.tiles_y, total_tiles))
+                if (!RAW && p.image_scale[tile / p.tiles_y] == 0.0f)
                     continue;
-                const int s = i % p.stages;
-                // the accumulators of the previous tile have been read, the planes are complete
-                ok = mbar_wait(smem_u32(&bar_tmem_empty), ((uint32_t)i & 1u) ^ 1u, abort_flag) &&
+                const int s = i % p.stages, set = i & 1;
+                // the accumulators have been read, the planes are complete
+                ok = mbar_wait(smem_u32(&bar_acc_empty[set]), ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag) &&
                      mbar_wait(smem_u32(&bar_full[s]), (uint32_t)(i / p.stages) & 1u, abort_flag);
                 if (!ok)
                     break;
                 tc_fence_after_sync();
-                const uint32_t x_hi = smem_base + (uint32_t)s * stage_bytes, x_lo = x_hi + (uint32_t)p.plane_bytes;
-                int ks = 0;
+                const uint32_t hi0 = stage_base + (uint32_t)s * stage_bytes;
+                const uint32_t d_even = tmem_base + (uint32_t)(set * 256), d_odd = d_even + 128u;
+                uint64_t db = filter0;
+                uint32_t accumulate = 0u;
                 const int rows = RAW && *const_cast<volatile float *>(&tile_scale[s]) == 0.0f ? 0 : p.kh;
                 for (int r = 0; r < rows; ++r) {
-                    for (int sx = 0; sx < p.kw; ++sx) {
-                        // the tap's pixels: the same box, (r * pw + sx) rows further on
-                        const uint32_t shift = (uint32_t)(r * p.pw + sx) * (uint32_t)kTH_RowB;
-                        const uint64_t db_hi = smem_desc_k<kTH_RowB>(x_hi + shift), db_lo = smem_desc_k<kTH_RowB>(x_lo + shift);
-#pragma unroll
-                        for (int kk = 0; kk < 2; ++kk, ++ks) {
-                            const uint32_t a_tmem = tmem_base + (uint32_t)(ks * 8);
-                            mma_f16_a_tmem(d1, a_tmem, db_hi + 2 * kk, idesc, ks == 0 ? 0u : 1u);
-                            mma_f16_a_tmem(d2, a_tmem, db_lo + 2 * kk, idesc, ks == 0 ? 0u : 1u);
+                    // the tap's pixels for the even and the odd output rows
+                    uint64_t even = smem_desc_k<kCP_RowB>(hi0 + (uint32_t)(r & 1) * region + (uint32_t)((r >> 1) * p.pw * kCP_RowB));
+                    uint64_t odd  = smem_desc_k<kCP_RowB>(hi0 + (uint32_t)((r + 1) & 1) * region + (uint32_t)(((r + 1) >> 1) * p.pw * kCP_RowB));
+                    for (int sx = 0; sx < p.kw; ++sx, even += kCP_RowB >> 4, odd += kCP_RowB >> 4, db += filter_step) {
+                        mma_f16(d_even, even, db, idesc2, accumulate);
+                        mma_f16(d_odd, odd, db, idesc2, accumulate);
+                        mma_f16(d_even + kop, even + lo_terms, db, idesc1, 1u);
+                        mma_f16(d_odd + kop, odd + lo_terms, db, idesc1, 1u);
+                        accumulate = 1u;
+                        if (two) {
+                            mma_f16(d_even, even + 2, db + 2, idesc2, 1u);
+                            mma_f16(d_odd, odd + 2, db + 2, idesc2, 1u);
+                            mma_f16(d_even + kop, even + lo_terms + 2, db + 2, idesc1, 1u);
+                            mma_f16(d_odd + kop, odd + lo_terms + 2, db + 2, idesc1, 1u);
                         }
                     }
                 }
-                tc_commit(smem_u32(&bar_empty[s]));  // the stage is free once these MMAs have retired
-                tc_commit(smem_u32(&bar_tmem_full)); // and the accumulators are complete
+                tc_commit(smem_u32(&bar_empty[s]));      // the stage is free once these MMAs have retired
+                tc_commit(smem_u32(&bar_acc_full[set])); // and the accumulators are complete
                 ++i;
             }
             if (!ok || *abort_flag) {
@@ -862,24 +888,24 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                 }
             }
         }
-    } else if (warp < 2 + kTH_CvtWarps) {
-        // ===== raw mode: float32 box -> float16 planes (warps before the epilogue's: see above) =====
+    } else if (warp < 2 + kCP_CvtWarps) {
+        // ===== raw mode: float32 box -> float16 planes (warps before the epilogue's: the schedulers favour older warps) =====
         if (RAW) {
             const int ct      = threadIdx.x - 64;
             const int npos    = p.box_rows * p.pw;
             const int cstride = p.box_rows * p.box_w; // floats between two channels of one position
+            const float *raw  = reinterpret_cast<const float *>(smem_ptr + (raw_base - smem_base));
             int i = 0;
             for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
-                const int rs = i % kTA_RawStages, s = i % p.stages;
-                bool got = mbar_wait_patient(smem_u32(&bar_raw_full[rs]), (uint32_t)(i / kTA_RawStages) & 1u, abort_flag);
+                const int s = i % p.stages;
+                bool got = mbar_wait_patient(smem_u32(&bar_raw_full), (uint32_t)i & 1u, abort_flag);
                 if (!__all_sync(0xffffffffu, got))
                     break;
-                const float *raw = reinterpret_cast<const float *>(smem_raw + (raw_base - smem_u32(smem_raw)) + (uint32_t)rs * (uint32_t)p.raw_stride);
                 // the tile's range (the whole box, alignment columns included: they are pixels or zero)
                 uint2 range       = make_uint2(0u, kNoneSmallest);
                 const float4 *r4  = reinterpret_cast<const float4 *>(raw);
 #pragma unroll 4
-                for (int e = ct; e < p.raw_bytes / 16; e += 32 * kTH_CvtWarps) {
+                for (int e = ct; e < p.raw_bytes / 16; e += 32 * kCP_CvtWarps) {
                     const float4 q = r4[e];
                     range_take(range, q.x), range_take(range, q.y), range_take(range, q.z), range_take(range, q.w);
                 }
@@ -894,7 +920,7 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                 if (!__all_sync(0xffffffffu, got))
                     break;
 #pragma unroll
-                for (int u = 0; u < kTH_CvtWarps; ++u)
+                for (int u = 0; u < kCP_CvtWarps; ++u)
                     range = range_join(range, cvt_range[i & 1][u]);
                 float scale, inverse;
                 const bool fits = half_range_fits(range, scale, inverse);
@@ -902,14 +928,14 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                     tile_scale[s]      = fits ? inverse : 0.0f;
                     p.tile_range[tile] = range;
                 }
-                uint8_t *x_hi = smem_raw + (smem_base - smem_u32(smem_raw)) + (uint32_t)s * stage_bytes;
-                uint8_t *x_lo = x_hi + p.plane_bytes;
-                // a thread takes a position: 32 channels become the 64-byte row y * pw + x of both planes, 16-byte
-                // chunk j at j ^ ((row >> 1) & 3), the 64-byte swizzle
-                for (int pos = fits ? ct : npos; pos < npos; pos += 32 * kTH_CvtWarps) {
-                    const int y = pos / p.pw, x = pos - y * p.pw;
+                uint8_t *planes = smem_ptr + p.filter_bytes + (uint32_t)s * stage_bytes;
+                // a thread takes a position (y, x): its 32 channels become row (y >> 1) * pw + x of region y & 1 in both
+                // planes, 16-byte chunk j at j ^ ((row >> 1) & 3), the 64-byte swizzle
+                for (int pos = fits ? ct : npos; pos < npos; pos += 32 * kCP_CvtWarps) {
+                    const int y = pos / p.pw, x = pos - y * p.pw, row = (y >> 1) * p.pw + x;
                     const float *src = raw + y * p.box_w + x + p.off_x;
-                    const uint32_t row_off = (uint32_t)pos * (uint32_t)kTH_RowB, sw = ((uint32_t)pos >> 1) & 3u;
+                    uint8_t *dst     = planes + (uint32_t)(y & 1) * region + (uint32_t)row * kCP_RowB;
+                    const uint32_t sw = ((uint32_t)row >> 1) & 3u;
 #pragma unroll
                     for (int half = 0; half < 2; ++half) {
                         float v[16];
@@ -920,12 +946,11 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                         for (int j = 0; j < 2; ++j) {
                             __half2 hi[4], lo[4];
 #pragma unroll
-                            for (int t = 0; t < 4; ++t) {
+                            for (int t = 0; t < 4; ++t)
                                 split_half_pair(__fmul_rn(v[8 * j + 2 * t], scale), __fmul_rn(v[8 * j + 2 * t + 1], scale), hi[t], lo[t]);
-                            }
-                            const uint32_t at = row_off + (((uint32_t)(2 * half + j) ^ sw) << 4);
-                            *reinterpret_cast<uint4 *>(x_hi + at) = *reinterpret_cast<uint4 *>(hi);
-                            *reinterpret_cast<uint4 *>(x_lo + at) = *reinterpret_cast<uint4 *>(lo);
+                            const uint32_t at = ((uint32_t)(2 * half + j) ^ sw) << 4;
+                            *reinterpret_cast<uint4 *>(dst + at)              = *reinterpret_cast<uint4 *>(hi);
+                            *reinterpret_cast<uint4 *>(dst + 2 * region + at) = *reinterpret_cast<uint4 *>(lo);
                         }
                     }
                 }
@@ -934,189 +959,84 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
                 __syncwarp();
                 if (lane == 0) {
                     mbar_arrive(smem_u32(&bar_full[s]));
-                    mbar_arrive(smem_u32(&bar_raw_empty[rs]));
+                    mbar_arrive(smem_u32(&bar_raw_empty));
                 }
             }
         }
     } else {
-        // ===== epilogue =====
-        const int quarter = warp & 3;                // TMEM lanes this warp may read
-        const int ew      = warp - 2 - kTH_CvtWarps; // 0..7: which channels this warp writes out
-        const int half    = ew >> 2;                 // which 64 columns of the accumulators it drains
-        uint32_t epi_phase = 0;
-        auto epi_sync = [&]() -> bool {
-            __syncwarp();
-            if (lane == 0)
-                mbar_arrive(smem_u32(&bar_epi));
-            bool ok = mbar_wait_patient(smem_u32(&bar_epi), epi_phase, abort_flag);
-            epi_phase ^= 1u;
-            return __all_sync(0xffffffffu, ok);
-        };
-        // where this lane's positions land, once for the whole kernel (see conv_tmem_filters_kernel)
-        int off[4], yy[4];
-        const int npos = p.th * p.pw;
-        const int pw2 = p.wo >> 1, ph2 = p.ho >> 1;
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-            const int pos = lane + 32 * g;
-            off[g] = -1, yy[g] = 0;
-            if (p.pool == 0) {
-                const int y = pos / p.pw, x = pos - y * p.pw;
-                if (pos < npos && x < p.wo)
-                    off[g] = y * p.wo + x, yy[g] = y;
-            } else {
-                const int py = pos / pw2, px = pos - py * pw2;
-                if (py < (p.th >> 1))
-                    off[g] = (2 * py) * p.pw + 2 * px, yy[g] = py; // here: the window's first position
-            }
-        }
-        float bias_r[64 / kTA_EpiWarps];
-#pragma unroll
-        for (int j = 0; j < 64 / kTA_EpiWarps; ++j) {
-            const int ch = ew + kTA_EpiWarps * j;
-            bias_r[j]    = (p.bias && ch < p.ko) ? p.bias[ch] : 0.0f;
-        }
-        const int m       = quarter * 32 + lane;
-        const float row_f = m < 64 ? filter_inv[m] : filter_inv[m - 64] * kHalfLoInv;
+        // ===== epilogue: a lane has a position, groups of sixteen channels in turn =====
+        const int quarter = warp & 3;                       // TMEM lanes this warp may read
+        const int half    = (warp - 2 - kCP_CvtWarps) >> 2; // which groups of channels are its
+        const int m = quarter * 32 + lane, j = m / p.pw, x = m - j * p.pw;
+        const int groups = p.kop >> 4;
+        const int64_t plane = p.pool ? (int64_t)(p.ho >> 1) * (p.wo >> 1) : (int64_t)p.ho * p.wo;
+        const bool inside = j < p.jp && x < p.wo && !(p.pool && (x & 1));
         int i = 0;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
+        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
             const int img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
-            if (!RAW && image_needs_tf32<RAW>(p, img, total_tiles)) {
-                --i;
+            if (!RAW && p.image_scale[img] == 0.0f)
                 continue;
-            }
-            bool got = mbar_wait_patient(smem_u32(&bar_tmem_full), (uint32_t)i & 1u, abort_flag);
+            const int set = i & 1, s = i % p.stages;
+            bool got = mbar_wait_patient(smem_u32(&bar_acc_full[set]), (uint32_t)(i >> 1) & 1u, abort_flag);
             if (!__all_sync(0xffffffffu, got))
                 break;
-            const float is = RAW ? *const_cast<volatile float *>(&tile_scale[i % p.stages]) : p.image_scale[img];
-            const int y0   = ty * p.th;
+            const float is = RAW ? *const_cast<volatile float *>(&tile_scale[s]) : p.image_scale[img];
             tc_fence_after_sync();
-            if (RAW && is == 0.0f) {
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(smem_u32(&bar_tmem_empty));
-                    mbar_arrive(smem_u32(&bar_scale_empty[i % p.stages]));
-                }
-                continue;
-            }
-            float4 *mine         = reinterpret_cast<float4 *>(staging + m * kTA_StageRowF + half * 64);
-            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 64);
-            // D1 + 2^-11 D2, sixteen columns of each at a time; the accumulators are handed back before anything
-            // is parked
-            float t[64];
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                uint32_t a[16], b[16];
-                tmem_ld_32x16(taddr + kTH_D1 + 16 * g, a);
-                tmem_ld_32x16(taddr + kTH_D2 + 16 * g, b);
+            const int y = (ty * p.jp + j) * 2; // the even row; the odd one may be past the image
+            const bool live_even = inside && y < p.ho, live_odd = inside && y + 1 < p.ho;
+            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(set * 256);
+            float *dst = p.out + ((int64_t)img * p.ko + half * 16) * plane + (p.pool ? (int64_t)(y >> 1) * (p.wo >> 1) + (x >> 1) : (int64_t)y * p.wo + x);
+            for (int g = half; g < groups && !(RAW && is == 0.0f); g += 2, dst += 32 * plane) {
+                uint32_t a[16], b[16], c[16], d[16];
+                tmem_ld_32x16(taddr + (uint32_t)(16 * g), a);
+                tmem_ld_32x16(taddr + (uint32_t)(p.kop + 16 * g), b);
+                tmem_ld_32x16(taddr + (uint32_t)(128 + 16 * g), c);
+                tmem_ld_32x16(taddr + (uint32_t)(128 + p.kop + 16 * g), d);
                 tmem_ld_wait();
+                float *at = dst;
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    t[16 * g + j] = __fadd_rn(__uint_as_float(a[j]), __fmul_rn(__uint_as_float(b[j]), kHalfLoInv));
+                for (int u = 0; u < 16; u += 4) {
+                    const float4 f4 = *reinterpret_cast<const float4 *>(filter_inv + 16 * g + u);
+                    const float4 b4 = *reinterpret_cast<const float4 *>(bias_s + 16 * g + u);
+                    const float fs[4] = {f4.x, f4.y, f4.z, f4.w}, bs[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q, at += plane) {
+                        auto value = [&](uint32_t main, uint32_t cross) {
+                            float v = __fadd_rn(__uint_as_float(main), __fmul_rn(__uint_as_float(cross), kHalfLoInv));
+                            v       = __fmul_rn(__fmul_rn(v, fs[q]), is);
+                            if (p.bias)
+                                v = __fadd_rn(v, bs[q]);
+                            if (p.act == CT_ACT_RELU)
+                                v = __fmul_rn(v, v > 0.0f ? 1.0f : 0.0f);
+                            return v;
+                        };
+                        const float even = value(a[u + q], b[u + q]), odd = value(c[u + q], d[u + q]);
+                        const bool filter = 16 * g + u + q < p.ko;
+                        if (p.pool == 0) {
+                            if (live_even && filter)
+                                at[0] = even;
+                            if (live_odd && filter)
+                                at[p.wo] = odd;
+                        } else {
+                            // window order and strict '>' as in maxpool2d
+                            const float even1 = __shfl_down_sync(0xffffffffu, even, 1), odd1 = __shfl_down_sync(0xffffffffu, odd, 1);
+                            float best = even1 > even ? even1 : even;
+                            const float low = odd1 > odd ? odd1 : odd;
+                            best = low > best ? low : best;
+                            if (live_odd && filter)
+                                at[0] = best;
+                        }
+                    }
+                }
             }
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive(smem_u32(&bar_tmem_empty)); // the next tile's MMAs may start
-                mbar_arrive(smem_u32(&bar_scale_empty[i % p.stages]));
+                mbar_arrive(smem_u32(&bar_acc_empty[set]));
+                if (RAW)
+                    mbar_arrive(smem_u32(&bar_scale_empty[s]));
             }
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-                mine[j] = make_float4(__fmul_rn(t[4 * j], row_f), __fmul_rn(t[4 * j + 1], row_f),
-                                      __fmul_rn(t[4 * j + 2], row_f), __fmul_rn(t[4 * j + 3], row_f));
-            if (!epi_sync())
-                break;
-            unsigned okmask = 0;
-#pragma unroll
-            for (int g = 0; g < 4; ++g)
-                if (off[g] >= 0 && (p.pool ? (y0 >> 1) + yy[g] < ph2 : y0 + yy[g] < p.ho))
-                    okmask |= 1u << g;
-            // two channels at a time, every load of the pair before the first dependent instruction, masked stores
-            if (p.pool == 0) {
-#pragma unroll
-                for (int jj = 0; jj < 64 / kTA_EpiWarps; jj += 2) {
-                    float h[2][4], l[2][4];
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const float *hi = staging + (ew + kTA_EpiWarps * (jj + u)) * kTA_StageRowF + lane, *lo = hi + 64 * kTA_StageRowF;
-#pragma unroll
-                        for (int g = 0; g < 4; ++g)
-                            h[u][g] = hi[32 * g], l[u][g] = lo[32 * g];
-                    }
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const int ch = ew + kTA_EpiWarps * (jj + u);
-                        float *plane = p.out + (((int64_t)img * p.ko + ch) * p.ho + y0) * p.wo;
-                        const unsigned mask = ch < p.ko ? okmask : 0u;
-#pragma unroll
-                        for (int g = 0; g < 4; ++g) {
-                            float v = __fmul_rn(__fadd_rn(h[u][g], l[u][g]), is);
-                            if (p.bias)
-                                v = __fadd_rn(v, bias_r[jj + u]);
-                            if (p.act == CT_ACT_RELU)
-                                v = __fmul_rn(v, v > 0.0f ? 1.0f : 0.0f);
-                            if (mask & (1u << g))
-                                plane[off[g]] = v;
-                        }
-                    }
-                }
-            } else {
-                // 2x2 max-pool of the activated values; window order and strict '>' as in maxpool2d.  Four channels
-                // at a time with all their loads first, a window row as one 8-byte read where rows are even: with
-                // scalar reads for two channels this phase took 3500 clocks per tile, the longest of all.
-                const int groups = ((p.th >> 1) * pw2 + 31) >> 5;
-                const bool even  = (p.pw & 1) == 0;
-#pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    if (g >= groups)
-                        break;
-                    const bool live = (okmask >> g) & 1u;
-                    const int pos   = live ? off[g] : 0;
-#pragma unroll
-                    for (int jj = 0; jj < 64 / kTA_EpiWarps; jj += 4) {
-                        float2 h[4][2], l[4][2];
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const float *hi = staging + (ew + kTA_EpiWarps * (jj + u)) * kTA_StageRowF + pos, *lo = hi + 64 * kTA_StageRowF;
-                            if (even) {
-                                h[u][0] = *reinterpret_cast<const float2 *>(hi), h[u][1] = *reinterpret_cast<const float2 *>(hi + p.pw);
-                                l[u][0] = *reinterpret_cast<const float2 *>(lo), l[u][1] = *reinterpret_cast<const float2 *>(lo + p.pw);
-                            } else {
-                                h[u][0] = make_float2(hi[0], hi[1]), h[u][1] = make_float2(hi[p.pw], hi[p.pw + 1]);
-                                l[u][0] = make_float2(lo[0], lo[1]), l[u][1] = make_float2(lo[p.pw], lo[p.pw + 1]);
-                            }
-                        }
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const int ch = ew + kTA_EpiWarps * (jj + u);
-                            const float hv[4] = {h[u][0].x, h[u][0].y, h[u][1].x, h[u][1].y};
-                            const float lv[4] = {l[u][0].x, l[u][0].y, l[u][1].x, l[u][1].y};
-                            float v[4];
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                v[q] = __fmul_rn(__fadd_rn(hv[q], lv[q]), is);
-                                if (p.bias)
-                                    v[q] = __fadd_rn(v[q], bias_r[jj + u]);
-                                if (p.act == CT_ACT_RELU)
-                                    v[q] = __fmul_rn(v[q], v[q] > 0.0f ? 1.0f : 0.0f);
-                            }
-                            float best = v[0];
-                            if (v[1] > best)
-                                best = v[1];
-                            if (v[2] > best)
-                                best = v[2];
-                            if (v[3] > best)
-                                best = v[3];
-                            if (live && ch < p.ko) {
-                                float *plane = p.out + (((int64_t)img * p.ko + ch) * ph2 + (y0 >> 1)) * pw2;
-                                plane[lane + 32 * g] = best; // pooled pixels of a tile are consecutive
-                            }
-                        }
-                    }
-                }
-            }
-            if (!epi_sync()) // the staging block is rewritten by the next tile
-                break;
+            ++i;
         }
     }
 
@@ -1132,6 +1052,37 @@ __global__ void __launch_bounds__(kTH_Threads, 1) conv_tmem_half_kernel(
 }
 
 } // namespace
+
+static bool conv_pair_plan(
+    ConvPairParams &p, int64_t c, int64_t h, int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t pad, bool raw, size_t *smem) {
+    p.ko = (int)ko, p.kop = (int)((ko + 15) / 16 * 16), p.c = (int)c;
+    p.kh = (int)kh, p.kw = (int)kw, p.pad = (int)pad;
+    p.pw  = (int)(wd + 2 * pad);
+    p.wo  = p.pw - (int)kw + 1;
+    p.ho  = (int)(h + 2 * pad - kh + 1);
+    if (p.pw > 128 || p.wo < 1 || p.ho < 1)
+        return false;
+    p.jp          = std::min(128 / p.pw, (p.ho + 1) / 2);
+    p.tiles_y     = ((p.ho + 1) / 2 + p.jp - 1) / p.jp;
+    p.box_rows    = 2 * p.jp + (int)kh - 1;
+    p.region_rows = (p.box_rows + 1) / 2;
+    // a tap's window of 128 rows may run past the region: reserve those rows too
+    const int rows = std::max(p.region_rows * p.pw, (int)(kh / 2) * p.pw + (int)kw - 1 + 128);
+    p.region_bytes = (rows * kCP_RowB + 1023) & ~1023;
+    p.filter_bytes = (int)((kh * kw * 2 * p.kop * kCP_RowB + 1023) & ~1023);
+    // raw mode: the box starts at the 16-byte boundary at or left of x = -pad and is a whole number of 16-byte units wide
+    p.off_x      = (((int)pad + 3) & ~3) - (int)pad;
+    p.box_w      = (p.off_x + p.pw + 3) & ~3;
+    p.raw_bytes  = 32 * p.box_rows * p.box_w * 4;
+    p.raw_stride = raw ? (p.raw_bytes + 127) & ~127 : 0;
+    if (p.box_w > 256 || p.box_rows > 256)
+        return false;
+    p.stages = std::min(kCP_MaxStages, (kCP_Smem - 1024 - p.filter_bytes - p.raw_stride) / (4 * p.region_bytes));
+    // the float32 filters lie for a moment where the stages will be
+    const int filters = (int)(ko * ((c * kh * kw) | 1) * 4), planes = p.stages * 4 * p.region_bytes + p.raw_stride;
+    *smem = 1024 + (size_t)p.filter_bytes + (size_t)std::max(filters, planes);
+    return p.stages >= 2 && *smem <= (size_t)kCP_Smem;
+}
 
 // Whether the filters-in-tensor-memory kernel takes this layer.  The answer does not depend on
 // whether a max-pool is fused, so that conv2d and conv2d + pool of one layer run the same arithmetic;
@@ -1154,8 +1105,10 @@ bool conv_tmem_applicable(int64_t c, int64_t h, int64_t w, int64_t ko, int64_t k
     if (!(th * pw >= 96 || th == ho))
         return false;
     if (pool_ok)
-        *pool_ok = (wo & 1) == 0 && (ho & 1) == 0 && th >= 2;
-    return true;
+        *pool_ok = (wo & 1) == 0 && (ho & 1) == 0 && (pw & 1) == 0 && th >= 2; // horizontal neighbours in one warp
+    ConvPairParams pairs;
+    size_t smem;
+    return conv_pair_plan(pairs, c, h, w, ko, kh, kw, pad, false, &smem);
 }
 
 // Shared-memory plan of a launch: tile rows, bytes per plane and per raw box, pipeline stages.
@@ -1200,11 +1153,14 @@ static bool conv_tmem_plan(
 // Whether the kernel can read this input as it is (NCHW float32) instead of pre-split NHWC planes:
 // the tensor map over it needs row strides of whole 16-byte units and an aligned base, and the raw
 // boxes have to fit into shared memory beside two stages of planes.
-static bool conv_tmem_reads_input_directly(const float *x, int64_t h, int64_t w, int64_t kh, int64_t kw, int64_t pad, int pool) {
+static bool conv_tmem_reads_input_directly(
+    const float *x, int64_t c, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw, int64_t pad, int pool) {
     if ((w & 3) != 0 || (reinterpret_cast<uintptr_t>(x) & 15u) != 0)
         return false;
     ConvTmemParams p;
-    return conv_tmem_plan(p, h, w, kh, kw, pad, pool, true);
+    ConvPairParams pairs;
+    size_t smem;
+    return conv_tmem_plan(p, h, w, kh, kw, pad, pool, true) && conv_pair_plan(pairs, c, h, w, ko, kh, kw, pad, true, &smem);
 }
 
 // x NCHW float32.  The layer in split float16, and behind it the tf32 form for the images that need it.  Where the
@@ -1214,49 +1170,50 @@ static bool conv_tmem_reads_input_directly(const float *x, int64_t h, int64_t w,
 ct_status conv_tmem_filters(
     DeviceState *st, const float *x, const float *w, const float *bias, int64_t batch, int64_t c, int64_t h, int64_t wd,
     int64_t ko, int64_t kh, int64_t kw, int64_t pad, int act, int pool, float *out) {
-    const bool raw = conv_tmem_reads_input_directly(x, h, wd, kh, kw, pad, pool);
-    ConvTmemParams p[2]; // float16, tf32
-    for (int f = 0; f < 2; ++f) {
-        p[f].w = w, p[f].bias = bias, p[f].out = out, p[f].flags = st->flags_dev;
-        p[f].ko = (int)ko, p[f].c = (int)c;
-        p[f].act = act, p[f].pool = pool;
-        p[f].image_scale = nullptr, p[f].tile_range = nullptr;
-        if (!conv_tmem_plan(p[f], h, wd, kh, kw, pad, pool, raw, f == 0 ? kTH_RowB : 128))
-            return fail(CT_ERR_INVALID, "conv2d: internal tile shape %d x %d not usable", p[f].th, p[f].pw);
-    }
-    const int64_t tiles = (int64_t)p[0].tiles_y * batch;
-    if (tiles > 0x7fffffffll)
+    const bool raw = conv_tmem_reads_input_directly(x, c, h, wd, ko, kh, kw, pad, pool);
+    ConvPairParams pp;
+    ConvTmemParams pt; // the tf32 form
+    size_t pair_smem;
+    if (!conv_pair_plan(pp, c, h, wd, ko, kh, kw, pad, raw, &pair_smem) || !conv_tmem_plan(pt, h, wd, kh, kw, pad, pool, raw))
+        return fail(CT_ERR_INVALID, "conv2d: internal tile shape not usable");
+    pp.w = pt.w = w, pp.bias = pt.bias = bias, pp.out = pt.out = out, pp.flags = pt.flags = st->flags_dev;
+    pt.ko = (int)ko, pt.c = (int)c;
+    pp.act = pt.act = act, pp.pool = pt.pool = pool;
+    pp.image_scale = pt.image_scale = nullptr, pp.tile_range = pt.tile_range = nullptr;
+    const int64_t tiles = (int64_t)pt.tiles_y * batch, pair_tiles = (int64_t)pp.tiles_y * batch;
+    if (tiles > 0x7fffffffll || pair_tiles > 0x7fffffffll)
         return fail(CT_ERR_TOO_LARGE, "conv2d: too many tiles");
+    pt.range_tiles = pp.tiles_y, pt.range_total = (int)pair_tiles;
     static bool attr_set_dev[16] = {}; // the attribute belongs to a device's context
     if (!attr_set_dev[st->device & 15]) {
         CT_CUDA(cudaFuncSetAttribute(conv_tmem_filters_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
         CT_CUDA(cudaFuncSetAttribute(conv_tmem_filters_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        CT_CUDA(cudaFuncSetAttribute(conv_tmem_half_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        CT_CUDA(cudaFuncSetAttribute(conv_tmem_half_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        CT_CUDA(cudaFuncSetAttribute(conv_pairs_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCP_Smem));
+        CT_CUDA(cudaFuncSetAttribute(conv_pairs_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCP_Smem));
         attr_set_dev[st->device & 15] = true;
     }
-    auto smem_of = [&](const ConvTmemParams &q) {
-        return (size_t)q.stages * 2 * q.plane_bytes + (raw ? (size_t)kTA_RawStages * q.raw_stride : 0) + kTA_StagingBytes + 1024;
-    };
-    const unsigned grid   = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
-    const unsigned grid32 = (unsigned)std::max<int64_t>(grid, (tiles + kTA_MaxOwn - 1) / kTA_MaxOwn);
+    const size_t smem32 = (size_t)pt.stages * 2 * pt.plane_bytes + (raw ? (size_t)kTA_RawStages * pt.raw_stride : 0) + kTA_StagingBytes + 1024;
+    const unsigned grid   = (unsigned)std::min<int64_t>(pair_tiles, st->sm_count);
+    const unsigned grid32 = (unsigned)std::max<int64_t>(std::min<int64_t>(tiles, st->sm_count), (tiles + kTA_MaxOwn - 1) / kTA_MaxOwn);
     if (raw) {
         // the input [batch][c][h][w]; box = box_w floats x box_rows rows x 32 channels of one image, not
         // swizzled; outside the image and past the last channel it reads as zero: padding for free
-        CUtensorMap map;
+        CUtensorMap map, map32;
         const uint64_t dims[4]    = {(uint64_t)wd, (uint64_t)h, (uint64_t)c, (uint64_t)batch};
         const uint64_t strides[3] = {4ull * (uint64_t)wd, 4ull * (uint64_t)wd * (uint64_t)h,
                                      4ull * (uint64_t)wd * (uint64_t)h * (uint64_t)c};
-        const uint32_t box[4]     = {(uint32_t)p[0].box_w, (uint32_t)p[0].box_rows, 32, 1};
+        const uint32_t box[4]     = {(uint32_t)pp.box_w, (uint32_t)pp.box_rows, 32, 1};
+        const uint32_t box32[4]   = {(uint32_t)pt.box_w, (uint32_t)pt.box_rows, 32, 1};
         CT_TRY(encode_tiled_map_f32(&map, x, 4, dims, strides, box, /*swizzle_bytes=*/0));
+        CT_TRY(encode_tiled_map_f32(&map32, x, 4, dims, strides, box32, /*swizzle_bytes=*/0));
         void *ranges = nullptr;
-        CT_TRY(ct_alloc(&ranges, (size_t)(tiles + 1) * sizeof(uint2)));
-        p[0].tile_range = p[1].tile_range = static_cast<uint2 *>(ranges);
+        CT_TRY(ct_alloc(&ranges, (size_t)(pair_tiles + 1) * sizeof(uint2)));
+        pp.tile_range = pt.tile_range = static_cast<uint2 *>(ranges);
         cudaError_t launched;
         {
             ProfScope prof("gemm_tc");
-            conv_tmem_half_kernel<true><<<grid, kTH_Threads, smem_of(p[0]), stream()>>>(map, map, p[0], (int)tiles);
-            conv_tmem_filters_kernel<true><<<grid32, kTA_ThreadsRaw, smem_of(p[1]), stream()>>>(map, map, p[1], (int)tiles);
+            conv_pairs_kernel<true><<<grid, kCP_Threads, pair_smem, stream()>>>(map, map, pp, (int)pair_tiles);
+            conv_tmem_filters_kernel<true><<<grid32, kTA_ThreadsRaw, smem32, stream()>>>(map32, map32, pt, (int)tiles);
             launched = cudaGetLastError();
         }
         CT_TRY(ct_free(ranges)); // in stream order, behind both
@@ -1266,33 +1223,38 @@ ct_status conv_tmem_filters(
         return CT_OK;
     }
     auto align_up       = [](size_t v) { return (v + 1023) & ~(size_t)1023; };
-    const size_t f_words = align_up((size_t)ko * 4), words = align_up((size_t)batch * 4), slot = (size_t)h * wd * 32 * 8;
+    const int64_t hs     = (h + 1) / 2; // rows of a sub-image: even and odd rows lie apart (float16 only)
+    const size_t f_words = align_up((size_t)ko * 4), words = align_up((size_t)batch * 4), slot = (size_t)hs * 2 * wd * 32 * 8;
     const size_t ranges  = align_up((size_t)batch * conv_range_slices(batch, c * h * wd) * 8);
     CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, f_words + words + ranges + (size_t)batch * slot));
     uint8_t *ws = static_cast<uint8_t *>(st->gemm_ws), *planes = ws + f_words + words + ranges;
     float *image_scale = reinterpret_cast<float *>(ws + f_words);
     CT_TRY(conv_prepass(st, x, w, batch, c, h, wd, 32, ko, kh * kw, nullptr, nullptr, 0, 0, reinterpret_cast<float *>(ws),
-                        ws + f_words + words, image_scale, planes, ConvSubImages{}));
-    p[0].image_scale = p[1].image_scale = image_scale;
-    // planes [batch][h][w][32 channels]; box = 32 channels x pw positions x (th + kh - 1) rows of one image,
-    // swizzled over a row; positions outside the image read as zero: the padding
-    auto encode = [&](CUtensorMap *map, const void *base, int elem) {
-        const uint64_t row = 32ull * (uint64_t)elem;
+                        ws + f_words + words, image_scale, planes, ConvSubImages{2, 1, 3u, true}));
+    pp.image_scale = pt.image_scale = image_scale;
+    // float16 planes [batch][row & 1][row >> 1][w][32 channels], box = 32 channels x pw positions x region_rows rows of one
+    // sub-image; tf32 planes [batch][h][w][32 channels]; swizzled over a row; outside the image they read as zero: the padding
+    auto encode16 = [&](CUtensorMap *map, const void *base) {
+        const uint64_t dims[5] = {32, (uint64_t)wd, (uint64_t)hs, 2, (uint64_t)batch};
+        const uint64_t strides[4] = {64, 64ull * (uint64_t)wd, 64ull * (uint64_t)(wd * hs), slot};
+        const uint32_t box[5] = {32, (uint32_t)pp.pw, (uint32_t)pp.region_rows, 1, 1};
+        return encode_tiled_map_f16(map, base, 5, dims, strides, box, kCP_RowB);
+    };
+    auto encode32 = [&](CUtensorMap *map, const void *base) {
         const uint64_t dims[4] = {32, (uint64_t)wd, (uint64_t)h, (uint64_t)batch};
-        const uint64_t strides[3] = {row, row * (uint64_t)wd, slot};
-        const uint32_t box[4] = {32, (uint32_t)p[0].pw, (uint32_t)p[0].box_rows, 1};
-        return elem == 4 ? encode_tiled_map_f32(map, base, 4, dims, strides, box, 128)
-                         : encode_tiled_map_f16(map, base, 4, dims, strides, box, kTH_RowB);
+        const uint64_t strides[3] = {128, 128ull * (uint64_t)wd, slot};
+        const uint32_t box[4] = {32, (uint32_t)pt.pw, (uint32_t)pt.box_rows, 1};
+        return encode_tiled_map_f32(map, base, 4, dims, strides, box, 128);
     };
     CUtensorMap m16_hi, m16_lo, m32_hi, m32_lo;
-    CT_TRY(encode(&m16_hi, planes, 2));
-    CT_TRY(encode(&m16_lo, planes + slot / 4, 2));
-    CT_TRY(encode(&m32_hi, planes, 4));
-    CT_TRY(encode(&m32_lo, planes + slot / 2, 4));
+    CT_TRY(encode16(&m16_hi, planes));
+    CT_TRY(encode16(&m16_lo, planes + slot / 4));
+    CT_TRY(encode32(&m32_hi, planes));
+    CT_TRY(encode32(&m32_lo, planes + slot / 2));
     ProfScope prof("gemm_tc");
-    conv_tmem_half_kernel<false><<<grid, kTH_Threads, smem_of(p[0]), stream()>>>(m16_hi, m16_lo, p[0], (int)tiles);
-    CT_LAUNCH_CHECK("conv_tmem_half");
-    conv_tmem_filters_kernel<false><<<grid32, kTA_Threads, smem_of(p[1]), stream()>>>(m32_hi, m32_lo, p[1], (int)tiles);
+    conv_pairs_kernel<false><<<grid, kCP_Threads, pair_smem, stream()>>>(m16_hi, m16_lo, pp, (int)pair_tiles);
+    CT_LAUNCH_CHECK("conv_pairs");
+    conv_tmem_filters_kernel<false><<<grid32, kTA_Threads, smem32, stream()>>>(m32_hi, m32_lo, pt, (int)tiles);
     CT_LAUNCH_CHECK("conv_tmem_filters");
     return CT_OK;
 }
