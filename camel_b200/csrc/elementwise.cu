@@ -130,6 +130,8 @@ __device__ __forceinline__ uint8_t apply_compare_d(int op, double a, double b) {
 // Generic driver: out[i] = f(i-th elements).  VEC=true: all pointers are vector-aligned and
 // the body covers numel/4 vectors; the tail (and the unaligned case) runs with VEC=false.
 template <bool VEC, typename F> __global__ void __launch_bounds__(kThreads) map_kernel(uint64_t count, F f) {
+    griddep_launch_dependents();
+    griddep_wait();
     uint64_t base = (uint64_t)blockIdx.x * (kThreads * kUnroll) + threadIdx.x;
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
@@ -137,6 +139,23 @@ template <bool VEC, typename F> __global__ void __launch_bounds__(kThreads) map_
         if (i < count)
             f(i);
     }
+}
+
+// Vectors and the up to three elements behind them in one launch: as two, the second cost as much as the first up to some
+// 100,000 elements.
+template <typename F, typename T>
+__global__ void __launch_bounds__(kThreads) map_tail_kernel(uint64_t count, F f, uint64_t tail, T t) {
+    griddep_launch_dependents();
+    griddep_wait();
+    uint64_t base = (uint64_t)blockIdx.x * (kThreads * kUnroll) + threadIdx.x;
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+        uint64_t i = base + (uint64_t)u * kThreads;
+        if (i < count)
+            f(i);
+    }
+    if (base < tail)
+        t(base);
 }
 
 template <typename F> ct_status launch_map(uint64_t count, F f, const char *name) {
@@ -147,7 +166,22 @@ template <typename F> ct_status launch_map(uint64_t count, F f, const char *name
     if (blocks > 0x7fffffffull)
         return fail(CT_ERR_TOO_LARGE, "%s: too many elements", name);
     ProfScope prof("elementwise");
-    map_kernel<true, F><<<(unsigned)blocks, kThreads, 0, stream()>>>(count, f);
+    CT_CUDA(launch_dependent(map_kernel<true, F>, dim3((unsigned)blocks), dim3(kThreads), 0, stream(), count, f));
+    CT_LAUNCH_CHECK(name);
+    return CT_OK;
+}
+// fv over `count` vectors, fs over `rest` elements: fewer than a vector's, or all where nothing is aligned.
+template <typename FV, typename FS> ct_status launch_map_tail(uint64_t count, FV fv, uint64_t rest, FS fs, const char *name) {
+    if (count == 0)
+        return launch_map(rest, fs, name);
+    if (rest == 0)
+        return launch_map(count, fv, name);
+    uint64_t per_block = (uint64_t)kThreads * kUnroll;
+    uint64_t blocks    = (count + per_block - 1) / per_block;
+    if (blocks > 0x7fffffffull)
+        return fail(CT_ERR_TOO_LARGE, "%s: too many elements", name);
+    ProfScope prof("elementwise");
+    CT_CUDA(launch_dependent(map_tail_kernel<FV, FS>, dim3((unsigned)blocks), dim3(kThreads), 0, stream(), count, fv, rest, fs));
     CT_LAUNCH_CHECK(name);
     return CT_OK;
 }
@@ -209,27 +243,20 @@ ct_status binary_typed(int op, const void *l, const void *r, uint64_t n, void *o
     const LT *lp = static_cast<const LT *>(l);
     const RT *rp = static_cast<const RT *>(r);
     OT *op_      = static_cast<OT *>(o);
-    uint64_t nv  = 0;
-    if (vec_aligned<LT>(l) && vec_aligned<RT>(r) && vec_aligned<OT>(o)) {
-        nv = n / kVec;
-        CT_TRY(launch_map(nv, BinaryGenericVec<LT, RT, OT>{lp, rp, op_, op, flags}, "binary"));
-    }
-    uint64_t done = nv * kVec;
-    return launch_map(
-        n - done, BinaryGenericScalar<LT, RT, OT>{lp, rp, op_, op, flags, done}, "binary(tail)");
+    const uint64_t nv   = vec_aligned<LT>(l) && vec_aligned<RT>(r) && vec_aligned<OT>(o) ? n / kVec : 0;
+    const uint64_t done = nv * kVec;
+    return launch_map_tail(
+        nv, BinaryGenericVec<LT, RT, OT>{lp, rp, op_, op, flags}, n - done,
+        BinaryGenericScalar<LT, RT, OT>{lp, rp, op_, op, flags, done}, "binary");
 }
 
 template <int OP>
 ct_status binary_f32(const float *l, const float *r, uint64_t n, float *o, uint32_t *flags) {
-    uint64_t nv = 0;
-    if (aligned16(l) && aligned16(r) && aligned16(o)) {
-        nv = n / kVec;
-        CT_TRY(launch_map(nv, BinaryF32Vec<OP>{l, r, o, flags}, "binary_f32"));
-    }
-    uint64_t done = nv * kVec;
-    return launch_map(
-        n - done, BinaryGenericScalar<float, float, float>{l, r, o, OP, flags, done},
-        "binary_f32(tail)");
+    const uint64_t nv   = aligned16(l) && aligned16(r) && aligned16(o) ? n / kVec : 0;
+    const uint64_t done = nv * kVec;
+    return launch_map_tail(
+        nv, BinaryF32Vec<OP>{l, r, o, flags}, n - done,
+        BinaryGenericScalar<float, float, float>{l, r, o, OP, flags, done}, "binary_f32");
 }
 
 template <typename LT, typename RT>
@@ -313,26 +340,20 @@ template <typename TT, typename OT>
 ct_status scalar_typed(int op, const void *t, double s, int left, uint64_t n, void *o, uint32_t *f) {
     const TT *tp = static_cast<const TT *>(t);
     OT *op_      = static_cast<OT *>(o);
-    uint64_t nv  = 0;
-    if (vec_aligned<TT>(t) && vec_aligned<OT>(o)) {
-        nv = n / kVec;
-        CT_TRY(launch_map(nv, ScalarBinary<TT, OT, true>{tp, op_, s, op, left, f, 0}, "binary_scalar"));
-    }
-    uint64_t done = nv * kVec;
-    return launch_map(
-        n - done, ScalarBinary<TT, OT, false>{tp, op_, s, op, left, f, done}, "binary_scalar(tail)");
+    const uint64_t nv   = vec_aligned<TT>(t) && vec_aligned<OT>(o) ? n / kVec : 0;
+    const uint64_t done = nv * kVec;
+    return launch_map_tail(
+        nv, ScalarBinary<TT, OT, true>{tp, op_, s, op, left, f, 0}, n - done,
+        ScalarBinary<TT, OT, false>{tp, op_, s, op, left, f, done}, "binary_scalar");
 }
 
 template <int OP>
 ct_status scalar_f32(const float *t, float s, int left, uint64_t n, float *o, uint32_t *f) {
-    uint64_t nv = 0;
-    if (aligned16(t) && aligned16(o)) {
-        nv = n / kVec;
-        CT_TRY(launch_map(nv, ScalarBinaryF32<OP, true>{t, o, s, left, f, 0}, "binary_scalar_f32"));
-    }
-    uint64_t done = nv * kVec;
-    return launch_map(
-        n - done, ScalarBinaryF32<OP, false>{t, o, s, left, f, done}, "binary_scalar_f32(tail)");
+    const uint64_t nv   = aligned16(t) && aligned16(o) ? n / kVec : 0;
+    const uint64_t done = nv * kVec;
+    return launch_map_tail(
+        nv, ScalarBinaryF32<OP, true>{t, o, s, left, f, 0}, n - done,
+        ScalarBinaryF32<OP, false>{t, o, s, left, f, done}, "binary_scalar_f32");
 }
 
 template <typename TT>
@@ -400,13 +421,11 @@ template <typename LT, typename RT>
 ct_status compare_typed(int op, const void *l, const void *r, uint64_t n, uint8_t *o) {
     const LT *lp = static_cast<const LT *>(l);
     const RT *rp = static_cast<const RT *>(r);
-    uint64_t nv  = 0;
-    if (vec_aligned<LT>(l) && vec_aligned<RT>(r) && vec_aligned<uint8_t>(o)) {
-        nv = n / kVec;
-        CT_TRY(launch_map(nv, CompareTT<LT, RT, true>{lp, rp, o, op, 0}, "compare"));
-    }
-    uint64_t done = nv * kVec;
-    return launch_map(n - done, CompareTT<LT, RT, false>{lp, rp, o, op, done}, "compare(tail)");
+    const uint64_t nv   = vec_aligned<LT>(l) && vec_aligned<RT>(r) && vec_aligned<uint8_t>(o) ? n / kVec : 0;
+    const uint64_t done = nv * kVec;
+    return launch_map_tail(
+        nv, CompareTT<LT, RT, true>{lp, rp, o, op, 0}, n - done,
+        CompareTT<LT, RT, false>{lp, rp, o, op, done}, "compare");
 }
 
 template <typename LT> ct_status compare_rhs(int op, int rdt, const void *l, const void *r, uint64_t n, uint8_t *o) {
@@ -423,13 +442,11 @@ template <typename LT> ct_status compare_rhs(int op, int rdt, const void *l, con
 template <typename TT>
 ct_status compare_scalar_typed(int op, const void *t, double s, int left, uint64_t n, uint8_t *o) {
     const TT *tp = static_cast<const TT *>(t);
-    uint64_t nv  = 0;
-    if (vec_aligned<TT>(t) && vec_aligned<uint8_t>(o)) {
-        nv = n / kVec;
-        CT_TRY(launch_map(nv, CompareTS<TT, true>{tp, o, s, op, left, 0}, "compare_scalar"));
-    }
-    uint64_t done = nv * kVec;
-    return launch_map(n - done, CompareTS<TT, false>{tp, o, s, op, left, done}, "compare_scalar(tail)");
+    const uint64_t nv   = vec_aligned<TT>(t) && vec_aligned<uint8_t>(o) ? n / kVec : 0;
+    const uint64_t done = nv * kVec;
+    return launch_map_tail(
+        nv, CompareTS<TT, true>{tp, o, s, op, left, 0}, n - done,
+        CompareTS<TT, false>{tp, o, s, op, left, done}, "compare_scalar");
 }
 
 // ---- unary ----------------------------------------------------------------------------
@@ -470,13 +487,11 @@ template <int OP, bool VEC> struct Unary {
 };
 
 template <int OP> ct_status unary(const float *t, uint64_t n, float *o, uint32_t *flags, const char *name) {
-    uint64_t nv = 0;
-    if (aligned16(t) && aligned16(o)) {
-        nv = n / kVec;
-        CT_TRY(launch_map(nv, Unary<OP, true>{t, o, flags, 0}, name));
-    }
-    uint64_t done = nv * kVec;
-    return launch_map(n - done, Unary<OP, false>{t, o, flags, done}, name);
+    const uint64_t nv   = aligned16(t) && aligned16(o) ? n / kVec : 0;
+    const uint64_t done = nv * kVec;
+    return launch_map_tail(
+        nv, Unary<OP, true>{t, o, flags, 0}, n - done,
+        Unary<OP, false>{t, o, flags, done}, name);
 }
 
 // ---- w - g * lr in one pass (the parameter update of the reference's training loops) ------
@@ -575,13 +590,11 @@ template <typename T> struct FillTail {
 
 template <typename T> ct_status fill_typed(T value, uint64_t n, void *out) {
     T *o        = static_cast<T *>(out);
-    uint64_t nv = 0;
-    if (vec_aligned<T>(out)) {
-        nv = n / kVec;
-        CT_TRY(launch_map(nv, FillVec<T>{o, value}, "fill"));
-    }
-    uint64_t done = nv * kVec;
-    return launch_map(n - done, FillTail<T>{o, value, done}, "fill(tail)");
+    const uint64_t nv   = vec_aligned<T>(out) ? n / kVec : 0;
+    const uint64_t done = nv * kVec;
+    return launch_map_tail(
+        nv, FillVec<T>{o, value}, n - done,
+        FillTail<T>{o, value, done}, "fill");
 }
 
 struct Eye {
@@ -816,13 +829,11 @@ ct_status ct_scaled_sub(const float *w, const float *g, double lr, uint64_t n, f
         return CT_OK;
     if (!w || !g || !out)
         return fail(CT_ERR_INVALID, "ct_scaled_sub: null pointer");
-    uint64_t nv = 0;
-    if (aligned16(w) && aligned16(g) && aligned16(out)) {
-        nv = n / kVec;
-        CT_TRY(launch_map(nv, ScaledSub<true>{w, g, out, lr, 0}, "scaled_sub"));
-    }
-    uint64_t done = nv * kVec;
-    return launch_map(n - done, ScaledSub<false>{w, g, out, lr, done}, "scaled_sub");
+    const uint64_t nv   = aligned16(w) && aligned16(g) && aligned16(out) ? n / kVec : 0;
+    const uint64_t done = nv * kVec;
+    return launch_map_tail(
+        nv, ScaledSub<true>{w, g, out, lr, 0}, n - done,
+        ScaledSub<false>{w, g, out, lr, done}, "scaled_sub");
 }
 
 ct_status ct_relu(const float *in, uint64_t n, float *out) {
