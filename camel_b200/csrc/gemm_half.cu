@@ -971,83 +971,115 @@ __global__ void __launch_bounds__(256) half_rows_kernel(
     half_rows<TPR, V>((int64_t)blockIdx.x, in, rows, k, kp, p, vec_ok);
 }
 
-// Largest finite magnitude of each column of in [k][n], by atomic maximum into col_max (zeroed before).
+// Largest finite magnitude of each column of in [k][n], by atomic maximum into col_max (zeroed before).  128 columns to a block,
+// a row of them to a warp.
 __global__ void __launch_bounds__(256) half_col_max_kernel(
-    const float *__restrict__ in, int64_t k, int64_t n, int64_t rows_per_block, uint32_t *__restrict__ col_max) {
-    __shared__ uint32_t max_s[8][32];
+    const float *__restrict__ in, int64_t k, int64_t n, int64_t rows_per_block, int vec_ok, uint32_t *__restrict__ col_max) {
+    __shared__ uint32_t max_s[8][128];
     griddep_launch_dependents();
     griddep_wait();
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t col = (int64_t)blockIdx.x * 32 + tx;
+    const int64_t n0 = (int64_t)blockIdx.x * 128;
     const int64_t r0 = (int64_t)blockIdx.y * rows_per_block, r1 = min(k, r0 + rows_per_block);
-    uint32_t mx = 0;
-    if (col < n)
+    uint32_t mx[4] = {0, 0, 0, 0};
+    if (vec_ok) {
+        if (n0 + tx * 4 < n)
 #pragma unroll 8
+            for (int64_t r = r0 + ty; r < r1; r += 8) {
+                const float4 v = *reinterpret_cast<const float4 *>(in + r * n + n0 + tx * 4);
+                mx[0] = max(mx[0], finite_magnitude(v.x)), mx[1] = max(mx[1], finite_magnitude(v.y));
+                mx[2] = max(mx[2], finite_magnitude(v.z)), mx[3] = max(mx[3], finite_magnitude(v.w));
+            }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            max_s[ty][tx * 4 + q] = mx[q];
+    } else {
+#pragma unroll 4
         for (int64_t r = r0 + ty; r < r1; r += 8)
-            mx = max(mx, finite_magnitude(in[r * n + col]));
-    max_s[ty][tx] = mx;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                mx[q] = max(mx[q], n0 + tx + 32 * q < n ? finite_magnitude(in[r * n + n0 + tx + 32 * q]) : 0u);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            max_s[ty][tx + 32 * q] = mx[q];
+    }
     __syncthreads();
-    if (ty == 0 && col < n) {
+    if (threadIdx.x < 128 && n0 + threadIdx.x < n) {
+        uint32_t all = max_s[0][threadIdx.x];
 #pragma unroll
         for (int w = 1; w < 8; ++w)
-            mx = max(mx, max_s[w][tx]);
-        atomicMax(col_max + col, mx);
+            all = max(all, max_s[w][threadIdx.x]);
+        atomicMax(col_max + n0 + threadIdx.x, all);
     }
 }
 
-// in [k][n] -> transposed float16 planes [n][kp], inverse column scales.  Blocks of 64 k x 32 columns, a warp to a
-// column: the first block of a column writes its scale, any of them its sign (both by OR, the scales start at zero).
+// in [k][n] -> transposed float16 planes [n][kp], inverse column scales.  Blocks of 64 k x 64 columns, eight values of k to a
+// thread and 16-byte stores: 16384 x 16384 with the maxima 813 us, with one half2 to a store and 32 columns to a block
+// 1030.  The first block of a column writes its scale, any of them its sign (both by OR, the scales start at zero).
 __global__ void __launch_bounds__(256) half_cols_kernel(
-    const float *__restrict__ in, int64_t k, int64_t n, int64_t kp, const HalfPlanes p, const uint32_t *__restrict__ col_max) {
-    __shared__ float tile[64][33];
+    const float *__restrict__ in, int64_t k, int64_t n, int64_t kp, const HalfPlanes p, int vec_ok, const uint32_t *__restrict__ col_max) {
+    __shared__ float tile[64][65];
     griddep_launch_dependents();
     griddep_wait();
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t n0 = (int64_t)blockIdx.x * 32, k0 = (int64_t)blockIdx.y * 64;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int64_t kk = k0 + ty + j * 8, nn = n0 + tx;
-        tile[ty + j * 8][tx] = (kk < k && nn < n) ? in[kk * n + nn] : 0.0f;
-    }
+    const int64_t n0 = (int64_t)blockIdx.x * 64, k0 = (int64_t)blockIdx.y * 64;
+    transpose_load(tile, in, k, n, k0, n0, vec_ok);
     __syncthreads();
+    const int kc = (threadIdx.x & 7) * 8;
+    const int64_t kk = k0 + kc;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int64_t nn = n0 + ty + j * 8, kk = k0 + tx * 2;
-        if (nn >= n)
-            break; // the whole warp
+    for (int j = 0; j < 2; ++j) {
+        const int col    = (threadIdx.x >> 3) + 32 * j;
+        const int64_t nn = n0 + col;
+        const bool there = nn < n && kk < kp;
         float scale, inverse;
-        const bool ok  = half_scale(col_max[nn], scale, inverse);
-        const float v0 = tile[tx * 2][ty + j * 8], v1 = tile[tx * 2 + 1][ty + j * 8];
-        uint32_t *word = reinterpret_cast<uint32_t *>(p.scale + nn);
-        if (blockIdx.y == 0 && tx == 0) {
+        const bool ok  = half_scale(nn < n ? col_max[nn] : 0u, scale, inverse);
+        uint32_t *word = reinterpret_cast<uint32_t *>(p.scale + (nn < n ? nn : 0));
+        if (nn < n && kk == 0) {
             atomicOr(word, __float_as_uint(inverse));
             if (!ok)
                 p.exceptions->wide = 1u;
         }
-        const bool special = half_exception(v0, scale) || half_exception(v1, scale) || !isfinite(v0) || !isfinite(v1);
-        if (kk < kp) {
-            __half2 hi, lo;
-            split_half_pair(v0 * scale, v1 * scale, hi, lo);
-            if (special) {
-                split_half(v0, scale, hi.x, lo.x);
-                split_half(v1, scale, hi.y, lo.y);
-            }
-            *reinterpret_cast<__half2 *>(p.hi16 + nn * kp + kk) = hi;
-            *reinterpret_cast<__half2 *>(p.lo16 + nn * kp + kk) = lo;
-            if (p.hi32) {
-                float2 h, l;
-                split_tf32_flat(v0, h.x, l.x);
-                split_tf32_flat(v1, h.y, l.y);
-                *reinterpret_cast<float2 *>(p.hi32 + nn * kp + kk) = h;
-                *reinterpret_cast<float2 *>(p.lo32 + nn * kp + kk) = l;
-            }
+        float v[8];
+        bool special = false;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            v[u] = tile[kc + u][col];
+            special |= half_exception(v[u], scale) || !isfinite(v[u]);
         }
-        if (__any_sync(0xffffffffu, special)) {
-            bool found = half_record(p.exceptions, v0, scale, p.operand, nn, kk);
-            found |= half_record(p.exceptions, v1, scale, p.operand, nn, kk + 1);
-            if (found && tx == 0)
-                atomicOr(word, 0x80000000u);
+        special = special && there;
+        if (there) {
+            __half2 hi[4], lo[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                split_half_pair(v[2 * u] * scale, v[2 * u + 1] * scale, hi[u], lo[u]);
+            if (special)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    split_half(v[2 * u], scale, hi[u].x, lo[u].x);
+                    split_half(v[2 * u + 1], scale, hi[u].y, lo[u].y);
+                }
+            *reinterpret_cast<uint4 *>(p.hi16 + nn * kp + kk) = *reinterpret_cast<uint4 *>(hi);
+            *reinterpret_cast<uint4 *>(p.lo16 + nn * kp + kk) = *reinterpret_cast<uint4 *>(lo);
+            if (p.hi32)
+#pragma unroll
+                for (int u = 0; u < 8; u += 4) {
+                    float4 h, l;
+                    split_tf32_flat(v[u], h.x, l.x);
+                    split_tf32_flat(v[u + 1], h.y, l.y);
+                    split_tf32_flat(v[u + 2], h.z, l.z);
+                    split_tf32_flat(v[u + 3], h.w, l.w);
+                    *reinterpret_cast<float4 *>(p.hi32 + nn * kp + kk + u) = h;
+                    *reinterpret_cast<float4 *>(p.lo32 + nn * kp + kk + u) = l;
+                }
         }
+        if (__any_sync(0xffffffffu, special))
+#pragma unroll 1
+            for (int u = 0; u < 8; ++u) {
+                const float value = there ? tile[kc + u][col] : 0.0f;
+                half_record(p.exceptions, value, scale, p.operand, nn, kk + u);
+                if (half_exception(value, scale))
+                    atomicOr(word, 0x80000000u);
+            }
     }
 }
 
@@ -1064,9 +1096,16 @@ __device__ __forceinline__ void half_cols_short(
     const int64_t n0 = (int64_t)block * kShortCols;
     const bool col_ok = n0 + tx < n;
     const float *src  = in + n0 + tx;
-#pragma unroll 8
-    for (int kk = ty; kk < (int)kp; kk += 32)
-        tile[kk * kShortPad + tx] = (col_ok && kk < k) ? src[(int64_t)kk * n] : 0.0f;
+    for (int kk0 = ty; kk0 < (int)kp; kk0 += 512) { // sixteen loads in flight
+        float v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            v[u] = (col_ok && kk0 + 32 * u < k) ? src[(int64_t)(kk0 + 32 * u) * n] : 0.0f;
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            if (kk0 + 32 * u < (int)kp)
+                tile[(kk0 + 32 * u) * kShortPad + tx] = v[u];
+    }
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint2 range    = make_uint2(0u, kNoneSmallest);
@@ -1313,7 +1352,8 @@ ct_status half_split_cols(
     DeviceState *st, const float *in, int64_t k, int64_t kp, const HalfOperand &o, bool both_forms, uint32_t *col_max) {
     const int64_t n    = o.rows;
     const HalfPlanes p = planes_of(o, both_forms);
-    const unsigned strips = (unsigned)((n + 31) / 32);
+    const unsigned strips = (unsigned)((n + 127) / 128);
+    const int vec         = (n & 3) == 0 && (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
     if (half_cols_is_short(kp)) {
         CT_CUDA(launch_dependent(half_cols_short_kernel, dim3((unsigned)((n + kShortCols - 1) / kShortCols)), dim3(256),
                                  (size_t)kp * kShortPad * 4, stream(), in, k, n, kp, p));
@@ -1326,9 +1366,9 @@ ct_status half_split_cols(
     const int64_t slabs = (kp + 63) / 64;
     if (slabs > 65535 || slices > 65535)
         return fail(CT_ERR_TOO_LARGE, "gemm: k too large for the operand pre-pass");
-    CT_CUDA(launch_dependent(half_col_max_kernel, dim3(strips, (unsigned)slices), dim3(256), 0, stream(), in, k, n, rows, col_max));
+    CT_CUDA(launch_dependent(half_col_max_kernel, dim3(strips, (unsigned)slices), dim3(256), 0, stream(), in, k, n, rows, vec, col_max));
     CT_LAUNCH_CHECK("half_col_max");
-    CT_CUDA(launch_dependent(half_cols_kernel, dim3(strips, (unsigned)slabs), dim3(256), 0, stream(), in, k, n, kp, p,
+    CT_CUDA(launch_dependent(half_cols_kernel, dim3((unsigned)((n + 63) / 64), (unsigned)slabs), dim3(256), 0, stream(), in, k, n, kp, p, vec,
                              static_cast<const uint32_t *>(col_max)));
     CT_LAUNCH_CHECK("half_cols");
     return CT_OK;

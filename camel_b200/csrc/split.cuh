@@ -43,4 +43,32 @@ __device__ __forceinline__ void split_tf32_flat(float v, float &hi, float &lo) {
     lo = __uint_as_float(v_special ? 0u : l);
 }
 
+// A 64 x 64 block of in [k][n] at (k0, n0) into shared memory, by 256 threads, zeros outside: rows of 256 contiguous bytes,
+// four 16-byte loads to a thread in flight where the rows are aligned (vec_ok).
+__device__ __forceinline__ void transpose_load(
+    float (&tile)[64][65], const float *__restrict__ in, int64_t k, int64_t n, int64_t k0, int64_t n0, int vec_ok) {
+    if (vec_ok) {
+        const int c = (threadIdx.x & 15) * 4, r = threadIdx.x >> 4;
+        float4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            v[j] = k0 + r + 16 * j < k && n0 + c < n ? __ldcs(reinterpret_cast<const float4 *>(in + (k0 + r + 16 * j) * n + n0 + c))
+                                                     : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float *dst = &tile[r + 16 * j][c];
+            dst[0] = v[j].x, dst[1] = v[j].y, dst[2] = v[j].z, dst[3] = v[j].w;
+        }
+    } else {
+        const int c = threadIdx.x & 63, r = threadIdx.x >> 6;
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            v[j] = k0 + r + 4 * j < k && n0 + c < n ? __ldcs(in + (k0 + r + 4 * j) * n + n0 + c) : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            tile[r + 4 * j][c] = v[j];
+    }
+}
+
 } // namespace ct
