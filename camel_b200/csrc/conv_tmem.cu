@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
 // image.  The converting warps also leave the range of every tile in the call's own scratch; conv_tmem_filters_kernel,
 // launched behind this one, computes the images that float16 pairs cannot hold.  A tile that shows that by itself is
 // not converted, multiplied or stored here.
-constexpr int kCP_CvtWarps  = 8;
+constexpr int kCP_CvtWarps  = 10; // a thread to a position of 28 x 28 images: 30 x 10
 constexpr int kCP_EpiWarps  = 8;
 constexpr int kCP_Threads   = 64 + 32 * (kCP_CvtWarps + kCP_EpiWarps);
 constexpr int kCP_RowB      = 64; // a position's 32 channels
@@ -895,26 +895,43 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
             const int npos    = p.box_rows * p.pw;
             const int cstride = p.box_rows * p.box_w; // floats between two channels of one position
             const float *raw  = reinterpret_cast<const float *>(smem_ptr + (raw_base - smem_base));
+            const bool one    = npos <= 32 * kCP_CvtWarps;
+            const int first_raw = ct / p.pw * p.box_w + ct % p.pw + p.off_x;
             int i = 0;
             for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
                 const int s = i % p.stages;
                 bool got = mbar_wait_patient(smem_u32(&bar_raw_full), (uint32_t)i & 1u, abort_flag);
                 if (!__all_sync(0xffffffffu, got))
                     break;
-                // the tile's range (the whole box, alignment columns included: they are pixels or zero)
-                uint2 range       = make_uint2(0u, kNoneSmallest);
-                const float4 *r4  = reinterpret_cast<const float4 *>(raw);
+                // The tile's range.  Where every thread has at most one position its channels stay in registers between the range
+                // and the split, and the box is free for the next tile's before this one's planes are.
+                uint2 range = make_uint2(0u, kNoneSmallest);
+                float v[32];
+                if (one) {
+                    const float *src = raw + (ct < npos ? first_raw : 0);
+#pragma unroll
+                    for (int t = 0; t < 32; ++t)
+                        v[t] = ct < npos ? src[t * cstride] : 0.0f;
+#pragma unroll
+                    for (int t = 0; t < 32; ++t)
+                        range_take(range, v[t]);
+                    __syncwarp();
+                    if (lane == 0)
+                        mbar_arrive(smem_u32(&bar_raw_empty));
+                } else { // the whole box, alignment columns included: they are pixels or zero
+                    const float4 *r4 = reinterpret_cast<const float4 *>(raw);
 #pragma unroll 4
-                for (int e = ct; e < p.raw_bytes / 16; e += 32 * kCP_CvtWarps) {
-                    const float4 q = r4[e];
-                    range_take(range, q.x), range_take(range, q.y), range_take(range, q.z), range_take(range, q.w);
+                    for (int e = ct; e < p.raw_bytes / 16; e += 32 * kCP_CvtWarps) {
+                        const float4 q = r4[e];
+                        range_take(range, q.x), range_take(range, q.y), range_take(range, q.z), range_take(range, q.w);
+                    }
                 }
                 range = range_warp(range);
                 if (lane == 0) {
                     cvt_range[i & 1][warp - 2] = range;
                     mbar_arrive(smem_u32(&bar_cvt));
                 }
-                got = mbar_wait(smem_u32(&bar_cvt), (uint32_t)i & 1u, abort_flag) && // all eight ranges
+                got = mbar_wait(smem_u32(&bar_cvt), (uint32_t)i & 1u, abort_flag) && // all ranges
                       mbar_wait_patient(smem_u32(&bar_empty[s]), ((uint32_t)(i / p.stages) & 1u) ^ 1u, abort_flag) &&
                       mbar_wait_patient(smem_u32(&bar_scale_empty[s]), ((uint32_t)(i / p.stages) & 1u) ^ 1u, abort_flag);
                 if (!__all_sync(0xffffffffu, got))
@@ -929,29 +946,34 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                     p.tile_range[tile] = range;
                 }
                 uint8_t *planes = smem_ptr + p.filter_bytes + (uint32_t)s * stage_bytes;
-                // a thread takes a position (y, x): its 32 channels become row (y >> 1) * pw + x of region y & 1 in both
-                // planes, 16-byte chunk j at j ^ ((row >> 1) & 3), the 64-byte swizzle
-                for (int pos = fits ? ct : npos; pos < npos; pos += 32 * kCP_CvtWarps) {
+                // a position's (y, x) 32 channels become row (y >> 1) * pw + x of region y & 1 in both planes, 16-byte chunk j
+                // at j ^ ((row >> 1) & 3), the 64-byte swizzle
+                auto put = [&](int pos) {
                     const int y = pos / p.pw, x = pos - y * p.pw, row = (y >> 1) * p.pw + x;
-                    const float *src = raw + y * p.box_w + x + p.off_x;
                     uint8_t *dst     = planes + (uint32_t)(y & 1) * region + (uint32_t)row * kCP_RowB;
                     const uint32_t sw = ((uint32_t)row >> 1) & 3u;
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        float v[16];
+                    for (int j = 0; j < 4; ++j) {
+                        __half2 hi[4], lo[4];
 #pragma unroll
-                        for (int t = 0; t < 16; ++t)
-                            v[t] = src[(16 * half + t) * cstride];
+                        for (int t = 0; t < 4; ++t)
+                            split_half_pair(__fmul_rn(v[8 * j + 2 * t], scale), __fmul_rn(v[8 * j + 2 * t + 1], scale), hi[t], lo[t]);
+                        const uint32_t at = ((uint32_t)j ^ sw) << 4;
+                        *reinterpret_cast<uint4 *>(dst + at)              = *reinterpret_cast<uint4 *>(hi);
+                        *reinterpret_cast<uint4 *>(dst + 2 * region + at) = *reinterpret_cast<uint4 *>(lo);
+                    }
+                };
+                if (one) {
+                    if (fits && ct < npos)
+                        put(ct);
+                } else {
+                    for (int pos = fits ? ct : npos; pos < npos; pos += 32 * kCP_CvtWarps) {
+                        const int y = pos / p.pw;
+                        const float *src = raw + y * p.box_w + pos - y * p.pw + p.off_x;
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) {
-                            __half2 hi[4], lo[4];
-#pragma unroll
-                            for (int t = 0; t < 4; ++t)
-                                split_half_pair(__fmul_rn(v[8 * j + 2 * t], scale), __fmul_rn(v[8 * j + 2 * t + 1], scale), hi[t], lo[t]);
-                            const uint32_t at = ((uint32_t)(2 * half + j) ^ sw) << 4;
-                            *reinterpret_cast<uint4 *>(dst + at)              = *reinterpret_cast<uint4 *>(hi);
-                            *reinterpret_cast<uint4 *>(dst + 2 * region + at) = *reinterpret_cast<uint4 *>(lo);
-                        }
+                        for (int t = 0; t < 32; ++t)
+                            v[t] = src[t * cstride];
+                        put(pos);
                     }
                 }
                 // written through the generic proxy, read by the tensor core's asynchronous proxy
@@ -959,7 +981,8 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                 __syncwarp();
                 if (lane == 0) {
                     mbar_arrive(smem_u32(&bar_full[s]));
-                    mbar_arrive(smem_u32(&bar_raw_empty));
+                    if (!one)
+                        mbar_arrive(smem_u32(&bar_raw_empty));
                 }
             }
         }
@@ -971,6 +994,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
         const int groups = p.kop >> 4;
         const int64_t plane = p.pool ? (int64_t)(p.ho >> 1) * (p.wo >> 1) : (int64_t)p.ho * p.wo;
         const bool inside = j < p.jp && x < p.wo && !(p.pool && (x & 1));
+        const bool has_bias = p.bias != nullptr, relu = p.act == CT_ACT_RELU;
         int i = 0;
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
             const int img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
@@ -983,49 +1007,58 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
             const float is = RAW ? *const_cast<volatile float *>(&tile_scale[s]) : p.image_scale[img];
             tc_fence_after_sync();
             const int y = (ty * p.jp + j) * 2; // the even row; the odd one may be past the image
-            const bool live_even = inside && y < p.ho, live_odd = inside && y + 1 < p.ho;
+            const bool live_even = inside && y < p.ho, live_low = inside && !p.pool && y + 1 < p.ho; // pooled rows are even and odd
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(set * 256);
             float *dst = p.out + ((int64_t)img * p.ko + half * 16) * plane + (p.pool ? (int64_t)(y >> 1) * (p.wo >> 1) + (x >> 1) : (int64_t)y * p.wo + x);
+            // Values of sixteen channels, then their neighbours, then the stores, without a branch among them: channel after
+            // channel, with the activation behind a branch, a group took 4300 clocks.
             for (int g = half; g < groups && !(RAW && is == 0.0f); g += 2, dst += 32 * plane) {
-                uint32_t a[16], b[16], c[16], d[16];
-                tmem_ld_32x16(taddr + (uint32_t)(16 * g), a);
-                tmem_ld_32x16(taddr + (uint32_t)(p.kop + 16 * g), b);
-                tmem_ld_32x16(taddr + (uint32_t)(128 + 16 * g), c);
-                tmem_ld_32x16(taddr + (uint32_t)(128 + p.kop + 16 * g), d);
-                tmem_ld_wait();
+                float even[16], odd[16];
+#pragma unroll
+                for (int h = 0; h < 16; h += 8) {
+                    uint32_t a[8], b[8], c[8], d[8];
+                    tmem_ld_32x8(taddr + (uint32_t)(16 * g + h), a);
+                    tmem_ld_32x8(taddr + (uint32_t)(p.kop + 16 * g + h), b);
+                    tmem_ld_32x8(taddr + (uint32_t)(128 + 16 * g + h), c);
+                    tmem_ld_32x8(taddr + (uint32_t)(128 + p.kop + 16 * g + h), d);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int u = 0; u < 8; u += 4) {
+                        const float4 f4 = *reinterpret_cast<const float4 *>(filter_inv + 16 * g + h + u);
+                        const float4 b4 = *reinterpret_cast<const float4 *>(bias_s + 16 * g + h + u);
+                        const float fs[4] = {f4.x, f4.y, f4.z, f4.w}, bs[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            auto value = [&](uint32_t main, uint32_t cross) {
+                                float v       = __fadd_rn(__uint_as_float(main), __fmul_rn(__uint_as_float(cross), kHalfLoInv));
+                                v             = __fmul_rn(__fmul_rn(v, fs[q]), is);
+                                const float w = __fadd_rn(v, bs[q]);
+                                v             = has_bias ? w : v;
+                                return __fmul_rn(v, !relu || v > 0.0f ? 1.0f : 0.0f);
+                            };
+                            even[h + u + q] = value(a[u + q], b[u + q]), odd[h + u + q] = value(c[u + q], d[u + q]);
+                        }
+                    }
+                }
+                const int filters = p.ko - 16 * g < 16 ? p.ko - 16 * g : 16;
+                if (p.pool) {
+#pragma unroll
+                    for (int u = 0; u < 16; ++u) {
+                        // window order and strict '>' as in maxpool2d
+                        const float even1 = __shfl_down_sync(0xffffffffu, even[u], 1), odd1 = __shfl_down_sync(0xffffffffu, odd[u], 1);
+                        even[u] = even1 > even[u] ? even1 : even[u];
+                        odd[u]  = odd1 > odd[u] ? odd1 : odd[u];
+                        even[u] = odd[u] > even[u] ? odd[u] : even[u];
+                    }
+                }
                 float *at = dst;
 #pragma unroll
-                for (int u = 0; u < 16; u += 4) {
-                    const float4 f4 = *reinterpret_cast<const float4 *>(filter_inv + 16 * g + u);
-                    const float4 b4 = *reinterpret_cast<const float4 *>(bias_s + 16 * g + u);
-                    const float fs[4] = {f4.x, f4.y, f4.z, f4.w}, bs[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-                    for (int q = 0; q < 4; ++q, at += plane) {
-                        auto value = [&](uint32_t main, uint32_t cross) {
-                            float v = __fadd_rn(__uint_as_float(main), __fmul_rn(__uint_as_float(cross), kHalfLoInv));
-                            v       = __fmul_rn(__fmul_rn(v, fs[q]), is);
-                            if (p.bias)
-                                v = __fadd_rn(v, bs[q]);
-                            if (p.act == CT_ACT_RELU)
-                                v = __fmul_rn(v, v > 0.0f ? 1.0f : 0.0f);
-                            return v;
-                        };
-                        const float even = value(a[u + q], b[u + q]), odd = value(c[u + q], d[u + q]);
-                        const bool filter = 16 * g + u + q < p.ko;
-                        if (p.pool == 0) {
-                            if (live_even && filter)
-                                at[0] = even;
-                            if (live_odd && filter)
-                                at[p.wo] = odd;
-                        } else {
-                            // window order and strict '>' as in maxpool2d
-                            const float even1 = __shfl_down_sync(0xffffffffu, even, 1), odd1 = __shfl_down_sync(0xffffffffu, odd, 1);
-                            float best = even1 > even ? even1 : even;
-                            const float low = odd1 > odd ? odd1 : odd;
-                            best = low > best ? low : best;
-                            if (live_odd && filter)
-                                at[0] = best;
-                        }
+                for (int u = 0; u < 16; ++u, at += plane) {
+                    if (u < filters) {
+                        if (live_even)
+                            at[0] = even[u];
+                        if (live_low)
+                            at[p.wo] = odd[u];
                     }
                 }
             }
