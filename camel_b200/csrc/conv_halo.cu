@@ -356,6 +356,7 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
             const int y = col / p.pw, x = col - y * p.pw;
             off[j] = (col < npos && x < p.wo) ? y * p.wo + x : -1;
         }
+        const bool relu = p.act == CT_ACT_RELU;
         int mains = 0, crosses = 0;
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
             int tm, ty, img;
@@ -364,7 +365,10 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
             const float inv    = p.image_scale[img];
             const bool wide    = inv == 0.0f;
             const float rs     = (!wide && row0 + lane < p.ko) ? p.filter_scale[row0 + lane] : 1.0f;
-            const float is     = wide ? 1.0f : inv;
+            // powers of two; a missing bias is -0, which no sum notices
+            const float scale  = wide ? 1.0f : __fmul_rn(rs, inv);
+            const int ch       = row0 + lane;
+            const float bias   = !p.bias || ch >= p.ko ? -0.0f : (ch < kH_BiasSlots ? bias_s[ch] : p.bias[ch]);
             const long long e0 = CH_CLOCK();
             float acc[128];
             const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 128);
@@ -426,45 +430,47 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
             // positions of rows past the image's last row (a partial last tile) are dropped:
             // position col lies in row col / pw, so the valid ones are col < rows_left * pw
             const int col_limit = (p.ho - y0 < p.th ? p.ho - y0 : p.th) * p.pw;
+            // Scales, bias and activation where a lane has a channel, with its constants in registers; what remains for the
+            // stores is a read, an address and the store.  (With them behind the exchange, a value took 35 instructions and
+            // a tile the epilogue 18,000 clocks, four thousand more than its MMAs.)
             const int64_t plane = (int64_t)p.ho * p.wo;
-            float *out_img = p.out + ((int64_t)img * p.ko) * p.ho * p.wo + (int64_t)y0 * p.wo;
+            float *out_img = p.out + ((int64_t)img * p.ko + row0) * plane + (int64_t)y0 * p.wo;
+            const int rows = p.ko - row0 < 32 ? p.ko - row0 : 32;
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-                if (half * 128 + g * 32 >= npos)
+                if (half * 128 + g * 32 >= npos || rows <= 0)
                     break;
                 float4 *mine = reinterpret_cast<float4 *>(stg + lane * kH_EpiRowBytes);
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    mine[j] = make_float4(__fmul_rn(acc[g * 32 + 4 * j], rs), __fmul_rn(acc[g * 32 + 4 * j + 1], rs),
-                                          __fmul_rn(acc[g * 32 + 4 * j + 2], rs), __fmul_rn(acc[g * 32 + 4 * j + 3], rs));
+                for (int j = 0; j < 8; ++j) {
+                    float y[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        y[q] = __fadd_rn(__fmul_rn(acc[g * 32 + 4 * j + q], scale), bias);
+                        y[q] = !relu || y[q] > 0.0f ? y[q] : __fmul_rn(y[q], 0.0f);
+                    }
+                    mine[j] = make_float4(y[0], y[1], y[2], y[3]);
+                }
                 __syncwarp();
                 // a column per lane, so that a store covers consecutive pixels of a channel (four columns per lane wrote every
-                // sector four times: 256 x 64 x 56 x 56 -> 128 530 us, 491 so); the reads of eight channels before their stores
-                const bool stored = off[g] >= 0 && half * 128 + g * 32 + lane < col_limit;
-                const float *src  = reinterpret_cast<const float *>(stg) + lane;
-                float *dst        = out_img + (int64_t)row0 * plane + (stored ? off[g] : 0);
-#pragma unroll 2
-                for (int r0 = 0; r0 < 32; r0 += 8) {
-                    if (row0 + r0 >= p.ko)
-                        break;
-                    float x[8], b[8];
+                // sector four times: 256 x 64 x 56 x 56 -> 128 530 us, 491 so)
+                const float *src = reinterpret_cast<const float *>(stg) + lane;
+                float *dst       = out_img + (off[g] < 0 ? 0 : off[g]);
+                if (off[g] >= 0 && half * 128 + g * 32 + lane < col_limit) {
+                    int r = 0;
+#pragma unroll 1
+                    for (; r + 8 <= rows; r += 8) {
+                        float x[8];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const int ch = row0 + r0 + u;
-                        x[u]         = src[(r0 + u) * (kH_EpiRowBytes / 4)];
-                        b[u]         = !p.bias || ch >= p.ko ? 0.0f : (ch < kH_BiasSlots ? bias_s[ch] : p.bias[ch]);
-                    }
+                        for (int u = 0; u < 8; ++u)
+                            x[u] = src[(r + u) * (kH_EpiRowBytes / 4)];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        float y = __fmul_rn(x[u], is);
-                        if (p.bias)
-                            y = __fadd_rn(y, b[u]);
-                        if (p.act == CT_ACT_RELU)
-                            y = __fmul_rn(y, y > 0.0f ? 1.0f : 0.0f);
-                        if (stored && row0 + r0 + u < p.ko)
-                            *dst = y;
-                        dst += plane;
+                        for (int u = 0; u < 8; ++u, dst += plane)
+                            *dst = x[u];
                     }
+#pragma unroll 1
+                    for (; r < rows; ++r, dst += plane)
+                        *dst = src[r * (kH_EpiRowBytes / 4)];
                 }
                 __syncwarp(); // the block is rewritten by the next columns
             }

@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
     }
     if (threadIdx.x < 64) {
         filter_inv[threadIdx.x] = 1.0f;
-        bias_s[threadIdx.x]     = p.bias && (int)threadIdx.x < p.ko ? p.bias[threadIdx.x] : 0.0f;
+        bias_s[threadIdx.x]     = p.bias && (int)threadIdx.x < p.ko ? p.bias[threadIdx.x] : -0.0f; // which no sum notices
     }
     __syncthreads();
     if (abort_flag_s)
@@ -994,7 +994,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
         const int groups = p.kop >> 4;
         const int64_t plane = p.pool ? (int64_t)(p.ho >> 1) * (p.wo >> 1) : (int64_t)p.ho * p.wo;
         const bool inside = j < p.jp && x < p.wo && !(p.pool && (x & 1));
-        const bool has_bias = p.bias != nullptr, relu = p.act == CT_ACT_RELU;
+        const bool relu = p.act == CT_ACT_RELU;
         int i = 0;
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
             const int img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
@@ -1026,15 +1026,14 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                     for (int u = 0; u < 8; u += 4) {
                         const float4 f4 = *reinterpret_cast<const float4 *>(filter_inv + 16 * g + h + u);
                         const float4 b4 = *reinterpret_cast<const float4 *>(bias_s + 16 * g + h + u);
-                        const float fs[4] = {f4.x, f4.y, f4.z, f4.w}, bs[4] = {b4.x, b4.y, b4.z, b4.w};
+                        const float fs[4] = {__fmul_rn(f4.x, is), __fmul_rn(f4.y, is), __fmul_rn(f4.z, is), __fmul_rn(f4.w, is)};
+                        const float bs[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
-                            auto value = [&](uint32_t main, uint32_t cross) {
-                                float v       = __fadd_rn(__uint_as_float(main), __fmul_rn(__uint_as_float(cross), kHalfLoInv));
-                                v             = __fmul_rn(__fmul_rn(v, fs[q]), is);
-                                const float w = __fadd_rn(v, bs[q]);
-                                v             = has_bias ? w : v;
-                                return __fmul_rn(v, !relu || v > 0.0f ? 1.0f : 0.0f);
+                            auto value = [&](uint32_t main, uint32_t cross) { // the products with powers of two are exact
+                                float v = __fmaf_rn(__uint_as_float(cross), kHalfLoInv, __uint_as_float(main));
+                                v       = __fadd_rn(__fmul_rn(v, fs[q]), bs[q]);
+                                return !relu || v > 0.0f ? v : __fmul_rn(v, 0.0f);
                             };
                             even[h + u + q] = value(a[u + q], b[u + q]), odd[h + u + q] = value(c[u + q], d[u + q]);
                         }

@@ -174,13 +174,6 @@ __device__ __forceinline__ void tma_load_5d(
         : "memory");
 }
 
-// Contiguous bytes global -> shared memory of this CTA: addresses and size in whole 16-byte units.
-__device__ __forceinline__ void bulk_load(uint32_t dst_smem, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_smem), "l"(src),
-                 "r"(bytes), "r"(bar)
-                 : "memory");
-}
-
 // ---- tensor memory ----------------------------------------------------------------------
 
 // Whole-warp instructions (.sync.aligned): call from all 32 lanes of one warp.
