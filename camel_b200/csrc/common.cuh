@@ -194,6 +194,10 @@ constexpr uint32_t kPackedMagic = 0x43545057u; // "CTPW"
 ct_status gemm_f32_tc(
     DeviceState *st, const float *a, const float *b, const float *bias, int64_t m, int64_t k,
     int64_t n, int act, float *out, const PackedWeights *packed = nullptr, bool a_is_km = false);
+// Products of a few tiles in one launch (gemm_direct.cu).
+bool gemm_direct_applicable(const DeviceState *st, int64_t m, int64_t k, int64_t n);
+ct_status gemm_direct(
+    DeviceState *st, const float *a, const float *b, const float *bias, int64_t m, int64_t k, int64_t n, int act, float *out);
 // One operand of gemm_half (gemm_half.cu): K-major planes [rows][kp] of float16 pairs with an inverse scale
 // per row, and of tf32 terms, which are read instead where the exceptions say so (or the caller forces it).
 struct HalfOperand {

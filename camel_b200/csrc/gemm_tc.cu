@@ -1773,6 +1773,8 @@ ct_status gemm_f32_tc(
                 CT_ERR_INVALID,
                 "dense: the packed weights were built from another matrix, shape, precision or device");
     }
+    if (mode == MODE_3X && !a_is_km && gemm_direct_applicable(st, m, k, n))
+        return gemm_direct(st, a, b, bias, m, k, n, act, out); // one launch; packed planes would save it nothing
     // One tile of rows, or at most nine tiles, and a long k: the product is a fraction of the operands' pre-pass, and what
     // the tf32 planes need - one pass over B and two launches less - outweighs it (70 x 4000 x 70 22.6 against 26.8 us,
     // 128 x 8000 x 128 26.5 against 32.6, 129 x 8000 x 129 30.8 against 35.7, 100 x 16000 x 9000 579 against 603; but

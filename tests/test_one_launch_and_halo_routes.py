@@ -1,0 +1,112 @@
+"""GPU: convolution layers at the edges of the halo and the paired-row kernels (strides, chunks of k, few filters, rows of
+positions that fill an accumulator), small products computed in one launch, right operands in 64 x 64 blocks and the elements
+behind the last vector of an elementwise operator.
+
+Bounds.  Products and layers: 6.3e-6 of the sum of magnitudes (a value is carried to 2^-23 of itself, a product of two so
+carried to 2^-21, at most 96 truncating additions of 2^-24 each into an accumulator).  bfloat16: 2^-8 per operand, 2^-7 of the
+sum of magnitudes.  Elementwise float32 operators: exact.
+"""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+BOUND = 6.3e-6
+
+
+@pytest.fixture(scope="module")
+def T():
+    from camel_b200 import tensor
+
+    return tensor
+
+
+@pytest.fixture(scope="module")
+def port():
+    oracle.build(ref=False)
+    return oracle.port()
+
+
+# n, c, h, w, ko, kh, kw, stride, pad.  Halo kernel: odd extents at strides 2 and 3 (sub-images of unequal size); taps that
+# leave sub-images unread; half of a channel block, and one channel more; k of two and three drains (c = 97, 193 with
+# nine taps; 33 with twenty-five); 17 and 129 filters; a tile of one row; partial last tiles.  Paired rows: an odd number of
+# rows, a row of 128 positions, 16 and 64 filters, 8 channels, an even filter, rows that no tensor map covers.
+LAYERS = [(2, 48, 57, 57, 96, 3, 3, 2, 1), (1, 33, 20, 23, 70, 3, 3, 3, 1), (2, 40, 30, 33, 64, 1, 1, 2, 0), (1, 16, 41, 40, 65, 5, 5, 2, 2),
+          (1, 97, 17, 30, 17, 3, 3, 1, 1), (1, 193, 15, 30, 129, 3, 3, 1, 0), (1, 33, 40, 61, 40, 5, 5, 1, 2), (1, 17, 20, 130, 80, 3, 3, 1, 1),
+          (2, 9, 33, 64, 80, 3, 3, 1, 1), (2, 32, 28, 28, 64, 3, 3, 1, 1), (1, 8, 27, 33, 16, 3, 3, 1, 1), (1, 20, 16, 126, 33, 3, 3, 1, 1),
+          (1, 31, 30, 29, 48, 2, 2, 1, 0), (1, 17, 12, 60, 17, 1, 5, 1, 0)]
+
+
+@pytest.mark.parametrize("layer", LAYERS)
+@pytest.mark.parametrize("kind", ["normal", "one image wide"])
+def test_layers_at_the_edges_of_their_tiles(T, port, layer, kind):
+    n, c, h, w, ko, kh, kw, stride, pad = layer
+    rng = np.random.default_rng(sum(layer))
+    x = rng.standard_normal((n, c, h, w)).astype(np.float32)
+    if kind != "normal":  # the last image spans more powers of two than float16 pairs hold
+        x[-1, 0, h // 2, w // 2] = 1e-20
+    f = rng.standard_normal((ko, c, kh, kw)).astype(np.float32)
+    b = rng.standard_normal(ko).astype(np.float32)
+    got = T.conv2d(T.from_numpy(x), T.from_numpy(f), T.from_numpy(b), stride, pad, "relu")
+    T.check_async()
+    want = port.conv2d(x, f, b, stride, pad, 1)
+    size = port.conv2d(np.abs(x), np.abs(f), np.abs(b), stride, pad, 0)
+    assert np.all(np.abs(got.numpy() - want) <= BOUND * size)
+    ho, wo = want.shape[2:]
+    if stride == 1 and ho % 2 == 0 and wo % 2 == 0:  # the fused pool has the bytes of the two steps
+        pooled = T.conv2d(T.from_numpy(x), T.from_numpy(f), T.from_numpy(b), stride, pad, "relu", pool=2)
+        assert pooled.numpy().tobytes() == T.maxpool2d(got, 2).numpy().tobytes()
+
+
+# rows and columns that fill no tile, k at the edges of a slice and of its sixteen-value steps, an empty last slice
+# (k = 770: eight slices of 112, the last one with none), rows and columns that are not 16-byte aligned
+@pytest.mark.parametrize("m,k,n", [(1, 193, 33), (64, 784, 1024), (129, 257, 127), (128, 512, 512), (100, 770, 130), (65, 1023, 70), (30, 1024, 1800)])
+@pytest.mark.parametrize("kind", ["plain", "small values", "ninety powers of two", "infinity"])
+def test_small_products_in_one_launch(T, m, k, n, kind):
+    rng = np.random.default_rng(m + 3 * k + n)
+    a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    b = rng.uniform(-1, 1, (k, n)).astype(np.float32)
+    if kind == "small values":
+        a[m // 2, k // 3], b[k // 2, n // 3] = 1e-20, 1e-25
+    if kind == "ninety powers of two":
+        a *= np.exp2(rng.integers(-45, 45, (m, k))).astype(np.float32)
+    if kind == "infinity":
+        a[m // 2, k - 1], b[0, n // 2] = np.inf, np.nan
+    got = T.matmul(T.from_numpy(a), T.from_numpy(b)).numpy()
+    T.check_async()
+    with np.errstate(invalid="ignore"):
+        want = a.astype(np.float64) @ b.astype(np.float64)
+    finite = np.isfinite(want)
+    assert np.array_equal(np.isfinite(got), finite)
+    size = np.abs(np.where(np.isfinite(a), a, 0)).astype(np.float64) @ np.abs(np.where(np.isfinite(b), b, 0))
+    assert np.all(np.abs(got - want)[finite] <= BOUND * size[finite])
+
+
+@pytest.mark.parametrize("k,n", [(1030, 130), (1100, 257), (2050, 64), (1088, 1)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_right_operands_in_blocks(T, k, n, precision):
+    from camel_b200._lib import lib, check
+
+    m = 2400  # several tiles of rows: no slices
+    rng = np.random.default_rng(k + n)
+    a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    b = rng.uniform(-1, 1, (k, max(n, 33))).astype(np.float32)
+    check(lib.ct_set_precision(precision))
+    try:
+        got = T.matmul(T.from_numpy(a), T.from_numpy(b)).numpy()
+        T.check_async()
+    finally:
+        check(lib.ct_set_precision(0))
+    a64, b64 = a.astype(np.float64), b.astype(np.float64)
+    assert np.all(np.abs(got - a64 @ b64) <= (2.0 ** -7 if precision else BOUND) * (np.abs(a64) @ np.abs(b64)))
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 4095, 4096, 4097, 16387])
+def test_elements_behind_the_last_vector(T, port, n):
+    rng = np.random.default_rng(n)
+    a, b = rng.standard_normal(n).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    ta, tb = T.from_numpy(a), T.from_numpy(b)
+    assert T.add(ta, tb).numpy().tobytes() == port.binary(oracle.ADD, a, b).tobytes()
+    assert T.multiply(ta, tb).numpy().tobytes() == port.binary(oracle.MUL, a, b).tobytes()
