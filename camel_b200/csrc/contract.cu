@@ -307,16 +307,25 @@ __global__ void __launch_bounds__(256) conv2d_c1_3x3_kernel(
     const float *__restrict__ x, const float *__restrict__ wt, const float *__restrict__ bias,
     int64_t n, int64_t h, int64_t w, int ko, int64_t pad, int64_t ho, int64_t wo, int act,
     float *__restrict__ out) {
-    extern __shared__ double w_s[]; // [ko][9]
+    extern __shared__ double w_s[]; // [ko][9], then the bias
     for (int i = threadIdx.x; i < ko * 9; i += 256)
         w_s[i] = (double)wt[i];
+    for (int i = threadIdx.x; bias && i < ko; i += 256)
+        w_s[ko * 9 + i] = (double)bias[i];
     __syncthreads();
     const int64_t quads = wo >> 2; // wo is a multiple of 4
     const int64_t pix   = ho * wo;
     const int64_t total = n * ho * quads;
     const int64_t step  = (int64_t)gridDim.x * 256;
+    const bool small    = total + step <= 0x7fffffff; // 64-bit divisions are a hundred instructions each
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += step) {
-        const int64_t qx = i % quads, oy = (i / quads) % ho, img = i / (quads * ho);
+        int64_t qx, oy, img;
+        if (small) {
+            const uint32_t row = (uint32_t)i / (uint32_t)quads;
+            qx = (uint32_t)i - row * (uint32_t)quads, img = row / (uint32_t)ho, oy = row - (uint32_t)img * (uint32_t)ho;
+        } else {
+            qx = i % quads, oy = (i / quads) % ho, img = i / (quads * ho);
+        }
         const int64_t ox = qx * 4;
         double patch[3][6];
 #pragma unroll
@@ -346,10 +355,7 @@ __global__ void __launch_bounds__(256) conv2d_c1_3x3_kernel(
             float v[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                double a = acc[j];
-                if (bias)
-                    a += (double)bias[o];
-                v[j] = (float)a;
+                v[j] = (float)(bias ? acc[j] + w_s[ko * 9 + o] : acc[j]);
                 if (act == CT_ACT_RELU)
                     v[j] = __fmul_rn(v[j], v[j] > 0.0f ? 1.0f : 0.0f);
             }
@@ -698,7 +704,12 @@ static ct_status conv2d_run(
     if (pool == 0 && c == 1 && kh == 3 && kw == 3 && stride == 1 && (wo & 3) == 0 && (pix & 3) == 0 && ko * 72 <= 48 * 1024 &&
         (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
         ProfScope prof("conv_small_c");
-        conv2d_c1_3x3_kernel<<<capped_blocks(st, n * ho * (wo >> 2), 16), 256, (size_t)ko * 72, stream()>>>(
+        static bool attr_set_dev[16] = {}; // the attribute belongs to a device's context
+        if (!attr_set_dev[st->device & 15]) {
+            CT_CUDA(cudaFuncSetAttribute(conv2d_c1_3x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 56 * 1024));
+            attr_set_dev[st->device & 15] = true;
+        }
+        conv2d_c1_3x3_kernel<<<capped_blocks(st, n * ho * (wo >> 2), 16), 256, (size_t)ko * 80, stream()>>>(
             x, w, bias, n, h, wd, (int)ko, pad, ho, wo, act, out);
         CT_LAUNCH_CHECK("conv2d_c1_3x3");
         return CT_OK;

@@ -1085,6 +1085,45 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
 
 } // namespace
 
+// Shared-memory plan of a launch: tile rows, bytes per plane and per raw box, pipeline stages.
+static bool conv_tmem_plan(
+    ConvTmemParams &p, int64_t h, int64_t wd, int64_t kh, int64_t kw, int64_t pad, int pool, bool raw, int row_bytes = 128) {
+    p.pad = (int)pad, p.kh = (int)kh, p.kw = (int)kw;
+    p.pw  = (int)(wd + 2 * pad);
+    p.wo  = p.pw - (int)kw + 1;
+    p.ho  = (int)(h + 2 * pad - kh + 1);
+    p.th  = kTA_N / p.pw < p.ho ? kTA_N / p.pw : p.ho;
+    if (pool)
+        p.th &= ~1;
+    if (p.th < 1)
+        return false;
+    p.tiles_y  = (p.ho + p.th - 1) / p.th;
+    p.ksteps   = (int)(kh * kw * 4);
+    p.box_rows = p.th + (int)kh - 1;
+    p.box_bytes = p.box_rows * p.pw * row_bytes;
+    // a tap's shifted window of kTA_N rows may run past the box: reserve those rows too
+    int rows_needed = ((int)kh - 1) * p.pw + ((int)kw - 1) + kTA_N;
+    if (rows_needed < p.box_rows * p.pw)
+        rows_needed = p.box_rows * p.pw;
+    p.plane_bytes = (rows_needed * row_bytes + 1023) & ~1023;
+    // raw mode: the box starts at the 16-byte boundary at or left of x = -pad and is a whole number
+    // of 16-byte units wide
+    const int pad_up = ((int)pad + 3) & ~3;
+    p.off_x      = pad_up - (int)pad;
+    p.box_w      = (p.off_x + p.pw + 3) & ~3;
+    p.raw_bytes  = 32 * p.box_rows * p.box_w * 4;
+    p.raw_stride = (p.raw_bytes + 127) & ~127;
+    if (raw && (p.box_w > 256 || p.box_rows > 256))
+        return false;
+    const int budget = 226 * 1024 - 1024 - kTA_StagingBytes - (raw ? kTA_RawStages * p.raw_stride : 0);
+    // (stages, boxes and the staging block also hold the filters for a moment at the start: at least 42 KB to spare over all
+    // shapes that conv_tmem_applicable accepts)
+    p.stages         = budget / (2 * p.plane_bytes);
+    if (p.stages > 4)
+        p.stages = 4;
+    return p.stages >= 2;
+}
+
 static bool conv_pair_plan(
     ConvPairParams &p, int64_t c, int64_t h, int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t pad, bool raw, size_t *smem) {
     p.ko = (int)ko, p.kop = (int)((ko + 15) / 16 * 16), p.c = (int)c;
@@ -1139,47 +1178,9 @@ bool conv_tmem_applicable(int64_t c, int64_t h, int64_t w, int64_t ko, int64_t k
     if (pool_ok)
         *pool_ok = (wo & 1) == 0 && (ho & 1) == 0 && (pw & 1) == 0 && th >= 2; // horizontal neighbours in one warp
     ConvPairParams pairs;
+    ConvTmemParams wide;
     size_t smem;
-    return conv_pair_plan(pairs, c, h, w, ko, kh, kw, pad, false, &smem);
-}
-
-// Shared-memory plan of a launch: tile rows, bytes per plane and per raw box, pipeline stages.
-static bool conv_tmem_plan(
-    ConvTmemParams &p, int64_t h, int64_t wd, int64_t kh, int64_t kw, int64_t pad, int pool, bool raw, int row_bytes = 128) {
-    p.pad = (int)pad, p.kh = (int)kh, p.kw = (int)kw;
-    p.pw  = (int)(wd + 2 * pad);
-    p.wo  = p.pw - (int)kw + 1;
-    p.ho  = (int)(h + 2 * pad - kh + 1);
-    p.th  = kTA_N / p.pw < p.ho ? kTA_N / p.pw : p.ho;
-    if (pool)
-        p.th &= ~1;
-    if (p.th < 1)
-        return false;
-    p.tiles_y  = (p.ho + p.th - 1) / p.th;
-    p.ksteps   = (int)(kh * kw * 4);
-    p.box_rows = p.th + (int)kh - 1;
-    p.box_bytes = p.box_rows * p.pw * row_bytes;
-    // a tap's shifted window of kTA_N rows may run past the box: reserve those rows too
-    int rows_needed = ((int)kh - 1) * p.pw + ((int)kw - 1) + kTA_N;
-    if (rows_needed < p.box_rows * p.pw)
-        rows_needed = p.box_rows * p.pw;
-    p.plane_bytes = (rows_needed * row_bytes + 1023) & ~1023;
-    // raw mode: the box starts at the 16-byte boundary at or left of x = -pad and is a whole number
-    // of 16-byte units wide
-    const int pad_up = ((int)pad + 3) & ~3;
-    p.off_x      = pad_up - (int)pad;
-    p.box_w      = (p.off_x + p.pw + 3) & ~3;
-    p.raw_bytes  = 32 * p.box_rows * p.box_w * 4;
-    p.raw_stride = (p.raw_bytes + 127) & ~127;
-    if (raw && (p.box_w > 256 || p.box_rows > 256))
-        return false;
-    const int budget = 226 * 1024 - 1024 - kTA_StagingBytes - (raw ? kTA_RawStages * p.raw_stride : 0);
-    // (stages, boxes and the staging block also hold the filters for a moment at the start: at least 42 KB to spare over all
-    // shapes that conv_tmem_applicable accepts)
-    p.stages         = budget / (2 * p.plane_bytes);
-    if (p.stages > 4)
-        p.stages = 4;
-    return p.stages >= 2;
+    return conv_pair_plan(pairs, c, h, w, ko, kh, kw, pad, false, &smem) && conv_tmem_plan(wide, h, w, kh, kw, pad, 0, false);
 }
 
 // Whether the kernel can read this input as it is (NCHW float32) instead of pre-split NHWC planes:

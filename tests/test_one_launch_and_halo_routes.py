@@ -84,6 +84,32 @@ def test_small_products_in_one_launch(T, m, k, n, kind):
     assert np.all(np.abs(got - want)[finite] <= BOUND * size[finite])
 
 
+# one tile of columns: chunks of 128 values of k that end ragged, slices of unequal length, rows that are not 16-byte aligned, and
+# operands that are left to the product from planes
+@pytest.mark.parametrize("m,k,n", [(3300, 2100, 100), (4200, 4099, 128), (6500, 2050, 33)])
+@pytest.mark.parametrize("kind", ["plain", "small value in A", "small value in B", "infinity", "ninety powers of two"])
+def test_tall_products_with_one_tile_of_columns(T, m, k, n, kind):
+    rng = np.random.default_rng(m + k + n)
+    a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    b = rng.uniform(-1, 1, (k, n)).astype(np.float32)
+    if kind == "small value in A":
+        a[m // 2, k // 3] = 1e-20
+    if kind == "small value in B":
+        b[k // 2, n // 3] = 1e-20
+    if kind == "infinity":
+        a[m - 1, k - 1] = np.inf
+    if kind == "ninety powers of two":
+        a *= np.exp2(rng.integers(-45, 45, (m, k))).astype(np.float32)
+    for _ in range(2):  # the mark of the first call is gone
+        got = T.matmul(T.from_numpy(a), T.from_numpy(b)).numpy()
+    T.check_async()
+    want   = a.astype(np.float64) @ b.astype(np.float64)
+    finite = np.isfinite(want)
+    assert np.array_equal(np.isfinite(got), finite)
+    size = np.abs(np.where(np.isfinite(a), a, 0)).astype(np.float64) @ np.abs(b).astype(np.float64)
+    assert np.all(np.abs(got - want)[finite] <= BOUND * size[finite])
+
+
 @pytest.mark.parametrize("k,n", [(1030, 130), (1100, 257), (2050, 64), (1088, 1)])
 @pytest.mark.parametrize("precision", [0, 1])
 def test_right_operands_in_blocks(T, k, n, precision):
