@@ -18,7 +18,7 @@ INCLUDE = ROOT.parent / "include"
 OBJ_DIR = ROOT / "build"
 LIB = ROOT / "libcamel_tensor_b200.so"
 
-SOURCES = ["runtime.cu", "elementwise.cu", "reduce.cu", "gemm_simt.cu", "gemm_tc.cu", "gemm_half.cu", "gemm_direct.cu", "contract.cu",
+SOURCES = ["runtime.cu", "elementwise.cu", "reduce.cu", "gemm_simt.cu", "gemm_tc.cu", "gemm_half.cu", "gemm_direct.cu", "gemm_panel.cu", "contract.cu",
            "graph.cu", "peak.cu", "conv_tmem.cu", "conv_halo.cu"]
 
 NVCC_FLAGS = [

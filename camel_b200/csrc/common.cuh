@@ -28,6 +28,7 @@ enum FlagWord : int {
     FLAG_LOG_DOMAIN = 1, // an input of log was <= 0
     FLAG_TIMEOUT    = 2, // a bounded in-kernel wait ran out (value = 1 + the block that gave up)
     FLAG_EXCEPTION_READERS = 4, // CTAs of a product that have read the exceptions of its operands (half_split.cuh)
+    FLAG_PANEL      = 5, // a panel product (gemm_panel.cu) left its operands to the kernels behind it
     FLAG_COUNT      = 8
 };
 
@@ -217,17 +218,23 @@ struct HalfBands {
     uint32_t *done = nullptr;
 };
 // out[z][m][n] = act(A . B[z]^T + bias) over prepared planes, B holding `batch` operands of b.rows / batch rows.
-// Exceptions that are the device state's are cleared by the launch for the next product.
+// Exceptions that are the device state's are cleared by the launch for the next product.  only_if: a device word; zero: the
+// launch returns at once, else it is cleared with them.
 ct_status gemm_half(
     DeviceState *st, const HalfOperand &a, const HalfOperand &b, int64_t kp, const float *bias, int act, float *out,
-    bool force_wide, bool allow_splitk, const HalfBands *bands, int batch = 1, bool bias_per_row = false);
+    bool force_wide, bool allow_splitk, const HalfBands *bands, int batch = 1, bool bias_per_row = false, uint32_t *only_if = nullptr);
+// Tall products of at most 128 columns whose k is sliced (gemm_panel.cu), from A as it is and B's planes; sets FLAG_PANEL
+// where the operands need the product from planes.
+bool gemm_panel_applicable(const DeviceState *st, int64_t m, int64_t k, int64_t n);
+ct_status gemm_panel(
+    DeviceState *st, const float *a, const HalfOperand &b, int64_t kp, const float *bias, int64_t m, int64_t k, int64_t n, int act, float *out);
 int gemm_tile_columns(const DeviceState *st, int64_t m, int64_t n, int64_t batch = 1); // of gemm_half and gemm_planes
 // Pre-passes: rows of a row-major matrix, columns of one (transposed planes); both record exceptions.  `zero`
 // words are cleared on the way (scales and col_max of a following half_split_cols, which needs them at zero).
 // both_forms: the tf32 planes are written as well (no half_wide_planes needed).
 ct_status half_split_rows(
     DeviceState *st, const float *in, int64_t k, int64_t kp, const HalfOperand &o, bool both_forms, uint32_t *zero,
-    int64_t zero_count);
+    int64_t zero_count, const uint32_t *only_if = nullptr);
 bool half_cols_is_short(int64_t kp); // one pass, which needs no col_max
 ct_status half_split_cols(
     DeviceState *st, const float *in, int64_t k, int64_t kp, const HalfOperand &o, bool both_forms, uint32_t *col_max);

@@ -617,17 +617,17 @@ static int pooled_tile_rows(int64_t ho, int64_t wo) {
 
 // Float32 layers that conv_halo takes: those that fit its tiles, but for layers with few channels on both sides, whose filters
 // stay on chip (conv_tmem.cu), and a handful of channels, most of whose block of 32 would be padding.  A 1 x 1 filter
-// has one use for a halo: up to 64 filters the kernels that put pixels on the rows are as fast or faster (88 x 95 x 29 x
-// 32 -> 22 46 us against 50), and a strided one reads a quarter of the planes (11 x 161 x 52 x 54 -> 37 27 against 33).
-// Below some 8,000 outputs per filter a strided layer's three launches cost more than its patches (9 x 16 x 18 x 18 -> 71
-// 17 against 18, 14 x 14 x 38 x 38 -> 22 26 against 31; 60 x 15 x 41 x 41 -> 27 34 both ways, 64 x 34 x 40 x 42 -> 78 45 against 41).
+// has one use for a halo: up to 64 filters or 32 channels the other kernels are as fast or faster (88 x 95 x 29 x 32 -> 22
+// 46 us against 50, 19 x 18 x 60 x 63 -> 115 145 against 149), and a strided one reads a quarter of the planes (11 x 161 x 52 x 54 -> 37 27 against 33).
+// Below some 16,000 outputs per filter a strided layer's three launches cost more than its patches (7 x 17 x 69 x 72 -> 74
+// 24 against 28, 14 x 14 x 38 x 38 -> 22 26 against 31; 60 x 15 x 41 x 41 -> 27 34 both ways, 64 x 34 x 40 x 42 -> 78 45 against 41).
 static bool conv2d_takes_halo(
     int64_t n, int64_t c, int64_t h, int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t stride, int64_t pad) {
     if (c < 8 || n > 65535 || conv_tmem_applicable(c, h, wd, ko, kh, kw, stride, pad))
         return false;
-    if (kh * kw == 1 && (ko <= 64 || stride > 1))
+    if (kh * kw == 1 && (ko <= 64 || c <= 32 || stride > 1))
         return false;
-    if (stride > 1 && n * ((h + 2 * pad - kh) / stride + 1) * ((wd + 2 * pad - kw) / stride + 1) < 8192)
+    if (stride > 1 && n * ((h + 2 * pad - kh) / stride + 1) * ((wd + 2 * pad - kw) / stride + 1) < 16384)
         return false;
     return conv_halo_applicable((c + 31) / 32 * 32, h, wd, ko, kh, kw, stride, pad);
 }

@@ -38,7 +38,7 @@ struct DirectParams {
     const float *a, *b, *bias;
     float *out;
     int64_t m, n, k;
-    int kc, slices, tiles_m; // values of k per slice, a multiple of 16
+    int kc, slices, tiles_m, bn; // values of k per slice, a multiple of 16; columns of a tile, 64 or 128
     int act, vec_a, vec_b, vec_out;
     uint32_t *flags;
 };
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(kGD_Threads, 1) gemm_direct_kernel(const __gri
         tmem_relinquish();
     }
     const int rank = (int)(blockIdx.x % p.slices), tile = (int)(blockIdx.x / p.slices);
-    const int64_t row0 = (int64_t)(tile % p.tiles_m) * 128, col0 = (int64_t)(tile / p.tiles_m) * 128, k0 = (int64_t)rank * p.kc;
+    const int64_t row0 = (int64_t)(tile % p.tiles_m) * 128, col0 = (int64_t)(tile / p.tiles_m) * p.bn, k0 = (int64_t)rank * p.kc;
     const int kn     = (int)(p.k - k0 < 0 ? 0 : (p.k - k0 < p.kc ? p.k - k0 : p.kc)); // the last slices may be empty
     const int ksteps = (kn + 15) >> 4;
     cluster_arrive(); // this CTA runs: the others may write to its shared memory
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(kGD_Threads, 1) gemm_direct_kernel(const __gri
     for (int i = 0; i < 8; ++i) {
         const int kk     = warp * 8 + i;
         const float *src = p.b + (k0 + kk) * p.n + col0 + 4 * lane;
-        const int left   = kk < kn ? (int)(p.n - col0 < 128 ? p.n - col0 : 128) - 4 * lane : 0;
+        const int left   = kk < kn ? (int)(p.n - col0 < p.bn ? p.n - col0 : p.bn) - 4 * lane : 0;
         if (p.vec_b) {
             bv[i] = left > 0 ? *reinterpret_cast<const float4 *>(src) : zero;
         } else {
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kGD_Threads, 1) gemm_direct_kernel(const __gri
 
     // ---- the product: leading accumulator in columns 0 .. 127, cross products behind it ----
     const uint32_t d_main = tmem_base, d_cross = tmem_base + 128u;
-    const uint32_t idesc  = make_idesc(wide ? 1u : 0u, 128, 128) | 1u << 16; // B is MN-major
+    const uint32_t idesc  = make_idesc(wide ? 1u : 0u, 128, (uint32_t)p.bn) | 1u << 16; // B is MN-major
     auto a_desc = [&](int plane, int ks) { return smem_desc_k<128>(smem_base + (uint32_t)(plane * kGD_Plane + (ks >> 2) * kGD_Block)) + 2 * (ks & 3); };
     auto b_desc = [&](int plane, int ks) { return desc_mn(smem_base + (uint32_t)(kGD_B + plane * kGD_Plane + ks * 2048)); };
     bool ok     = !failed;
@@ -245,7 +245,9 @@ __global__ void __launch_bounds__(kGD_Threads, 1) gemm_direct_kernel(const __gri
 
     // ---- its sums, 32 columns of 32 rows to a warp, to the CTAs that add up those rows: rows of 512 bytes, float4 slots
     // XOR-swizzled, slice after slice ----
-    const int rows_each = 128 / p.slices;
+    // Between the CTAs they move at some 11 bytes per clock (64 KB in 3.8 us), so only what the output has is sent: the rows
+    // there are, dealt out evenly, and tiles of 64 columns where the machine holds twice as many.
+    const int valid = (int)(p.m - row0 < 128 ? p.m - row0 : 128), rows_each = (valid + p.slices - 1) / p.slices;
     {
         const int quarter = warp & 3, cg = warp >> 2, row = quarter * 32 + lane;
         uint32_t main[32], cross[32];
@@ -255,7 +257,8 @@ __global__ void __launch_bounds__(kGD_Threads, 1) gemm_direct_kernel(const __gri
         tmem_ld_wait();
         const float weight = wide ? 1.0f : kHalfLoInv, rs = wide ? 1.0f : row_inv[row];
         cluster_wait();
-        const uint32_t part = mapa(smem_base + (uint32_t)(kGD_Sums + (rank * rows_each + row % rows_each) * 512), (uint32_t)(row / rows_each));
+        const bool send     = row < valid && cg * 32 < p.bn;
+        const uint32_t part = mapa(smem_base + (uint32_t)(kGD_Sums + (rank * rows_each + row % rows_each) * 512), (uint32_t)(send ? row / rows_each : 0));
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const float4 c = wide ? make_float4(1.0f, 1.0f, 1.0f, 1.0f) : *reinterpret_cast<const float4 *>(col_inv + cg * 32 + 4 * j);
@@ -263,7 +266,8 @@ __global__ void __launch_bounds__(kGD_Threads, 1) gemm_direct_kernel(const __gri
                 const float v = __fadd_rn(__uint_as_float(main[4 * j + u]), __fmul_rn(__uint_as_float(cross[4 * j + u]), weight));
                 return ksteps > 0 ? __fmul_rn(__fmul_rn(v, rs), s) : 0.0f;
             };
-            st_cluster_f4(part + (uint32_t)(((cg * 8 + j) ^ (row & 7)) << 4), make_float4(value(0, c.x), value(1, c.y), value(2, c.z), value(3, c.w)));
+            if (send)
+                st_cluster_f4(part + (uint32_t)(((cg * 8 + j) ^ (row % rows_each & 7)) << 4), make_float4(value(0, c.x), value(1, c.y), value(2, c.z), value(3, c.w)));
         }
     }
     tc_fence_before_sync();
@@ -282,7 +286,7 @@ __global__ void __launch_bounds__(kGD_Threads, 1) gemm_direct_kernel(const __gri
     if (!failed && !*abort_flag)
         for (int r = warp; r < rows_each; r += kGD_Warps) {
             const int64_t row = row0 + rank * rows_each + r;
-            if (row >= p.m || col >= p.n)
+            if (rank * rows_each + r >= valid || slot * 4 >= p.bn || col >= p.n)
                 break;
             const uint8_t *at = smem + kGD_Sums + r * 512 + ((slot ^ (r & 7)) << 4);
             float4 v          = *reinterpret_cast<const float4 *>(at);
@@ -335,19 +339,23 @@ int direct_clusters(const DeviceState *st, int size) {
 
 // Slices of k, a power of two of at most 128 values each; 0: the product is not for this kernel.  It takes those whose slices
 // run at once, all clusters of them; k of one slice is left to the kernels whose bytes ct_matmul_packed_rows has.
-int direct_slices(const DeviceState *st, int64_t m, int64_t k, int64_t n) {
+int direct_slices(const DeviceState *st, int64_t m, int64_t k, int64_t n, int *bn) {
     if (k <= 192 || k > 8 * kGD_K || m > (1 << 20) || n > (1 << 20))
         return 0;
     int slices = 2;
     while (slices * kGD_K < k)
         slices *= 2;
-    const int64_t tiles = ((m + 127) / 128) * ((n + 127) / 128);
-    return tiles <= direct_clusters(st, slices) ? slices : 0;
+    const int64_t rows = (m + 127) / 128, most = direct_clusters(st, slices);
+    *bn                = n <= 64 || rows * ((n + 63) / 64) <= most ? 64 : 128;
+    return rows * ((n + 127) / 128) <= most ? slices : 0;
 }
 
 } // namespace
 
-bool gemm_direct_applicable(const DeviceState *st, int64_t m, int64_t k, int64_t n) { return direct_slices(st, m, k, n) > 0; }
+bool gemm_direct_applicable(const DeviceState *st, int64_t m, int64_t k, int64_t n) {
+    int bn;
+    return direct_slices(st, m, k, n, &bn) > 0;
+}
 
 ct_status gemm_direct(
     DeviceState *st, const float *a, const float *b, const float *bias, int64_t m, int64_t k, int64_t n, int act, float *out) {
@@ -355,13 +363,13 @@ ct_status gemm_direct(
     DirectParams p{};
     p.a = a, p.b = b, p.bias = bias, p.out = out;
     p.m = m, p.n = n, p.k = k;
-    p.slices  = direct_slices(st, m, k, n);
+    p.slices  = direct_slices(st, m, k, n, &p.bn);
     p.kc      = (int)((k + p.slices - 1) / p.slices + 15) & ~15;
     p.tiles_m = (int)((m + 127) / 128);
     p.act     = act;
     p.vec_a = (k & 3) == 0 && aligned(a), p.vec_b = (n & 3) == 0 && aligned(b), p.vec_out = (n & 3) == 0 && aligned(out);
     p.flags = st->flags_dev;
-    const unsigned grid = (unsigned)(p.tiles_m * ((n + 127) / 128) * p.slices);
+    const unsigned grid = (unsigned)(p.tiles_m * ((n + p.bn - 1) / p.bn) * p.slices);
     ProfScope prof("gemm_tc");
     CT_CUDA(launch_dependent_cluster(gemm_direct_kernel, p.slices, dim3(grid), dim3(kGD_Threads), (size_t)kGD_Smem, stream(), p));
     CT_LAUNCH_CHECK("gemm_direct");

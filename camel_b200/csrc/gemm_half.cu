@@ -82,6 +82,7 @@ struct HalfGemmParams {
     int64_t out_batch_stride;
     uint32_t *flags;
     int force_wide;                         // the tf32 planes hold the operands, whatever the exceptions say
+    uint32_t *only_if;                      // zero there: nothing to do
     HalfExceptions *reset;                  // the library's own list, if one of them is that: the last CTA clears it
     // row bands, see ct_matmul_packed_bands
     int bands;
@@ -352,6 +353,23 @@ __global__ void __launch_bounds__(kHThreads, 1)
     // everything above is set-up that does not depend on earlier kernels; the planes, the words and the
     // output may
     griddep_wait();
+    const bool idle = p.only_if && *reinterpret_cast<volatile uint32_t *>(p.only_if) == 0u;
+    if (idle) { // behind a panel product that left nothing
+        __syncthreads();
+        if (slices > 1 || CG == 2)
+            cluster_sync();
+        if (warp == 1) {
+            if (CG == 2)
+                tmem_dealloc_pair(tmem_base, 512);
+            else
+                tmem_dealloc(tmem_base, 512);
+        }
+        if (threadIdx.x == 0 && p.reset && atomicAdd(p.flags + FLAG_EXCEPTION_READERS, 1u) + 1u == gridDim.x) {
+            p.flags[FLAG_EXCEPTION_READERS] = 0u;
+            p.reset->wide = p.reset->count = 0u;
+        }
+        return;
+    }
     const bool wide = p.force_wide || half_wide(p.exceptions_a, p.exceptions_b);
     const int k_step    = wide ? RB / 4 : RB / 2; // values of k per stage
     const int per_group = 64 / k_step;            // stages per 64 values of k
@@ -803,6 +821,8 @@ __global__ void __launch_bounds__(kHThreads, 1)
             if (atomicAdd(p.flags + FLAG_EXCEPTION_READERS, 1u) + 1u == gridDim.x) {
                 p.flags[FLAG_EXCEPTION_READERS] = 0u;
                 p.reset->wide = p.reset->count = 0u;
+                if (p.only_if)
+                    *p.only_if = 0u;
             }
         }
     }
@@ -963,9 +983,19 @@ __device__ __forceinline__ void half_rows(
 template <int TPR, int V>
 __global__ void __launch_bounds__(256) half_rows_kernel(
     const float *__restrict__ in, int64_t rows, int64_t k, int64_t kp, const HalfPlanes p, int vec_ok,
-    uint32_t *__restrict__ zero, int64_t zero_count) {
+    uint32_t *__restrict__ zero, int64_t zero_count, const uint32_t *__restrict__ only_if) {
     griddep_launch_dependents();
     griddep_wait();
+    if (only_if) { // behind a panel product, which seldom leaves anything: few blocks, which walk the rows
+        if (*reinterpret_cast<const volatile uint32_t *>(only_if) == 0u)
+            return;
+        constexpr int64_t rows_each = 256 / TPR;
+        for (int64_t block = blockIdx.x; block * rows_each < rows; block += gridDim.x) {
+            half_rows<TPR, V>(block, in, rows, k, kp, p, vec_ok);
+            __syncthreads();
+        }
+        return;
+    }
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < zero_count; i += (int64_t)gridDim.x * 256)
         zero[i] = 0u; // scales and column maxima of the right operand, accumulated by the next kernels
     half_rows<TPR, V>((int64_t)blockIdx.x, in, rows, k, kp, p, vec_ok);
@@ -1096,16 +1126,9 @@ __device__ __forceinline__ void half_cols_short(
     const int64_t n0 = (int64_t)block * kShortCols;
     const bool col_ok = n0 + tx < n;
     const float *src  = in + n0 + tx;
-    for (int kk0 = ty; kk0 < (int)kp; kk0 += 512) { // sixteen loads in flight
-        float v[16];
-#pragma unroll
-        for (int u = 0; u < 16; ++u)
-            v[u] = (col_ok && kk0 + 32 * u < k) ? src[(int64_t)(kk0 + 32 * u) * n] : 0.0f;
-#pragma unroll
-        for (int u = 0; u < 16; ++u)
-            if (kk0 + 32 * u < (int)kp)
-                tile[(kk0 + 32 * u) * kShortPad + tx] = v[u];
-    }
+#pragma unroll 8
+    for (int kk = ty; kk < (int)kp; kk += 32)
+        tile[kk * kShortPad + tx] = (col_ok && kk < k) ? src[(int64_t)kk * n] : 0.0f;
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint2 range    = make_uint2(0u, kNoneSmallest);
@@ -1321,15 +1344,14 @@ ct_status launch_half(DeviceState *st, const HalfOperand &a, const HalfOperand &
 
 ct_status half_split_rows(
     DeviceState *st, const float *in, int64_t k, int64_t kp, const HalfOperand &o, bool both_forms, uint32_t *zero,
-    int64_t zero_count) {
-    (void)st;
+    int64_t zero_count, const uint32_t *only_if) {
     const int64_t rows = o.rows;
     const int vec      = (k & 3) == 0 && (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
     const HalfPlanes p = planes_of(o, both_forms);
     // a warp per row while a row fits its registers (eight float4 per lane), else a block per row
 #define CT_ROWS(TPR, V, GRID)                                                                                       \
-    CT_CUDA(launch_dependent(half_rows_kernel<TPR, V>, dim3((unsigned)(GRID)), dim3(256), 0, stream(), in, rows, k, \
-                             kp, p, vec, zero, zero_count))
+    CT_CUDA(launch_dependent(half_rows_kernel<TPR, V>, dim3((unsigned)(only_if ? std::min<int64_t>((GRID), st->sm_count) : (GRID))), dim3(256), 0, stream(), in, rows, k, \
+                             kp, p, vec, zero, zero_count, only_if))
     if (kp <= 512)
         CT_ROWS(32, 4, (rows + 7) / 8);
     else if (kp <= 1024)
@@ -1445,7 +1467,7 @@ int gemm_tile_columns(const DeviceState *st, int64_t m, int64_t n, int64_t batch
 
 ct_status gemm_half(
     DeviceState *st, const HalfOperand &a, const HalfOperand &b, int64_t kp, const float *bias, int act, float *out,
-    bool force_wide, bool allow_splitk, const HalfBands *bands, int batch, bool bias_per_row) {
+    bool force_wide, bool allow_splitk, const HalfBands *bands, int batch, bool bias_per_row, uint32_t *only_if) {
     const int64_t m = a.rows, n = b.rows / batch;
     const int bn    = gemm_tile_columns(st, m, n, batch);
     HalfGemmParams p{};
@@ -1457,6 +1479,7 @@ ct_status gemm_half(
     p.row_scale   = a.scale;
     p.col_scale   = b.scale;
     p.flags       = st->flags_dev;
+    p.only_if     = only_if;
     p.a_hi = static_cast<const __half *>(a.hi16), p.a_lo = static_cast<const __half *>(a.lo16);
     p.b_hi = static_cast<const __half *>(b.hi16), p.b_lo = static_cast<const __half *>(b.lo16);
     p.kp           = (int)kp;

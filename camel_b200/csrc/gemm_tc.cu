@@ -236,11 +236,55 @@ __global__ void __launch_bounds__(256) split_transpose_kernel(
     }
 }
 
+// The same in blocks of 32 x 32, for operands that give the blocks above less than two to an SM.
+template <int MODE>
+__global__ void __launch_bounds__(256) split_transpose_small_kernel(
+    const float *__restrict__ in, int64_t k, int64_t n, int64_t kp, void *__restrict__ p_hi,
+    void *__restrict__ p_lo, int64_t in_batch_stride, int64_t out_batch_stride) {
+    __shared__ float tile[32][33];
+    griddep_launch_dependents();
+    griddep_wait();
+    int tx     = threadIdx.x & 31;
+    int ty     = threadIdx.x >> 5;
+    int64_t n0 = (int64_t)blockIdx.x * 32;
+    int64_t k0 = (int64_t)blockIdx.y * 32;
+    // blockIdx.z walks a batch of [k][n] matrices (conv: one [c][h*w] image each)
+    in += (int64_t)blockIdx.z * in_batch_stride;
+    const int64_t out_base = (int64_t)blockIdx.z * out_batch_stride;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        int64_t kk = k0 + ty + j * 8, nn = n0 + tx;
+        tile[ty + j * 8][tx] = (kk < k && nn < n) ? in[kk * n + nn] : 0.0f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        int64_t nn = n0 + ty + j * 8, kk = k0 + tx;
+        if (nn < n && kk < kp) {
+            float v     = tile[tx][ty + j * 8];
+            int64_t at  = out_base + nn * kp + kk;
+            if (MODE == MODE_3X) {
+                float hi, lo;
+                split_tf32(v, hi, lo);
+                static_cast<float *>(p_hi)[at] = hi;
+                static_cast<float *>(p_lo)[at] = lo;
+            } else {
+                static_cast<__nv_bfloat16 *>(p_hi)[at] = __float2bfloat16_rn(v);
+            }
+        }
+    }
+}
+
 // Errors are the caller's launch check's.
 template <int MODE>
 void launch_split_transpose(
     const float *in, int64_t k, int64_t n, int64_t kp, void *hi, void *lo, int64_t batch = 1, int64_t in_batch_stride = 0,
     int64_t out_batch_stride = 0) {
+    if (((n + 63) / 64) * ((kp + 63) / 64) * batch < 2 * 148) {
+        (void)launch_dependent(split_transpose_small_kernel<MODE>, dim3((unsigned)((n + 31) / 32), (unsigned)(kp / 32), (unsigned)batch),
+                               dim3(256), 0, stream(), in, k, n, kp, hi, lo, in_batch_stride, out_batch_stride);
+        return;
+    }
     const int vec = (n & 3) == 0 && (in_batch_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
     (void)launch_dependent(split_transpose_kernel<MODE>, dim3((unsigned)((n + 63) / 64), (unsigned)((kp + 63) / 64), (unsigned)batch),
                            dim3(256), 0, stream(), in, k, n, kp, hi, lo, vec, in_batch_stride, out_batch_stride);
@@ -1719,6 +1763,24 @@ static ct_status gemm_f32_split(
     if (packed) {
         ob.hi32 = packed->hi, ob.lo32 = packed->lo, ob.scale = packed->scale, ob.exceptions = packed->exceptions;
         ob.hi16 = force_wide ? packed->hi : packed->hi16, ob.lo16 = force_wide ? packed->lo : packed->lo16;
+    }
+    if (!a_is_km && !force_wide && gemm_panel_applicable(st, m, k, n)) {
+        // from A as it is; behind it, for operands that it leaves, the product from planes
+        uint32_t *left = st->flags_dev + FLAG_PANEL;
+        if (!packed) {
+            ProfScope prof("gemm_prepass");
+            CT_CUDA(cudaMemsetAsync(b_scale, 0, 2 * b_words, stream()));
+            CT_TRY(half_split_cols(st, b, k, kp, ob, both_forms, b_max));
+        }
+        CT_TRY(gemm_panel(st, a, ob, kp, bias, m, k, n, act, out));
+        {
+            ProfScope prof("gemm_prepass");
+            CT_TRY(half_split_rows(st, a, k, kp, oa, both_forms, nullptr, 0, left));
+            if (!both_forms)
+                CT_TRY(half_wide_planes(st, oa.exceptions, ob.exceptions, a, m, a_is_km, const_cast<void *>(oa.hi32), const_cast<void *>(oa.lo32), b,
+                                        packed ? 0 : n, const_cast<void *>(ob.hi32), const_cast<void *>(ob.lo32), k, kp));
+        }
+        return gemm_half(st, oa, ob, kp, bias, act, out, force_wide, true, nullptr, 1, false, left);
     }
     {
         ProfScope prof("gemm_prepass");
