@@ -281,7 +281,11 @@ __device__ __noinline__ void half_finish_slices(
 
 // LEFT: behind a panel product, for the operands that it leaves (p.only_if).  An instantiation of its own: with the early
 // exit in the ordinary one the compiler arranged the rest less well, two layers of 4096 x 1024 x 1024 85.4 -> 89.3 us.
-template <int BN, int CG, bool LEFT>
+// LINES: rows of the result that are not 16-byte aligned, at most one tile to a CTA or pair.  The operand stages are idle when
+// the tile is stored, so a warp's rows go through them whole and are stored in 128-byte lines, wherever in a line a row
+// begins; with a fixed 32 columns to a store every store has two partial sectors.  1537 x 771 x 2050 42.8 -> 41.4 us, 10453 x 199 x 222 31.0 -> 28.4.  In the
+// ordinary kernel (for a CTA's last tile) the same code cost others 3 %: 4096 x 1024 x 1024 twice 86.1 -> 88.6, 7853 x 118 x 8502 219 -> 237.
+template <int BN, int CG, bool LEFT, bool LINES>
 __global__ void __launch_bounds__(kHThreads, 1)
     gemm_half_kernel(const __grid_constant__ HalfMaps maps, const __grid_constant__ HalfGemmParams p) {
     using C            = HalfCfg<BN, CG>;
@@ -655,6 +659,49 @@ __global__ void __launch_bounds__(kHThreads, 1)
             float *out_z        = p.out + (int64_t)tz * p.out_batch_stride + (p.bands > 0 ? p.band_out_off[band] : 0);
             const bool vec      = (p.n & 3) == 0 && (reinterpret_cast<uintptr_t>(out_z) & 15u) == 0;
             const int rows_left = (int)(p.m - row0 < 32 ? (p.m - row0 < 0 ? 0 : p.m - row0) : 32);
+            if (LINES && !lacking) { // every MMA has retired
+                uint8_t *block = smem_raw + (smem_base - smem_u32(smem_raw)) + (uint32_t)ew * (32u * C::kCols * 4u);
+                float2 *columns = reinterpret_cast<float2 *>(stg); // scale and bias
+#pragma unroll
+                for (int g = 0; g < C::kCols / 32; ++g)
+                    columns[g * 32 + lane] = make_float2(cs[g], bb[g]);
+#pragma unroll
+                for (int j = 0; j < C::kCols / 4; ++j)
+                    *reinterpret_cast<float4 *>(block + lane * (C::kCols * 4) + ((j ^ (lane & 7)) << 4)) =
+                        make_float4(__fmul_rn(acc[4 * j], rs), __fmul_rn(acc[4 * j + 1], rs), __fmul_rn(acc[4 * j + 2], rs),
+                                    __fmul_rn(acc[4 * j + 3], rs));
+                __syncwarp();
+                const int64_t left = p.n - tile_c0 - half * C::kCols;
+                const int width    = (int)(left < C::kCols ? (left < 0 ? 0 : left) : C::kCols);
+                float *dst         = out_z + row0 * p.n + tile_c0 + half * C::kCols;
+#pragma unroll 1
+                for (int r = 0; r < rows_left; ++r, dst += p.n) {
+                    const int first = lane - (int)((reinterpret_cast<uintptr_t>(dst) >> 2) & 31u);
+                    const float rb  = __shfl_sync(0xffffffffu, row_bias, r);
+                    float x[C::kCols / 32 + 1];
+                    float2 cb[C::kCols / 32 + 1];
+#pragma unroll
+                    for (int j = 0; j <= C::kCols / 32; ++j) {
+                        const int col  = first + 32 * j;
+                        const bool in  = col >= 0 && col < width;
+                        const int from = in ? col : 0;
+                        x[j]  = *reinterpret_cast<const float *>(block + r * (C::kCols * 4) + (((from >> 2) ^ (r & 7)) << 4) + (from & 3) * 4);
+                        cb[j] = columns[from];
+                    }
+#pragma unroll
+                    for (int j = 0; j <= C::kCols / 32; ++j) {
+                        const int col = first + 32 * j;
+                        float y       = __fmul_rn(x[j], cb[j].x);
+                        if (p.bias)
+                            y = __fadd_rn(y, p.bias_per_row ? rb : cb[j].y);
+                        if (p.act == CT_ACT_RELU)
+                            y = __fmul_rn(y, y > 0.0f ? 1.0f : 0.0f);
+                        if (col >= 0 && col < width)
+                            dst[col] = y;
+                    }
+                }
+                __syncwarp();
+            } else
 #pragma unroll
             for (int g = 0; g < C::kCols / 32; ++g) {
                 const int c0        = half * C::kCols + g * 32; // column of the tile
@@ -1308,7 +1355,7 @@ ct_status plane_map(CUtensorMap *map, const void *base, int elem, int64_t rows, 
                      : encode_tiled_map_f16(map, base, 2, dims, strides, box, row_bytes);
 }
 
-template <int BN, int CG, bool LEFT = false>
+template <int BN, int CG, bool LEFT = false, bool LINES = false>
 ct_status launch_half(DeviceState *st, const HalfOperand &a, const HalfOperand &b, int64_t kp, HalfGemmParams &p, int splits) {
     using C = HalfCfg<BN, CG>;
     HalfMaps maps;
@@ -1329,14 +1376,14 @@ ct_status launch_half(DeviceState *st, const HalfOperand &a, const HalfOperand &
     p.group_m     = 16 / CG;
     static bool attr_set_dev[16] = {}; // the attribute belongs to a device's context
     if (!attr_set_dev[st->device & 15]) {
-        CT_CUDA(cudaFuncSetAttribute(gemm_half_kernel<BN, CG, LEFT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
+        CT_CUDA(cudaFuncSetAttribute(gemm_half_kernel<BN, CG, LEFT, LINES>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
         attr_set_dev[st->device & 15] = true;
     }
     const int units     = st->sm_count / CG;
     const unsigned grid = (unsigned)(tiles < units ? tiles : units) * CG;
     const int cluster   = p.cluster_split > 1 ? p.cluster_split : CG;
     ProfScope prof("gemm_tc");
-    CT_CUDA(launch_dependent_cluster(gemm_half_kernel<BN, CG, LEFT>, cluster, dim3(grid), dim3(kHThreads), (size_t)C::kSmemBytes, stream(), maps, p));
+    CT_CUDA(launch_dependent_cluster(gemm_half_kernel<BN, CG, LEFT, LINES>, cluster, dim3(grid), dim3(kHThreads), (size_t)C::kSmemBytes, stream(), maps, p));
     CT_LAUNCH_CHECK("gemm_half");
     return CT_OK;
 }
@@ -1457,8 +1504,8 @@ static int half_clusters(const DeviceState *st, int size) {
         cfg.gridDim = dim3((unsigned)(st->sm_count / size * size)), cfg.blockDim = dim3(kHThreads);
         cfg.dynamicSmemBytes = C::kSmemBytes;
         cfg.attrs = attr, cfg.numAttrs = 1;
-        if (cudaFuncSetAttribute(gemm_half_kernel<128, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&count, gemm_half_kernel<128, 1, false>, &cfg) != cudaSuccess || count < 1) {
+        if (cudaFuncSetAttribute(gemm_half_kernel<128, 1, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&count, gemm_half_kernel<128, 1, false, false>, &cfg) != cudaSuccess || count < 1) {
             cudaGetLastError();
             count = st->sm_count / size / 2 + 1; // not known: half of the machine
         }
@@ -1529,8 +1576,11 @@ ct_status gemm_half(
         p.bias = bias, p.act = act, p.out = out;
         if (only_if)
             return launch_half<128, 1, true>(st, a, b, kp, p, splits);
-        if (bn == 256 && !bands && m > kHM)
-            return launch_half<256, 2>(st, a, b, kp, p, 1);
+        if (bn == 256 && !bands && m > kHM) {
+            const int64_t pairs = (m + 2 * kHM - 1) / (2 * kHM) * ((n + 255) / 256) * batch;
+            return (n & 3) != 0 && pairs <= st->sm_count / 2 ? launch_half<256, 2, false, true>(st, a, b, kp, p, 1)
+                                                             : launch_half<256, 2>(st, a, b, kp, p, 1);
+        }
         return bn == 256 ? launch_half<256, 1>(st, a, b, kp, p, 1) : launch_half<128, 1>(st, a, b, kp, p, splits);
     }
     CT_TRY(ensure_ws(&st->splitk_ws, &st->splitk_ws_bytes, (size_t)splits * m * n * sizeof(float)));

@@ -111,6 +111,32 @@ def test_tall_products_with_one_tile_of_columns(T, m, k, n, kind):
     assert np.all(np.abs(got[finite] - want[finite]) <= BOUND * size[finite])
 
 
+# rows of the result that begin anywhere in a line, one tile to a pair: a last tile of one, 33 and 129 columns, whole last tiles, rows
+# that end inside a warp's 32
+@pytest.mark.parametrize("m,k,n", [(1281, 65, 1793), (2305, 771, 1057), (1537, 100, 1665), (1280, 40, 2047), (4609, 130, 514)])
+@pytest.mark.parametrize("kind", ["plain", "small value", "infinity"])
+def test_results_whose_rows_are_not_aligned(T, m, k, n, kind):
+    rng = np.random.default_rng(m + k + n)
+    a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    b = rng.uniform(-1, 1, (k, n)).astype(np.float32)
+    c = rng.uniform(-1, 1, n).astype(np.float32)
+    if kind == "small value":
+        a[m // 2, k // 3] = 1e-20
+    if kind == "infinity":
+        a[m - 1, k - 1] = np.inf
+    got = T.dense(T.from_numpy(a), T.from_numpy(b), T.from_numpy(c), "relu").numpy()
+    plain = T.matmul(T.from_numpy(a), T.from_numpy(b)).numpy()
+    T.check_async()
+    a64, b64 = a.astype(np.float64), b.astype(np.float64)
+    product = a64 @ b64
+    want, rows = np.maximum(product + c, 0.0), np.isfinite(a).all(axis=1)
+    size = np.abs(a64[rows]) @ np.abs(b64) + np.abs(c)
+    assert np.all(np.abs(got[rows] - want[rows]) <= BOUND * size)
+    assert np.all(np.abs(plain[rows] - product[rows]) <= BOUND * size)
+    # infinity, or NaN where the two terms of the other operand's value have opposite signs (inf - inf)
+    assert not np.isfinite(plain[~rows]).any()
+
+
 @pytest.mark.parametrize("k,n", [(1030, 130), (1100, 257), (2050, 64), (1088, 1)])
 @pytest.mark.parametrize("precision", [0, 1])
 def test_right_operands_in_blocks(T, k, n, precision):
