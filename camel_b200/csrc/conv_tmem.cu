@@ -1,5 +1,7 @@
 // conv2d for layers with few channels on both sides (at most 32 in, at most 64 out, a small
-// filter; the 32 -> 64 channel 3x3 layer of a small CNN): the filters live in tensor memory.
+// filter; the 32 -> 64 channel 3x3 layer of a small CNN).  Two forms: conv_pairs_kernel, on float16 pairs, computes
+// almost every image and has its own comment further down; the tf32 form that this comment is about computes, behind it, the
+// images whose values float16 pairs cannot hold.  In it the filters live in tensor memory.
 //
 // Why another kernel.  With 64 output channels the tensor core cannot be given a wide tile:
 // measured on B200 (ct_measure_mma_rate), tcgen05.mma kind::tf32 of 128 x N x 8 takes ~138 clocks

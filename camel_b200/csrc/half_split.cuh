@@ -15,8 +15,8 @@
 // a few per hundred million, so the pre-pass stores zeros for them, lists up to kHalfExceptions of a product, marks
 // their rows by the sign of the scale, and the product's epilogue adds value . other operand to the outputs of
 // those rows and columns.  A matrix with more of them, or with a row whose exponent is beyond +-60, is computed from
-// tf32 planes instead (same launch sequence, no host involvement).  Convolutions of stride 1 decide that per image
-// (and per layer for its filters), see half_range_fits.
+// tf32 planes instead (same launch sequence, no host involvement).  Convolutions, but those through patches, decide
+// that per image (and per layer for its filters), see half_range_fits.
 #pragma once
 
 #include <cuda_fp16.h>
