@@ -236,7 +236,8 @@ __global__ void __launch_bounds__(256) split_transpose_kernel(
     }
 }
 
-// The same in blocks of 32 x 32, for operands that give the blocks above less than two to an SM.
+// The same in blocks of 32 x 32, for operands that give the blocks above less than two to an SM: 582 x 2210 x 107 30 us, with
+// the larger ones 35; 8192 x 8192 goes the other way, 153 us against 101.
 template <int MODE>
 __global__ void __launch_bounds__(256) split_transpose_small_kernel(
     const float *__restrict__ in, int64_t k, int64_t n, int64_t kp, void *__restrict__ p_hi,
