@@ -7,9 +7,9 @@
 // along the values that an accumulator sums, so each row of each chunk has its own, and the accumulators - one set
 // computes while the other is read - are drained every chunk, in float32 with round-to-nearest adds.  B's planes come
 // by TMA as for the other products; the slices of a tile's k are CTAs of a cluster, which add up through distributed
-// shared memory.  8192 x 12544 x 128: 261 -> 190 us, 9000 x 2100 x 64: 64 -> 55.  What bounds it: what the SMs draw from L2, 64 KB of
-// A and 64 KB of B's planes a chunk, 4600 clocks at the 28 bytes a clock that each SM gets when all draw; a chunk takes about 6400
-// (the splitting warps wait for their loads and for the drain one after the other), where A alone from memory would take 2480.
+// shared memory.  8192 x 12544 x 128: 261 -> 184 us, 9000 x 2100 x 64: 64 -> 56.  What bounds it: what the SMs draw from L2, 64 KB of
+// A and 64 KB of B's planes a chunk, 4600 clocks at the 28 bytes a clock that each SM gets when all draw; a chunk takes about 5800,
+// where A alone from memory would take 2480.
 //
 // Values of A that float16 pairs cannot hold are listed, zeros in their place, and their products with B's row added to the sums
 // in float32, B's own list likewise.  More than the lists hold, infinities, NaN or exponents beyond the scales leave a mark:
@@ -290,10 +290,15 @@ __global__ void __launch_bounds__(kGP_Threads, 1) gemm_panel_kernel(
             __syncwarp();
             if (lane == 0)
                 mbar_arrive(smem_u32(&bar_a_full[b]));
-            load(c + 1);
             prefetch(c + 3);
+            // one half of the warps loads while the other drains: 8192 x 12544 x 128 184 us, 194 with all in one order
+            const bool later = (w >> 2) & 1;
+            if (!later)
+                load(c + 1);
             if (c > 0)
                 drain(c - 1);
+            if (later)
+                load(c + 1);
         }
         if (ok && chunks > 0)
             drain(chunks - 1);
@@ -309,12 +314,14 @@ __global__ void __launch_bounds__(kGP_Threads, 1) gemm_panel_kernel(
             if (x.row != row)
                 continue;
             const int64_t kk = (int64_t)chunk0 * kGP_K + x.chunk_k;
-#pragma unroll 8
-            for (int j = 0; j < 32; ++j)
-                if (cg * 32 + j < p.n) {
-                    const int64_t at = (cg * 32 + j) * p.kp + kk;
-                    acc[j] = __fmaf_rn(x.value, __half2float(p.b_hi[at]) + __half2float(p.b_lo[at]) * kHalfLoInv, acc[j]);
-                }
+#pragma unroll 1
+            for (int j = 0; j < 32 && cg * 32 + j < p.n; ++j) {
+                const int64_t at = (cg * 32 + j) * p.kp + kk;
+                const float b    = __half2float(p.b_hi[at]) + __half2float(p.b_lo[at]) * kHalfLoInv;
+#pragma unroll
+                for (int q = 0; q < 32; ++q) // no index that is not constant: the sums would leave their registers for the whole kernel
+                    acc[q] = q == j ? __fmaf_rn(x.value, b, acc[q]) : acc[q];
+            }
         }
         const int listed_b = (int)p.exceptions_b->count;
         for (int i = 0; i < listed_b; ++i) {
