@@ -563,14 +563,22 @@ __global__ void __launch_bounds__(256) conv_range_kernel(
 // images are taken last to first: the end of the tensor is what conv_range_kernel has just left in L2.
 // Sub-images (ConvSubImages, hs x ws each): zeros where the image has no such row or column, those that no tap reads are
 // left out.
+//
+// What bounds it is issue (0.83 of the slots at 128 x 64 x 56 x 56), so the moduli are constants, the one division left is a
+// multiplication, and one warp works the image's scale out for all: 64 x 48 x 57 x 57 -> 96 at stride 2 76 -> 69 us (31 of it this kernel
+// before), 256 x 64 x 56 x 56 -> 128 428 -> 425.
 struct PlaneGeom {
     int h, w, hs, ws;
+    uint32_t width_inv; // 2^32 / (ws * col_mod), rounded up; 0 for a width of 1
     ConvSubImages sub;
 };
+template <int ROW_MOD, int COL_MOD>
 __global__ void __launch_bounds__(256) conv_planes_kernel(
     const float *__restrict__ x, int c, const PlaneGeom geom, int c_pad, const uint2 *__restrict__ ranges, int slices,
     const float *__restrict__ filter_scale, int ko, uint8_t *__restrict__ slots, float *__restrict__ image_scale) {
     __shared__ float tile[64][65];
+    __shared__ float scale_s;
+    __shared__ int fits_s;
     griddep_launch_dependents();
     griddep_wait();
     const int64_t img = gridDim.z - 1 - blockIdx.z;
@@ -578,15 +586,19 @@ __global__ void __launch_bounds__(256) conv_planes_kernel(
     const int c0      = (int)blockIdx.y * 64;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t in_hw = (int64_t)geom.h * geom.w;
-    const int row_mod = geom.sub.row_mod, col_mod = geom.sub.col_mod, width = geom.ws * col_mod;
-    const int64_t hw  = (int64_t)geom.hs * row_mod * width; // positions of the image grown to whole multiples
-    const bool apart  = row_mod * col_mod > 1;
-    const float *src  = x + (img * c + c0) * in_hw;
+    const int width  = geom.ws * COL_MOD;
+    const int64_t hw = (int64_t)geom.hs * ROW_MOD * width; // positions of the image grown to whole multiples
+    constexpr bool apart = ROW_MOD * COL_MOD > 1;
+    const float *src = x + (img * c + c0) * in_hw;
+    auto row_of = [&](int64_t q) { // q < 2^31: the rounded-up quotient is one too high at most
+        const int row = geom.width_inv ? (int)__umulhi((uint32_t)q, geom.width_inv) : (int)q;
+        return row - (row * width > (int)q ? 1 : 0);
+    };
     // position q of the grown image in the input (-1: not there)
     auto source = [&](int64_t q) -> int64_t {
         if (!apart)
             return q < hw ? q : -1;
-        const int row = (int)q / width, col = (int)q - row * width;
+        const int row = row_of(q), col = (int)q - row * width;
         return q < hw && row < geom.h && col < geom.w ? (int64_t)row * geom.w + col : -1;
     };
     float v[16]; // every load before the first use of any
@@ -599,19 +611,25 @@ __global__ void __launch_bounds__(256) conv_planes_kernel(
             v[2 * j + t] = (c0 + ch < c && from >= 0) ? __ldcs(src + ch * in_hw + from) : 0.0f;
         }
     }
-    uint2 r = make_uint2(0u, kNoneSmallest);
-    for (int s = lane; s < slices; s += 32)
-        r = range_join(r, ranges[img * slices + s]);
+    if (warp == 0) {
+        uint2 r = make_uint2(0u, kNoneSmallest);
+        for (int s = lane; s < slices; s += 32)
+            r = range_join(r, ranges[img * slices + s]);
+        float s, inverse;
+        const bool all = half_range_fits(range_warp(r), s, inverse);
+        if (lane == 0)
+            scale_s = s, fits_s = all;
+    }
     int bad_filter = 0;
     for (int o = threadIdx.x; o < ko; o += 256)
         bad_filter |= filter_scale[o] == 0.0f ? 1 : 0;
 #pragma unroll
     for (int j = 0; j < 16; ++j)
         tile[warp + 8 * (j >> 1)][lane + 32 * (j & 1)] = v[j];
-    float scale, inverse;
-    const bool fits = half_range_fits(range_warp(r), scale, inverse) & !__syncthreads_or(bad_filter);
+    const bool fits   = !__syncthreads_or(bad_filter) && fits_s;
+    const float scale = scale_s;
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
-        image_scale[img] = fits ? inverse : 0.0f;
+        image_scale[img] = fits ? 1.0f / scale : 0.0f; // a power of two
     const int64_t plane = hw * c_pad;
     uint8_t *slot       = slots + img * plane * 8;
 #pragma unroll
@@ -621,11 +639,11 @@ __global__ void __launch_bounds__(256) conv_planes_kernel(
             continue;
         int64_t to = q0 + q;
         if (apart) {
-            const int row = (int)to / width, col = (int)to - row * width, sub = row % row_mod * col_mod + col % col_mod;
+            const int row = row_of(to), col = (int)to - row * width, sub = row % ROW_MOD * COL_MOD + col % COL_MOD;
             if (!(geom.sub.used >> sub & 1u))
                 continue;
             if (fits || !geom.sub.tf32_plain)
-                to = ((int64_t)sub * geom.hs + row / row_mod) * geom.ws + col / col_mod;
+                to = ((int64_t)sub * geom.hs + row / ROW_MOD) * geom.ws + col / COL_MOD;
             else if (row < geom.h && col < geom.w)
                 to = (int64_t)row * geom.w + col;
             else
@@ -725,11 +743,22 @@ ct_status conv_prepass(
     CT_CUDA(launch_dependent(conv_range_kernel, dim3((unsigned)(ko + batch * slices)), dim3(256), 0, stream(), w, (int)c, (int)taps,
                              (int)c_pad, (int)ko, f, x, count, slices, vec, static_cast<uint2 *>(ranges)));
     CT_LAUNCH_CHECK("conv_range");
-    const PlaneGeom geom{(int)h, (int)wd, (int)((h + sub.row_mod - 1) / sub.row_mod), (int)((wd + sub.col_mod - 1) / sub.col_mod), sub};
-    const int64_t positions = (int64_t)geom.hs * geom.ws * sub.row_mod * sub.col_mod;
+    PlaneGeom geom{(int)h, (int)wd, (int)((h + sub.row_mod - 1) / sub.row_mod), (int)((wd + sub.col_mod - 1) / sub.col_mod), 0, sub};
+    const int64_t width = (int64_t)geom.ws * sub.col_mod, positions = geom.hs * width * sub.row_mod;
+    geom.width_inv = width > 1 ? (uint32_t)(((1ull << 32) + width - 1) / width) : 0;
     const dim3 grid((unsigned)((positions + 63) / 64), (unsigned)((c_pad + 63) / 64), (unsigned)batch);
-    CT_CUDA(launch_dependent(conv_planes_kernel, grid, dim3(256), 0, stream(), x, (int)c, geom, (int)c_pad, static_cast<const uint2 *>(ranges),
-                             slices, static_cast<const float *>(filter_scale), (int)ko, static_cast<uint8_t *>(slots), image_scale));
+    auto planes = [&](auto kernel) {
+        return launch_dependent(kernel, grid, dim3(256), 0, stream(), x, (int)c, geom, (int)c_pad, static_cast<const uint2 *>(ranges), slices,
+                                static_cast<const float *>(filter_scale), (int)ko, static_cast<uint8_t *>(slots), image_scale);
+    };
+    if (sub.row_mod == 1 && sub.col_mod == 1)
+        CT_CUDA(planes(conv_planes_kernel<1, 1>));
+    else if (sub.row_mod == 2 && sub.col_mod == 1)
+        CT_CUDA(planes(conv_planes_kernel<2, 1>));
+    else if (sub.row_mod == 2 && sub.col_mod == 2)
+        CT_CUDA(planes(conv_planes_kernel<2, 2>));
+    else
+        CT_CUDA(planes(conv_planes_kernel<3, 3>));
     CT_LAUNCH_CHECK("conv_planes");
     return CT_OK;
 }
