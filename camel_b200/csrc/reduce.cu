@@ -11,16 +11,10 @@
 namespace ct {
 namespace {
 
-// Launches a kernel over `values` values.  Large ones start while their predecessor ends (launch_dependent): eleven operators
-// on 8192 x 8192 520 -> 504 us.  That way of launching costs the host about a microsecond more, which is what small ones are
-// bound by (94 x 96: 69 us, 81 if they did it too), so they are launched as usual.
-constexpr int64_t kOverlapFrom = 1 << 20;
-template <typename... KArgs, typename... Args>
-void launch(int64_t values, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args &&...args) {
-    if (values >= kOverlapFrom)
-        (void)launch_dependent(kernel, grid, block, smem, stream(), std::forward<Args>(args)...);
-    else
-        kernel<<<grid, block, smem, stream()>>>(std::forward<Args>(args)...);
+// Every kernel starts while its predecessor ends (launch_dependent): eleven operators on 8192 x 8192 520 -> 504 us, on 740 x 3261
+// 82 -> 73, on 94 x 96 69 -> 62.  Errors are the caller's launch check's.
+template <typename... KArgs, typename... Args> void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args &&...args) {
+    (void)launch_dependent(kernel, grid, block, smem, stream(), std::forward<Args>(args)...);
 }
 
 __device__ __forceinline__ double as_double(float v) { return (double)v; }
@@ -122,7 +116,7 @@ template <typename T> ct_status sum_typed(DeviceState *st, const T *in, uint64_t
     ProfScope prof("reduce");
     if (sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(in) & 15u) == 0 && n >= 4096) {
         uint64_t nvec = n / 4;
-        launch((int64_t)n, sum_partial_f32x4_kernel, dim3(blocks), dim3(kSumThreads), 0,
+        launch(sum_partial_f32x4_kernel, dim3(blocks), dim3(kSumThreads), 0,
             reinterpret_cast<const float4 *>(in), nvec, partials);
         CT_LAUNCH_CHECK("sum(pass 1)");
         tail   = in + nvec * 4;
@@ -131,10 +125,10 @@ template <typename T> ct_status sum_typed(DeviceState *st, const T *in, uint64_t
         uint64_t want = (n + kSumThreads - 1) / kSumThreads;
         if (want < (uint64_t)blocks)
             used = (int)(want ? want : 1);
-        launch((int64_t)n, sum_partial_kernel<T>, dim3(used), dim3(kSumThreads), 0, in, n, partials);
+        launch(sum_partial_kernel<T>, dim3(used), dim3(kSumThreads), 0, in, n, partials);
         CT_LAUNCH_CHECK("sum(pass 1)");
     }
-    launch((int64_t)n, sum_final_kernel<T>, dim3(1), dim3(kSumThreads), 0, partials, used, tail, tail_n, out);
+    launch(sum_final_kernel<T>, dim3(1), dim3(kSumThreads), 0, partials, used, tail, tail_n, out);
     CT_LAUNCH_CHECK("sum(pass 2)");
     CT_CUDA(cudaMemcpyAsync(result, out, sizeof(double), cudaMemcpyDeviceToHost, stream()));
     CT_CUDA(cudaStreamSynchronize(stream()));
@@ -314,16 +308,16 @@ ct_status reduce_axis_typed(const T *in, int64_t rows, int64_t cols, int axis, O
             return CT_OK;
         if (cols <= 2048) {
             unsigned blocks = (unsigned)((rows + 7) / 8);
-            launch(rows * cols, reduce_rows_warp_kernel<KIND, T, OT>, dim3(blocks), dim3(256), 0, in, rows, cols, out);
+            launch(reduce_rows_warp_kernel<KIND, T, OT>, dim3(blocks), dim3(256), 0, in, rows, cols, out);
         } else {
-            launch(rows * cols, reduce_rows_block_kernel<KIND, T, OT>, dim3((unsigned)rows), dim3(256), 0, in, rows, cols, out);
+            launch(reduce_rows_block_kernel<KIND, T, OT>, dim3((unsigned)rows), dim3(256), 0, in, rows, cols, out);
         }
         CT_LAUNCH_CHECK("reduce(axis=1)");
     } else {
         if (cols == 0)
             return CT_OK;
         unsigned blocks = (unsigned)((cols + 31) / 32);
-        launch(rows * cols, reduce_cols_kernel<KIND, T, OT>, dim3(blocks), dim3(256), 0, in, rows, cols, out);
+        launch(reduce_cols_kernel<KIND, T, OT>, dim3(blocks), dim3(256), 0, in, rows, cols, out);
         CT_LAUNCH_CHECK("reduce(axis=0)");
     }
     return CT_OK;
@@ -634,18 +628,18 @@ ct_status reduce_axis_f32(DeviceState *st, const float *in, int64_t rows, int64_
             return CT_OK;
         if (cols >= 2 && cols <= 32 && (cols & 1) == 0 && rows >= 256 * (int64_t)st->sm_count &&
             (reinterpret_cast<uintptr_t>(in) & 7u) == 0) {
-            launch(rows * cols, reduce_rows_direct_f32_kernel<KIND, OT>, dim3((unsigned)((rows + 255) / 256)), dim3(256), 0, in, rows, (int)cols, out);
+            launch(reduce_rows_direct_f32_kernel<KIND, OT>, dim3((unsigned)((rows + 255) / 256)), dim3(256), 0, in, rows, (int)cols, out);
         } else if (cols <= 32 && rows >= 1024 * (int64_t)st->sm_count && cols <= 11) {
             // many short rows: four rows per thread (up to 44 KB of a block's rows in flight)
             const unsigned blocks = (unsigned)((rows + 1023) / 1024);
-            launch(rows * cols, reduce_rows_narrow_f32_kernel<KIND, OT, 4>, dim3(blocks), dim3(256), (size_t)1024 * cols * sizeof(float), in, rows, (int)cols, out);
+            launch(reduce_rows_narrow_f32_kernel<KIND, OT, 4>, dim3(blocks), dim3(256), (size_t)1024 * cols * sizeof(float), in, rows, (int)cols, out);
         } else if (cols <= 32) {
             const unsigned blocks = (unsigned)((rows + 255) / 256);
-            launch(rows * cols, reduce_rows_narrow_f32_kernel<KIND, OT, 1>, dim3(blocks), dim3(256), (size_t)256 * cols * sizeof(float), in, rows, (int)cols, out);
+            launch(reduce_rows_narrow_f32_kernel<KIND, OT, 1>, dim3(blocks), dim3(256), (size_t)256 * cols * sizeof(float), in, rows, (int)cols, out);
         } else if (cols <= 1024) {
-            launch(rows * cols, reduce_rows_f32_kernel<KIND, OT, 32>, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, in, rows, cols, out);
+            launch(reduce_rows_f32_kernel<KIND, OT, 32>, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, in, rows, cols, out);
         } else {
-            launch(rows * cols, reduce_rows_f32_kernel<KIND, OT, 256>, dim3((unsigned)rows), dim3(256), 0, in, rows, cols, out);
+            launch(reduce_rows_f32_kernel<KIND, OT, 256>, dim3((unsigned)rows), dim3(256), 0, in, rows, cols, out);
         }
         CT_LAUNCH_CHECK("reduce(axis=1)");
         return CT_OK;
@@ -669,9 +663,9 @@ ct_status reduce_axis_f32(DeviceState *st, const float *in, int64_t rows, int64_
     int64_t *pidx = reinterpret_cast<int64_t *>(psum + per);
     float *pv     = reinterpret_cast<float *>(pidx + per);
     dim3 grid((unsigned)col_blocks, (unsigned)slices);
-    launch(rows * cols, reduce_cols_f32_kernel<KIND>, dim3(grid), dim3(256), 0, in, rows, cols, rows_per_slice, psum, pv, pidx);
+    launch(reduce_cols_f32_kernel<KIND>, dim3(grid), dim3(256), 0, in, rows, cols, rows_per_slice, psum, pv, pidx);
     CT_LAUNCH_CHECK("reduce(axis=0)");
-    launch(rows * cols, reduce_cols_finish_f32_kernel<KIND, OT>, dim3((unsigned)((cols + 255) / 256)), dim3(256), 0, in, cols, (int)slices, psum, pv, pidx, out);
+    launch(reduce_cols_finish_f32_kernel<KIND, OT>, dim3((unsigned)((cols + 255) / 256)), dim3(256), 0, in, cols, (int)slices, psum, pv, pidx, out);
     CT_LAUNCH_CHECK("reduce(axis=0, finish)");
     return CT_OK;
 }
@@ -1044,7 +1038,7 @@ ct_status concat_typed(
     if (blocks > cap)
         blocks = cap;
     ProfScope prof("concat");
-    launch((int64_t)total, concat_kernel<U>, dim3((unsigned)blocks), dim3(256), 0,
+    launch(concat_kernel<U>, dim3((unsigned)blocks), dim3(256), 0,
         static_cast<const U *>(l), static_cast<const U *>(r), outer, ll, rl, static_cast<U *>(o));
     CT_LAUNCH_CHECK("concat");
     return CT_OK;
@@ -1106,24 +1100,24 @@ ct_status ct_softmax_rows(const float *in, int64_t rows, int64_t cols, float *ou
     unsigned wblocks = (unsigned)((rows + 7) / 8);
     ProfScope prof("softmax");
     if (cols <= 32)
-        launch(rows * cols, softmax_rows_warp_kernel<1>, dim3(wblocks), dim3(256), 0, in, rows, cols, out);
+        launch(softmax_rows_warp_kernel<1>, dim3(wblocks), dim3(256), 0, in, rows, cols, out);
     else if (cols <= 128)
-        launch(rows * cols, softmax_rows_warp_kernel<4>, dim3(wblocks), dim3(256), 0, in, rows, cols, out);
+        launch(softmax_rows_warp_kernel<4>, dim3(wblocks), dim3(256), 0, in, rows, cols, out);
     else if (cols <= 512)
-        launch(rows * cols, softmax_rows_warp_kernel<16>, dim3(wblocks), dim3(256), 0, in, rows, cols, out);
+        launch(softmax_rows_warp_kernel<16>, dim3(wblocks), dim3(256), 0, in, rows, cols, out);
     else if (cols <= 8192 && (cols & 3) == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0) {
         if (cols <= 2048)
-            launch(rows * cols, softmax_rows_wide_kernel<1, 512>, dim3((unsigned)rows), dim3(512), 0, in, rows, cols, out);
+            launch(softmax_rows_wide_kernel<1, 512>, dim3((unsigned)rows), dim3(512), 0, in, rows, cols, out);
         else if (cols <= 4096)
-            launch(rows * cols, softmax_rows_wide_kernel<2, 512>, dim3((unsigned)rows), dim3(512), 0, in, rows, cols, out);
+            launch(softmax_rows_wide_kernel<2, 512>, dim3((unsigned)rows), dim3(512), 0, in, rows, cols, out);
         else
-            launch(rows * cols, softmax_rows_wide_kernel<4, 512>, dim3((unsigned)rows), dim3(512), 0, in, rows, cols, out);
+            launch(softmax_rows_wide_kernel<4, 512>, dim3((unsigned)rows), dim3(512), 0, in, rows, cols, out);
     } else if (cols <= 2048)
-        launch(rows * cols, softmax_rows_kernel<8, 256>, dim3((unsigned)rows), dim3(256), 0, in, rows, cols, out);
+        launch(softmax_rows_kernel<8, 256>, dim3((unsigned)rows), dim3(256), 0, in, rows, cols, out);
     else if (cols <= 8192)
-        launch(rows * cols, softmax_rows_kernel<8, 1024>, dim3((unsigned)rows), dim3(1024), 0, in, rows, cols, out);
+        launch(softmax_rows_kernel<8, 1024>, dim3((unsigned)rows), dim3(1024), 0, in, rows, cols, out);
     else
-        launch(rows * cols, softmax_rows_stream_kernel, dim3((unsigned)rows), dim3(256), 0, in, rows, cols, out);
+        launch(softmax_rows_stream_kernel, dim3((unsigned)rows), dim3(256), 0, in, rows, cols, out);
     CT_LAUNCH_CHECK("softmax_rows");
     return CT_OK;
 }
@@ -1143,22 +1137,22 @@ ct_status ct_transpose(ct_dtype dt, const void *in, int64_t rows, int64_t cols, 
     if (dt == CT_F32 && (rows & 3) == 0 && (cols & 3) == 0 && (rows + 63) / 64 <= 65535 &&
         ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0) {
         dim3 grid64((unsigned)((cols + 63) / 64), (unsigned)((rows + 63) / 64));
-        launch(rows * cols, transpose_f32x4_kernel, dim3(grid64), dim3(256), 0,
+        launch(transpose_f32x4_kernel, dim3(grid64), dim3(256), 0,
             static_cast<const float *>(in), rows, cols, static_cast<float *>(out));
         CT_LAUNCH_CHECK("transpose");
         return CT_OK;
     }
     switch (dt) {
     case CT_F32:
-        launch(rows * cols, transpose_kernel<float>, dim3(grid), dim3(256), 0,
+        launch(transpose_kernel<float>, dim3(grid), dim3(256), 0,
             static_cast<const float *>(in), rows, cols, static_cast<float *>(out));
         break;
     case CT_I64:
-        launch(rows * cols, transpose_kernel<int64_t>, dim3(grid), dim3(256), 0,
+        launch(transpose_kernel<int64_t>, dim3(grid), dim3(256), 0,
             static_cast<const int64_t *>(in), rows, cols, static_cast<int64_t *>(out));
         break;
     default:
-        launch(rows * cols, transpose_kernel<uint8_t>, dim3(grid), dim3(256), 0,
+        launch(transpose_kernel<uint8_t>, dim3(grid), dim3(256), 0,
             static_cast<const uint8_t *>(in), rows, cols, static_cast<uint8_t *>(out));
         break;
     }
