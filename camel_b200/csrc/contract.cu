@@ -247,6 +247,8 @@ __global__ void __launch_bounds__(256) conv2d_small_c_kernel(
     const float *__restrict__ x, const float *__restrict__ wt, const float *__restrict__ bias,
     int64_t n, int c, int64_t h, int64_t w, int ko, int kh, int kw, int64_t stride, int64_t pad,
     int64_t ho, int64_t wo, int act, float *__restrict__ out) {
+    griddep_launch_dependents();
+    griddep_wait();
     // [ko][kdim], widened to float64 once per block: float32 -> float64 conversions are the slow
     // instruction here, so none is left in the multiply-add loop when the patch is short
     extern __shared__ double w_s[];
@@ -307,6 +309,8 @@ __global__ void __launch_bounds__(256) conv2d_c1_3x3_kernel(
     const float *__restrict__ x, const float *__restrict__ wt, const float *__restrict__ bias,
     int64_t n, int64_t h, int64_t w, int ko, int64_t pad, int64_t ho, int64_t wo, int act,
     float *__restrict__ out) {
+    griddep_launch_dependents();
+    griddep_wait();
     extern __shared__ double w_s[]; // [ko][9], then the bias
     for (int i = threadIdx.x; i < ko * 9; i += 256)
         w_s[i] = (double)wt[i];
@@ -368,6 +372,8 @@ __global__ void __launch_bounds__(256) conv2d_c1_3x3_kernel(
 __global__ void __launch_bounds__(256) maxpool2d_kernel(
     const float *__restrict__ x, int64_t planes, int64_t h, int64_t w, int64_t win, int64_t ho,
     int64_t wo, float *__restrict__ out) {
+    griddep_launch_dependents();
+    griddep_wait();
     int64_t total = planes * ho * wo;
     int64_t step  = (int64_t)gridDim.x * 256;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += step) {
@@ -389,6 +395,8 @@ __global__ void __launch_bounds__(256) maxpool2d_kernel(
 __global__ void __launch_bounds__(256) maxpool2x2_kernel(
     const float *__restrict__ x, int64_t planes, int64_t h, int64_t w, int64_t ho, int64_t wo,
     float *__restrict__ out) {
+    griddep_launch_dependents();
+    griddep_wait();
     int64_t total = planes * ho * wo;
     int64_t step  = (int64_t)gridDim.x * 256;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += step) {
@@ -414,6 +422,8 @@ template <typename IDX>
 __global__ void __launch_bounds__(256) maxpool2x2_wide_kernel(
     const float *__restrict__ x, int64_t planes, int64_t h, int64_t w, int64_t ho, int64_t wo,
     float *__restrict__ out) {
+    griddep_launch_dependents();
+    griddep_wait();
     const IDX pairs = (IDX)(wo >> 1), rows = (IDX)ho;
     const IDX total = (IDX)(planes * ho) * pairs;
     const IDX step  = (IDX)gridDim.x * 256;
@@ -709,7 +719,7 @@ static ct_status conv2d_run(
             CT_CUDA(cudaFuncSetAttribute(conv2d_c1_3x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 56 * 1024));
             attr_set_dev[st->device & 15] = true;
         }
-        conv2d_c1_3x3_kernel<<<capped_blocks(st, n * ho * (wo >> 2), 16), 256, (size_t)ko * 80, stream()>>>(
+        (void)launch_dependent(conv2d_c1_3x3_kernel, dim3(capped_blocks(st, n * ho * (wo >> 2), 16)), dim3(256), (size_t)ko * 80, stream(),
             x, w, bias, n, h, wd, (int)ko, pad, ho, wo, act, out);
         CT_LAUNCH_CHECK("conv2d_c1_3x3");
         return CT_OK;
@@ -720,13 +730,13 @@ static ct_status conv2d_run(
         size_t smem     = (size_t)(ko * kdim * 8);
 #define CT_SMALL_C_ARGS x, w, bias, n, (int)c, h, wd, (int)ko, (int)kh, (int)kw, stride, pad, ho, wo, act, out
         if (kdim <= 9)
-            conv2d_small_c_kernel<9><<<blocks, 256, smem, stream()>>>(CT_SMALL_C_ARGS);
+            (void)launch_dependent(conv2d_small_c_kernel<9>, dim3(blocks), dim3(256), smem, stream(), CT_SMALL_C_ARGS);
         else if (kdim <= 16)
-            conv2d_small_c_kernel<16><<<blocks, 256, smem, stream()>>>(CT_SMALL_C_ARGS);
+            (void)launch_dependent(conv2d_small_c_kernel<16>, dim3(blocks), dim3(256), smem, stream(), CT_SMALL_C_ARGS);
         else if (kdim <= 32)
-            conv2d_small_c_kernel<32><<<blocks, 256, smem, stream()>>>(CT_SMALL_C_ARGS);
+            (void)launch_dependent(conv2d_small_c_kernel<32>, dim3(blocks), dim3(256), smem, stream(), CT_SMALL_C_ARGS);
         else
-            conv2d_small_c_kernel<64><<<blocks, 256, smem, stream()>>>(CT_SMALL_C_ARGS);
+            (void)launch_dependent(conv2d_small_c_kernel<64>, dim3(blocks), dim3(256), smem, stream(), CT_SMALL_C_ARGS);
 #undef CT_SMALL_C_ARGS
         CT_LAUNCH_CHECK("conv2d_small_c");
         return CT_OK;
@@ -862,13 +872,13 @@ ct_status ct_maxpool2d(
     if (window == 2 && (w & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 &&
         (reinterpret_cast<uintptr_t>(out) & 7u) == 0)
         if (total / 2 + (int64_t)st->sm_count * 32 * 256 < 0x7fffffffll)
-            maxpool2x2_wide_kernel<uint32_t><<<capped_blocks(st, total / 2, 32), 256, 0, stream()>>>(x, n * c, h, w, ho, wo, out);
+            (void)launch_dependent(maxpool2x2_wide_kernel<uint32_t>, dim3(capped_blocks(st, total / 2, 32)), dim3(256), 0, stream(), x, n * c, h, w, ho, wo, out);
         else
-            maxpool2x2_wide_kernel<uint64_t><<<capped_blocks(st, total / 2, 32), 256, 0, stream()>>>(x, n * c, h, w, ho, wo, out);
+            (void)launch_dependent(maxpool2x2_wide_kernel<uint64_t>, dim3(capped_blocks(st, total / 2, 32)), dim3(256), 0, stream(), x, n * c, h, w, ho, wo, out);
     else if (window == 2 && (w & 1) == 0 && (reinterpret_cast<uintptr_t>(x) & 7u) == 0)
-        maxpool2x2_kernel<<<capped_blocks(st, total, 32), 256, 0, stream()>>>(x, n * c, h, w, ho, wo, out);
+        (void)launch_dependent(maxpool2x2_kernel, dim3(capped_blocks(st, total, 32)), dim3(256), 0, stream(), x, n * c, h, w, ho, wo, out);
     else
-        maxpool2d_kernel<<<capped_blocks(st, total, 32), 256, 0, stream()>>>(x, n * c, h, w, window, ho, wo, out);
+        (void)launch_dependent(maxpool2d_kernel, dim3(capped_blocks(st, total, 32)), dim3(256), 0, stream(), x, n * c, h, w, window, ho, wo, out);
     CT_LAUNCH_CHECK("maxpool2d");
     return CT_OK;
 }

@@ -196,6 +196,7 @@ template <bool RAW>
 __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
     const __grid_constant__ CUtensorMap map_x_hi, const __grid_constant__ CUtensorMap map_x_lo,
     const ConvTmemParams p, const int total_tiles) {
+    griddep_wait(); // no early successor: it could take the tensor memory that an image of wide range will need here
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t bar_full[4];
     __shared__ uint64_t bar_empty[4];
@@ -699,6 +700,8 @@ template <bool RAW>
 __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
     const __grid_constant__ CUtensorMap map_x_hi, const __grid_constant__ CUtensorMap map_x_lo,
     const __grid_constant__ ConvPairParams p, const int total_tiles) {
+    griddep_launch_dependents(); // the tf32 form, which allocates no tensor memory before this kernel ends
+    griddep_wait();
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t bar_full[kCP_MaxStages], bar_empty[kCP_MaxStages];
     __shared__ uint64_t bar_raw_full, bar_raw_empty;
@@ -1247,8 +1250,8 @@ ct_status conv_tmem_filters(
         cudaError_t launched;
         {
             ProfScope prof("gemm_tc");
-            conv_pairs_kernel<true><<<grid, kCP_Threads, pair_smem, stream()>>>(map, map, pp, (int)pair_tiles);
-            conv_tmem_filters_kernel<true><<<grid32, kTA_ThreadsRaw, smem32, stream()>>>(map32, map32, pt, (int)tiles);
+            (void)launch_dependent(conv_pairs_kernel<true>, dim3(grid), dim3(kCP_Threads), pair_smem, stream(), map, map, pp, (int)pair_tiles);
+            (void)launch_dependent(conv_tmem_filters_kernel<true>, dim3(grid32), dim3(kTA_ThreadsRaw), smem32, stream(), map32, map32, pt, (int)tiles);
             launched = cudaGetLastError();
         }
         CT_TRY(ct_free(ranges)); // in stream order, behind both
@@ -1287,9 +1290,9 @@ ct_status conv_tmem_filters(
     CT_TRY(encode32(&m32_hi, planes));
     CT_TRY(encode32(&m32_lo, planes + slot / 2));
     ProfScope prof("gemm_tc");
-    conv_pairs_kernel<false><<<grid, kCP_Threads, pair_smem, stream()>>>(m16_hi, m16_lo, pp, (int)pair_tiles);
+    (void)launch_dependent(conv_pairs_kernel<false>, dim3(grid), dim3(kCP_Threads), pair_smem, stream(), m16_hi, m16_lo, pp, (int)pair_tiles);
     CT_LAUNCH_CHECK("conv_pairs");
-    conv_tmem_filters_kernel<false><<<grid32, kTA_Threads, smem32, stream()>>>(m32_hi, m32_lo, pt, (int)tiles);
+    (void)launch_dependent(conv_tmem_filters_kernel<false>, dim3(grid32), dim3(kTA_Threads), smem32, stream(), m32_hi, m32_lo, pt, (int)tiles);
     CT_LAUNCH_CHECK("conv_tmem_filters");
     return CT_OK;
 }
