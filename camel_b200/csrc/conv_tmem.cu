@@ -1048,11 +1048,12 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                 if (p.pool) {
 #pragma unroll
                     for (int u = 0; u < 16; ++u) {
-                        // window order and strict '>' as in maxpool2d
+                        // window order and strict '>' as in maxpool2d, one after the other: the maximum of the lower row by itself
+                        // would lose its second element where the first is NaN
                         const float even1 = __shfl_down_sync(0xffffffffu, even[u], 1), odd1 = __shfl_down_sync(0xffffffffu, odd[u], 1);
                         even[u] = even1 > even[u] ? even1 : even[u];
-                        odd[u]  = odd1 > odd[u] ? odd1 : odd[u];
                         even[u] = odd[u] > even[u] ? odd[u] : even[u];
+                        even[u] = odd1 > even[u] ? odd1 : even[u];
                     }
                 }
                 float *at = dst;

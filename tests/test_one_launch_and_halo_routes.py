@@ -163,3 +163,23 @@ def test_elements_behind_the_last_vector(T, port, n):
     ta, tb = T.from_numpy(a), T.from_numpy(b)
     assert T.add(ta, tb).numpy().tobytes() == port.binary(oracle.ADD, a, b).tobytes()
     assert T.multiply(ta, tb).numpy().tobytes() == port.binary(oracle.MUL, a, b).tobytes()
+
+
+def test_fused_pool_takes_its_window_in_the_order_of_maxpool2d(T):
+    """A window (small, small, NaN, large): an output beyond the range of float32 is -infinity, which relu makes NaN, beside
+    finite ones.  The largest value behind the NaN counts, in the fused form as in the two steps."""
+    n, c, h, w, ko = 2, 32, 28, 32, 64
+    rng = np.random.default_rng(5)
+    x = rng.uniform(0.5, 1, (n, c, h, w)) * 2.0 ** 40
+    x[:, :, 1::2, 0::2], x[:, :, 1::2, 1::2] = -1.99 * 2.0 ** 60, 1.99 * 2.0 ** 60
+    f = np.zeros((ko, c, 1, 5))
+    f[:, :, 0, 0], f[:, :, 0, 1] = 1.9 * 2.0 ** 60, -1.9 * 2.0 ** 60  # lower rows: -+ 3.2e38 in turn
+    b = np.full(ko, -1e38)  # the negative ones leave the range, the positive ones are 2.2e38
+    tx, tf, tb = (T.from_numpy(v.astype(np.float32)) for v in (x, f, b))
+    full = T.conv2d(tx, tf, tb, 1, 0, "relu")
+    values = full.numpy()
+    assert np.isnan(values[:, :, 1::2, 0::2]).all() and (values[:, :, 1::2, 1::2] > 2e38).all()
+    fused = T.conv2d(tx, tf, tb, 1, 0, "relu", pool=2).numpy()
+    T.check_async()
+    assert fused.tobytes() == T.maxpool2d(full, 2).numpy().tobytes()
+    assert (fused > 2e38).all()
