@@ -945,7 +945,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                 for (int u = 0; u < kCP_CvtWarps; ++u)
                     range = range_join(range, cvt_range[i & 1][u]);
                 float scale, inverse;
-                const bool fits = half_range_fits(range, scale, inverse);
+                const bool fits = half_tile_fits(range, scale, inverse);
                 if (ct == 0) {
                     tile_scale[s]      = fits ? inverse : 0.0f;
                     p.tile_range[tile] = range;

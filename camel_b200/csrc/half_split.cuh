@@ -82,6 +82,14 @@ __device__ __forceinline__ bool half_range_fits(uint2 r, float &scale, float &in
     return ok && (r.y == kNoneSmallest || __uint_as_float(r.y + 1u) * scale >= kHalfExact);
 }
 
+// The same for a part of an image, by itself: true for every part of an image that fits.  A part may lie wholly below the smallest
+// exponent where its image does not (a scale of 2^74 holds all that an image that fits can have, 2^-86 and up), so it has
+// that scale and no floor of its own.
+__device__ __forceinline__ bool half_tile_fits(uint2 r, float &scale, float &inverse) {
+    half_scale(r.x, scale, inverse);
+    return r.x < (uint32_t)(kHalfMaxExponent + 128) << 23 && (r.y == kNoneSmallest || __uint_as_float(r.y + 1u) * scale >= kHalfExact);
+}
+
 __device__ __forceinline__ bool half_exception(float v, float scale) { return v != 0.0f && fabsf(v * scale) < kHalfSmallest; }
 
 // Returns true, and zeros, for an exception.

@@ -183,3 +183,27 @@ def test_fused_pool_takes_its_window_in_the_order_of_maxpool2d(T):
     T.check_async()
     assert fused.tobytes() == T.maxpool2d(full, 2).numpy().tobytes()
     assert (fused > 2e38).all()
+
+
+# the rows of the input that hold 2^-50, the others hold 2^-66: the image fits float16 pairs, tiles of its rows lie below 2^-60
+@pytest.mark.parametrize("rows", [(0, 14), (20, 28)])
+@pytest.mark.parametrize("pool", [0, 2])
+def test_tiles_below_the_smallest_exponent_of_an_image_that_fits(T, port, rows, pool):
+    from camel_b200._lib import check, lib
+
+    n, c, h, w, ko = 3, 32, 28, 28, 64
+    rng = np.random.default_rng(rows[0])
+    x = rng.uniform(0.5, 1, (n, c, h, w)) * rng.choice([-1, 1], (n, c, h, w))
+    x *= np.where((np.arange(h) >= rows[0]) & (np.arange(h) < rows[1]), 2.0 ** -50, 2.0 ** -66)[:, None]
+    x, f = x.astype(np.float32), rng.uniform(0.1, 1, (ko, c, 3, 3)).astype(np.float32)
+    want, size = port.conv2d(x, f, np.zeros(ko, np.float32), 1, 1, 0), port.conv2d(np.abs(x), f, np.zeros(ko, np.float32), 1, 1, 0)
+    side = h // 2 if pool else h
+    out = T.full((n, ko, side, side), 7.0)  # what a tile that nobody computes would keep
+    tx, tf = T.from_numpy(x), T.from_numpy(f)
+    check((lib.ct_conv2d_maxpool2 if pool else lib.ct_conv2d)(tx.ptr, tf.ptr, None, n, c, h, w, ko, 3, 3, 1, 1, 0, out.ptr))
+    got = out.numpy()
+    T.check_async()
+    if pool:
+        assert got.tobytes() == T.maxpool2d(T.conv2d(tx, tf, None, 1, 1, None), 2).numpy().tobytes()
+        want, size = (v.reshape(n, ko, side, 2, side, 2).max(axis=(3, 5)) for v in (want, size))
+    assert np.all(np.abs(got - want) <= BOUND * size)
