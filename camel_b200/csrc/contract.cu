@@ -758,8 +758,9 @@ static ct_status conv2d_run(
     // patch matrix is never materialised - each k-block is one shifted 4-D TMA box.
     const int th = (stride == 1 && c >= 16 && wo <= 256 && wd <= 0x7fffffff && h <= 0x7fffffff)
                        ? conv_tile_rows(ho, wo) : 0;
-    if ((th > 0 || c >= 8) && mode == 0 && conv_tmem_applicable(c, h, wd, ko, kh, kw, stride, pad)) {
-        // few channels on both sides: the filters stay in tensor memory, a tile's input is fetched once
+    if ((th > 0 || (c >= 8 && n <= 65535)) && mode == 0 && conv_tmem_applicable(c, h, wd, ko, kh, kw, stride, pad)) {
+        // few channels on both sides: the filters stay on chip, a tile's input is fetched once.  (Input that it cannot read as
+        // it is takes a pre-pass of at most 65,535 images; more of them go through patches where th is 0.)
         return conv_tmem_filters(st, x, w, bias, n, c, h, wd, ko, kh, kw, pad, act, pool, out);
     }
     if (mode == 0 && pool == 0 && conv2d_takes_halo(n, c, h, wd, ko, kh, kw, stride, pad))

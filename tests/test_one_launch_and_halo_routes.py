@@ -207,3 +207,17 @@ def test_tiles_below_the_smallest_exponent_of_an_image_that_fits(T, port, rows, 
         assert got.tobytes() == T.maxpool2d(T.conv2d(tx, tf, None, 1, 1, None), 2).numpy().tobytes()
         want, size = (v.reshape(n, ko, side, 2, side, 2).max(axis=(3, 5)) for v in (want, size))
     assert np.all(np.abs(got - want) <= BOUND * size)
+
+
+@pytest.mark.parametrize("layer", [(65540, 8, 8, 9, 16, 3, 3, 1, 1), (65540, 17, 8, 9, 16, 3, 3, 1, 1)])
+def test_more_images_than_a_pre_pass_takes(T, port, layer):
+    n, c, h, w, ko, kh, kw, stride, pad = layer
+    rng = np.random.default_rng(c)
+    x = rng.standard_normal((n, c, h, w), dtype=np.float32)
+    f, b = rng.standard_normal((ko, c, kh, kw)).astype(np.float32), rng.standard_normal(ko).astype(np.float32)
+    got = T.conv2d(T.from_numpy(x), T.from_numpy(f), T.from_numpy(b), stride, pad, "relu").numpy()
+    T.check_async()
+    some = np.r_[0:6, 65530:n]
+    want = port.conv2d(x[some], f, b, stride, pad, 1)
+    size = port.conv2d(np.abs(x[some]), np.abs(f), np.abs(b), stride, pad, 0)
+    assert np.all(np.abs(got[some] - want) <= BOUND * size)
