@@ -307,13 +307,19 @@ __global__ void __launch_bounds__(kGP_Threads, 1) gemm_panel_kernel(
     }
     __syncthreads(); // the list is complete
     if (warp >= 2) {
-        // what the sums lack, before their column scales: A's exceptions times B's planes, A times B's exceptions
+// What the sums lack, before their column scales: A's exceptions times B's planes, A times B's exceptions.  Both in order of
+        // k, whatever order the lists were filled in: that varies from run to run.
         const int row = quarter * 32 + lane, listed = listed_s < kGP_Listed ? listed_s : kGP_Listed;
-        for (int i = 0; i < listed; ++i) {
-            const PanelException x = list_s[i];
-            if (x.row != row)
-                continue;
+        for (int after = -1;;) {
+            int next = -1;
+            for (int i = 0; i < listed; ++i)
+                if (list_s[i].row == row && list_s[i].chunk_k > after && (next < 0 || list_s[i].chunk_k < list_s[next].chunk_k))
+                    next = i;
+            if (next < 0)
+                break;
+            const PanelException x = list_s[next];
             const int64_t kk = (int64_t)chunk0 * kGP_K + x.chunk_k;
+            after            = x.chunk_k;
 #pragma unroll 1
             for (int j = 0; j < 32 && cg * 32 + j < p.n; ++j) {
                 const int64_t at = (cg * 32 + j) * p.kp + kk;
@@ -324,16 +330,27 @@ __global__ void __launch_bounds__(kGP_Threads, 1) gemm_panel_kernel(
             }
         }
         const int listed_b = (int)p.exceptions_b->count;
-        for (int i = 0; i < listed_b; ++i) {
-            const HalfException x = p.exceptions_b->e[i];
-            const int64_t first = (int64_t)chunk0 * kGP_K;
-            const int col = x.line >> 1;
-            if (!(x.line & 1) || x.k < first || x.k >= first + (int64_t)chunks * kGP_K || col >> 5 != cg || row0 + row >= p.m)
-                continue;
-            const float add = __fmul_rn(p.a[(row0 + row) * p.k + x.k], x.value / fabsf(p.col_scale[col]));
+        const int64_t first = (int64_t)chunk0 * kGP_K, last = first + (int64_t)chunks * kGP_K;
+        for (int64_t after = first - 1;;) {
+            int64_t next = last;
+            for (int i = 0; i < listed_b; ++i) {
+                const HalfException x = p.exceptions_b->e[i];
+                if ((x.line & 1) && x.line >> 6 == cg && x.k > after && x.k < next)
+                    next = x.k;
+            }
+            if (next == last)
+                break;
+            after = next;
+            for (int i = 0; i < listed_b; ++i) { // a column each
+                const HalfException x = p.exceptions_b->e[i];
+                const int col = x.line >> 1;
+                if (!(x.line & 1) || x.line >> 6 != cg || x.k != next || row0 + row >= p.m)
+                    continue;
+                const float add = __fmul_rn(p.a[(row0 + row) * p.k + x.k], x.value / fabsf(p.col_scale[col]));
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-                acc[j] = (col & 31) == j ? __fadd_rn(acc[j], add) : acc[j];
+                for (int j = 0; j < 32; ++j)
+                    acc[j] = (col & 31) == j ? __fadd_rn(acc[j], add) : acc[j];
+            }
         }
     }
 

@@ -221,3 +221,41 @@ def test_more_images_than_a_pre_pass_takes(T, port, layer):
     want = port.conv2d(x[some], f, b, stride, pad, 1)
     size = port.conv2d(np.abs(x[some]), np.abs(f), np.abs(b), stride, pad, 0)
     assert np.all(np.abs(got[some] - want) <= BOUND * size)
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_tall_products_add_what_float16_pairs_cannot_hold_in_order_of_k(T, packed):
+    """Several such values in a column, from blocks of the pre-pass that finish in any order, and in a row.  The outputs that
+    consist of them alone are the float32 sums in order of k, to the bit."""
+    m, k, n, row, col = 3200, 4100, 100, 777, 41
+    rng = np.random.default_rng(11)
+    a, b = rng.uniform(-1, 1, (m, k)).astype(np.float32), (rng.integers(-255, 256, (k, n)) / 256).astype(np.float32)
+    meet = np.arange(128, 1024, 128)  # in the first slice of k; what keeps the scales of row and column meets zeros there
+    b[meet] = 0.0
+    a[row] = 0.0
+    a[row, meet] = 0.75
+    ks_a = np.sort(np.concatenate([meet[:4] + d for d in (1, 40, 127)]))
+    a[row, ks_a] = rng.uniform(1, 2, ks_a.size) * np.exp2(rng.integers(-40, -30, ks_a.size))
+    rows = np.arange(100, 110)
+    a[rows, 0] = 0.0
+    b[:, col], b[0, col] = 0.0, 0.75
+    ks_b = 66 * np.arange(1, 15)
+    b[ks_b, col] = rng.uniform(1, 2, ks_b.size) * np.exp2(rng.integers(-40, -30, ks_b.size))
+    ta, tb = T.from_numpy(a), T.from_numpy(b)
+    T.set_weight_cache(packed)
+    try:
+        outs = [T.dense(ta, tb).numpy() for _ in range(10)]
+    finally:
+        T.set_weight_cache(True)
+    T.check_async()
+    assert all(o.tobytes() == outs[0].tobytes() for o in outs)
+    for r in rows:
+        want = np.float32(0)
+        for kk in ks_b:
+            want = np.float32(want + np.float32(a[r, kk] * b[kk, col]))
+        assert outs[0][r, col] == want
+    others = np.delete(np.arange(n), col)
+    want = np.zeros(n - 1, np.float32)
+    for kk in ks_a:  # one rounding: the product and the sum fit 53 bits
+        want = (want.astype(np.float64) + a[row, kk].astype(np.float64) * b[kk, others].astype(np.float64)).astype(np.float32)
+    assert np.array_equal(outs[0][row, others], want)

@@ -193,9 +193,11 @@ def _with_exceptions(rng, m, k, n, count):
     return a, b, rows, cols
 
 
-# slices in a cluster; two passes over B; pairs; slices through the workspace; one wave of small tiles; more than a list holds
+# slices in a cluster; two passes over B; pairs; slices through the workspace; one wave of small tiles; more than a list holds;
+# a tall left operand split inside the product, in four slices and in two
 @pytest.mark.parametrize("m,k,n,count", [(128, 96, 200, 5), (300, 600, 300, 9), (600, 1500, 400, 12), (2600, 1100, 1500, 30),
-                                         (1290, 4700, 128, 7), (1000, 300, 1000, 20), (700, 1200, 800, 40)])
+                                         (1290, 4700, 128, 7), (1000, 300, 1000, 20), (700, 1200, 800, 40),
+                                         (3200, 4100, 100, 12), (6500, 2100, 100, 30)])
 @pytest.mark.parametrize("form", ["plain", "transposed", "weights", "rows"])
 def test_values_that_float16_pairs_cannot_hold_are_put_right(T, m, k, n, count, form):
     import ctypes as C
