@@ -312,7 +312,8 @@ __global__ void __launch_bounds__(kGD_Threads, 1) gemm_direct_kernel(const __gri
                         dst[q] = x[q];
             }
         }
-    if (threadIdx.x == 0 && !failed && !ok)
+    // every thread has waited by a clock of its own: one that gave up has kept the CTA from storing, whatever thread 0 saw
+    if (threadIdx.x == 0 && !failed && (!ok || *abort_flag))
         atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
 }
 
