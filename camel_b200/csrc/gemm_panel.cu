@@ -438,7 +438,7 @@ int panel_clusters(const DeviceState *st, int size) {
 // have the bytes of ct_matmul_packed_rows), which fill two thirds of the machine, and where A is most of the work.
 int panel_slices(const DeviceState *st, int64_t m, int64_t k, int64_t n) {
     const int64_t tiles = (m + 127) / 128;
-    if (n > 128 || k < 2048 || tiles * 2 > st->sm_count || tiles < 17) // fewer: more slices than a cluster has
+    if (n > 128 || k < 2048 || tiles * 2 > st->sm_count || st->sm_count / tiles > 8) // gemm_half, behind it, would use more slices than a cluster has
         return 0;
     int slices = 2;
     while (slices < 8 && tiles <= panel_clusters(st, slices * 2) && k >= slices * 2 * 1024)

@@ -279,9 +279,9 @@ __global__ void __launch_bounds__(256) split_transpose_small_kernel(
 // Errors are the caller's launch check's.
 template <int MODE>
 void launch_split_transpose(
-    const float *in, int64_t k, int64_t n, int64_t kp, void *hi, void *lo, int64_t batch = 1, int64_t in_batch_stride = 0,
+    int sm_count, const float *in, int64_t k, int64_t n, int64_t kp, void *hi, void *lo, int64_t batch = 1, int64_t in_batch_stride = 0,
     int64_t out_batch_stride = 0) {
-    if (((n + 63) / 64) * ((kp + 63) / 64) * batch < 2 * 148) {
+    if (((n + 63) / 64) * ((kp + 63) / 64) * batch < 2 * sm_count) {
         (void)launch_dependent(split_transpose_small_kernel<MODE>, dim3((unsigned)((n + 31) / 32), (unsigned)(kp / 32), (unsigned)batch),
                                dim3(256), 0, stream(), in, k, n, kp, hi, lo, in_batch_stride, out_batch_stride);
         return;
@@ -1709,9 +1709,9 @@ ct_status nhwc_planes(
         return fail(CT_ERR_TOO_LARGE, "conv2d: batch or channel count too large for the layout pre-pass");
     // per image: [c][hw] -> [hw][c_pad], i.e. the B-operand pre-pass of the GEMM with k = c, n = hw
     if (mode == MODE_3X)
-        launch_split_transpose<MODE_3X>(x, c, hw, c_pad, hi, lo, batch, c * hw, hw * c_pad);
+        launch_split_transpose<MODE_3X>(st->sm_count, x, c, hw, c_pad, hi, lo, batch, c * hw, hw * c_pad);
     else
-        launch_split_transpose<MODE_BF>(x, c, hw, c_pad, hi, lo, batch, c * hw, hw * c_pad);
+        launch_split_transpose<MODE_BF>(st->sm_count, x, c, hw, c_pad, hi, lo, batch, c * hw, hw * c_pad);
     CT_LAUNCH_CHECK("nhwc_planes");
     return CT_OK;
 }
@@ -1868,9 +1868,9 @@ ct_status gemm_f32_tc(
         if (kp / 32 > 65535)
             return fail(CT_ERR_TOO_LARGE, "gemm: k too large for the operand pre-pass");
         if (mode == MODE_3X)
-            launch_split_transpose<MODE_3X>(a, k, m, kp, a_hi, a_lo);
+            launch_split_transpose<MODE_3X>(st->sm_count, a, k, m, kp, a_hi, a_lo);
         else
-            launch_split_transpose<MODE_BF>(a, k, m, kp, a_hi, a_lo);
+            launch_split_transpose<MODE_BF>(st->sm_count, a, k, m, kp, a_hi, a_lo);
         CT_LAUNCH_CHECK("split_transpose");
     } else {
         ProfScope prof("gemm_prepass");
@@ -1881,9 +1881,9 @@ ct_status gemm_f32_tc(
         if (kp / 32 > 65535)
             return fail(CT_ERR_TOO_LARGE, "gemm: k too large for the operand pre-pass");
         if (mode == MODE_3X)
-            launch_split_transpose<MODE_3X>(b, k, n, kp, b_hi, b_lo);
+            launch_split_transpose<MODE_3X>(st->sm_count, b, k, n, kp, b_hi, b_lo);
         else
-            launch_split_transpose<MODE_BF>(b, k, n, kp, b_hi, b_lo);
+            launch_split_transpose<MODE_BF>(st->sm_count, b, k, n, kp, b_hi, b_lo);
         CT_LAUNCH_CHECK("split_transpose");
     }
 
@@ -1943,9 +1943,9 @@ extern "C" ct_status ct_weights_pack(const float *w, int64_t k, int64_t n, void 
     {
         ProfScope prof("weights_pack");
         if (mode == MODE_3X)
-            launch_split_transpose<MODE_3X>(w, k, n, kp, hi, lo);
+            launch_split_transpose<MODE_3X>(st->sm_count, w, k, n, kp, hi, lo);
         else
-            launch_split_transpose<MODE_BF>(w, k, n, kp, hi, lo);
+            launch_split_transpose<MODE_BF>(st->sm_count, w, k, n, kp, hi, lo);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
             ct_free(base);
@@ -2328,7 +2328,7 @@ extern "C" ct_status ct_matmul_f32_static(
             blocks = cap;
         split_rows_kernel<MODE_3X><<<(unsigned)blocks, 256, 0, stream()>>>(a_dev, m, k, kp, a_hi, a_lo);
         CT_LAUNCH_CHECK("split_rows(static scratch)");
-        launch_split_transpose<MODE_3X>(b_dev, k, n, kp, b_hi, b_lo);
+        launch_split_transpose<MODE_3X>(s->sm_count, b_dev, k, n, kp, b_hi, b_lo);
         CT_LAUNCH_CHECK("split_transpose(static scratch)");
     }
     int64_t tiles256 = ((m + BM - 1) / BM) * ((n + 255) / 256);
