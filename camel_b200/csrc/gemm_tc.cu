@@ -195,12 +195,11 @@ __global__ void __launch_bounds__(256) split_rows_vec_kernel(
     }
 }
 
-// in [k][n] row-major  ->  transposed planes [n][kp].  Blocks of 64 x 64 through shared memory, 16 bytes of a column's k to
-// a store: 8192 x 8192 to bfloat16 101 us, with 32 x 32 blocks and 2-byte stores 153.
-template <int MODE>
-__global__ void __launch_bounds__(256) split_transpose_kernel(
-    const float *__restrict__ in, int64_t k, int64_t n, int64_t kp, void *__restrict__ p_hi,
-    void *__restrict__ p_lo, int vec_ok, int64_t in_batch_stride, int64_t out_batch_stride) {
+// in [k][n] row-major  ->  a transposed bfloat16 plane [n][kp].  Blocks of 64 x 64 through shared memory, 16 bytes of a column's k
+// to a store: 8192 x 8192 101 us, with 32 x 32 blocks and 2-byte stores 153.
+__global__ void __launch_bounds__(256) split_transpose_bf_kernel(
+    const float *__restrict__ in, int64_t k, int64_t n, int64_t kp, __nv_bfloat16 *__restrict__ plane, int vec_ok,
+    int64_t in_batch_stride, int64_t out_batch_stride) {
     __shared__ float tile[64][65];
     griddep_launch_dependents();
     griddep_wait();
@@ -215,31 +214,19 @@ __global__ void __launch_bounds__(256) split_transpose_kernel(
         const int col = (threadIdx.x >> 3) + 32 * j, kk = (threadIdx.x & 7) * 8;
         if (n0 + col >= n || k0 + kk >= kp)
             continue;
-        const int64_t at = out_base + (n0 + col) * kp + k0 + kk;
-        if (MODE == MODE_3X) {
+        __nv_bfloat162 v[4];
 #pragma unroll
-            for (int h = 0; h < 8; h += 4) {
-                float hi[4], lo[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    split_tf32(tile[kk + h + u][col], hi[u], lo[u]);
-                *reinterpret_cast<float4 *>(static_cast<float *>(p_hi) + at + h) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<float4 *>(static_cast<float *>(p_lo) + at + h) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-            }
-        } else {
-            __nv_bfloat162 v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                v[u] = __floats2bfloat162_rn(tile[kk + 2 * u][col], tile[kk + 2 * u + 1][col]);
-            *reinterpret_cast<uint4 *>(static_cast<__nv_bfloat16 *>(p_hi) + at) = *reinterpret_cast<uint4 *>(v);
-        }
+        for (int u = 0; u < 4; ++u)
+            v[u] = __floats2bfloat162_rn(tile[kk + 2 * u][col], tile[kk + 2 * u + 1][col]);
+        *reinterpret_cast<uint4 *>(plane + out_base + (n0 + col) * kp + k0 + kk) = *reinterpret_cast<uint4 *>(v);
     }
 }
 
-// The same in blocks of 32 x 32, for operands that give the blocks above less than two to an SM: 582 x 2210 x 107 30 us, with
-// the larger ones 35; 8192 x 8192 goes the other way, 153 us against 101.
+// in [k][n] row-major  ->  transposed planes [n][kp], in blocks of 32 x 32: bfloat16 where the blocks above would be fewer than two
+// to an SM (582 x 2210 x 107 30 us, with the larger ones 35), and tf32 terms always, whose stores are whole lines here too: the product
+// of 121 x 12306 x 1643 108 us, with blocks of 64 x 64 122, 100 x 16000 x 9000 555 and 640.
 template <int MODE>
-__global__ void __launch_bounds__(256) split_transpose_small_kernel(
+__global__ void __launch_bounds__(256) split_transpose_kernel(
     const float *__restrict__ in, int64_t k, int64_t n, int64_t kp, void *__restrict__ p_hi,
     void *__restrict__ p_lo, int64_t in_batch_stride, int64_t out_batch_stride) {
     __shared__ float tile[32][33];
@@ -281,14 +268,14 @@ template <int MODE>
 void launch_split_transpose(
     int sm_count, const float *in, int64_t k, int64_t n, int64_t kp, void *hi, void *lo, int64_t batch = 1, int64_t in_batch_stride = 0,
     int64_t out_batch_stride = 0) {
-    if (((n + 63) / 64) * ((kp + 63) / 64) * batch < 2 * sm_count) {
-        (void)launch_dependent(split_transpose_small_kernel<MODE>, dim3((unsigned)((n + 31) / 32), (unsigned)(kp / 32), (unsigned)batch),
+    if (MODE == MODE_3X || ((n + 63) / 64) * ((kp + 63) / 64) * batch < 2 * sm_count) {
+        (void)launch_dependent(split_transpose_kernel<MODE>, dim3((unsigned)((n + 31) / 32), (unsigned)(kp / 32), (unsigned)batch),
                                dim3(256), 0, stream(), in, k, n, kp, hi, lo, in_batch_stride, out_batch_stride);
         return;
     }
     const int vec = (n & 3) == 0 && (in_batch_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
-    (void)launch_dependent(split_transpose_kernel<MODE>, dim3((unsigned)((n + 63) / 64), (unsigned)((kp + 63) / 64), (unsigned)batch),
-                           dim3(256), 0, stream(), in, k, n, kp, hi, lo, vec, in_batch_stride, out_batch_stride);
+    (void)launch_dependent(split_transpose_bf_kernel, dim3((unsigned)((n + 63) / 64), (unsigned)((kp + 63) / 64), (unsigned)batch),
+                           dim3(256), 0, stream(), in, k, n, kp, static_cast<__nv_bfloat16 *>(hi), vec, in_batch_stride, out_batch_stride);
 }
 
 // ---- main kernel ------------------------------------------------------------------------
