@@ -130,8 +130,8 @@ __device__ __forceinline__ uint8_t apply_compare_d(int op, double a, double b) {
 // Generic driver: out[i] = f(i-th elements).  VEC=true: all pointers are vector-aligned and
 // the body covers numel/4 vectors; the tail (and the unaligned case) runs with VEC=false.
 template <bool VEC, typename F> __global__ void __launch_bounds__(kThreads) map_kernel(uint64_t count, F f) {
-    griddep_launch_dependents();
     griddep_wait();
+    griddep_launch_dependents();
     uint64_t base = (uint64_t)blockIdx.x * (kThreads * kUnroll) + threadIdx.x;
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
@@ -145,8 +145,8 @@ template <bool VEC, typename F> __global__ void __launch_bounds__(kThreads) map_
 // 100,000 elements.
 template <typename F, typename T>
 __global__ void __launch_bounds__(kThreads) map_tail_kernel(uint64_t count, F f, uint64_t tail, T t) {
-    griddep_launch_dependents();
     griddep_wait();
+    griddep_launch_dependents();
     uint64_t base = (uint64_t)blockIdx.x * (kThreads * kUnroll) + threadIdx.x;
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {

@@ -666,8 +666,8 @@ template <int NMAX, int R>
 __global__ void __launch_bounds__(kTnMaxThreads, 2) gemm_tn_skinny_kernel(
     const float *__restrict__ a_km, const float *__restrict__ b, int64_t m, int64_t k, int n, int64_t k_per_slice,
     double *__restrict__ partial) {
-    griddep_launch_dependents();
     griddep_wait();
+    griddep_launch_dependents();
     constexpr int G  = kTnGroup;
     constexpr int BL = (kTnChunk * NMAX + kTnMinThreads - 1) / kTnMinThreads; // staged b values per thread
     __shared__ __align__(16) double bs[2][kTnChunk][NMAX];
@@ -794,8 +794,8 @@ __global__ void __launch_bounds__(kTnMaxThreads, 2) gemm_tn_skinny_kernel(
 // sums are added in a fixed butterfly - the same order on every run.
 __global__ void __launch_bounds__(256) gemm_tn_skinny_finish_kernel(
     const double *__restrict__ partial, int64_t mn, int slices, float *__restrict__ out) {
-    griddep_launch_dependents();
     griddep_wait();
+    griddep_launch_dependents();
     const int lane  = threadIdx.x & 31;
     const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 5;
     if (i >= mn)
@@ -841,8 +841,13 @@ static ct_status launch_tn_skinny(
     CT_TRY(ensure_ws(&st->splitk_ws, &st->splitk_ws_bytes, (size_t)slices * m * n * sizeof(double)));
     auto *partial = static_cast<double *>(st->splitk_ws);
     dim3 grid((unsigned)mblocks, (unsigned)slices);
-    // both start while their predecessor ends: one update of 60000 x 785 x 10 175.4 -> 173.6 us, of 1710 x 181 x 4 20.2 -> 18.6
-    (void)launch_dependent(gemm_tn_skinny_kernel<NMAX, R>, dim3(grid), dim3(threads), 0, stream(), a_km, b, m, k, n, k_per_slice, partial);
+    // Both start while their predecessor ends (9018 x 1088 x 10 62.5 -> 60.3 us with what precedes and follows it, 878 x 854 x 8
+    // 23.8 -> 21.5), but for many small blocks with several chunks each: those crowd on the SMs that are free first (one update
+    // of 96854 x 191 x 16 178, started on an idle machine 169; 33930 x 76 x 4 38 and 33).
+    if (threads > kTnMinThreads || k_per_slice == kTnChunk)
+        (void)launch_dependent(gemm_tn_skinny_kernel<NMAX, R>, grid, dim3(threads), 0, stream(), a_km, b, m, k, n, k_per_slice, partial);
+    else
+        gemm_tn_skinny_kernel<NMAX, R><<<grid, threads, 0, stream()>>>(a_km, b, m, k, n, k_per_slice, partial);
     CT_LAUNCH_CHECK("gemm_tn_skinny");
     const int64_t mn = m * n;
     (void)launch_dependent(gemm_tn_skinny_finish_kernel, dim3((unsigned)((mn * 32 + 255) / 256)), dim3(256), 0, stream(), partial, mn, (int)slices, out);
