@@ -658,7 +658,12 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
 // whole launch, hi terms before lo terms for each tap.  Per 16 channels and tap two MMAs an accumulator:
 //     [main | cross] += X_hi x [W_hi; W_lo]     N = 2 kop
 //             cross  += X_lo x W_hi             N = kop
-// with the low terms stored 2^11 times larger and the cross products in columns of their own, as in gemm_half.cu.
+// with the low terms stored 2^11 times larger and the cross products in columns of their own, as in gemm_half.cu.  The product of
+// two low terms (2^-24 of a product) is left out: it would be half as much work again (256 x 32 x 28 x 28 -> 64 44 us, with it 54).
+// What errs most are the additions, which truncate.  So the leading product of the last k-step does not join the others': when all
+// cross products are in, this MMA moves their columns down by 2^11, by the scale of its D, and adds to them, and the chain
+// is a step shorter (256 x 32 x 28 x 28 -> 64 44.2 -> 44.9 us).  That makes up for the product of the low terms: against 64 bits
+// 3.66e-7 -> 3.39e-7, with them 3.64e-7; 16 channels 2.19e-7 -> 1.93e-7.
 //
 // Why so.  With the filters on the rows and in tensor memory (hi and lo terms on rows 0 - 63 and 64 - 127, the layout of the
 // tf32 form above) the two halves of an output met in shared memory, 128 KB a tile of 128 positions, and that epilogue
@@ -847,6 +852,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
             const uint64_t filter0 = smem_desc_k<kCP_RowB>(smem_base), lo_terms = (uint64_t)(2 * region >> 4);
             const uint64_t filter_step = (uint64_t)(2 * p.kop * kCP_RowB >> 4);
             const uint32_t kop = (uint32_t)p.kop;
+            const uint64_t w_lo = (uint64_t)(p.kop * kCP_RowB >> 4);
             int i   = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
@@ -868,7 +874,8 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                     // the tap's pixels for the even and the odd output rows
                     uint64_t even = smem_desc_k<kCP_RowB>(hi0 + (uint32_t)(r & 1) * region + (uint32_t)((r >> 1) * p.pw * kCP_RowB));
                     uint64_t odd  = smem_desc_k<kCP_RowB>(hi0 + (uint32_t)((r + 1) & 1) * region + (uint32_t)(((r + 1) >> 1) * p.pw * kCP_RowB));
-                    for (int sx = 0; sx < p.kw; ++sx, even += kCP_RowB >> 4, odd += kCP_RowB >> 4, db += filter_step) {
+                    const int taps = r + 1 < rows ? p.kw : p.kw - 1; // all but the last
+                    for (int sx = 0; sx < taps; ++sx, even += kCP_RowB >> 4, odd += kCP_RowB >> 4, db += filter_step) {
                         mma_f16(d_even, even, db, idesc2, accumulate);
                         mma_f16(d_odd, odd, db, idesc2, accumulate);
                         mma_f16(d_even + kop, even + lo_terms, db, idesc1, 1u);
@@ -880,6 +887,21 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                             mma_f16(d_even + kop, even + lo_terms + 2, db + 2, idesc1, 1u);
                             mma_f16(d_odd + kop, odd + lo_terms + 2, db + 2, idesc1, 1u);
                         }
+                    }
+                    if (r + 1 == rows) {
+                        if (two) {
+                            mma_f16(d_even, even, db, idesc2, 1u);
+                            mma_f16(d_odd, odd, db, idesc2, 1u);
+                            mma_f16(d_even + kop, even + lo_terms, db, idesc1, 1u);
+                            mma_f16(d_odd + kop, odd + lo_terms, db, idesc1, 1u);
+                            even += 2, odd += 2, db += 2;
+                        }
+                        mma_f16(d_even + kop, even + lo_terms, db, idesc1, 1u);
+                        mma_f16(d_odd + kop, odd + lo_terms, db, idesc1, 1u);
+                        mma_f16(d_even + kop, even, db + w_lo, idesc1, 1u);
+                        mma_f16(d_odd + kop, odd, db + w_lo, idesc1, 1u);
+                        mma_f16_shifted<kHalfLoBits>(d_even + kop, even, db, idesc1);
+                        mma_f16_shifted<kHalfLoBits>(d_odd + kop, odd, db, idesc1);
                     }
                 }
                 tc_commit(smem_u32(&bar_empty[s]));      // the stage is free once these MMAs have retired
@@ -1036,7 +1058,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             auto value = [&](uint32_t main, uint32_t cross) { // the products with powers of two are exact
-                                float v = __fmaf_rn(__uint_as_float(cross), kHalfLoInv, __uint_as_float(main));
+                                float v = __fadd_rn(__uint_as_float(main), __uint_as_float(cross));
                                 v       = __fadd_rn(__fmul_rn(v, fs[q]), bs[q]);
                                 return !relu || v > 0.0f ? v : __fmul_rn(v, 0.0f);
                             };
@@ -1137,7 +1159,7 @@ static bool conv_pair_plan(
     p.pw  = (int)(wd + 2 * pad);
     p.wo  = p.pw - (int)kw + 1;
     p.ho  = (int)(h + 2 * pad - kh + 1);
-    if (p.pw > 128 || p.wo < 1 || p.ho < 1)
+    if (p.pw > 128 || p.wo < 1 || p.ho < 1 || kh * kw < 2) // one tap would leave the leading columns empty
         return false;
     p.jp          = std::min(128 / p.pw, (p.ho + 1) / 2);
     p.tiles_y     = ((p.ho + 1) / 2 + p.jp - 1) / p.jp;

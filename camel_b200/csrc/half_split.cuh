@@ -25,6 +25,7 @@
 
 namespace ct {
 
+constexpr int kHalfLoBits       = 11;
 constexpr float kHalfLoScale    = 2048.0f;              // 2^11
 constexpr float kHalfLoInv      = 1.0f / 2048.0f;
 constexpr float kHalfSmallest   = 1.0f / (1u << 13);    // scaled magnitudes below this are exceptions

@@ -230,6 +230,20 @@ __device__ __forceinline__ void mma_f16(
         : "memory");
 }
 
+// D = A . B + D * 2^-SHIFT (0 .. 15)
+template <int SHIFT>
+__device__ __forceinline__ void mma_f16_shifted(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.ne.b32 p, 1, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %4;\n\t"
+        "}\n"
+        :
+        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(SHIFT)
+        : "memory");
+}
+
 // ---- CTA pairs (clusters of two CTAs that work on one 256-row tile) ----------------------------
 //
 // With cta_group::2 one thread of the leader (rank 0) issues MMAs of 256 rows: each CTA of the pair holds
