@@ -675,17 +675,30 @@ ct_status ct_conv2d_maxpool2(
     bool tmem_pool         = false;
     const bool tmem_kernel = kblock == 32 && conv_tmem_applicable(c, h, wd, ko, kh, kw, stride, pad, &tmem_pool);
     const bool halo_kernel = kblock == 32 && conv2d_takes_halo(n, c, h, wd, ko, kh, kw, stride, pad);
-    const bool fused = tensor_core && !halo_kernel && stride == 1 && c >= 16 && (wo & 1) == 0 && (ho & 1) == 0 && conv_tile_rows(ho, wo) > 0 &&
-                       n > 0 && (tmem_kernel ? tmem_pool : swap_kernel);
-    if (fused)
+    const bool fusable = tensor_core && stride == 1 && c >= 16 && (wo & 1) == 0 && (ho & 1) == 0 && conv_tile_rows(ho, wo) > 0 &&
+                         n > 0 && (tmem_kernel ? tmem_pool : swap_kernel);
+    if (fusable && !halo_kernel)
         return conv2d_run(x, w, bias, n, c, h, wd, ko, kh, kw, stride, pad, act, out, 2);
-    // not a shape of the fused kernel: the convolution into a temporary, then maxpool2d
+    // The convolution into a temporary, then maxpool2d.  For layers that the pixels-on-rows kernel could pool in its epilogue the halo
+    // kernel is the faster one all the same, in most cases (64 x 64 x 56 x 56 -> 64 171 us fused, 130 so; 256 x 33 x 14 x 14 -> 17
+    // 66 and 46; not with 16 x 16 outputs, two tiles of 14 rows and 2, 1024 x 64 x 16 x 16 -> 64 189 and 223), but they take no more
+    // than 256 MB for it: the batch goes in parts, which the images of that kernel, each with a scale of its own, do not notice.
+    int64_t part = n;
+    if (fusable) {
+        const int64_t most = std::max<int64_t>(1, (256ll << 20) / (ko * ho * wo * (int64_t)sizeof(float)));
+        const int64_t parts = (n + most - 1) / most;
+        part = (n + parts - 1) / parts;
+    }
     void *tmp      = nullptr;
-    size_t bytes   = (size_t)(n * ko * ho * wo > 0 ? n * ko * ho * wo : 1) * sizeof(float);
+    size_t bytes   = (size_t)(part * ko * ho * wo > 0 ? part * ko * ho * wo : 1) * sizeof(float);
     CT_TRY(ct_alloc(&tmp, bytes));
-    ct_status s = conv2d_run(x, w, bias, n, c, h, wd, ko, kh, kw, stride, pad, act, static_cast<float *>(tmp), 0);
-    if (s == CT_OK)
-        s = ct_maxpool2d(static_cast<const float *>(tmp), n, ko, ho, wo, 2, out);
+    ct_status s = CT_OK;
+    for (int64_t at = 0; s == CT_OK && (at == 0 || at < n); at += part) {
+        const int64_t images = std::min(part, n - at);
+        s = conv2d_run(x + at * c * h * wd, w, bias, images, c, h, wd, ko, kh, kw, stride, pad, act, static_cast<float *>(tmp), 0);
+        if (s == CT_OK)
+            s = ct_maxpool2d(static_cast<const float *>(tmp), images, ko, ho, wo, 2, out + at * ko * (ho / 2) * (wo / 2));
+    }
     ct_status f = ct_free(tmp);
     return s != CT_OK ? s : f;
 }

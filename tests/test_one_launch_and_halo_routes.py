@@ -259,3 +259,18 @@ def test_tall_products_add_what_float16_pairs_cannot_hold_in_order_of_k(T, packe
     for kk in ks_a:  # one rounding: the product and the sum fit 53 bits
         want = (want.astype(np.float64) + a[row, kk].astype(np.float64) * b[kk, others].astype(np.float64)).astype(np.float32)
     assert np.array_equal(outs[0][row, others], want)
+
+
+def test_pooled_layer_in_parts_of_the_batch(T):
+    """More than 256 MB of activations: three parts of 190, 190 and 188 images, the bytes of the two steps over the whole batch.
+    Images of wide range, which decide for themselves, lie on both sides of the cuts."""
+    n, c, h, w, ko = 568, 33, 64, 64, 64
+    rng = np.random.default_rng(8)
+    x = rng.standard_normal((n, c, h, w), dtype=np.float32)
+    x[[0, 189, 190, 380, 567], 5, 30, 20] = 1e-20
+    f, b = (rng.standard_normal((ko, c, 3, 3)) / 17).astype(np.float32), rng.standard_normal(ko).astype(np.float32)
+    tx, tf, tb = T.from_numpy(x), T.from_numpy(f), T.from_numpy(b)
+    fused = T.conv2d(tx, tf, tb, 1, 1, "relu", pool=2).numpy()
+    full = T.conv2d(tx, tf, tb, 1, 1, "relu")
+    T.check_async()
+    assert full.nbytes > 2 * (256 << 20) and fused.tobytes() == T.maxpool2d(full, 2).numpy().tobytes()
