@@ -706,7 +706,9 @@ def test_dlpack_zero_copy_with_torch(T):
     assert mask.dtype == 2 and mask.numpy().astype(np.uint8).tolist() == [1, 0, 1]
 
 
-def test_dense_packed_weights(T):
+# in float32: one launch, which reads the weights themselves; one slice of k; several
+@pytest.mark.parametrize("m,k,n", [(300, 200, 150), (300, 190, 150), (1200, 1100, 500)])
+def test_dense_packed_weights(T, m, k, n):
     """The tensor-core layout of a weight tensor is built once and kept with the tensor: same bytes
     as the per-call pre-pass, in both precisions; a handle from another matrix is refused."""
     import ctypes as C
@@ -715,9 +717,9 @@ def test_dense_packed_weights(T):
     from camel_b200._lib import check, lib
 
     rng = np.random.default_rng(21)
-    x = T.from_numpy(rng.uniform(0, 1, (300, 200)).astype(np.float32))
-    w_np = rng.uniform(-0.1, 0.1, (200, 150)).astype(np.float32)
-    b = T.from_numpy(rng.uniform(-0.1, 0.1, 150).astype(np.float32))
+    x = T.from_numpy(rng.uniform(0, 1, (m, k)).astype(np.float32))
+    w_np = rng.uniform(-0.1, 0.1, (k, n)).astype(np.float32)
+    b = T.from_numpy(rng.uniform(-0.1, 0.1, n).astype(np.float32))
     for prec in (camel_b200._lib.PREC_3XTF32, camel_b200._lib.PREC_BF16):
         check(lib.ct_set_precision(prec))
         try:
@@ -736,9 +738,9 @@ def test_dense_packed_weights(T):
             check(lib.ct_set_precision(camel_b200._lib.PREC_3XTF32))
             T.set_weight_cache(True)
     other = T.from_numpy(w_np)
-    out = T.Tensor(0, (300, 150))
+    out = T.Tensor(0, (m, n))
     with pytest.raises(camel_b200.CamelTensorError, match="packed weights"):
-        check(lib.ct_dense_packed(x.ptr, other.ptr, w3x._packed[camel_b200._lib.PREC_3XTF32], None, 300, 200, 150, 0,
+        check(lib.ct_dense_packed(x.ptr, other.ptr, w3x._packed[camel_b200._lib.PREC_3XTF32], None, m, k, n, 0,
                                   out.ptr, None))
     h = C.c_void_p()
     with pytest.raises(camel_b200.CamelTensorError):

@@ -32,11 +32,12 @@ def port():
 # n, c, h, w, ko, kh, kw, stride, pad.  Halo kernel: odd extents at strides 2 and 3 (sub-images of unequal size); taps that
 # leave sub-images unread; half of a channel block, and one channel more; k of two and three drains (c = 97, 193 with
 # nine taps; 33 with twenty-five); 17 and 129 filters; a tile of one row; partial last tiles.  Paired rows: an odd number of
-# rows, a row of 128 positions, 16 and 64 filters, 8 channels, an even filter, rows that no tensor map covers.
+# rows, a row of 128 positions, 16 and 64 filters, 8 channels, an even filter, rows that no tensor map covers.  Halo again: more
+# filters than have their bias in shared memory.
 LAYERS = [(2, 48, 57, 57, 96, 3, 3, 2, 1), (1, 33, 20, 23, 70, 3, 3, 3, 1), (2, 40, 30, 33, 64, 1, 1, 2, 0), (1, 16, 41, 40, 65, 5, 5, 2, 2),
           (1, 97, 17, 30, 17, 3, 3, 1, 1), (1, 193, 15, 30, 129, 3, 3, 1, 0), (1, 33, 40, 61, 40, 5, 5, 1, 2), (1, 17, 20, 130, 80, 3, 3, 1, 1),
           (2, 9, 33, 64, 80, 3, 3, 1, 1), (2, 32, 28, 28, 64, 3, 3, 1, 1), (1, 8, 27, 33, 16, 3, 3, 1, 1), (1, 20, 16, 126, 33, 3, 3, 1, 1),
-          (1, 31, 30, 29, 48, 2, 2, 1, 0), (1, 17, 12, 60, 17, 1, 5, 1, 0)]
+          (1, 31, 30, 29, 48, 2, 2, 1, 0), (1, 17, 12, 60, 17, 1, 5, 1, 0), (1, 40, 20, 30, 300, 3, 3, 1, 1)]
 
 
 @pytest.mark.parametrize("layer", LAYERS)
@@ -84,9 +85,9 @@ def test_small_products_in_one_launch(T, m, k, n, kind):
     assert np.all(np.abs(got[finite] - want[finite]) <= BOUND * size[finite])
 
 
-# one tile of columns: chunks of 128 values of k that end ragged, slices of unequal length, rows that are not 16-byte aligned, and
-# operands that are left to the product from planes
-@pytest.mark.parametrize("m,k,n", [(3300, 2100, 100), (4200, 4099, 128), (6500, 2050, 33)])
+# one tile of columns: chunks of 128 values of k that end ragged, slices of unequal length, rows that are 16-byte aligned and rows that are
+# not, and operands that are left to the product from planes; the first has too few tiles for it
+@pytest.mark.parametrize("m,k,n", [(3300, 2100, 100), (4200, 4099, 128), (6500, 2050, 33), (6500, 2100, 100), (4200, 4100, 128)])
 @pytest.mark.parametrize("kind", ["plain", "small value in A", "small value in B", "infinity", "ninety powers of two"])
 def test_tall_products_with_one_tile_of_columns(T, m, k, n, kind):
     rng = np.random.default_rng(m + k + n)
@@ -109,6 +110,40 @@ def test_tall_products_with_one_tile_of_columns(T, m, k, n, kind):
     assert np.array_equal(np.isfinite(got), finite)
     size = np.abs(np.where(np.isfinite(a), a, 0)).astype(np.float64) @ np.abs(b).astype(np.float64)
     assert np.all(np.abs(got[finite] - want[finite]) <= BOUND * size[finite])
+
+
+# the same as layers, with bias and relu, from the weights and from packed ones: panel product, the three launches behind it, and
+# two that prepare the weights where they are not packed
+@pytest.mark.parametrize("m,k,n", [(6500, 2100, 100), (4200, 4100, 128), (4200, 4099, 128), (6500, 2050, 33)])
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("kind", ["plain", "small values", "infinity"])
+def test_tall_layers_with_one_tile_of_columns(T, m, k, n, packed, kind):
+    from camel_b200._lib import lib
+
+    rng = np.random.default_rng(m + k + n)
+    a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    w = rng.uniform(-1, 1, (k, n)).astype(np.float32)
+    b = rng.uniform(-1, 1, n).astype(np.float32)
+    if kind == "small values":
+        a[m // 2, k // 3], w[k // 2, n // 3] = 1e-20, 1e-25
+    if kind == "infinity":
+        a[m - 1, k - 1] = np.inf
+    ta, tw, tb = T.from_numpy(a), T.from_numpy(w), T.from_numpy(b)
+    T.set_weight_cache(packed)
+    try:
+        first = T.dense(ta, tw, tb, "relu").numpy()
+        launches = lib.ct_launch_count()
+        got = T.dense(ta, tw, tb, "relu")
+        launches = lib.ct_launch_count() - launches
+        got = got.numpy()
+    finally:
+        T.set_weight_cache(True)
+    T.check_async()
+    assert launches == (4 if packed else 6) and got.tobytes() == first.tobytes()
+    rows = np.isfinite(a).all(axis=1)
+    a64, w64 = a[rows].astype(np.float64), w.astype(np.float64)
+    assert np.all(np.abs(got[rows] - np.maximum(a64 @ w64 + b, 0.0)) <= BOUND * (np.abs(a64) @ np.abs(w64) + np.abs(b)))
+    assert not np.isfinite(got[~rows]).any()
 
 
 # rows of the result that begin anywhere in a line, one tile to a pair: a last tile of one, 33 and 129 columns, whole last tiles, rows
