@@ -630,14 +630,17 @@ static int pooled_tile_rows(int64_t ho, int64_t wo) {
 // has one use for a halo: up to 64 filters or 32 channels the other kernels are as fast or faster (88 x 95 x 29 x 32 -> 22
 // 46 us against 50, 19 x 18 x 60 x 63 -> 115 145 against 149), and a strided one reads a quarter of the planes (11 x 161 x 52 x 54 -> 37 27 against 33).
 // Below some 16,000 outputs per filter a strided layer's three launches cost more than its patches (7 x 17 x 69 x 72 -> 74
-// 24 against 28, 14 x 14 x 38 x 38 -> 22 26 against 31; 60 x 15 x 41 x 41 -> 27 34 both ways, 64 x 34 x 40 x 42 -> 78 45 against 41).
+// 24 against 28, 14 x 14 x 38 x 38 -> 22 26 against 31; 60 x 15 x 41 x 41 -> 27 34 both ways, 64 x 34 x 40 x 42 -> 78 45 against 41),
+// and below some 8,000 those of a layer of less than half a block of channels (4 x 8 x 38 x 40 -> 64, 5 x 5, 22 against 26, 4 x 8 x 40 x 40
+// -> 96 19 against 21; 9 x 10 x 39 x 42 -> 21, 5 x 5, 30 against 28, 16 x 8 x 40 x 40 -> 96 32 against 23).
 static bool conv2d_takes_halo(
     int64_t n, int64_t c, int64_t h, int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t stride, int64_t pad) {
     if (c < 8 || n > 65535 || conv_tmem_applicable(c, h, wd, ko, kh, kw, stride, pad))
         return false;
     if (kh * kw == 1 && (ko <= 64 || c <= 32 || stride > 1))
         return false;
-    if (stride > 1 && n * ((h + 2 * pad - kh) / stride + 1) * ((wd + 2 * pad - kw) / stride + 1) < 16384)
+    const int64_t least = stride > 1 ? 16384 : (c < 16 ? 8192 : 0);
+    if (n * ((h + 2 * pad - kh) / stride + 1) * ((wd + 2 * pad - kw) / stride + 1) < least)
         return false;
     return conv_halo_applicable((c + 31) / 32 * 32, h, wd, ko, kh, kw, stride, pad);
 }
