@@ -21,7 +21,7 @@
 //
 // Strides: the rows and columns of the input that are alike modulo the stride are sub-images of the planes, and a tap is a
 // shift inside one of them, so a strided layer is the same loop with a halo per sub-image; its patches are never written
-// (64 x 48 x 57 x 57 -> 96 at stride 2: 121 us through a patch matrix, 77 so).  Longer k than 1024: the leading
+// (64 x 48 x 57 x 57 -> 96 at stride 2: 121 us through a patch matrix, 70 so).  Longer k than 1024: the leading
 // accumulator is drained every 1024 values, as in gemm_half.cu.  The channel blocks are taken last to first: additions into an
 // accumulator truncate, and those of a block that is mostly padding cost least while the sums are small (45 x 33 x 64 x 64 -> 35
 // 6.0e-7 -> 4.0e-7 against 64 bits, 49 channels 7.5e-7 -> 6.2e-7, the same time).

@@ -675,7 +675,10 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
 // image.  The converting warps also leave the range of every tile in the call's own scratch; conv_tmem_filters_kernel,
 // launched behind this one, computes the images that float16 pairs cannot hold.  A tile that shows that by itself is
 // not converted, multiplied or stored here.
-constexpr int kCP_CvtWarps  = 10; // a thread to a position of 28 x 28 images: 30 x 10
+// Converting warps: with ten the boxes of up to 320 positions are held in registers (30 x 10 of a 28 x 28 image), larger ones are read
+// twice.  Against the kernel before, 256 images, 3 x 3: 32 -> 64 channels at 12 x 12 36 -> 23 us, 28 x 28 65 -> 44, 32 x 32 90 -> 61,
+// 40 x 40 146 -> 114, 60 x 60 298 -> 238; 16 -> 32 at 56 x 56 233 -> 151.
+constexpr int kCP_CvtWarps  = 10;
 constexpr int kCP_EpiWarps  = 8;
 constexpr int kCP_Threads   = 64 + 32 * (kCP_CvtWarps + kCP_EpiWarps);
 constexpr int kCP_RowB      = 64; // a position's 32 channels

@@ -283,8 +283,10 @@ __device__ __noinline__ void half_finish_slices(
 // exit in the ordinary one the compiler arranged the rest less well, two layers of 4096 x 1024 x 1024 85.4 -> 89.3 us.
 // LINES: rows of the result that are not 16-byte aligned, at most one tile to a CTA or pair.  The operand stages are idle when
 // the tile is stored, so a warp's rows go through them whole and are stored in 128-byte lines, wherever in a line a row
-// begins; with a fixed 32 columns to a store every store has two partial sectors.  1537 x 771 x 2050 42.8 -> 41.4 us, 10453 x 199 x 222 31.0 -> 28.4.  In the
-// ordinary kernel (for a CTA's last tile) the same code cost others 3 %: 4096 x 1024 x 1024 twice 86.1 -> 88.6, 7853 x 118 x 8502 219 -> 237.
+// begins; with a fixed 32 columns to a store every store has two partial sectors.  Timed in turn without it, runs of one side 0.1 %
+// apart: 1537 x 771 x 2050 42.6 -> 41.6 us, 2305 x 771 x 1057 41.1 -> 40.1, 3000 x 500 x 1001 34.9 -> 33.0, 9000 x 300 x 301 29.9 -> 28.0,
+// 10453 x 199 x 222 29.4 -> 27.6, 4609 x 130 x 514 26.2 -> 24.0, 1281 x 65 x 1793 23.3 -> 21.1.  In the ordinary kernel (for a CTA's
+// last tile) the same code cost others 3 %: 4096 x 1024 x 1024 twice 86.1 -> 88.6, 7853 x 118 x 8502 219 -> 237.
 template <int BN, int CG, bool LEFT, bool LINES>
 __global__ void __launch_bounds__(kHThreads, 1)
     gemm_half_kernel(const __grid_constant__ HalfMaps maps, const __grid_constant__ HalfGemmParams p) {

@@ -435,7 +435,9 @@ int panel_clusters(const DeviceState *st, int size) {
 }
 
 // Slices of k; 0: the product is not for this kernel.  It takes those with one tile of columns whose k is sliced (the others
-// have the bytes of ct_matmul_packed_rows), which fill two thirds of the machine, and where A is most of the work.
+// have the bytes of ct_matmul_packed_rows), which fill two thirds of the machine, and where A is most of the work.  With slices
+// a power of two, and 74 clusters of two, 33 of four and 15 of eight at once, that is 25 to 33 row tiles where k is 4096 and
+// more, and 50 to 74 from 2048 on.
 int panel_slices(const DeviceState *st, int64_t m, int64_t k, int64_t n) {
     const int64_t tiles = (m + 127) / 128;
     if (n > 128 || k < 2048 || tiles * 2 > st->sm_count || st->sm_count / tiles > 8) // gemm_half, behind it, would use more slices than a cluster has

@@ -535,7 +535,7 @@ def conv2d(x: Tensor, w: Tensor, b: Tensor | None = None, stride: int = 1, pad: 
            activation: str | None = None, pool: int = 0) -> Tensor:
     """conv2d, + bias, activation; with pool=2 also the 2x2 max-pool of the result (the values of
     maxpool2d(conv2d(...), 2), without writing the full-resolution activation where the layer has
-    at most 32 channels and 64 filters)."""
+    at most 32 channels and 64 filters, else through a temporary of it)."""
     if pool not in (0, 2):
         raise _invalid("conv2d: pool must be 0 or 2")
     if x.rank != 4 or w.rank != 4:

@@ -72,9 +72,11 @@ typedef enum ct_precision {
                          * row and column, which hold 27 powers of two as well as tf32 terms do.  Smaller
                          * values beside a row's largest are multiplied in float32 apart, up to 32 of them
                          * in a product's operands; with more, or a row whose largest exponent is beyond
-                         * +-60, the product is computed from tf32 terms.  Convolutions of stride 1 take
-                         * tf32 terms for the images that span more than 26 powers of two, and for all
-                         * images where a filter does.  All of it is decided on the device. */
+                         * +-60, the product is computed from tf32 terms; small and tall products decide
+                         * so for parts of their operands, small ones with bfloat16 terms.  Convolutions of
+                         * stride 1 to 3, but those through patches, take tf32 terms for the images that
+                         * span more than 26 powers of two, and for all images where a filter does.  All
+                         * of it is decided on the device. */
     CT_PREC_BF16   = 1  /* inputs rounded to bf16 once, fp32 accumulate (reported separately) */
 } ct_precision;
 
@@ -292,7 +294,8 @@ ct_status ct_dense(
  * under the current precision and returns a handle; ct_dense_packed is ct_dense with that handle
  * and skips the per-call pre-pass over the weights (packed == NULL: exactly ct_dense).  The
  * handle must come from the same w_dev, k, n, precision and device, else CT_ERR_INVALID; the
- * caller keeps w_dev unchanged and alive (shapes with n <= 32 read w_dev itself).  Tensors of the
+ * caller keeps w_dev unchanged and alive (shapes with n <= 32 read w_dev itself, and so do small
+ * float32 products with k from 193 to 1024, which are one launch).  Tensors of the
  * reference are immutable values (every operator returns a new tensor), which is what makes
  * caching by tensor sound; the reference itself has no counterpart of these two calls.
  * A handle holds 12 bytes of device memory per value (float16 pairs and tf32 terms; 2 under
@@ -345,7 +348,9 @@ ct_status ct_conv2d(
 /* conv2d followed by a 2x2 max-pool (window == stride == 2), as one call: the same values as
  * ct_conv2d then ct_maxpool2d.  For stride-1 layers with at most 32 channels and 64 filters the pooling
  * happens in the convolution's epilogue and the full-resolution activation is never written; most other
- * shapes run the two steps.  out_dev is [n][k_out][h_out/2][w_out/2]. */
+ * shapes run the two steps, through a temporary of the whole activation (of at most 256 MB, part of the
+ * batch after part, for layers of up to 64 filters that the first sentence could have been true of).
+ * out_dev is [n][k_out][h_out/2][w_out/2]. */
 ct_status ct_conv2d_maxpool2(
     const float *x_dev, const float *w_dev, const float *bias_dev, int64_t n, int64_t c, int64_t h,
     int64_t w, int64_t k_out, int64_t kh, int64_t kw, int64_t stride, int64_t pad, ct_activation act,
