@@ -22,9 +22,9 @@
 // Strides: the rows and columns of the input that are alike modulo the stride are sub-images of the planes, and a tap is a
 // shift inside one of them, so a strided layer is the same loop with a halo per sub-image; its patches are never written
 // (64 x 48 x 57 x 57 -> 96 at stride 2: 121 us through a patch matrix, 70 so).  Longer k than 1024: the leading
-// accumulator is drained every 1024 values, as in gemm_half.cu.  The channel blocks are taken last to first: additions into an
-// accumulator truncate, and those of a block that is mostly padding cost least while the sums are small (45 x 33 x 64 x 64 -> 35
-// 6.0e-7 -> 4.0e-7 against 64 bits, 49 channels 7.5e-7 -> 6.2e-7, the same time).
+// accumulator is drained every 1024 values, as in gemm_half.cu.  Additions into an accumulator truncate, and those of k-steps that
+// are mostly padding cost least while the sums are small, so where channels do not fill the k-steps the last block is taken first
+// (45 x 33 x 64 x 64 -> 35 6.0e-7 -> 4.0e-7 against 64 bits, 49 channels 7.5e-7 -> 6.2e-7, the same time).
 //
 // One CTA per SM walks the tiles.  Both accumulators (512 columns) belong to one tile; the epilogue reads the
 // cross products first, which the next tile starts with, so the tensor pipe waits for about the drain of
@@ -101,6 +101,7 @@ struct ConvHaloParams {
     int chunk_blocks;                   // blocks of 32 channels per drain of the leading accumulator
     int chunk_wide;                     // tf32 images: blocks of 16
     int c;                              // channels of the layer
+    int last_first;                     // the channel blocks in descending order
     const float *filter_scale; // [ko] inverse scales
     const float *image_scale;  // [batch]; 0: this image's planes are tf32
     int c_pad;        // channels of the planes (k offset of a tap in the filter planes: tap * c_pad)
@@ -195,7 +196,8 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                 const CUtensorMap *mw_hi = wide ? &maps.w32_hi : &maps.w16_hi, *mw_lo = wide ? &maps.w32_lo : &maps.w16_lo;
                 const CUtensorMap *mx_hi = wide ? &maps.x32_hi : &maps.x16_hi, *mx_lo = wide ? &maps.x32_lo : &maps.x16_lo;
                 const int block_k = wide ? 16 : 32, cblocks = p.c_pad / block_k; // channels per k-block
-                for (int cb = cblocks - 1; cb >= 0 && ok; --cb) { // the block with padding first
+                for (int b = 0; b < cblocks && ok; ++b) {
+                    const int cb = p.last_first ? cblocks - 1 - b : b;
                     for (int h = 0; h < p.halos && ok; ++h, ++kh2) {
                         const int hs = kh2 % p.halo_stages;
                         if (!mbar_wait(smem_u32(&bar_h_empty[hs]), ((uint32_t)(kh2 / p.halo_stages) & 1u) ^ 1u, abort_flag)) {
@@ -260,7 +262,8 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                 };
                 const uint32_t d_main = tmem_base, d_cross = tmem_base + 256u;
                 bool first_cross = true, first_main = true;
-                for (int cb = cblocks - 1; cb >= 0 && ok; --cb) {
+                for (int b = 0; b < cblocks && ok; ++b) {
+                    const int cb   = p.last_first ? cblocks - 1 - b : b;
                     const bool two = p.c - cb * 32 > 16; // k-steps of this block that hold channels
                     for (int h = 0; h < p.halos && ok; ++h, ++kh2) {
                         const int hs = kh2 % p.halo_stages;
@@ -324,7 +327,7 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                         if (ok)
                             tc_commit(smem_u32(&bar_h_empty[hs])); // the halo is free once its taps' MMAs have retired
                     }
-                    if (ok && cb > 0 && (cblocks - cb) % chunk == 0) {
+                    if (ok && b + 1 < cblocks && (b + 1) % chunk == 0) {
                         tc_commit(smem_u32(&bar_tmem_full[0]));
                         first_main = true;
                     }
@@ -811,6 +814,7 @@ ct_status conv_halo(
     // 64 bits at 48 channels, 3 x 3; all 64 images 110 -> 117 us); unstrided, with the cross products apart, 4.0e-6 -> 1.4e-6
     p.chunk_wide = stride > 1 ? 1 : 2 * p.chunk_blocks;
     p.c       = (int)c;
+    p.last_first = c % 16 != 0;
     p.c_pad   = (int)c_pad;
     p.n_mma   = g.n_mma;
     p.box_bytes        = g.box_rows * g.pw * kH_RowB;
