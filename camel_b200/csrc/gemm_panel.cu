@@ -36,7 +36,7 @@ constexpr int kGP_Buffer  = 2 * kGP_Plane;    // A hi and lo of a chunk; two of 
 constexpr int kGP_BStages = 3;                // 64 values of k each, hi and lo
 constexpr int kGP_B       = 2 * kGP_Buffer;
 constexpr int kGP_Listed  = 16;               // exceptions of a CTA's part of A
-constexpr int kGP_Smem    = kGP_B + kGP_BStages * 2 * kGP_Block; // with the static 2 KB all that a CTA can have
+constexpr int kGP_Smem    = kGP_B + kGP_BStages * 2 * kGP_Block; // with the static 3 KB all that a CTA can have
 
 struct PanelParams {
     const float *a, *bias, *col_scale;
