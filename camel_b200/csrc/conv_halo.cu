@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
 
     if (warp == 0) {
         // ===== TMA producer =====
-        if (lane == 0) {
+        if (elect_one()) {
             int ka = 0, kh2 = 0; // filter k-blocks and halos issued so far
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
         }
     } else if (warp == 1) {
         // ===== MMA issuer =====
-        if (lane == 0) {
+        if (elect_one()) {
             int ka = 0, kh2 = 0, i = 0, crosses = 0, mains = 0; // accumulations begun so far
             bool ok = true;
             const long long t_start = CH_CLOCK();

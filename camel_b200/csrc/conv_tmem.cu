@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
 
     if (warp == 0) {
         // ===== TMA producer: one halo box per plane and tile (raw mode: one box of the input) =====
-        if (lane == 0) {
+        if (elect_one()) {
             int i = 0;
             bool ok = true;
             const int nstages = RAW ? kTA_RawStages : p.stages;
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
         }
     } else if (warp == 1) {
         // ===== MMA issuer =====
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc  = make_idesc(2u, 128, (uint32_t)kTA_N);
             const uint32_t d_tmem = tmem_base + (uint32_t)kTA_DCol;
             int i = 0;
@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
     stage_filters(p.w, p.ko, p.c * taps, filters, warp, kCP_Threads / 32, lane, [&](int f, uint2 range) {
         float scale, inverse;
         const bool fits = half_range_fits(range_warp(range), scale, inverse);
-        if (lane == 0) {
+        if (elect_one()) {
             filter_inv[f] = inverse;
             if (!fits)
                 filters_wide_s = 1;
@@ -808,7 +808,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
     if (filters_wide) {
     } else if (warp == 0) {
         // ===== TMA producer: one box per plane and region (raw mode: one box of the input) =====
-        if (lane == 0) {
+        if (elect_one()) {
             int i = 0;
             const int nstages = RAW ? 1 : p.stages;
             for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {

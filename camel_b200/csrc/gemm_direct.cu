@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kGD_Threads, 1) gemm_direct_kernel(const __gri
     auto b_desc = [&](int plane, int ks) { return desc_mn(smem_base + (uint32_t)(kGD_B + plane * kGD_Plane + ks * 2048)); };
     bool ok     = !failed;
     if (ok && ksteps > 0) {
-        if (threadIdx.x == 0) {
+        if (warp == 0 && elect_one()) {
             for (int ks = 0; ks < ksteps; ++ks) {
                 const uint64_t ah = a_desc(0, ks), al = a_desc(1, ks), bh = b_desc(0, ks), bl = b_desc(1, ks);
                 mma_f16(d_cross, al, bh, idesc, ks > 0);
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kGD_Threads, 1) gemm_direct_kernel(const __gri
                 split_bf16(0, i, av[i], true), split_bf16(kGD_B, i, bv[i], true);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncthreads();
-            if (threadIdx.x == 0) {
+            if (warp == 0 && elect_one()) {
                 for (int ks = 0; ks < ksteps; ++ks) {
                     mma_f16(d_cross, a_desc(1, ks), b_desc(0, ks), idesc, 1u);
                     mma_f16(d_cross, a_desc(0, ks), b_desc(1, ks), idesc, 1u);

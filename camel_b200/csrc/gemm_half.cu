@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(kHThreads, 1)
             }
     } else if (warp == 0) {
         // ===== TMA producer: stages numbered across tiles =====
-        if (lane == 0) {
+        if (elect_one()) {
             const CUtensorMap *ma_hi = wide ? &maps.a32_hi : &maps.a16_hi, *ma_lo = wide ? &maps.a32_lo : &maps.a16_lo;
             const CUtensorMap *mb_hi = wide ? &maps.b32_hi : &maps.b16_hi, *mb_lo = wide ? &maps.b32_lo : &maps.b16_lo;
             int s = 0, issued = 0;
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(kHThreads, 1)
         }
     } else if (warp == 1) {
         // ===== MMA issuer (the leader's, for the pair) =====
-        if (lane == 0 && rank == 0) {
+        if (elect_one() && rank == 0) {
             const uint32_t idesc = make_idesc(wide ? 2u : 0u, kHM * CG, BN);
             int s = 0, i = 0;
             uint32_t phase = 0;

@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kGP_Threads, 1) gemm_panel_kernel(
     bool ok = true;
     if (warp == 0) {
         // ===== B's planes =====
-        if (lane == 0) {
+        if (elect_one()) {
             int i = 0;
             for (; i < 2 * chunks; ++i) {
                 const int s = i % kGP_BStages;
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(kGP_Threads, 1) gemm_panel_kernel(
         }
     } else if (warp == 1) {
         // ===== MMA issuer =====
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc(0u, 128, 128);
             bool go = true;
             for (int c = 0, i = 0; c < chunks && go; ++c) {

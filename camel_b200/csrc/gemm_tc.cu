@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(Cfg<BN, MODE, RB>::kThreads, 1) gemm_tc_kernel
 
     if (warp == 0) {
         // ===== TMA producer =====
-        if (lane == 0) {
+        if (elect_one()) {
             int issued = 0;
             for (int kb = 0; kb < nkb; ++kb) {
                 int s       = kb % C::kStages;
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(Cfg<BN, MODE, RB>::kThreads, 1) gemm_tc_kernel
         }
     } else if (warp == 1) {
         // ===== MMA issuer =====
-        if (lane == 0) {
+        if (elect_one()) {
             // MMA shape 128 x tile_n x (32 bytes of k): tile_n == BN except for conv tiles
             const uint32_t idesc = make_idesc(MODE == MODE_3X ? 2u : 1u, BM, (uint32_t)p.tile_n);
             int kb = 0;
@@ -762,7 +762,7 @@ __global__ void __launch_bounds__(Cfg<BN, MODE, 64>::kThreads, 1) gemm_tc_stream
 
     if (warp == 0) {
         // ===== TMA producer: k-blocks numbered across tiles =====
-        if (lane == 0) {
+        if (elect_one()) {
             int kbg = 0; // k-blocks issued so far
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
@@ -815,7 +815,7 @@ __global__ void __launch_bounds__(Cfg<BN, MODE, 64>::kThreads, 1) gemm_tc_stream
         }
     } else if (warp == 1) {
         // ===== MMA issuer: accumulator buffer i & 1 for the CTA's i-th tile =====
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc(MODE == MODE_3X ? 2u : 1u, BM, (uint32_t)p.tile_n);
             int kbg = 0, i = 0;
             bool ok = true;
@@ -1091,7 +1091,7 @@ __global__ void __launch_bounds__(SwapCfg<MODE>::kThreads, 1) conv_swap_stream_k
 
     if (warp == 0) {
         // ===== TMA producer =====
-        if (lane == 0) {
+        if (elect_one()) {
             int kbg = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
@@ -1137,7 +1137,7 @@ __global__ void __launch_bounds__(SwapCfg<MODE>::kThreads, 1) conv_swap_stream_k
         }
     } else if (warp == 1) {
         // ===== MMA issuer =====
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc(MODE == MODE_3X ? 2u : 1u, BM, (uint32_t)p.n_mma);
             int kbg = 0, i = 0;
             bool ok = true;
