@@ -1,36 +1,41 @@
 // Implicit-GEMM conv2d (stride 1 to 3): the input halo of a tile is fetched once per channel block and serves all
 // filter taps.
 //
-// The streaming implicit GEMM of gemm_tc.cu fetches, for every (tap, channel block), the tile's
-// pixels again - the same values shifted by the tap.  Shared memory then carries, per k-block of 16
-// channels, 28 KB of pixel planes and 16 KB of filter planes in (TMA) plus 66 KB out (six MMAs read
-// their operands), and that traffic, not the tensor pipe, sets the kernel's pace (0.65 of the
-// measured 3xTF32 ceiling on 64 -> 128 channels, 56 x 56).  Here a tile is th output rows of
-// PW = w + 2 pad positions (the two halo columns of every row are computed and dropped), its
-// input for one block of 16 channels - th + kh - 1 rows of PW positions, zeros outside the image -
-// is ONE 4-D TMA box per plane, and tap (r, s) reads the same shared memory through a descriptor
-// moved by r * PW + s rows of 64 bytes (a position's row in the box is y * PW + x).  Pixel planes
-// enter shared memory once per nine taps; per k-block 19 KB in instead of 44.
+// The rows and columns of the input that are alike modulo the stride are sub-images, each written by the pre-pass as planes
+// [position][channel] with the padding in them, pw positions to a row.  Position q of the output, q = y * pw + x (the pw - wo
+// columns behind a row's end are computed and dropped), reads position q + shift of a tap's sub-image, whatever q: so a tile is any
+// 128 consecutive positions, whole rows or not, its halo the 128 + (largest shift) positions from its first one on, and a tap
+// the same shared memory through a descriptor moved by `shift` rows of 64 bytes.  Nothing is wasted on tiles that rows do not fill.
+//
+// Pixels are the accumulator's rows: a tile of 256 x n belongs to a pair of CTAs (cta_group::2), 128 positions each, n filters (a
+// multiple of 32, at most 128) shared out between them.  What bounds such a kernel is shared memory, 128 bytes per clock: with the
+// filters on the rows of a CTA by itself and 240 positions on its columns, the operands took 98 of them, the filters' stream 23, and
+// the exchange through which the sums reached the pixels' order 18 more; a tile of 13,000 clocks of MMAs took 18,800.  Here the
+// filters of a layer stay in shared memory where they fit beside two halos (64 -> 128 channels, 3 x 3: 144 KB a CTA; a ring of
+// stages otherwise), half of a filter operand is read by each CTA, and a lane of the epilogue has a pixel and its registers
+// channels, so that scale, bias, activation and the store need no exchange.
 //
 // Arithmetic: split float16 (half_split.cuh), scaled per filter and per image - a scale has to be constant
 // along k, and an output's patch crosses the whole halo - with the cross products in an accumulator of their
-// own, as in gemm_half.cu.  A 64-byte row then holds 32 channels, so the layer takes half the MMAs, half the
-// filter stages and half the plane traffic of the tf32 form.  An image that spans too many powers of two - or
-// every image, where a filter does - has tf32 planes in the same place, and this kernel runs the same loop over
-// those for its tiles (16 channels per row); the other images of the batch are not touched by it.
+// own, as in gemm_half.cu.  An image that spans too many powers of two - or every image, where a filter does - has tf32 planes in
+// the same place (16 channels to a row of 64 bytes) and runs the same loop over those.  The two tiles of a pair may be of images of
+// different forms: then the pair runs twice and each tile is stored once.
 //
-// Strides: the rows and columns of the input that are alike modulo the stride are sub-images of the planes, and a tap is a
-// shift inside one of them, so a strided layer is the same loop with a halo per sub-image; its patches are never written
-// (64 x 48 x 57 x 57 -> 96 at stride 2: 121 us through a patch matrix, 70 so).  Longer k than 1024: the leading
-// accumulator is drained every 1024 values, as in gemm_half.cu.  Additions into an accumulator truncate, and those of k-steps that
-// are mostly padding cost least while the sums are small, so where channels do not fill the k-steps the last block is taken first
-// (45 x 33 x 64 x 64 -> 35 6.0e-7 -> 4.0e-7 against 64 bits, 49 channels 7.5e-7 -> 6.2e-7, the same time).
+// MMAs per 16 channels and tap (8 in tf32), two ways of sharing the filters out.  THREE: X_hi x W_hi, X_hi x W_lo, X_lo x W_hi, n columns each, every
+// CTA holding half of the hi and half of the lo terms.  Otherwise X_hi x [W_hi; W_lo], 2 n columns, the leader holding the hi and its peer the
+// lo terms, and X_lo x W_hi from another copy of half of the hi terms in each.  An MMA takes half a clock per column but not less than 49,
+// so the second is the faster one for n < 96; the first takes two thirds of the memory, and serves fewer filters too where that decides
+// whether they stay, or has them streamed.
 //
-// One CTA per SM walks the tiles.  Both accumulators (512 columns) belong to one tile; the epilogue reads the
-// cross products first, which the next tile starts with, so the tensor pipe waits for about the drain of
-// the leading accumulator (a few hundred of ~14,000 clocks per tile of 64 channels) and the store runs under
-// the next tile's MMAs.  Two rings of stages: filter k-blocks (one per tap and channel block) and halos (one
-// per channel block).  Rows = 128 output channels, columns = positions.  Every wait is bounded.
+// k beyond 1024 values: both accumulators are drained every 1024 and added up in registers.  Additions into an accumulator truncate, and
+// those of k-steps that are mostly padding cost least while the sums are small, so where channels do not fill the k-steps the last block
+// is taken first (45 x 33 x 64 x 64 -> 35 6.0e-7 -> 4.0e-7 against 64 bits, 49 channels 7.5e-7 -> 6.2e-7, the same time).
+//
+// A pair per two SMs walks the tiles, filters outermost; two sets of accumulators, so that a tile is drained and stored under the next
+// one's MMAs.  Every wait is bounded.  Measured: the roles run as whole warps with uniform control flow, so that descriptors stay in
+// uniform registers; entered by one thread, the issuer took 11,000 clocks for a tile of 6900 clocks of MMAs, and is told what
+// a halo holds by the producer (8400).  Sixteen epilogue warps: with eight a tile's drain and store took longer than its MMAs.
+// 256 x 64 x 56 x 56 -> 128: kernel 307 -> 235 us, layer 484 -> 436; 64 x 48 x 57 x 57 -> 96 at stride 2, layer 69.5 -> 61.7.
 #include "common.cuh"
 #include "half_split.cuh"
 #include "split.cuh"
@@ -39,461 +44,504 @@
 
 #include <algorithm>
 
-// Optional per-CTA clock accounting for tuning; compiled in only with -DCT_CONV_TRACE.
-#ifdef CT_CONV_TRACE
-__device__ unsigned long long g_halo_trace[256 * 16];
-#define CH_CLOCK() clock64()
-#define CH_ACCUM(slot, cycles)                                                          \
-    do {                                                                                \
-        if (blockIdx.x < 256)                                                           \
-            g_halo_trace[blockIdx.x * 16 + (slot)] += (unsigned long long)(cycles);     \
-    } while (0)
-extern "C" int ct_debug_halo_trace(unsigned long long *host, int count, int clear) {
-    int rc = (int)cudaMemcpyFromSymbol(host, g_halo_trace, sizeof(unsigned long long) * (size_t)count);
-    if (clear) {
-        static unsigned long long zeros[256 * 16];
-        cudaMemcpyToSymbol(g_halo_trace, zeros, sizeof(zeros));
-    }
-    return rc;
-}
-#else
-#define CH_CLOCK() 0ll
-#define CH_ACCUM(slot, cycles) do { } while (0)
-#endif
-
 namespace ct {
 namespace {
 
 using namespace ptx;
 
 constexpr int kH_RowB       = 64;                     // bytes of k per operand row and k-block: 32 float16 / 16 tf32
-constexpr int kH_AStages    = 4;
+constexpr int kH_MaxSlots   = 96;                     // filter k-blocks in shared memory (a tap and channel block each)
 constexpr int kH_HaloStages = 4;                      // at most; as many as shared memory holds
-constexpr int kH_ABytes     = 128 * kH_RowB;          // one filter plane of a k-block
-constexpr int kH_AStageBytes = 2 * kH_ABytes;         // hi + lo
-constexpr int kH_EpiWarps   = 8;
+constexpr int kH_EpiWarps   = 16;
 constexpr int kH_Threads    = 64 + 32 * kH_EpiWarps;
-constexpr int kH_EpiRowBytes  = 32 * 4 + 16;          // 32 columns staged at a time, rows padded
-constexpr int kH_EpiWarpBytes = 32 * kH_EpiRowBytes;
-constexpr int kH_EpiBytes     = kH_EpiWarps * kH_EpiWarpBytes;
+constexpr int kH_Smem       = 220 * 1024;             // 227 KB per CTA less the static shared memory
 constexpr int kH_MinFilters = 17;
 constexpr int kH_MaxTaps    = 32;
 constexpr int kH_MaxStride  = 3;
 constexpr int kH_MaxHalos   = kH_MaxStride * kH_MaxStride;
-constexpr int kH_MaxK       = 1024; // values of k per drain of the leading accumulator
-constexpr int kH_BiasSlots    = 256;                  // output channels whose bias is kept in shared memory
+// What the leader's producer tells the MMA issuer about a halo, beside its first tap and the tap behind its last (six bits each)
+constexpr uint32_t kH_Wide = 1u << 12, kH_Two = 1u << 13, kH_Load = 1u << 14, kH_Begin = 1u << 15, kH_End = 1u << 16, kH_Set = 1u << 17,
+                   kH_Reload = 1u << 18, kH_Over = 1u << 19;
+constexpr int kH_MaxK       = 1024; // values of k per drain of the accumulators
+
+// n / d for n < 2^31, from inv = 2^32 / d rounded up (0 for d = 1): the rounded-up quotient is one too high at most.
+struct FastDiv {
+    uint32_t d, inv;
+};
+__device__ __forceinline__ int fast_div(int n, const FastDiv &f) {
+    const uint32_t q = f.inv ? __umulhi((uint32_t)n, f.inv) : (uint32_t)n;
+    return (int)(q - (q * f.d > (uint32_t)n ? 1u : 0u));
+}
+FastDiv fast_divisor(int64_t d) { return {(uint32_t)d, d > 1 ? (uint32_t)(((1ull << 32) + d - 1) / d) : 0u}; }
 
 struct ConvHaloParams {
-    const float *bias;
     float *out;       // [batch][ko][ho][wo]
     uint32_t *flags;
-    int ko, tiles_m;
-    int ho, wo, pw;   // pw: positions of a tile row
-    int th, tiles_y;
-    // The filter taps in the order of the halos that they read (one halo for stride 1; the rows and columns of the input
-    // that are alike modulo the stride are a sub-image each).
+    int ko, n;        // n: filters of a tile
+    int ho, wo, pw;   // pw: positions of a row
+    int image_tiles;  // of 128 positions
+    int total_tiles, pairs; // of the batch; pairs of them
+    int items;        // pairs times filter tiles
+    // The filter taps in the order of the halos that they read (one halo for stride 1; a sub-image each otherwise).
     int halos;                          // per channel block
-    uint8_t halo_image[kH_MaxHalos];    // its sub-image
+    int halo_at[kH_MaxHalos];           // position of its sub-image in the planes
     uint8_t halo_taps[kH_MaxHalos + 1]; // its first tap in the list; the last entry is the number of taps
     uint8_t tap[kH_MaxTaps];            // r * kw + s
-    uint16_t tap_shift[kH_MaxTaps];     // position of the tap's first pixel in the box
-    int box_x0, box_y0;                 // of tile row 0 in the sub-images
-    int chunk_blocks;                   // blocks of 32 channels per drain of the leading accumulator
+    uint16_t tap_shift[kH_MaxTaps];     // positions between an output and the tap's pixel in the sub-image, in units of descriptors
+    int chunk_blocks;                   // blocks of 32 channels per drain of the accumulators
     int chunk_wide;                     // tf32 images: blocks of 16
+    int chunks, chunks_wide;            // drains
     int c;                              // channels of the layer
     int last_first;                     // the channel blocks in descending order
-    const float *filter_scale; // [ko] inverse scales
+    const float *filter_scale; // [ko rounded up to whole tiles] inverse scales
+    const float *bias;         // the same, -0 where there is none: no sum notices
     const float *image_scale;  // [batch]; 0: this image's planes are tf32
     int c_pad;        // channels of the planes (k offset of a tap in the filter planes: tap * c_pad)
-    int n_mma;        // th * pw rounded up to 16
-    int box_bytes;    // one plane's halo box
+    int box_rows, boxes; // positions of a TMA box, boxes of a halo
     int halo_plane_bytes, halo_stages;
+    int slots, slot_bytes, resident; // filter k-blocks in shared memory; resident: all of a set
     int act;
+    FastDiv by_pairs, by_tiles, by_pw; // pairs, image_tiles, pw
 };
 
 struct ConvHaloMaps {
-    CUtensorMap w16_hi, w16_lo, x16_hi, x16_lo;
-    CUtensorMap w32_hi, w32_lo, x32_hi, x32_lo;
+    CUtensorMap x16_hi, x16_lo, x32_hi, x32_lo;
+    // THREE: hi and lo terms, boxes of n / 2 filters.  Otherwise hi (n / 2), lo (n), hi (n).
+    CUtensorMap w16[3], w32[3];
 };
 
+// Tile load of three dimensions into THIS CTA's shared memory whose bytes are counted on a barrier of this CTA or the leader.
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst_smem, const void *map, uint32_t cluster_bar, int32_t c0, int32_t c1, int32_t c2) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5}], [%2];"
+        :
+        : "r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(cluster_bar), "r"(c0), "r"(c1), "r"(c2)
+        : "memory");
+}
+
+// The work of a pair, in the order that all its roles walk it: items (filter tile, pair of pixel tiles), each in one form or in
+// both.  The scales of the images that say which are fetched an item ahead.
+struct HaloWalk {
+    const ConvHaloParams &p;
+    int item, stride, form;
+    int tn, tile[2], img[2];
+    bool wide[2];
+    float scale[2], next[2];
+
+    __device__ __forceinline__ void fetch(int it) {
+        if (it < p.items) {
+            const int u = it - fast_div(it, p.by_pairs) * p.pairs;
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+                next[r] = p.image_scale[fast_div(min(2 * u + r, p.total_tiles - 1), p.by_tiles)];
+        }
+    }
+    __device__ __forceinline__ HaloWalk(const ConvHaloParams &params, int first, int step) : p(params), item(first - step), stride(step), form(1) {
+        wide[0] = wide[1] = false;
+        fetch(first);
+    }
+    // the next pass; false: none
+    __device__ __forceinline__ bool advance() {
+        if (form == 0 && (wide[0] || wide[1])) {
+            form = 1;
+            return true;
+        }
+        item += stride;
+        if (item >= p.items)
+            return false;
+        tn          = fast_div(item, p.by_pairs);
+        const int u = item - tn * p.pairs;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            tile[r] = min(2 * u + r, p.total_tiles - 1);
+            img[r]  = fast_div(tile[r], p.by_tiles);
+            scale[r] = next[r];
+            wide[r]  = __any_sync(0xffffffffu, next[r] == 0.0f) != 0; // the same for all lanes, and known to be
+        }
+        form = wide[0] && wide[1] ? 1 : 0;
+        fetch(item + stride);
+        return true;
+    }
+    __device__ __forceinline__ int cblocks() const { return p.c_pad >> (form ? 4 : 5); }
+    __device__ __forceinline__ int chunk() const { return form ? p.chunk_wide : p.chunk_blocks; }
+    __device__ __forceinline__ int block(int b) const { return p.last_first ? cblocks() - 1 - b : b; }
+    // Filter k-blocks come in sets of c_pad / 32 channel blocks (two to a tf32 pass); -1: not the first block of one
+    __device__ __forceinline__ int set_of(int b) const {
+        const int each = p.c_pad >> 5;
+        return b == 0 ? tn * 3 + form : (b == each ? tn * 3 + 2 : -1);
+    }
+};
+
+template <bool THREE>
 __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
-    const __grid_constant__ ConvHaloMaps maps, const __grid_constant__ ConvHaloParams p, const int all_tiles) {
+    const __grid_constant__ ConvHaloMaps maps, const __grid_constant__ ConvHaloParams p) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t bar_a_full[kH_AStages], bar_a_empty[kH_AStages];
+    __shared__ uint64_t bar_f_full[kH_MaxSlots], bar_f_empty[kH_MaxSlots], bar_reload;
     __shared__ uint64_t bar_h_full[kH_HaloStages], bar_h_empty[kH_HaloStages];
-    __shared__ uint64_t bar_tmem_full[2], bar_tmem_empty[2]; // 0: leading accumulator, 1: cross products
+    __shared__ uint64_t bar_acc_full[2], bar_acc_empty[2];
+    __shared__ uint32_t halo_word[kH_HaloStages];
     __shared__ uint64_t bar_done;
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag_s;
-    // the layer's bias, read once: a load per stored row would put a trip to L2 in front of the add
-    __shared__ float bias_s[kH_BiasSlots];
+    // scales and bias of the filters of an epilogue warp: from global memory, between the stores, they cost more than the stores
+    __shared__ __align__(16) float scale_s[kH_EpiWarps][32], bias_s[kH_EpiWarps][32];
     volatile int *abort_flag = &abort_flag_s;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); // known to be the same for the warp
     const int lane = threadIdx.x & 31;
+    const int rank = (int)(blockIdx.x & 1); // in the cluster of two
 
     griddep_launch_dependents();
     const uint32_t smem_base  = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t halo_base  = smem_base + kH_AStages * kH_AStageBytes;
     const uint32_t halo_stage = 2u * (uint32_t)p.halo_plane_bytes;
-    uint8_t *epi_base = smem_raw + (smem_base - smem_u32(smem_raw)) + kH_AStages * kH_AStageBytes + (uint32_t)p.halo_stages * halo_stage;
+    const uint32_t slot_base  = smem_base + (uint32_t)p.halo_stages * halo_stage;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kH_AStages; ++s) {
-            mbar_init(smem_u32(&bar_a_full[s]), 1);
-            mbar_init(smem_u32(&bar_a_empty[s]), 1);
+        for (int s = 0; s < p.slots; ++s) {
+            mbar_init(smem_u32(&bar_f_full[s]), 1);
+            mbar_init(smem_u32(&bar_f_empty[s]), 1);
         }
-        for (int s = 0; s < kH_HaloStages; ++s) {
+        for (int s = 0; s < p.halo_stages; ++s) {
             mbar_init(smem_u32(&bar_h_full[s]), 1);
             mbar_init(smem_u32(&bar_h_empty[s]), 1);
         }
         for (int b = 0; b < 2; ++b) {
-            mbar_init(smem_u32(&bar_tmem_full[b]), 1);
-            mbar_init(smem_u32(&bar_tmem_empty[b]), kH_EpiWarps);
+            mbar_init(smem_u32(&bar_acc_full[b]), 1);
+            mbar_init(smem_u32(&bar_acc_empty[b]), 2 * kH_EpiWarps); // both CTAs'
         }
+        mbar_init(smem_u32(&bar_reload), 1);
         mbar_init(smem_u32(&bar_done), 1);
         mbar_fence_init();
-        prefetch_tensormap(&maps.w16_hi);
-        prefetch_tensormap(&maps.w16_lo);
         prefetch_tensormap(&maps.x16_hi);
         prefetch_tensormap(&maps.x16_lo);
+        prefetch_tensormap(&maps.w16[0]);
+        prefetch_tensormap(&maps.w16[1]);
     }
     if (warp == 1) {
-        tmem_alloc(smem_u32(&tmem_base_slot), 512);
-        tmem_relinquish();
+        tmem_alloc_pair(smem_u32(&tmem_base_slot), 512);
+        tmem_relinquish_pair();
     }
     griddep_wait(); // the planes, the scales and what the caller's earlier kernels wrote
     if (threadIdx.x == 0)
         abort_flag_s = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
-    for (int c = threadIdx.x; c < kH_BiasSlots; c += kH_Threads)
-        bias_s[c] = (p.bias && c < p.ko) ? p.bias[c] : 0.0f;
     tc_fence_before_sync();
     __syncthreads();
+    cluster_sync(); // the partner's barriers exist before anything is signalled on them
     tc_fence_after_sync();
-    const uint32_t tmem_base = tmem_base_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
     const bool failed        = abort_flag_s != 0; // an earlier launch failed: no work
-    const int total_tiles    = failed ? 0 : all_tiles;
     __syncthreads(); // every thread has read abort_flag_s before a role may raise it
+    const int first = (int)(blockIdx.x >> 1), stride = (int)(gridDim.x >> 1);
 
-    // tile -> (row tile of output channels, tile row, image): neighbouring CTAs take the row tiles
-    // of one pixel tile, so they read the same halo out of L2
-    auto coords = [&](int tile, int &tm, int &ty, int &img) {
-        tm       = tile % p.tiles_m;
-        int rest = tile / p.tiles_m;
-        img      = rest / p.tiles_y;
-        ty       = rest - img * p.tiles_y;
-    };
-
-    if (warp == 0) {
-        // ===== TMA producer =====
-        if (elect_one()) {
-            int ka = 0, kh2 = 0; // filter k-blocks and halos issued so far
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-                int tm, ty, img;
-                coords(tile, tm, ty, img);
-                const bool wide          = p.image_scale[img] == 0.0f;
-                const CUtensorMap *mw_hi = wide ? &maps.w32_hi : &maps.w16_hi, *mw_lo = wide ? &maps.w32_lo : &maps.w16_lo;
-                const CUtensorMap *mx_hi = wide ? &maps.x32_hi : &maps.x16_hi, *mx_lo = wide ? &maps.x32_lo : &maps.x16_lo;
-                const int block_k = wide ? 16 : 32, cblocks = p.c_pad / block_k; // channels per k-block
-                for (int b = 0; b < cblocks && ok; ++b) {
-                    const int cb = p.last_first ? cblocks - 1 - b : b;
-                    for (int h = 0; h < p.halos && ok; ++h, ++kh2) {
-                        const int hs = kh2 % p.halo_stages;
-                        if (!mbar_wait(smem_u32(&bar_h_empty[hs]), ((uint32_t)(kh2 / p.halo_stages) & 1u) ^ 1u, abort_flag)) {
-                            ok = false;
-                            break;
+    if (failed) {
+    } else if (warp == 0) {
+        // ===== TMA producer: this CTA's halos and its share of the filters, counted on the leader's barriers =====
+        int ka = 0, s = 0, kh2 = 0, hs = 0, held = -1, sets = 0; // filter k-blocks, halos and sets of filters issued so far
+        uint32_t f_phase = 1, h_phase = 1;
+        bool ok = true;
+        HaloWalk walk(p, first, stride);
+        while (ok && walk.advance()) {
+            const CUtensorMap *x_hi = walk.form ? &maps.x32_hi : &maps.x16_hi, *x_lo = walk.form ? &maps.x32_lo : &maps.x16_lo;
+            const CUtensorMap *w    = walk.form ? maps.w32 : maps.w16;
+            const int block_k       = walk.form ? 16 : 32; // channels per k-block
+            const int img  = rank ? walk.img[1] : walk.img[0], tile = rank ? walk.tile[1] : walk.tile[0];
+            const int at   = (tile - img * p.image_tiles) * 128, cblocks = walk.cblocks();
+            const int chunk = walk.chunk();
+            bool load       = true;
+            int in_chunk    = 0;
+            for (int b = 0; b < cblocks && ok; ++b) {
+                const int c0  = walk.block(b) * block_k;
+                uint32_t word = walk.form ? kH_Wide | kH_Two : (p.c - c0 > 16 ? kH_Two : 0u); // k-steps that hold channels
+                bool reload   = false;
+                if (p.resident) {
+                    const int set = walk.set_of(b);
+                    if (set >= 0) {
+                        load   = set != held;
+                        held   = set;
+                        reload = load && sets++ > 0;
+                        word |= kH_Set | (reload ? kH_Reload : 0u);
+                    }
+                }
+                word |= (load ? kH_Load : 0u) | (in_chunk == 0 ? kH_Begin : 0u);
+                const bool last = ++in_chunk == chunk || b + 1 == cblocks;
+                if (last)
+                    in_chunk = 0;
+                for (int h = 0; h < p.halos && ok; ++h) {
+                    ok = mbar_wait_patient_warp(smem_u32(&bar_h_empty[hs]), h_phase, abort_flag);
+                    if (!ok)
+                        break;
+                    if (elect_one()) {
+                        const uint32_t full = smem_u32(&bar_h_full[hs]), dst = smem_base + (uint32_t)hs * halo_stage;
+                        if (rank == 0) {
+                            halo_word[hs] = word | (uint32_t)p.halo_taps[h] | (uint32_t)p.halo_taps[h + 1] << 6 |
+                                            (last && h + 1 == p.halos ? kH_End : 0u);
+                            mbar_expect_tx(full, 2u * 2u * (uint32_t)(p.boxes * p.box_rows * kH_RowB));
                         }
-                        const uint32_t hfull = smem_u32(&bar_h_full[hs]);
-                        const uint32_t hdst  = halo_base + (uint32_t)hs * halo_stage;
-                        const int y0 = ty * p.th + p.box_y0, sub = p.halo_image[h];
-                        mbar_expect_tx(hfull, 2u * (uint32_t)p.box_bytes);
-                        tma_load_5d(hdst, mx_hi, hfull, cb * block_k, p.box_x0, y0, sub, img);
-                        tma_load_5d(hdst + (uint32_t)p.halo_plane_bytes, mx_lo, hfull, cb * block_k, p.box_x0, y0, sub, img);
-                        for (int t = p.halo_taps[h]; t < p.halo_taps[h + 1]; ++t, ++ka) {
-                            const int s = ka % kH_AStages;
-                            if (!mbar_wait(smem_u32(&bar_a_empty[s]), ((uint32_t)(ka / kH_AStages) & 1u) ^ 1u, abort_flag)) {
-                                ok = false;
+                        for (int x = 0; x < p.boxes; ++x) {
+                            const uint32_t off = (uint32_t)(x * p.box_rows * kH_RowB);
+                            tma_load_3d_pair(dst + off, x_hi, leader_addr(full), c0, p.halo_at[h] + at + x * p.box_rows, img);
+                            tma_load_3d_pair(dst + (uint32_t)p.halo_plane_bytes + off, x_lo, leader_addr(full), c0,
+                                             p.halo_at[h] + at + x * p.box_rows, img);
+                        }
+                    }
+                    __syncwarp();
+                    ++kh2;
+                    if (++hs == p.halo_stages)
+                        hs = 0, h_phase ^= 1u;
+                    word &= ~(kH_Begin | kH_Set | kH_Reload);
+                    if (reload) // everything that read the last set has retired; the issuer has been told to say so
+                        ok = mbar_wait_patient_warp(smem_u32(&bar_reload), (uint32_t)sets & 1u, abort_flag);
+                    reload = false;
+                    if (!ok)
+                        break;
+                    for (int t = p.halo_taps[h]; load && t < p.halo_taps[h + 1]; ++t) {
+                        if (!p.resident) {
+                            ok = mbar_wait_patient_warp(smem_u32(&bar_f_empty[s]), f_phase, abort_flag);
+                            if (!ok)
                                 break;
-                            }
-                            const uint32_t full = smem_u32(&bar_a_full[s]);
-                            const uint32_t dst  = smem_base + (uint32_t)s * kH_AStageBytes;
-                            mbar_expect_tx(full, (uint32_t)kH_AStageBytes);
-                            const int32_t kc = p.tap[t] * p.c_pad + cb * block_k;
-                            tma_load_2d(dst, mw_hi, full, kc, tm * 128);
-                            tma_load_2d(dst + kH_ABytes, mw_lo, full, kc, tm * 128);
                         }
-                    }
-                }
-            }
-            if (*abort_flag) {
-                // unwind: let the copies still in flight land before the CTA goes away
-                for (int k2 = ka - kH_AStages < 0 ? 0 : ka - kH_AStages; k2 < ka; ++k2) {
-                    const uint64_t t0 = globaltimer_ns();
-                    while (!mbar_try_wait(smem_u32(&bar_a_full[k2 % kH_AStages]), (uint32_t)(k2 / kH_AStages) & 1u) &&
-                           globaltimer_ns() - t0 < kWaitBudgetNs) {
-                    }
-                }
-                for (int k2 = kh2 - p.halo_stages < 0 ? 0 : kh2 - p.halo_stages; k2 < kh2; ++k2) {
-                    const uint64_t t0 = globaltimer_ns();
-                    while (!mbar_try_wait(smem_u32(&bar_h_full[k2 % p.halo_stages]), (uint32_t)(k2 / p.halo_stages) & 1u) &&
-                           globaltimer_ns() - t0 < kWaitBudgetNs) {
+                        if (elect_one()) {
+                            const uint32_t full = smem_u32(&bar_f_full[s]), dst = slot_base + (uint32_t)(s * p.slot_bytes);
+                            if (rank == 0)
+                                mbar_expect_tx(full, 2u * (uint32_t)p.slot_bytes);
+                            const int32_t kc = p.tap[t] * p.c_pad + c0, row = walk.tn * p.n, half = row + rank * (p.n >> 1);
+                            if (THREE) {
+                                tma_load_2d_pair(dst, &w[0], leader_addr(full), kc, half);
+                                tma_load_2d_pair(dst + (uint32_t)(p.n >> 1) * kH_RowB, &w[1], leader_addr(full), kc, half);
+                            } else {
+                                tma_load_2d_pair(dst, rank ? &w[1] : &w[2], leader_addr(full), kc, row);
+                                tma_load_2d_pair(dst + (uint32_t)p.n * kH_RowB, &w[0], leader_addr(full), kc, half);
+                            }
+                        }
+                        __syncwarp();
+                        ++ka;
+                        if (++s == p.slots)
+                            s = 0, f_phase ^= 1u;
                     }
                 }
             }
         }
-    } else if (warp == 1) {
-        // ===== MMA issuer =====
-        if (elect_one()) {
-            int ka = 0, kh2 = 0, i = 0, crosses = 0, mains = 0; // accumulations begun so far
-            bool ok = true;
-            const long long t_start = CH_CLOCK();
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++i) {
-                int tm, ty, img;
-                coords(tile, tm, ty, img);
-                const bool wide      = p.image_scale[img] == 0.0f; // looked up while the MMAs of the last tile run
-                const uint32_t idesc = make_idesc(wide ? 2u : 0u, 128, (uint32_t)p.n_mma);
-                const int cblocks = p.c_pad / (wide ? 16 : 32), chunk = wide ? p.chunk_wide : p.chunk_blocks;
-                // what the accumulator held before has been read
-                auto wait_empty = [&](int acc) {
-                    const bool got = mbar_wait(smem_u32(&bar_tmem_empty[acc]), ((uint32_t)(acc ? crosses++ : mains++) & 1u) ^ 1u, abort_flag);
-                    tc_fence_after_sync();
-                    return got;
-                };
-                const uint32_t d_main = tmem_base, d_cross = tmem_base + 256u;
-                bool first_cross = true, first_main = true;
-                for (int b = 0; b < cblocks && ok; ++b) {
-                    const int cb   = p.last_first ? cblocks - 1 - b : b;
-                    const bool two = p.c - cb * 32 > 16; // k-steps of this block that hold channels
-                    for (int h = 0; h < p.halos && ok; ++h, ++kh2) {
-                        const int hs = kh2 % p.halo_stages;
-                        const long long t1 = CH_CLOCK();
-                        if (!mbar_wait(smem_u32(&bar_h_full[hs]), (uint32_t)(kh2 / p.halo_stages) & 1u, abort_flag)) {
-                            ok = false;
-                            break;
-                        }
-                        CH_ACCUM(1, CH_CLOCK() - t1); // waiting for a halo
-                        const uint32_t x_hi = halo_base + (uint32_t)hs * halo_stage;
-                        const uint32_t x_lo = x_hi + (uint32_t)p.halo_plane_bytes;
-                        for (int t = p.halo_taps[h]; t < p.halo_taps[h + 1]; ++t, ++ka) {
-                            const int s = ka % kH_AStages;
-                            const long long t2 = CH_CLOCK();
-                            if (!mbar_wait(smem_u32(&bar_a_full[s]), (uint32_t)(ka / kH_AStages) & 1u, abort_flag)) {
-                                ok = false;
-                                break;
-                            }
-                            CH_ACCUM(2, CH_CLOCK() - t2); // waiting for filter planes
-                            tc_fence_after_sync();
-                            const uint32_t a_hi = smem_base + (uint32_t)s * kH_AStageBytes, a_lo = a_hi + kH_ABytes;
-                            // the tap's pixels: the halo, so many rows of 64 bytes further on
-                            const uint32_t shift = (uint32_t)p.tap_shift[t] * (uint32_t)kH_RowB;
-                            const uint64_t da_hi = smem_desc_k<kH_RowB>(a_hi), da_lo = smem_desc_k<kH_RowB>(a_lo);
-                            const uint64_t db_hi = smem_desc_k<kH_RowB>(x_hi + shift), db_lo = smem_desc_k<kH_RowB>(x_lo + shift);
-                            if (first_cross && !wait_empty(1)) {
-                                ok = false;
-                                break;
-                            }
-                            if (!wide) {
-                                mma_f16(d_cross, da_lo, db_hi, idesc, first_cross ? 0u : 1u);
-                                mma_f16(d_cross, da_hi, db_lo, idesc, 1u);
-                                if (two) {
-                                    mma_f16(d_cross, da_lo + 2, db_hi + 2, idesc, 1u);
-                                    mma_f16(d_cross, da_hi + 2, db_lo + 2, idesc, 1u);
-                                }
-                            } else {
-#pragma unroll
-                                for (int kk = 0; kk < kH_RowB / 32; ++kk) {
-                                    mma_tf32(d_cross, da_lo + 2 * kk, db_hi + 2 * kk, idesc, first_cross && kk == 0 ? 0u : 1u);
-                                    mma_tf32(d_cross, da_hi + 2 * kk, db_lo + 2 * kk, idesc, 1u);
-                                }
-                            }
-                            if (first_main && !wait_empty(0)) {
-                                ok = false;
-                                break;
-                            }
-                            if (!wide) {
-                                mma_f16(d_main, da_hi, db_hi, idesc, first_main ? 0u : 1u);
-                                if (two)
-                                    mma_f16(d_main, da_hi + 2, db_hi + 2, idesc, 1u);
-                            } else {
-#pragma unroll
-                                for (int kk = 0; kk < kH_RowB / 32; ++kk)
-                                    mma_tf32(d_main, da_hi + 2 * kk, db_hi + 2 * kk, idesc, first_main && kk == 0 ? 0u : 1u);
-                            }
-                            first_cross = false;
-                            first_main = false;
-                            tc_commit(smem_u32(&bar_a_empty[s]));
-                        }
-                        if (ok)
-                            tc_commit(smem_u32(&bar_h_empty[hs])); // the halo is free once its taps' MMAs have retired
-                    }
-                    if (ok && b + 1 < cblocks && (b + 1) % chunk == 0) {
-                        tc_commit(smem_u32(&bar_tmem_full[0]));
-                        first_main = true;
-                    }
-                }
-                if (ok) {
-                    tc_commit(smem_u32(&bar_tmem_full[1]));
-                    tc_commit(smem_u32(&bar_tmem_full[0]));
+        if (ok && rank == 0) {
+            ok = mbar_wait_patient_warp(smem_u32(&bar_h_empty[hs]), h_phase, abort_flag);
+            if (ok && elect_one()) {
+                halo_word[hs] = kH_Over;
+                mbar_arrive(smem_u32(&bar_h_full[hs]));
+            }
+            __syncwarp();
+        }
+        if (*abort_flag && rank == 0) {
+            // unwind: let the copies still in flight land before the CTA goes away (the leader's barriers
+            // count the partner's copies too, and neither CTA leaves before the other)
+            for (int k2 = ka - p.slots < 0 ? 0 : ka - p.slots; k2 < ka; ++k2) {
+                const uint64_t t0 = globaltimer_ns();
+                while (!mbar_try_wait(smem_u32(&bar_f_full[k2 % p.slots]), (uint32_t)(k2 / p.slots) & 1u) &&
+                       globaltimer_ns() - t0 < kWaitBudgetNs) {
                 }
             }
-            CH_ACCUM(3, CH_CLOCK() - t_start); // the MMA thread's whole loop
-            CH_ACCUM(4, i);
+            for (int k2 = kh2 - p.halo_stages < 0 ? 0 : kh2 - p.halo_stages; k2 < kh2; ++k2) {
+                const uint64_t t0 = globaltimer_ns();
+                while (!mbar_try_wait(smem_u32(&bar_h_full[k2 % p.halo_stages]), (uint32_t)(k2 / p.halo_stages) & 1u) &&
+                       globaltimer_ns() - t0 < kWaitBudgetNs) {
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ===== MMA issuer: the leader's, for the pair =====
+        if (rank == 0) {
+            // What a pass is made of is worked out by the producer (2400 clocks a pass here, while the tensor pipe ran dry), and
+            // of a descriptor only the low word, the address, is computed.
+            const uint32_t unit  = kH_RowB / 16, slot_step = (uint32_t)p.slot_bytes >> 4;
+            const uint32_t f_0   = (uint32_t)smem_desc_k<kH_RowB>(slot_base), to_f1 = (uint32_t)(THREE ? p.n >> 1 : p.n) * unit;
+            const uint32_t to_lo = (uint32_t)p.halo_plane_bytes >> 4;
+            auto desc = [](uint32_t low) { return smem_desc_k<kH_RowB>(0) & 0xffffffff00000000ull | low; };
+            int s = 0, hs = 0, acc = 0;
+            uint32_t f_phase = 0, h_phase = 0, acc_phase = 3u; // a bit per set of accumulators
+            uint32_t d_main = 0, d_cross = 0, f = f_0;
+            bool ok = true;
+            while (ok) {
+                ok = mbar_wait_warp(smem_u32(&bar_h_full[hs]), h_phase, abort_flag);
+                if (!ok)
+                    break;
+                tc_fence_after_sync();
+                const uint32_t word = __shfl_sync(0xffffffffu, *const_cast<volatile uint32_t *>(&halo_word[hs]), 0);
+                if (word & kH_Over)
+                    break;
+                if (word & kH_Reload)
+                    tc_commit_pair_warp(smem_u32(&bar_reload));
+                if (word & kH_Set)
+                    s = 0, f = f_0;
+                uint32_t accumulate = 1u;
+                if (word & kH_Begin) { // what the accumulators held before has been read
+                    ok = mbar_wait_warp(smem_u32(&bar_acc_empty[acc]), acc_phase >> acc & 1u, abort_flag);
+                    if (!ok)
+                        break;
+                    tc_fence_after_sync();
+                    acc_phase ^= 1u << acc;
+                    d_main = tmem_base + (uint32_t)(acc * 256), d_cross = d_main + (uint32_t)p.n;
+                    accumulate = 0u;
+                }
+                const uint32_t idesc = make_idesc(word & kH_Wide ? 2u : 0u, 256, (uint32_t)p.n);
+                const uint32_t idesc2 = make_idesc(word & kH_Wide ? 2u : 0u, 256, (uint32_t)(2 * p.n));
+                const uint32_t x = (uint32_t)smem_desc_k<kH_RowB>(smem_base + (uint32_t)hs * halo_stage);
+                const int t1 = (int)(word >> 6 & 63u);
+                for (int t = (int)(word & 63u); t < t1; ++t) {
+                    if (word & kH_Load) {
+                        ok = mbar_wait_warp(smem_u32(&bar_f_full[s]), f_phase, abort_flag);
+                        if (!ok)
+                            break;
+                        tc_fence_after_sync();
+                    }
+                    // the tap's pixels: the halo, so many rows of 64 bytes further on
+                    const uint32_t xh = x + p.tap_shift[t], xl = xh + to_lo;
+                    auto issue = [&](auto mma, uint32_t k) {
+                        if (THREE) {
+                            mma(d_main, desc(xh + k), desc(f + k), idesc, accumulate);
+                            mma(d_cross, desc(xh + k), desc(f + to_f1 + k), idesc, accumulate);
+                            mma(d_cross, desc(xl + k), desc(f + k), idesc, 1u);
+                        } else {
+                            mma(d_main, desc(xh + k), desc(f + k), idesc2, accumulate);
+                            mma(d_cross, desc(xl + k), desc(f + to_f1 + k), idesc, 1u);
+                        }
+                        accumulate = 1u;
+                    };
+                    if (!(word & kH_Wide)) {
+                        issue(mma_f16_pair_warp, 0);
+                        if (word & kH_Two)
+                            issue(mma_f16_pair_warp, 2);
+                    } else {
+                        issue(mma_tf32_pair_warp, 0);
+                        issue(mma_tf32_pair_warp, 2);
+                    }
+                    if (!p.resident)
+                        tc_commit_pair_warp(smem_u32(&bar_f_empty[s]));
+                    f += slot_step;
+                    if (++s == p.slots) {
+                        s = 0, f = f_0;
+                        if (word & kH_Load)
+                            f_phase ^= 1u;
+                    }
+                }
+                if (!ok)
+                    break;
+                tc_commit_pair_warp(smem_u32(&bar_h_empty[hs])); // the halo is free once its taps' MMAs have retired
+                if (++hs == p.halo_stages)
+                    hs = 0, h_phase ^= 1u;
+                if (word & kH_End) {
+                    tc_commit_pair_warp(smem_u32(&bar_acc_full[acc]));
+                    acc ^= 1;
+                }
+            }
             if (!ok || *abort_flag) {
-                tc_commit(smem_u32(&bar_done));
+                // unwind: wait until every MMA issued so far has retired
+                __syncwarp();
+                tc_commit_pair_warp(smem_u32(&bar_done));
                 const uint64_t t0 = globaltimer_ns();
                 while (!mbar_try_wait(smem_u32(&bar_done), 0) && globaltimer_ns() - t0 < kWaitBudgetNs) {
                 }
             }
         }
     } else {
-        // ===== epilogue: drain tile i to registers, release the accumulator, then store =====
-        const int ew      = warp - 2;
-        const int quarter = warp & 3;
-        const int half    = ew >> 2;
-        uint8_t *stg      = epi_base + (uint32_t)ew * kH_EpiWarpBytes;
-        // where this lane's columns land: column col = half * 128 + 32 j + lane is position
-        // (y, x) = (col / pw, col % pw); -1 for the halo columns and past the tile
-        int off[4];
-        const int npos = p.th * p.pw;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int col = half * 128 + 32 * j + lane;
-            const int y = col / p.pw, x = col - y * p.pw;
-            off[j] = (col < npos && x < p.wo) ? y * p.wo + x : -1;
-        }
-        const bool relu = p.act == CT_ACT_RELU;
-        int mains = 0, crosses = 0;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-            int tm, ty, img;
-            coords(tile, tm, ty, img);
-            const int row0     = tm * 128 + quarter * 32; // first output channel of this warp's block
-            const float inv    = p.image_scale[img];
-            const bool wide    = inv == 0.0f;
-            const float rs     = (!wide && row0 + lane < p.ko) ? p.filter_scale[row0 + lane] : 1.0f;
-            // powers of two; a missing bias is -0, which no sum notices
-            const float scale  = wide ? 1.0f : __fmul_rn(rs, inv);
-            const int ch       = row0 + lane;
-            const float bias   = !p.bias || ch >= p.ko ? -0.0f : (ch < kH_BiasSlots ? bias_s[ch] : p.bias[ch]);
-            const long long e0 = CH_CLOCK();
-            float acc[128];
-            const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 128);
-            auto await = [&](int which) {
-                const bool got = mbar_wait(smem_u32(&bar_tmem_full[which]), (uint32_t)(which ? crosses++ : mains++) & 1u, abort_flag);
+        // ===== epilogue: a lane has a position, a warp a quarter of the channels =====
+        const int quarter = warp & 3; // TMEM lanes this warp may read: 32 * quarter ..
+        const int share   = (warp - 2) >> 2, each = p.n >> 2, groups = p.n >> 5; // its channels, and groups of eight of them
+        const bool relu   = p.act == CT_ACT_RELU;
+        const int64_t plane = (int64_t)p.ho * p.wo;
+        float *scales = scale_s[warp - 2], *biases = bias_s[warp - 2];
+        int acc = 0, held = -1;
+        uint32_t acc_phase = 0;
+        bool ok = true;
+        HaloWalk walk(p, first, stride);
+        while (ok && walk.advance()) {
+            const bool wide    = walk.form != 0;
+            const float weight = wide ? 1.0f : kHalfLoInv;
+            const int img = rank ? walk.img[1] : walk.img[0], tile = rank ? walk.tile[1] : walk.tile[0];
+            // stored in the form that its image has, and once: the last tile of an odd number has no partner
+            const bool store = (rank ? walk.wide[1] : walk.wide[0]) == wide && !(rank && walk.tile[0] == walk.tile[1]);
+            const float inv  = rank ? walk.scale[1] : walk.scale[0];
+            const int q = (tile - img * p.image_tiles) * 128 + quarter * 32 + lane, y = fast_div(q, p.by_pw), x = q - y * p.pw;
+            const int ch0 = walk.tn * p.n + share * each, chunks = wide ? p.chunks_wide : p.chunks;
+            if (walk.tn != held) {
+                held = walk.tn;
+                __syncwarp();
+                if (lane < each)
+                    scales[lane] = p.filter_scale[ch0 + lane], biases[lane] = p.bias[ch0 + lane];
+                __syncwarp();
+            }
+            float sum[32];
+#pragma unroll 1
+            for (int e = 0; e < chunks; ++e) {
+                ok = mbar_wait_patient_warp(smem_u32(&bar_acc_full[acc]), acc_phase >> acc & 1u, abort_flag);
+                if (!ok)
+                    break;
+                acc_phase ^= 1u << acc;
                 tc_fence_after_sync();
-                return __all_sync(0xffffffffu, got) != 0;
-            };
-            auto hand_back = [&](int which) {
+                const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * 256 + share * each);
+                auto take = [&](int at, uint32_t main, uint32_t cross) {
+                    const float v = __fadd_rn(__uint_as_float(main), __fmul_rn(__uint_as_float(cross), weight));
+                    sum[at]       = e == 0 ? v : __fadd_rn(sum[at], v);
+                };
+#pragma unroll
+                for (int g = 0; g < 4; g += 2) {
+                    if (groups >= g + 2) {
+                        uint32_t m[16], c[16];
+                        tmem_ld_32x16(taddr + (uint32_t)(8 * g), m);
+                        tmem_ld_32x16(taddr + (uint32_t)(p.n + 8 * g), c);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int u = 0; u < 16; ++u)
+                            take(8 * g + u, m[u], c[u]);
+                    } else if (groups == g + 1) {
+                        uint32_t m[8], c[8];
+                        tmem_ld_32x8(taddr + (uint32_t)(8 * g), m);
+                        tmem_ld_32x8(taddr + (uint32_t)(p.n + 8 * g), c);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int u = 0; u < 8; ++u)
+                            take(8 * g + u, m[u], c[u]);
+                    }
+                }
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0)
-                    mbar_arrive(smem_u32(&bar_tmem_empty[which]));
-            };
-            // The leading accumulator of every chunk but the last, the cross products, the last chunk.
-            // The first of them straight into the sums, with one wait for all columns.
-            const int cblocks = p.c_pad / (wide ? 16 : 32), chunk = wide ? p.chunk_wide : p.chunk_blocks, chunks = (cblocks + chunk - 1) / chunk;
-            const int events  = chunks + 1;
-            const float cross = wide ? 1.0f : kHalfLoInv;
-            auto which_of     = [&](int e) { return e == chunks - 1 ? 1 : 0; };
-            const int first_acc = which_of(0);
-            if (!await(first_acc))
-                break;
-            {
-                uint32_t r[4][32];
-#pragma unroll
-                for (int g = 0; g < 4; ++g)
-                    tmem_ld_32x32(lane_base + (uint32_t)(first_acc * 256 + g * 32), r[g]);
-                tmem_ld_wait();
-                hand_back(first_acc);
-                const float weight = first_acc ? cross : 1.0f;
-#pragma unroll
-                for (int j = 0; j < 128; ++j)
-                    acc[j] = __fmul_rn(__uint_as_float(r[j / 32][j % 32]), weight);
-            }
-            bool ok = true;
-#pragma unroll 1
-            for (int e = 1; e < events; ++e) {
-                const int which    = which_of(e);
-                const float weight = which ? cross : 1.0f;
-                ok                 = await(which);
-                if (!ok)
-                    break;
-#pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                    uint32_t r[16];
-                    tmem_ld_32x16(lane_base + (uint32_t)(which * 256 + g * 16), r);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        acc[g * 16 + j] = __fadd_rn(acc[g * 16 + j], __fmul_rn(__uint_as_float(r[j]), weight));
-                }
-                hand_back(which);
+                    mbar_arrive_cluster(leader_addr(smem_u32(&bar_acc_empty[acc])));
+                acc ^= 1;
             }
             if (!ok)
                 break;
-            const long long e1 = CH_CLOCK();
-
-            const int y0   = ty * p.th;
-            // positions of rows past the image's last row (a partial last tile) are dropped:
-            // position col lies in row col / pw, so the valid ones are col < rows_left * pw
-            const int col_limit = (p.ho - y0 < p.th ? p.ho - y0 : p.th) * p.pw;
-            // Scales, bias and activation where a lane has a channel, with its constants in registers; what remains for the
-            // stores is a read, an address and the store.  (With them behind the exchange, a value took 35 instructions and
-            // a tile the epilogue 18,000 clocks, four thousand more than its MMAs.)
-            const int64_t plane = (int64_t)p.ho * p.wo;
-            float *out_img = p.out + ((int64_t)img * p.ko + row0) * plane + (int64_t)y0 * p.wo;
-            const int rows = p.ko - row0 < 32 ? p.ko - row0 : 32;
+            if (store) {
+                const bool live = x < p.wo && y < p.ho;
+                float *at       = p.out + ((int64_t)img * p.ko + ch0) * plane + (int64_t)y * p.wo + x;
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                if (half * 128 + g * 32 >= npos || rows <= 0)
-                    break;
-                float4 *mine = reinterpret_cast<float4 *>(stg + lane * kH_EpiRowBytes);
+                for (int g = 0; g < 4; ++g) {
+                    if (g < groups && ch0 + 8 * g < p.ko) {
+                        float fs[8], bs[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    float y[4];
+                        for (int u = 0; u < 8; u += 4) {
+                            *reinterpret_cast<float4 *>(fs + u) = *reinterpret_cast<const float4 *>(scales + 8 * g + u);
+                            *reinterpret_cast<float4 *>(bs + u) = *reinterpret_cast<const float4 *>(biases + 8 * g + u);
+                        }
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        y[q] = __fadd_rn(__fmul_rn(acc[g * 32 + 4 * j + q], scale), bias);
-                        y[q] = !relu || y[q] > 0.0f ? y[q] : __fmul_rn(y[q], 0.0f);
+                        for (int u = 0; u < 8; ++u, at += plane) {
+                            const float scale = wide ? 1.0f : __fmul_rn(fs[u], inv); // powers of two
+                            float v = __fadd_rn(__fmul_rn(sum[8 * g + u], scale), bs[u]);
+                            v       = !relu || v > 0.0f ? v : __fmul_rn(v, 0.0f);
+                            if (live && ch0 + 8 * g + u < p.ko)
+                                *at = v;
+                        }
                     }
-                    mine[j] = make_float4(y[0], y[1], y[2], y[3]);
                 }
-                __syncwarp();
-                // a column per lane, so that a store covers consecutive pixels of a channel (four columns per lane wrote every
-                // sector four times: 256 x 64 x 56 x 56 -> 128 530 us, 491 so)
-                const float *src = reinterpret_cast<const float *>(stg) + lane;
-                float *dst       = out_img + (off[g] < 0 ? 0 : off[g]);
-                if (off[g] >= 0 && half * 128 + g * 32 + lane < col_limit) {
-                    int r = 0;
-#pragma unroll 1
-                    for (; r + 8 <= rows; r += 8) {
-                        float x[8];
-#pragma unroll
-                        for (int u = 0; u < 8; ++u)
-                            x[u] = src[(r + u) * (kH_EpiRowBytes / 4)];
-#pragma unroll
-                        for (int u = 0; u < 8; ++u, dst += plane)
-                            *dst = x[u];
-                    }
-#pragma unroll 1
-                    for (; r < rows; ++r, dst += plane)
-                        *dst = src[r * (kH_EpiRowBytes / 4)];
-                }
-                __syncwarp(); // the block is rewritten by the next columns
-            }
-            if (warp == 2 && lane == 0) {
-                CH_ACCUM(5, e1 - e0);          // epilogue: waiting for a complete accumulator
-                CH_ACCUM(6, CH_CLOCK() - e1);  // drain and store
             }
         }
     }
 
     tc_fence_before_sync();
     __syncthreads();
+    cluster_sync(); // neither CTA goes while the other's MMAs, copies or arrivals may still reach it
     if (warp == 1) {
         __syncwarp();
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, 512);
+        tmem_dealloc_pair(tmem_base, 512);
     }
     if (threadIdx.x == 0 && !failed && *abort_flag)
         atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
@@ -511,6 +559,8 @@ struct FilterPlanes {
     __half *hi16, *lo16;
     float *hi32, *lo32;
     float *scale;
+    const float *bias; // the layer's, or null
+    float *bias_out;   // its copy, -0 where there is none; null: not wanted
 };
 __global__ void __launch_bounds__(256) conv_range_kernel(
     const float *__restrict__ w, int c, int taps, int c_pad, int ko, const FilterPlanes f, const float *__restrict__ x,
@@ -551,8 +601,11 @@ __global__ void __launch_bounds__(256) conv_range_kernel(
     }
     float scale, inverse;
     const bool fits = half_range_fits(r, scale, inverse);
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0) {
         f.scale[o] = fits ? inverse : 0.0f;
+        if (f.bias_out)
+            f.bias_out[o] = f.bias ? f.bias[o] : -0.0f;
+    }
     if (f.hi16 == nullptr)
         return;
     for (int i = threadIdx.x; i < taps * c_pad; i += 256) {
@@ -568,14 +621,14 @@ __global__ void __launch_bounds__(256) conv_range_kernel(
 // under the image's scale, or tf32 terms (image_scale 0) where the image or any filter does not fit those.  A
 // block takes 64 channels by 64 positions through shared memory: reads of 256 contiguous bytes, writes of 128.  The
 // images are taken last to first: the end of the tensor is what conv_range_kernel has just left in L2.
-// Sub-images (ConvSubImages, hs x ws each): zeros where the image has no such row or column, those that no tap reads are
-// left out.
+// Sub-images (ConvSubImages, hs x ws each, from row y0 and column x0 of the input on): zeros where the image has no such row or
+// column, which is a layer's padding; those that no tap reads are left out.
 //
 // What bounds it is issue (0.83 of the slots at 128 x 64 x 56 x 56), so the moduli are constants, the one division left is a
 // multiplication, and one warp works the image's scale out for all: 64 x 48 x 57 x 57 -> 96 at stride 2 76 -> 69 us (31 of it this kernel
 // before), 256 x 64 x 56 x 56 -> 128 428 -> 425.
 struct PlaneGeom {
-    int h, w, hs, ws;
+    int h, w, hs, ws, y0, x0;
     uint32_t width_inv; // 2^32 / (ws * col_mod), rounded up; 0 for a width of 1
     ConvSubImages sub;
 };
@@ -594,8 +647,7 @@ __global__ void __launch_bounds__(256) conv_planes_kernel(
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t in_hw = (int64_t)geom.h * geom.w;
     const int width  = geom.ws * COL_MOD;
-    const int64_t hw = (int64_t)geom.hs * ROW_MOD * width; // positions of the image grown to whole multiples
-    constexpr bool apart = ROW_MOD * COL_MOD > 1;
+    const int64_t hw = (int64_t)geom.hs * ROW_MOD * width; // positions of the grown image
     const float *src = x + (img * c + c0) * in_hw;
     auto row_of = [&](int64_t q) { // q < 2^31: the rounded-up quotient is one too high at most
         const int row = geom.width_inv ? (int)__umulhi((uint32_t)q, geom.width_inv) : (int)q;
@@ -603,10 +655,8 @@ __global__ void __launch_bounds__(256) conv_planes_kernel(
     };
     // position q of the grown image in the input (-1: not there)
     auto source = [&](int64_t q) -> int64_t {
-        if (!apart)
-            return q < hw ? q : -1;
-        const int row = row_of(q), col = (int)q - row * width;
-        return q < hw && row < geom.h && col < geom.w ? (int64_t)row * geom.w + col : -1;
+        const int row = row_of(q), y = row + geom.y0, x = (int)q - row * width + geom.x0;
+        return q < hw && (unsigned)y < (unsigned)geom.h && (unsigned)x < (unsigned)geom.w ? (int64_t)y * geom.w + x : -1;
     };
     float v[16]; // every load before the first use of any
 #pragma unroll
@@ -645,7 +695,7 @@ __global__ void __launch_bounds__(256) conv_planes_kernel(
         if (q0 + q >= hw || c0 + chunk * 8 >= c_pad)
             continue;
         int64_t to = q0 + q;
-        if (apart) {
+        if (ROW_MOD * COL_MOD > 1) {
             const int row = row_of(to), col = (int)to - row * width, sub = row % ROW_MOD * COL_MOD + col % COL_MOD;
             if (!(geom.sub.used >> sub & 1u))
                 continue;
@@ -681,44 +731,58 @@ __global__ void __launch_bounds__(256) conv_planes_kernel(
 }
 
 struct HaloGeom {
-    int pw, wo, ho, th, n_mma, box_rows, plane_bytes, stages;
-    int hs, ws;         // extents of a sub-image
+    int pw, wo, ho;
+    int hs;             // rows of a sub-image; it has pw columns
     int y_min, x_min;   // smallest row and column offset of a tap in its sub-image
+    int image_tiles, box_rows, boxes, plane_bytes, stages;
+    int n, tiles_n, slots, slot_bytes, resident, three;
     size_t smem;
 };
 
 int floor_div(int64_t a, int64_t b) { return (int)(a >= 0 ? a / b : -((-a + b - 1) / b)); }
 
 // Tap (r, q) of output (oy, ox) reads input row oy * stride - pad + r = stride * (oy + a) + py: row oy + a of the
-// sub-image py, and so for columns.  A tile is th rows of pw = wo + (largest - smallest b) positions.
-bool halo_geometry(int64_t h, int64_t w, int64_t kh, int64_t kw, int64_t stride, int64_t pad, HaloGeom *g) {
+// sub-image py, and so for columns.  The planes hold rows y_min .. of each sub-image and pw = wo + (largest - smallest b)
+// columns from x_min on.
+bool halo_geometry(int64_t c_pad, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw, int64_t stride, int64_t pad, HaloGeom *g) {
     if (w + 2 * pad < kw || h + 2 * pad < kh || pad > 256 || kh > 256 || kw > 256)
         return false;
     const int64_t wo = (w + 2 * pad - kw) / stride + 1, ho = (h + 2 * pad - kh) / stride + 1;
     g->y_min = floor_div(-pad, stride), g->x_min = floor_div(-pad, stride);
     const int64_t span_y = floor_div(kh - 1 - pad, stride) - g->y_min, span_x = floor_div(kw - 1 - pad, stride) - g->x_min;
     const int64_t pw = wo + span_x;
-    g->hs = (int)((h + stride - 1) / stride), g->ws = (int)((w + stride - 1) / stride);
     if (pw > 256)
         return false;
-    // as many rows as 256 columns of the accumulator and the shared memory take
-    for (int64_t th = std::min<int64_t>(256 / pw, ho); th >= 1; --th) {
-        if (th + span_y > 256)
-            continue;
-        g->pw = (int)pw, g->wo = (int)wo, g->ho = (int)ho, g->th = (int)th;
-        g->n_mma    = (int)((th * pw + 15) / 16 * 16);
-        g->box_rows = (int)(th + span_y);
-        // a tap's shifted window of n_mma rows may run past the box: reserve those rows too
-        const int64_t rows = std::max<int64_t>(span_y * pw + span_x + g->n_mma, (int64_t)g->box_rows * pw);
-        g->plane_bytes     = (int)((rows * kH_RowB + 1023) & ~1023ll);
-        // 227 KB per CTA less the kernel's static shared memory
-        const int rest = 225 * 1024 - kH_AStages * kH_AStageBytes - kH_EpiBytes - 1024;
-        g->stages      = std::min(kH_HaloStages, rest / (2 * g->plane_bytes));
-        g->smem = (size_t)kH_AStages * kH_AStageBytes + (size_t)g->stages * 2 * g->plane_bytes + kH_EpiBytes + 1024;
-        if (g->stages >= 2)
-            return true;
+    g->pw = (int)pw, g->wo = (int)wo, g->ho = (int)ho, g->hs = (int)(ho + span_y);
+    g->image_tiles = (int)((ho * pw + 127) / 128);
+    // a halo: the tile's positions and those that its last one's taps reach, in boxes of whole swizzle atoms
+    const int64_t rows = 128 + span_y * pw + span_x;
+    g->boxes       = (int)((rows + 255) / 256);
+    g->box_rows    = (int)(((rows + g->boxes - 1) / g->boxes + 7) / 8 * 8);
+    g->plane_bytes = (g->boxes * g->box_rows * kH_RowB + 1023) & ~1023;
+    // tiles of equal numbers of filters, in steps of 32 (the columns of an MMA of two CTAs)
+    g->tiles_n    = (int)((ko + 127) / 128);
+    g->n          = (int)(((ko + g->tiles_n - 1) / g->tiles_n + 31) / 32 * 32);
+    const int64_t all = kh * kw * (c_pad / 32);
+    const int budget  = kH_Smem - 1024, halo = 2 * g->plane_bytes;
+    // the terms shared out by halves (see the top) for many filters, and where the other way's memory does not hold them all
+    const int both = g->n * kH_RowB * 3 / 2;
+    auto fits      = [&](int64_t bytes) { return all <= kH_MaxSlots && all * bytes + 2 * halo <= budget; };
+    g->three       = g->n >= 96 || !fits(both);
+    g->slot_bytes  = g->three ? g->n * kH_RowB : both;
+    g->resident    = fits(g->slot_bytes);
+    if (g->resident) {
+        g->slots  = (int)all;
+        g->stages = std::min(kH_HaloStages, (budget - g->slots * g->slot_bytes) / halo);
+    } else {
+        // a third halo where that leaves a ring of eight k-blocks
+        g->stages = 3 * halo + 8 * g->slot_bytes <= budget ? 3 : 2;
+        g->slots  = (int)std::min<int64_t>(std::min<int64_t>(16, all), (budget - g->stages * halo) / g->slot_bytes);
+        if (budget < g->stages * halo || g->slots < std::min<int64_t>(4, all))
+            return false;
     }
-    return false;
+    g->smem = 1024 + (size_t)g->stages * halo + (size_t)g->slots * g->slot_bytes;
+    return true;
 }
 
 } // namespace
@@ -733,24 +797,22 @@ int conv_range_slices(int64_t batch, int64_t count) {
 // The pre-pass of a layer: the filters' scales and (filters16 non-null) planes, the images' planes and scales.
 // ranges: batch * conv_range_slices(batch, c * hw) pairs of words.
 ct_status conv_prepass(
-    DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t h, int64_t wd, int64_t c_pad, int64_t ko,
-    int64_t taps, void *filters16, void *filters32, size_t plane16, size_t plane32, float *filter_scale, void *ranges, float *image_scale,
-    void *slots, const ConvSubImages &sub) {
-    (void)st;
-    const int64_t hw = h * wd;
+    const float *x, const float *w, int64_t batch, int64_t c, int64_t h, int64_t wd, int64_t c_pad, int64_t ko, int64_t taps,
+    void *filters16, void *filters32, size_t plane16, size_t plane32, float *filter_scale, const float *bias, float *bias_copy,
+    void *ranges, float *image_scale, void *slots, const ConvSubImages &sub) {
     if (batch > 65535 || c_pad / 32 > 65535)
         return fail(CT_ERR_TOO_LARGE, "conv2d: batch or channel count too large for the layout pre-pass");
-    const int64_t count = c * hw;
+    const int64_t count = c * h * wd;
     const int slices    = conv_range_slices(batch, count);
     const int vec       = (count & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
     uint8_t *f16 = static_cast<uint8_t *>(filters16), *f32 = static_cast<uint8_t *>(filters32);
     const FilterPlanes f{reinterpret_cast<__half *>(f16), reinterpret_cast<__half *>(f16 + plane16), reinterpret_cast<float *>(f32),
-                         reinterpret_cast<float *>(f32 + plane32), filter_scale};
+                         reinterpret_cast<float *>(f32 + plane32), filter_scale, bias, bias_copy};
     ProfScope prof("conv_prepass");
     CT_CUDA(launch_dependent(conv_range_kernel, dim3((unsigned)(ko + batch * slices)), dim3(256), 0, stream(), w, (int)c, (int)taps,
                              (int)c_pad, (int)ko, f, x, count, slices, vec, static_cast<uint2 *>(ranges)));
     CT_LAUNCH_CHECK("conv_range");
-    PlaneGeom geom{(int)h, (int)wd, (int)((h + sub.row_mod - 1) / sub.row_mod), (int)((wd + sub.col_mod - 1) / sub.col_mod), 0, sub};
+    PlaneGeom geom{(int)h, (int)wd, sub.rows, sub.cols, sub.y0, sub.x0, 0, sub};
     const int64_t width = (int64_t)geom.ws * sub.col_mod, positions = geom.hs * width * sub.row_mod;
     geom.width_inv = width > 1 ? (uint32_t)(((1ull << 32) + width - 1) / width) : 0;
     const dim3 grid((unsigned)((positions + 63) / 64), (unsigned)((c_pad + 63) / 64), (unsigned)batch);
@@ -770,56 +832,62 @@ ct_status conv_prepass(
     return CT_OK;
 }
 
-// Whether the halo kernel takes this layer (float32 mode only): filters and strides within its tables, whole k-blocks
-// of a tap list within one drain, and a tile that is reasonably full.
+// Whether the halo kernel takes this layer (float32 mode only): filters and strides within its tables, planes whose positions
+// 32 bits count, and tiles that are reasonably full.
 bool conv_halo_applicable(int64_t c_pad, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw, int64_t stride,
                           int64_t pad) {
     HaloGeom g;
     if (stride < 1 || stride > kH_MaxStride || ko < kH_MinFilters || kh * kw > kH_MaxTaps || (c_pad % 32) != 0 ||
         c_pad > (1 << 20) || h > 0x3fff || w > 0x3fff)
         return false;
-    if (!halo_geometry(h, w, kh, kw, stride, pad, &g))
+    if (!halo_geometry(c_pad, h, w, ko, kh, kw, stride, pad, &g))
         return false;
-    // at least 70 % of the columns carry an output, and not a few rows only because shared memory holds no more
-    return (int64_t)g.th * g.wo * 10 >= (int64_t)g.n_mma * 7 && (g.n_mma >= 128 || g.th == g.ho);
+    // measured down to 47 % of the rows with an output (256 x 64 x 11 x 11 -> 128 38 us, 73 through patches)
+    return (int64_t)g.ho * g.wo * 100 >= (int64_t)g.image_tiles * 128 * 45;
 }
 
-// Workspace: [filter scale][image scale][image ranges][w hi16][w lo16][w hi][w lo][image slots]; a slot holds an
+// Workspace: [filter scale][bias][image scale][image ranges][w hi16][w lo16][w hi][w lo][image slots]; a slot holds an
 // image's planes, float16 pairs or, where it does not fit those, tf32: no more than tf32 planes alone take.
 ct_status conv_halo(
     DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t c_pad, int64_t h, int64_t wd, int64_t ko,
     int64_t kh, int64_t kw, int64_t stride, int64_t pad, const float *bias, int act, float *out) {
     HaloGeom g;
-    if (!halo_geometry(h, wd, kh, kw, stride, pad, &g))
+    if (!halo_geometry(c_pad, h, wd, ko, kh, kw, stride, pad, &g))
         return fail(CT_ERR_INVALID, "conv2d: internal tile shape not usable");
     auto align_up          = [](size_t v) { return (v + 1023) & ~(size_t)1023; };
-    const int64_t taps     = kh * kw, subs = stride * stride, sub = (int64_t)g.hs * g.ws, hw = sub * subs;
+    const int64_t taps     = kh * kw, subs = stride * stride, sub = (int64_t)g.hs * g.pw, positions = sub * subs;
+    const int64_t tiles    = g.image_tiles * batch, pairs = (tiles + 1) / 2, items = pairs * g.tiles_n;
+    if (items > 0x3fffffffll || positions > 0x3fffffffll)
+        return fail(CT_ERR_TOO_LARGE, "conv2d: too many tiles");
     const size_t w16       = align_up((size_t)ko * taps * c_pad * 2), w32 = align_up((size_t)ko * taps * c_pad * 4);
-    const size_t slot      = (size_t)hw * c_pad * 8;
-    const size_t w_words   = align_up((size_t)ko * 4), x_words = align_up((size_t)batch * 4);
+    const size_t slot      = (size_t)positions * c_pad * 8;
+    const size_t w_words   = align_up((size_t)g.n * g.tiles_n * 4), x_words = align_up((size_t)batch * 4);
     const size_t ranges    = align_up((size_t)batch * conv_range_slices(batch, c * h * wd) * 8);
-    CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, w_words + x_words + ranges + 2 * w16 + 2 * w32 + (size_t)batch * slot));
+    CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, 2 * w_words + x_words + ranges + 2 * w16 + 2 * w32 + (size_t)batch * slot));
     uint8_t *ws            = static_cast<uint8_t *>(st->gemm_ws);
-    float *filter_scale    = reinterpret_cast<float *>(ws), *image_scale = reinterpret_cast<float *>(ws + w_words);
-    uint8_t *w16_hi        = ws + w_words + x_words + ranges, *w32_hi = w16_hi + 2 * w16, *xp = w32_hi + 2 * w32;
+    float *filter_scale    = reinterpret_cast<float *>(ws), *bias_copy = reinterpret_cast<float *>(ws + w_words);
+    float *image_scale     = reinterpret_cast<float *>(ws + 2 * w_words);
+    uint8_t *range_words   = ws + 2 * w_words + x_words;
+    uint8_t *w16_hi        = range_words + ranges, *w32_hi = w16_hi + 2 * w16, *xp = w32_hi + 2 * w32;
     ConvHaloParams p;
-    p.filter_scale = filter_scale, p.image_scale = image_scale;
-    p.bias = bias, p.out = out, p.flags = st->flags_dev;
-    p.ko = (int)ko, p.tiles_m = (int)((ko + 127) / 128);
-    p.ho = g.ho, p.wo = g.wo, p.pw = g.pw, p.th = g.th;
-    p.tiles_y = (g.ho + g.th - 1) / g.th;
-    p.box_x0 = g.x_min, p.box_y0 = g.y_min;
+    p.filter_scale = filter_scale, p.bias = bias_copy, p.image_scale = image_scale;
+    p.out = out, p.flags = st->flags_dev;
+    p.ko = (int)ko, p.n = g.n;
+    p.ho = g.ho, p.wo = g.wo, p.pw = g.pw;
+    p.image_tiles = g.image_tiles, p.total_tiles = (int)tiles, p.pairs = (int)pairs, p.items = (int)items;
     p.chunk_blocks = (int)std::max<int64_t>(1, kH_MaxK / (32 * taps));
     // a strided layer's tf32 images: no longer chains of truncating additions than the float16 ones have (3.0e-6 -> 3.7e-7 against
     // 64 bits at 48 channels, 3 x 3; all 64 images 110 -> 117 us); unstrided, with the cross products apart, 4.0e-6 -> 1.4e-6
     p.chunk_wide = stride > 1 ? 1 : 2 * p.chunk_blocks;
+    p.chunks     = (int)(c_pad / 32 + p.chunk_blocks - 1) / p.chunk_blocks, p.chunks_wide = (int)(c_pad / 16 + p.chunk_wide - 1) / p.chunk_wide;
     p.c       = (int)c;
     p.last_first = c % 16 != 0;
     p.c_pad   = (int)c_pad;
-    p.n_mma   = g.n_mma;
-    p.box_bytes        = g.box_rows * g.pw * kH_RowB;
+    p.box_rows = g.box_rows, p.boxes = g.boxes;
     p.halo_plane_bytes = g.plane_bytes, p.halo_stages = g.stages;
+    p.slots = g.slots, p.slot_bytes = g.slot_bytes, p.resident = g.resident;
     p.act = act;
+    p.by_pairs = fast_divisor(pairs), p.by_tiles = fast_divisor(g.image_tiles), p.by_pw = fast_divisor(g.pw);
     p.halos = 0, p.halo_taps[0] = 0;
     uint32_t used = 0;
     for (int image = 0, listed = 0; image < (int)subs; ++image) {
@@ -828,46 +896,44 @@ ct_status conv_halo(
             if ((r - a * (int)stride) * (int)stride + (q - b * (int)stride) != image)
                 continue;
             p.tap[listed]         = (uint8_t)t;
-            p.tap_shift[listed++] = (uint16_t)((a - g.y_min) * g.pw + (b - g.x_min));
+            p.tap_shift[listed++] = (uint16_t)(((a - g.y_min) * g.pw + (b - g.x_min)) * (kH_RowB / 16));
         }
         if (listed > p.halo_taps[p.halos]) {
-            p.halo_image[p.halos]  = (uint8_t)image;
+            p.halo_at[p.halos]     = (int)(image * sub);
             p.halo_taps[++p.halos] = (uint8_t)listed;
             used |= 1u << image;
         }
     }
-    CT_TRY(conv_prepass(st, x, w, batch, c, h, wd, c_pad, ko, taps, w16_hi, w32_hi, w16, w32, filter_scale, ws + w_words + x_words,
-                        image_scale, xp, ConvSubImages{(int)stride, (int)stride, used, false}));
-    const int64_t tiles = (int64_t)p.tiles_m * p.tiles_y * batch;
-    if (tiles > 0x7fffffffll)
-        return fail(CT_ERR_TOO_LARGE, "conv2d: too many tiles");
+    const ConvSubImages images{(int)stride, (int)stride, used, false, g.hs, g.pw, g.y_min * (int)stride, g.x_min * (int)stride};
+    CT_TRY(conv_prepass(x, w, batch, c, h, wd, c_pad, ko, taps, w16_hi, w32_hi, w16, w32, filter_scale, bias, bias_copy, range_words,
+                        image_scale, xp, images));
     ConvHaloMaps maps;
-    auto encode = [&](CUtensorMap *mw, const uint8_t *wp, CUtensorMap *mx, const uint8_t *xpl, int elem) {
+    const bool three = g.three != 0;
+    auto encode = [&](CUtensorMap *mw, const uint8_t *wp, size_t w_plane, CUtensorMap *mx_hi, CUtensorMap *mx_lo, int elem) {
         const uint64_t kp = (uint64_t)(taps * c_pad), row = (uint64_t)(c_pad * elem);
         const uint64_t wdims[2] = {kp, (uint64_t)ko}, wstr[1] = {kp * (uint64_t)elem};
-        const uint32_t wbox[2]  = {(uint32_t)(kH_RowB / elem), 128};
-        const uint64_t xdims[5] = {(uint64_t)c_pad, (uint64_t)g.ws, (uint64_t)g.hs, (uint64_t)subs, (uint64_t)batch};
-        const uint64_t xstr[4]  = {row, row * (uint64_t)g.ws, row * (uint64_t)sub, slot};
-        const uint32_t xbox[5]  = {(uint32_t)(kH_RowB / elem), (uint32_t)g.pw, (uint32_t)g.box_rows, 1, 1};
+        const uint32_t whalf[2] = {(uint32_t)(kH_RowB / elem), (uint32_t)(g.n / 2)}, wfull[2] = {(uint32_t)(kH_RowB / elem), (uint32_t)g.n};
+        const uint64_t xdims[3] = {(uint64_t)c_pad, (uint64_t)positions, (uint64_t)batch}, xstr[2] = {row, slot};
+        const uint32_t xbox[3]  = {(uint32_t)(kH_RowB / elem), (uint32_t)g.box_rows, 1};
         auto fn = elem == 4 ? encode_tiled_map_f32 : encode_tiled_map_f16;
-        CT_TRY(fn(mw, wp, 2, wdims, wstr, wbox, kH_RowB));
-        return fn(mx, xpl, 5, xdims, xstr, xbox, kH_RowB);
+        CT_TRY(fn(&mw[0], wp, 2, wdims, wstr, whalf, kH_RowB));
+        CT_TRY(fn(&mw[1], wp + w_plane, 2, wdims, wstr, three ? whalf : wfull, kH_RowB));
+        CT_TRY(fn(&mw[2], wp, 2, wdims, wstr, wfull, kH_RowB));
+        CT_TRY(fn(mx_hi, xp, 3, xdims, xstr, xbox, kH_RowB));
+        return fn(mx_lo, xp + (size_t)positions * c_pad * elem, 3, xdims, xstr, xbox, kH_RowB);
     };
-    CT_TRY(encode(&maps.w16_hi, w16_hi, &maps.x16_hi, xp, 2));
-    CT_TRY(encode(&maps.w16_lo, w16_hi + w16, &maps.x16_lo, xp + slot / 4, 2));
-    CT_TRY(encode(&maps.w32_hi, w32_hi, &maps.x32_hi, xp, 4));
-    CT_TRY(encode(&maps.w32_lo, w32_hi + w32, &maps.x32_lo, xp + slot / 2, 4));
-    // the kernel also has a little static shared memory (barriers, the bias): ask for exactly what
-    // this geometry needs, remembering the largest request per device
-    static size_t attr_bytes_dev[16] = {};
-    size_t &attr_bytes = attr_bytes_dev[st->device & 15];
-    if (g.smem > attr_bytes) {
-        CT_CUDA(cudaFuncSetAttribute(conv_halo_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
-        attr_bytes = g.smem;
+    CT_TRY(encode(maps.w16, w16_hi, w16, &maps.x16_hi, &maps.x16_lo, 2));
+    CT_TRY(encode(maps.w32, w32_hi, w32, &maps.x32_hi, &maps.x32_lo, 4));
+    static bool attr_set_dev[16] = {}; // the attribute belongs to a device's context
+    if (!attr_set_dev[st->device & 15]) {
+        CT_CUDA(cudaFuncSetAttribute(conv_halo_stream_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kH_Smem));
+        CT_CUDA(cudaFuncSetAttribute(conv_halo_stream_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kH_Smem));
+        attr_set_dev[st->device & 15] = true;
     }
-    const unsigned grid = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
+    const unsigned grid = 2u * (unsigned)std::min<int64_t>(items, st->sm_count / 2);
     ProfScope prof("gemm_tc");
-    CT_CUDA(launch_dependent(conv_halo_stream_kernel, dim3(grid), dim3(kH_Threads), g.smem, stream(), maps, p, (int)tiles));
+    CT_CUDA(launch_dependent_cluster(three ? conv_halo_stream_kernel<true> : conv_halo_stream_kernel<false>, 2, dim3(grid), dim3(kH_Threads),
+                                     g.smem, stream(), maps, p));
     CT_LAUNCH_CHECK("conv_halo_stream");
     return CT_OK;
 }

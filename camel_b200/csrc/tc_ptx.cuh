@@ -128,6 +128,18 @@ __device__ __forceinline__ bool mbar_wait_patient(uint32_t bar, uint32_t parity,
     }
 }
 
+// The two for a converged warp: the answer is the same for all lanes, and known to be.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    bool got = mbar_try_wait(bar, parity);
+    if (!__all_sync(0xffffffffu, got))
+        got = mbar_wait(bar, parity, abort_flag);
+    return __all_sync(0xffffffffu, got) != 0;
+}
+__device__ __forceinline__ bool mbar_wait_patient_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    const bool got = mbar_wait_patient(bar, parity, abort_flag);
+    return __all_sync(0xffffffffu, got) != 0;
+}
+
 // ---- TMA --------------------------------------------------------------------------------
 
 __device__ __forceinline__ void prefetch_tensormap(const void *map) {
@@ -345,6 +357,45 @@ __device__ __forceinline__ void mma_tf32_pair(
         "}\n"
         :
         : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// The same for a whole converged warp whose control flow and operands are uniform, of which one lane issues: addresses and
+// descriptors then stay in the uniform registers that the instruction reads.
+__device__ __forceinline__ void mma_f16_pair_warp(
+    uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "}\n"
+        :
+        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void mma_tf32_pair_warp(
+    uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t"
+        "}\n"
+        :
+        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tc_commit_pair_warp(uint32_t bar) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t"
+        "}\n" ::"r"(bar),
+        "h"((uint16_t)3)
         : "memory");
 }
 

@@ -35,12 +35,14 @@ struct ConvSubImages {
     int row_mod = 1, col_mod = 1;
     uint32_t used = 1;
     bool tf32_plain = false;
+    int rows = 0, cols = 0; // of a sub-image
+    int y0 = 0, x0 = 0;     // the input's row and column that row 0 and column 0 of the first one are
 };
 int conv_range_slices(int64_t batch, int64_t count);
 ct_status conv_prepass(
-    DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t h, int64_t wd, int64_t c_pad, int64_t ko,
-    int64_t taps, void *filters16, void *filters32, size_t plane16, size_t plane32, float *filter_scale, void *ranges, float *image_scale,
-    void *slots, const ConvSubImages &sub);
+    const float *x, const float *w, int64_t batch, int64_t c, int64_t h, int64_t wd, int64_t c_pad, int64_t ko, int64_t taps,
+    void *filters16, void *filters32, size_t plane16, size_t plane32, float *filter_scale, const float *bias, float *bias_copy,
+    void *ranges, float *image_scale, void *slots, const ConvSubImages &sub);
 // x NCHW and w OIHW float32; c_pad: channels rounded up to 32.
 ct_status conv_halo(
     DeviceState *st, const float *x, const float *w, int64_t batch, int64_t c, int64_t c_pad, int64_t h, int64_t wd, int64_t ko,

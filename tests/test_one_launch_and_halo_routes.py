@@ -61,6 +61,26 @@ def test_layers_at_the_edges_of_their_tiles(T, port, layer, kind):
         assert pooled.numpy().tobytes() == T.maxpool2d(got, 2).numpy().tobytes()
 
 
+# Several passes to a pair of blocks: images of both forms next to each other, one tile to an image (the halves of a pair differ, and the
+# last has no partner) and two; filters that stay in shared memory, in both layouts, and filters that are streamed, in two tiles.
+@pytest.mark.parametrize("layer", [(161, 40, 10, 10, 40, 3, 3, 1, 1), (80, 40, 12, 12, 128, 3, 3, 1, 1), (45, 196, 13, 13, 130, 3, 3, 1, 1)])
+def test_images_of_both_forms_in_one_batch(T, port, layer):
+    n, c, h, w, ko, kh, kw, stride, pad = layer
+    rng = np.random.default_rng(sum(layer))
+    x = rng.standard_normal((n, c, h, w)).astype(np.float32)
+    wide = rng.random(n) < 0.3
+    wide[-1], wide[-2] = True, False
+    x[wide, 0, 3, 3] = 1e-20
+    f = rng.standard_normal((ko, c, kh, kw)).astype(np.float32)
+    tf = T.from_numpy(f)
+    got = T.conv2d(T.from_numpy(x), tf, None, stride, pad).numpy()
+    T.check_async()
+    assert np.all(np.abs(got - port.conv2d(x, f, None, stride, pad, 0)) <= BOUND * port.conv2d(np.abs(x), np.abs(f), None, stride, pad, 0))
+    for i in (0, 7, n - 2, n - 1):  # an image's bytes do not depend on the others
+        same = T.conv2d(T.from_numpy(np.stack([x[i]] * n)), tf, None, stride, pad).numpy()
+        assert same[0].tobytes() == same[-1].tobytes() == got[i].tobytes()
+
+
 # rows and columns that fill no tile, k at the edges of a slice and of its sixteen-value steps, an empty last slice
 # (k = 770: eight slices of 112, the last one with none), rows and columns that are not 16-byte aligned
 @pytest.mark.parametrize("m,k,n", [(1, 193, 33), (64, 784, 1024), (129, 257, 127), (128, 512, 512), (100, 770, 130), (65, 1023, 70), (30, 1024, 1800)])
