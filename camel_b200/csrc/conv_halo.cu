@@ -50,7 +50,7 @@ namespace {
 using namespace ptx;
 
 constexpr int kH_RowB       = 64;                     // bytes of k per operand row and k-block: 32 float16 / 16 tf32
-constexpr int kH_MaxSlots   = 96;                     // filter k-blocks in shared memory (a tap and channel block each)
+constexpr int kH_MaxSlots   = 96;                     // groups of filter k-blocks in shared memory (a few taps of a channel block each)
 constexpr int kH_HaloStages = 4;                      // at most; as many as shared memory holds
 constexpr int kH_EpiWarps   = 16;
 constexpr int kH_Threads    = 64 + 32 * kH_EpiWarps;
@@ -86,7 +86,6 @@ struct ConvHaloParams {
     int halos;                          // per channel block
     int halo_at[kH_MaxHalos];           // position of its sub-image in the planes
     uint8_t halo_taps[kH_MaxHalos + 1]; // its first tap in the list; the last entry is the number of taps
-    uint8_t tap[kH_MaxTaps];            // r * kw + s
     uint16_t tap_shift[kH_MaxTaps];     // positions between an output and the tap's pixel in the sub-image, in units of descriptors
     int chunk_blocks;                   // blocks of 32 channels per drain of the accumulators
     int chunk_wide;                     // tf32 images: blocks of 16
@@ -99,24 +98,35 @@ struct ConvHaloParams {
     int c_pad;        // channels of the planes (k offset of a tap in the filter planes: tap * c_pad)
     int box_rows, boxes; // positions of a TMA box, boxes of a halo
     int halo_plane_bytes, halo_stages;
-    int slots, slot_bytes, resident; // filter k-blocks in shared memory; resident: all of a set
+    int slots, slot_bytes; // groups of filter k-blocks in shared memory
+    int group, tap_bytes, f1;        // taps of a group, bytes between two of them, and from the first operand's terms to the second's
     int act;
     FastDiv by_pairs, by_tiles, by_pw; // pairs, image_tiles, pw
 };
 
 struct ConvHaloMaps {
     CUtensorMap x16_hi, x16_lo, x32_hi, x32_lo;
-    // THREE: hi and lo terms, boxes of n / 2 filters.  Otherwise hi (n / 2), lo (n), hi (n).
-    CUtensorMap w16[3], w32[3];
+    // THREE: hi and lo terms of n / 2 filters in one box.  Otherwise one plane's of n filters, and of n / 2.
+    CUtensorMap w16[2], w32[2];
 };
 
-// Tile load of three dimensions into THIS CTA's shared memory whose bytes are counted on a barrier of this CTA or the leader.
+// Tile loads of three and five dimensions into THIS CTA's shared memory whose bytes are counted on a barrier of this CTA or the leader.
 __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst_smem, const void *map, uint32_t cluster_bar, int32_t c0, int32_t c1, int32_t c2) {
     asm volatile(
         "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
         " [%0], [%1, {%3, %4, %5}], [%2];"
         :
         : "r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(cluster_bar), "r"(c0), "r"(c1), "r"(c2)
+        : "memory");
+}
+
+__device__ __forceinline__ void tma_load_5d_pair(
+    uint32_t dst_smem, const void *map, uint32_t cluster_bar, int32_t c0, int32_t c1, int32_t c2, int32_t c3, int32_t c4) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+        :
+        : "r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(cluster_bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
         : "memory");
 }
 
@@ -173,7 +183,7 @@ struct HaloWalk {
     }
 };
 
-template <bool THREE>
+template <bool THREE, bool RING>
 __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
     const __grid_constant__ ConvHaloMaps maps, const __grid_constant__ ConvHaloParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -254,7 +264,7 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                 const int c0  = walk.block(b) * block_k;
                 uint32_t word = walk.form ? kH_Wide | kH_Two : (p.c - c0 > 16 ? kH_Two : 0u); // k-steps that hold channels
                 bool reload   = false;
-                if (p.resident) {
+                if (!RING) {
                     const int set = walk.set_of(b);
                     if (set >= 0) {
                         load   = set != held;
@@ -295,8 +305,8 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                     reload = false;
                     if (!ok)
                         break;
-                    for (int t = p.halo_taps[h]; load && t < p.halo_taps[h + 1]; ++t) {
-                        if (!p.resident) {
+                    for (int t = p.halo_taps[h]; (RING || load) && t < p.halo_taps[h + 1]; t += RING ? p.group : 1) {
+                        if (RING) {
                             ok = mbar_wait_patient_warp(smem_u32(&bar_f_empty[s]), f_phase, abort_flag);
                             if (!ok)
                                 break;
@@ -305,13 +315,13 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                             const uint32_t full = smem_u32(&bar_f_full[s]), dst = slot_base + (uint32_t)(s * p.slot_bytes);
                             if (rank == 0)
                                 mbar_expect_tx(full, 2u * (uint32_t)p.slot_bytes);
-                            const int32_t kc = p.tap[t] * p.c_pad + c0, row = walk.tn * p.n, half = row + rank * (p.n >> 1);
+                            const int32_t cb = walk.block(b), row = walk.tn * p.n, half = row + rank * (p.n >> 1);
+                            // (a group's box may run on past its halo's taps: what it then holds is not used)
                             if (THREE) {
-                                tma_load_2d_pair(dst, &w[0], leader_addr(full), kc, half);
-                                tma_load_2d_pair(dst + (uint32_t)(p.n >> 1) * kH_RowB, &w[1], leader_addr(full), kc, half);
+                                tma_load_5d_pair(dst, &w[0], leader_addr(full), 0, half, t, cb, 0);
                             } else {
-                                tma_load_2d_pair(dst, rank ? &w[1] : &w[2], leader_addr(full), kc, row);
-                                tma_load_2d_pair(dst + (uint32_t)p.n * kH_RowB, &w[0], leader_addr(full), kc, half);
+                                tma_load_5d_pair(dst, &w[0], leader_addr(full), 0, row, t, cb, rank);
+                                tma_load_5d_pair(dst + (uint32_t)p.f1, &w[1], leader_addr(full), 0, half, t, cb, 0);
                             }
                         }
                         __syncwarp();
@@ -351,9 +361,10 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
         if (rank == 0) {
             // What a pass is made of is worked out by the producer (2400 clocks a pass here, while the tensor pipe ran dry), and
             // of a descriptor only the low word, the address, is computed.
-            const uint32_t unit  = kH_RowB / 16, slot_step = (uint32_t)p.slot_bytes >> 4;
-            const uint32_t f_0   = (uint32_t)smem_desc_k<kH_RowB>(slot_base), to_f1 = (uint32_t)(THREE ? p.n >> 1 : p.n) * unit;
-            const uint32_t to_lo = (uint32_t)p.halo_plane_bytes >> 4;
+            const uint32_t slot_step = (uint32_t)p.slot_bytes >> 4, tap_step = (uint32_t)p.tap_bytes >> 4, to_f1 = (uint32_t)p.f1 >> 4;
+            const uint32_t q_step    = THREE ? tap_step : tap_step >> 1; // of the second operand's terms
+            const uint32_t f_0       = (uint32_t)smem_desc_k<kH_RowB>(slot_base);
+            const uint32_t to_lo     = (uint32_t)p.halo_plane_bytes >> 4;
             auto desc = [](uint32_t low) { return smem_desc_k<kH_RowB>(0) & 0xffffffff00000000ull | low; };
             int s = 0, hs = 0, acc = 0;
             uint32_t f_phase = 0, h_phase = 0, acc_phase = 3u; // a bit per set of accumulators
@@ -385,23 +396,28 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                 const uint32_t idesc2 = make_idesc(word & kH_Wide ? 2u : 0u, 256, (uint32_t)(2 * p.n));
                 const uint32_t x = (uint32_t)smem_desc_k<kH_RowB>(smem_base + (uint32_t)hs * halo_stage);
                 const int t1 = (int)(word >> 6 & 63u);
+                int in_group = 0;
+                uint32_t f0 = f, f1 = f + to_f1;
                 for (int t = (int)(word & 63u); t < t1; ++t) {
-                    if (word & kH_Load) {
-                        ok = mbar_wait_warp(smem_u32(&bar_f_full[s]), f_phase, abort_flag);
-                        if (!ok)
-                            break;
-                        tc_fence_after_sync();
+                    if (!RING || in_group == 0) {
+                        f0 = f, f1 = f + to_f1;
+                        if (RING || (word & kH_Load)) {
+                            ok = mbar_wait_warp(smem_u32(&bar_f_full[s]), f_phase, abort_flag);
+                            if (!ok)
+                                break;
+                            tc_fence_after_sync();
+                        }
                     }
                     // the tap's pixels: the halo, so many rows of 64 bytes further on
                     const uint32_t xh = x + p.tap_shift[t], xl = xh + to_lo;
                     auto issue = [&](auto mma, uint32_t k) {
                         if (THREE) {
-                            mma(d_main, desc(xh + k), desc(f + k), idesc, accumulate);
-                            mma(d_cross, desc(xh + k), desc(f + to_f1 + k), idesc, accumulate);
-                            mma(d_cross, desc(xl + k), desc(f + k), idesc, 1u);
+                            mma(d_main, desc(xh + k), desc(f0 + k), idesc, accumulate);
+                            mma(d_cross, desc(xh + k), desc(f1 + k), idesc, accumulate);
+                            mma(d_cross, desc(xl + k), desc(f0 + k), idesc, 1u);
                         } else {
-                            mma(d_main, desc(xh + k), desc(f + k), idesc2, accumulate);
-                            mma(d_cross, desc(xl + k), desc(f + to_f1 + k), idesc, 1u);
+                            mma(d_main, desc(xh + k), desc(f0 + k), idesc2, accumulate);
+                            mma(d_cross, desc(xl + k), desc(f1 + k), idesc, 1u);
                         }
                         accumulate = 1u;
                     };
@@ -413,13 +429,22 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                         issue(mma_tf32_pair_warp, 0);
                         issue(mma_tf32_pair_warp, 2);
                     }
-                    if (!p.resident)
-                        tc_commit_pair_warp(smem_u32(&bar_f_empty[s]));
-                    f += slot_step;
-                    if (++s == p.slots) {
-                        s = 0, f = f_0;
-                        if (word & kH_Load)
-                            f_phase ^= 1u;
+                    bool next = true; // group
+                    if (RING) {
+                        f0 += tap_step, f1 += q_step;
+                        next = ++in_group == p.group || t + 1 == t1;
+                    }
+                    if (next) {
+                        if (RING) {
+                            in_group = 0;
+                            tc_commit_pair_warp(smem_u32(&bar_f_empty[s]));
+                        }
+                        f += slot_step;
+                        if (++s == p.slots) {
+                            s = 0, f = f_0;
+                            if (RING || (word & kH_Load))
+                                f_phase ^= 1u;
+                        }
                     }
                 }
                 if (!ok)
@@ -552,18 +577,19 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
 // Two launches: the range of every image, in slices, next to the filters (both forms of their planes, a block per
 // filter); then the input as NHWC planes, in the form that the image's range allows.
 
-// Blocks 0 .. ko - 1: filter [c][taps] -> planes [taps * c_pad], tap-major k (none if hi16 is null), and its inverse
+// Blocks 0 .. ko - 1: filter [c][taps] -> planes [taps in the order given][c_pad] (none if hi16 is null), and its inverse
 // scale, 0 where the range of the filter does not fit float16 pairs.  The others: slice (blockIdx.x - ko) of the images
 // ([batch][count] floats, `slices` to an image).
 struct FilterPlanes {
     __half *hi16, *lo16;
     float *hi32, *lo32;
     float *scale;
+    uint8_t order[kH_MaxTaps]; // place of each tap in the planes
     const float *bias; // the layer's, or null
     float *bias_out;   // its copy, -0 where there is none; null: not wanted
 };
 __global__ void __launch_bounds__(256) conv_range_kernel(
-    const float *__restrict__ w, int c, int taps, int c_pad, int ko, const FilterPlanes f, const float *__restrict__ x,
+    const float *__restrict__ w, int c, int taps, int c_pad, int ko, const __grid_constant__ FilterPlanes f, const float *__restrict__ x,
     int64_t count, int slices, int vec_ok, uint2 *__restrict__ ranges) {
     __shared__ uint2 part[8];
     griddep_launch_dependents();
@@ -611,120 +637,159 @@ __global__ void __launch_bounds__(256) conv_range_kernel(
     for (int i = threadIdx.x; i < taps * c_pad; i += 256) {
         const int tap = i / c_pad, ic = i - tap * c_pad;
         const float v    = ic < c ? src[ic * taps + tap] : 0.0f;
-        const int64_t at = o * taps * c_pad + i;
+        const int64_t at = (o * taps + f.order[tap]) * c_pad + ic;
         split_half(v, scale, f.hi16[at], f.lo16[at]);
         split_tf32(v, f.hi32[at], f.lo32[at]);
     }
 }
 
-// x [batch][c][hw] -> NHWC planes [hw][c_pad], hi then lo, in the image's slot of 8 bytes per value: float16 pairs
-// under the image's scale, or tf32 terms (image_scale 0) where the image or any filter does not fit those.  A
-// block takes 64 channels by 64 positions through shared memory: reads of 256 contiguous bytes, writes of 128.  The
-// images are taken last to first: the end of the tensor is what conv_range_kernel has just left in L2.
-// Sub-images (ConvSubImages, hs x ws each, from row y0 and column x0 of the input on): zeros where the image has no such row or
-// column, which is a layer's padding; those that no tap reads are left out.
+// x [batch][c][hw] -> NHWC planes [position][c_pad], hi then lo, in the image's slot of 8 bytes per value: float16 pairs
+// under the image's scale, or tf32 terms (image_scale 0) where the image or any filter does not fit those.  Positions are those of the
+// sub-images (ConvSubImages, hs x ws each, from row y0 and column x0 of the input on): zeros where the image has no such row or
+// column, which is a layer's padding; those that no tap reads are left out.  The images are taken last to first: the end of the tensor
+// is what conv_range_kernel has just left in L2.
 //
-// What bounds it is issue (0.83 of the slots at 128 x 64 x 56 x 56), so the moduli are constants, the one division left is a
-// multiplication, and one warp works the image's scale out for all: 64 x 48 x 57 x 57 -> 96 at stride 2 76 -> 69 us (31 of it this kernel
-// before), 256 x 64 x 56 x 56 -> 128 428 -> 425.
+// A warp takes 32 channels of 32 pixels, a pixel to a lane, all loads in flight at once: what a lane has split are then whole
+// 16-byte pieces of the planes, and its own shared memory only brings them into an order in which four lanes write 64 contiguous bytes.  No barrier
+// but the one behind which the block knows its image's form: blocks of 64 channels by 64 pixels, with barriers between reading and
+// writing, took 96 us for 256 x 64 x 56 x 56 where this takes 81 (of 55 to 65 at the copy rate; without loads and stores 40: a block's wait for
+// its image's range and its own start), and 22 for 64 x 48 x 57 x 57 at stride 2, where this takes 18.
 struct PlaneGeom {
     int h, w, hs, ws, y0, x0;
-    uint32_t width_inv; // 2^32 / (ws * col_mod), rounded up; 0 for a width of 1
     ConvSubImages sub;
+    int groups, items; // groups of 32 channels; warps' shares of an image
+    FastDiv by_w, by_groups, by_cols, by_chunks, by_pad; // image width, groups, columns of the grown image, eights of channels, padding columns
+    int pad_top, pad_rows, mid_rows, pad_left, pad_cols; // the grown image's positions that no pixel has: rows above, all such rows ...
 };
 template <int ROW_MOD, int COL_MOD>
-__global__ void __launch_bounds__(256) conv_planes_kernel(
-    const float *__restrict__ x, int c, const PlaneGeom geom, int c_pad, const uint2 *__restrict__ ranges, int slices,
+__global__ void __launch_bounds__(256, 3) conv_planes_kernel(
+    const float *__restrict__ x, int c, const __grid_constant__ PlaneGeom g, int c_pad, const uint2 *__restrict__ ranges, int slices,
     const float *__restrict__ filter_scale, int ko, uint8_t *__restrict__ slots, float *__restrict__ image_scale) {
-    __shared__ float tile[64][65];
+    __shared__ uint4 stage_s[8][128];
     __shared__ float scale_s;
-    __shared__ int fits_s;
     griddep_launch_dependents();
     griddep_wait();
-    const int64_t img = gridDim.z - 1 - blockIdx.z;
-    const int64_t q0  = (int64_t)blockIdx.x * 64;
-    const int c0      = (int)blockIdx.y * 64;
+    const int img  = (int)(gridDim.y - 1 - blockIdx.y);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t in_hw = (int64_t)geom.h * geom.w;
-    const int width  = geom.ws * COL_MOD;
-    const int64_t hw = (int64_t)geom.hs * ROW_MOD * width; // positions of the grown image
-    const float *src = x + (img * c + c0) * in_hw;
-    auto row_of = [&](int64_t q) { // q < 2^31: the rounded-up quotient is one too high at most
-        const int row = geom.width_inv ? (int)__umulhi((uint32_t)q, geom.width_inv) : (int)q;
-        return row - (row * width > (int)q ? 1 : 0);
+    const int item = (int)blockIdx.x * 8 + warp, hw = g.h * g.w;
+    const int px_tile = fast_div(item, g.by_groups), c0 = (item - px_tile * g.groups) * 32;
+    const int q = px_tile * 32 + lane;
+    const bool live  = item < g.items && q < hw;
+    const float *src = x + ((int64_t)img * c + c0) * hw + q;
+    float v[32]; // every load before the first use of any
+    // (the address goes from channel to channel in two instructions; left to the compiler, each was worked out anew, in seven)
+    auto channel = [&]() {
+        const float value = __ldcs(src);
+        asm volatile("add.s64 %0, %0, %1;" : "+l"(src) : "l"((int64_t)hw * 4));
+        return value;
     };
-    // position q of the grown image in the input (-1: not there)
-    auto source = [&](int64_t q) -> int64_t {
-        const int row = row_of(q), y = row + geom.y0, x = (int)q - row * width + geom.x0;
-        return q < hw && (unsigned)y < (unsigned)geom.h && (unsigned)x < (unsigned)geom.w ? (int64_t)y * geom.w + x : -1;
-    };
-    float v[16]; // every load before the first use of any
+    if (live && c0 + 32 <= c) {
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        const int64_t from = source(q0 + lane + 32 * t);
+        for (int j = 0; j < 32; ++j)
+            v[j] = channel();
+    } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int ch = warp + 8 * j;
-            v[2 * j + t] = (c0 + ch < c && from >= 0) ? __ldcs(src + ch * in_hw + from) : 0.0f;
-        }
+        for (int j = 0; j < 32; ++j)
+            v[j] = live && c0 + j < c ? channel() : 0.0f;
     }
     if (warp == 0) {
         uint2 r = make_uint2(0u, kNoneSmallest);
         for (int s = lane; s < slices; s += 32)
-            r = range_join(r, ranges[img * slices + s]);
-        float s, inverse;
-        const bool all = half_range_fits(range_warp(r), s, inverse);
+            r = range_join(r, ranges[(int64_t)img * slices + s]);
+        float scale, inverse;
+        const bool all = half_range_fits(range_warp(r), scale, inverse);
         if (lane == 0)
-            scale_s = s, fits_s = all;
+            scale_s = all ? scale : 0.0f;
     }
     int bad_filter = 0;
     for (int o = threadIdx.x; o < ko; o += 256)
         bad_filter |= filter_scale[o] == 0.0f ? 1 : 0;
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        tile[warp + 8 * (j >> 1)][lane + 32 * (j & 1)] = v[j];
-    const bool fits   = !__syncthreads_or(bad_filter) && fits_s;
-    const float scale = scale_s;
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+    const bool filters_fit = !__syncthreads_or(bad_filter);
+    const float scale      = filters_fit ? scale_s : 0.0f;
+    const bool fits        = scale != 0.0f;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
         image_scale[img] = fits ? 1.0f / scale : 0.0f; // a power of two
-    const int64_t plane = hw * c_pad;
-    uint8_t *slot       = slots + img * plane * 8;
+    const int rows = g.hs * ROW_MOD, cols = g.ws * COL_MOD;
+    const bool plain    = !fits && g.sub.tf32_plain;
+    const int64_t plane = (int64_t)rows * cols * c_pad;
+    uint8_t *slot       = slots + (int64_t)img * plane * 8;
+    auto place = [&](int row, int col) { // of the grown image; -1: not wanted
+        if (ROW_MOD * COL_MOD == 1)
+            return row * cols + col;
+        const int sub = row % ROW_MOD * COL_MOD + col % COL_MOD;
+        return g.sub.used >> sub & 1u ? (sub * g.hs + row / ROW_MOD) * g.ws + col / COL_MOD : -1;
+    };
+    int to = -1;
+    if (live) {
+        const int y = fast_div(q, g.by_w), row = y - g.y0, col = q - y * g.w - g.x0;
+        to = plain ? q : ((unsigned)row < (unsigned)rows && (unsigned)col < (unsigned)cols ? place(row, col) : -1);
+    }
+    // 64 bytes of each lane's pixel to `dst`, pixels `stride` bytes apart: chunk j of pixel p lies at j ^ ((p >> 1) & 3)
+    uint4 *stage = stage_s[warp];
+    auto emit = [&](const uint4 (&piece)[4], uint8_t *dst, int stride) {
+        __syncwarp(); // the last one's have been read
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        const int chunk = threadIdx.x & 7, q = (threadIdx.x >> 3) + 32 * t;
-        if (q0 + q >= hw || c0 + chunk * 8 >= c_pad)
-            continue;
-        int64_t to = q0 + q;
-        if (ROW_MOD * COL_MOD > 1) {
-            const int row = row_of(to), col = (int)to - row * width, sub = row % ROW_MOD * COL_MOD + col % COL_MOD;
-            if (!(geom.sub.used >> sub & 1u))
-                continue;
-            if (fits || !geom.sub.tf32_plain)
-                to = ((int64_t)sub * geom.hs + row / ROW_MOD) * geom.ws + col / COL_MOD;
-            else if (row < geom.h && col < geom.w)
-                to = (int64_t)row * geom.w + col;
-            else
-                continue;
+        for (int j = 0; j < 4; ++j)
+            stage[lane * 4 + (j ^ (lane >> 1 & 3))] = piece[j];
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int p = 8 * k + (lane >> 2), j = lane & 3, at = __shfl_sync(0xffffffffu, to, p);
+            if (at >= 0)
+                *reinterpret_cast<uint4 *>(dst + (int64_t)at * stride + 16 * j) = stage[p * 4 + (j ^ (p >> 1 & 3))];
         }
-        const int64_t at = to * c_pad + c0 + chunk * 8;
+    };
+    if (item < g.items) {
         if (fits) {
-            __half2 hi[4], lo[4];
+            uint4 hi[4], lo[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                split_half_pair(tile[chunk * 8 + 2 * j][q] * scale, tile[chunk * 8 + 2 * j + 1][q] * scale, hi[j], lo[j]);
-            __half *p_hi = reinterpret_cast<__half *>(slot) + at;
-            *reinterpret_cast<uint4 *>(p_hi)         = *reinterpret_cast<uint4 *>(hi);
-            *reinterpret_cast<uint4 *>(p_hi + plane) = *reinterpret_cast<uint4 *>(lo);
+            for (int j = 0; j < 4; ++j) {
+                __half2 h[4], l[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    split_half_pair(__fmul_rn(v[8 * j + 2 * t], scale), __fmul_rn(v[8 * j + 2 * t + 1], scale), h[t], l[t]);
+                hi[j] = *reinterpret_cast<uint4 *>(h), lo[j] = *reinterpret_cast<uint4 *>(l);
+            }
+            emit(hi, slot + c0 * 2, c_pad * 2);
+            emit(lo, slot + plane * 2 + c0 * 2, c_pad * 2);
         } else {
-            float *p_hi = reinterpret_cast<float *>(slot) + at;
 #pragma unroll
-            for (int j = 0; j < 8; j += 4) {
-                float hi[4], lo[4];
+            for (int half = 0; half < 2; ++half) {
+                uint4 hi[4], lo[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    split_tf32_flat(tile[chunk * 8 + j + u][q], hi[u], lo[u]);
-                *reinterpret_cast<float4 *>(p_hi + j)         = make_float4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<float4 *>(p_hi + plane + j) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+                for (int j = 0; j < 4; ++j) {
+                    float h[4], l[4];
+#pragma unroll
+                    for (int t = 0; t < 4; ++t)
+                        split_tf32_flat(v[16 * half + 4 * j + t], h[t], l[t]);
+                    hi[j] = *reinterpret_cast<uint4 *>(h), lo[j] = *reinterpret_cast<uint4 *>(l);
+                }
+                emit(hi, slot + (c0 + 16 * half) * 4, c_pad * 4);
+                emit(lo, slot + plane * 4 + (c0 + 16 * half) * 4, c_pad * 4);
+            }
+        }
+    }
+    // positions that no pixel has: the layer's padding, shared out between the blocks of the image
+    if (!plain) {
+        const int chunks = c_pad >> 3, whole = g.pad_rows * cols, all = (whole + g.mid_rows * g.pad_cols) * chunks;
+        for (int i = (int)blockIdx.x * 256 + (int)threadIdx.x; i < all; i += (int)gridDim.x * 256) {
+            const int j = fast_div(i, g.by_chunks), chunk = i - j * chunks;
+            int row, col;
+            if (j < whole) {
+                row = fast_div(j, g.by_cols), col = j - row * cols;
+                row += row < g.pad_top ? 0 : g.mid_rows;
+            } else {
+                row = fast_div(j - whole, g.by_pad), col = j - whole - row * g.pad_cols;
+                row += g.pad_top, col += col < g.pad_left ? 0 : cols - g.pad_cols;
+            }
+            const int at = place(row, col);
+            if (at >= 0) {
+                const int size = fits ? 16 : 32; // bytes of eight channels
+                for (int b = 0; b < size; b += 16) {
+                    uint8_t *dst = slot + ((int64_t)at * chunks + chunk) * size + b;
+                    *reinterpret_cast<uint4 *>(dst)                              = make_uint4(0u, 0u, 0u, 0u);
+                    *reinterpret_cast<uint4 *>(dst + plane * (fits ? 2 : 4)) = make_uint4(0u, 0u, 0u, 0u);
+                }
             }
         }
     }
@@ -735,7 +800,7 @@ struct HaloGeom {
     int hs;             // rows of a sub-image; it has pw columns
     int y_min, x_min;   // smallest row and column offset of a tap in its sub-image
     int image_tiles, box_rows, boxes, plane_bytes, stages;
-    int n, tiles_n, slots, slot_bytes, resident, three;
+    int n, tiles_n, group, slots, slot_bytes, ring, three;
     size_t smem;
 };
 
@@ -763,22 +828,26 @@ bool halo_geometry(int64_t c_pad, int64_t h, int64_t w, int64_t ko, int64_t kh, 
     // tiles of equal numbers of filters, in steps of 32 (the columns of an MMA of two CTAs)
     g->tiles_n    = (int)((ko + 127) / 128);
     g->n          = (int)(((ko + g->tiles_n - 1) / g->tiles_n + 31) / 32 * 32);
+    const int budget = kH_Smem - 1024, halo = 2 * g->plane_bytes;
+    // All filters of a tile, by halves (see the top) for many, and where the other way's memory does not hold them all.
     const int64_t all = kh * kw * (c_pad / 32);
-    const int budget  = kH_Smem - 1024, halo = 2 * g->plane_bytes;
-    // the terms shared out by halves (see the top) for many filters, and where the other way's memory does not hold them all
-    const int both = g->n * kH_RowB * 3 / 2;
-    auto fits      = [&](int64_t bytes) { return all <= kH_MaxSlots && all * bytes + 2 * halo <= budget; };
-    g->three       = g->n >= 96 || !fits(both);
-    g->slot_bytes  = g->three ? g->n * kH_RowB : both;
-    g->resident    = fits(g->slot_bytes);
-    if (g->resident) {
+    const int one = g->n * kH_RowB, both = one / 2 * 3;
+    auto fits     = [&](int64_t bytes) { return all <= kH_MaxSlots && all * bytes + 2 * halo <= budget; };
+    g->three      = g->n >= 96 || !fits(both);
+    g->group      = 1;
+    g->slot_bytes = g->three ? one : both;
+    g->ring       = !fits(g->slot_bytes);
+    if (!g->ring) {
         g->slots  = (int)all;
         g->stages = std::min(kH_HaloStages, (budget - g->slots * g->slot_bytes) / halo);
     } else {
-        // a third halo where that leaves a ring of eight k-blocks
-        g->stages = 3 * halo + 8 * g->slot_bytes <= budget ? 3 : 2;
-        g->slots  = (int)std::min<int64_t>(std::min<int64_t>(16, all), (budget - g->stages * halo) / g->slot_bytes);
-        if (budget < g->stages * halo || g->slots < std::min<int64_t>(4, all))
+        // In a ring, groups of taps, a row of them where a halo serves whole rows: with a tap by itself copies, waits and commits took 700
+        // clocks, where those of 64 filters take 290 (40 x 100 x 50 x 50 -> 64, 5 x 5, 207 us, 168 so).  A third halo where that leaves 64 KB.
+        if (stride == 1 && 2 * halo + 4 * kw * one <= budget)
+            g->group = (int)kw, g->slot_bytes *= (int)kw;
+        g->stages = 3 * halo + 64 * 1024 <= budget ? 3 : 2;
+        g->slots  = (int)std::min<int64_t>(std::min<int64_t>(16, all / g->group), (budget - g->stages * halo) / g->slot_bytes);
+        if (budget < g->stages * halo || g->slots < std::min<int64_t>(g->group > 1 ? 2 : 4, all / g->group))
             return false;
     }
     g->smem = 1024 + (size_t)g->stages * halo + (size_t)g->slots * g->slot_bytes;
@@ -798,7 +867,7 @@ int conv_range_slices(int64_t batch, int64_t count) {
 // ranges: batch * conv_range_slices(batch, c * hw) pairs of words.
 ct_status conv_prepass(
     const float *x, const float *w, int64_t batch, int64_t c, int64_t h, int64_t wd, int64_t c_pad, int64_t ko, int64_t taps,
-    void *filters16, void *filters32, size_t plane16, size_t plane32, float *filter_scale, const float *bias, float *bias_copy,
+    void *filters16, void *filters32, size_t plane16, size_t plane32, const uint8_t *order, float *filter_scale, const float *bias, float *bias_copy,
     void *ranges, float *image_scale, void *slots, const ConvSubImages &sub) {
     if (batch > 65535 || c_pad / 32 > 65535)
         return fail(CT_ERR_TOO_LARGE, "conv2d: batch or channel count too large for the layout pre-pass");
@@ -806,16 +875,26 @@ ct_status conv_prepass(
     const int slices    = conv_range_slices(batch, count);
     const int vec       = (count & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
     uint8_t *f16 = static_cast<uint8_t *>(filters16), *f32 = static_cast<uint8_t *>(filters32);
-    const FilterPlanes f{reinterpret_cast<__half *>(f16), reinterpret_cast<__half *>(f16 + plane16), reinterpret_cast<float *>(f32),
-                         reinterpret_cast<float *>(f32 + plane32), filter_scale, bias, bias_copy};
+    FilterPlanes f{reinterpret_cast<__half *>(f16), reinterpret_cast<__half *>(f16 + plane16), reinterpret_cast<float *>(f32),
+                   reinterpret_cast<float *>(f32 + plane32), filter_scale, {}, bias, bias_copy};
+    for (int t = 0; order && t < (int)taps; ++t)
+        f.order[t] = order[t];
     ProfScope prof("conv_prepass");
     CT_CUDA(launch_dependent(conv_range_kernel, dim3((unsigned)(ko + batch * slices)), dim3(256), 0, stream(), w, (int)c, (int)taps,
                              (int)c_pad, (int)ko, f, x, count, slices, vec, static_cast<uint2 *>(ranges)));
     CT_LAUNCH_CHECK("conv_range");
-    PlaneGeom geom{(int)h, (int)wd, sub.rows, sub.cols, sub.y0, sub.x0, 0, sub};
-    const int64_t width = (int64_t)geom.ws * sub.col_mod, positions = geom.hs * width * sub.row_mod;
-    geom.width_inv = width > 1 ? (uint32_t)(((1ull << 32) + width - 1) / width) : 0;
-    const dim3 grid((unsigned)((positions + 63) / 64), (unsigned)((c_pad + 63) / 64), (unsigned)batch);
+    const int64_t width = (int64_t)sub.cols * sub.col_mod, grown = (int64_t)sub.rows * sub.row_mod, hw = h * wd;
+    if ((grown * width + 1) * (c_pad / 8) > 0x7fffffffll || (hw + 31) / 32 * (c_pad / 32) > 0x7ffffff0ll)
+        return fail(CT_ERR_TOO_LARGE, "conv2d: image too large for the layout pre-pass");
+    PlaneGeom geom{};
+    geom.h = (int)h, geom.w = (int)wd, geom.hs = sub.rows, geom.ws = sub.cols, geom.y0 = sub.y0, geom.x0 = sub.x0, geom.sub = sub;
+    geom.groups = (int)(c_pad / 32), geom.items = (int)((hw + 31) / 32) * geom.groups;
+    const int64_t top = std::min<int64_t>(-geom.y0, grown), left = std::min<int64_t>(-geom.x0, width);
+    geom.mid_rows = (int)std::min<int64_t>(h, grown - top), geom.pad_top = (int)top, geom.pad_rows = (int)grown - geom.mid_rows;
+    geom.pad_left = (int)left, geom.pad_cols = (int)(width - std::min<int64_t>(wd, width - left));
+    geom.by_w = fast_divisor(wd), geom.by_groups = fast_divisor(geom.groups), geom.by_cols = fast_divisor(width);
+    geom.by_chunks = fast_divisor(c_pad / 8), geom.by_pad = fast_divisor(std::max(1, geom.pad_cols));
+    const dim3 grid((unsigned)((geom.items + 7) / 8), (unsigned)batch);
     auto planes = [&](auto kernel) {
         return launch_dependent(kernel, grid, dim3(256), 0, stream(), x, (int)c, geom, (int)c_pad, static_cast<const uint2 *>(ranges), slices,
                                 static_cast<const float *>(filter_scale), (int)ko, static_cast<uint8_t *>(slots), image_scale);
@@ -885,17 +964,19 @@ ct_status conv_halo(
     p.c_pad   = (int)c_pad;
     p.box_rows = g.box_rows, p.boxes = g.boxes;
     p.halo_plane_bytes = g.plane_bytes, p.halo_stages = g.stages;
-    p.slots = g.slots, p.slot_bytes = g.slot_bytes, p.resident = g.resident;
+    p.slots = g.slots, p.slot_bytes = g.slot_bytes;
     p.act = act;
     p.by_pairs = fast_divisor(pairs), p.by_tiles = fast_divisor(g.image_tiles), p.by_pw = fast_divisor(g.pw);
+    p.group = g.group, p.tap_bytes = g.three ? g.n / 2 * kH_RowB : g.n * kH_RowB, p.f1 = g.group * p.tap_bytes;
     p.halos = 0, p.halo_taps[0] = 0;
+    uint8_t order[kH_MaxTaps] = {};
     uint32_t used = 0;
     for (int image = 0, listed = 0; image < (int)subs; ++image) {
         for (int t = 0; t < (int)taps; ++t) {
             const int r = t / (int)kw - (int)pad, q = t % (int)kw - (int)pad, a = floor_div(r, stride), b = floor_div(q, stride);
             if ((r - a * (int)stride) * (int)stride + (q - b * (int)stride) != image)
                 continue;
-            p.tap[listed]         = (uint8_t)t;
+            order[t]              = (uint8_t)listed;
             p.tap_shift[listed++] = (uint16_t)(((a - g.y_min) * g.pw + (b - g.x_min)) * (kH_RowB / 16));
         }
         if (listed > p.halo_taps[p.halos]) {
@@ -905,20 +986,22 @@ ct_status conv_halo(
         }
     }
     const ConvSubImages images{(int)stride, (int)stride, used, false, g.hs, g.pw, g.y_min * (int)stride, g.x_min * (int)stride};
-    CT_TRY(conv_prepass(x, w, batch, c, h, wd, c_pad, ko, taps, w16_hi, w32_hi, w16, w32, filter_scale, bias, bias_copy, range_words,
+    CT_TRY(conv_prepass(x, w, batch, c, h, wd, c_pad, ko, taps, w16_hi, w32_hi, w16, w32, order, filter_scale, bias, bias_copy, range_words,
                         image_scale, xp, images));
     ConvHaloMaps maps;
     const bool three = g.three != 0;
     auto encode = [&](CUtensorMap *mw, const uint8_t *wp, size_t w_plane, CUtensorMap *mx_hi, CUtensorMap *mx_lo, int elem) {
-        const uint64_t kp = (uint64_t)(taps * c_pad), row = (uint64_t)(c_pad * elem);
-        const uint64_t wdims[2] = {kp, (uint64_t)ko}, wstr[1] = {kp * (uint64_t)elem};
-        const uint32_t whalf[2] = {(uint32_t)(kH_RowB / elem), (uint32_t)(g.n / 2)}, wfull[2] = {(uint32_t)(kH_RowB / elem), (uint32_t)g.n};
+        const uint64_t row = (uint64_t)(c_pad * elem), block = (uint64_t)(kH_RowB / elem);
+        // a filter's channels of a block, filters, taps, blocks, hi and lo terms
+        const uint64_t wdims[5] = {block, (uint64_t)ko, (uint64_t)taps, (uint64_t)c_pad / block, 2};
+        const uint64_t wstr[4]  = {(uint64_t)taps * row, row, (uint64_t)kH_RowB, (uint64_t)w_plane};
+        const uint32_t wbox[2][5] = {{(uint32_t)block, (uint32_t)(three ? g.n / 2 : g.n), (uint32_t)g.group, 1, three ? 2u : 1u},
+                                     {(uint32_t)block, (uint32_t)(g.n / 2), (uint32_t)g.group, 1, 1}};
         const uint64_t xdims[3] = {(uint64_t)c_pad, (uint64_t)positions, (uint64_t)batch}, xstr[2] = {row, slot};
-        const uint32_t xbox[3]  = {(uint32_t)(kH_RowB / elem), (uint32_t)g.box_rows, 1};
+        const uint32_t xbox[3]  = {(uint32_t)block, (uint32_t)g.box_rows, 1};
         auto fn = elem == 4 ? encode_tiled_map_f32 : encode_tiled_map_f16;
-        CT_TRY(fn(&mw[0], wp, 2, wdims, wstr, whalf, kH_RowB));
-        CT_TRY(fn(&mw[1], wp + w_plane, 2, wdims, wstr, three ? whalf : wfull, kH_RowB));
-        CT_TRY(fn(&mw[2], wp, 2, wdims, wstr, wfull, kH_RowB));
+        for (int i = 0; i < 2; ++i)
+            CT_TRY(fn(&mw[i], wp, 5, wdims, wstr, wbox[i], kH_RowB));
         CT_TRY(fn(mx_hi, xp, 3, xdims, xstr, xbox, kH_RowB));
         return fn(mx_lo, xp + (size_t)positions * c_pad * elem, 3, xdims, xstr, xbox, kH_RowB);
     };
@@ -926,14 +1009,14 @@ ct_status conv_halo(
     CT_TRY(encode(maps.w32, w32_hi, w32, &maps.x32_hi, &maps.x32_lo, 4));
     static bool attr_set_dev[16] = {}; // the attribute belongs to a device's context
     if (!attr_set_dev[st->device & 15]) {
-        CT_CUDA(cudaFuncSetAttribute(conv_halo_stream_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kH_Smem));
-        CT_CUDA(cudaFuncSetAttribute(conv_halo_stream_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kH_Smem));
+        for (auto kernel : {conv_halo_stream_kernel<false, false>, conv_halo_stream_kernel<true, false>, conv_halo_stream_kernel<true, true>})
+            CT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kH_Smem));
         attr_set_dev[st->device & 15] = true;
     }
     const unsigned grid = 2u * (unsigned)std::min<int64_t>(items, st->sm_count / 2);
     ProfScope prof("gemm_tc");
-    CT_CUDA(launch_dependent_cluster(three ? conv_halo_stream_kernel<true> : conv_halo_stream_kernel<false>, 2, dim3(grid), dim3(kH_Threads),
-                                     g.smem, stream(), maps, p));
+    const auto kernel = g.ring ? conv_halo_stream_kernel<true, true> : (three ? conv_halo_stream_kernel<true, false> : conv_halo_stream_kernel<false, false>);
+    CT_CUDA(launch_dependent_cluster(kernel, 2, dim3(grid), dim3(kH_Threads), g.smem, stream(), maps, p));
     CT_LAUNCH_CHECK("conv_halo_stream");
     return CT_OK;
 }

@@ -1293,7 +1293,7 @@ ct_status conv_tmem_filters(
     CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, f_words + words + ranges + (size_t)batch * slot));
     uint8_t *ws = static_cast<uint8_t *>(st->gemm_ws), *planes = ws + f_words + words + ranges;
     float *image_scale = reinterpret_cast<float *>(ws + f_words);
-    CT_TRY(conv_prepass(x, w, batch, c, h, wd, 32, ko, kh * kw, nullptr, nullptr, 0, 0, reinterpret_cast<float *>(ws), nullptr, nullptr,
+    CT_TRY(conv_prepass(x, w, batch, c, h, wd, 32, ko, kh * kw, nullptr, nullptr, 0, 0, nullptr, reinterpret_cast<float *>(ws), nullptr, nullptr,
                         ws + f_words + words, image_scale, planes, ConvSubImages{2, 1, 3u, true, (int)hs, (int)wd}));
     pp.image_scale = pt.image_scale = image_scale;
     // float16 planes [batch][row & 1][row >> 1][w][32 channels], box = 32 channels x pw positions x region_rows rows of one

@@ -41,7 +41,7 @@ struct ConvSubImages {
 int conv_range_slices(int64_t batch, int64_t count);
 ct_status conv_prepass(
     const float *x, const float *w, int64_t batch, int64_t c, int64_t h, int64_t wd, int64_t c_pad, int64_t ko, int64_t taps,
-    void *filters16, void *filters32, size_t plane16, size_t plane32, float *filter_scale, const float *bias, float *bias_copy,
+    void *filters16, void *filters32, size_t plane16, size_t plane32, const uint8_t *order, float *filter_scale, const float *bias, float *bias_copy,
     void *ranges, float *image_scale, void *slots, const ConvSubImages &sub);
 // x NCHW and w OIHW float32; c_pad: channels rounded up to 32.
 ct_status conv_halo(
