@@ -110,23 +110,13 @@ struct ConvHaloMaps {
     CUtensorMap w16[2], w32[2];
 };
 
-// Tile loads of three and five dimensions into THIS CTA's shared memory whose bytes are counted on a barrier of this CTA or the leader.
+// Tile load of three dimensions into THIS CTA's shared memory whose bytes are counted on a barrier of this CTA or the leader.
 __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst_smem, const void *map, uint32_t cluster_bar, int32_t c0, int32_t c1, int32_t c2) {
     asm volatile(
         "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
         " [%0], [%1, {%3, %4, %5}], [%2];"
         :
         : "r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(cluster_bar), "r"(c0), "r"(c1), "r"(c2)
-        : "memory");
-}
-
-__device__ __forceinline__ void tma_load_5d_pair(
-    uint32_t dst_smem, const void *map, uint32_t cluster_bar, int32_t c0, int32_t c1, int32_t c2, int32_t c3, int32_t c4) {
-    asm volatile(
-        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-        :
-        : "r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(cluster_bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
         : "memory");
 }
 
@@ -191,6 +181,7 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
     __shared__ uint64_t bar_h_full[kH_HaloStages], bar_h_empty[kH_HaloStages];
     __shared__ uint64_t bar_acc_full[2], bar_acc_empty[2];
     __shared__ uint32_t halo_word[kH_HaloStages];
+    __shared__ int epi_word[2];
     __shared__ uint64_t bar_done;
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag_s;
@@ -473,7 +464,7 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
         const bool relu   = p.act == CT_ACT_RELU;
         const int64_t plane = (int64_t)p.ho * p.wo;
         float *scales = scale_s[warp - 2], *biases = bias_s[warp - 2];
-        int acc = 0, held = -1;
+        int acc = 0, held = -1, turn = 0;
         uint32_t acc_phase = 0;
         bool ok = true;
         HaloWalk walk(p, first, stride);
@@ -496,7 +487,9 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
             float sum[32];
 #pragma unroll 1
             for (int e = 0; e < chunks; ++e) {
-                ok = mbar_wait_patient_warp(smem_u32(&bar_acc_full[acc]), acc_phase >> acc & 1u, abort_flag);
+                ok = group_wait(
+                    warp == 2, [&] { return mbar_wait(smem_u32(&bar_acc_full[acc]), acc_phase >> acc & 1u, abort_flag); }, epi_word, turn++, 1,
+                    32 * kH_EpiWarps);
                 if (!ok)
                     break;
                 acc_phase ^= 1u << acc;
@@ -529,7 +522,7 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0)
-                    mbar_arrive_cluster(leader_addr(smem_u32(&bar_acc_empty[acc])));
+                    mbar_arrive_peer(leader_addr(smem_u32(&bar_acc_empty[acc])));
                 acc ^= 1;
             }
             if (!ok)

@@ -148,15 +148,27 @@ __device__ __forceinline__ int next_own(const uint32_t *mask, int q, int own) {
 template <typename Seen>
 __device__ __forceinline__ void stage_filters(const float *w, int ko, int row, float *rows, int warp, int warps, int lane, Seen seen) {
     const int stride = row | 1;
-    for (int f = warp; f < ko; f += warps) {
-        uint2 range = make_uint2(0u, kNoneSmallest);
-#pragma unroll 4
+    // four of the warp's filters at a time, so that their loads are in flight together
+    for (int f0 = warp; f0 < ko; f0 += 4 * warps) {
+        uint2 range[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            range[q] = make_uint2(0u, kNoneSmallest);
+#pragma unroll 2
         for (int e = lane; e < row; e += 32) {
-            const float v = w[(int64_t)f * row + e];
-            range_take(range, v);
-            rows[f * stride + e] = v;
+            float v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                v[q] = f0 + q * warps < ko ? w[(int64_t)(f0 + q * warps) * row + e] : 0.0f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (f0 + q * warps < ko)
+                    range_take(range[q], v[q]), rows[(f0 + q * warps) * stride + e] = v[q];
         }
-        seen(f, range);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (f0 + q * warps < ko)
+                seen(f0 + q * warps, range[q]);
     }
 }
 // ... and of a region that the asynchronous proxy writes next.
@@ -652,10 +664,10 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
 //
 // Two 11-bit terms in float16 instead of tf32 (half_split.cuh), pixels on the accumulator rows.  A tile is 2 jp output
 // rows of an image: its even rows are the 128 rows of one accumulator, its odd rows those of another, positions j * pw + x
-// each.  The input rows of a tile lie in shared memory as two regions, even and odd rows of the box, so that filter tap
+// each.  Two tiles belong to a pair of CTAs, a tile to each, whose MMAs (cta_group::2) are issued by the leader.  The input rows of a tile lie in shared memory as two regions, even and odd rows of the box, so that filter tap
 // (r, s) is, for the even (odd) output rows, region r & 1 ((r + 1) & 1) through a descriptor moved by
 // (r >> 1) * pw + s (((r + 1) >> 1) * pw + s) rows.  The filters are the B operand and stay in shared memory for the
-// whole launch, hi terms before lo terms for each tap.  Per 16 channels and tap two MMAs an accumulator:
+// whole launch, the leader holding the hi and its peer the lo terms, and each half of the hi terms once more.  Per 16 channels and tap two MMAs an accumulator:
 //     [main | cross] += X_hi x [W_hi; W_lo]     N = 2 kop
 //             cross  += X_lo x W_hi             N = kop
 // with the low terms stored 2^11 times larger and the cross products in columns of their own, as in gemm_half.cu.  The product of
@@ -671,6 +683,12 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
 // rows are vertical neighbours, horizontal ones are lanes, so the sum, the activation, the 2x2 maximum and the store
 // need no shared memory at all, and a store covers consecutive pixels of a channel.
 //
+// Shared memory is what bounds it (128 bytes per clock): a CTA by itself read 14 KB for the two MMAs of a k-step, 5900 clocks a
+// tile with what the conversion reads and writes; each CTA of a pair reads 11 KB, 3600 clocks of a tile's 6500, and what is left is
+// the epilogue (5000), which waits for the same memory.  8192 x 32 x 28 x 28 -> 64 with the pool 915 -> 805 us; 64 x 32 x 60 x 60 -> 64
+// 72.7 -> 56, 300 x 20 x 30 x 29 -> 48 75.9 -> 57.4, 5 x 32 x 28 x 28 -> 64 17.5 -> 17.1; layers of few tiles from planes lose (3 x 31 x 30 x
+// 29 -> 48, 2 x 2, 16.6 -> 19).  Sixteen epilogue warps instead of eight are no faster (889 us: 72 registers a thread).
+//
 // Scales: per filter, and per tile (raw: the converting warps see the whole box before they split it) or, from planes, per
 // image.  The converting warps also leave the range of every tile in the call's own scratch; conv_tmem_filters_kernel,
 // launched behind this one, computes the images that float16 pairs cannot hold.  A tile that shows that by itself is
@@ -678,6 +696,28 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
 // Converting warps: with ten the boxes of up to 320 positions are held in registers (30 x 10 of a 28 x 28 image), larger ones are read
 // twice.  Against the kernel before, 256 images, 3 x 3: 32 -> 64 channels at 12 x 12 36 -> 23 us, 28 x 28 65 -> 44, 32 x 32 90 -> 61,
 // 40 x 40 146 -> 114, 60 x 60 298 -> 238; 16 -> 32 at 56 x 56 233 -> 151.
+// Two float32 operations in one instruction, each rounded as by itself.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t pack2(uint32_t a, uint32_t b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 constexpr int kCP_CvtWarps  = 10;
 constexpr int kCP_EpiWarps  = 8;
 constexpr int kCP_Threads   = 64 + 32 * (kCP_CvtWarps + kCP_EpiWarps);
@@ -690,7 +730,7 @@ struct ConvPairParams {
     const float *bias;
     float *out;        // [batch][ko][ho][wo], or [batch][ko][ho/2][wo/2] with pool
     uint32_t *flags;
-    int ko, kop, c, kh, kw, pad; // kop: ko rounded up to 16
+    int ko, kop, c, kh, kw, pad; // kop: ko rounded up to 32, the columns of an MMA of two CTAs
     int ho, wo, pw;    // pw = input width + 2 pad
     int jp, tiles_y;   // pairs of output rows per tile, tiles per image
     int region_rows;   // input rows of a region
@@ -715,15 +755,16 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
     __shared__ uint64_t bar_raw_full, bar_raw_empty;
     __shared__ uint64_t bar_scale_empty[kCP_MaxStages]; // the tile's scale has been read by the epilogue
     __shared__ uint64_t bar_acc_full[2], bar_acc_empty[2]; // tiles alternate between two sets of 256 columns
-    __shared__ uint64_t bar_done, bar_cvt;
+    __shared__ uint64_t bar_done;
     __shared__ uint32_t tmem_base_slot;
-    __shared__ int abort_flag_s, filters_wide_s;
+    __shared__ int abort_flag_s, filters_wide_s, cvt_word[2], epi_word[2];
     __shared__ uint2 cvt_range[2][kCP_CvtWarps];
     __shared__ float tile_scale[kCP_MaxStages]; // inverse scale of the tile in each plane stage; 0: left to the tf32 form
     __shared__ __align__(16) float filter_inv[64], bias_s[64];
     volatile int *abort_flag = &abort_flag_s;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31; // known to be the same for the warp
+    const int rank = (int)(blockIdx.x & 1), first = (int)(blockIdx.x >> 1), stride = (int)(gridDim.x >> 1), pairs = (total_tiles + 1) / 2;
     if (threadIdx.x == 0) {
         abort_flag_s   = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
         filters_wide_s = 0;
@@ -732,9 +773,6 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
         filter_inv[threadIdx.x] = 1.0f;
         bias_s[threadIdx.x]     = p.bias && (int)threadIdx.x < p.ko ? p.bias[threadIdx.x] : -0.0f; // which no sum notices
     }
-    __syncthreads();
-    if (abort_flag_s)
-        return;
 
     const uint32_t smem_base   = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *const smem_ptr    = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -745,7 +783,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
-            mbar_init(smem_u32(&bar_full[s]), RAW ? kCP_CvtWarps : 1);
+            mbar_init(smem_u32(&bar_full[s]), RAW ? 2 * kCP_CvtWarps : 1); // of both CTAs
             mbar_init(smem_u32(&bar_empty[s]), 1);
             mbar_init(smem_u32(&bar_scale_empty[s]), kCP_EpiWarps);
         }
@@ -753,41 +791,44 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
         mbar_init(smem_u32(&bar_raw_empty), kCP_CvtWarps);
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&bar_acc_full[b]), 1);
-            mbar_init(smem_u32(&bar_acc_empty[b]), kCP_EpiWarps);
+            mbar_init(smem_u32(&bar_acc_empty[b]), 2 * kCP_EpiWarps);
         }
         mbar_init(smem_u32(&bar_done), 1);
-        mbar_init(smem_u32(&bar_cvt), kCP_CvtWarps);
         mbar_fence_init();
         prefetch_tensormap(&map_x_hi);
         prefetch_tensormap(&map_x_lo);
     }
+    __syncthreads(); // the defaults of filter_inv
     float *filters = reinterpret_cast<float *>(smem_ptr + p.filter_bytes); // where the stages will be
     const int taps = p.kh * p.kw, filter_stride = (p.c * taps) | 1;
     stage_filters(p.w, p.ko, p.c * taps, filters, warp, kCP_Threads / 32, lane, [&](int f, uint2 range) {
         float scale, inverse;
         const bool fits = half_range_fits(range_warp(range), scale, inverse);
-        if (elect_one()) {
+        if (lane == 0) {
             filter_inv[f] = inverse;
             if (!fits)
                 filters_wide_s = 1;
         }
     });
     if (warp == 1) {
-        tmem_alloc(smem_u32(&tmem_base_slot), 512);
-        tmem_relinquish();
+        tmem_alloc_pair(smem_u32(&tmem_base_slot), 512);
+        tmem_relinquish_pair();
     }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = tmem_base_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
+    const bool failed        = abort_flag_s != 0;   // an earlier launch failed: no work
     const bool filters_wide  = filters_wide_s != 0; // every tile is left to the tf32 form
     if (RAW && blockIdx.x == 0 && threadIdx.x == 0)
         p.tile_range[total_tiles] = make_uint2(filters_wide ? 1u : 0u, 0u);
 
-    // ---- the filters' planes, once: per tap kop rows of hi terms, then kop of lo terms, 64-byte rows, swizzled ----
+    // ---- the filters' planes, once, 64-byte rows, swizzled: per tap kop rows of the leader's hi or its peer's lo terms; behind those
+    // of all taps, per tap half of the hi terms; then half of the last tap's lo terms ----
+    const int half_rows = p.kop >> 1, q_at = taps * p.kop, r_at = q_at + taps * half_rows, shift = p.kop == 64 ? 6 : 5;
     if (!filters_wide)
-        for (int i = threadIdx.x; i < taps * p.kop * 4; i += kCP_Threads) {
-            const int chunk = i & 3, f = (i >> 2) % p.kop, tap = (i >> 2) / p.kop, c0 = chunk * 8;
+        for (int i = threadIdx.x; i < q_at * 4; i += kCP_Threads) {
+            const int chunk = i & 3, row = i >> 2, tap = row >> shift, f = row & (p.kop - 1), c0 = chunk * 8;
             const float *src  = filters + f * filter_stride;
             const float scale = 1.0f / filter_inv[f]; // both are powers of two
             __half2 hi[4], lo[4];
@@ -798,28 +839,46 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                 const float b = (f < p.ko && ic + 1 < p.c) ? src[(ic + 1) * taps + tap] : 0.0f;
                 split_half_pair(a * scale, b * scale, hi[j], lo[j]);
             }
-            auto at = [&](int row) { return smem_ptr + ((size_t)tap * 2 * p.kop + row) * kCP_RowB + ((chunk ^ ((row >> 1) & 3)) << 4); };
-            *reinterpret_cast<uint4 *>(at(f))         = *reinterpret_cast<uint4 *>(hi);
-            *reinterpret_cast<uint4 *>(at(p.kop + f)) = *reinterpret_cast<uint4 *>(lo);
+            auto put = [&](int to, const __half2 (&v)[4]) {
+                *reinterpret_cast<uint4 *>(smem_ptr + (size_t)to * kCP_RowB + ((chunk ^ ((to >> 1) & 3)) << 4)) = *reinterpret_cast<const uint4 *>(v);
+            };
+            if (rank)
+                put(row, lo);
+            else
+                put(row, hi);
+            const int mine = f - rank * half_rows;
+            if (mine >= 0 && mine < half_rows) {
+                put(q_at + tap * half_rows + mine, hi);
+                if (tap == taps - 1)
+                    put(r_at + mine, lo);
+            }
         }
     filters_taken();
     __syncthreads();
+    cluster_sync(); // the MMAs read both CTAs' filters, and nothing is signalled on the partner's barriers before they exist
 
-    if (filters_wide) {
+    // this CTA's tile of pair u (the last may have one only: then both compute it, and the leader stores it), and, from planes, whether
+    // either image of the pair is left to this kernel
+    auto tile_of = [&](int u) { return min(2 * u + rank, total_tiles - 1); };
+    auto wanted  = [&](int u) {
+        return RAW || __any_sync(0xffffffffu, p.image_scale[2 * u / p.tiles_y] != 0.0f || p.image_scale[min(2 * u + 1, total_tiles - 1) / p.tiles_y] != 0.0f);
+    };
+
+    if (filters_wide || failed) {
     } else if (warp == 0) {
         // ===== TMA producer: one box per plane and region (raw mode: one box of the input) =====
-        if (elect_one()) {
-            int i = 0;
-            const int nstages = RAW ? 1 : p.stages;
-            for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-                const int img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
-                if (!RAW && p.image_scale[img] == 0.0f)
-                    continue;
-                const int s       = i % nstages;
-                const uint32_t ph = (uint32_t)(i / nstages) & 1u;
-                if (!mbar_wait_patient(smem_u32(RAW ? &bar_raw_empty : &bar_empty[s]), ph ^ 1u, abort_flag))
-                    break;
-                const int32_t h0 = ty * 2 * p.jp - p.pad;
+        int i = 0;
+        const int nstages = RAW ? 1 : p.stages;
+        for (int u = first; u < pairs; u += stride) {
+            if (!wanted(u))
+                continue;
+            const int tile = tile_of(u), img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
+            const int s       = i % nstages;
+            const uint32_t ph = (uint32_t)(i / nstages) & 1u;
+            if (!mbar_wait_patient_warp(smem_u32(RAW ? &bar_raw_empty : &bar_empty[s]), ph ^ 1u, abort_flag))
+                break;
+            const int32_t h0 = ty * 2 * p.jp - p.pad;
+            if (elect_one()) {
                 if (RAW) {
                     const uint32_t full = smem_u32(&bar_raw_full);
                     mbar_expect_tx(full, (uint32_t)p.raw_bytes);
@@ -827,92 +886,92 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                     tma_load_4d(raw_base, &map_x_hi, full, -p.pad - p.off_x, h0, 0, img);
                 } else {
                     const uint32_t full = smem_u32(&bar_full[s]), dst = stage_base + (uint32_t)s * stage_bytes;
-                    mbar_expect_tx(full, 4u * (uint32_t)(p.region_rows * p.pw * kCP_RowB));
+                    if (rank == 0) // both CTAs' bytes are counted on the leader's barrier
+                        mbar_expect_tx(full, 2u * 4u * (uint32_t)(p.region_rows * p.pw * kCP_RowB));
                     for (int g = 0; g < 2; ++g) { // region g: rows h0 + g + 2 i, which lie in one of the two sub-images
                         const int32_t row = (h0 + g) >> 1, sub = (h0 + g) & 1;
-                        tma_load_5d(dst + (uint32_t)g * region, &map_x_hi, full, 0, -p.pad, row, sub, img);
-                        tma_load_5d(dst + (uint32_t)(2 + g) * region, &map_x_lo, full, 0, -p.pad, row, sub, img);
+                        tma_load_5d_pair(dst + (uint32_t)g * region, &map_x_hi, leader_addr(full), 0, -p.pad, row, sub, img);
+                        tma_load_5d_pair(dst + (uint32_t)(2 + g) * region, &map_x_lo, leader_addr(full), 0, -p.pad, row, sub, img);
                     }
                 }
-                ++i;
             }
-            if (*abort_flag) {
-                // unwind: let the copies still in flight land before the CTA goes away
-                for (int k2 = i - nstages < 0 ? 0 : i - nstages; k2 < i; ++k2) {
-                    const uint32_t bar = smem_u32(RAW ? &bar_raw_full : &bar_full[k2 % nstages]);
-                    const uint64_t t0  = globaltimer_ns();
-                    while (!mbar_try_wait(bar, (uint32_t)(k2 / nstages) & 1u) && globaltimer_ns() - t0 < kWaitBudgetNs) {
-                    }
+            __syncwarp();
+            ++i;
+        }
+        if (*abort_flag && (RAW || rank == 0)) {
+            // unwind: let the copies still in flight land before the CTA goes away (from planes the leader's barriers count the
+            // partner's copies too, and neither CTA leaves before the other)
+            for (int k2 = i - nstages < 0 ? 0 : i - nstages; k2 < i; ++k2) {
+                const uint32_t bar = smem_u32(RAW ? &bar_raw_full : &bar_full[k2 % nstages]);
+                const uint64_t t0  = globaltimer_ns();
+                while (!mbar_try_wait(bar, (uint32_t)(k2 / nstages) & 1u) && globaltimer_ns() - t0 < kWaitBudgetNs) {
                 }
             }
         }
     } else if (warp == 1) {
         // ===== MMA issuer =====
-        if (lane == 0) {
-            const uint32_t idesc2 = make_idesc(0u, 128, (uint32_t)(2 * p.kop)), idesc1 = make_idesc(0u, 128, (uint32_t)p.kop);
+        // (the leader's, for the pair; a whole warp with uniform control flow, so that descriptors stay in uniform registers)
+        if (rank == 0) {
+            const uint32_t idesc2 = make_idesc(0u, 256, (uint32_t)(2 * p.kop)), idesc1 = make_idesc(0u, 256, (uint32_t)p.kop);
             const bool two = p.c > 16; // k-steps that hold channels
             // descriptors are moved by adding to their address field (16-byte units; shared memory is far below its range)
-            const uint64_t filter0 = smem_desc_k<kCP_RowB>(smem_base), lo_terms = (uint64_t)(2 * region >> 4);
-            const uint64_t filter_step = (uint64_t)(2 * p.kop * kCP_RowB >> 4);
-            const uint32_t kop = (uint32_t)p.kop;
-            const uint64_t w_lo = (uint64_t)(p.kop * kCP_RowB >> 4);
-            int i   = 0;
+            const uint32_t unit = kCP_RowB >> 4, lo_terms = 2 * region >> 4, kop = (uint32_t)p.kop;
+            const uint32_t p_0 = (uint32_t)smem_desc_k<kCP_RowB>(smem_base), q_0 = p_0 + (uint32_t)q_at * unit, last_lo = p_0 + (uint32_t)r_at * unit;
+            auto desc = [](uint32_t low) { return smem_desc_k<kCP_RowB>(0) & 0xffffffff00000000ull | low; };
+            int i   = 0, s = 0;
+            uint32_t full_phase = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-                if (!RAW && p.image_scale[tile / p.tiles_y] == 0.0f)
+            for (int u = first; u < pairs; u += stride) {
+                if (!wanted(u))
                     continue;
-                const int s = i % p.stages, set = i & 1;
+                const int set = i & 1;
                 // the accumulators have been read, the planes are complete
-                ok = mbar_wait(smem_u32(&bar_acc_empty[set]), ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag) &&
-                     mbar_wait(smem_u32(&bar_full[s]), (uint32_t)(i / p.stages) & 1u, abort_flag);
+                ok = mbar_wait_warp(smem_u32(&bar_acc_empty[set]), ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag) &&
+                     mbar_wait_warp(smem_u32(&bar_full[s]), full_phase, abort_flag);
                 if (!ok)
                     break;
                 tc_fence_after_sync();
                 const uint32_t hi0 = stage_base + (uint32_t)s * stage_bytes;
                 const uint32_t d_even = tmem_base + (uint32_t)(set * 256), d_odd = d_even + 128u;
-                uint64_t db = filter0;
-                uint32_t accumulate = 0u;
-                const int rows = RAW && *const_cast<volatile float *>(&tile_scale[s]) == 0.0f ? 0 : p.kh;
-                for (int r = 0; r < rows; ++r) {
+                uint32_t w_p = p_0, w_q = q_0, accumulate = 0u;
+                auto step = [&](uint32_t even, uint32_t odd, uint32_t k, uint32_t acc) {
+                    mma_f16_pair_warp(d_even, desc(even + k), desc(w_p + k), idesc2, acc);
+                    mma_f16_pair_warp(d_odd, desc(odd + k), desc(w_p + k), idesc2, acc);
+                    mma_f16_pair_warp(d_even + kop, desc(even + lo_terms + k), desc(w_q + k), idesc1, 1u);
+                    mma_f16_pair_warp(d_odd + kop, desc(odd + lo_terms + k), desc(w_q + k), idesc1, 1u);
+                };
+                for (int r = 0; r < p.kh; ++r) {
                     // the tap's pixels for the even and the odd output rows
-                    uint64_t even = smem_desc_k<kCP_RowB>(hi0 + (uint32_t)(r & 1) * region + (uint32_t)((r >> 1) * p.pw * kCP_RowB));
-                    uint64_t odd  = smem_desc_k<kCP_RowB>(hi0 + (uint32_t)((r + 1) & 1) * region + (uint32_t)(((r + 1) >> 1) * p.pw * kCP_RowB));
-                    const int taps = r + 1 < rows ? p.kw : p.kw - 1; // all but the last
-                    for (int sx = 0; sx < taps; ++sx, even += kCP_RowB >> 4, odd += kCP_RowB >> 4, db += filter_step) {
-                        mma_f16(d_even, even, db, idesc2, accumulate);
-                        mma_f16(d_odd, odd, db, idesc2, accumulate);
-                        mma_f16(d_even + kop, even + lo_terms, db, idesc1, 1u);
-                        mma_f16(d_odd + kop, odd + lo_terms, db, idesc1, 1u);
+                    uint32_t even = (uint32_t)smem_desc_k<kCP_RowB>(hi0 + (uint32_t)(r & 1) * region + (uint32_t)((r >> 1) * p.pw * kCP_RowB));
+                    uint32_t odd  = (uint32_t)smem_desc_k<kCP_RowB>(hi0 + (uint32_t)((r + 1) & 1) * region + (uint32_t)(((r + 1) >> 1) * p.pw * kCP_RowB));
+                    const int whole = r + 1 < p.kh ? p.kw : p.kw - 1; // all but the last tap
+                    for (int sx = 0; sx < whole; ++sx, even += unit, odd += unit, w_p += kop * unit, w_q += (kop >> 1) * unit) {
+                        step(even, odd, 0, accumulate);
                         accumulate = 1u;
-                        if (two) {
-                            mma_f16(d_even, even + 2, db + 2, idesc2, 1u);
-                            mma_f16(d_odd, odd + 2, db + 2, idesc2, 1u);
-                            mma_f16(d_even + kop, even + lo_terms + 2, db + 2, idesc1, 1u);
-                            mma_f16(d_odd + kop, odd + lo_terms + 2, db + 2, idesc1, 1u);
-                        }
+                        if (two)
+                            step(even, odd, 2, 1u);
                     }
-                    if (r + 1 == rows) {
-                        if (two) {
-                            mma_f16(d_even, even, db, idesc2, 1u);
-                            mma_f16(d_odd, odd, db, idesc2, 1u);
-                            mma_f16(d_even + kop, even + lo_terms, db, idesc1, 1u);
-                            mma_f16(d_odd + kop, odd + lo_terms, db, idesc1, 1u);
-                            even += 2, odd += 2, db += 2;
-                        }
-                        mma_f16(d_even + kop, even + lo_terms, db, idesc1, 1u);
-                        mma_f16(d_odd + kop, odd + lo_terms, db, idesc1, 1u);
-                        mma_f16(d_even + kop, even, db + w_lo, idesc1, 1u);
-                        mma_f16(d_odd + kop, odd, db + w_lo, idesc1, 1u);
-                        mma_f16_shifted<kHalfLoBits>(d_even + kop, even, db, idesc1);
-                        mma_f16_shifted<kHalfLoBits>(d_odd + kop, odd, db, idesc1);
+                    if (r + 1 == p.kh) {
+                        uint32_t k = 0;
+                        if (two)
+                            step(even, odd, 0, 1u), k = 2;
+                        mma_f16_pair_warp(d_even + kop, desc(even + lo_terms + k), desc(w_q + k), idesc1, 1u);
+                        mma_f16_pair_warp(d_odd + kop, desc(odd + lo_terms + k), desc(w_q + k), idesc1, 1u);
+                        mma_f16_pair_warp(d_even + kop, desc(even + k), desc(last_lo + k), idesc1, 1u);
+                        mma_f16_pair_warp(d_odd + kop, desc(odd + k), desc(last_lo + k), idesc1, 1u);
+                        mma_f16_shifted_pair_warp<kHalfLoBits>(d_even + kop, desc(even + k), desc(w_q + k), idesc1);
+                        mma_f16_shifted_pair_warp<kHalfLoBits>(d_odd + kop, desc(odd + k), desc(w_q + k), idesc1);
                     }
                 }
-                tc_commit(smem_u32(&bar_empty[s]));      // the stage is free once these MMAs have retired
-                tc_commit(smem_u32(&bar_acc_full[set])); // and the accumulators are complete
+                tc_commit_pair_warp(smem_u32(&bar_empty[s]));      // the stage is free once these MMAs have retired
+                tc_commit_pair_warp(smem_u32(&bar_acc_full[set])); // and the accumulators are complete
                 ++i;
+                if (++s == p.stages)
+                    s = 0, full_phase ^= 1u;
             }
             if (!ok || *abort_flag) {
-                tc_commit(smem_u32(&bar_done));
+                __syncwarp();
+                tc_commit_pair_warp(smem_u32(&bar_done));
                 const uint64_t t0 = globaltimer_ns();
                 while (!mbar_try_wait(smem_u32(&bar_done), 0) && globaltimer_ns() - t0 < kWaitBudgetNs) {
                 }
@@ -927,11 +986,12 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
             const float *raw  = reinterpret_cast<const float *>(smem_ptr + (raw_base - smem_base));
             const bool one    = npos <= 32 * kCP_CvtWarps;
             const int first_raw = ct / p.pw * p.box_w + ct % p.pw + p.off_x;
-            int i = 0;
-            for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++i) {
-                const int s = i % p.stages;
-                bool got = mbar_wait_patient(smem_u32(&bar_raw_full), (uint32_t)i & 1u, abort_flag);
-                if (!__all_sync(0xffffffffu, got))
+            int i = 0, s = 0;
+            uint32_t stage_phase = 1u;
+            for (int u = first; u < pairs; u += stride, ++i) {
+                const int tile = tile_of(u);
+                if (!group_wait(
+                        warp == 2, [&] { return mbar_wait(smem_u32(&bar_raw_full), (uint32_t)i & 1u, abort_flag); }, cvt_word, 0, 1, 32 * kCP_CvtWarps))
                     break;
                 // The tile's range.  Where every thread has at most one position its channels stay in registers between the range
                 // and the split, and the box is free for the next tile's before this one's planes are.
@@ -957,24 +1017,24 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                     }
                 }
                 range = range_warp(range);
-                if (lane == 0) {
+                if (lane == 0)
                     cvt_range[i & 1][warp - 2] = range;
-                    mbar_arrive(smem_u32(&bar_cvt));
-                }
-                got = mbar_wait(smem_u32(&bar_cvt), (uint32_t)i & 1u, abort_flag) && // all ranges
-                      mbar_wait_patient(smem_u32(&bar_empty[s]), ((uint32_t)(i / p.stages) & 1u) ^ 1u, abort_flag) &&
-                      mbar_wait_patient(smem_u32(&bar_scale_empty[s]), ((uint32_t)(i / p.stages) & 1u) ^ 1u, abort_flag);
-                if (!__all_sync(0xffffffffu, got))
+                // all ranges are there, the stage is free, and so is its scale
+                if (!group_wait(
+                        warp == 2,
+                        [&] {
+                            return mbar_wait(smem_u32(&bar_empty[s]), stage_phase, abort_flag) &&
+                                   mbar_wait(smem_u32(&bar_scale_empty[s]), stage_phase, abort_flag);
+                        },
+                        cvt_word, 1, 1, 32 * kCP_CvtWarps))
                     break;
 #pragma unroll
                 for (int u = 0; u < kCP_CvtWarps; ++u)
                     range = range_join(range, cvt_range[i & 1][u]);
                 float scale, inverse;
                 const bool fits = half_tile_fits(range, scale, inverse);
-                if (ct == 0) {
-                    tile_scale[s]      = fits ? inverse : 0.0f;
-                    p.tile_range[tile] = range;
-                }
+                if (ct == 0)
+                    tile_scale[s] = fits ? inverse : 0.0f;
                 uint8_t *planes = smem_ptr + p.filter_bytes + (uint32_t)s * stage_bytes;
                 // a position's (y, x) 32 channels become row (y >> 1) * pw + x of region y & 1 in both planes, 16-byte chunk j
                 // at j ^ ((row >> 1) & 3), the 64-byte swizzle
@@ -1010,10 +1070,14 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive(smem_u32(&bar_full[s]));
+                    mbar_arrive_peer(leader_addr(smem_u32(&bar_full[s])));
                     if (!one)
                         mbar_arrive(smem_u32(&bar_raw_empty));
                 }
+                if (ct == 0)
+                    p.tile_range[tile] = range;
+                if (++s == p.stages)
+                    s = 0, stage_phase ^= 1u;
             }
         }
     } else {
@@ -1025,14 +1089,16 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
         const int64_t plane = p.pool ? (int64_t)(p.ho >> 1) * (p.wo >> 1) : (int64_t)p.ho * p.wo;
         const bool inside = j < p.jp && x < p.wo && !(p.pool && (x & 1));
         const bool relu = p.act == CT_ACT_RELU;
-        int i = 0;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-            const int img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
-            if (!RAW && p.image_scale[img] == 0.0f)
+        int i = 0, s = 0;
+        for (int u = first; u < pairs; u += stride) {
+            if (!wanted(u))
                 continue;
-            const int set = i & 1, s = i % p.stages;
-            bool got = mbar_wait_patient(smem_u32(&bar_acc_full[set]), (uint32_t)(i >> 1) & 1u, abort_flag);
-            if (!__all_sync(0xffffffffu, got))
+            const int tile = tile_of(u), img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
+            const bool mine = 2 * u + rank < total_tiles;
+            const int set = i & 1;
+            if (!group_wait(
+                    warp == 2 + kCP_CvtWarps, [&] { return mbar_wait(smem_u32(&bar_acc_full[set]), (uint32_t)(i >> 1) & 1u, abort_flag); }, epi_word, i, 2,
+                    32 * kCP_EpiWarps))
                 break;
             const float is = RAW ? *const_cast<volatile float *>(&tile_scale[s]) : p.image_scale[img];
             tc_fence_after_sync();
@@ -1040,9 +1106,10 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
             const bool live_even = inside && y < p.ho, live_low = inside && !p.pool && y + 1 < p.ho; // pooled rows are even and odd
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(set * 256);
             float *dst = p.out + ((int64_t)img * p.ko + half * 16) * plane + (p.pool ? (int64_t)(y >> 1) * (p.wo >> 1) + (x >> 1) : (int64_t)y * p.wo + x);
+            const uint64_t is2 = pack2(is, is);
             // Values of sixteen channels, then their neighbours, then the stores, without a branch among them: channel after
             // channel, with the activation behind a branch, a group took 4300 clocks.
-            for (int g = half; g < groups && !(RAW && is == 0.0f); g += 2, dst += 32 * plane) {
+            for (int g = half; g < groups && is != 0.0f && mine; g += 2, dst += 32 * plane) {
                 float even[16], odd[16];
 #pragma unroll
                 for (int h = 0; h < 16; h += 8) {
@@ -1056,16 +1123,18 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                     for (int u = 0; u < 8; u += 4) {
                         const float4 f4 = *reinterpret_cast<const float4 *>(filter_inv + 16 * g + h + u);
                         const float4 b4 = *reinterpret_cast<const float4 *>(bias_s + 16 * g + h + u);
-                        const float fs[4] = {__fmul_rn(f4.x, is), __fmul_rn(f4.y, is), __fmul_rn(f4.z, is), __fmul_rn(f4.w, is)};
-                        const float bs[4] = {b4.x, b4.y, b4.z, b4.w};
+                        const uint64_t fs[2] = {mul2(pack2(f4.x, f4.y), is2), mul2(pack2(f4.z, f4.w), is2)}, bs[2] = {pack2(b4.x, b4.y), pack2(b4.z, b4.w)};
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            auto value = [&](uint32_t main, uint32_t cross) { // the products with powers of two are exact
-                                float v = __fadd_rn(__uint_as_float(main), __uint_as_float(cross));
-                                v       = __fadd_rn(__fmul_rn(v, fs[q]), bs[q]);
-                                return !relu || v > 0.0f ? v : __fmul_rn(v, 0.0f);
+                        for (int q = 0; q < 4; q += 2) {
+                            auto value = [&](const uint32_t (&main)[8], const uint32_t (&cross)[8], float *to) { // the products with powers of two are exact
+                                const uint64_t v = add2(mul2(add2(pack2(main[u + q], main[u + q + 1]), pack2(cross[u + q], cross[u + q + 1])), fs[q / 2]), bs[q / 2]);
+                                float x, y, x0, y0;
+                                unpack2(v, x, y);
+                                unpack2(mul2(v, 0ull), x0, y0);
+                                to[0] = !relu || x > 0.0f ? x : x0;
+                                to[1] = !relu || y > 0.0f ? y : y0;
                             };
-                            even[h + u + q] = value(a[u + q], b[u + q]), odd[h + u + q] = value(c[u + q], d[u + q]);
+                            value(a, b, even + h + u + q), value(c, d, odd + h + u + q);
                         }
                     }
                 }
@@ -1095,22 +1164,25 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive(smem_u32(&bar_acc_empty[set]));
+                mbar_arrive_peer(leader_addr(smem_u32(&bar_acc_empty[set])));
                 if (RAW)
                     mbar_arrive(smem_u32(&bar_scale_empty[s]));
             }
             ++i;
+            if (++s == p.stages)
+                s = 0;
         }
     }
 
     tc_fence_before_sync();
     __syncthreads();
+    cluster_sync(); // neither CTA goes while the other's MMAs, copies or arrivals may still reach it
     if (warp == 1) {
         __syncwarp();
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, 512);
+        tmem_dealloc_pair(tmem_base, 512);
     }
-    if (threadIdx.x == 0 && *abort_flag)
+    if (threadIdx.x == 0 && !failed && *abort_flag)
         atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
 }
 
@@ -1157,7 +1229,7 @@ static bool conv_tmem_plan(
 
 static bool conv_pair_plan(
     ConvPairParams &p, int64_t c, int64_t h, int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t pad, bool raw, size_t *smem) {
-    p.ko = (int)ko, p.kop = (int)((ko + 15) / 16 * 16), p.c = (int)c;
+    p.ko = (int)ko, p.kop = (int)((ko + 31) / 32 * 32), p.c = (int)c;
     p.kh = (int)kh, p.kw = (int)kw, p.pad = (int)pad;
     p.pw  = (int)(wd + 2 * pad);
     p.wo  = p.pw - (int)kw + 1;
@@ -1171,7 +1243,7 @@ static bool conv_pair_plan(
     // a tap's window of 128 rows may run past the region: reserve those rows too
     const int rows = std::max(p.region_rows * p.pw, (int)(kh / 2) * p.pw + (int)kw - 1 + 128);
     p.region_bytes = (rows * kCP_RowB + 1023) & ~1023;
-    p.filter_bytes = (int)((kh * kw * 2 * p.kop * kCP_RowB + 1023) & ~1023);
+    p.filter_bytes = (int)(((kh * kw * 3 + 1) * (p.kop / 2) * kCP_RowB + 1023) & ~1023);
     // raw mode: the box starts at the 16-byte boundary at or left of x = -pad and is a whole number of 16-byte units wide
     p.off_x      = (((int)pad + 3) & ~3) - (int)pad;
     p.box_w      = (p.off_x + p.pw + 3) & ~3;
@@ -1257,7 +1329,7 @@ ct_status conv_tmem_filters(
         attr_set_dev[st->device & 15] = true;
     }
     const size_t smem32 = (size_t)pt.stages * 2 * pt.plane_bytes + (raw ? (size_t)kTA_RawStages * pt.raw_stride : 0) + kTA_StagingBytes + 1024;
-    const unsigned grid   = (unsigned)std::min<int64_t>(pair_tiles, st->sm_count);
+    const unsigned grid   = 2u * (unsigned)std::min<int64_t>((pair_tiles + 1) / 2, st->sm_count / 2);
     const unsigned grid32 = (unsigned)std::max<int64_t>(std::min<int64_t>(tiles, st->sm_count), (tiles + kTA_MaxOwn - 1) / kTA_MaxOwn);
     if (raw) {
         // the input [batch][c][h][w]; box = box_w floats x box_rows rows x 32 channels of one image, not
@@ -1276,7 +1348,7 @@ ct_status conv_tmem_filters(
         cudaError_t launched;
         {
             ProfScope prof("gemm_tc");
-            (void)launch_dependent(conv_pairs_kernel<true>, dim3(grid), dim3(kCP_Threads), pair_smem, stream(), map, map, pp, (int)pair_tiles);
+            (void)launch_dependent_cluster(conv_pairs_kernel<true>, 2, dim3(grid), dim3(kCP_Threads), pair_smem, stream(), map, map, pp, (int)pair_tiles);
             (void)launch_dependent(conv_tmem_filters_kernel<true>, dim3(grid32), dim3(kTA_ThreadsRaw), smem32, stream(), map32, map32, pt, (int)tiles);
             launched = cudaGetLastError();
         }
@@ -1316,7 +1388,7 @@ ct_status conv_tmem_filters(
     CT_TRY(encode32(&m32_hi, planes));
     CT_TRY(encode32(&m32_lo, planes + slot / 2));
     ProfScope prof("gemm_tc");
-    (void)launch_dependent(conv_pairs_kernel<false>, dim3(grid), dim3(kCP_Threads), pair_smem, stream(), m16_hi, m16_lo, pp, (int)pair_tiles);
+    (void)launch_dependent_cluster(conv_pairs_kernel<false>, 2, dim3(grid), dim3(kCP_Threads), pair_smem, stream(), m16_hi, m16_lo, pp, (int)pair_tiles);
     CT_LAUNCH_CHECK("conv_pairs");
     (void)launch_dependent(conv_tmem_filters_kernel<false>, dim3(grid32), dim3(kTA_Threads), smem32, stream(), m32_hi, m32_lo, pt, (int)tiles);
     CT_LAUNCH_CHECK("conv_tmem_filters");

@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(kHThreads, 1)
                 __syncwarp();
                 if (lane == 0) {
                     if (CG == 2)
-                        mbar_arrive_cluster(leader_addr(bar));
+                        mbar_arrive_peer(leader_addr(bar));
                     else
                         mbar_arrive(bar);
                 }

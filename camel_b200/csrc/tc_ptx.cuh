@@ -140,6 +140,21 @@ __device__ __forceinline__ bool mbar_wait_patient_warp(uint32_t bar, uint32_t pa
     return __all_sync(0xffffffffu, got) != 0;
 }
 
+// A wait of several warps: the first of them waits, the others stop at named barrier `id` of `threads` threads, which takes no issue
+// slots (an mbarrier wait polls: with eighteen warps of the few-channel convolution waiting by themselves a third of all its
+// instructions, 65 of 200 million at 2048 images, were theirs).  All get the same answer, so that all leave when it ran out; `word` holds
+// it, two of them in turn.  As bounded as the first warp's wait.
+template <typename Wait>
+__device__ __forceinline__ bool group_wait(bool waits, Wait wait, volatile int *word, int turn, int id, int threads) {
+    if (waits) {
+        const bool all = __all_sync(0xffffffffu, wait()) != 0;
+        if ((threadIdx.x & 31) == 0)
+            word[turn & 1] = all ? 1 : 0;
+    }
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+    return __any_sync(0xffffffffu, word[turn & 1]) != 0;
+}
+
 // ---- TMA --------------------------------------------------------------------------------
 
 __device__ __forceinline__ void prefetch_tensormap(const void *map) {
@@ -248,20 +263,6 @@ __device__ __forceinline__ void mma_f16(
         : "memory");
 }
 
-// D = A . B + D * 2^-SHIFT (0 .. 15)
-template <int SHIFT>
-__device__ __forceinline__ void mma_f16_shifted(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, 1, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %4;\n\t"
-        "}\n"
-        :
-        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(SHIFT)
-        : "memory");
-}
-
 // ---- CTA pairs (clusters of two CTAs that work on one 256-row tile) ----------------------------
 //
 // With cta_group::2 one thread of the leader (rank 0) issues MMAs of 256 rows: each CTA of the pair holds
@@ -305,8 +306,12 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
                  : "memory");
     return v;
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+// An arrival on the leader's barrier where nothing is published to the other CTA's threads: a warp that hands back tensor memory (what it has read is in
+// registers, tcgen05.wait::ld, and ordered by tcgen05.fence), or that has filled its own CTA's operands (visible to the tensor core by
+// fence.proxy.async).  With release at cluster scope the arrival waits until the thread's earlier stores to global memory are in L2:
+// 2200 clocks of a tile of the few-channel convolution, whose epilogue stores before it hands back.
+__device__ __forceinline__ void mbar_arrive_peer(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 // Tile load into THIS CTA's shared memory whose bytes are counted on a barrier of this CTA or the leader.
 __device__ __forceinline__ void tma_load_2d_pair(
@@ -316,6 +321,15 @@ __device__ __forceinline__ void tma_load_2d_pair(
         " [%0], [%1, {%3, %4}], [%2];"
         :
         : "r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(cluster_bar), "r"(c0), "r"(c1)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_5d_pair(
+    uint32_t dst_smem, const void *map, uint32_t cluster_bar, int32_t c0, int32_t c1, int32_t c2, int32_t c3, int32_t c4) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+        :
+        : "r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(cluster_bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
         : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t columns) {
@@ -386,6 +400,20 @@ __device__ __forceinline__ void mma_tf32_pair_warp(
         "}\n"
         :
         : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// D = A . B + D * 2^-SHIFT (0 .. 15)
+template <int SHIFT>
+__device__ __forceinline__ void mma_f16_shifted_pair_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, 1, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p, %4;\n\t"
+        "}\n"
+        :
+        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(SHIFT)
         : "memory");
 }
 __device__ __forceinline__ void tc_commit_pair_warp(uint32_t bar) {
