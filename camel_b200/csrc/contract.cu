@@ -305,24 +305,30 @@ __global__ void __launch_bounds__(256) conv2d_small_c_kernel(
 // 8-byte broadcast read and the layer is bound by the return bandwidth of shared memory (128 B per
 // clock and SM), four times above what writing the result costs.  Same arithmetic: float64
 // accumulation in (r, s) order, bias last, one rounding.
-__global__ void __launch_bounds__(256) conv2d_c1_3x3_kernel(
+//
+// What bounds it: the float64 pipe, 36 multiply-adds with operands from all over the register file (0.41 of them per clock and
+// quarter of an SM, 0.47 from few registers) and four narrowings per filter, 165 us at 8192 x 1 x 28 x 28 -> 32 where writing the
+// result takes 125.  Blocks of 128 threads with 72 registers put 28 warps on an SM instead of 24 and let the compiler walk the
+// filters by one pointer: 205 -> 190 us.  Two or four filters at a time (193 and 196, more registers) gain less.
+constexpr int kC1Threads = 128;
+__global__ void __launch_bounds__(kC1Threads, 7) conv2d_c1_3x3_kernel(
     const float *__restrict__ x, const float *__restrict__ wt, const float *__restrict__ bias,
     int64_t n, int64_t h, int64_t w, int ko, int64_t pad, int64_t ho, int64_t wo, int act,
     float *__restrict__ out) {
     griddep_wait();
     griddep_launch_dependents();
-    extern __shared__ double w_s[]; // [ko][9], then the bias
-    for (int i = threadIdx.x; i < ko * 9; i += 256)
-        w_s[i] = (double)wt[i];
-    for (int i = threadIdx.x; bias && i < ko; i += 256)
-        w_s[ko * 9 + i] = (double)bias[i];
+    extern __shared__ double w_s[]; // [ko][10]: nine taps and the bias
+    for (int i = threadIdx.x; i < ko * 9; i += kC1Threads)
+        w_s[i / 9 * 10 + i % 9] = (double)wt[i];
+    for (int i = threadIdx.x; bias && i < ko; i += kC1Threads)
+        w_s[i * 10 + 9] = (double)bias[i];
     __syncthreads();
     const int64_t quads = wo >> 2; // wo is a multiple of 4
     const int64_t pix   = ho * wo;
     const int64_t total = n * ho * quads;
-    const int64_t step  = (int64_t)gridDim.x * 256;
+    const int64_t step  = (int64_t)gridDim.x * kC1Threads;
     const bool small    = total + step <= 0x7fffffff; // 64-bit divisions are a hundred instructions each
-    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += step) {
+    for (int64_t i = (int64_t)blockIdx.x * kC1Threads + threadIdx.x; i < total; i += step) {
         int64_t qx, oy, img;
         if (small) {
             const uint32_t row = (uint32_t)i / (uint32_t)quads;
@@ -344,8 +350,9 @@ __global__ void __launch_bounds__(256) conv2d_c1_3x3_kernel(
             }
         }
         float *dst = out + img * ko * pix + oy * wo + ox;
-        for (int o = 0; o < ko; ++o) {
-            const double *wr = w_s + o * 9;
+        const double *wr = w_s;
+#pragma unroll 1
+        for (int o = 0; o < ko; ++o, wr += 10, dst += pix) {
             double acc[4]    = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
             for (int r = 0; r < 3; ++r)
@@ -359,11 +366,11 @@ __global__ void __launch_bounds__(256) conv2d_c1_3x3_kernel(
             float v[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                v[j] = (float)(bias ? acc[j] + w_s[ko * 9 + o] : acc[j]);
+                v[j] = (float)(bias ? acc[j] + wr[9] : acc[j]);
                 if (act == CT_ACT_RELU)
                     v[j] = __fmul_rn(v[j], v[j] > 0.0f ? 1.0f : 0.0f);
             }
-            *reinterpret_cast<float4 *>(dst + (int64_t)o * pix) = make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
         }
     }
 }
@@ -735,7 +742,7 @@ static ct_status conv2d_run(
             CT_CUDA(cudaFuncSetAttribute(conv2d_c1_3x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 56 * 1024));
             attr_set_dev[st->device & 15] = true;
         }
-        (void)launch_dependent(conv2d_c1_3x3_kernel, dim3(capped_blocks(st, n * ho * (wo >> 2), 16)), dim3(256), (size_t)ko * 80, stream(),
+        (void)launch_dependent(conv2d_c1_3x3_kernel, dim3(capped_blocks(st, n * ho * (wo >> 2) * 2, 32)), dim3(kC1Threads), (size_t)ko * 80, stream(),
             x, w, bias, n, h, wd, (int)ko, pad, ho, wo, act, out);
         CT_LAUNCH_CHECK("conv2d_c1_3x3");
         return CT_OK;

@@ -373,6 +373,49 @@ __global__ void __launch_bounds__(kHThreads, 1)
         }
         return;
     }
+    // One stage by TMA: values of k from kc, rows of A from a_row and of B from b_row.
+    auto load_stage = [&](const CUtensorMap *ma_hi, const CUtensorMap *ma_lo, const CUtensorMap *mb_hi, const CUtensorMap *mb_lo,
+                          int s, int32_t kc, int32_t a_row, int32_t b_row) {
+        uint32_t full      = smem_u32(&bar_full[s]);
+        const uint32_t dst = stage_addr(s);
+        if (CG == 2) {
+            // both CTAs' bytes are counted on the leader's barrier
+            if (rank == 0)
+                mbar_expect_tx(full, 2u * (uint32_t)C::kStageBytes);
+            full = leader_addr(full);
+            tma_load_2d_pair(dst, ma_hi, full, kc, a_row);
+            tma_load_2d_pair(dst + 2 * C::kABytes, mb_hi, full, kc, b_row);
+            tma_load_2d_pair(dst + C::kABytes, ma_lo, full, kc, a_row);
+            tma_load_2d_pair(dst + 2 * C::kABytes + C::kBBytes, mb_lo, full, kc, b_row);
+        } else {
+            mbar_expect_tx(full, (uint32_t)C::kStageBytes);
+            tma_load_2d(dst, ma_hi, full, kc, a_row);
+            tma_load_2d(dst + 2 * C::kABytes, mb_hi, full, kc, b_row);
+            tma_load_2d(dst + C::kABytes, ma_lo, full, kc, a_row);
+            tma_load_2d(dst + 2 * C::kABytes + C::kBBytes, mb_lo, full, kc, b_row);
+        }
+    };
+    auto rows_of = [&](int tm, int tn, int tz, int32_t &a_row, int32_t &b_row) {
+        a_row = (tm * CG + rank) * kHM;
+        b_row = (p.batch > 1 ? tz * (int32_t)p.n : 0) + tn * BN + rank * C::kBRows;
+    };
+    // The first tile's first float16 stages are fetched before it is known whether there are too many exceptions (that word
+    // comes from L2, 0.7 us behind the wait above); where there are, the issuer passes them over.
+    int ahead = 0;
+    if (!LEFT && !p.force_wide && !failed && first < p.total_tiles) {
+        int tm, tn, tz, band;
+        half_tile(p, first, tm, tn, tz, band);
+        const int first_group = p.groups_per_split > 0 ? tz * p.groups_per_split : 0;
+        const int left        = p.k_groups > first_group ? p.k_groups - first_group : 0;
+        ahead = (p.groups_per_split > 0 && left > p.groups_per_split ? p.groups_per_split : left) * (64 / (RB / 2));
+        ahead = ahead < C::kStages ? ahead : C::kStages;
+        if (warp == 0 && elect_one()) {
+            int32_t a_row, b_row;
+            rows_of(tm, tn, tz, a_row, b_row);
+            for (int s = 0; s < ahead; ++s)
+                load_stage(&maps.a16_hi, &maps.a16_lo, &maps.b16_hi, &maps.b16_lo, s, first_group * 64 + s * (RB / 2), a_row, b_row);
+        }
+    }
     const bool wide = p.force_wide || half_wide(p.exceptions_a, p.exceptions_b);
     const int k_step    = wide ? RB / 4 : RB / 2; // values of k per stage
     const int per_group = 64 / k_step;            // stages per 64 values of k
@@ -396,38 +439,23 @@ __global__ void __launch_bounds__(kHThreads, 1)
         if (elect_one()) {
             const CUtensorMap *ma_hi = wide ? &maps.a32_hi : &maps.a16_hi, *ma_lo = wide ? &maps.a32_lo : &maps.a16_lo;
             const CUtensorMap *mb_hi = wide ? &maps.b32_hi : &maps.b16_hi, *mb_lo = wide ? &maps.b32_lo : &maps.b16_lo;
-            int s = 0, issued = 0;
-            uint32_t phase = 1;
+            int s = ahead == C::kStages ? 0 : ahead, issued = ahead;
+            uint32_t phase = ahead == C::kStages ? 0 : 1;
             bool ok        = true;
             for (int tile = first; tile < p.total_tiles && ok; tile += stride) {
                 int tm, tn, tz, band, first_group, nkb;
                 half_tile(p, tile, tm, tn, tz, band);
                 k_range(tz, first_group, nkb);
-                int32_t kc             = first_group * 64;
-                const int32_t a_row    = (tm * CG + rank) * kHM, b_row = (p.batch > 1 ? tz * (int32_t)p.n : 0) + tn * BN + rank * C::kBRows;
-                for (int kb = 0; kb < nkb; ++kb, kc += k_step, ++issued) {
+                int32_t a_row, b_row;
+                rows_of(tm, tn, tz, a_row, b_row);
+                int kb     = tile == first && !wide ? ahead : 0;
+                int32_t kc = first_group * 64 + kb * k_step;
+                for (; kb < nkb; ++kb, kc += k_step, ++issued) {
                     if (!mbar_wait(smem_u32(&bar_empty[s]), phase, abort_flag)) {
                         ok = false;
                         break;
                     }
-                    uint32_t full      = smem_u32(&bar_full[s]);
-                    const uint32_t dst = stage_addr(s);
-                    if (CG == 2) {
-                        // both CTAs' bytes are counted on the leader's barrier
-                        if (rank == 0)
-                            mbar_expect_tx(full, 2u * (uint32_t)C::kStageBytes);
-                        full = leader_addr(full);
-                        tma_load_2d_pair(dst, ma_hi, full, kc, a_row);
-                        tma_load_2d_pair(dst + 2 * C::kABytes, mb_hi, full, kc, b_row);
-                        tma_load_2d_pair(dst + C::kABytes, ma_lo, full, kc, a_row);
-                        tma_load_2d_pair(dst + 2 * C::kABytes + C::kBBytes, mb_lo, full, kc, b_row);
-                    } else {
-                        mbar_expect_tx(full, (uint32_t)C::kStageBytes);
-                        tma_load_2d(dst, ma_hi, full, kc, a_row);
-                        tma_load_2d(dst + 2 * C::kABytes, mb_hi, full, kc, b_row);
-                        tma_load_2d(dst + C::kABytes, ma_lo, full, kc, a_row);
-                        tma_load_2d(dst + 2 * C::kABytes + C::kBBytes, mb_lo, full, kc, b_row);
-                    }
+                    load_stage(ma_hi, ma_lo, mb_hi, mb_lo, s, kc, a_row, b_row);
                     if (++s == C::kStages)
                         s = 0, phase ^= 1u;
                 }
@@ -475,6 +503,12 @@ __global__ void __launch_bounds__(kHThreads, 1)
                 tc_fence_after_sync();
                 return got;
             };
+            for (int b = 0; wide && b < ahead && ok; ++b) {
+                ok = mbar_wait(smem_u32(&bar_full[s]), phase, abort_flag);
+                commit(smem_u32(&bar_empty[s]));
+                if (++s == C::kStages)
+                    s = 0, phase ^= 1u;
+            }
             for (int tile = first; tile < p.total_tiles && ok; tile += stride, ++i) {
                 int tm, tn, tz, band, first_group, nkb;
                 half_tile(p, tile, tm, tn, tz, band);
