@@ -300,8 +300,9 @@ ct_status launch_skinny_smem(
 // of the block - feed R float64 FMAs each.  What bounds it: per step a warp takes 2 n shared-memory cycles and
 // n R / 2 cycles of the SM's float64 pipe, so R = 8 leaves the pipe (and the read of x) as the bound; with rows
 // on lanes and a broadcast weight per FMA, as before, shared memory took four times what the pipe did.
-// 60000 x 785 x 10: 139 -> 80 us (the pipe alone 26, the read of x 29); the rest is issue, two other instructions
-// per FMA, of them the conversions to float64 at 16 per clock and SM.
+// 60000 x 785 x 10: 139 -> 74 us (the pipe alone 33, the read of x 29); the rest is issue, nearly two other instructions
+// per FMA, of them the conversions to float64 at 16 per clock and SM.  (From eight columns on many rows take gemm_tall_kernel.)
+// The weights come in whole lines, the first of them before the activations: 1024 x 10 at 4096 rows 13.0 -> 11.4 us.
 //
 // The float64 sums of the lanes are added by exchanging rows first (each step halves the rows a lane keeps),
 // then across what is left; every lane of a group of 32 / R then holds its row's n sums, adds the bias, rounds
@@ -448,22 +449,47 @@ __global__ void __launch_bounds__(32 * kFewWarps, 1) gemm_few_columns_kernel(
         copy_async_commit();
         f_slot = f_slot + 1 == D ? 0 : f_slot + 1;
     };
+    // the weights, widened once per block: whole lines of w, the first of them asked for before the activations
+    const int elements = k * n, e_rows = (32 * kFewWarps) / n, e_cols = (32 * kFewWarps) % n;
+    int e_row = (int)threadIdx.x / n, e_col = (int)threadIdx.x % n;
+    constexpr int kBatch = 16;
+    float e_v[kBatch];
+    auto ask = [&](int e) {
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+            e_v[u] = e + u * 32 * kFewWarps < elements ? __ldg(w + e + u * 32 * kFewWarps) : 0.0f;
+    };
+    ask((int)threadIdx.x);
 #pragma unroll 1
     for (int d = 0; d < D - 1; ++d)
         fetch();
-    // the weights, widened once per block: a thread takes rows of w
-#pragma unroll 4
-    for (int kk = threadIdx.x; kk < steps * 32; kk += 32 * kFewWarps) {
-        float v[NE];
+    for (int e = (int)threadIdx.x; e < elements;) {
 #pragma unroll
-        for (int j = 0; j < NE; ++j)
-            v[j] = (kk < k && j < n) ? __ldg(w + (int64_t)kk * n + j) : 0.0f;
-#pragma unroll
-        for (int j = 0; j < NE; j += 2)
-            *reinterpret_cast<double2 *>(w_few + kk * S + j) = make_double2((double)v[j], (double)v[j + 1]);
+        for (int u = 0; u < kBatch; ++u) {
+            if (e + u * 32 * kFewWarps < elements)
+                w_few[e_row * S + e_col] = (double)e_v[u];
+            e_row += e_rows, e_col += e_cols;
+            if (e_col >= n)
+                e_col -= n, ++e_row;
+        }
+        e += kBatch * 32 * kFewWarps;
+        if (e < elements)
+            ask(e);
     }
+    if (n < NE)
+        for (int kk = threadIdx.x; kk < k; kk += 32 * kFewWarps)
+            for (int j = n; j < NE; ++j)
+                w_few[kk * S + j] = 0.0;
+    for (int e = k * S + (int)threadIdx.x; e < steps * 32 * S; e += 32 * kFewWarps)
+        w_few[e] = 0.0;
     __syncthreads();
+    // A step's activations are read and widened while the one before is multiplied.
     int slot = 0;
+    double xv[R];
+    copy_async_wait<D - 2>();
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        xv[r] = (double)ring[r * 32];
     for (int64_t t = first; t < tiles; t += stride) {
         const int64_t row0 = t * R;
         double acc[R][NE];
@@ -474,12 +500,13 @@ __global__ void __launch_bounds__(32 * kFewWarps, 1) gemm_few_columns_kernel(
                 acc[r][j] = 0.0;
 #pragma unroll 1
         for (int step = 0; step < steps; ++step) {
-            copy_async_wait<D - 2>();
-            double xv[R];
+            copy_async_wait<D - 3>();
+            slot = slot + 1 == D ? 0 : slot + 1;
+            float next[R];
 #pragma unroll
             for (int r = 0; r < R; ++r)
-                xv[r] = (double)ring[(slot * R + r) * 32];
-            slot = slot + 1 == D ? 0 : slot + 1;
+                next[r] = ring[(slot * R + r) * 32];
+            fetch(); // into the slot before the last, whose values have been used
             const double2 *wp = reinterpret_cast<const double2 *>(w_few + (step * 32 + lane) * S);
 #pragma unroll
             for (int j = 0; j < NE / 2; ++j) {
@@ -491,13 +518,216 @@ __global__ void __launch_bounds__(32 * kFewWarps, 1) gemm_few_columns_kernel(
                     acc[r][2 * j + 1] = __fma_rn(xv[r], wv.y, acc[r][2 * j + 1]);
                 }
             }
-            fetch(); // into the slot before this one, whose values have been used
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                xv[r] = (double)next[r];
         }
         double sum[NE];
         few_reduce<R, NE>(acc, lane, sum);
         constexpr int group = 32 / R;
         const int64_t row   = row0 + lane / group;
         few_finish<NE, group>(sum, bias, row, row < m, n, act, lane % group, out, argmax);
+    }
+}
+
+// Eight columns and more, weights that leave room for the ring: the first eight columns (all, above twelve) by the float64 MMA, 8 rows
+// x 8 columns x 4 values of k to an instruction, the others by multiply-adds.  The MMA is exact products and rounded
+// additions like those, at the full rate of the float64 pipe (65 of 64 nominal per clock and SM against 52 of multiply-adds with
+// operands from all over the register file), takes one issue slot for eight, and its sums lie in two registers a
+// lane, so sixteen warps fit an SM and hardly anything is left to add up across lanes.
+//
+// A warp walks tiles of 8 T rows, 32 values of k a step, fed by its ring like the kernel above.  Lane 4 r + q has row r and the
+// values 8 q .. 8 q + 7 of a step (which four values of k meet in an MMA is free), two 16-byte reads; rows are 36 floats
+// apart, so eight lanes' reads cover all banks.  The weights lie as the lanes read them, 16 bytes each.
+//
+// 60000 x 785 x 10: 74.4 -> 55.7 us, x 8 62.5 -> 45.9, x 16 121 -> 80; 8192 x 785 x 10 16.2 -> 12.2.  The float64 pipe takes 31 of the 55.7, the
+// read of x 29; what bounds it is the 4-byte asynchronous copies (some 6 clocks for 128 bytes) next to the reads of the weights.
+constexpr int kTallWarps = 16, kTallRow = 36, kTallRing = 48; // floats of a ring row; rows in a warp's ring
+template <int NE> struct TallCfg {
+    static constexpr int kTiles = NE > 12 ? 2 : 1, kExtra = NE > 12 ? 0 : NE - 8;
+    static constexpr int kUnits = kTiles * 128 + kExtra * 16; // of 16 bytes, 32 values of k
+    static constexpr size_t smem(int64_t k) { return (size_t)((k + 31) / 32) * kUnits * 16 + (size_t)kTallWarps * kTallRing * kTallRow * 4; }
+};
+
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
+
+template <int NE, int T>
+__global__ void __launch_bounds__(32 * kTallWarps, 1) gemm_tall_kernel(
+    const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ bias, int64_t m, int k, int n,
+    int act, float *__restrict__ out, int64_t *__restrict__ argmax) {
+    using C = TallCfg<NE>;
+    constexpr int R = 8 * T, D = kTallRing / R, NT = C::kTiles, NX = C::kExtra;
+    constexpr int CH = T == 1 ? 2 : 1; // chains of sums per tile of the result
+    constexpr bool kAhead = T == 1;     // few warps have tiles: a step's activations are read while the one before is multiplied
+    extern __shared__ __align__(16) double2 w_tall[]; // [steps][units], then the warps' rings [D][R][kTallRow] floats
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int steps = (k + 31) >> 5;
+    griddep_launch_dependents();
+    griddep_wait(); // activations (and possibly weights) come from the previous kernel
+    const int64_t tiles = (m + R - 1) / R, first = (int64_t)blockIdx.x + (int64_t)warp * gridDim.x;
+    const int64_t stride = (int64_t)gridDim.x * kTallWarps;
+    float *ring = reinterpret_cast<float *>(w_tall + (size_t)steps * C::kUnits) + warp * kTallRing * kTallRow;
+    const uint32_t ring_a = (uint32_t)__cvta_generic_to_shared(ring + lane);
+    int64_t f_tile = first;
+    int f_step = 0, f_slot = 0;
+    bool f_whole = f_tile * R + R <= m;
+    const float *f_src = x + first * R * k + lane; // this lane's element of the first row
+    auto fetch = [&]() {
+        if (f_tile < tiles) {
+            const uint32_t dst = ring_a + (uint32_t)(f_slot * R * kTallRow) * 4u;
+            const int kk       = f_step * 32 + lane;
+            if (f_whole && f_step * 32 + 32 <= k) {
+                const float *src = f_src;
+#pragma unroll
+                for (int r = 0; r < R; ++r, src += k)
+                    copy_async_4(dst + (uint32_t)(r * kTallRow) * 4u, src);
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const bool ok = kk < k && f_tile * R + r < m;
+                    copy_async_4(dst + (uint32_t)(r * kTallRow) * 4u, ok ? f_src + (int64_t)r * k : x, ok);
+                }
+            }
+            f_src += 32;
+            if (++f_step == steps) {
+                f_step = 0, f_tile += stride;
+                f_whole = f_tile * R + R <= m;
+                f_src   = x + f_tile * R * k + lane;
+            }
+        }
+        copy_async_commit();
+        f_slot = f_slot + 1 == D ? 0 : f_slot + 1;
+    };
+    // the weights, widened once per block and laid out by 16-byte units; the first of them are asked for before the activations
+    constexpr int kBatch = 10;
+    const int units = steps * C::kUnits;
+    float v0[kBatch], v1[kBatch];
+    auto weight = [&](int kk, int j) { return kk < k && j < n ? __ldg(w + (int64_t)kk * n + j) : 0.0f; };
+    auto ask    = [&](int first_unit) {
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+            const int at = first_unit + i * 32 * kTallWarps, block = at / C::kUnits, u = at - block * C::kUnits;
+            if (at < units && u < NT * 128) { // [tile][pair of values of k][lane]
+                const int kk = block * 32 + (u & 3) * 8 + ((u >> 5) & 3) * 2, j = (u >> 7) * 8 + ((u & 31) >> 2);
+                v0[i] = weight(kk, j), v1[i] = weight(kk + 1, j);
+            } else if (at < units) { // [value of k][pair of columns][q]
+                const int e = u - NT * 128, pairs = NX / 2 > 0 ? NX / 2 : 1;
+                const int kk = block * 32 + (e & 3) * 8 + (e >> 2) / pairs, j = 8 + (e >> 2) % pairs * 2;
+                v0[i] = weight(kk, j), v1[i] = weight(kk, j + 1);
+            }
+        }
+    };
+    ask((int)threadIdx.x);
+#pragma unroll 1
+    for (int d = 0; d < D - 1; ++d)
+        fetch();
+    for (int at = (int)threadIdx.x; at < units;) {
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i)
+            if (at + i * 32 * kTallWarps < units)
+                w_tall[at + i * 32 * kTallWarps] = make_double2((double)v0[i], (double)v1[i]);
+        at += kBatch * 32 * kTallWarps;
+        if (at < units)
+            ask(at);
+    }
+    __syncthreads();
+    const float *mine = ring + (lane >> 2) * kTallRow + (lane & 3) * 8;
+    int slot = 0;
+    float4 xf[T][2];
+    auto read = [&](float4 (&to)[T][2]) {
+#pragma unroll
+        for (int a = 0; a < T; ++a)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                to[a][h] = *reinterpret_cast<const float4 *>(mine + (slot * R + a * 8) * kTallRow + h * 4);
+        slot = slot + 1 == D ? 0 : slot + 1;
+    };
+    if (kAhead) {
+        copy_async_wait<D - 2>();
+        __syncwarp();
+        read(xf);
+    }
+    for (int64_t t = first; t < tiles; t += stride) {
+        double acc[T][NT][CH][2], extra[T][CH][NX > 0 ? NX : 1];
+#pragma unroll
+        for (int a = 0; a < T; ++a) {
+#pragma unroll
+            for (int b = 0; b < NT * CH; ++b)
+                acc[a][b / CH][b % CH][0] = acc[a][b / CH][b % CH][1] = 0.0;
+#pragma unroll
+            for (int j = 0; j < NX * CH; ++j)
+                extra[a][NX > 0 ? j / NX : 0][NX > 0 ? j % NX : 0] = 0.0;
+        }
+        const double2 *wp = w_tall;
+#pragma unroll 1
+        for (int step = 0; step < steps; ++step, wp += C::kUnits) {
+            // every lane's copies are there, and every lane has read the slot that is fetched next
+            copy_async_wait<kAhead ? D - 3 : D - 2>();
+            __syncwarp();
+            float4 next[T][2];
+            if (kAhead)
+                read(next);
+            else
+                fetch(), read(xf);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                double2 wv[NT];
+#pragma unroll
+                for (int b = 0; b < NT; ++b)
+                    wv[b] = wp[(b * 4 + p) * 32 + lane];
+#pragma unroll
+                for (int o = 0; o < 2; ++o) {
+                    double2 we[NX / 2 > 0 ? NX / 2 : 1];
+#pragma unroll
+                    for (int j = 0; j < NX / 2; ++j)
+                        we[j] = wp[NT * 128 + ((2 * p + o) * (NX / 2) + j) * 4 + (lane & 3)];
+#pragma unroll
+                    for (int a = 0; a < T; ++a) {
+                        const float4 q  = xf[a][p >> 1];
+                        const double xv = (double)((p & 1) ? (o ? q.w : q.z) : (o ? q.y : q.x));
+#pragma unroll
+                        for (int b = 0; b < NT; ++b)
+                            mma_f64(acc[a][b][o % CH], xv, o ? wv[b].y : wv[b].x);
+                        // float32 x float32 is exact in float64, so the fused form rounds like mul, add
+#pragma unroll
+                        for (int j = 0; j < NX / 2; ++j) {
+                            extra[a][o % CH][2 * j]     = __fma_rn(xv, we[j].x, extra[a][o % CH][2 * j]);
+                            extra[a][o % CH][2 * j + 1] = __fma_rn(xv, we[j].y, extra[a][o % CH][2 * j + 1]);
+                        }
+                    }
+                }
+            }
+            if (kAhead) {
+                fetch();
+#pragma unroll
+                for (int h = 0; h < 2 * T; ++h)
+                    xf[h / 2][h % 2] = next[h / 2][h % 2];
+            }
+        }
+        // a lane has two columns of each tile: all of its row's sums to each of the row's four lanes
+#pragma unroll
+        for (int a = 0; a < T; ++a) {
+            double sum[NE];
+#pragma unroll
+            for (int j = 0; j < NE; ++j) {
+                if (j < NT * 8) {
+                    double c = acc[a][j / 8][0][j % 2];
+                    if (CH == 2)
+                        c += acc[a][j / 8][CH - 1][j % 2];
+                    sum[j] = __shfl_sync(0xffffffffu, c, (lane & 28) | (j % 8) / 2);
+                } else {
+                    double c = extra[a][0][NX > 0 ? (j - 8) % NX : 0];
+                    if (CH == 2)
+                        c += extra[a][CH - 1][NX > 0 ? (j - 8) % NX : 0];
+                    c += __shfl_xor_sync(0xffffffffu, c, 1);
+                    sum[j] = c + __shfl_xor_sync(0xffffffffu, c, 2);
+                }
+            }
+            const int64_t row = t * R + a * 8 + (lane >> 2);
+            few_finish<NE, 4>(sum, bias, row, row < m, n, act, lane & 3, out, argmax);
+        }
     }
 }
 
@@ -587,6 +817,30 @@ ct_status launch_few(
     const int wave       = m <= 2 * st->sm_count ? few_rows_per_wave<NE, 2>(st) : few_rows_per_wave<NE, 4>(st);
     const double by_rows = 1.5 + (double)((blocks + wave - 1) / wave) * ((NE > 12 ? 2.0 : 0.8) + 6e-4 * NE * (double)std::min<int64_t>(k, 800));
     const double resident = 3.5 + 7e-4 * NE * (double)k + (double)m * (double)k * (6e-7 + 7e-8 * NE);
+    if constexpr (NE >= 8) {
+        // From where the kernel below walks a second time (32 rows to an SM; from half of that where no column is left to the
+        // multiply-adds).  785 x 8 / 10 / 12 / 16 in us, there and here: 7.4 / 7.7 / 8.9 / 10.3 and 8.0 / 9.3 / 10.0 / 11.1 at 2000 rows, 8.9 / 9.5 /
+        // 11.0 / 13.1 and 8.0 / 9.4 / 10.4 / 11.0 at 3000, 13.6 / 14.4 / 16.7 / 19.6 and 9.4 / 12.0 / 13.6 / 13.6 at 6000; 1024 x 10 at 4096
+        // 11.4 and 12.2.
+        const bool many = m > 32 * (int64_t)st->sm_count || (TallCfg<NE>::kExtra == 0 && m > 16 * (int64_t)st->sm_count);
+        if (many && TallCfg<NE>::smem(k) <= kMost && resident < by_rows) {
+            static bool tall_attr_set_dev[16] = {};
+            if (!tall_attr_set_dev[st->device & 15]) {
+                CT_CUDA(cudaFuncSetAttribute(gemm_tall_kernel<NE, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
+                CT_CUDA(cudaFuncSetAttribute(gemm_tall_kernel<NE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
+                tall_attr_set_dev[st->device & 15] = true;
+            }
+            // sixteen rows to a warp where tiles of eight would be walked twice: 785 x 10 19.0 and 18.8 at 16000 rows, 26.3 and 24.2 at
+            // 20000; 785 x 8 13.3 and 14.1, 19.5 and 16.7
+            const bool deep     = m > (int64_t)st->sm_count * kTallWarps * 8;
+            const int64_t tiles = deep ? (m + 15) / 16 : (m + 7) / 8;
+            const unsigned grid = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
+            CT_CUDA(launch_dependent(deep ? gemm_tall_kernel<NE, 2> : gemm_tall_kernel<NE, 1>, dim3(grid), dim3(32 * kTallWarps), TallCfg<NE>::smem(k), stream(),
+                a, b, bias, m, (int)k, n, act, out, argmax));
+            CT_LAUNCH_CHECK("gemm_tall");
+            return CT_OK;
+        }
+    }
     if (smem <= kMost && resident < by_rows) {
         // eight rows per warp where there are rows enough for two such tiles each and the sums stay in registers
         const bool deep = NE <= 12 && !longer && m >= (int64_t)st->sm_count * kFewWarps * 8 * 2;

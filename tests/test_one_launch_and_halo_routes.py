@@ -105,6 +105,35 @@ def test_small_products_in_one_launch(T, m, k, n, kind):
     assert np.all(np.abs(got[finite] - want[finite]) <= BOUND * size[finite])
 
 
+# Many rows and eight to sixteen columns (the float64 MMA): columns beside the first eight, columns that there are not, tiles of eight
+# and of sixteen rows that end ragged, k of less than a step, of one value more and of several steps.
+# Bound: products are exact and summed in float64 (k additions of 2^-53 of the sum of magnitudes), rounded to float32 once.
+@pytest.mark.parametrize("m,k,n", [(2401, 785, 13), (2403, 31, 8), (4741, 33, 10), (4740, 128, 12), (4739, 1, 9), (18951, 97, 16), (18949, 65, 7),
+                                   (18945, 40, 8), (38001, 70, 11), (5001, 896, 15)])
+@pytest.mark.parametrize("act", ["none", "softmax"])
+def test_many_rows_of_few_columns(T, port, m, k, n, act):
+    rng = np.random.default_rng(m + k + n)
+    x, w, b = (rng.standard_normal(shape).astype(np.float32) for shape in ((m, k), (k, n), (n,)))
+    if act == "none":
+        x[m - 1, k - 1], x[m // 2, 0] = np.nan, np.inf
+    got = T.dense(T.from_numpy(x), T.from_numpy(w), T.from_numpy(b), act).numpy()
+    T.check_async()
+    with np.errstate(invalid="ignore"):
+        want = x.astype(np.float64) @ w.astype(np.float64) + b
+    if act == "softmax":
+        # a logit is off by half a unit in the last place, 2^-24 of it; its exponential, the sum and the quotient by 2^-21 in all, and below
+        # the smallest normal value nothing is promised
+        e = np.exp(want - want.max(axis=1, keepdims=True))
+        want = e / e.sum(axis=1, keepdims=True)
+        logit = np.abs(x.astype(np.float64) @ w + b).max()
+        assert np.all(np.abs(got - want) <= want * (2.0**-21 + 2.0**-22 * logit) + 2.0**-126)
+        return
+    finite = np.isfinite(want)
+    assert np.array_equal(np.isfinite(got), finite) and np.array_equal(np.isnan(got), np.isnan(want))
+    size = np.abs(np.where(np.isfinite(x), x, 0)).astype(np.float64) @ np.abs(w).astype(np.float64) + np.abs(b)
+    assert np.all(np.abs(got[finite] - want[finite]) <= 2.0**-24 * np.abs(want[finite]) + (k + 1) * 2.0**-53 * size[finite])
+
+
 # one tile of columns: chunks of 128 values of k that end ragged, slices of unequal length, rows that are 16-byte aligned and rows that are
 # not, and operands that are left to the product from planes; the first has too few tiles for it
 @pytest.mark.parametrize("m,k,n", [(3300, 2100, 100), (4200, 4099, 128), (6500, 2050, 33), (6500, 2100, 100), (4200, 4100, 128)])
