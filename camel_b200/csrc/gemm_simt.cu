@@ -903,9 +903,9 @@ ct_status matmul_generic(
 // equal at n = 10.
 //
 // R and the warps of a block are chosen so that the block's warps cover the output rows evenly: with blocks of
-// 4 x 128 rows, 785 features made every other block a quarter full.  785 x 60000 x 10: 94 -> 90 us, 785 x 256 x 10:
-// 18 us.
-constexpr int kTnMinThreads = 64, kTnMaxThreads = 160; // two blocks to an SM at 200 registers
+// 4 x 128 rows, 785 features made every other block a quarter full.  785 x 60000 x 10: 94 -> 90 us (eight columns and more have the
+// kernel behind this one now).
+constexpr int kTnMinThreads = 64, kTnMaxThreads = 160; // two blocks to an SM at 168 registers
 constexpr int kTnChunk   = 32; // rows of b staged per step
 constexpr int kTnGroup   = 2;  // k steps fetched together
 constexpr int kTnGroups  = 6;  // groups in a warp's ring, all but one in flight
@@ -1044,6 +1044,165 @@ __global__ void __launch_bounds__(kTnMaxThreads, 2) gemm_tn_skinny_kernel(
     }
 }
 
+// Eight to sixteen columns: the first eight (all, above ten) by the float64 MMA, 8 rows of the result x 8 columns x 4 values of k
+// to an instruction, as in gemm_tall_kernel, with the grid, slices and staging of b of the kernel above.  A ring holds four
+// values of k at a time; lane 4 f + q has the q-th of them and the 4 R rows of the result from 4 R f on, which its 16-byte reads take
+// in turn as row f of 4 R tiles, and one weight of b serves them all.
+//
+// Bound by the 4-byte asynchronous copies (some 6 clocks for 128 bytes) and the float64 pipe, 30 to 40 us each at 785 x 60000 x 10 where
+// the read of X takes 29, which overlap as far as there are warps: 88.4 us by multiply-adds, with R = 5 / 4 / 3 / 2 spills / 97 / 75.4 /
+// 71.9; x 8 76.3 -> 59.7, x 16 145 -> 95; 300 x 5000 x 10 14.9 -> 11.6.
+template <int NMAX, int R>
+__global__ void __launch_bounds__(kTnMaxThreads, 3) gemm_tn_tall_kernel(
+    const float *__restrict__ a_km, const float *__restrict__ b, int64_t m, int64_t k, int n, int64_t k_per_slice,
+    double *__restrict__ partial) {
+    griddep_wait();
+    griddep_launch_dependents();
+    constexpr int G = 4, GROUPS = 3, NT = NMAX > 10 ? 2 : 1, NX = NMAX == 10 ? 2 : 0;
+    constexpr int NB = NT * 8 + NX;                       // columns of b staged
+    constexpr int ROW = 32 * R + 4;                       // floats of a ring row
+    constexpr int BL  = (kTnChunk * NB + kTnMinThreads - 1) / kTnMinThreads; // staged b values per thread
+    __shared__ __align__(16) double bs[2][kTnChunk][NB];
+    __shared__ __align__(16) float ring_s[kTnMaxThreads / 32][GROUPS][G][ROW];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, threads = (int)blockDim.x;
+    const int64_t warp_row = ((int64_t)blockIdx.x * (threads / 32) + warp) * (32 * R);
+    const int64_t row0     = warp_row + lane;
+    const int64_t k0       = (int64_t)blockIdx.y * k_per_slice;
+    const int64_t k1       = k0 + k_per_slice < k ? k0 + k_per_slice : k;
+
+    float bnext[BL];
+    auto fetch_b = [&](int64_t kc) {
+#pragma unroll
+        for (int u = 0; u < BL; ++u) {
+            const int idx = threadIdx.x + u * threads;
+            if (u * threads >= kTnChunk * NB)
+                break;
+            const int kk = idx / NB, j = idx - kk * NB;
+            bnext[u] = (idx < kTnChunk * NB && kc + kk < k1 && j < n) ? __ldg(b + (kc + kk) * n + j) : 0.0f;
+        }
+    };
+    auto store_b = [&](int buf) {
+#pragma unroll
+        for (int u = 0; u < BL; ++u) {
+            const int idx = threadIdx.x + u * threads;
+            if (u * threads >= kTnChunk * NB)
+                break;
+            if (idx < kTnChunk * NB)
+                (&bs[buf][0][0])[idx] = (double)bnext[u];
+        }
+    };
+
+    double acc[4 * R][NT][2], extra[4 * R][NX > 0 ? NX : 1];
+#pragma unroll
+    for (int t = 0; t < 4 * R; ++t) {
+#pragma unroll
+        for (int u = 0; u < NT; ++u)
+            acc[t][u][0] = acc[t][u][1] = 0.0;
+#pragma unroll
+        for (int j = 0; j < NX; ++j)
+            extra[t][j] = 0.0;
+    }
+    float(*ring)[G][ROW] = ring_s[warp];
+    const float *pa      = a_km + k0 * m + row0; // row `next` of the operand, this lane's first column
+    int64_t next         = k0;
+    int put = 0, get = 0;
+    const uint32_t ring_a = (uint32_t)__cvta_generic_to_shared(&ring[0][0][lane]);
+    const bool full       = warp_row + 32 * R <= m;
+    auto fetch_a = [&]() {
+        const uint32_t dst = ring_a + (uint32_t)put * (G * ROW * 4u);
+        const bool whole   = full && next + G <= k1;
+        const float *src   = pa;
+#pragma unroll
+        for (int u = 0; u < G; ++u, src += m)
+            if (whole) {
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    copy_async_4(dst + (uint32_t)(u * ROW + 32 * r) * 4u, src + 32 * r);
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const bool ok = next + u < k1 && row0 + 32 * r < m;
+                    copy_async_4(dst + (uint32_t)(u * ROW + 32 * r) * 4u, ok ? src + 32 * r : a_km, ok);
+                }
+            }
+        copy_async_commit();
+        pa += G * m;
+        next += G;
+        put = put + 1 == GROUPS ? 0 : put + 1;
+    };
+    auto compute = [&](int buf, int g) {
+        copy_async_wait<GROUPS - 2>();
+        __syncwarp(); // every lane's copies are there, and every lane has read the group before
+        double bv[NT];
+#pragma unroll
+        for (int u = 0; u < NT; ++u)
+            bv[u] = bs[buf][g + (lane & 3)][u * 8 + (lane >> 2)];
+        double2 be = make_double2(0.0, 0.0);
+        if (NX > 0)
+            be = *reinterpret_cast<const double2 *>(&bs[buf][g + (lane & 3)][NB - 2]);
+        const float *mine = &ring[get][lane & 3][(lane >> 2) * (4 * R)];
+#pragma unroll
+        for (int h = 0; h < R; ++h) {
+            const float4 q   = *reinterpret_cast<const float4 *>(mine + 4 * h);
+            const float v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const double av = (double)v[e];
+#pragma unroll
+                for (int u = 0; u < NT; ++u)
+                    mma_f64(acc[4 * h + e][u], av, bv[u]);
+                if (NX > 0) { // float32 x float32 is exact in float64
+                    extra[4 * h + e][0]               = __fma_rn(av, be.x, extra[4 * h + e][0]);
+                    extra[4 * h + e][NX > 0 ? NX - 1 : 0] = __fma_rn(av, be.y, extra[4 * h + e][NX > 0 ? NX - 1 : 0]);
+                }
+            }
+        }
+        get = get + 1 == GROUPS ? 0 : get + 1;
+    };
+    fetch_b(k0);
+    const bool has_rows = warp_row < m; // a block's last warps may have none
+#pragma unroll 1
+    for (int d = 0; has_rows && d < GROUPS - 1; ++d)
+        fetch_a();
+    store_b(0);
+    __syncthreads();
+    int buf = 0;
+    for (int64_t kc = k0; kc < k1; kc += kTnChunk, buf ^= 1) {
+        const bool more = kc + kTnChunk < k1;
+        if (more)
+            fetch_b(kc + kTnChunk);
+#pragma unroll 1
+        for (int g = 0; has_rows && g < kTnChunk; g += G) {
+            compute(buf, g);
+            fetch_a(); // may already belong to the next chunk; zeros past the slice
+        }
+        if (more)
+            store_b(buf ^ 1); // nobody reads that buffer any more: all warps passed the last barrier
+        __syncthreads();
+    }
+#pragma unroll
+    for (int t = 0; t < 4 * R; ++t) {
+        const int64_t row = warp_row + (lane >> 2) * (4 * R) + t;
+        double *dst       = partial + ((int64_t)blockIdx.y * m + row) * n;
+#pragma unroll
+        for (int u = 0; u < NT; ++u)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int j = u * 8 + (lane & 3) * 2 + i;
+                if (row < m && j < n)
+                    dst[j] = acc[t][u][i];
+            }
+#pragma unroll
+        for (int x = 0; x < NX; ++x) {
+            double c = extra[t][x];
+            c += __shfl_xor_sync(0xffffffffu, c, 1);
+            c += __shfl_xor_sync(0xffffffffu, c, 2);
+            if (row < m && (lane & 3) == x && NT * 8 + x < n)
+                dst[NT * 8 + x] = c;
+        }
+    }
+}
+
 // One warp per output element: lane l adds the slices l, l + 32, ... in that order, then the lanes'
 // sums are added in a fixed butterfly - the same order on every run.
 __global__ void __launch_bounds__(256) gemm_tn_skinny_finish_kernel(
@@ -1067,6 +1226,13 @@ __global__ void __launch_bounds__(256) gemm_tn_skinny_finish_kernel(
 template <int NMAX, int R>
 static ct_status launch_tn_skinny(
     DeviceState *st, const float *a_km, const float *b, int64_t m, int64_t k, int n, float *out) {
+    auto choose = [] {
+        if constexpr (NMAX >= 8 && NMAX <= 16)
+            return gemm_tn_tall_kernel<NMAX, R>;
+        else
+            return gemm_tn_skinny_kernel<NMAX, R>;
+    };
+    const auto kernel = choose();
     const int64_t warps   = (m + 32 * R - 1) / (32 * R);
     const int64_t mblocks = (warps + kTnMaxThreads / 32 - 1) / (kTnMaxThreads / 32);
     const int threads     = (int)std::max<int64_t>(kTnMinThreads, (warps + mblocks - 1) / mblocks * 32);
@@ -1074,7 +1240,7 @@ static ct_status launch_tn_skinny(
     static std::atomic<int> per_sm[kTnMaxThreads / 32 + 1];
     int fit = per_sm[threads / 32].load(std::memory_order_relaxed);
     if (fit == 0) {
-        CT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, gemm_tn_skinny_kernel<NMAX, R>, threads, 0));
+        CT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, threads, 0));
         fit = fit < 1 ? 1 : fit;
         per_sm[threads / 32].store(fit, std::memory_order_relaxed);
     }
@@ -1099,9 +1265,9 @@ static ct_status launch_tn_skinny(
     // 23.8 -> 21.5), but for many small blocks with several chunks each: those crowd on the SMs that are free first (one update
     // of 96854 x 191 x 16 178, started on an idle machine 169; 33930 x 76 x 4 38 and 33).
     if (threads > kTnMinThreads || k_per_slice == kTnChunk)
-        (void)launch_dependent(gemm_tn_skinny_kernel<NMAX, R>, grid, dim3(threads), 0, stream(), a_km, b, m, k, n, k_per_slice, partial);
+        (void)launch_dependent(kernel, grid, dim3(threads), 0, stream(), a_km, b, m, k, n, k_per_slice, partial);
     else
-        gemm_tn_skinny_kernel<NMAX, R><<<grid, threads, 0, stream()>>>(a_km, b, m, k, n, k_per_slice, partial);
+        kernel<<<grid, threads, 0, stream()>>>(a_km, b, m, k, n, k_per_slice, partial);
     CT_LAUNCH_CHECK("gemm_tn_skinny");
     const int64_t mn = m * n;
     (void)launch_dependent(gemm_tn_skinny_finish_kernel, dim3((unsigned)((mn * 32 + 255) / 256)), dim3(256), 0, stream(), partial, mn, (int)slices, out);
@@ -1128,11 +1294,11 @@ ct_status gemm_f32_tn_skinny(
     case 1: CT_TN(2);
     case 2: CT_TN(4);
     case 3: CT_TN(6);
-    case 4: CT_TN(8);
-    case 5: CT_TN(10);
-    case 6: return launch_tn_skinny<12, 3>(st, a_km, b, m, k, (int)n, out);
-    case 7: return launch_tn_skinny<14, 3>(st, a_km, b, m, k, (int)n, out);
-    case 8: return launch_tn_skinny<16, 3>(st, a_km, b, m, k, (int)n, out);
+    case 4: return launch_tn_skinny<8, 2>(st, a_km, b, m, k, (int)n, out);
+    case 5: return launch_tn_skinny<10, 2>(st, a_km, b, m, k, (int)n, out);
+    case 6: return launch_tn_skinny<12, 2>(st, a_km, b, m, k, (int)n, out);
+    case 7: return launch_tn_skinny<14, 2>(st, a_km, b, m, k, (int)n, out);
+    case 8: return launch_tn_skinny<16, 2>(st, a_km, b, m, k, (int)n, out);
     default: break;
     }
 #undef CT_TN

@@ -134,6 +134,23 @@ def test_many_rows_of_few_columns(T, port, m, k, n, act):
     assert np.all(np.abs(got[finite] - want[finite]) <= 2.0**-24 * np.abs(want[finite]) + (k + 1) * 2.0**-53 * size[finite])
 
 
+# The transposed left operand with eight to sixteen columns: rows that end in each part of a warp's 64 and leave a warp without any,
+# k of less than four values, of one more than a chunk and of several slices.  The bound is the one above.
+@pytest.mark.parametrize("m,k,n", [(1, 3, 8), (63, 33, 10), (65, 32, 9), (321, 500, 12), (785, 5003, 10), (257, 20001, 16), (130, 77, 7), (640, 129, 13)])
+def test_transposed_operand_and_few_columns(T, m, k, n):
+    rng = np.random.default_rng(m + k + n)
+    x, y = (rng.standard_normal(shape).astype(np.float32) for shape in ((k, m), (k, n)))
+    x[0, m - 1], x[k - 1, 0] = np.inf, np.nan
+    got = T.matmul_tn(T.from_numpy(x), T.from_numpy(y)).numpy()
+    T.check_async()
+    with np.errstate(invalid="ignore"):
+        want = x.T.astype(np.float64) @ y.astype(np.float64)
+    finite = np.isfinite(want)
+    assert np.array_equal(np.isfinite(got), finite) and np.array_equal(np.isnan(got), np.isnan(want))
+    size = np.abs(np.where(np.isfinite(x), x, 0)).T.astype(np.float64) @ np.abs(y).astype(np.float64)
+    assert np.all(np.abs(got[finite] - want[finite]) <= 2.0**-24 * np.abs(want[finite]) + (k + 1) * 2.0**-53 * size[finite])
+
+
 # one tile of columns: chunks of 128 values of k that end ragged, slices of unequal length, rows that are 16-byte aligned and rows that are
 # not, and operands that are left to the product from planes; the first has too few tiles for it
 @pytest.mark.parametrize("m,k,n", [(3300, 2100, 100), (4200, 4099, 128), (6500, 2050, 33), (6500, 2100, 100), (4200, 4100, 128)])
