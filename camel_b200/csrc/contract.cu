@@ -634,19 +634,22 @@ static int pooled_tile_rows(int64_t ho, int64_t wo) {
 
 // Float32 layers that conv_halo takes: those that fit its tiles, but for layers with few channels on both sides, whose filters
 // stay on chip (conv_tmem.cu), and a handful of channels, most of whose block of 32 would be padding.  A 1 x 1 filter
-// has one use for a halo: up to 64 filters or 32 channels the other kernels are as fast or faster (88 x 95 x 29 x 32 -> 22
-// 46 us against 50, 19 x 18 x 60 x 63 -> 115 145 against 149), and a strided one reads a quarter of the planes (11 x 161 x 52 x 54 -> 37 27 against 33).
-// Below some 16,000 outputs per filter a strided layer's three launches cost more than its patches (7 x 17 x 69 x 72 -> 74
-// 24 against 28, 14 x 14 x 38 x 38 -> 22 26 against 31; 60 x 15 x 41 x 41 -> 27 34 both ways, 64 x 34 x 40 x 42 -> 78 45 against 41),
-// and below some 8,000 those of a layer of less than half a block of channels (4 x 8 x 38 x 40 -> 64, 5 x 5, 22 against 26, 4 x 8 x 40 x 40
-// -> 96 19 against 21; 9 x 10 x 39 x 42 -> 21, 5 x 5, 30 against 28, 16 x 8 x 40 x 40 -> 96 32 against 23).
+// has one use for a halo, so a block of channels or less is left to the others (8 x 32 x 30 x 30 -> 300 14.8 us against 17.6, at 64 x 56 x 56
+// 121 against 102); from 33 channels on it is as fast or faster (64 x 95 x 56 x 56 -> 64 116 -> 73, at stride 2 64 x 64 x 57 x 57 -> 128
+// 72 -> 43, 64 x 256 -> 64 189 -> 118).
+// Patches do not pad a tap's channels to whole k-steps: where c is not a multiple of 16 their chains of truncating additions are shorter
+// (8 channels 1.6e-7 against 2.1e-7 from 64 bits, 17 with 5 x 5 filters 5.6e-7 against 8.7e-7), so below some 16,000 outputs per filter strided
+// layers, below 8,000 layers of less than half a block of channels are theirs, though the halo is up to 1.4 times as fast.  Otherwise
+// the halo has the smaller errors (128 channels 11.8e-7 -> 9.2e-7) and is the faster one at stride 2 (16 x 128 x 57 x 57 -> 64 96 -> 37 us,
+// 1 x 64 x 16 x 16 -> 64 22.6 -> 18.8), for one k-step a tap from about 1,000 outputs on (4 x 16 x 28 x 28 -> 128 15.4 against 17.1, 2 x 57 x 57
+// 18.7 -> 17.3); at stride 3 its nine sub-images cost what they save.
 static bool conv2d_takes_halo(
     int64_t n, int64_t c, int64_t h, int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t stride, int64_t pad) {
     if (c < 8 || n > 65535 || conv_tmem_applicable(c, h, wd, ko, kh, kw, stride, pad))
         return false;
-    if (kh * kw == 1 && (ko <= 64 || c <= 32 || stride > 1))
+    if (kh * kw == 1 && (c <= 32 || stride > 2))
         return false;
-    const int64_t least = stride > 1 ? 16384 : (c < 16 ? 8192 : 0);
+    const int64_t least = stride == 2 && c % 16 == 0 ? (c == 16 ? 1024 : 0) : (stride > 1 ? 16384 : (c < 16 ? 8192 : 0));
     if (n * ((h + 2 * pad - kh) / stride + 1) * ((wd + 2 * pad - kw) / stride + 1) < least)
         return false;
     return conv_halo_applicable((c + 31) / 32 * 32, h, wd, ko, kh, kw, stride, pad);

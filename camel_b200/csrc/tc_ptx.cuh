@@ -196,17 +196,6 @@ __device__ __forceinline__ void tma_load_4d(
         : "memory");
 }
 
-__device__ __forceinline__ void tma_load_5d(
-    uint32_t dst_smem, const void *map, uint32_t bar, int32_t c0, int32_t c1, int32_t c2, int32_t c3, int32_t c4) {
-    asm volatile(
-        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-        :
-        : "r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2),
-          "r"(c3), "r"(c4)
-        : "memory");
-}
-
 // ---- tensor memory ----------------------------------------------------------------------
 
 // Whole-warp instructions (.sync.aligned): call from all 32 lanes of one warp.
