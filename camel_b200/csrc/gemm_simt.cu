@@ -541,7 +541,8 @@ __global__ void __launch_bounds__(32 * kFewWarps, 1) gemm_few_columns_kernel(
 // apart, so eight lanes' reads cover all banks.  The weights lie as the lanes read them, 16 bytes each.
 //
 // 60000 x 785 x 10: 74.4 -> 55.7 us, x 8 62.5 -> 45.9, x 16 121 -> 80; 8192 x 785 x 10 16.2 -> 12.2.  The float64 pipe takes 31 of the 55.7, the
-// read of x 29; what bounds it is the 4-byte asynchronous copies (some 6 clocks for 128 bytes) next to the reads of the weights.
+// read of x 29.  Warps wait for that pipe first (2.7 of 9 stalled per issue), then for dependences; the reads of shared memory, half of
+// them for the columns beside the first eight, and the 4-byte copies keep its pipe at 0.57.
 constexpr int kTallWarps = 16, kTallRow = 36, kTallRing = 48; // floats of a ring row; rows in a warp's ring
 template <int NE> struct TallCfg {
     static constexpr int kTiles = NE > 12 ? 2 : 1, kExtra = NE > 12 ? 0 : NE - 8;
@@ -1049,9 +1050,10 @@ __global__ void __launch_bounds__(kTnMaxThreads, 2) gemm_tn_skinny_kernel(
 // values of k at a time; lane 4 f + q has the q-th of them and the 4 R rows of the result from 4 R f on, which its 16-byte reads take
 // in turn as row f of 4 R tiles, and one weight of b serves them all.
 //
-// Bound by the 4-byte asynchronous copies (some 6 clocks for 128 bytes) and the float64 pipe, 30 to 40 us each at 785 x 60000 x 10 where
-// the read of X takes 29, which overlap as far as there are warps: 88.4 us by multiply-adds, with R = 5 / 4 / 3 / 2 spills / 97 / 75.4 /
-// 71.9; x 8 76.3 -> 59.7, x 16 145 -> 95; 300 x 5000 x 10 14.9 -> 11.6.
+// At 785 x 60000 x 10 the float64 pipe takes 32 us, the read of X 29, the shared-memory pipe is at 0.57: they overlap as far as there are
+// warps (what they wait for: dependences 1.9, the chunks' barrier 1.5, copies 1.1, the float64 pipe 1.1 per issue), so few rows to a warp are
+// best: 88.4 us by multiply-adds, with R = 5 / 4 / 3 / 2 spills / 97 / 75.4 / 71.9; x 8 76.3 -> 59.7, x 16 145 -> 95; 300 x 5000 x 10
+// 14.9 -> 11.6.
 template <int NMAX, int R>
 __global__ void __launch_bounds__(kTnMaxThreads, 3) gemm_tn_tall_kernel(
     const float *__restrict__ a_km, const float *__restrict__ b, int64_t m, int64_t k, int n, int64_t k_per_slice,
