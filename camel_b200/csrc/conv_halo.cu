@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                     s = 0, f = f_0;
                 uint32_t accumulate = 1u;
                 if (word & kH_Begin) { // what the accumulators held before has been read
-                    ok = mbar_wait_warp(smem_u32(&bar_acc_empty[acc]), acc_phase >> acc & 1u, abort_flag);
+                    ok = mbar_wait_warp<kClusterRead>(smem_u32(&bar_acc_empty[acc]), acc_phase >> acc & 1u, abort_flag);
                     if (!ok)
                         break;
                     tc_fence_after_sync();
@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(kH_Threads, 1) conv_halo_stream_kernel(
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0)
-                    mbar_arrive_peer(leader_addr(smem_u32(&bar_acc_empty[acc])));
+                    mbar_arrive_peer_read(leader_addr(smem_u32(&bar_acc_empty[acc])));
                 acc ^= 1;
             }
             if (!ok)

@@ -753,7 +753,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t bar_full[kCP_MaxStages], bar_empty[kCP_MaxStages];
     __shared__ uint64_t bar_raw_full, bar_raw_empty;
-    __shared__ uint64_t bar_scale_empty[kCP_MaxStages]; // the tile's scale has been read by the epilogue
+    __shared__ uint64_t bar_scale_full[kCP_MaxStages], bar_scale_empty[kCP_MaxStages]; // the tile's scale is there, has been read by the epilogue
     __shared__ uint64_t bar_acc_full[2], bar_acc_empty[2]; // tiles alternate between two sets of 256 columns
     __shared__ uint64_t bar_done;
     __shared__ uint32_t tmem_base_slot;
@@ -785,6 +785,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
         for (int s = 0; s < p.stages; ++s) {
             mbar_init(smem_u32(&bar_full[s]), RAW ? 2 * kCP_CvtWarps : 1); // of both CTAs
             mbar_init(smem_u32(&bar_empty[s]), 1);
+            mbar_init(smem_u32(&bar_scale_full[s]), 1);
             mbar_init(smem_u32(&bar_scale_empty[s]), kCP_EpiWarps);
         }
         mbar_init(smem_u32(&bar_raw_full), 1);
@@ -926,8 +927,8 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                     continue;
                 const int set = i & 1;
                 // the accumulators have been read, the planes are complete
-                ok = mbar_wait_warp(smem_u32(&bar_acc_empty[set]), ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag) &&
-                     mbar_wait_warp(smem_u32(&bar_full[s]), full_phase, abort_flag);
+                ok = mbar_wait_warp<kClusterRead>(smem_u32(&bar_acc_empty[set]), ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag) &&
+                     mbar_wait_warp<RAW ? kClusterWritten : kCta>(smem_u32(&bar_full[s]), full_phase, abort_flag);
                 if (!ok)
                     break;
                 tc_fence_after_sync();
@@ -1033,8 +1034,10 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                     range = range_join(range, cvt_range[i & 1][u]);
                 float scale, inverse;
                 const bool fits = half_tile_fits(range, scale, inverse);
-                if (ct == 0)
+                if (ct == 0) {
                     tile_scale[s] = fits ? inverse : 0.0f;
+                    mbar_arrive(smem_u32(&bar_scale_full[s])); // the planes' barrier is the leader's
+                }
                 uint8_t *planes = smem_ptr + p.filter_bytes + (uint32_t)s * stage_bytes;
                 // a position's (y, x) 32 channels become row (y >> 1) * pw + x of region y & 1 in both planes, 16-byte chunk j
                 // at j ^ ((row >> 1) & 3), the 64-byte swizzle
@@ -1070,7 +1073,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive_peer(leader_addr(smem_u32(&bar_full[s])));
+                    mbar_arrive_peer_written(leader_addr(smem_u32(&bar_full[s])));
                     if (!one)
                         mbar_arrive(smem_u32(&bar_raw_empty));
                 }
@@ -1090,6 +1093,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
         const bool inside = j < p.jp && x < p.wo && !(p.pool && (x & 1));
         const bool relu = p.act == CT_ACT_RELU;
         int i = 0, s = 0;
+        uint32_t scale_phase = 0;
         for (int u = first; u < pairs; u += stride) {
             if (!wanted(u))
                 continue;
@@ -1097,8 +1101,12 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
             const bool mine = 2 * u + rank < total_tiles;
             const int set = i & 1;
             if (!group_wait(
-                    warp == 2 + kCP_CvtWarps, [&] { return mbar_wait(smem_u32(&bar_acc_full[set]), (uint32_t)(i >> 1) & 1u, abort_flag); }, epi_word, i, 2,
-                    32 * kCP_EpiWarps))
+                    warp == 2 + kCP_CvtWarps,
+                    [&] {
+                        return mbar_wait(smem_u32(&bar_acc_full[set]), (uint32_t)(i >> 1) & 1u, abort_flag) &&
+                               (!RAW || mbar_wait(smem_u32(&bar_scale_full[s]), scale_phase, abort_flag));
+                    },
+                    epi_word, i, 2, 32 * kCP_EpiWarps))
                 break;
             const float is = RAW ? *const_cast<volatile float *>(&tile_scale[s]) : p.image_scale[img];
             tc_fence_after_sync();
@@ -1164,13 +1172,13 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive_peer(leader_addr(smem_u32(&bar_acc_empty[set])));
+                mbar_arrive_peer_read(leader_addr(smem_u32(&bar_acc_empty[set])));
                 if (RAW)
                     mbar_arrive(smem_u32(&bar_scale_empty[s]));
             }
             ++i;
             if (++s == p.stages)
-                s = 0;
+                s = 0, scale_phase ^= 1u;
         }
     }
 

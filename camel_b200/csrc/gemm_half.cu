@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(kHThreads, 1)
                     tc_commit(bar);
             };
             auto wait_empty = [&](int acc) {
-                const bool got = mbar_wait(smem_u32(&bar_acc_empty[acc]), (empty_phase >> acc) & 1u, abort_flag);
+                const bool got = mbar_wait<CG == 2 ? kClusterRead : kCta>(smem_u32(&bar_acc_empty[acc]), (empty_phase >> acc) & 1u, abort_flag);
                 empty_phase ^= 1u << acc;
                 tc_fence_after_sync();
                 return got;
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(kHThreads, 1)
                 __syncwarp();
                 if (lane == 0) {
                     if (CG == 2)
-                        mbar_arrive_peer(leader_addr(bar));
+                        mbar_arrive_peer_read(leader_addr(bar));
                     else
                         mbar_arrive(bar);
                 }

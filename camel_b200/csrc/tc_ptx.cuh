@@ -55,17 +55,29 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// What a wait orders: what this CTA's threads and copies wrote before they arrived; what threads of the whole cluster wrote
+// (mbar_arrive_peer_written); or nothing but the execution (mbar_arrive_peer_read: tcgen05.fence does the rest).
+enum WaitFor { kCta, kClusterWritten, kClusterRead };
+template <WaitFor FOR = kCta>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
+#define CT_TRY_WAIT(SEM)                                                \
+    asm volatile(                                                       \
+        "{\n\t"                                                         \
+        ".reg .pred p;\n\t"                                             \
+        "mbarrier.try_wait.parity" SEM ".shared::cta.b64 p, [%1], %2;\n\t" \
+        "selp.u32 %0, 1, 0, p;\n\t"                                     \
+        "}\n"                                                           \
+        : "=r"(ok)                                                      \
+        : "r"(bar), "r"(parity)                                         \
+        : "memory")
+    if (FOR == kClusterWritten)
+        CT_TRY_WAIT(".acquire.cluster");
+    else if (FOR == kClusterRead)
+        CT_TRY_WAIT(".relaxed.cluster");
+    else
+        CT_TRY_WAIT("");
+#undef CT_TRY_WAIT
     return ok != 0;
 }
 
@@ -93,12 +105,13 @@ constexpr uint64_t kWaitBudgetNs = 1000ull * 1000ull * 1000ull; // 1 s
 
 // Bounded wait.  Returns false when the budget ran out or when another role has already
 // given up (*abort_flag != 0); in the first case it raises *abort_flag itself.
+template <WaitFor FOR = kCta>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-    if (mbar_try_wait(bar, parity))
+    if (mbar_try_wait<FOR>(bar, parity))
         return true;
     uint64_t t0 = globaltimer_ns();
     for (uint32_t it = 1;; ++it) {
-        if (mbar_try_wait(bar, parity))
+        if (mbar_try_wait<FOR>(bar, parity))
             return true;
         if ((it & 63u) == 0) {
             if (*abort_flag)
@@ -129,10 +142,11 @@ __device__ __forceinline__ bool mbar_wait_patient(uint32_t bar, uint32_t parity,
 }
 
 // The two for a converged warp: the answer is the same for all lanes, and known to be.
+template <WaitFor FOR = kCta>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-    bool got = mbar_try_wait(bar, parity);
+    bool got = mbar_try_wait<FOR>(bar, parity);
     if (!__all_sync(0xffffffffu, got))
-        got = mbar_wait(bar, parity, abort_flag);
+        got = mbar_wait<FOR>(bar, parity, abort_flag);
     return __all_sync(0xffffffffu, got) != 0;
 }
 __device__ __forceinline__ bool mbar_wait_patient_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
@@ -295,12 +309,16 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
                  : "memory");
     return v;
 }
-// An arrival on the leader's barrier where nothing is published to the other CTA's threads: a warp that hands back tensor memory (what it has read is in
-// registers, tcgen05.wait::ld, and ordered by tcgen05.fence), or that has filled its own CTA's operands (visible to the tensor core by
-// fence.proxy.async).  With release at cluster scope the arrival waits until the thread's earlier stores to global memory are in L2:
-// 2200 clocks of a tile of the few-channel convolution, whose epilogue stores before it hands back.
-__device__ __forceinline__ void mbar_arrive_peer(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+// Arrivals on the leader's barrier.  A warp that has filled its CTA's operands publishes them to the issuer, a thread of the other
+// CTA: release at cluster scope, and the issuer waits with kClusterWritten.
+__device__ __forceinline__ void mbar_arrive_peer_written(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+// A warp that hands back tensor memory publishes nothing: what it has read is in its registers (tcgen05.wait::ld), and tcgen05.fence orders
+// that before the arrival; the issuer waits with kClusterRead.  A release would wait until the thread's earlier stores to
+// global memory are in L2, 2200 clocks of a tile of the few-channel convolution, whose epilogue stores before it hands back.
+__device__ __forceinline__ void mbar_arrive_peer_read(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 // Tile load into THIS CTA's shared memory whose bytes are counted on a barrier of this CTA or the leader.
 __device__ __forceinline__ void tma_load_2d_pair(

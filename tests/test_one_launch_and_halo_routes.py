@@ -82,6 +82,31 @@ def test_images_of_both_forms_in_one_batch(T, port, layer):
         assert same[0].tobytes() == same[-1].tobytes() == got[i].tobytes()
 
 
+# Few channels: five passes and more to a pair of blocks, an odd number of tiles, three to an image; from the input as it is (with and without the pool,
+# 64 filters) and from planes (48 filters).  Images that no float16 pair holds stand alone, in pairs and in rows, so that every mixture of the two forms
+# meets every accumulator set and stage; each image's bytes are those of the same image in a batch of its own.
+@pytest.mark.parametrize("layer", [(251, 32, 26, 28, 64), (251, 20, 26, 29, 48)])
+def test_few_channel_layers_of_many_passes(T, port, layer):
+    n, c, h, w, ko = layer
+    rng = np.random.default_rng(sum(layer))
+    kinds = rng.standard_normal((6, c, h, w)).astype(np.float32)
+    kinds[4, 1, 9, 9] = 1e-20           # one tile spans too much
+    kinds[5, 0, 2], kinds[5, 2, -2] = 1e-15, 2e10  # two do
+    f = rng.standard_normal((ko, c, 3, 3)).astype(np.float32)
+    tf = T.from_numpy(f)
+    alone = np.concatenate([T.conv2d(T.from_numpy(kinds[i : i + 1]), tf, None, 1, 0).numpy() for i in range(6)])
+    assert np.all(np.abs(alone - port.conv2d(kinds, f, None, 1, 0, 0)) <= BOUND * port.conv2d(np.abs(kinds), np.abs(f), None, 1, 0, 0))
+    which = np.where(rng.random(n) < 0.4, rng.integers(4, 6, n), rng.integers(0, 4, n))
+    which[100:110], which[-1] = 5, 4
+    x = T.from_numpy(kinds[which])
+    got, pooled = T.conv2d(x, tf, None, 1, 0).numpy(), T.conv2d(x, tf, None, 1, 0, pool=2).numpy()
+    T.check_async()
+    small = T.maxpool2d(T.from_numpy(alone), 2).numpy()
+    for i in range(n):
+        assert got[i].tobytes() == alone[which[i]].tobytes(), i
+        assert pooled[i].tobytes() == small[which[i]].tobytes(), i
+
+
 # rows and columns that fill no tile, k at the edges of a slice and of its sixteen-value steps, an empty last slice
 # (k = 770: eight slices of 112, the last one with none), rows and columns that are not 16-byte aligned
 @pytest.mark.parametrize("m,k,n", [(1, 193, 33), (64, 784, 1024), (129, 257, 127), (128, 512, 512), (100, 770, 130), (65, 1023, 70), (30, 1024, 1800)])
