@@ -664,10 +664,12 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
 //
 // Two 11-bit terms in float16 instead of tf32 (half_split.cuh), pixels on the accumulator rows.  A tile is 2 jp output
 // rows of an image: its even rows are the 128 rows of one accumulator, its odd rows those of another, positions j * pw + x
-// each.  Two tiles belong to a pair of CTAs, a tile to each, whose MMAs (cta_group::2) are issued by the leader.  The input rows of a tile lie in shared memory as two regions, even and odd rows of the box, so that filter tap
+// each.  A CTA has a tile, or two tiles belong to a pair of CTAs whose MMAs (cta_group::2) are issued by the leader.  The input rows of a
+// tile lie in shared memory as two regions, even and odd rows of the box, so that filter tap
 // (r, s) is, for the even (odd) output rows, region r & 1 ((r + 1) & 1) through a descriptor moved by
 // (r >> 1) * pw + s (((r + 1) >> 1) * pw + s) rows.  The filters are the B operand and stay in shared memory for the
-// whole launch, the leader holding the hi and its peer the lo terms, and each half of the hi terms once more.  Per 16 channels and tap two MMAs an accumulator:
+// whole launch: hi and lo terms in a CTA by itself; in a pair the leader has the hi and its peer the lo terms, and each half of the hi
+// terms once more.  Per 16 channels and tap two MMAs an accumulator:
 //     [main | cross] += X_hi x [W_hi; W_lo]     N = 2 kop
 //             cross  += X_lo x W_hi             N = kop
 // with the low terms stored 2^11 times larger and the cross products in columns of their own, as in gemm_half.cu.  The product of
@@ -683,11 +685,11 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
 // rows are vertical neighbours, horizontal ones are lanes, so the sum, the activation, the 2x2 maximum and the store
 // need no shared memory at all, and a store covers consecutive pixels of a channel.
 //
-// Shared memory is what bounds it (128 bytes per clock): a CTA by itself read 14 KB for the two MMAs of a k-step, 5900 clocks a
-// tile with what the conversion reads and writes; each CTA of a pair reads 11 KB, 3600 clocks of a tile's 6500, and what is left is
-// the epilogue (5000), which waits for the same memory.  8192 x 32 x 28 x 28 -> 64 with the pool 915 -> 805 us; 64 x 32 x 60 x 60 -> 64
-// 72.7 -> 56, 300 x 20 x 30 x 29 -> 48 75.9 -> 57.4, 5 x 32 x 28 x 28 -> 64 17.5 -> 17.1; layers of few tiles from planes lose (3 x 31 x 30 x
-// 29 -> 48, 2 x 2, 16.6 -> 19).  Sixteen epilogue warps instead of eight are no faster (889 us: 72 registers a thread).
+// Shared memory is what bounds it (128 bytes per clock): at 32 channels and 64 filters a CTA by itself reads 14 KB for the two MMAs of a k-step,
+// 5900 clocks a tile with what the conversion reads and writes; each CTA of a pair reads 11 KB, 3600 clocks of a tile's 6500, and
+// what is left is the epilogue (5000), which waits for the same memory.  With one k-step to a tap or fewer filters the pair's
+// larger start and padding cost more than that (conv_pair_form has both sides).  Sixteen epilogue warps instead of eight are no faster (889
+// us: 72 registers a thread).
 //
 // Scales: per filter, and per tile (raw: the converting warps see the whole box before they split it) or, from planes, per
 // image.  The converting warps also leave the range of every tile in the call's own scratch; conv_tmem_filters_kernel,
@@ -730,7 +732,7 @@ struct ConvPairParams {
     const float *bias;
     float *out;        // [batch][ko][ho][wo], or [batch][ko][ho/2][wo/2] with pool
     uint32_t *flags;
-    int ko, kop, c, kh, kw, pad; // kop: ko rounded up to 32, the columns of an MMA of two CTAs
+    int ko, kop, c, kh, kw, pad; // kop: ko rounded up to 16, for a pair to 32, the columns of an MMA
     int ho, wo, pw;    // pw = input width + 2 pad
     int jp, tiles_y;   // pairs of output rows per tile, tiles per image
     int region_rows;   // input rows of a region
@@ -744,7 +746,7 @@ struct ConvPairParams {
     int box_w, off_x, box_rows, raw_bytes, raw_stride;
 };
 
-template <bool RAW>
+template <bool RAW, int CG>
 __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
     const __grid_constant__ CUtensorMap map_x_hi, const __grid_constant__ CUtensorMap map_x_lo,
     const __grid_constant__ ConvPairParams p, const int total_tiles) {
@@ -764,7 +766,8 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
     volatile int *abort_flag = &abort_flag_s;
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31; // known to be the same for the warp
-    const int rank = (int)(blockIdx.x & 1), first = (int)(blockIdx.x >> 1), stride = (int)(gridDim.x >> 1), pairs = (total_tiles + 1) / 2;
+    const int rank = CG == 2 ? (int)(blockIdx.x & 1) : 0; // in the cluster of two
+    const int first = (int)blockIdx.x / CG, stride = (int)gridDim.x / CG, passes = (total_tiles + CG - 1) / CG;
     if (threadIdx.x == 0) {
         abort_flag_s   = *reinterpret_cast<volatile uint32_t *>(p.flags + FLAG_TIMEOUT) != 0 ? 1 : 0;
         filters_wide_s = 0;
@@ -783,7 +786,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
-            mbar_init(smem_u32(&bar_full[s]), RAW ? 2 * kCP_CvtWarps : 1); // of both CTAs
+            mbar_init(smem_u32(&bar_full[s]), RAW ? CG * kCP_CvtWarps : 1); // of both CTAs
             mbar_init(smem_u32(&bar_empty[s]), 1);
             mbar_init(smem_u32(&bar_scale_full[s]), 1);
             mbar_init(smem_u32(&bar_scale_empty[s]), kCP_EpiWarps);
@@ -792,7 +795,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
         mbar_init(smem_u32(&bar_raw_empty), kCP_CvtWarps);
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&bar_acc_full[b]), 1);
-            mbar_init(smem_u32(&bar_acc_empty[b]), 2 * kCP_EpiWarps);
+            mbar_init(smem_u32(&bar_acc_empty[b]), CG * kCP_EpiWarps);
         }
         mbar_init(smem_u32(&bar_done), 1);
         mbar_fence_init();
@@ -812,8 +815,13 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
         }
     });
     if (warp == 1) {
-        tmem_alloc_pair(smem_u32(&tmem_base_slot), 512);
-        tmem_relinquish_pair();
+        if (CG == 2) {
+            tmem_alloc_pair(smem_u32(&tmem_base_slot), 512);
+            tmem_relinquish_pair();
+        } else {
+            tmem_alloc(smem_u32(&tmem_base_slot), 512);
+            tmem_relinquish();
+        }
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -824,12 +832,14 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
     if (RAW && blockIdx.x == 0 && threadIdx.x == 0)
         p.tile_range[total_tiles] = make_uint2(filters_wide ? 1u : 0u, 0u);
 
-    // ---- the filters' planes, once, 64-byte rows, swizzled: per tap kop rows of the leader's hi or its peer's lo terms; behind those
-    // of all taps, per tap half of the hi terms; then half of the last tap's lo terms ----
-    const int half_rows = p.kop >> 1, q_at = taps * p.kop, r_at = q_at + taps * half_rows, shift = p.kop == 64 ? 6 : 5;
+    // ---- the filters' planes, once, 64-byte rows, swizzled.  One CTA: per tap kop rows of hi, then of lo terms.  A pair: per tap kop rows of
+    // the leader's hi or its peer's lo terms; behind those of all taps, per tap half of the hi terms; then half of the last tap's lo
+    // terms ----
+    const int half_rows = p.kop >> 1, q_at = CG == 2 ? taps * p.kop : 0, r_at = CG == 2 ? q_at + taps * half_rows : (2 * taps - 1) * p.kop;
+    const int shift = p.kop == 64 ? 6 : 5; // a pair's is 32 or 64
     if (!filters_wide)
-        for (int i = threadIdx.x; i < q_at * 4; i += kCP_Threads) {
-            const int chunk = i & 3, row = i >> 2, tap = row >> shift, f = row & (p.kop - 1), c0 = chunk * 8;
+        for (int i = threadIdx.x; i < taps * p.kop * 4; i += kCP_Threads) {
+            const int chunk = i & 3, row = i >> 2, tap = CG == 2 ? row >> shift : row / p.kop, f = row - tap * p.kop, c0 = chunk * 8;
             const float *src  = filters + f * filter_stride;
             const float scale = 1.0f / filter_inv[f]; // both are powers of two
             __half2 hi[4], lo[4];
@@ -843,6 +853,11 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
             auto put = [&](int to, const __half2 (&v)[4]) {
                 *reinterpret_cast<uint4 *>(smem_ptr + (size_t)to * kCP_RowB + ((chunk ^ ((to >> 1) & 3)) << 4)) = *reinterpret_cast<const uint4 *>(v);
             };
+            if (CG == 1) {
+                put(row + tap * p.kop, hi);
+                put(row + tap * p.kop + p.kop, lo);
+                continue;
+            }
             if (rank)
                 put(row, lo);
             else
@@ -856,13 +871,15 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
         }
     filters_taken();
     __syncthreads();
-    cluster_sync(); // the MMAs read both CTAs' filters, and nothing is signalled on the partner's barriers before they exist
+    if (CG == 2)
+        cluster_sync(); // the MMAs read both CTAs' filters, and nothing is signalled on the partner's barriers before they exist
 
-    // this CTA's tile of pair u (the last may have one only: then both compute it, and the leader stores it), and, from planes, whether
-    // either image of the pair is left to this kernel
-    auto tile_of = [&](int u) { return min(2 * u + rank, total_tiles - 1); };
+    // this CTA's tile of pass u (the last may have one for a pair: then both compute it, and the leader stores it), and, from planes, whether
+    // either image of the pass is left to this kernel
+    auto tile_of = [&](int u) { return CG == 2 ? min(2 * u + rank, total_tiles - 1) : u; };
     auto wanted  = [&](int u) {
-        return RAW || __any_sync(0xffffffffu, p.image_scale[2 * u / p.tiles_y] != 0.0f || p.image_scale[min(2 * u + 1, total_tiles - 1) / p.tiles_y] != 0.0f);
+        return RAW || __any_sync(0xffffffffu, p.image_scale[CG * u / p.tiles_y] != 0.0f ||
+                                                  (CG == 2 && p.image_scale[min(2 * u + 1, total_tiles - 1) / p.tiles_y] != 0.0f));
     };
 
     if (filters_wide || failed) {
@@ -870,7 +887,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
         // ===== TMA producer: one box per plane and region (raw mode: one box of the input) =====
         int i = 0;
         const int nstages = RAW ? 1 : p.stages;
-        for (int u = first; u < pairs; u += stride) {
+        for (int u = first; u < passes; u += stride) {
             if (!wanted(u))
                 continue;
             const int tile = tile_of(u), img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
@@ -888,11 +905,16 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                 } else {
                     const uint32_t full = smem_u32(&bar_full[s]), dst = stage_base + (uint32_t)s * stage_bytes;
                     if (rank == 0) // both CTAs' bytes are counted on the leader's barrier
-                        mbar_expect_tx(full, 2u * 4u * (uint32_t)(p.region_rows * p.pw * kCP_RowB));
+                        mbar_expect_tx(full, (uint32_t)CG * 4u * (uint32_t)(p.region_rows * p.pw * kCP_RowB));
                     for (int g = 0; g < 2; ++g) { // region g: rows h0 + g + 2 i, which lie in one of the two sub-images
                         const int32_t row = (h0 + g) >> 1, sub = (h0 + g) & 1;
-                        tma_load_5d_pair(dst + (uint32_t)g * region, &map_x_hi, leader_addr(full), 0, -p.pad, row, sub, img);
-                        tma_load_5d_pair(dst + (uint32_t)(2 + g) * region, &map_x_lo, leader_addr(full), 0, -p.pad, row, sub, img);
+                        if (CG == 2) {
+                            tma_load_5d_pair(dst + (uint32_t)g * region, &map_x_hi, leader_addr(full), 0, -p.pad, row, sub, img);
+                            tma_load_5d_pair(dst + (uint32_t)(2 + g) * region, &map_x_lo, leader_addr(full), 0, -p.pad, row, sub, img);
+                        } else {
+                            tma_load_5d(dst + (uint32_t)g * region, &map_x_hi, full, 0, -p.pad, row, sub, img);
+                            tma_load_5d(dst + (uint32_t)(2 + g) * region, &map_x_lo, full, 0, -p.pad, row, sub, img);
+                        }
                     }
                 }
             }
@@ -911,24 +933,25 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
         }
     } else if (warp == 1) {
         // ===== MMA issuer =====
-        // (the leader's, for the pair; a whole warp with uniform control flow, so that descriptors stay in uniform registers)
+        // (the leader's, for a pair; a whole warp with uniform control flow, so that descriptors stay in uniform registers)
         if (rank == 0) {
-            const uint32_t idesc2 = make_idesc(0u, 256, (uint32_t)(2 * p.kop)), idesc1 = make_idesc(0u, 256, (uint32_t)p.kop);
+            const uint32_t idesc2 = make_idesc(0u, 128 * CG, (uint32_t)(2 * p.kop)), idesc1 = make_idesc(0u, 128 * CG, (uint32_t)p.kop);
             const bool two = p.c > 16; // k-steps that hold channels
             // descriptors are moved by adding to their address field (16-byte units; shared memory is far below its range)
             const uint32_t unit = kCP_RowB >> 4, lo_terms = 2 * region >> 4, kop = (uint32_t)p.kop;
+            const uint32_t p_step = (CG == 2 ? kop : 2 * kop) * unit, q_step = (CG == 2 ? kop >> 1 : 2 * kop) * unit;
             const uint32_t p_0 = (uint32_t)smem_desc_k<kCP_RowB>(smem_base), q_0 = p_0 + (uint32_t)q_at * unit, last_lo = p_0 + (uint32_t)r_at * unit;
             auto desc = [](uint32_t low) { return smem_desc_k<kCP_RowB>(0) & 0xffffffff00000000ull | low; };
             int i   = 0, s = 0;
             uint32_t full_phase = 0;
             bool ok = true;
-            for (int u = first; u < pairs; u += stride) {
+            for (int u = first; u < passes; u += stride) {
                 if (!wanted(u))
                     continue;
                 const int set = i & 1;
                 // the accumulators have been read, the planes are complete
-                ok = mbar_wait_warp<kClusterRead>(smem_u32(&bar_acc_empty[set]), ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag) &&
-                     mbar_wait_warp<RAW ? kClusterWritten : kCta>(smem_u32(&bar_full[s]), full_phase, abort_flag);
+                ok = mbar_wait_warp<CG == 2 ? kClusterRead : kCta>(smem_u32(&bar_acc_empty[set]), ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag) &&
+                     mbar_wait_warp<RAW && CG == 2 ? kClusterWritten : kCta>(smem_u32(&bar_full[s]), full_phase, abort_flag);
                 if (!ok)
                     break;
                 tc_fence_after_sync();
@@ -936,17 +959,17 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                 const uint32_t d_even = tmem_base + (uint32_t)(set * 256), d_odd = d_even + 128u;
                 uint32_t w_p = p_0, w_q = q_0, accumulate = 0u;
                 auto step = [&](uint32_t even, uint32_t odd, uint32_t k, uint32_t acc) {
-                    mma_f16_pair_warp(d_even, desc(even + k), desc(w_p + k), idesc2, acc);
-                    mma_f16_pair_warp(d_odd, desc(odd + k), desc(w_p + k), idesc2, acc);
-                    mma_f16_pair_warp(d_even + kop, desc(even + lo_terms + k), desc(w_q + k), idesc1, 1u);
-                    mma_f16_pair_warp(d_odd + kop, desc(odd + lo_terms + k), desc(w_q + k), idesc1, 1u);
+                    mma_f16_warp<CG>(d_even, desc(even + k), desc(w_p + k), idesc2, acc);
+                    mma_f16_warp<CG>(d_odd, desc(odd + k), desc(w_p + k), idesc2, acc);
+                    mma_f16_warp<CG>(d_even + kop, desc(even + lo_terms + k), desc(w_q + k), idesc1, 1u);
+                    mma_f16_warp<CG>(d_odd + kop, desc(odd + lo_terms + k), desc(w_q + k), idesc1, 1u);
                 };
                 for (int r = 0; r < p.kh; ++r) {
                     // the tap's pixels for the even and the odd output rows
                     uint32_t even = (uint32_t)smem_desc_k<kCP_RowB>(hi0 + (uint32_t)(r & 1) * region + (uint32_t)((r >> 1) * p.pw * kCP_RowB));
                     uint32_t odd  = (uint32_t)smem_desc_k<kCP_RowB>(hi0 + (uint32_t)((r + 1) & 1) * region + (uint32_t)(((r + 1) >> 1) * p.pw * kCP_RowB));
                     const int whole = r + 1 < p.kh ? p.kw : p.kw - 1; // all but the last tap
-                    for (int sx = 0; sx < whole; ++sx, even += unit, odd += unit, w_p += kop * unit, w_q += (kop >> 1) * unit) {
+                    for (int sx = 0; sx < whole; ++sx, even += unit, odd += unit, w_p += p_step, w_q += q_step) {
                         step(even, odd, 0, accumulate);
                         accumulate = 1u;
                         if (two)
@@ -956,23 +979,23 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                         uint32_t k = 0;
                         if (two)
                             step(even, odd, 0, 1u), k = 2;
-                        mma_f16_pair_warp(d_even + kop, desc(even + lo_terms + k), desc(w_q + k), idesc1, 1u);
-                        mma_f16_pair_warp(d_odd + kop, desc(odd + lo_terms + k), desc(w_q + k), idesc1, 1u);
-                        mma_f16_pair_warp(d_even + kop, desc(even + k), desc(last_lo + k), idesc1, 1u);
-                        mma_f16_pair_warp(d_odd + kop, desc(odd + k), desc(last_lo + k), idesc1, 1u);
-                        mma_f16_shifted_pair_warp<kHalfLoBits>(d_even + kop, desc(even + k), desc(w_q + k), idesc1);
-                        mma_f16_shifted_pair_warp<kHalfLoBits>(d_odd + kop, desc(odd + k), desc(w_q + k), idesc1);
+                        mma_f16_warp<CG>(d_even + kop, desc(even + lo_terms + k), desc(w_q + k), idesc1, 1u);
+                        mma_f16_warp<CG>(d_odd + kop, desc(odd + lo_terms + k), desc(w_q + k), idesc1, 1u);
+                        mma_f16_warp<CG>(d_even + kop, desc(even + k), desc(last_lo + k), idesc1, 1u);
+                        mma_f16_warp<CG>(d_odd + kop, desc(odd + k), desc(last_lo + k), idesc1, 1u);
+                        mma_f16_shifted_warp<kHalfLoBits, CG>(d_even + kop, desc(even + k), desc(w_q + k), idesc1);
+                        mma_f16_shifted_warp<kHalfLoBits, CG>(d_odd + kop, desc(odd + k), desc(w_q + k), idesc1);
                     }
                 }
-                tc_commit_pair_warp(smem_u32(&bar_empty[s]));      // the stage is free once these MMAs have retired
-                tc_commit_pair_warp(smem_u32(&bar_acc_full[set])); // and the accumulators are complete
+                tc_commit_warp<CG>(smem_u32(&bar_empty[s]));      // the stage is free once these MMAs have retired
+                tc_commit_warp<CG>(smem_u32(&bar_acc_full[set])); // and the accumulators are complete
                 ++i;
                 if (++s == p.stages)
                     s = 0, full_phase ^= 1u;
             }
             if (!ok || *abort_flag) {
                 __syncwarp();
-                tc_commit_pair_warp(smem_u32(&bar_done));
+                tc_commit_warp<CG>(smem_u32(&bar_done));
                 const uint64_t t0 = globaltimer_ns();
                 while (!mbar_try_wait(smem_u32(&bar_done), 0) && globaltimer_ns() - t0 < kWaitBudgetNs) {
                 }
@@ -989,7 +1012,7 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
             const int first_raw = ct / p.pw * p.box_w + ct % p.pw + p.off_x;
             int i = 0, s = 0;
             uint32_t stage_phase = 1u;
-            for (int u = first; u < pairs; u += stride, ++i) {
+            for (int u = first; u < passes; u += stride, ++i) {
                 const int tile = tile_of(u);
                 if (!group_wait(
                         warp == 2, [&] { return mbar_wait(smem_u32(&bar_raw_full), (uint32_t)i & 1u, abort_flag); }, cvt_word, 0, 1, 32 * kCP_CvtWarps))
@@ -1073,7 +1096,10 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive_peer_written(leader_addr(smem_u32(&bar_full[s])));
+                    if (CG == 2)
+                        mbar_arrive_peer_written(leader_addr(smem_u32(&bar_full[s])));
+                    else
+                        mbar_arrive(smem_u32(&bar_full[s]));
                     if (!one)
                         mbar_arrive(smem_u32(&bar_raw_empty));
                 }
@@ -1094,11 +1120,11 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
         const bool relu = p.act == CT_ACT_RELU;
         int i = 0, s = 0;
         uint32_t scale_phase = 0;
-        for (int u = first; u < pairs; u += stride) {
+        for (int u = first; u < passes; u += stride) {
             if (!wanted(u))
                 continue;
             const int tile = tile_of(u), img = tile / p.tiles_y, ty = tile - img * p.tiles_y;
-            const bool mine = 2 * u + rank < total_tiles;
+            const bool mine = CG * u + rank < total_tiles;
             const int set = i & 1;
             if (!group_wait(
                     warp == 2 + kCP_CvtWarps,
@@ -1172,7 +1198,10 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive_peer_read(leader_addr(smem_u32(&bar_acc_empty[set])));
+                if (CG == 2)
+                    mbar_arrive_peer_read(leader_addr(smem_u32(&bar_acc_empty[set])));
+                else
+                    mbar_arrive(smem_u32(&bar_acc_empty[set]));
                 if (RAW)
                     mbar_arrive(smem_u32(&bar_scale_empty[s]));
             }
@@ -1184,11 +1213,15 @@ __global__ void __launch_bounds__(kCP_Threads, 1) conv_pairs_kernel(
 
     tc_fence_before_sync();
     __syncthreads();
-    cluster_sync(); // neither CTA goes while the other's MMAs, copies or arrivals may still reach it
+    if (CG == 2)
+        cluster_sync(); // neither CTA goes while the other's MMAs, copies or arrivals may still reach it
     if (warp == 1) {
         __syncwarp();
         tc_fence_after_sync();
-        tmem_dealloc_pair(tmem_base, 512);
+        if (CG == 2)
+            tmem_dealloc_pair(tmem_base, 512);
+        else
+            tmem_dealloc(tmem_base, 512);
     }
     if (threadIdx.x == 0 && !failed && *abort_flag)
         atomicExch(p.flags + FLAG_TIMEOUT, 1u + (uint32_t)blockIdx.x);
@@ -1236,8 +1269,8 @@ static bool conv_tmem_plan(
 }
 
 static bool conv_pair_plan(
-    ConvPairParams &p, int64_t c, int64_t h, int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t pad, bool raw, size_t *smem) {
-    p.ko = (int)ko, p.kop = (int)((ko + 31) / 32 * 32), p.c = (int)c;
+    ConvPairParams &p, int64_t c, int64_t h, int64_t wd, int64_t ko, int64_t kh, int64_t kw, int64_t pad, bool raw, int cg, size_t *smem) {
+    p.ko = (int)ko, p.kop = (int)((ko + 16 * cg - 1) / (16 * cg) * (16 * cg)), p.c = (int)c;
     p.kh = (int)kh, p.kw = (int)kw, p.pad = (int)pad;
     p.pw  = (int)(wd + 2 * pad);
     p.wo  = p.pw - (int)kw + 1;
@@ -1251,7 +1284,7 @@ static bool conv_pair_plan(
     // a tap's window of 128 rows may run past the region: reserve those rows too
     const int rows = std::max(p.region_rows * p.pw, (int)(kh / 2) * p.pw + (int)kw - 1 + 128);
     p.region_bytes = (rows * kCP_RowB + 1023) & ~1023;
-    p.filter_bytes = (int)(((kh * kw * 3 + 1) * (p.kop / 2) * kCP_RowB + 1023) & ~1023);
+    p.filter_bytes = (int)(((cg == 2 ? kh * kw * 3 + 1 : kh * kw * 4) * (p.kop / 2) * kCP_RowB + 1023) & ~1023);
     // raw mode: the box starts at the 16-byte boundary at or left of x = -pad and is a whole number of 16-byte units wide
     p.off_x      = (((int)pad + 3) & ~3) - (int)pad;
     p.box_w      = (p.off_x + p.pw + 3) & ~3;
@@ -1291,20 +1324,36 @@ bool conv_tmem_applicable(int64_t c, int64_t h, int64_t w, int64_t ko, int64_t k
     ConvPairParams pairs;
     ConvTmemParams wide;
     size_t smem;
-    return conv_pair_plan(pairs, c, h, w, ko, kh, kw, pad, false, &smem) && conv_tmem_plan(wide, h, w, kh, kw, pad, 0, false);
+    return (conv_pair_plan(pairs, c, h, w, ko, kh, kw, pad, false, 2, &smem) || conv_pair_plan(pairs, c, h, w, ko, kh, kw, pad, false, 1, &smem)) &&
+           conv_tmem_plan(wide, h, w, kh, kw, pad, 0, false);
 }
 
-// Whether the kernel can read this input as it is (NCHW float32) instead of pre-split NHWC planes:
-// the tensor map over it needs row strides of whole 16-byte units and an aligned base, and the raw
-// boxes have to fit into shared memory beside two stages of planes.
-static bool conv_tmem_reads_input_directly(
-    const float *x, int64_t c, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw, int64_t pad, int pool) {
-    if ((w & 3) != 0 || (reinterpret_cast<uintptr_t>(x) & 15u) != 0)
-        return false;
-    ConvTmemParams p;
-    ConvPairParams pairs;
-    size_t smem;
-    return conv_tmem_plan(p, h, w, kh, kw, pad, pool, true) && conv_pair_plan(pairs, c, h, w, ko, kh, kw, pad, true, &smem);
+// The form in which the layer runs: the input read as it is (NCHW float32) where a tensor map covers it, which needs row strides of
+// whole 16-byte units and an aligned base, and where the raw boxes fit into shared memory beside two stages of planes; else from
+// pre-split NHWC planes.  Pairs of CTAs, which read a fifth less shared memory for an MMA, where that decides: two k-steps to a tap, more
+// than four taps, many tiles, and no padding of the filters to 32 unless the boxes are read twice or come as planes (8192 x 32 x
+// 28 x 28 -> 64 with the pool 932 us by single CTAs, 887 by pairs, 2000 x 24 x 30 x 29 -> 32 269 and 252, 256 x 60 x 60 -> 16 128 and 125).  Elsewhere
+// single CTAs, which start without a cluster and pad filters to 16 (4 x 16 x 28 x 28 -> 64 16.9 us and 18.5, 1024 x 16 x 28 x 28 -> 32 75
+// and 89, 2048 x 48 129 and 165, 512 x 24 x 56 x 56 -> 16, 2 x 2, 118 and 156, 640 tiles of 32 -> 64 33.0 and 33.6).
+static bool conv_pair_form(
+    ConvPairParams &p, ConvTmemParams &wide, const float *x, int64_t batch, int64_t c, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw,
+    int64_t pad, int pool, int64_t sms, bool *raw, int *cg, size_t *smem) {
+    const bool mapped = (w & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    for (const bool as_is : {true, false}) {
+        if ((as_is && !mapped) || !conv_tmem_plan(wide, h, w, kh, kw, pad, pool, as_is))
+            continue;
+        *raw = as_is;
+        const bool padded = (ko - 1) % 32 < 16;
+        if (c > 16 && kh * kw > 4 && conv_pair_plan(p, c, h, w, ko, kh, kw, pad, as_is, 2, smem) && p.tiles_y * batch >= 6 * sms &&
+            !(padded && as_is && p.box_rows * p.pw <= 32 * kCP_CvtWarps)) {
+            *cg = 2;
+            return true;
+        }
+        for (*cg = 1; *cg <= 2; ++*cg)
+            if (conv_pair_plan(p, c, h, w, ko, kh, kw, pad, as_is, *cg, smem))
+                return true;
+    }
+    return false;
 }
 
 // x NCHW float32.  The layer in split float16, and behind it the tf32 form for the images that need it.  Where the
@@ -1314,11 +1363,12 @@ static bool conv_tmem_reads_input_directly(
 ct_status conv_tmem_filters(
     DeviceState *st, const float *x, const float *w, const float *bias, int64_t batch, int64_t c, int64_t h, int64_t wd,
     int64_t ko, int64_t kh, int64_t kw, int64_t pad, int act, int pool, float *out) {
-    const bool raw = conv_tmem_reads_input_directly(x, c, h, wd, ko, kh, kw, pad, pool);
+    bool raw;
+    int cg;
     ConvPairParams pp;
     ConvTmemParams pt; // the tf32 form
     size_t pair_smem;
-    if (!conv_pair_plan(pp, c, h, wd, ko, kh, kw, pad, raw, &pair_smem) || !conv_tmem_plan(pt, h, wd, kh, kw, pad, pool, raw))
+    if (!conv_pair_form(pp, pt, x, batch, c, h, wd, ko, kh, kw, pad, pool, st->sm_count, &raw, &cg, &pair_smem))
         return fail(CT_ERR_INVALID, "conv2d: internal tile shape not usable");
     pp.w = pt.w = w, pp.bias = pt.bias = bias, pp.out = pt.out = out, pp.flags = pt.flags = st->flags_dev;
     pt.ko = (int)ko, pt.c = (int)c;
@@ -1332,12 +1382,12 @@ ct_status conv_tmem_filters(
     if (!attr_set_dev[st->device & 15]) {
         CT_CUDA(cudaFuncSetAttribute(conv_tmem_filters_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
         CT_CUDA(cudaFuncSetAttribute(conv_tmem_filters_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        CT_CUDA(cudaFuncSetAttribute(conv_pairs_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCP_Smem));
-        CT_CUDA(cudaFuncSetAttribute(conv_pairs_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCP_Smem));
+        for (auto kernel : {conv_pairs_kernel<false, 1>, conv_pairs_kernel<false, 2>, conv_pairs_kernel<true, 1>, conv_pairs_kernel<true, 2>})
+            CT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCP_Smem));
         attr_set_dev[st->device & 15] = true;
     }
     const size_t smem32 = (size_t)pt.stages * 2 * pt.plane_bytes + (raw ? (size_t)kTA_RawStages * pt.raw_stride : 0) + kTA_StagingBytes + 1024;
-    const unsigned grid   = 2u * (unsigned)std::min<int64_t>((pair_tiles + 1) / 2, st->sm_count / 2);
+    const unsigned grid   = (unsigned)cg * (unsigned)std::min<int64_t>((pair_tiles + cg - 1) / cg, st->sm_count / cg);
     const unsigned grid32 = (unsigned)std::max<int64_t>(std::min<int64_t>(tiles, st->sm_count), (tiles + kTA_MaxOwn - 1) / kTA_MaxOwn);
     if (raw) {
         // the input [batch][c][h][w]; box = box_w floats x box_rows rows x 32 channels of one image, not
@@ -1356,7 +1406,7 @@ ct_status conv_tmem_filters(
         cudaError_t launched;
         {
             ProfScope prof("gemm_tc");
-            (void)launch_dependent_cluster(conv_pairs_kernel<true>, 2, dim3(grid), dim3(kCP_Threads), pair_smem, stream(), map, map, pp, (int)pair_tiles);
+            (void)launch_dependent_cluster(cg == 2 ? conv_pairs_kernel<true, 2> : conv_pairs_kernel<true, 1>, cg, dim3(grid), dim3(kCP_Threads), pair_smem, stream(), map, map, pp, (int)pair_tiles);
             (void)launch_dependent(conv_tmem_filters_kernel<true>, dim3(grid32), dim3(kTA_ThreadsRaw), smem32, stream(), map32, map32, pt, (int)tiles);
             launched = cudaGetLastError();
         }
@@ -1396,7 +1446,7 @@ ct_status conv_tmem_filters(
     CT_TRY(encode32(&m32_hi, planes));
     CT_TRY(encode32(&m32_lo, planes + slot / 2));
     ProfScope prof("gemm_tc");
-    (void)launch_dependent_cluster(conv_pairs_kernel<false>, 2, dim3(grid), dim3(kCP_Threads), pair_smem, stream(), m16_hi, m16_lo, pp, (int)pair_tiles);
+    (void)launch_dependent_cluster(cg == 2 ? conv_pairs_kernel<false, 2> : conv_pairs_kernel<false, 1>, cg, dim3(grid), dim3(kCP_Threads), pair_smem, stream(), m16_hi, m16_lo, pp, (int)pair_tiles);
     CT_LAUNCH_CHECK("conv_pairs");
     (void)launch_dependent(conv_tmem_filters_kernel<false>, dim3(grid32), dim3(kTA_Threads), smem32, stream(), m32_hi, m32_lo, pt, (int)tiles);
     CT_LAUNCH_CHECK("conv_tmem_filters");

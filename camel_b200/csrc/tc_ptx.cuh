@@ -210,6 +210,16 @@ __device__ __forceinline__ void tma_load_4d(
         : "memory");
 }
 
+__device__ __forceinline__ void tma_load_5d(
+    uint32_t dst_smem, const void *map, uint32_t bar, int32_t c0, int32_t c1, int32_t c2, int32_t c3, int32_t c4) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+        :
+        : "r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+        : "memory");
+}
+
 // ---- tensor memory ----------------------------------------------------------------------
 
 // Whole-warp instructions (.sync.aligned): call from all 32 lanes of one warp.
@@ -382,56 +392,69 @@ __device__ __forceinline__ void mma_tf32_pair(
 }
 
 // The same for a whole converged warp whose control flow and operands are uniform, of which one lane issues: addresses and
-// descriptors then stay in the uniform registers that the instruction reads.
-__device__ __forceinline__ void mma_f16_pair_warp(
-    uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, q;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-        "}\n"
-        :
-        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
+// descriptors then stay in the uniform registers that the instruction reads.  CG: one CTA, or the leader for a pair.
+#define CT_MMA_WARP(GROUP, KIND)                                                      \
+    asm volatile(                                                                     \
+        "{\n\t"                                                                       \
+        ".reg .pred p, q;\n\t"                                                        \
+        "elect.sync _|q, 0xffffffff;\n\t"                                             \
+        "setp.ne.b32 p, %4, 0;\n\t"                                                   \
+        "@q tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], %1, %2, %3, p;\n\t" \
+        "}\n"                                                                         \
+        :                                                                             \
+        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)          \
+        : "memory")
+template <int CG = 2>
+__device__ __forceinline__ void mma_f16_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    if (CG == 2)
+        CT_MMA_WARP("2", "f16");
+    else
+        CT_MMA_WARP("1", "f16");
 }
 __device__ __forceinline__ void mma_tf32_pair_warp(
     uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, q;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@q tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t"
-        "}\n"
-        :
-        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
+    CT_MMA_WARP("2", "tf32");
 }
+#undef CT_MMA_WARP
 // D = A . B + D * 2^-SHIFT (0 .. 15)
-template <int SHIFT>
-__device__ __forceinline__ void mma_f16_shifted_pair_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, q;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
-        "setp.ne.b32 p, 1, 0;\n\t"
-        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p, %4;\n\t"
-        "}\n"
-        :
-        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(SHIFT)
-        : "memory");
+template <int SHIFT, int CG>
+__device__ __forceinline__ void mma_f16_shifted_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+#define CT_MMA_SHIFTED(GROUP)                                                        \
+    asm volatile(                                                                    \
+        "{\n\t"                                                                      \
+        ".reg .pred p, q;\n\t"                                                       \
+        "elect.sync _|q, 0xffffffff;\n\t"                                            \
+        "setp.ne.b32 p, 1, 0;\n\t"                                                   \
+        "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], %1, %2, %3, p, %4;\n\t" \
+        "}\n"                                                                        \
+        :                                                                            \
+        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(SHIFT)              \
+        : "memory")
+    if (CG == 2)
+        CT_MMA_SHIFTED("2");
+    else
+        CT_MMA_SHIFTED("1");
+#undef CT_MMA_SHIFTED
 }
-__device__ __forceinline__ void tc_commit_pair_warp(uint32_t bar) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred q;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
-        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t"
-        "}\n" ::"r"(bar),
-        "h"((uint16_t)3)
-        : "memory");
+template <int CG = 2>
+__device__ __forceinline__ void tc_commit_warp(uint32_t bar) {
+    if (CG == 2)
+        asm volatile(
+            "{\n\t"
+            ".reg .pred q;\n\t"
+            "elect.sync _|q, 0xffffffff;\n\t"
+            "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t"
+            "}\n" ::"r"(bar),
+            "h"((uint16_t)3)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t"
+            ".reg .pred q;\n\t"
+            "elect.sync _|q, 0xffffffff;\n\t"
+            "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+            "}\n" ::"r"(bar)
+            : "memory");
 }
 
 // 32 lanes x 32 consecutive 32-bit columns: thread i of the warp receives row (lane base + i).

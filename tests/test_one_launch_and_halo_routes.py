@@ -82,10 +82,11 @@ def test_images_of_both_forms_in_one_batch(T, port, layer):
         assert same[0].tobytes() == same[-1].tobytes() == got[i].tobytes()
 
 
-# Few channels: five passes and more to a pair of blocks, an odd number of tiles, three to an image; from the input as it is (with and without the pool,
-# 64 filters) and from planes (48 filters).  Images that no float16 pair holds stand alone, in pairs and in rows, so that every mixture of the two forms
-# meets every accumulator set and stage; each image's bytes are those of the same image in a batch of its own.
-@pytest.mark.parametrize("layer", [(251, 32, 26, 28, 64), (251, 20, 26, 29, 48)])
+# Few channels: five passes and more to a block or pair of blocks, an odd number of tiles, three to an image; by pairs from the input as it is and
+# from planes, by single blocks so (up to 16 channels; filters that pairs would pad).  Images that no float16 pair holds stand alone, in
+# pairs and in rows, so that every mixture of the two forms meets every accumulator set and stage; each image's bytes are those of the same image in a
+# batch of its own, which single blocks compute.
+@pytest.mark.parametrize("layer", [(301, 32, 26, 28, 64), (301, 20, 26, 29, 48), (251, 14, 26, 28, 40), (251, 14, 26, 29, 40), (301, 20, 26, 28, 48)])
 def test_few_channel_layers_of_many_passes(T, port, layer):
     n, c, h, w, ko = layer
     rng = np.random.default_rng(sum(layer))
