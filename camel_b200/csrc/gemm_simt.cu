@@ -302,7 +302,8 @@ ct_status launch_skinny_smem(
 // on lanes and a broadcast weight per FMA, as before, shared memory took four times what the pipe did.
 // 60000 x 785 x 10: 139 -> 74 us (the pipe alone 33, the read of x 29); the rest is issue, nearly two other instructions
 // per FMA, of them the conversions to float64 at 16 per clock and SM.  (From eight columns on many rows take gemm_tall_kernel.)
-// The weights come in whole lines, the first of them before the activations: 1024 x 10 at 4096 rows 13.0 -> 11.4 us.
+// From eight columns on the weights come in whole lines, the first of them before the activations: 1024 x 10 at 4000 rows 13.6 -> 12.2 us,
+// 1600 x 14 at 20000 84.9 -> 80.5; below, a thread takes rows of them, 200 x 5 at 20000 rows 11.2 us in whole lines and 10.6 so.
 //
 // The float64 sums of the lanes are added by exchanging rows first (each step halves the rows a lane keeps),
 // then across what is left; every lane of a group of 32 / R then holds its row's n sums, adds the bias, rounds
@@ -412,6 +413,7 @@ __global__ void __launch_bounds__(32 * kFewWarps, 1) gemm_few_columns_kernel(
     const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ bias, int64_t m, int k, int n,
     int act, float *__restrict__ out, int64_t *__restrict__ argmax) {
     constexpr int S = FewStride<NE>::value, D = RING / R; // steps in the ring
+    constexpr bool kLines = NE >= 8; // weights staged by whole lines
     extern __shared__ __align__(16) double w_few[]; // [k rounded up to 32][S], then the warps' rings [D][R][32] floats
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int steps = (k + 31) >> 5;
@@ -449,47 +451,54 @@ __global__ void __launch_bounds__(32 * kFewWarps, 1) gemm_few_columns_kernel(
         copy_async_commit();
         f_slot = f_slot + 1 == D ? 0 : f_slot + 1;
     };
-    // the weights, widened once per block: whole lines of w, the first of them asked for before the activations
+    // the weights, widened once per block
     const int elements = k * n, e_rows = (32 * kFewWarps) / n, e_cols = (32 * kFewWarps) % n;
     int e_row = (int)threadIdx.x / n, e_col = (int)threadIdx.x % n;
     constexpr int kBatch = 16;
-    float e_v[kBatch];
+    float e_v[kLines ? kBatch : 1];
     auto ask = [&](int e) {
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u)
+        for (int u = 0; kLines && u < kBatch; ++u)
             e_v[u] = e + u * 32 * kFewWarps < elements ? __ldg(w + e + u * 32 * kFewWarps) : 0.0f;
     };
     ask((int)threadIdx.x);
 #pragma unroll 1
     for (int d = 0; d < D - 1; ++d)
         fetch();
-    for (int e = (int)threadIdx.x; e < elements;) {
+    if (kLines) { // whole lines of w, the first of them asked for before the activations
+        for (int e = (int)threadIdx.x; e < elements;) {
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-            if (e + u * 32 * kFewWarps < elements)
-                w_few[e_row * S + e_col] = (double)e_v[u];
-            e_row += e_rows, e_col += e_cols;
-            if (e_col >= n)
-                e_col -= n, ++e_row;
+            for (int u = 0; u < kBatch; ++u) {
+                if (e + u * 32 * kFewWarps < elements)
+                    w_few[e_row * S + e_col] = (double)e_v[kLines ? u : 0];
+                e_row += e_rows, e_col += e_cols;
+                if (e_col >= n)
+                    e_col -= n, ++e_row;
+            }
+            e += kBatch * 32 * kFewWarps;
+            if (e < elements)
+                ask(e);
         }
-        e += kBatch * 32 * kFewWarps;
-        if (e < elements)
-            ask(e);
-    }
-    if (n < NE)
-        for (int kk = threadIdx.x; kk < k; kk += 32 * kFewWarps)
-            for (int j = n; j < NE; ++j)
-                w_few[kk * S + j] = 0.0;
-    for (int e = k * S + (int)threadIdx.x; e < steps * 32 * S; e += 32 * kFewWarps)
-        w_few[e] = 0.0;
-    __syncthreads();
-    // A step's activations are read and widened while the one before is multiplied.
-    int slot = 0;
-    double xv[R];
-    copy_async_wait<D - 2>();
+        if (n < NE)
+            for (int kk = threadIdx.x; kk < k; kk += 32 * kFewWarps)
+                for (int j = n; j < NE; ++j)
+                    w_few[kk * S + j] = 0.0;
+        for (int e = k * S + (int)threadIdx.x; e < steps * 32 * S; e += 32 * kFewWarps)
+            w_few[e] = 0.0;
+    } else { // a thread takes rows of w
+#pragma unroll 4
+        for (int kk = threadIdx.x; kk < steps * 32; kk += 32 * kFewWarps) {
+            float v[NE];
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-        xv[r] = (double)ring[r * 32];
+            for (int j = 0; j < NE; ++j)
+                v[j] = (kk < k && j < n) ? __ldg(w + (int64_t)kk * n + j) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < NE; j += 2)
+                *reinterpret_cast<double2 *>(w_few + kk * S + j) = make_double2((double)v[j], (double)v[j + 1]);
+        }
+    }
+    __syncthreads();
+    int slot = 0;
     for (int64_t t = first; t < tiles; t += stride) {
         const int64_t row0 = t * R;
         double acc[R][NE];
@@ -500,13 +509,12 @@ __global__ void __launch_bounds__(32 * kFewWarps, 1) gemm_few_columns_kernel(
                 acc[r][j] = 0.0;
 #pragma unroll 1
         for (int step = 0; step < steps; ++step) {
-            copy_async_wait<D - 3>();
-            slot = slot + 1 == D ? 0 : slot + 1;
-            float next[R];
+            copy_async_wait<D - 2>();
+            double xv[R];
 #pragma unroll
             for (int r = 0; r < R; ++r)
-                next[r] = ring[(slot * R + r) * 32];
-            fetch(); // into the slot before the last, whose values have been used
+                xv[r] = (double)ring[(slot * R + r) * 32];
+            slot = slot + 1 == D ? 0 : slot + 1;
             const double2 *wp = reinterpret_cast<const double2 *>(w_few + (step * 32 + lane) * S);
 #pragma unroll
             for (int j = 0; j < NE / 2; ++j) {
@@ -518,9 +526,7 @@ __global__ void __launch_bounds__(32 * kFewWarps, 1) gemm_few_columns_kernel(
                     acc[r][2 * j + 1] = __fma_rn(xv[r], wv.y, acc[r][2 * j + 1]);
                 }
             }
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                xv[r] = (double)next[r];
+            fetch(); // into the slot before this one, whose values have been used
         }
         double sum[NE];
         few_reduce<R, NE>(acc, lane, sum);
@@ -824,6 +830,9 @@ ct_status launch_few(
         // 11.0 / 13.1 and 8.0 / 9.4 / 10.4 / 11.0 at 3000, 13.6 / 14.4 / 16.7 / 19.6 and 9.4 / 12.0 / 13.6 / 13.6 at 6000; 1024 x 10 at 4096
         // 11.4 and 12.2.
         const bool many = m > 32 * (int64_t)st->sm_count || (TallCfg<NE>::kExtra == 0 && m > 16 * (int64_t)st->sm_count);
+        // sixteen rows to a warp where tiles of eight would be walked twice: 785 x 10 19.0 and 18.8 at 16000 rows, 26.3 and 24.2 at
+        // 20000; 785 x 8 13.3 and 14.1, 19.5 and 16.7
+        const bool deep = m > (int64_t)st->sm_count * kTallWarps * 8;
         if (many && TallCfg<NE>::smem(k) <= kMost && resident < by_rows) {
             static bool tall_attr_set_dev[16] = {};
             if (!tall_attr_set_dev[st->device & 15]) {
@@ -831,9 +840,6 @@ ct_status launch_few(
                 CT_CUDA(cudaFuncSetAttribute(gemm_tall_kernel<NE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
                 tall_attr_set_dev[st->device & 15] = true;
             }
-            // sixteen rows to a warp where tiles of eight would be walked twice: 785 x 10 19.0 and 18.8 at 16000 rows, 26.3 and 24.2 at
-            // 20000; 785 x 8 13.3 and 14.1, 19.5 and 16.7
-            const bool deep     = m > (int64_t)st->sm_count * kTallWarps * 8;
             const int64_t tiles = deep ? (m + 15) / 16 : (m + 7) / 8;
             const unsigned grid = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
             CT_CUDA(launch_dependent(deep ? gemm_tall_kernel<NE, 2> : gemm_tall_kernel<NE, 1>, dim3(grid), dim3(32 * kTallWarps), TallCfg<NE>::smem(k), stream(),
@@ -858,7 +864,11 @@ ct_status launch_few(
         const unsigned grid = (unsigned)(tiles < st->sm_count ? tiles : st->sm_count);
         auto kernel         = longer ? gemm_few_columns_kernel<NE, 4, kFewRingShort>
                                      : (deep ? gemm_few_columns_kernel<NE, kDeep, kFewRing> : gemm_few_columns_kernel<NE, 4, kFewRing>);
-        CT_CUDA(launch_dependent(kernel, dim3(grid), dim3(32 * kFewWarps), smem, stream(), a, b, bias, m, (int)k, n, act, out, argmax));
+        // One block comes to an SM.  Where two would fit, they crowd on the SMs that are free first, and shared memory is set aside for both, so that L1,
+        // which has to keep the lines that two steps share, gets the little that is left: 785 x 3 at 60000 rows 62 us, so 50, and an update
+        // with such a product 170 and 112.
+        const size_t alone = std::max<size_t>(smem, smem > 80 * 1024 ? 115 * 1024 : 0);
+        CT_CUDA(launch_dependent(kernel, dim3(grid), dim3(32 * kFewWarps), alone, stream(), a, b, bias, m, (int)k, n, act, out, argmax));
         CT_LAUNCH_CHECK("gemm_few_columns");
         return CT_OK;
     }
