@@ -833,7 +833,12 @@ ct_status launch_few(
         // sixteen rows to a warp where tiles of eight would be walked twice: 785 x 10 19.0 and 18.8 at 16000 rows, 26.3 and 24.2 at
         // 20000; 785 x 8 13.3 and 14.1, 19.5 and 16.7
         const bool deep = m > (int64_t)st->sm_count * kTallWarps * 8;
-        if (many && TallCfg<NE>::smem(k) <= kMost && resident < by_rows) {
+        // Rows that are no whole lines share a line between two steps, which has to stay in L1 meanwhile: 196 KB of shared memory leave that 60 KB,
+        // more leave 28.  There the kernel is ahead for one pass only: 1400 x 8 30.4 us and above 41.9 at 16000 rows, 82.3 and 72.4 at
+        // 40000 (1200 x 8, with 60 KB, 53.4 and 64.5), 1200 x 10 30.0 and 39.9, 80.7 and 72.0; whole lines, 1600 x 8, 39.1 and 50.3 at 20000.
+        // Beyond twelve columns it is ahead all the same (785 x 16 64.2 and 80.8 at 40000 rows).
+        const bool cached = NE > 12 || TallCfg<NE>::smem(k) <= 195 * 1024 || k % 32 == 0;
+        if (many && TallCfg<NE>::smem(k) <= kMost && (cached || !deep) && resident < by_rows) {
             static bool tall_attr_set_dev[16] = {};
             if (!tall_attr_set_dev[st->device & 15]) {
                 CT_CUDA(cudaFuncSetAttribute(gemm_tall_kernel<NE, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));

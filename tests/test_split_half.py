@@ -400,10 +400,10 @@ def test_convolution_narrow_and_wide(T, shape, kind):
 
 
 # blocks of two and four rows, resident weights with four and (19001 rows) eight rows to a warp: up to six columns, and eight to twelve where the float64
-# MMA has no room for its ring (1300 x 12, 1600 x 10, 1900 x 8); with that MMA (33 x 16, 785 x 10, 96 x 13);
+# MMA has no room for its ring (1300 x 12, 1600 x 10, 1900 x 8) or only up to 18944 rows (1400 x 8); with that MMA (33 x 16, 785 x 10, 96 x 13);
 # weights that leave room for a short ring (2300 x 10, 1400 x 16), for no ring (1600 x 16) and none at all (2700 x 12)
 @pytest.mark.parametrize("m", [1, 2, 3, 297, 597, 2051, 4099, 19001])
-@pytest.mark.parametrize("k,n", [(1, 3), (31, 1), (785, 4), (130, 6), (33, 16), (785, 10), (96, 13), (1900, 8), (1600, 10), (1300, 12), (2300, 10), (1400, 16),
+@pytest.mark.parametrize("k,n", [(1, 3), (31, 1), (785, 4), (130, 6), (33, 16), (785, 10), (96, 13), (1400, 8), (1900, 8), (1600, 10), (1300, 12), (2300, 10), (1400, 16),
                                  (1600, 16), (2700, 12)])
 def test_few_columns(T, m, k, n):
     rng = np.random.default_rng(m + k + n)
