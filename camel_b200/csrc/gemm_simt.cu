@@ -1243,8 +1243,9 @@ __global__ void __launch_bounds__(256) gemm_tn_skinny_finish_kernel(
 template <int NMAX, int R>
 static ct_status launch_tn_skinny(
     DeviceState *st, const float *a_km, const float *b, int64_t m, int64_t k, int n, float *out) {
-    auto choose = [] {
-        if constexpr (NMAX >= 8 && NMAX <= 16)
+    constexpr bool kTall = NMAX >= 8 && NMAX <= 16;
+    auto choose         = [] {
+        if constexpr (kTall)
             return gemm_tn_tall_kernel<NMAX, R>;
         else
             return gemm_tn_skinny_kernel<NMAX, R>;
@@ -1274,6 +1275,12 @@ static ct_status launch_tn_skinny(
     k_per_slice         = (k_per_slice + kTnChunk - 1) / kTnChunk * kTnChunk;
     if (k_per_slice < kTnChunk)
         k_per_slice = kTnChunk;
+    // Small blocks with a chunk or two each that nearly fill the machine leave the kernels before and behind them no registers to start with, and
+    // more sums to add up than the chunk saved: one chunk more to each then (one product behind another, 100 x 33000 x 13 60 us, 1032
+    // blocks in 1184 places, and 21, 256 x 17000 x 8 26.3 and 16.6, 192 x 45000 x 8 35 and 18; at 0.63 of the places 12.0 and 14.9 for 40 x 17000 x
+    // 13; blocks of five warps lose, 600 x 12000 x 13 25.7 and 30.1).
+    if (kTall && threads < kTnMaxThreads && k_per_slice <= 2 * kTnChunk && mblocks * ((k + k_per_slice - 1) / k_per_slice) * 5 > 4 * fit * (int64_t)st->sm_count)
+        k_per_slice += kTnChunk;
     slices = k > 0 ? (k + k_per_slice - 1) / k_per_slice : 1;
     CT_TRY(ensure_ws(&st->splitk_ws, &st->splitk_ws_bytes, (size_t)slices * m * n * sizeof(double)));
     auto *partial = static_cast<double *>(st->splitk_ws);

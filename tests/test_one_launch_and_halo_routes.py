@@ -162,8 +162,10 @@ def test_many_rows_of_few_columns(T, port, m, k, n, act):
 
 
 # The transposed left operand with eight to sixteen columns: rows that end in each part of a warp's 64 and leave a warp without any,
-# k of less than four values, of one more than a chunk and of several slices.  The bound is the one above.
-@pytest.mark.parametrize("m,k,n", [(1, 3, 8), (63, 33, 10), (65, 32, 9), (321, 500, 12), (785, 5003, 10), (257, 20001, 16), (130, 77, 7), (640, 129, 13)])
+# k of less than four values, of one more than a chunk and of several slices; single chunks that would nearly fill the machine, and pairs of them.
+# The bound is the one above.
+@pytest.mark.parametrize("m,k,n", [(1, 3, 8), (63, 33, 10), (65, 32, 9), (321, 500, 12), (785, 5003, 10), (257, 20001, 16), (130, 77, 7), (640, 129, 13),
+                                   (100, 32999, 13), (250, 17003, 8), (190, 45001, 10)])
 def test_transposed_operand_and_few_columns(T, m, k, n):
     rng = np.random.default_rng(m + k + n)
     x, y = (rng.standard_normal(shape).astype(np.float32) for shape in ((k, m), (k, n)))
