@@ -849,10 +849,13 @@ bool halo_geometry(int64_t c_pad, int64_t h, int64_t w, int64_t ko, int64_t kh, 
         g->stages = std::min(kH_HaloStages, (budget - g->slots * g->slot_bytes) / halo);
     } else {
         // In a ring, groups of taps, a row of them where a halo serves whole rows: with a tap by itself copies, waits and commits took 700
-        // clocks, where those of 64 filters take 290 (40 x 100 x 50 x 50 -> 64, 5 x 5, 207 us, 168 so).  A third halo where that leaves 64 KB.
-        if (stride == 1 && 2 * halo + 4 * kw * one <= budget)
-            g->group = (int)kw, g->slot_bytes *= (int)kw;
-        g->stages = 3 * halo + 64 * 1024 <= budget ? 3 : 2;
+        // clocks, where those of 64 filters take 290 (40 x 100 x 50 x 50 -> 64, 5 x 5, 207 us, 168 so).  Room for three slots beside two halos is enough for that (12 x
+        // 151 x 46 x 46 -> 115, 5 x 5, 116 us by single taps, 94 so).  Where a row is too much or the halos of a strided layer have parts of rows, by threes, from
+        // 16 taps on (20 x 107 x 58 x 58 -> 108, 5 x 5 at stride 2, 104 and 88; nine taps lose by what the boxes bring for nothing, 43 x 200 x 45 x
+        // 47 -> 67, 3 x 3, 102 and 110).  A third halo where that leaves 64 KB and two slots.
+        const int row = stride == 1 && 2 * halo + 3 * kw * one <= budget ? (int)kw : (kh * kw >= 16 && 2 * halo + 3 * 3 * one <= budget ? 3 : 1);
+        g->group      = row, g->slot_bytes *= row;
+        g->stages = 3 * halo + std::max(64 * 1024, 2 * g->slot_bytes) <= budget ? 3 : 2;
         g->slots  = (int)std::min<int64_t>(std::min<int64_t>(16, all / g->group), (budget - g->stages * halo) / g->slot_bytes);
         if (budget < g->stages * halo || g->slots < std::min<int64_t>(g->group > 1 ? 2 : 4, all / g->group))
             return false;

@@ -33,12 +33,14 @@ def port():
 # leave sub-images unread; half of a channel block, and one channel more; k of two and three drains (c = 97, 193 with
 # nine taps; 33 with twenty-five); 17 and 129 filters; a tile of one row; partial last tiles.  Paired rows: an odd number of
 # rows, a row of 128 positions, 16 and 64 filters, 8 channels, an even filter, rows that no tensor map covers.  Halo again: more
-# filters than have their bias in shared memory; 1 x 1 filters with and without a stride, a strided layer of one tile.
+# filters than have their bias in shared memory; 1 x 1 filters with and without a stride, a strided layer of one tile; filters that are streamed by rows of
+# taps and, of a strided layer, by threes.
 LAYERS = [(2, 48, 57, 57, 96, 3, 3, 2, 1), (1, 33, 20, 23, 70, 3, 3, 3, 1), (2, 40, 30, 33, 64, 1, 1, 2, 0), (1, 16, 41, 40, 65, 5, 5, 2, 2),
           (1, 97, 17, 30, 17, 3, 3, 1, 1), (1, 193, 15, 30, 129, 3, 3, 1, 0), (1, 33, 40, 61, 40, 5, 5, 1, 2), (1, 17, 20, 130, 80, 3, 3, 1, 1),
           (2, 9, 33, 64, 80, 3, 3, 1, 1), (2, 32, 28, 28, 64, 3, 3, 1, 1), (1, 8, 27, 33, 16, 3, 3, 1, 1), (1, 20, 16, 126, 33, 3, 3, 1, 1),
           (1, 31, 30, 29, 48, 2, 2, 1, 0), (1, 17, 12, 60, 17, 1, 5, 1, 0), (1, 40, 20, 30, 300, 3, 3, 1, 1),
-          (2, 48, 30, 33, 64, 1, 1, 2, 0), (1, 16, 65, 64, 40, 3, 3, 2, 1), (1, 64, 9, 8, 70, 3, 3, 2, 1), (1, 70, 20, 30, 33, 1, 1, 1, 0)]
+          (2, 48, 30, 33, 64, 1, 1, 2, 0), (1, 16, 65, 64, 40, 3, 3, 2, 1), (1, 64, 9, 8, 70, 3, 3, 2, 1), (1, 70, 20, 30, 33, 1, 1, 1, 0),
+          (1, 130, 30, 33, 100, 5, 5, 1, 2), (1, 100, 41, 37, 130, 5, 5, 2, 2), (1, 70, 20, 61, 130, 5, 5, 1, 0)]
 
 
 @pytest.mark.parametrize("layer", LAYERS)
