@@ -592,34 +592,37 @@ __global__ void __launch_bounds__(256) conv_range_kernel(
     const int slice   = filter ? 0 : (int)(blockIdx.x - ko - o * slices);
     const float *src  = filter ? w + o * c * taps : x + o * count;
     const int64_t n   = filter ? (int64_t)c * taps : count;
-    const int64_t step = filter ? 256 : (int64_t)slices * 256;
+    const int step    = filter ? 256 : slices * 256;
     uint2 r            = make_uint2(0u, kNoneSmallest);
-    // eight loads in flight, also where fewer are left (zeros are not noticed): as a loop that was only to be unrolled they came one by one, 3 x
-    // 31 x 30 x 29 6.9 us, so 5.6, 32 x 64 x 56 x 56 13.1 and 8.2
-    if (!filter && vec_ok) {
-        const float4 *s4 = reinterpret_cast<const float4 *>(src);
-        for (int64_t i = (int64_t)slice * 256 + threadIdx.x; i < n / 4; i += 8 * step) {
-            float4 q[8];
+    // Eight loads in flight, also where fewer are left (zeros are not noticed): as a loop that was only to be unrolled they came one by one, 3 x
+    // 31 x 30 x 29 4.2 us, so 3.3, 32 x 64 x 56 x 56 8.9 and 7.0, 73 x 122 x 47 x 47 27.8 and 23.7 (each load with a condition of its own 29.8).
+    auto walk = [&](auto zero, auto take) {
+        using V      = decltype(zero);
+        const V *at  = reinterpret_cast<const V *>(src) + (int64_t)slice * 256 + threadIdx.x;
+        const V *end = reinterpret_cast<const V *>(src) + n / (int64_t)(sizeof(V) / 4);
+        for (; at + 7 * step < end; at += 8 * step) {
+            V q[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u)
-                q[u] = i + u * step < n / 4 ? s4[i + u * step] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                q[u] = at[u * step];
 #pragma unroll
             for (int u = 0; u < 8; ++u)
-                range_take(r, q[u].x), range_take(r, q[u].y), range_take(r, q[u].z), range_take(r, q[u].w);
+                take(q[u]);
         }
-    } else {
-        const float *at = src + (int64_t)slice * 256 + threadIdx.x, *end = src + n;
-        for (; at < end; at += 8 * step) {
-            float q[8];
-            const float *a = at;
-#pragma unroll
-            for (int u = 0; u < 8; ++u, a += step)
-                q[u] = a < end ? *a : 0.0f;
+        if (at < end) {
+            V q[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u)
-                range_take(r, q[u]);
+                q[u] = at + u * step < end ? at[u * step] : zero;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                take(q[u]);
         }
-    }
+    };
+    if (!filter && vec_ok)
+        walk(make_float4(0.0f, 0.0f, 0.0f, 0.0f), [&](const float4 &q) { range_take(r, q.x), range_take(r, q.y), range_take(r, q.z), range_take(r, q.w); });
+    else
+        walk(0.0f, [&](float q) { range_take(r, q); });
     r = range_warp(r);
     if ((threadIdx.x & 31) == 0)
         part[threadIdx.x >> 5] = r;
