@@ -721,13 +721,13 @@ __global__ void __launch_bounds__(256, 3) conv_planes_kernel(
         image_scale[img] = fits ? 1.0f / scale : 0.0f; // a power of two
     const int rows = g.hs * ROW_MOD, cols = g.ws * COL_MOD;
     const bool plain    = !fits && g.sub.tf32_plain;
-    const int64_t plane = (int64_t)rows * cols * c_pad;
+    const int64_t plane = (int64_t)__popc(g.sub.used) * g.hs * g.ws * c_pad;
     uint8_t *slot       = slots + (int64_t)img * plane * 8;
     auto place = [&](int row, int col) { // of the grown image; -1: not wanted
         if (ROW_MOD * COL_MOD == 1)
             return row * cols + col;
         const int sub = row % ROW_MOD * COL_MOD + col % COL_MOD;
-        return g.sub.used >> sub & 1u ? (sub * g.hs + row / ROW_MOD) * g.ws + col / COL_MOD : -1;
+        return g.sub.used >> sub & 1u ? (__popc(g.sub.used & ((1u << sub) - 1u)) * g.hs + row / ROW_MOD) * g.ws + col / COL_MOD : -1;
     };
     int to = -1;
     if (live) {
@@ -947,12 +947,40 @@ ct_status conv_halo(
     if (!halo_geometry(c_pad, h, wd, ko, kh, kw, stride, pad, &g))
         return fail(CT_ERR_INVALID, "conv2d: internal tile shape not usable");
     auto align_up          = [](size_t v) { return (v + 1023) & ~(size_t)1023; };
-    const int64_t taps     = kh * kw, subs = stride * stride, sub = (int64_t)g.hs * g.pw, positions = sub * subs;
+    const int64_t taps = kh * kw, subs = stride * stride, sub = (int64_t)g.hs * g.pw;
+    ConvHaloParams p;
+    p.halos = 0, p.halo_taps[0] = 0;
+    uint8_t order[kH_MaxTaps] = {};
+    uint32_t used = 0;
+    for (int image = 0, listed = 0; image < (int)subs; ++image) {
+        for (int t = 0; t < (int)taps; ++t) {
+            const int r = t / (int)kw - (int)pad, q = t % (int)kw - (int)pad, a = floor_div(r, stride), b = floor_div(q, stride);
+            if ((r - a * (int)stride) * (int)stride + (q - b * (int)stride) != image)
+                continue;
+            order[t]              = (uint8_t)listed;
+            p.tap_shift[listed++] = (uint16_t)(((a - g.y_min) * g.pw + (b - g.x_min)) * (kH_RowB / 16));
+        }
+        if (listed > p.halo_taps[p.halos]) { // the planes hold the sub-images that a tap reads, one behind the other
+            p.halo_at[p.halos]     = (int)(p.halos * sub);
+            p.halo_taps[++p.halos] = (uint8_t)listed;
+            used |= 1u << image;
+        }
+    }
+    const int64_t positions = sub * p.halos;
+    const size_t slot       = (size_t)positions * c_pad * 8;
+    // At most 4 GB of planes, one image at least: the batch goes in parts, which the images, each with a scale of its own, do not notice.
+    const int64_t most = std::max<int64_t>(1, (int64_t)((4ull << 30) / slot));
+    if (batch > most) {
+        const int64_t parts = (batch + most - 1) / most, part = (batch + parts - 1) / parts;
+        for (int64_t at = 0; at < batch; at += part)
+            CT_TRY(conv_halo(st, x + at * c * h * wd, w, std::min(part, batch - at), c, c_pad, h, wd, ko, kh, kw, stride, pad, bias, act,
+                             out + at * ko * g.ho * g.wo));
+        return CT_OK;
+    }
     const int64_t tiles    = g.image_tiles * batch, pairs = (tiles + 1) / 2, items = pairs * g.tiles_n;
     if (items > 0x3fffffffll || positions > 0x3fffffffll)
         return fail(CT_ERR_TOO_LARGE, "conv2d: too many tiles");
     const size_t w16       = align_up((size_t)ko * taps * c_pad * 2), w32 = align_up((size_t)ko * taps * c_pad * 4);
-    const size_t slot      = (size_t)positions * c_pad * 8;
     const size_t w_words   = align_up((size_t)g.n * g.tiles_n * 4), x_words = align_up((size_t)batch * 4);
     const size_t ranges    = align_up((size_t)batch * conv_range_slices(batch, c * h * wd) * 8);
     CT_TRY(ensure_ws(&st->gemm_ws, &st->gemm_ws_bytes, 2 * w_words + x_words + ranges + 2 * w16 + 2 * w32 + (size_t)batch * slot));
@@ -961,7 +989,6 @@ ct_status conv_halo(
     float *image_scale     = reinterpret_cast<float *>(ws + 2 * w_words);
     uint8_t *range_words   = ws + 2 * w_words + x_words;
     uint8_t *w16_hi        = range_words + ranges, *w32_hi = w16_hi + 2 * w16, *xp = w32_hi + 2 * w32;
-    ConvHaloParams p;
     p.filter_scale = filter_scale, p.bias = bias_copy, p.image_scale = image_scale;
     p.out = out, p.flags = st->flags_dev;
     p.ko = (int)ko, p.n = g.n;
@@ -981,23 +1008,6 @@ ct_status conv_halo(
     p.act = act;
     p.by_pairs = fast_divisor(pairs), p.by_tiles = fast_divisor(g.image_tiles), p.by_pw = fast_divisor(g.pw);
     p.group = g.group, p.tap_bytes = g.three ? g.n / 2 * kH_RowB : g.n * kH_RowB, p.f1 = g.group * p.tap_bytes;
-    p.halos = 0, p.halo_taps[0] = 0;
-    uint8_t order[kH_MaxTaps] = {};
-    uint32_t used = 0;
-    for (int image = 0, listed = 0; image < (int)subs; ++image) {
-        for (int t = 0; t < (int)taps; ++t) {
-            const int r = t / (int)kw - (int)pad, q = t % (int)kw - (int)pad, a = floor_div(r, stride), b = floor_div(q, stride);
-            if ((r - a * (int)stride) * (int)stride + (q - b * (int)stride) != image)
-                continue;
-            order[t]              = (uint8_t)listed;
-            p.tap_shift[listed++] = (uint16_t)(((a - g.y_min) * g.pw + (b - g.x_min)) * (kH_RowB / 16));
-        }
-        if (listed > p.halo_taps[p.halos]) {
-            p.halo_at[p.halos]     = (int)(image * sub);
-            p.halo_taps[++p.halos] = (uint8_t)listed;
-            used |= 1u << image;
-        }
-    }
     const ConvSubImages images{(int)stride, (int)stride, used, false, g.hs, g.pw, g.y_min * (int)stride, g.x_min * (int)stride};
     CT_TRY(conv_prepass(x, w, batch, c, h, wd, c_pad, ko, taps, w16_hi, w32_hi, w16, w32, order, filter_scale, bias, bias_copy, range_words,
                         image_scale, xp, images));

@@ -30,7 +30,7 @@ ct_status conv_tmem_filters(
 bool conv_halo_applicable(int64_t c_pad, int64_t h, int64_t w, int64_t ko, int64_t kh, int64_t kw, int64_t stride,
                           int64_t pad);
 // The float16 planes of an image: sub-images of the rows (columns) that are alike modulo row_mod (col_mod), a bit of `used`
-// for each that is needed.  tf32_plain: tf32 planes are not taken apart.
+// for each that is needed; the others have no place in the planes.  tf32_plain: tf32 planes are not taken apart.
 struct ConvSubImages {
     int row_mod = 1, col_mod = 1;
     uint32_t used = 1;

@@ -110,6 +110,21 @@ def test_few_channel_layers_of_many_passes(T, port, layer):
         assert pooled[i].tobytes() == small[which[i]].tobytes(), i
 
 
+def test_a_batch_whose_planes_come_in_parts(T, port):
+    """4.7 GB of planes where 4 are taken at a time: an odd batch in two unequal parts, each image as by itself."""
+    rng = np.random.default_rng(3)
+    kinds = rng.standard_normal((5, 64, 64, 64)).astype(np.float32)
+    kinds[4, 0, 3, 3] = 1e-20
+    f = rng.standard_normal((17, 64, 3, 3)).astype(np.float32)
+    tf = T.from_numpy(f)
+    alone = T.conv2d(T.from_numpy(kinds), tf, None, 1, 1).numpy()
+    assert np.all(np.abs(alone - port.conv2d(kinds, f, None, 1, 1, 0)) <= BOUND * port.conv2d(np.abs(kinds), np.abs(f), None, 1, 1, 0))
+    which = rng.integers(0, 5, 2101)
+    got = T.conv2d(T.from_numpy(kinds[which]), tf, None, 1, 1).numpy()
+    T.check_async()
+    assert all(got[i].tobytes() == alone[k].tobytes() for i, k in enumerate(which))
+
+
 # rows and columns that fill no tile, k at the edges of a slice and of its sixteen-value steps, an empty last slice
 # (k = 770: eight slices of 112, the last one with none), rows and columns that are not 16-byte aligned
 @pytest.mark.parametrize("m,k,n", [(1, 193, 33), (64, 784, 1024), (129, 257, 127), (128, 512, 512), (100, 770, 130), (65, 1023, 70), (30, 1024, 1800)])
