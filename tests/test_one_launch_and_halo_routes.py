@@ -110,6 +110,25 @@ def test_few_channel_layers_of_many_passes(T, port, layer):
         assert pooled[i].tobytes() == small[which[i]].tobytes(), i
 
 
+# Stride 3 takes its nine sub-images to the halo kernel from 16384 outputs per filter on: odd and unequal extents, padding, taps that leave five
+# sub-images unread, rows and columns that no tap reaches, and images of both forms.
+@pytest.mark.parametrize("layer", [(33, 48, 72, 72, 64, 3, 1), (33, 33, 73, 71, 70, 3, 1), (41, 40, 67, 70, 40, 2, 0), (30, 40, 71, 74, 40, 5, 2)])
+def test_layers_at_stride_three(T, port, layer):
+    n, c, h, w, ko, kern, pad = layer
+    rng = np.random.default_rng(sum(layer))
+    kinds = rng.standard_normal((3, c, h, w)).astype(np.float32)
+    kinds[2, 1, 9, 7] = 1e-20
+    f, b = (rng.standard_normal(shape).astype(np.float32) for shape in ((ko, c, kern, kern), (ko,)))
+    which = rng.integers(0, 3, n)
+    got = T.conv2d(T.from_numpy(kinds[which]), T.from_numpy(f), T.from_numpy(b), 3, pad).numpy()
+    T.check_async()
+    want = port.conv2d(kinds, f, b, 3, pad, 0)
+    size = port.conv2d(np.abs(kinds), np.abs(f), np.abs(b), 3, pad, 0)
+    for i, k in enumerate(which):
+        assert np.all(np.abs(got[i] - want[k]) <= BOUND * size[k]), i
+        assert got[i].tobytes() == got[np.flatnonzero(which == k)[0]].tobytes(), i
+
+
 def test_a_batch_whose_planes_come_in_parts(T, port):
     """4.7 GB of planes where 4 are taken at a time: an odd batch in two unequal parts, each image as by itself."""
     rng = np.random.default_rng(3)

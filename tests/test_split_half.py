@@ -236,8 +236,8 @@ def test_values_that_float16_pairs_cannot_hold_are_put_right(T, m, k, n, count, 
         assert abs(got[rows[t], cols[t]] - want[rows[t], cols[t]]) <= SINGLE * abs(want[rows[t], cols[t]])
 
 
-# strided; halo; filters in tensor memory from the input itself, from planes, and with a tile of odd rows
-@pytest.mark.parametrize("shape", [(2, 48, 21, 23, 70, 3, 2, 1), (2, 64, 30, 28, 128, 3, 1, 1), (2, 32, 28, 28, 64, 3, 1, 1),
+# patches; strided and unstrided halos; few channels from the input itself, from planes, and with a tile of odd rows
+@pytest.mark.parametrize("shape", [(2, 49, 21, 23, 70, 3, 2, 1), (2, 48, 21, 23, 70, 3, 2, 1), (2, 64, 30, 28, 128, 3, 1, 1), (2, 32, 28, 28, 64, 3, 1, 1),
                                    (2, 20, 26, 27, 40, 3, 1, 1), (2, 20, 16, 18, 40, 3, 1, 0)])
 @pytest.mark.parametrize("kind", ["input", "isolated", "filters"])
 @pytest.mark.parametrize("lowest", [-9, -16, -44])
@@ -331,8 +331,8 @@ def test_few_channel_layers_on_two_streams_share_no_state(T):
         assert all(o.numpy().tobytes() == want[j] for o in outs[j])
 
 
-# filters in tensor memory, halos, patches; a product of one wave and one with a conditional launch in front
-@pytest.mark.parametrize("what", [(6, 32, 28, 28, 64, 3, 1, 1), (3, 64, 30, 28, 128, 3, 1, 1), (2, 48, 21, 23, 70, 3, 2, 1),
+# few channels, unstrided and strided halos, patches; a product of one wave and one with a conditional launch in front
+@pytest.mark.parametrize("what", [(6, 32, 28, 28, 64, 3, 1, 1), (3, 64, 30, 28, 128, 3, 1, 1), (2, 48, 21, 23, 70, 3, 2, 1), (2, 49, 21, 23, 70, 3, 2, 1),
                                   (256, 200, 256), (1500, 700, 900)])
 def test_recorded_calls_decide_on_every_replay(T, what):
     """The same graph over ordinary values, one small one, and values that need tf32 terms: the bytes of eager calls."""
@@ -375,9 +375,9 @@ def test_recorded_calls_decide_on_every_replay(T, what):
         check(lib.ct_graph_destroy(graph))
 
 
-# (n, c, h, w, ko, kernel, stride, pad): patches in registers and read twice (k = 1200), odd sizes; halos with a
+# (n, c, h, w, ko, kernel, stride, pad): patches in registers and read twice (k = 1200), odd sizes; halos with a stride, with a
 # partial last tile, channels that do not fill a block, more than 128 filters, 1 x 1 and 5 x 5 taps
-CONVS = [(3, 48, 21, 23, 70, 3, 2, 1), (2, 8, 33, 21, 20, 3, 2, 0), (2, 48, 15, 16, 40, 5, 3, 2), (2, 12, 24, 24, 65, 5, 1, 2),
+CONVS = [(3, 49, 21, 23, 70, 3, 2, 1), (3, 48, 21, 23, 70, 3, 2, 1), (2, 8, 33, 21, 20, 3, 2, 0), (2, 48, 15, 16, 40, 5, 3, 2), (2, 12, 24, 24, 65, 5, 1, 2),
          (2, 64, 30, 28, 128, 3, 1, 1), (3, 40, 14, 14, 136, 3, 1, 0), (2, 100, 17, 19, 72, 1, 1, 0), (2, 20, 57, 56, 72, 5, 1, 2)]
 
 
