@@ -693,9 +693,9 @@ ct_status ct_conv2d_maxpool2(
     if (fusable && !halo_kernel)
         return conv2d_run(x, w, bias, n, c, h, wd, ko, kh, kw, stride, pad, act, out, 2);
     // The convolution into a temporary, then maxpool2d.  For layers that the pixels-on-rows kernel could pool in its epilogue the halo
-    // kernel is the faster one all the same, in most cases (64 x 64 x 56 x 56 -> 64 171 us fused, 130 so; 256 x 33 x 14 x 14 -> 17
-    // 66 and 46; not with 16 x 16 outputs, two tiles of 14 rows and 2, 1024 x 64 x 16 x 16 -> 64 189 and 223), but they take no more
-    // than 256 MB for it: the batch goes in parts, which the images of that kernel, each with a scale of its own, do not notice.
+    // kernel is the faster one all the same (64 x 64 x 56 x 56 -> 64 140 us fused, 96 so; 256 x 33 x 14 x 14 -> 17 65 and 37; 1024 x 64 x
+    // 16 x 16 -> 64 160 and 143), but they take no more than 256 MB for it: the batch goes in parts, which the images of that kernel,
+    // each with a scale of its own, do not notice.
     int64_t part = n;
     if (fusable) {
         const int64_t most = std::max<int64_t>(1, (256ll << 20) / (ko * ho * wo * (int64_t)sizeof(float)));

@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(kTA_ThreadsRaw, 1) conv_tmem_filters_kernel(
 // Scales: per filter, and per tile (raw: the converting warps see the whole box before they split it) or, from planes, per
 // image.  The converting warps also leave the range of every tile in the call's own scratch; conv_tmem_filters_kernel,
 // launched behind this one, computes the images that float16 pairs cannot hold.  A tile that shows that by itself is
-// not converted, multiplied or stored here.
+// neither converted nor stored here; what its stage happens to hold is multiplied, and nobody reads the sums.
 // Converting warps: with ten the boxes of up to 320 positions are held in registers (30 x 10 of a 28 x 28 image), larger ones are read
 // twice.  Against the kernel before, 256 images, 3 x 3: 32 -> 64 channels at 12 x 12 36 -> 23 us, 28 x 28 65 -> 44, 32 x 32 90 -> 61,
 // 40 x 40 146 -> 114, 60 x 60 298 -> 238; 16 -> 32 at 56 x 56 233 -> 151.

@@ -4,7 +4,7 @@
 // them again took 15 us at 512 x 512 x 512, of which the MMAs are one.  Here a CTA has one 128 x 128 tile and at most 128
 // values of k; it loads its float32 operands once into registers (sixteen 16-byte loads a thread, all in flight), splits
 // them into float16 pairs in shared memory and multiplies; the CTAs of a cluster are the slices of a tile's k and add up
-// through distributed shared memory: 15.3 -> 8.7 us, a 64-sample request of two hidden layers and a classifier 36 -> 24.4.  A's
+// through distributed shared memory: 15.3 -> 8.7 us, a 64-sample request of two hidden layers and a classifier 36 -> 24.6.  A's
 // planes are K-major, B's stay as they lie (rows of n, an MN-major operand), so nothing is transposed.
 //
 // What bounds it is the chain: operands 1.4 us after the wait, their ranges 1.1, planes 1.3, the last MMA 0.7 behind them, sums

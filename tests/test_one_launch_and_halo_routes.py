@@ -32,7 +32,8 @@ def port():
 # n, c, h, w, ko, kh, kw, stride, pad.  Halo kernel: odd extents at strides 2 and 3 (sub-images of unequal size); taps that
 # leave sub-images unread; half of a channel block, and one channel more; k of two and three drains (c = 97, 193 with
 # nine taps; 33 with twenty-five); 17 and 129 filters; a tile of one row; partial last tiles.  Paired rows: an odd number of
-# rows, a row of 128 positions, 16 and 64 filters, 8 channels, an even filter, rows that no tensor map covers.  Halo again: more
+# rows, a row of 128 positions, 16 and 64 filters, 8 channels, an even filter, rows that no tensor map covers, filters (4 x 3, 6 x 2) that fit
+# single blocks or pairs of them only.  Halo again: more
 # filters than have their bias in shared memory; 1 x 1 filters with and without a stride, a strided layer of one tile; filters that are streamed by rows of
 # taps and, of a strided layer, by threes.
 LAYERS = [(2, 48, 57, 57, 96, 3, 3, 2, 1), (1, 33, 20, 23, 70, 3, 3, 3, 1), (2, 40, 30, 33, 64, 1, 1, 2, 0), (1, 16, 41, 40, 65, 5, 5, 2, 2),
@@ -40,7 +41,7 @@ LAYERS = [(2, 48, 57, 57, 96, 3, 3, 2, 1), (1, 33, 20, 23, 70, 3, 3, 3, 1), (2, 
           (2, 9, 33, 64, 80, 3, 3, 1, 1), (2, 32, 28, 28, 64, 3, 3, 1, 1), (1, 8, 27, 33, 16, 3, 3, 1, 1), (1, 20, 16, 126, 33, 3, 3, 1, 1),
           (1, 31, 30, 29, 48, 2, 2, 1, 0), (1, 17, 12, 60, 17, 1, 5, 1, 0), (1, 40, 20, 30, 300, 3, 3, 1, 1),
           (2, 48, 30, 33, 64, 1, 1, 2, 0), (1, 16, 65, 64, 40, 3, 3, 2, 1), (1, 64, 9, 8, 70, 3, 3, 2, 1), (1, 70, 20, 30, 33, 1, 1, 1, 0),
-          (1, 130, 30, 33, 100, 5, 5, 1, 2), (1, 100, 41, 37, 130, 5, 5, 2, 2), (1, 70, 20, 61, 130, 5, 5, 1, 0)]
+          (1, 16, 40, 82, 48, 4, 3, 1, 1), (3, 32, 40, 46, 64, 6, 2, 1, 1), (1, 130, 30, 33, 100, 5, 5, 1, 2), (1, 100, 41, 37, 130, 5, 5, 2, 2), (1, 70, 20, 61, 130, 5, 5, 1, 0)]
 
 
 @pytest.mark.parametrize("layer", LAYERS)
